@@ -172,13 +172,11 @@ __global__ void __launch_bounds__(256) rs_adamw8bit_kernel(const float* const* g
                                                            const unsigned* flags, unsigned epoch, long long max_cycles,
                                                            KernelStatus* status) {
   __shared__ int sh_ok;
-  __shared__ float cs[256], cu[256], red_m[8], red_v[8];
-  __shared__ uint8_t ts[cbk::kTable], tu[cbk::kTable];
-  cs[threadIdx.x] = cb_signed[threadIdx.x];
-  cu[threadIdx.x] = cb_unsigned[threadIdx.x];
-  __syncthreads();
-  cbk::build_table(cs, ts);
-  cbk::build_table(cu, tu);
+  __shared__ float red_m[8], red_v[8];
+  __shared__ cbk::Book<true> cs;
+  __shared__ cbk::Book<false> cu;
+  cs.build(cb_signed);
+  cu.build(cb_unsigned);
   if (!cta_wait_peers(flags, W, rank, epoch, max_cycles, status, &sh_ok)) return;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   for (long b = blockIdx.x; b < nblocks; b += gridDim.x) {
@@ -186,8 +184,8 @@ __global__ void __launch_bounds__(256) rs_adamw8bit_kernel(const float* const* g
     float gr = 0.f;
     for (int p = 0; p < W; ++p) gr += grads[p][static_cast<long>(rank) * S + i];
     gr *= scale;
-    const float mm = a.beta1 * (cs[mq[i]] * mabs[b]) + (1.f - a.beta1) * gr;
-    const float vv = a.beta2 * (cu[vq[i]] * vabs[b]) + (1.f - a.beta2) * gr * gr;
+    const float mm = a.beta1 * (cs.value[mq[i]] * mabs[b]) + (1.f - a.beta1) * gr;
+    const float vv = a.beta2 * (cu.value[vq[i]] * vabs[b]) + (1.f - a.beta2) * gr * gr;
     float wt = static_cast<float>(p_shard[i]);
     if (wd_mask == nullptr || wd_mask[b]) wt *= (1.f - a.lr * a.wd);
     wt -= (a.lr / a.bc1) * mm / (sqrtf(vv) / a.bc2_sqrt + a.eps);
@@ -201,8 +199,8 @@ __global__ void __launch_bounds__(256) rs_adamw8bit_kernel(const float* const* g
     am = red_m[0]; av = red_v[0];
 #pragma unroll
     for (int k = 1; k < 8; ++k) { am = fmaxf(am, red_m[k]); av = fmaxf(av, red_v[k]); }
-    mq[i] = static_cast<uint8_t>(cbk::nearest_code(cs, ts, mm / fmaxf(am, 1e-30f)));
-    vq[i] = static_cast<uint8_t>(cbk::nearest_code(cu, tu, vv / fmaxf(av, 1e-30f)));
+    mq[i] = static_cast<uint8_t>(cs.nearest(mm / fmaxf(am, 1e-30f)));
+    vq[i] = static_cast<uint8_t>(cu.nearest(vv / fmaxf(av, 1e-30f)));
     if (threadIdx.x == 0) { mabs[b] = am; vabs[b] = av; }
   }
 }

@@ -65,6 +65,13 @@ int nsa_adamw_step(void* p, const void* g, float* m, float* v, float* master, co
 int nsa_adamw8bit_step(void* p, const void* g, uint8_t* mq, float* mabs, uint8_t* vq, float* vabs,
                        const float* cb_signed, const float* cb_unsigned, const float* grad_scale, long n, int p_fp32,
                        int g_fp32, int step, float lr, float b1, float b2, float eps, float wd, cudaStream_t st);
+/* The same updates over a list of tensors, one launch per 48.  words: 7 per tensor, {p, g, m, v, a, b, n} with a =
+ * fp32 master copy or 0 and b unused for fp32 state, a / b = scales of the moments for 8-bit state. */
+int nsa_adamw_multi(const long long* words, int tensors, const float* grad_scale, int p_fp32, int g_fp32, int step,
+                    float lr, float b1, float b2, float eps, float wd, cudaStream_t st);
+int nsa_adamw8bit_multi(const long long* words, int tensors, const float* cb_signed, const float* cb_unsigned,
+                        const float* grad_scale, int p_fp32, int g_fp32, int step, float lr, float b1, float b2, float eps,
+                        float wd, cudaStream_t st);
 int nsa_sumsq_parts(void);
 int nsa_sumsq(const void* g, long n, int g_fp32, float* partial, float* out, int accumulate, cudaStream_t st);
 int nsa_cross_entropy(void* logits, const long* labels, float* loss_rows, const float* inv_count, long rows, int V,

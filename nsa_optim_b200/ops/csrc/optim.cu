@@ -2,7 +2,8 @@
 //   * fused AdamW (decoupled weight decay, bias correction, optional fp32 master copy);
 //   * 8-bit AdamW: moments stored as uint8 codes of a 256-entry dynamic-tree code book with
 //     one fp32 absmax per 256-element block (signed map for the first moment, unsigned for
-//     the second); one CTA per block: dequantise, update, block absmax, requantise;
+//     the second); one warp per block: dequantise, update, block absmax, requantise;
+//   both over lists of tensors in one launch;
 //   * sum of squares for the global gradient norm (deterministic two-stage reduction);
 //   * softmax cross-entropy over a (rows, vocab) bf16 logits block: per-row loss and the
 //     logits overwritten in place by d(loss)/d(logits).
@@ -32,25 +33,6 @@ struct AdamArgs {
   float lr, beta1, beta2, eps, wd, bc1, bc2_sqrt;   // bc1 = 1-beta1^t, bc2_sqrt = sqrt(1-beta2^t)
 };
 
-template <typename PT, typename GT>
-__global__ void __launch_bounds__(256) adamw_kernel(PT* __restrict__ p, const GT* __restrict__ g, float* __restrict__ m,
-                                                    float* __restrict__ v, float* __restrict__ master,
-                                                    const float* __restrict__ grad_scale, long n, AdamArgs a) {
-  const float gs = grad_scale ? *grad_scale : 1.f;
-  for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const float gr = static_cast<float>(g[i]) * gs;
-    float w = master ? master[i] : static_cast<float>(p[i]);
-    w *= (1.f - a.lr * a.wd);
-    const float mm = a.beta1 * m[i] + (1.f - a.beta1) * gr;
-    const float vv = a.beta2 * v[i] + (1.f - a.beta2) * gr * gr;
-    m[i] = mm;
-    v[i] = vv;
-    w -= (a.lr / a.bc1) * mm / (sqrtf(vv) / a.bc2_sqrt + a.eps);
-    if (master) master[i] = w;
-    p[i] = static_cast<PT>(w);
-  }
-}
-
 __device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
   const float4 x = *reinterpret_cast<const float4*>(p);
   v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
@@ -71,78 +53,142 @@ __device__ __forceinline__ void store4(bf16* p, const float (&v)[4]) {
   *reinterpret_cast<uint2*>(p) = x;
 }
 
-// A CTA of 256 threads takes four 256-element quantisation blocks per iteration: 64 threads per
-// block, four consecutive elements per thread (8- or 16-byte loads of p and g, 4-byte loads of
-// the state codes).
+// ------------------------------------------------------------------------------------
+// AdamW updates over a list of tensors.  A model has hundreds of parameters and most of them (norms,
+// per-head vectors, convolution taps) are too small to fill the GPU for the time a launch takes, so one
+// launch updates up to kMaxItems of them: the work is numbered through all tensors, and a CTA that
+// walks it moves on in the list (uniform constant-memory reads) whenever its number passes an end.
+// ------------------------------------------------------------------------------------
+constexpr int kMaxItems = 48;         // 48 x 64 bytes of kernel arguments
+struct AdamItem {
+  void* p;
+  const void* g;
+  void* m;             // fp32, or uint8 codes
+  void* v;
+  float* a;            // fp32 master copy or null; 8-bit: scales of the first moment
+  float* b;            // 8-bit: scales of the second moment
+  long n;              // elements
+  long end;            // units (chunks, blocks) up to and including this tensor; -end - 1 for tensors whose
+};                     //   addresses do not allow 16-byte accesses (fp32 state only)
+struct AdamList {
+  AdamItem item[kMaxItems];
+  int count;
+};
+
+// fp32 state: bound by memory (12 to 28 bytes per element).  A unit is 1024 elements, four consecutive ones
+// per thread with 8- or 16-byte accesses.
 template <typename PT, typename GT>
-__global__ void __launch_bounds__(256) adamw8bit_kernel(PT* __restrict__ p, const GT* __restrict__ g,
-                                                        uint8_t* __restrict__ mq, float* __restrict__ mabs,
-                                                        uint8_t* __restrict__ vq, float* __restrict__ vabs,
-                                                        const float* __restrict__ cb_signed,
-                                                        const float* __restrict__ cb_unsigned,
-                                                        const float* __restrict__ grad_scale, long nblocks, AdamArgs a) {
-  __shared__ float cs[256], cu[256];
-  __shared__ uint8_t ts[cbk::kTable], tu[cbk::kTable];
-  __shared__ float red_m[8], red_v[8];
-  cs[threadIdx.x] = cb_signed[threadIdx.x];
-  cu[threadIdx.x] = cb_unsigned[threadIdx.x];
-  __syncthreads();
-  cbk::build_table(cs, ts);
-  cbk::build_table(cu, tu);
-  __syncthreads();
+__global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ AdamList list, const float* __restrict__ grad_scale,
+                                                    long units, AdamArgs a) {
   const float gs = grad_scale ? *grad_scale : 1.f;
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const int grp = threadIdx.x >> 6, t64 = threadIdx.x & 63;
-  const long quads = (nblocks + 3) / 4;
   const float decay = 1.f - a.lr * a.wd, step_size = a.lr / a.bc1;
-  for (long q = blockIdx.x; q < quads; q += gridDim.x) {
-    const long b = q * 4 + grp;
-    const bool live = b < nblocks;
-    const long i = b * 256 + t64 * 4;
-    float mm[4], vv[4];
-    float am = 0.f, av = 0.f;
-    if (live) {
-      float gr[4], wt[4];
+  int k = 0;
+  long first = 0;                     // first unit of item k
+  for (long u = blockIdx.x; u < units; u += gridDim.x) {
+    long end = list.item[k].end;
+    while (u >= (end < 0 ? -end - 1 : end)) {
+      first = end < 0 ? -end - 1 : end;
+      end = list.item[++k].end;
+    }
+    const AdamItem& it = list.item[k];
+    PT* p = static_cast<PT*>(it.p);
+    const GT* g = static_cast<const GT*>(it.g);
+    float *m = static_cast<float*>(it.m), *v = static_cast<float*>(it.v), *master = it.a;
+    const long i = (u - first) * 1024 + threadIdx.x * 4;
+    auto update = [&](float& w, float gr, float& mm, float& vv) {
+      gr *= gs;
+      w *= decay;
+      mm = a.beta1 * mm + (1.f - a.beta1) * gr;
+      vv = a.beta2 * vv + (1.f - a.beta2) * gr * gr;
+      w -= step_size * mm / (sqrtf(vv) / a.bc2_sqrt + a.eps);
+    };
+    if (end > 0 && i + 4 <= it.n) {
+      float w[4], gr[4], mm[4], vv[4];
       load4(g + i, gr);
-      load4(p + i, wt);
-      const uchar4 mc = *reinterpret_cast<const uchar4*>(mq + i);
-      const uchar4 vc = *reinterpret_cast<const uchar4*>(vq + i);
-      const float ms = mabs[b], vs = vabs[b];
-      const float m0[4] = {cs[mc.x], cs[mc.y], cs[mc.z], cs[mc.w]};
-      const float v0[4] = {cu[vc.x], cu[vc.y], cu[vc.z], cu[vc.w]};
+      load4(m + i, mm);
+      load4(v + i, vv);
+      if (master) load4(master + i, w);
+      else load4(p + i, w);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float x = gr[k] * gs;
-        mm[k] = a.beta1 * (m0[k] * ms) + (1.f - a.beta1) * x;
-        vv[k] = a.beta2 * (v0[k] * vs) + (1.f - a.beta2) * x * x;
-        wt[k] = wt[k] * decay - step_size * mm[k] / (sqrtf(vv[k]) / a.bc2_sqrt + a.eps);
-        am = fmaxf(am, fabsf(mm[k]));
-        av = fmaxf(av, vv[k]);
+      for (int j = 0; j < 4; ++j) update(w[j], gr[j], mm[j], vv[j]);
+      store4(m + i, mm);
+      store4(v + i, vv);
+      if (master) store4(master + i, w);
+      store4(p + i, w);
+    } else {
+      for (long e = i; e < min(i + 4, it.n); ++e) {
+        float w = master ? master[e] : static_cast<float>(p[e]), mm = m[e], vv = v[e];
+        update(w, static_cast<float>(g[e]), mm, vv);
+        m[e] = mm;
+        v[e] = vv;
+        if (master) master[e] = w;
+        p[e] = static_cast<PT>(w);
       }
-      store4(p + i, wt);
+    }
+  }
+}
+
+// 8-bit state.  A warp owns a 256-element quantisation block (two groups of four consecutive elements per
+// lane), so the block's absolute maximum is a warp reduction and the CTA never synchronises; decoding
+// is one shared-memory read per value and encoding two (codebook.cuh).
+template <typename PT, typename GT>
+__global__ void __launch_bounds__(256, 4) adamw8bit_kernel(const __grid_constant__ AdamList list,
+                                                           const float* __restrict__ cb_signed,
+                                                           const float* __restrict__ cb_unsigned,
+                                                           const float* __restrict__ grad_scale, long nblocks, AdamArgs a) {
+  __shared__ cbk::Book<true> cs;
+  __shared__ cbk::Book<false> cu;
+  cs.build(cb_signed);
+  cu.build(cb_unsigned);
+  const float gs = grad_scale ? *grad_scale : 1.f;
+  const int lane = threadIdx.x & 31;
+  const float decay = 1.f - a.lr * a.wd, step_size = a.lr / a.bc1;
+  int k = 0;
+  long first = 0;                     // first block of item k
+  for (long u = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5); u < nblocks; u += static_cast<long>(gridDim.x) * 8) {
+    while (u >= list.item[k].end) first = list.item[k++].end;
+    const AdamItem& it = list.item[k];
+    PT* p = static_cast<PT*>(it.p);
+    const GT* g = static_cast<const GT*>(it.g);
+    uint8_t *mq = static_cast<uint8_t*>(it.m), *vq = static_cast<uint8_t*>(it.v);
+    const long b = u - first, i = b * 256 + lane * 4;
+    float gr[2][4], wt[2][4], mm[2][4], vv[2][4];
+    uchar4 mc[2], vc[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      load4(g + i + h * 128, gr[h]);
+      load4(p + i + h * 128, wt[h]);
+      mc[h] = *reinterpret_cast<const uchar4*>(mq + i + h * 128);
+      vc[h] = *reinterpret_cast<const uchar4*>(vq + i + h * 128);
+    }
+    const float ms = it.a[b], vs = it.b[b];
+    float am = 0.f, av = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float m0[4] = {cs.value[mc[h].x], cs.value[mc[h].y], cs.value[mc[h].z], cs.value[mc[h].w]};
+      const float v0[4] = {cu.value[vc[h].x], cu.value[vc[h].y], cu.value[vc[h].z], cu.value[vc[h].w]};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float x = gr[h][e] * gs;
+        mm[h][e] = a.beta1 * (m0[e] * ms) + (1.f - a.beta1) * x;
+        vv[h][e] = a.beta2 * (v0[e] * vs) + (1.f - a.beta2) * x * x;
+        wt[h][e] = wt[h][e] * decay - step_size * mm[h][e] / (sqrtf(vv[h][e]) / a.bc2_sqrt + a.eps);
+        am = fmaxf(am, fabsf(mm[h][e]));
+        av = fmaxf(av, vv[h][e]);
+      }
+      store4(p + i + h * 128, wt[h]);
     }
     am = warp_max(am);
     av = warp_max(av);
-    __syncthreads();               // previous iteration's readers of red_* are done
-    if (l == 0) { red_m[w] = am; red_v[w] = av; }
-    __syncthreads();
-    am = fmaxf(red_m[2 * grp], red_m[2 * grp + 1]);
-    av = fmaxf(red_v[2 * grp], red_v[2 * grp + 1]);
-    if (live) {
-      const float dm = fmaxf(am, 1e-30f), dv = fmaxf(av, 1e-30f);
-      uchar4 mc, vc;
-      mc.x = static_cast<uint8_t>(cbk::nearest_code(cs, ts, mm[0] / dm));
-      mc.y = static_cast<uint8_t>(cbk::nearest_code(cs, ts, mm[1] / dm));
-      mc.z = static_cast<uint8_t>(cbk::nearest_code(cs, ts, mm[2] / dm));
-      mc.w = static_cast<uint8_t>(cbk::nearest_code(cs, ts, mm[3] / dm));
-      vc.x = static_cast<uint8_t>(cbk::nearest_code(cu, tu, vv[0] / dv));
-      vc.y = static_cast<uint8_t>(cbk::nearest_code(cu, tu, vv[1] / dv));
-      vc.z = static_cast<uint8_t>(cbk::nearest_code(cu, tu, vv[2] / dv));
-      vc.w = static_cast<uint8_t>(cbk::nearest_code(cu, tu, vv[3] / dv));
-      *reinterpret_cast<uchar4*>(mq + i) = mc;
-      *reinterpret_cast<uchar4*>(vq + i) = vc;
-      if (t64 == 0) { mabs[b] = am; vabs[b] = av; }
+    const float dm = fmaxf(am, 1e-30f), dv = fmaxf(av, 1e-30f);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      mc[h] = make_uchar4(cs.nearest(mm[h][0] / dm), cs.nearest(mm[h][1] / dm), cs.nearest(mm[h][2] / dm), cs.nearest(mm[h][3] / dm));
+      vc[h] = make_uchar4(cu.nearest(vv[h][0] / dv), cu.nearest(vv[h][1] / dv), cu.nearest(vv[h][2] / dv), cu.nearest(vv[h][3] / dv));
+      *reinterpret_cast<uchar4*>(mq + i + h * 128) = mc[h];
+      *reinterpret_cast<uchar4*>(vq + i + h * 128) = vc[h];
     }
+    if (lane == 0) { it.a[b] = am; it.b[b] = av; }
   }
 }
 
@@ -309,37 +355,89 @@ __global__ void __launch_bounds__(256) affine_dequant_kernel(const uint8_t* __re
 }
 }  // namespace
 
-// p: bf16 (p_fp32 = 0) or fp32; g: bf16 (g_fp32 = 0) or fp32; m, v fp32; master fp32 or null.
+// Seven 64-bit words per tensor: p, g, m, v, a, b (addresses; see AdamItem) and the element count.
+static bool next_item(const long long* w, AdamItem& it) {
+  it.p = reinterpret_cast<void*>(w[0]);
+  it.g = reinterpret_cast<const void*>(w[1]);
+  it.m = reinterpret_cast<void*>(w[2]);
+  it.v = reinterpret_cast<void*>(w[3]);
+  it.a = reinterpret_cast<float*>(w[4]);
+  it.b = reinterpret_cast<float*>(w[5]);
+  it.n = w[6];
+  return it.n > 0;
+}
+
+// fp32 state.  p: bf16 (p_fp32 = 0) or fp32; g: bf16 (g_fp32 = 0) or fp32; m, v fp32; a: fp32 master or null.
+extern "C" int nsa_adamw_multi(const long long* words, int tensors, const float* grad_scale, int p_fp32, int g_fp32, int step,
+                               float lr, float b1, float b2, float eps, float wd, cudaStream_t st) {
+  const AdamArgs a = make_args(step, lr, b1, b2, eps, wd);
+  for (int t = 0; t < tensors;) {
+    AdamList list;
+    list.count = 0;
+    long units = 0;
+    for (; t < tensors && list.count < kMaxItems; ++t) {
+      AdamItem& it = list.item[list.count];
+      if (!next_item(words + 7 * t, it)) continue;
+      const uintptr_t all = reinterpret_cast<uintptr_t>(it.m) | reinterpret_cast<uintptr_t>(it.v) | reinterpret_cast<uintptr_t>(it.a);
+      const bool wide = !(all & 15) && !(reinterpret_cast<uintptr_t>(it.p) & (p_fp32 ? 15 : 7)) &&
+                        !(reinterpret_cast<uintptr_t>(it.g) & (g_fp32 ? 15 : 7));
+      units += (it.n + 1023) / 1024;
+      it.end = wide ? units : -units - 1;
+      ++list.count;
+    }
+    if (units == 0) continue;
+    const int grid = grid_cap(units, 8);
+    if (p_fp32 && g_fp32) adamw_kernel<float, float><<<grid, 256, 0, st>>>(list, grad_scale, units, a);
+    else if (p_fp32) adamw_kernel<float, bf16><<<grid, 256, 0, st>>>(list, grad_scale, units, a);
+    else if (g_fp32) adamw_kernel<bf16, float><<<grid, 256, 0, st>>>(list, grad_scale, units, a);
+    else adamw_kernel<bf16, bf16><<<grid, 256, 0, st>>>(list, grad_scale, units, a);
+    nsa::count_launch();
+  }
+  return 0;
+}
 extern "C" int nsa_adamw_step(void* p, const void* g, float* m, float* v, float* master, const float* grad_scale,
                               long n, int p_fp32, int g_fp32, int step, float lr, float b1, float b2, float eps, float wd,
                               cudaStream_t st) {
-  if (n <= 0) return 0;
-  const AdamArgs a = make_args(step, lr, b1, b2, eps, wd);
-  const int grid = grid_cap((n + 255) / 256, 16);
-  if (p_fp32 && g_fp32) adamw_kernel<float, float><<<grid, 256, 0, st>>>((float*)p, (const float*)g, m, v, master, grad_scale, n, a);
-  else if (p_fp32) adamw_kernel<float, bf16><<<grid, 256, 0, st>>>((float*)p, (const bf16*)g, m, v, master, grad_scale, n, a);
-  else if (g_fp32) adamw_kernel<bf16, float><<<grid, 256, 0, st>>>((bf16*)p, (const float*)g, m, v, master, grad_scale, n, a);
-  else adamw_kernel<bf16, bf16><<<grid, 256, 0, st>>>((bf16*)p, (const bf16*)g, m, v, master, grad_scale, n, a);
-  nsa::count_launch();
-  return 0;
+  const long long w[7] = {(long long)p, (long long)g, (long long)m, (long long)v, (long long)master, 0, n};
+  return nsa_adamw_multi(w, 1, grad_scale, p_fp32, g_fp32, step, lr, b1, b2, eps, wd, st);
 }
 
-// n must be a multiple of 256.  cb_signed / cb_unsigned: device pointers to 256 fp32 entries.
+// 8-bit state: m, v codes; a, b their scales.  Element counts must be multiples of 256.
+// cb_signed / cb_unsigned: device pointers to 256 fp32 entries.
+extern "C" int nsa_adamw8bit_multi(const long long* words, int tensors, const float* cb_signed, const float* cb_unsigned,
+                                   const float* grad_scale, int p_fp32, int g_fp32, int step, float lr, float b1, float b2,
+                                   float eps, float wd, cudaStream_t st) {
+  for (int t = 0; t < tensors; ++t)
+    if (words[7 * t + 6] > 0 && words[7 * t + 6] % 256)
+      return nsa::fail(NSA_ERR_SHAPE, "adamw8bit: element count must be a multiple of 256");
+  const AdamArgs a = make_args(step, lr, b1, b2, eps, wd);
+  for (int t = 0; t < tensors;) {
+    AdamList list;
+    list.count = 0;
+    long nb = 0;
+    for (; t < tensors && list.count < kMaxItems; ++t) {
+      AdamItem& it = list.item[list.count];
+      if (!next_item(words + 7 * t, it)) continue;
+      nb += it.n / 256;
+      it.end = nb;
+      ++list.count;
+    }
+    if (nb == 0) continue;
+    const int grid = grid_cap((nb + 7) / 8, 4);
+    if (p_fp32 && g_fp32) adamw8bit_kernel<float, float><<<grid, 256, 0, st>>>(list, cb_signed, cb_unsigned, grad_scale, nb, a);
+    else if (p_fp32) adamw8bit_kernel<float, bf16><<<grid, 256, 0, st>>>(list, cb_signed, cb_unsigned, grad_scale, nb, a);
+    else if (g_fp32) adamw8bit_kernel<bf16, float><<<grid, 256, 0, st>>>(list, cb_signed, cb_unsigned, grad_scale, nb, a);
+    else adamw8bit_kernel<bf16, bf16><<<grid, 256, 0, st>>>(list, cb_signed, cb_unsigned, grad_scale, nb, a);
+    nsa::count_launch();
+  }
+  return 0;
+}
 extern "C" int nsa_adamw8bit_step(void* p, const void* g, uint8_t* mq, float* mabs, uint8_t* vq, float* vabs,
                                   const float* cb_signed, const float* cb_unsigned, const float* grad_scale, long n,
                                   int p_fp32, int g_fp32, int step, float lr, float b1, float b2, float eps, float wd,
                                   cudaStream_t st) {
-  if (n <= 0) return 0;
-  if (n % 256) return nsa::fail(NSA_ERR_SHAPE, "adamw8bit: element count must be a multiple of 256");
-  const AdamArgs a = make_args(step, lr, b1, b2, eps, wd);
-  const long nb = n / 256;
-  const int grid = grid_cap((nb + 3) / 4, 8);
-  if (p_fp32 && g_fp32) adamw8bit_kernel<float, float><<<grid, 256, 0, st>>>((float*)p, (const float*)g, mq, mabs, vq, vabs, cb_signed, cb_unsigned, grad_scale, nb, a);
-  else if (p_fp32) adamw8bit_kernel<float, bf16><<<grid, 256, 0, st>>>((float*)p, (const bf16*)g, mq, mabs, vq, vabs, cb_signed, cb_unsigned, grad_scale, nb, a);
-  else if (g_fp32) adamw8bit_kernel<bf16, float><<<grid, 256, 0, st>>>((bf16*)p, (const float*)g, mq, mabs, vq, vabs, cb_signed, cb_unsigned, grad_scale, nb, a);
-  else adamw8bit_kernel<bf16, bf16><<<grid, 256, 0, st>>>((bf16*)p, (const bf16*)g, mq, mabs, vq, vabs, cb_signed, cb_unsigned, grad_scale, nb, a);
-  nsa::count_launch();
-  return 0;
+  const long long w[7] = {(long long)p, (long long)g, (long long)mq, (long long)vq, (long long)mabs, (long long)vabs, n};
+  return nsa_adamw8bit_multi(w, 1, cb_signed, cb_unsigned, grad_scale, p_fp32, g_fp32, step, lr, b1, b2, eps, wd, st);
 }
 
 // out (device scalar) = [out +] sum(g^2).  partial: scratch of nsa_sumsq_parts() floats.

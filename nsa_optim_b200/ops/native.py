@@ -832,36 +832,51 @@ def _require_numel(what: str, t: Optional[Tensor], n: int) -> None:
         raise ValueError(f"optimizer state '{what}' has {t.numel()} elements, the kernel needs {n}")
 
 
-def adamw_step(p, g, m, v, master, step, lr, b1, b2, eps, wd, grad_scale):
-    n = p.numel()
-    _require_numel("grad", g, n)
-    _require_numel("exp_avg", m, n)
-    _require_numel("exp_avg_sq", v, n)
-    _require_numel("master", master, n)
+def _adamw_words(items, states) -> ctypes.Array:
+    """Seven 64-bit words per tensor, (p, g, m, v, a, b, n); every state tensor is checked against n."""
+    words = []
+    for it in items:
+        n = it[0].numel()
+        for (name, div), t in zip(states, it[1:]):
+            _require_numel(name, t, n // div)
+        words += [0 if t is None else t.data_ptr() for t in it] + [n]
+    return (c_longlong * len(words))(*words)
+
+
+def adamw_multi(items, step, lr, b1, b2, eps, wd, grad_scale) -> None:
+    """AdamW over (p, g, exp_avg, exp_avg_sq, master or None, None) tuples that share a device, dtypes and step."""
+    p, g = items[0][:2]
+    words = _adamw_words(items, (("grad", 1), ("exp_avg", 1), ("exp_avg_sq", 1), ("master", 1), ("", 1)))
     gs = None if grad_scale is None else grad_scale.reshape(1).float()
-    _check(load().nsa_adamw_step(_p(p), _p(g), _p(m), _p(v), _p(master), _p(gs), c_long(p.numel()),
-                                 c_int(int(p.dtype == torch.float32)), c_int(int(g.dtype == torch.float32)),
-                                 c_int(step), c_float(lr), c_float(b1), c_float(b2), c_float(eps), c_float(wd), _stream()))
+    _check(load().nsa_adamw_multi(words, c_int(len(items)), _p(gs), c_int(int(p.dtype == torch.float32)),
+                                  c_int(int(g.dtype == torch.float32)), c_int(step), c_float(lr), c_float(b1), c_float(b2),
+                                  c_float(eps), c_float(wd), _stream()))
 
 
-def adamw8bit_step(p, g, mq, mabs, vq, vabs, step, lr, b1, b2, eps, wd, grad_scale, block):
+def adamw8bit_multi(items, step, lr, b1, b2, eps, wd, grad_scale, block) -> None:
+    """8-bit AdamW over (p, g, codes m, codes v, scales m, scales v) tuples that share a device, dtypes and step."""
     if block != 256:
         raise ValueError("the native 8-bit AdamW kernel uses 256-element blocks")
-    n = p.numel()
-    if n % block:
-        raise ValueError(f"8-bit AdamW needs a multiple of {block} elements, got {n}")
-    _require_numel("grad", g, n)
-    _require_numel("exp_avg", mq, n)
-    _require_numel("exp_avg_sq", vq, n)
-    _require_numel("exp_avg_absmax", mabs, n // block)
-    _require_numel("exp_avg_sq_absmax", vabs, n // block)
+    for it in items:
+        if it[0].numel() % block:
+            raise ValueError(f"8-bit AdamW needs a multiple of {block} elements, got {it[0].numel()}")
+    p, g = items[0][:2]
+    words = _adamw_words(items, (("grad", 1), ("exp_avg", 1), ("exp_avg_sq", 1), ("exp_avg_absmax", block),
+                                 ("exp_avg_sq_absmax", block)))
     gs = None if grad_scale is None else grad_scale.reshape(1).float()
     cs = quant.codebook(8, True, p.device)
     cu = quant.codebook(8, False, p.device)
-    _check(load().nsa_adamw8bit_step(_p(p), _p(g), _p(mq), _p(mabs), _p(vq), _p(vabs), _p(cs), _p(cu), _p(gs),
-                                     c_long(p.numel()), c_int(int(p.dtype == torch.float32)),
-                                     c_int(int(g.dtype == torch.float32)), c_int(step), c_float(lr), c_float(b1),
-                                     c_float(b2), c_float(eps), c_float(wd), _stream()))
+    _check(load().nsa_adamw8bit_multi(words, c_int(len(items)), _p(cs), _p(cu), _p(gs), c_int(int(p.dtype == torch.float32)),
+                                      c_int(int(g.dtype == torch.float32)), c_int(step), c_float(lr), c_float(b1),
+                                      c_float(b2), c_float(eps), c_float(wd), _stream()))
+
+
+def adamw_step(p, g, m, v, master, step, lr, b1, b2, eps, wd, grad_scale):
+    adamw_multi([(p, g, m, v, master, None)], step, lr, b1, b2, eps, wd, grad_scale)
+
+
+def adamw8bit_step(p, g, mq, mabs, vq, vabs, step, lr, b1, b2, eps, wd, grad_scale, block):
+    adamw8bit_multi([(p, g, mq, vq, mabs, vabs)], step, lr, b1, b2, eps, wd, grad_scale, block)
 
 
 # --------------------------------------------------------------------------------------

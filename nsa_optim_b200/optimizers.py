@@ -89,6 +89,28 @@ def _grad_of(p: Tensor) -> Optional[Tensor]:
     return g if g is not None else p.grad
 
 
+class _NativeBatch:
+    """Native updates of one parameter group, collected and launched as a few kernels over lists of
+    tensors: those that share device, dtypes, state form and step number go together."""
+
+    def __init__(self):
+        self.lists: Dict[tuple, list] = {}
+
+    def add(self, quantised: bool, step: int, p: Tensor, g: Tensor, *state: Optional[Tensor]) -> None:
+        self.lists.setdefault((quantised, step, p.device, p.dtype, g.dtype), []).append((p, g) + state)
+
+    def run(self, lr, b1, b2, eps, wd, grad_scale, block: int = 256) -> None:
+        if not self.lists:
+            return
+        from . import ops
+        nat = ops.native_module()
+        for (quantised, step, *_), items in self.lists.items():
+            if quantised:
+                nat.adamw8bit_multi(items, step, lr, b1, b2, eps, wd, grad_scale, block)
+            else:
+                nat.adamw_multi(items, step, lr, b1, b2, eps, wd, grad_scale)
+
+
 def _scaled(grad: Tensor, grad_scale: Optional[Tensor]) -> Tensor:
     g = grad.float()
     return g if grad_scale is None else g * grad_scale.to(g.device, torch.float32)
@@ -119,6 +141,7 @@ class AdamW(Optimizer):
         for group in self.param_groups:
             b1, b2 = group["betas"]
             lr, eps, wd = group["lr"], group["eps"], group["weight_decay"]
+            batch = _NativeBatch()
             for p in group["params"]:
                 g_ = _grad_of(p)
                 if g_ is None:
@@ -130,8 +153,7 @@ class AdamW(Optimizer):
                 t = st["step"]
                 nat = _native_for(p)
                 if nat is not None and nat.supports("adamw", p):
-                    nat.adamw_step(p, g_, st["exp_avg"], st["exp_avg_sq"], st.get("master"),
-                                   t, lr, b1, b2, eps, wd, grad_scale)
+                    batch.add(False, t, p, g_, st["exp_avg"], st["exp_avg_sq"], st.get("master"), None)
                     continue
                 g = _scaled(g_, grad_scale)
                 w = st.get("master")
@@ -142,6 +164,7 @@ class AdamW(Optimizer):
                 denom = (st["exp_avg_sq"].sqrt() / math.sqrt(1 - b2 ** t)).add_(eps)
                 w.addcdiv_(st["exp_avg"], denom, value=-lr / (1 - b1 ** t))
                 p.copy_(w)
+            batch.run(lr, b1, b2, eps, wd, grad_scale)
         return loss
 
 
@@ -195,6 +218,7 @@ class AdamWLowBit(Optimizer):
         for group in self.param_groups:
             b1, b2 = group["betas"]
             lr, eps, wd = group["lr"], group["eps"], group["weight_decay"]
+            batch = _NativeBatch()
             for p in group["params"]:
                 g_ = _grad_of(p)
                 if g_ is None:
@@ -207,13 +231,8 @@ class AdamWLowBit(Optimizer):
                 quantised = st["exp_avg"].dtype == torch.uint8
                 nat = _native_for(p)
                 if nat is not None and nat.supports("adamw_lowbit", p) and (self.bits == 8 or not quantised):
-                    if quantised:
-                        nat.adamw8bit_step(p, g_, st["exp_avg"], st["exp_avg_absmax"],
-                                           st["exp_avg_sq"], st["exp_avg_sq_absmax"],
-                                           t, lr, b1, b2, eps, wd, grad_scale, B)
-                    else:
-                        nat.adamw_step(p, g_, st["exp_avg"], st["exp_avg_sq"], None,
-                                       t, lr, b1, b2, eps, wd, grad_scale)
+                    batch.add(quantised, t, p, g_, st["exp_avg"], st["exp_avg_sq"], st.get("exp_avg_absmax"),
+                              st.get("exp_avg_sq_absmax"))
                     continue
                 g = _scaled(g_, grad_scale).reshape(-1)
                 if quantised:
@@ -231,6 +250,7 @@ class AdamWLowBit(Optimizer):
                 if quantised:
                     st["exp_avg"], st["exp_avg_absmax"] = quant.quantize_blockwise(m, self.bits, True, B)
                     st["exp_avg_sq"], st["exp_avg_sq_absmax"] = quant.quantize_blockwise(v, self.bits, False, B)
+            batch.run(lr, b1, b2, eps, wd, grad_scale, B)
         return loss
 
 

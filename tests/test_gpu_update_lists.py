@@ -1,0 +1,82 @@
+"""AdamW updates over lists of tensors: the 8-bit code search against brute force at every boundary of the
+code books, and a list (several launches, odd lengths, unaligned views) against one call per tensor."""
+import numpy as np
+import pytest
+import torch
+
+from nsa_optim_b200.ops import quant
+
+pytestmark = pytest.mark.gpu
+HYPER = (1e-2, 0.9, 0.95, 1e-8, 0.1)
+
+
+def _nearest(x, book):
+    """Index of the nearest entry, ties to the lower one, with the comparison in fp32."""
+    lo = np.clip(np.searchsorted(book, x, side="right") - 1, 0, 254)
+    return np.where(x - book[lo] <= book[lo + 1] - x, lo, lo + 1)
+
+
+@pytest.mark.parametrize("signed", [True, False])
+def test_codes_at_every_boundary(native, signed):
+    book = quant.codebook(8, signed, "cpu").numpy()
+    mid = ((book[:-1] + book[1:]) / 2).astype(np.float32)
+    x = np.concatenate([book, mid] + [np.nextafter(mid, np.float32(s)) for s in (-2, 2)] + [np.nextafter(book, np.float32(s)) for s in (-2, 2)])
+    x = np.clip(np.concatenate([x, np.float32([0.0, -0.0, 1e-30, 1e-9])]), -1 if signed else 0, 1).astype(np.float32)
+    x = np.pad(x, (0, -x.size % 255)).reshape(-1, 255)
+    x = np.concatenate([np.ones((x.shape[0], 1), np.float32), x], 1)              # every block has absmax 1
+    n = x.size
+    # first moment: beta1 = 0 makes it the gradient.  second: gradient 0 and beta2 = 1 make it the decoded old
+    # state, so there the books' own entries are checked through beta2 = 0 with g = sqrt(x), as far as squares reach
+    g = torch.from_numpy(x.reshape(-1) if signed else np.sqrt(x.reshape(-1))).cuda()
+    p, mq, vq = torch.zeros(n, device="cuda"), *(torch.zeros(n, dtype=torch.uint8, device="cuda") for _ in range(2))
+    ma, va = torch.zeros(n // 256, device="cuda"), torch.zeros(n // 256, device="cuda")
+    native.adamw8bit_step(p, g, mq, ma, vq, va, 1, 1e-3, 0.0, 0.0, 1e-8, 0.0, None, 256)
+    assert torch.equal(ma, torch.ones_like(ma)) and torch.equal(va, torch.ones_like(va))
+    gn = g.cpu().numpy()
+    want = _nearest(gn if signed else (gn * gn).astype(np.float32), book)
+    assert np.array_equal((mq if signed else vq).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("pdt,gdt,master", [(torch.bfloat16, torch.bfloat16, True), (torch.bfloat16, torch.float32, False),
+                                            (torch.float32, torch.float32, False)])
+def test_list_of_fp32_state_updates_equals_single_calls(native, pdt, gdt, master):
+    torch.manual_seed(0)
+    sizes = [1, 3, 4, 1023, 1024, 1025, 5000, 64, 0, 70000] + [33 + k for k in range(50)]       # more than one launch
+    def make():
+        torch.manual_seed(1)
+        out = []
+        for i, n in enumerate(sizes):
+            off = i % 3                                                                      # some views are unaligned
+            f = lambda dt: torch.randn(n + off, device="cuda").to(dt)[off:]                   # noqa: E731
+            p = f(pdt)
+            out.append((p, f(gdt), f(torch.float32) * 0.1, f(torch.float32).abs() * 0.1, p.float().clone() if master else None, None))
+        return out
+    a, b = make(), make()
+    scale = torch.tensor(0.5, device="cuda")
+    native.adamw_multi(a, 3, *HYPER, scale)
+    for it in b:
+        if it[0].numel():
+            native.adamw_step(it[0], it[1], it[2], it[3], it[4], 3, *HYPER, scale)
+    for x, y in zip(a, b):
+        assert all(torch.equal(s, t) for s, t in zip(x, y) if s is not None)
+
+
+@pytest.mark.parametrize("pdt,gdt", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
+def test_list_of_8bit_updates_equals_single_calls(native, pdt, gdt):
+    sizes = [256, 512, 256 * 9, 256 * 33] + [256] * 50
+    def make():
+        torch.manual_seed(2)
+        out = []
+        for n in sizes:
+            out.append((torch.randn(n, device="cuda").to(pdt), torch.randn(n, device="cuda").to(gdt),
+                        torch.randint(0, 256, (n,), device="cuda", dtype=torch.uint8), torch.randint(0, 256, (n,), device="cuda", dtype=torch.uint8),
+                        torch.rand(n // 256, device="cuda"), torch.rand(n // 256, device="cuda")))
+        return out
+    a, b = make(), make()
+    native.adamw8bit_multi(a, 3, *HYPER, None, 256)
+    for p, g, mq, vq, ma, va in b:
+        native.adamw8bit_step(p, g, mq, ma, vq, va, 3, *HYPER, None, 256)
+    for x, y in zip(a, b):
+        assert all(torch.equal(s, t) for s, t in zip(x, y))
+    with pytest.raises(ValueError):
+        native.adamw8bit_multi([(torch.zeros(100, device="cuda"),) * 6], 1, *HYPER, None, 256)
