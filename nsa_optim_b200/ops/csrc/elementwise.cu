@@ -890,236 +890,197 @@ __global__ void __launch_bounds__(256) rope_kernel(const bf16* __restrict__ x, c
 }
 
 // ------------------------------------------------------------------------------------
-// Causal depthwise conv1d, width W <= 4, channel-last (B, T, C), optional bias and SiLU.
-// A CTA owns CT_C channels and walks CT_SEG consecutive tiles of CT_T time steps.  The rows of a
-// tile reach shared memory through cp.async, the next tile's rows while the current tile is
-// computed, so global loads are always in flight and never on a thread's dependency chain; the
-// taps read shared memory.  Thread (rg, c8): 8 channels c8*8.., rows rg, rg+16, ... of the tile.
+// Causal depthwise conv1d, width 4, channel-last (B, T, C), optional bias and SiLU.
+// Bound by memory when the arithmetic stays out of the way: a lane owns four channels (8-byte
+// accesses, a warp covers 256 contiguous bytes of a row) and walks `rows` consecutive time steps
+// with the last three rows in registers, so every element is read and widened once and no row
+// passes through shared memory; the next four rows are in flight while four are computed.  The
+// taps are packed fp32 FMAs (two channels per instruction).  The eight warps of a CTA own eight
+// consecutive time segments.
 // ------------------------------------------------------------------------------------
-constexpr int CT_T = 64, CT_C = 128, CT_SEG = 8, CT_THREADS = 256, CT_RG = CT_THREADS / (CT_C / 8);
-constexpr int CONV_TCHUNK = CT_T * CT_SEG;
+constexpr int CT_WARPS = 8, CT_C = 128, CT_U = 4;
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pred) {   // zero fill when !pred
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  const int n = pred ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gmem), "r"(n) : "memory");
+// Two fp32 lanes per instruction; each lane rounds as the scalar instruction does.
+__device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+        "l"(reinterpret_cast<const unsigned long long&>(c)));
+  return d;
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-template <int W>
-__global__ void __launch_bounds__(CT_THREADS) conv1d_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                                                const bf16* __restrict__ bias, bf16* __restrict__ y,
-                                                                int T, int C, long ldx, int act) {
-  constexpr int XR = CT_T + W - 1;
-  __shared__ __align__(16) bf16 sx[2][XR * CT_C];                // x rows t0-(W-1) .. t0+CT_T-1 of a tile
-  const int c8 = threadIdx.x % (CT_C / 8), rg = threadIdx.x / (CT_C / 8);
-  const int c = blockIdx.x * CT_C + c8 * 8;
-  const long b = blockIdx.z;
-  const bool c_ok = c < C;
-  const int seg0 = blockIdx.y * CT_SEG;
-  const int n_tiles = min(CT_SEG, (T + CT_T - 1) / CT_T - seg0);
-  auto load_tile = [&](int n, int buf) {
-    const int t0 = (seg0 + n) * CT_T;
-    for (int i = rg; i < XR; i += CT_RG) {
-      const int t = t0 - (W - 1) + i;
-      const bool ok = c_ok && t >= 0 && t < T;
-      cp_async16(sx[buf] + i * CT_C + c8 * 8, ok ? x + (b * T + t) * ldx + c : x, ok);
-    }
-    cp_async_commit();
-  };
-  load_tile(0, 0);
-  float wv[W][8], bv[8];
+struct Quad {        // four channels
+  float2 a, b;
+};
+__device__ __forceinline__ Quad quad_unpack(const uint2& u) {
+  Quad q;
+  q.a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+  q.b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+  return q;
+}
+__device__ __forceinline__ uint2 quad_pack(const Quad& q) {
+  uint2 u;
+  *reinterpret_cast<__nv_bfloat162*>(&u.x) = __floats2bfloat162_rn(q.a.x, q.a.y);
+  *reinterpret_cast<__nv_bfloat162*>(&u.y) = __floats2bfloat162_rn(q.b.x, q.b.y);
+  return u;
+}
+__device__ __forceinline__ Quad quad_fma(const Quad& x, const Quad& y, const Quad& z) {
+  return Quad{fma2(x.a, y.a, z.a), fma2(x.b, y.b, z.b)};
+}
+__device__ __forceinline__ Quad quad_zero() { return Quad{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
+__device__ __forceinline__ void conv_taps(const bf16* __restrict__ w, const bf16* __restrict__ bias, int c, bool c_ok,
+                                          Quad (&wv)[4], Quad& bv) {
+  float t[4][4], s[4];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    bv[k] = (bias && c_ok) ? __bfloat162float(bias[c + k]) : 0.f;
+  for (int k = 0; k < 4; ++k) {
+    s[k] = (bias && c_ok) ? __bfloat162float(bias[c + k]) : 0.f;
 #pragma unroll
-    for (int j = 0; j < W; ++j) wv[j][k] = c_ok ? __bfloat162float(w[(c + k) * W + j]) : 0.f;
+    for (int j = 0; j < 4; ++j) t[j][k] = c_ok ? __bfloat162float(w[(c + k) * 4 + j]) : 0.f;
   }
-  for (int n = 0; n < n_tiles; ++n) {
-    const int buf = n & 1;
-    if (n + 1 < n_tiles) { load_tile(n + 1, buf ^ 1); cp_async_wait<1>(); }
-    else cp_async_wait<0>();
-    __syncthreads();
-    const int t0 = (seg0 + n) * CT_T;
-    if (c_ok) {
-      for (int i = rg; i < CT_T; i += CT_RG) {
-        const int t = t0 + i;
-        if (t >= T) break;
-        float o[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) o[k] = bv[k];
+  for (int j = 0; j < 4; ++j) wv[j] = Quad{make_float2(t[j][0], t[j][1]), make_float2(t[j][2], t[j][3])};
+  bv = Quad{make_float2(s[0], s[1]), make_float2(s[2], s[3])};
+}
+
+__global__ void __launch_bounds__(CT_WARPS * 32) conv1d_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
+                                                                   const bf16* __restrict__ bias, bf16* __restrict__ y,
+                                                                   int T, int C, long ldx, int act, int rows) {
+  const int c = blockIdx.x * CT_C + (threadIdx.x & 31) * 4;
+  const int t0 = (blockIdx.y * CT_WARPS + (threadIdx.x >> 5)) * rows;
+  if (c >= C || t0 >= T) return;
+  const bf16* xp = x + static_cast<long>(blockIdx.z) * T * ldx + c;
+  bf16* yp = y + static_cast<long>(blockIdx.z) * T * C + c;
+  const int t1 = min(t0 + rows, T);
+  auto load = [&](int t) {
+    return t >= 0 && t < t1 ? *reinterpret_cast<const uint2*>(xp + t * ldx) : make_uint2(0u, 0u);
+  };
+  uint2 next[CT_U];
 #pragma unroll
-        for (int j = 0; j < W; ++j) {
-          float xv[8];
-          unpack8(*reinterpret_cast<const uint4*>(sx[buf] + (i + j) * CT_C + c8 * 8), xv);
+  for (int u = 0; u < CT_U; ++u) next[u] = load(t0 + u);
+  Quad x0 = quad_unpack(load(t0 - 3)), x1 = quad_unpack(load(t0 - 2)), x2 = quad_unpack(load(t0 - 1));
+  Quad wv[4], bv;
+  conv_taps(w, bias, c, true, wv, bv);
+  for (int t = t0; t < t1; t += CT_U) {
+    uint2 cur[CT_U];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) o[k] += wv[j][k] * xv[k];
-        }
+    for (int u = 0; u < CT_U; ++u) cur[u] = next[u];
+#pragma unroll
+    for (int u = 0; u < CT_U; ++u) next[u] = load(t + CT_U + u);
+#pragma unroll
+    for (int u = 0; u < CT_U; ++u) {
+      const Quad x3 = quad_unpack(cur[u]);
+      Quad o = quad_fma(wv[3], x3, quad_fma(wv[2], x2, quad_fma(wv[1], x1, quad_fma(wv[0], x0, bv))));
+      x0 = x1; x1 = x2; x2 = x3;
+      if (act) o = Quad{make_float2(silu_f(o.a.x), silu_f(o.a.y)), make_float2(silu_f(o.b.x), silu_f(o.b.y))};
+      if (t + u < t1) *reinterpret_cast<uint2*>(yp + static_cast<long>(t + u) * C) = quad_pack(o);
+    }
+  }
+}
+
+// Backward: dpre[t] = dy[t] (times SiLU'(pre[t]), pre recomputed from x), dx[s] = sum_j w[j] dpre[s + 3 - j],
+// dw[j] = sum_t dpre[t] x[t - 3 + j], db = sum_t dpre[t].  The walk of the forward with dx three rows
+// behind: a segment also computes dpre on the three rows after its end, which the next one counts.
+// Weight and bias gradients stay in registers, the warps of a CTA meet through shared memory in a
+// fixed order, and one partial sum leaves per (CTA in time, batch): partial layout [chunk][5][C]
+// (row 4 = bias gradient), chunk = blockIdx.z * gridDim.y + blockIdx.y.
+__global__ void __launch_bounds__(CT_WARPS * 32, 2) conv1d_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
+                                                                      const bf16* __restrict__ bias, const bf16* __restrict__ dy,
+                                                                      bf16* __restrict__ dx, float* __restrict__ partial,
+                                                                      int T, int C, long ldx, int act, int rows) {
+  __shared__ __align__(16) float sred[CT_WARPS][5][CT_C];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * CT_C + lane * 4;
+  const bool c_ok = c < C;
+  const int t0 = (blockIdx.y * CT_WARPS + warp) * rows;
+  const int t1 = min(t0 + rows, T);
+  Quad dw[4], db = quad_zero();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) dw[j] = quad_zero();
+  if (c_ok && t0 < T) {
+    const bf16* xp = x + static_cast<long>(blockIdx.z) * T * ldx + c;
+    const bf16* gp = dy + static_cast<long>(blockIdx.z) * T * C + c;
+    bf16* dp = dx + static_cast<long>(blockIdx.z) * T * C + c;
+    const int te = min(t1 + 3, T);               // dpre is needed on [t0, te); rows past T count as zero
+    auto load_x = [&](int t) {
+      return t >= 0 && t < te ? *reinterpret_cast<const uint2*>(xp + t * ldx) : make_uint2(0u, 0u);
+    };
+    auto load_g = [&](int t) {
+      return t < te ? *reinterpret_cast<const uint2*>(gp + static_cast<long>(t) * C) : make_uint2(0u, 0u);
+    };
+    uint2 nx[CT_U], ng[CT_U];
+#pragma unroll
+    for (int u = 0; u < CT_U; ++u) { nx[u] = load_x(t0 + u); ng[u] = load_g(t0 + u); }
+    Quad x0 = quad_unpack(load_x(t0 - 3)), x1 = quad_unpack(load_x(t0 - 2)), x2 = quad_unpack(load_x(t0 - 1));
+    Quad wv[4], bv;
+    conv_taps(w, bias, c, true, wv, bv);
+    Quad d0 = quad_zero(), d1 = quad_zero(), d2 = quad_zero();
+    for (int t = t0; t < t1 + 3; t += CT_U) {
+      uint2 cx[CT_U], cg[CT_U];
+#pragma unroll
+      for (int u = 0; u < CT_U; ++u) { cx[u] = nx[u]; cg[u] = ng[u]; }
+#pragma unroll
+      for (int u = 0; u < CT_U; ++u) { nx[u] = load_x(t + CT_U + u); ng[u] = load_g(t + CT_U + u); }
+#pragma unroll
+      for (int u = 0; u < CT_U; ++u) {
+        const Quad x3 = quad_unpack(cx[u]);
+        Quad d3 = quad_unpack(cg[u]);            // zero past T, and so is dpre
         if (act) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) o[k] = silu_f(o[k]);
+          const Quad p = quad_fma(wv[3], x3, quad_fma(wv[2], x2, quad_fma(wv[1], x1, quad_fma(wv[0], x0, bv))));
+          d3.a.x *= dsilu_f(p.a.x); d3.a.y *= dsilu_f(p.a.y);
+          d3.b.x *= dsilu_f(p.b.x); d3.b.y *= dsilu_f(p.b.y);
         }
-        store8(y + (b * T + t) * C + c, o);
-      }
-    }
-    __syncthreads();                                // the buffer is refilled two tiles on
-  }
-}
-
-// Backward: dpre[t] = dy[t] (times SiLU'(pre[t]), pre recomputed from x), dx[s] = sum_j w[j] dpre[s + (W-1) - j],
-// dw[j] = sum_t dpre[t] x[t - (W-1) + j], db = sum_t dpre[t].  A tile needs dpre on CT_T + W - 1
-// rows, hence x on CT_T + 2 (W - 1) rows.  Weight and bias gradients stay in registers over the
-// CTA's tiles and leave as one partial sum per (time segment, batch): partial layout
-// [chunk][W + 1][C] (row W = bias gradient), chunk = blockIdx.z * gridDim.y + blockIdx.y; each time
-// step is counted by one tile only, and every sum runs in a fixed order.
-template <int W>
-__global__ void __launch_bounds__(CT_THREADS) conv1d_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                                                const bf16* __restrict__ bias, const bf16* __restrict__ dy,
-                                                                bf16* __restrict__ dx, float* __restrict__ partial,
-                                                                int T, int C, long ldx, int act) {
-  constexpr int XR = CT_T + 2 * (W - 1), DR = CT_T + W - 1;
-  extern __shared__ __align__(16) uint8_t conv_smem[];
-  bf16* sx0 = reinterpret_cast<bf16*>(conv_smem);                // [2][XR][CT_C]  x rows t0-(W-1) ..
-  bf16* sdy0 = sx0 + 2 * XR * CT_C;                              // [2][DR][CT_C]  dy rows t0 ..
-  float* sdp = reinterpret_cast<float*>(sdy0 + 2 * DR * CT_C);   // [DR][CT_C]     dpre rows t0 ..
-  float* sred = reinterpret_cast<float*>(conv_smem);             // [warps][W + 1][CT_C], over the x tiles once they are dead
-  const int c8 = threadIdx.x % (CT_C / 8), rg = threadIdx.x / (CT_C / 8);
-  const int c = blockIdx.x * CT_C + c8 * 8;
-  const long b = blockIdx.z;
-  const bool c_ok = c < C;
-  const int seg0 = blockIdx.y * CT_SEG;
-  const int n_tiles = min(CT_SEG, (T + CT_T - 1) / CT_T - seg0);
-  auto load_tile = [&](int n, int buf) {
-    const int t0 = (seg0 + n) * CT_T;
-    bf16* sx = sx0 + buf * XR * CT_C;
-    bf16* sdy = sdy0 + buf * DR * CT_C;
-    for (int i = rg; i < XR; i += CT_RG) {
-      const int t = t0 - (W - 1) + i;
-      const bool ok = c_ok && t >= 0 && t < T;
-      cp_async16(sx + i * CT_C + c8 * 8, ok ? x + (b * T + t) * ldx + c : x, ok);
-    }
-    for (int i = rg; i < DR; i += CT_RG) {
-      const int t = t0 + i;
-      const bool ok = c_ok && t < T;
-      cp_async16(sdy + i * CT_C + c8 * 8, ok ? dy + (b * T + t) * C + c : dy, ok);
-    }
-    cp_async_commit();
-  };
-  load_tile(0, 0);
-  float wv[W][8], bv[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    bv[k] = (bias && c_ok) ? __bfloat162float(bias[c + k]) : 0.f;
-#pragma unroll
-    for (int j = 0; j < W; ++j) wv[j][k] = c_ok ? __bfloat162float(w[(c + k) * W + j]) : 0.f;
-  }
-  float dwacc[W][8], dbacc[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    dbacc[k] = 0.f;
-#pragma unroll
-    for (int j = 0; j < W; ++j) dwacc[j][k] = 0.f;
-  }
-  for (int n = 0; n < n_tiles; ++n) {
-    const int buf = n & 1;
-    const bf16* sx = sx0 + buf * XR * CT_C;
-    const bf16* sdy = sdy0 + buf * DR * CT_C;
-    if (n + 1 < n_tiles) { load_tile(n + 1, buf ^ 1); cp_async_wait<1>(); }
-    else cp_async_wait<0>();
-    __syncthreads();
-    const int t0 = (seg0 + n) * CT_T;
-    // ---- dpre (rows past T hold dy = 0, so their dpre is 0)
-    for (int i = rg; i < DR; i += CT_RG) {
-      float dv[8], dp[8];
-      unpack8(*reinterpret_cast<const uint4*>(sdy + i * CT_C + c8 * 8), dv);
-      if (act) {
-        float pre[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) pre[k] = bv[k];
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-          float xv[8];
-          unpack8(*reinterpret_cast<const uint4*>(sx + (i + j) * CT_C + c8 * 8), xv);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) pre[k] += wv[j][k] * xv[k];
+        if (t + u < t1) {
+          dw[0] = quad_fma(d3, x0, dw[0]);
+          dw[1] = quad_fma(d3, x1, dw[1]);
+          dw[2] = quad_fma(d3, x2, dw[2]);
+          dw[3] = quad_fma(d3, x3, dw[3]);
+          db.a.x += d3.a.x; db.a.y += d3.a.y; db.b.x += d3.b.x; db.b.y += d3.b.y;
         }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) dp[k] = dv[k] * dsilu_f(pre[k]);
-      } else {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) dp[k] = dv[k];
-      }
-      float4* d4 = reinterpret_cast<float4*>(sdp + i * CT_C + c8 * 8);
-      d4[0] = make_float4(dp[0], dp[1], dp[2], dp[3]);
-      d4[1] = make_float4(dp[4], dp[5], dp[6], dp[7]);
-    }
-    __syncthreads();
-    // ---- dx, and this thread's share of dw / db (its rows only)
-    for (int i = rg; i < CT_T; i += CT_RG) {
-      const int t = t0 + i;
-      if (t >= T) break;
-      float o[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) o[k] = 0.f;
-#pragma unroll
-      for (int j = 0; j < W; ++j) {
-        const float4* d4 = reinterpret_cast<const float4*>(sdp + (i + (W - 1) - j) * CT_C + c8 * 8);
-        const float4 a = d4[0], e = d4[1];
-        const float dq[8] = {a.x, a.y, a.z, a.w, e.x, e.y, e.z, e.w};
-#pragma unroll
-        for (int k = 0; k < 8; ++k) o[k] += wv[j][k] * dq[k];
-      }
-      if (c_ok) store8(dx + (b * T + t) * C + c, o);
-      const float4* p4 = reinterpret_cast<const float4*>(sdp + i * CT_C + c8 * 8);
-      const float4 a = p4[0], e = p4[1];
-      const float dp[8] = {a.x, a.y, a.z, a.w, e.x, e.y, e.z, e.w};
-#pragma unroll
-      for (int k = 0; k < 8; ++k) dbacc[k] += dp[k];
-#pragma unroll
-      for (int j = 0; j < W; ++j) {
-        float xv[8];
-        unpack8(*reinterpret_cast<const uint4*>(sx + (i + j) * CT_C + c8 * 8), xv);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) dwacc[j][k] += dp[k] * xv[k];
-      }
-    }
-    __syncthreads();                                // sdp and this buffer are rewritten next
-  }
-  // ---- the two row groups of a warp meet by shuffle, the warps through shared memory, in a fixed order
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    dbacc[k] += __shfl_xor_sync(0xffffffffu, dbacc[k], 16);
-#pragma unroll
-    for (int j = 0; j < W; ++j) dwacc[j][k] += __shfl_xor_sync(0xffffffffu, dwacc[j][k], 16);
-  }
-  const int warp = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) < 16) {
-#pragma unroll
-    for (int j = 0; j <= W; ++j) {
-      float4* d4 = reinterpret_cast<float4*>(sred + (warp * (W + 1) + j) * CT_C + c8 * 8);
-      if (j < W) {
-        d4[0] = make_float4(dwacc[j][0], dwacc[j][1], dwacc[j][2], dwacc[j][3]);
-        d4[1] = make_float4(dwacc[j][4], dwacc[j][5], dwacc[j][6], dwacc[j][7]);
-      } else {
-        d4[0] = make_float4(dbacc[0], dbacc[1], dbacc[2], dbacc[3]);
-        d4[1] = make_float4(dbacc[4], dbacc[5], dbacc[6], dbacc[7]);
+        const int s = t + u - 3;
+        if (s >= t0 && s < t1)
+          *reinterpret_cast<uint2*>(dp + static_cast<long>(s) * C) =
+              quad_pack(quad_fma(wv[3], d0, quad_fma(wv[2], d1, quad_fma(wv[1], d2, quad_fma(wv[0], d3, quad_zero())))));
+        x0 = x1; x1 = x2; x2 = x3;
+        d0 = d1; d1 = d2; d2 = d3;
       }
     }
   }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&sred[warp][j][lane * 4]) = make_float4(dw[j].a.x, dw[j].a.y, dw[j].b.x, dw[j].b.y);
+  *reinterpret_cast<float4*>(&sred[warp][4][lane * 4]) = make_float4(db.a.x, db.a.y, db.b.x, db.b.y);
   __syncthreads();
-  const long chunk = static_cast<long>(blockIdx.z) * gridDim.y + blockIdx.y;
-  float* pp = partial + chunk * (W + 1) * C;
-  for (int e = threadIdx.x; e < (W + 1) * CT_C; e += CT_THREADS) {
+  float* pp = partial + (static_cast<long>(blockIdx.z) * gridDim.y + blockIdx.y) * 5 * C;
+  for (int e = threadIdx.x; e < 5 * CT_C; e += CT_WARPS * 32) {
     const int j = e / CT_C, cc = e - j * CT_C;
     const int cg = blockIdx.x * CT_C + cc;
     if (cg >= C) continue;
     float acc = 0.f;
 #pragma unroll
-    for (int wi = 0; wi < CT_THREADS / 32; ++wi) acc += sred[(wi * (W + 1) + j) * CT_C + cc];
+    for (int wi = 0; wi < CT_WARPS; ++wi) acc += sred[wi][j][cc];
     pp[static_cast<long>(j) * C + cg] = acc;
   }
+}
+
+// partial [parts][5][C] -> dw (C, 4) and db (C), fp32 or bf16, in a fixed order.  CTA: 32 channels, 8 groups of parts.
+template <typename OT>
+__global__ void __launch_bounds__(256) conv1d_dw_kernel(const float* __restrict__ partial, int parts, int C,
+                                                        OT* __restrict__ dw, OT* __restrict__ db) {
+  __shared__ float s[8][5][32];
+  const int cl = threadIdx.x & 31, g = threadIdx.x >> 5, c = blockIdx.x * 32 + cl;
+  float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  if (c < C)
+    for (int p = g; p < parts; p += 8)
+#pragma unroll
+      for (int j = 0; j < 5; ++j) acc[j] += partial[(static_cast<long>(p) * 5 + j) * C + c];
+#pragma unroll
+  for (int j = 0; j < 5; ++j) s[g][j][cl] = acc[j];
+  __syncthreads();
+  if (g >= 5 || c >= C) return;
+  float v = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v += s[k][g][cl];
+  if (g < 4) dw[static_cast<long>(c) * 4 + g] = static_cast<OT>(v);
+  else if (db) db[c] = static_cast<OT>(v);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1558,32 +1519,39 @@ extern "C" int nsa_rope(const void* x, const float* cos_t, const float* sin_t, v
   return 0;
 }
 
+// Time steps per warp: 64 keeps the rows read twice (3 of x ahead of a segment, 3 of dpre behind it) under
+// a tenth; short sequences take 32, 16 or 8 so that four CTAs per SM still find work.
+static int conv_rows(int B, int T, int C) {
+  int rows = 64;
+  auto ctas = [&](int r) { return static_cast<long>(B) * ((C + CT_C - 1) / CT_C) * ((T + CT_WARPS * r - 1) / (CT_WARPS * r)); };
+  while (rows > 8 && ctas(rows) < 4L * nsa::sm_count()) rows >>= 1;
+  return rows;
+}
 extern "C" int nsa_conv1d_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, long ldx,
                               int width, int act, cudaStream_t st) {
   if (C % 8 || ldx % 8 || width != 4) return nsa::fail(NSA_ERR_SHAPE, "conv1d: channels multiple of 8 and width 4 required");
-  dim3 grid((C + CT_C - 1) / CT_C, (T + CONV_TCHUNK - 1) / CONV_TCHUNK, B);
-  conv1d_fwd_kernel<4><<<grid, CT_THREADS, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)y, T, C, ldx, act);
+  const int rows = conv_rows(B, T, C);
+  dim3 grid((C + CT_C - 1) / CT_C, (T + CT_WARPS * rows - 1) / (CT_WARPS * rows), B);
+  conv1d_fwd_kernel<<<grid, CT_WARPS * 32, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)y, T, C, ldx, act, rows);
   nsa::count_launch();
   return 0;
 }
-extern "C" long nsa_conv1d_bwd_parts(int B, int T) { return static_cast<long>(B) * ((T + CONV_TCHUNK - 1) / CONV_TCHUNK); }
-// partial: scratch of parts * 5 * C floats.  dw_f32: [4*C] laid out [j][c]; db_f32: [C].
+extern "C" long nsa_conv1d_bwd_parts(int B, int T, int C) {
+  const int span = CT_WARPS * conv_rows(B, T, C);
+  return static_cast<long>(B) * ((T + span - 1) / span);
+}
+// partial: scratch of nsa_conv1d_bwd_parts(B, T, C) * 5 * C floats.  dw: [C][4]; db: [C] or null; both fp32
+// (dw_fp32 = 1) or bf16.
 extern "C" int nsa_conv1d_bwd(const void* x, const void* w, const void* bias, const void* dy, void* dx, float* partial,
-                              float* dwdb_f32, int B, int T, int C, long ldx, int width, int act, cudaStream_t st) {
+                              void* dw, void* db, int dw_fp32, int B, int T, int C, long ldx, int width, int act, cudaStream_t st) {
   if (C % 8 || ldx % 8 || width != 4) return nsa::fail(NSA_ERR_SHAPE, "conv1d: channels multiple of 8 and width 4 required");
-  dim3 grid((C + CT_C - 1) / CT_C, (T + CONV_TCHUNK - 1) / CONV_TCHUNK, B);
-  constexpr int smem = 2 * (CT_T + 6) * CT_C * 2 + 2 * (CT_T + 3) * CT_C * 2 + (CT_T + 3) * CT_C * 4;
-  static_assert((CT_THREADS / 32) * 5 * CT_C * 4 <= 2 * (CT_T + 6) * CT_C * 2, "conv1d: reduction scratch");
-  static bool cfg = false;
-  if (!cfg) {
-    cudaError_t e = cudaFuncSetAttribute(conv1d_bwd_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return nsa::fail_cuda(e, "conv1d_bwd: shared memory attribute");
-    cfg = true;
-  }
-  conv1d_bwd_kernel<4><<<grid, CT_THREADS, smem, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (const bf16*)dy, (bf16*)dx,
-                                                       partial, T, C, ldx, act);
-  const int parts = static_cast<int>(nsa_conv1d_bwd_parts(B, T));
-  reduce_partials_kernel<<<(5 * C + 255) / 256, 256, 0, st>>>(partial, parts, 5 * C, nullptr, dwdb_f32);
+  const int rows = conv_rows(B, T, C);
+  dim3 grid((C + CT_C - 1) / CT_C, (T + CT_WARPS * rows - 1) / (CT_WARPS * rows), B);
+  conv1d_bwd_kernel<<<grid, CT_WARPS * 32, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (const bf16*)dy, (bf16*)dx,
+                                                    partial, T, C, ldx, act, rows);
+  const int parts = static_cast<int>(nsa_conv1d_bwd_parts(B, T, C));
+  if (dw_fp32) conv1d_dw_kernel<float><<<(C + 31) / 32, 256, 0, st>>>(partial, parts, C, (float*)dw, (float*)db);
+  else conv1d_dw_kernel<bf16><<<(C + 31) / 32, 256, 0, st>>>(partial, parts, C, (bf16*)dw, (bf16*)db);
   nsa::count_launch(2);
   return 0;
 }

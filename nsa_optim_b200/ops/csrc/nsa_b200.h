@@ -54,9 +54,10 @@ int nsa_rope(const void* x, const float* cos_t, const float* sin_t, void* y, lon
              int backward, cudaStream_t st);
 int nsa_conv1d_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, long ldx, int width,
                    int act, cudaStream_t st);
-long nsa_conv1d_bwd_parts(int B, int T);
-int nsa_conv1d_bwd(const void* x, const void* w, const void* bias, const void* dy, void* dx, float* partial,
-                   float* dwdb_f32, int B, int T, int C, long ldx, int width, int act, cudaStream_t st);
+long nsa_conv1d_bwd_parts(int B, int T, int C);
+/* partial: scratch of nsa_conv1d_bwd_parts(B, T, C) * 5 * C floats; dw [C][4], db [C] or null, fp32 or bf16. */
+int nsa_conv1d_bwd(const void* x, const void* w, const void* bias, const void* dy, void* dx, float* partial, void* dw,
+                   void* db, int dw_fp32, int B, int T, int C, long ldx, int width, int act, cudaStream_t st);
 int nsa_embedding_fwd(const long* ids, const void* w, void* y, long n, int d, long vocab, cudaStream_t st);
 int nsa_embedding_bwd(const long* sorted_ids, const long* perm, const void* dy, float* dw, long n, int d, cudaStream_t st);
 

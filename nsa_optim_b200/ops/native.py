@@ -724,13 +724,16 @@ class _Conv1d(torch.autograd.Function):
         W = wb.shape[-1]
         dyc = dy.contiguous()
         dx = _empty(B, T, C, dtype=dy.dtype, device=dy.device)
-        parts = int(load().nsa_conv1d_bwd_parts(c_int(B), c_int(T)))
+        parts = int(load().nsa_conv1d_bwd_parts(c_int(B), c_int(T), c_int(C)))
         partial = _empty(parts * (W + 1) * C, dtype=torch.float32, device=dy.device)
-        dwdb = _empty((W + 1) * C, dtype=torch.float32, device=dy.device)
-        _check(load().nsa_conv1d_bwd(_p(xv), _p(wb), _p(bb), _p(dyc), _p(dx), _p(partial), _p(dwdb), c_int(B), c_int(T),
-                                     c_int(C), c_long(xv.stride(1)), c_int(W), c_int(int(ctx.activation)), _stream()))
-        dw = dwdb[: W * C].view(W, C).t().contiguous().to(ctx.wdtype)
-        db = dwdb[W * C:].to(ctx.wdtype) if ctx.has_bias else None
+        out = ctx.wdtype if ctx.wdtype == torch.bfloat16 else torch.float32
+        dw = _empty(C, W, dtype=out, device=dy.device)
+        db = _empty(C, dtype=out, device=dy.device) if ctx.has_bias else None
+        _check(load().nsa_conv1d_bwd(_p(xv), _p(wb), _p(bb), _p(dyc), _p(dx), _p(partial), _p(dw), _p(db),
+                                     c_int(int(out == torch.float32)), c_int(B), c_int(T), c_int(C), c_long(xv.stride(1)),
+                                     c_int(W), c_int(int(ctx.activation)), _stream()))
+        dw = dw.to(ctx.wdtype)
+        db = db.to(ctx.wdtype) if ctx.has_bias else None
         return dx, dw, db, None
 
 
