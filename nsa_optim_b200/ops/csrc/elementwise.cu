@@ -292,52 +292,6 @@ __global__ void reduce_partials_kernel(const float* __restrict__ partial, int pa
   if (out_f32) out_f32[c] = s;
 }
 
-// out[o][i] = sum_p in[o][p][i] over bf16 partial results, summed in fp32 in ascending p (the same
-// bits on every run), 8 elements per thread.
-__global__ void __launch_bounds__(256) sum_parts_bf16_kernel(const bf16* __restrict__ in, bf16* __restrict__ out,
-                                                             int parts, long n8, long outer) {
-  for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8 * outer;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long o = i / n8, e = i - o * n8;
-    const uint4* src = reinterpret_cast<const uint4*>(in) + (o * parts) * n8 + e;
-    float acc[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc[k] = 0.f;
-    for (int p = 0; p < parts; ++p) {
-      float v[8];
-      unpack8(src[static_cast<long>(p) * n8], v);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] += v[k];
-    }
-    store8(out + i * 8, acc);
-  }
-}
-
-// Rows of D bf16 between head-major (B, H, Ts, D) and token-major (B, Tt, H, D) storage, one warp per
-// row: to_token = 1 reads (b, h, t) and writes (b, t, h); to_token = 0 the reverse.  Only t < min(Ts, Tt)
-// is copied; when the destination is head-major and longer, its rows t >= Tt are zeroed.
-__global__ void __launch_bounds__(256) permute_rows_kernel(const bf16* __restrict__ src, bf16* __restrict__ dst, int B, int H,
-                                                           int Th, int Tt, int D, int to_token) {
-  const int d8 = D / 8;
-  const int Tloop = to_token ? Tt : Th;            // rows of the destination per (b, h)
-  const long rows = static_cast<long>(B) * H * Tloop;
-  const int lane = threadIdx.x & 31;
-  for (long row = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5); row < rows; row += static_cast<long>(gridDim.x) * 8) {
-    long b, h, t;
-    if (to_token) { b = row / (static_cast<long>(Tt) * H); const long r2 = row - b * Tt * H; t = r2 / H; h = r2 - t * H; }
-    else { b = row / (static_cast<long>(H) * Th); const long r2 = row - b * H * Th; h = r2 / Th; t = r2 - h * Th; }
-    const bf16* hp = (to_token ? src : dst) + ((b * H + h) * Th + t) * D;     // head-major address
-    const bf16* tp = (to_token ? dst : src) + ((b * Tt + t) * H + h) * D;     // token-major address
-    if (to_token) {
-      if (t < Th)
-        for (int j = lane; j < d8; j += 32) reinterpret_cast<uint4*>(const_cast<bf16*>(tp))[j] = reinterpret_cast<const uint4*>(hp)[j];
-    } else {
-      for (int j = lane; j < d8; j += 32)
-        reinterpret_cast<uint4*>(const_cast<bf16*>(hp))[j] = t < Tt ? reinterpret_cast<const uint4*>(tp)[j] : make_uint4(0, 0, 0, 0);
-    }
-  }
-}
-
 // ------------------------------------------------------------------------------------
 // L2 norm over the last dimension (d <= 512, warp per row)
 // ------------------------------------------------------------------------------------
@@ -569,293 +523,6 @@ __global__ void __launch_bounds__(256) nsa_pool_bwd_kernel(const bf16* __restric
     for (int j = 0; j < 8; ++j) acc[j] *= inv;
     store8(dx + i * 8, acc);
   }
-}
-
-// ------------------------------------------------------------------------------------
-// Gated DeltaNet layout pass.  q, k (B, T, H, 128) and v (B, T, H, V) arrive token-major; the
-// chunk kernels want head-major rows (B*H, Tp, .) with Tp the padded length.  One warp per row
-// writes the copies qh, kh, vh and the decay-scaled operands qd = q * sq, kt = k * sk in one pass
-// (rows >= T are zero).  The backward folds the five incoming gradients back to token-major and
-// reduces d sq = sum(dqd * q), d sk = sum(dkt * k).
-// ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) gdn_pack_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
-                                                           const bf16* __restrict__ v, const float* __restrict__ sq,
-                                                           const float* __restrict__ sk, bf16* __restrict__ qh,
-                                                           bf16* __restrict__ kh, bf16* __restrict__ vh,
-                                                           bf16* __restrict__ qd, bf16* __restrict__ kt, int B, int T,
-                                                           int Tp, int H, int V) {
-  constexpr int K = 128;
-  const int lane = threadIdx.x & 31;
-  const long row = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);     // (b*H + h) * Tp + t
-  if (row >= static_cast<long>(B) * H * Tp) return;
-  const int t = static_cast<int>(row % Tp);
-  const long bh = row / Tp;
-  const int h = static_cast<int>(bh % H);
-  const long b = bh / H;
-  const bool live = t < T;
-  const long tok = (b * T + (live ? t : 0)) * H + h;
-  float x[8], y[8];
-  const int part = lane >> 4, c = (lane & 15) * 8;                             // lanes 0-15: q, 16-31: k
-  const bf16* src = (part ? k : q) + tok * K + c;
-  const float s = live ? (part ? sk : sq)[row] : 0.f;
-  if (live) load8(src, x);
-  else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = 0.f;
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) y[j] = x[j] * s;
-  store8((part ? kh : qh) + row * K + c, x);
-  store8((part ? kt : qd) + row * K + c, y);
-  for (int cv = lane * 8; cv < V; cv += 256) {
-    if (live) load8(v + tok * V + cv, x);
-    store8(vh + row * V + cv, x);            // x is zero on padded rows
-  }
-}
-__global__ void __launch_bounds__(256) gdn_pack_bwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
-                                                           const float* __restrict__ sq, const float* __restrict__ sk,
-                                                           const bf16* __restrict__ dqh, const bf16* __restrict__ dkh,
-                                                           const bf16* __restrict__ dvh, const bf16* __restrict__ dqd,
-                                                           const bf16* __restrict__ dkt, bf16* __restrict__ dq,
-                                                           bf16* __restrict__ dk, bf16* __restrict__ dv,
-                                                           float* __restrict__ dsq, float* __restrict__ dsk, int B, int T,
-                                                           int Tp, int H, int V) {
-  constexpr int K = 128;
-  const int lane = threadIdx.x & 31;
-  const long row = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  if (row >= static_cast<long>(B) * H * Tp) return;
-  const int t = static_cast<int>(row % Tp);
-  const long bh = row / Tp;
-  const int h = static_cast<int>(bh % H);
-  const long b = bh / H;
-  const int part = lane >> 4, c = (lane & 15) * 8;
-  if (t >= T) {                                                                // padded row: no token, zero scale gradients
-    if ((lane & 15) == 0) (part ? dsk : dsq)[row] = 0.f;
-    return;
-  }
-  const long tok = (b * T + t) * H + h;
-  float x[8], g1[8], g2[8], o[8];
-  load8((part ? k : q) + tok * K + c, x);
-  const bf16* a = part ? dkh : dqh;
-  const bf16* d = part ? dkt : dqd;
-  if (a) load8(a + row * K + c, g1);
-  else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) g1[j] = 0.f;
-  }
-  if (d) load8(d + row * K + c, g2);
-  else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) g2[j] = 0.f;
-  }
-  const float s = (part ? sk : sq)[row];
-  float dot = 0.f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    o[j] = g1[j] + g2[j] * s;
-    dot += g2[j] * x[j];
-  }
-  store8((part ? dk : dq) + tok * K + c, o);
-#pragma unroll
-  for (int m = 8; m > 0; m >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, m);   // within each half-warp
-  if ((lane & 15) == 0) (part ? dsk : dsq)[row] = dot;
-  for (int cv = lane * 8; cv < V; cv += 256) {
-    if (dvh) load8(dvh + row * V + cv, o);
-    else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = 0.f;
-    }
-    store8(dv + tok * V + cv, o);
-  }
-}
-
-// ------------------------------------------------------------------------------------
-// Gated DeltaNet per-chunk matrices (chunk 64), one CTA of 64 threads per chunk.
-//   A[i][j] = beta_i * kk[i][j] * exp(gc_i - gc_j)   (i > j)       kk = K K^T of the chunk
-//   X = (I + A)^-1    by forward substitution, thread c owning column c in registers
-//   Tu = X diag(beta),  Tw = X diag(beta * exp(gc)),  qk[i][j] = scale * qkr[i][j] * exp(gc_i - gc_j)  (i >= j)
-// The backward takes dA = -(X^T dX X^T) (two batched matmuls done by the caller) and folds it,
-// together with dTu, dTw, dqk, into dkk, dqkr, d gc and d beta.
-// ------------------------------------------------------------------------------------
-constexpr int GC = 64;
-
-__device__ __forceinline__ void load_row64(const bf16* p, float (&v)[GC]) {
-#pragma unroll
-  for (int j = 0; j < GC / 8; ++j) {
-    float t[8];
-    load8(p + 8 * j, t);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[8 * j + e] = t[e];
-  }
-}
-__device__ __forceinline__ void store_row64(bf16* p, const float (&v)[GC]) {
-#pragma unroll
-  for (int j = 0; j < GC / 8; ++j) {
-    float t[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) t[e] = v[8 * j + e];
-    store8(p + 8 * j, t);
-  }
-}
-
-__global__ void __launch_bounds__(64) gdn_tmat_fwd_kernel(const bf16* __restrict__ kk, const bf16* __restrict__ qkr,
-                                                          const float* __restrict__ gc, const float* __restrict__ beta,
-                                                          bf16* __restrict__ Tu, bf16* __restrict__ Tw, bf16* __restrict__ qk,
-                                                          float* __restrict__ X, float scale) {
-  __shared__ float As[GC][GC + 1];
-  __shared__ float g_s[GC], b_s[GC];
-  const long ch = blockIdx.x;
-  const int i = threadIdx.x;
-  const long mat = ch * GC * GC;
-  g_s[i] = gc[ch * GC + i];
-  b_s[i] = beta[ch * GC + i];
-  __syncthreads();
-  const float gi = g_s[i], bi = b_s[i];
-  float row[GC];
-  load_row64(kk + mat + i * GC, row);
-#pragma unroll
-  for (int j = 0; j < GC; ++j) As[i][j] = (j < i) ? bi * row[j] * __expf(gi - g_s[j]) : 0.f;
-  // qk row while the A tile settles
-  load_row64(qkr + mat + i * GC, row);
-#pragma unroll
-  for (int j = 0; j < GC; ++j) row[j] = (j <= i) ? scale * row[j] * __expf(gi - g_s[j]) : 0.f;
-  store_row64(qk + mat + i * GC, row);
-  __syncthreads();
-  // column c = threadIdx.x of X: x[r] = [r == c] - sum_{j < r} A[r][j] x[j]
-  const int c = i;
-  float x[GC];
-#pragma unroll
-  for (int r = 0; r < GC; ++r) {
-    float acc = (r == c) ? 1.f : 0.f;
-#pragma unroll
-    for (int j = 0; j < r; ++j) acc = fmaf(-As[r][j], x[j], acc);
-    x[r] = acc;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < GC; ++r) As[r][c] = x[r];          // reuse the tile for X
-  __syncthreads();
-  float tu[GC], tw[GC];
-#pragma unroll
-  for (int j = 0; j < GC; ++j) {
-    const float xv = As[i][j];
-    row[j] = xv;
-    tu[j] = xv * b_s[j];
-    tw[j] = tu[j] * __expf(g_s[j]);
-  }
-  float4* xo = reinterpret_cast<float4*>(X + mat + i * GC);
-#pragma unroll
-  for (int j = 0; j < GC / 4; ++j) xo[j] = make_float4(row[4 * j], row[4 * j + 1], row[4 * j + 2], row[4 * j + 3]);
-  store_row64(Tu + mat + i * GC, tu);
-  store_row64(Tw + mat + i * GC, tw);
-}
-
-// dX[i][c] = (dTu[i][c] + dTw[i][c] * exp(gc_c)) * beta_c   for c <= i, else 0
-__global__ void __launch_bounds__(64) gdn_tmat_dx_kernel(const bf16* __restrict__ dTu, const bf16* __restrict__ dTw,
-                                                         const float* __restrict__ gc, const float* __restrict__ beta,
-                                                         float* __restrict__ dX) {
-  __shared__ float g_s[GC], b_s[GC];
-  const long ch = blockIdx.x;
-  const int i = threadIdx.x;
-  const long mat = ch * GC * GC;
-  g_s[i] = __expf(gc[ch * GC + i]);
-  b_s[i] = beta[ch * GC + i];
-  __syncthreads();
-  float a[GC], b[GC];
-  load_row64(dTu + mat + i * GC, a);
-  load_row64(dTw + mat + i * GC, b);
-  float4* o = reinterpret_cast<float4*>(dX + mat + i * GC);
-#pragma unroll
-  for (int j = 0; j < GC; ++j) a[j] = (j <= i) ? (a[j] + b[j] * g_s[j]) * b_s[j] : 0.f;
-#pragma unroll
-  for (int j = 0; j < GC / 4; ++j) o[j] = make_float4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
-}
-
-__global__ void __launch_bounds__(64) gdn_tmat_bwd_kernel(const float* __restrict__ dA, const bf16* __restrict__ kk,
-                                                          const bf16* __restrict__ qkr, const bf16* __restrict__ dqk,
-                                                          const bf16* __restrict__ dTu, const bf16* __restrict__ dTw,
-                                                          const float* __restrict__ X, const float* __restrict__ gc,
-                                                          const float* __restrict__ beta, bf16* __restrict__ dkk,
-                                                          bf16* __restrict__ dqkr, float* __restrict__ dgc,
-                                                          float* __restrict__ dbeta, float scale) {
-  __shared__ float Cg[GC][GC + 1];      // per element: contribution to d gc of its column index
-  __shared__ float Cb[GC][GC + 1];      // per element: contribution to d beta of its column index
-  __shared__ float g_s[GC], b_s[GC];
-  const long ch = blockIdx.x;
-  const int i = threadIdx.x;
-  const long mat = ch * GC * GC;
-  g_s[i] = gc[ch * GC + i];
-  b_s[i] = beta[ch * GC + i];
-  __syncthreads();
-  const float gi = g_s[i], bi = b_s[i];
-  float r1[GC], r2[GC], out[GC];
-  float dg_row = 0.f, db_row = 0.f;
-  // ---- A part: dA (fp32 row) with kk
-  load_row64(kk + mat + i * GC, r1);
-  const float4* da4 = reinterpret_cast<const float4*>(dA + mat + i * GC);
-#pragma unroll
-  for (int j = 0; j < GC / 4; ++j) {
-    const float4 v = da4[j];
-    r2[4 * j] = v.x; r2[4 * j + 1] = v.y; r2[4 * j + 2] = v.z; r2[4 * j + 3] = v.w;
-  }
-#pragma unroll
-  for (int j = 0; j < GC; ++j) {
-    float cg = 0.f;
-    out[j] = 0.f;
-    if (j < i) {
-      const float e = __expf(gi - g_s[j]);
-      const float araw = r1[j] * e;
-      const float d = r2[j];
-      out[j] = d * bi * e;
-      db_row += d * araw;
-      const float t = d * bi * araw;
-      dg_row += t;
-      cg = -t;
-    }
-    Cg[i][j] = cg;
-  }
-  store_row64(dkk + mat + i * GC, out);
-  // ---- qk part
-  load_row64(qkr + mat + i * GC, r1);
-  load_row64(dqk + mat + i * GC, r2);
-#pragma unroll
-  for (int j = 0; j < GC; ++j) {
-    out[j] = 0.f;
-    if (j <= i) {
-      const float e = __expf(gi - g_s[j]);
-      out[j] = r2[j] * scale * e;
-      const float t = out[j] * r1[j];
-      dg_row += t;
-      Cg[i][j] -= t;
-    }
-  }
-  store_row64(dqkr + mat + i * GC, out);
-  // ---- Tu / Tw part (column-indexed scalings)
-  load_row64(dTu + mat + i * GC, r1);
-  load_row64(dTw + mat + i * GC, r2);
-  const float4* x4 = reinterpret_cast<const float4*>(X + mat + i * GC);
-#pragma unroll
-  for (int j = 0; j < GC / 4; ++j) {
-    const float4 v = x4[j];
-    out[4 * j] = v.x; out[4 * j + 1] = v.y; out[4 * j + 2] = v.z; out[4 * j + 3] = v.w;
-  }
-#pragma unroll
-  for (int j = 0; j < GC; ++j) {
-    float cb = 0.f;
-    if (j <= i) {
-      const float eg = __expf(g_s[j]);
-      const float xv = out[j];
-      cb = (r1[j] + r2[j] * eg) * xv;
-      Cg[i][j] += r2[j] * xv * b_s[j] * eg;
-    }
-    Cb[i][j] = cb;
-  }
-  __syncthreads();
-  float dg_col = 0.f, db_col = 0.f;
-#pragma unroll 8
-  for (int r = 0; r < GC; ++r) { dg_col += Cg[r][i]; db_col += Cb[r][i]; }
-  dgc[ch * GC + i] = dg_row + dg_col;
-  dbeta[ch * GC + i] = db_row + db_col;
 }
 
 // ------------------------------------------------------------------------------------
@@ -1436,76 +1103,6 @@ extern "C" int nsa_pool_bwd(const void* dy, void* dx, int B, int T, int width, i
   const int nC = (T - block) / stride + 1;
   const long n = static_cast<long>(B) * T * (width / 8);
   nsa_pool_bwd_kernel<<<grid_for(n, 256), 256, 0, st>>>((const bf16*)dy, (bf16*)dx, T, nC, width / 8, block, stride, n);
-  nsa::count_launch();
-  return 0;
-}
-
-// q, k: [B, T, H, 128]; v: [B, T, H, V] (V multiple of 8); sq, sk: [B*H, Tp] fp32;
-// outputs [B*H, Tp, 128 or V] bf16.
-extern "C" int nsa_gdn_pack_fwd(const void* q, const void* k, const void* v, const float* sq, const float* sk, void* qh,
-                                void* kh, void* vh, void* qd, void* kt, int B, int T, int Tp, int H, int K, int V,
-                                cudaStream_t st) {
-  if (K != 128 || V % 8 || Tp < T) return nsa::fail(NSA_ERR_SHAPE, "gdn_pack: key width 128 and value width multiple of 8 required");
-  const long rows = static_cast<long>(B) * H * Tp;
-  gdn_pack_fwd_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const bf16*)q, (const bf16*)k, (const bf16*)v, sq, sk, (bf16*)qh,
-                                                                  (bf16*)kh, (bf16*)vh, (bf16*)qd, (bf16*)kt, B, T, Tp, H, V);
-  nsa::count_launch();
-  return 0;
-}
-// dqh, dkh, dvh, dqd, dkt may be null (treated as zero).  dq, dk, dv: token-major outputs; dsq, dsk: [B*H, Tp] fp32.
-extern "C" int nsa_gdn_pack_bwd(const void* q, const void* k, const float* sq, const float* sk, const void* dqh,
-                                const void* dkh, const void* dvh, const void* dqd, const void* dkt, void* dq, void* dk,
-                                void* dv, float* dsq, float* dsk, int B, int T, int Tp, int H, int K, int V, cudaStream_t st) {
-  if (K != 128 || V % 8 || Tp < T) return nsa::fail(NSA_ERR_SHAPE, "gdn_pack: key width 128 and value width multiple of 8 required");
-  const long rows = static_cast<long>(B) * H * Tp;
-  gdn_pack_bwd_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const bf16*)q, (const bf16*)k, sq, sk, (const bf16*)dqh,
-                                                                  (const bf16*)dkh, (const bf16*)dvh, (const bf16*)dqd, (const bf16*)dkt,
-                                                                  (bf16*)dq, (bf16*)dk, (bf16*)dv, dsq, dsk, B, T, Tp, H, V);
-  nsa::count_launch();
-  return 0;
-}
-
-// Per-chunk matrices of the gated delta rule; n_chunks = B*H*NC, every matrix 64 x 64 row-major.
-extern "C" int nsa_gdn_tmat_fwd(const void* kk, const void* qkr, const float* gc, const float* beta, void* Tu, void* Tw,
-                                void* qk, float* X, long n_chunks, float scale, cudaStream_t st) {
-  if (n_chunks <= 0 || n_chunks > 2147483647L) return nsa::fail(NSA_ERR_SHAPE, "gdn_tmat: bad chunk count");
-  gdn_tmat_fwd_kernel<<<(unsigned)n_chunks, 64, 0, st>>>((const bf16*)kk, (const bf16*)qkr, gc, beta, (bf16*)Tu, (bf16*)Tw,
-                                                        (bf16*)qk, X, scale);
-  nsa::count_launch();
-  return 0;
-}
-extern "C" int nsa_gdn_tmat_dx(const void* dTu, const void* dTw, const float* gc, const float* beta, float* dX,
-                               long n_chunks, cudaStream_t st) {
-  if (n_chunks <= 0 || n_chunks > 2147483647L) return nsa::fail(NSA_ERR_SHAPE, "gdn_tmat: bad chunk count");
-  gdn_tmat_dx_kernel<<<(unsigned)n_chunks, 64, 0, st>>>((const bf16*)dTu, (const bf16*)dTw, gc, beta, dX);
-  nsa::count_launch();
-  return 0;
-}
-extern "C" int nsa_gdn_tmat_bwd(const float* dA, const void* kk, const void* qkr, const void* dqk, const void* dTu,
-                                const void* dTw, const float* X, const float* gc, const float* beta, void* dkk, void* dqkr,
-                                float* dgc, float* dbeta, long n_chunks, float scale, cudaStream_t st) {
-  if (n_chunks <= 0 || n_chunks > 2147483647L) return nsa::fail(NSA_ERR_SHAPE, "gdn_tmat: bad chunk count");
-  gdn_tmat_bwd_kernel<<<(unsigned)n_chunks, 64, 0, st>>>(dA, (const bf16*)kk, (const bf16*)qkr, (const bf16*)dqk, (const bf16*)dTu,
-                                                        (const bf16*)dTw, X, gc, beta, (bf16*)dkk, (bf16*)dqkr, dgc, dbeta, scale);
-  nsa::count_launch();
-  return 0;
-}
-
-// Head-major (B, H, Th, D) <-> token-major (B, Tt, H, D) copy of bf16 rows (D a multiple of 8); see the kernel.
-extern "C" int nsa_permute_rows(const void* src, void* dst, int B, int H, int Th, int Tt, int D, int to_token, cudaStream_t st) {
-  if (D % 8) return nsa::fail(NSA_ERR_SHAPE, "permute_rows: width must be a multiple of 8");
-  const long rows = static_cast<long>(B) * H * (to_token ? Tt : Th);
-  if (rows <= 0) return 0;
-  permute_rows_kernel<<<grid_for(rows, 8, 16), 256, 0, st>>>((const bf16*)src, (bf16*)dst, B, H, Th, Tt, D, to_token);
-  nsa::count_launch();
-  return 0;
-}
-
-// in: [outer][parts][n] bf16 contiguous -> out: [outer][n] bf16 (n a multiple of 8).
-extern "C" int nsa_sum_parts_bf16(const void* in, void* out, long outer, int parts, long n, cudaStream_t st) {
-  if (n % 8 || parts <= 0) return nsa::fail(NSA_ERR_SHAPE, "sum_parts: width must be a multiple of 8");
-  const long total = outer * (n / 8);
-  sum_parts_bf16_kernel<<<grid_for(total, 256), 256, 0, st>>>((const bf16*)in, (bf16*)out, parts, n / 8, outer);
   nsa::count_launch();
   return 0;
 }

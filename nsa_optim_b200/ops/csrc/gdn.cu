@@ -2,22 +2,20 @@
 // forward and backward, on tcgen05 tensor cores with the K x V state resident in tensor
 // memory.  Chunk length 64, key width 128, value width a multiple of 64.
 //
-// Per head, with S the K x V state entering chunk c (fp32), and per-chunk inputs prepared by
-// the parallel pre-pass (w, q_dec, k_tail: 64 x K; u: 64 x V; gamma = exp(total log-decay)):
-//     v_new   = u - w S                 o_inter = q_dec S
-//     S_next  = gamma S + k_tail^T v_new
-// One CTA owns one (head, 64-wide V tile) and walks the chunks in order.  Each step is two
-// MMA groups: D1[128 x 64] = [w ; q_dec] * S  and  S += k_tail^T * v_new, with S kept in TMEM
-// as fp32 and mirrored to shared memory as the bf16 B operand of the next step.  Operand
-// tiles for chunk c+1 arrive by TMA while chunk c computes.
+// Per head, with S the K x V state entering chunk c (fp32), w (64 x K), u (64 x V), qk (64 x 64) and the
+// cumulative log-decay gc from gdn_chunk.cu, and q, k as the caller has them:
+//     v_new   = u - w S                 o = sq (q S) + qk v_new            sq_i = scale e^gc_i
+//     S_next  = e^gc_last S + k^T (sk v_new)                               sk_i = e^(gc_last - gc_i)
+// One CTA owns one (head, 64-wide V tile) and walks the chunks in order.  The loop is one dependent
+// chain and there are fewer CTAs than SMs at the usual head counts, so its length is what a call
+// takes: row scalings are applied to accumulator rows in registers instead of to operands, the
+// output's part of a chunk (its second product, the read-back, the store) runs behind the
+// next chunk's first product, and o leaves token-major.
 //
-// Backward walks the chunks in reverse with dS (K x 64 tile) in TMEM:
-//     dv_tot  = dv_new + k_tail dS              du      = dv_tot
-//     dk_tail = v_new dS^T   (partial over V tiles)
-//     dw      = -dv_tot S^T  (partial)          dq_dec  = do S^T  (partial)
-//     dgamma  = <S, dS>      (partial)
-//     dS_prev = gamma dS + q_dec^T do - w^T dv_tot
-// Partials are written per V tile and summed by the caller (deterministic).
+// Backward walks the chunks in reverse with dS (K x 64 tile, gradient of the state leaving the chunk) in TMEM:
+//     du      = qk^T do + sk (k dS)     dgamma = <S, dS>  (partial per V tile)
+//     dS_prev = e^gc_last dS + q^T (sq do) - w^T du
+// It stores dS per chunk; what only needs S and dS of one chunk (dw, dq, dk) is left to gdn_post_kernel.
 #include "host.cuh"
 #include "tc5.cuh"
 
@@ -56,11 +54,6 @@ __device__ __forceinline__ void load_row_global(const bf16* src, uint32_t (&pack
     packed[4 * j] = v.x; packed[4 * j + 1] = v.y; packed[4 * j + 2] = v.z; packed[4 * j + 3] = v.w;
   }
 }
-__device__ __forceinline__ void store_row_global(bf16* dst, const uint32_t (&packed)[32]) {
-  uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) d4[j] = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
-}
 __device__ __forceinline__ void unpack_row(const uint32_t (&packed)[32], float (&out)[64]) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
@@ -92,37 +85,40 @@ __device__ __forceinline__ void pack_row(const float (&in)[64], uint32_t (&packe
 
 struct FwdParams {
   const bf16* u;        // [BH, NC, 64, V]
-  const float* gamma;   // [BH, NC]
-  bf16* v_new;          // [BH, NC, 64, V]
-  bf16* o_inter;        // [BH, NC, 64, V]  (rounded once here: it is added to a bf16 product next)
-  bf16* S_all;          // [BH, NC, KD, V]  state entering each chunk
-  int NC, V;
+  const float* gc;      // [BH, NC, 64]
+  int store_states;     // also write v_new and S_all (the backward needs them)
+  int NC, V, H;
+  float scale;
   KernelStatus* status;
 };
 
-constexpr int FWD_STAGE = 2 * 2 * BOX /*[w;qd] two k-blocks*/ + 2 * BOX /*k_tail*/;   // 48 KB
-constexpr int FWD_SMEM = 2 * FWD_STAGE + 2 * BOX /*Sb*/ + BOX /*Vb*/ + BOX /*Ob*/ + 1024 + 128;
+// stage: k-block kb of [w ; q] (2 x 16 KB), k (16 KB), [0 ; qk] (16 KB, first half zero)
+constexpr int FWD_STAGE = 8 * BOX;
+constexpr int FWD_TX = 7 * BOX;                                                       // bytes that arrive per chunk
+constexpr int FWD_SMEM = 2 * FWD_STAGE + 2 * BOX /*Sb*/ + 2 * BOX /*Vb, Vs*/ + BOX /*Ob*/ + 1024 + 128;
 
 __global__ void __launch_bounds__(128, 1)
-gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_qd,
-                   const __grid_constant__ CUtensorMap tm_kt, const __grid_constant__ CUtensorMap tm_vn,
-                   const __grid_constant__ CUtensorMap tm_oi, const __grid_constant__ CUtensorMap tm_sa,
-                   const FwdParams p) {
+gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_q,
+                   const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_qk,
+                   const __grid_constant__ CUtensorMap tm_vn, const __grid_constant__ CUtensorMap tm_o,
+                   const __grid_constant__ CUtensorMap tm_sa, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* Sb = smem + 2 * FWD_STAGE;           // [KD rows][64] bf16, B operand of MMA1
-  uint8_t* Vb = Sb + 2 * BOX;                   // [64 rows][64] bf16, B operand of MMA2
-  uint8_t* Ob = Vb + BOX;                       // [64 rows][64] bf16: o_inter on its way out
+  uint8_t* Sb = smem + 2 * FWD_STAGE;           // [KD rows][64] bf16 state, B operand
+  uint8_t* Vb = Sb + 2 * BOX;                   // [64 rows][64] v_new
+  uint8_t* Vs = Vb + BOX;                       // [64 rows][64] sk v_new
+  uint8_t* Ob = Vs + BOX;                       // [64 rows][64] o on its way out
   uint64_t* bars = reinterpret_cast<uint64_t*>(Ob + BOX);
   uint64_t* full = bars;        // [2]
   uint64_t* m1 = bars + 2;
   uint64_t* m2 = bars + 3;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
+  uint64_t* m3 = bars + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int r = threadIdx.x;               // TMEM lane / tile row owned by this thread
   const int warp = r >> 5;
-  const int vt = blockIdx.x, bh = blockIdx.y;
+  const int vt = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
   const int NC = p.NC, V = p.V;
 
   if (r == 0) {
@@ -131,15 +127,17 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     tc5::mbar_init(&full[1], 1);
     tc5::mbar_init(m1, 1);
     tc5::mbar_init(m2, 1);
+    tc5::mbar_init(m3, 1);
     tc5::fence_barrier_init();
   }
-  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 128); tc5::tmem_relinquish(); }
-  // S = 0: bf16 mirror in shared memory
+  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
+  // S = 0: bf16 mirror in shared memory; the constant zero half of both [0 ; qk] operands
   {
     uint32_t z[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) z[j] = 0u;
     write_row_swz(Sb, r, z);
+    write_row_swz(smem + (r >> 6) * FWD_STAGE + 6 * BOX, r & 63, z);
   }
   tc5::fence_proxy_async();
   tc5::fence_before_sync();
@@ -147,21 +145,20 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_off = static_cast<uint32_t>(warp * 32) << 16;
-  const uint32_t tD1 = tmem + lane_off;          // columns [0, 64)
-  const uint32_t tS = tmem + lane_off + 64;      // columns [64, 128)
+  // TMEM columns: D1 = [w ; q] S [0, 64)   S [64, 128)   D2 = [0 ; qk] v_new [128, 192)
+  const uint32_t cD1 = 0, cS = 64, cD2 = 128;
   {
     float z[64];
 #pragma unroll
     for (int j = 0; j < 64; ++j) z[j] = 0.f;
-    tmem_st_row64(tS, z);
+    tmem_st_row64(tmem + lane_off + cS, z);
   }
   tc5::fence_before_sync();
   __syncthreads();
-  // Outputs leave as TMA stores from the swizzled tiles they are in anyway (a thread owns a row, so
-  // direct stores would be 32 separate 16-byte writes per instruction; they were a third of the
-  // chunk loop).  One thread issues and waits; at most one store group stays pending across a point
-  // where a tile is overwritten.  Chunk 0 enters with the zero state that Sb holds now.
-  if (r == 0) {
+  // Outputs leave as TMA stores from the swizzled tiles they are in anyway.  Thread 0 stores v_new and the
+  // state, thread 64 the output; each waits until its earlier store has read a tile before that tile is
+  // rewritten.  Chunk 0 enters with the zero state that Sb holds now.
+  if (r == 0 && p.store_states) {
     tc5::tma_store_2d(&tm_sa, Sb, vt * VT, bh * NC * KD);
     tc5::tma_store_commit();
   }
@@ -170,26 +167,50 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const int s = c & 1;
     uint8_t* st = smem + s * FWD_STAGE;
     const int row0 = (bh * NC + c) * CH;
-    tc5::mbar_expect_tx(&full[s], FWD_STAGE);
+    tc5::mbar_expect_tx(&full[s], FWD_TX);
 #pragma unroll
     for (int kb = 0; kb < 2; ++kb) {
       tc5::tma_load_2d(st + kb * 2 * BOX, &tm_w, &full[s], kb * 64, row0);
-      tc5::tma_load_2d(st + kb * 2 * BOX + BOX, &tm_qd, &full[s], kb * 64, row0);
-      tc5::tma_load_2d(st + 4 * BOX + kb * BOX, &tm_kt, &full[s], kb * 64, row0);
+      tc5::tma_load_4d(st + kb * 2 * BOX + BOX, &tm_q, &full[s], kb * 64, h, c * CH, b);
+      tc5::tma_load_4d(st + 4 * BOX + kb * BOX, &tm_k, &full[s], kb * 64, h, c * CH, b);
     }
+    tc5::tma_load_2d(st + 7 * BOX, &tm_qk, &full[s], 0, row0);
   };
   if (r == 0) issue_loads(0);
 
   constexpr uint32_t idesc1 = tc5::make_idesc_bf16(128, VT, 0, 1);   // A K-major, B MN-major
-  constexpr uint32_t idesc2 = tc5::make_idesc_bf16(128, VT, 1, 1);   // A MN-major (k_tail^T), B MN-major
+  constexpr uint32_t idesc2 = tc5::make_idesc_bf16(128, VT, 1, 1);   // A MN-major (k^T), B MN-major
   bool ok = true;
-  // The chunk loop is one dependent chain, so every global load in it would add its full latency to
-  // every chunk: the u row and the decay of the next chunk are fetched one chunk ahead instead.
+  // Global loads of the chain (u row, gates) are fetched one chunk ahead.
+  const float* gc = p.gc + static_cast<long>(bh) * NC * CH;
   uint32_t upk_next[32];
 #pragma unroll
   for (int j = 0; j < 32; ++j) upk_next[j] = 0u;
   if (r < CH) load_row_global(p.u + (static_cast<long>(bh * NC) * CH + r) * V + vt * VT, upk_next);
-  float g_next = NC > 1 ? p.gamma[bh * NC + 1] : 0.f;
+  float gr_next = gc[r & 63], gl_next = gc[CH - 1];
+  float oi[64];                                    // sq (q S) of the chunk whose output is still open (rows 64..127)
+  // Output of chunk c: D2 joins oi; runs while the tensor core works on chunk c + 1.
+  auto finish_output = [&](int c) {
+    if (!tc5::mbar_wait(m3, c & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
+    __syncwarp();
+    tc5::fence_after_sync();
+    if (r < CH) return;                            // warps 2 and 3 stay together, also after a wait that gave up
+    float d2[64];
+    tmem_ld_row64(tmem + lane_off + cD2, d2);
+#pragma unroll
+    for (int j = 0; j < 64; ++j) d2[j] += oi[j];
+    uint32_t pk[32];
+    pack_row(d2, pk);
+    if (r == CH) tc5::tma_store_wait_read<0>();    // the previous output tile has been read
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+    write_row_swz(Ob, r - CH, pk);
+    tc5::fence_proxy_async();
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+    if (r == CH && ok) {                           // rows past T are clipped by the copy engine
+      tc5::tma_store_4d(&tm_o, Ob, vt * VT, h, c * CH, b);
+      tc5::tma_store_commit();
+    }
+  };
   for (int c = 0; c < NC && ok; ++c) {
     const int s = c & 1;
     uint8_t* st = smem + s * FWD_STAGE;
@@ -197,7 +218,7 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     uint32_t upk[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) upk[j] = upk_next[j];
-    const float g = g_next;                        // decay applied to the state that enters chunk c + 1
+    const float g_row = gr_next, g_last = gl_next;
     if (warp == 0) {
       // The issuing warp stays converged and one elected lane issues: descriptors then live in
       // uniform registers and an MMA costs the issuing thread a few cycles instead of 70 to 100,
@@ -209,55 +230,69 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         if (lead) {
 #pragma unroll
           for (int kk = 0; kk < KD / 16; ++kk)
-            tc5::mma_ss(tmem, a1 + static_cast<uint64_t>(((kk >> 2) * 2 * BOX + (kk & 3) * 32) >> 4),
+            tc5::mma_ss(tmem + cD1, a1 + static_cast<uint64_t>(((kk >> 2) * 2 * BOX + (kk & 3) * 32) >> 4),
                         sb + static_cast<uint64_t>((kk * 2048) >> 4), idesc1, kk > 0 ? 1u : 0u);
           tc5::mma_commit(m1);
-          if (c + 1 < NC) issue_loads(c + 1);
         }
       }
       __syncwarp();
     }
-    // next chunk's u row (rows 0..63 only) and the decay after it, in flight while this chunk computes
-    if (c + 1 < NC && r < CH) load_row_global(p.u + (row0 + CH + r) * V + vt * VT, upk_next);
-    if (c + 2 < NC) g_next = p.gamma[bh * NC + c + 2];
-    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous chunk's v_new / o_inter tiles have been read
-    if (!tc5::mbar_wait(m1, c & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
+    // next chunk's u row (rows 0..63 only) and gates, in flight while this chunk computes
+    if (c + 1 < NC) {
+      if (r < CH) load_row_global(p.u + (row0 + CH + r) * V + vt * VT, upk_next);
+      gr_next = gc[(c + 1) * CH + (r & 63)];
+      gl_next = gc[(c + 1) * CH + CH - 1];
+    }
+    if (c > 0) finish_output(c - 1);
+    // the stage of chunk c + 1 was last read by chunk c - 1's second group of MMAs, complete since finish_output
+    if (r == 0 && ok && c + 1 < NC) issue_loads(c + 1);
+    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous v_new tile has been read
+    if (ok && !tc5::mbar_wait(m1, c & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc5::fence_after_sync();
     {
       float d1[64];
-      tmem_ld_row64(tD1, d1);
+      tmem_ld_row64(tmem + lane_off + cD1, d1);
       if (r < CH) {
         float uf[64];
         unpack_row(upk, uf);
+        const float sk = __expf(g_last - g_row);
+        uint32_t pk[32], ps[32];
 #pragma unroll
         for (int j = 0; j < 64; ++j) d1[j] = uf[j] - d1[j];
-        uint32_t pk[32];
         pack_row(d1, pk);
+#pragma unroll
+        for (int j = 0; j < 64; ++j) d1[j] *= sk;
+        pack_row(d1, ps);
         write_row_swz(Vb, r, pk);
+        write_row_swz(Vs, r, ps);
       } else {
-        uint32_t pk[32];
-        pack_row(d1, pk);
-        write_row_swz(Ob, r - CH, pk);
+        const float sq = p.scale * __expf(g_row);
+#pragma unroll
+        for (int j = 0; j < 64; ++j) oi[j] = sq * d1[j];
       }
     }
     tc5::fence_proxy_async();
     tc5::fence_before_sync();
     __syncthreads();
-    if (r == 0) {
+    if (r == 0 && p.store_states) {
       tc5::tma_store_2d(&tm_vn, Vb, vt * VT, static_cast<int>(row0));
-      tc5::tma_store_2d(&tm_oi, Ob, vt * VT, static_cast<int>(row0));
       tc5::tma_store_commit();
     }
     if (warp == 0) {
       const bool lead = tc5::elect_one();
       tc5::fence_after_sync();
-      const uint64_t kt = tc5::desc_mnmajor(tc5::smem_u32(st + 4 * BOX), BOX), vb = tc5::desc_mnmajor(tc5::smem_u32(Vb), BOX);
+      const uint64_t kt = tc5::desc_mnmajor(tc5::smem_u32(st + 4 * BOX), BOX), vs = tc5::desc_mnmajor(tc5::smem_u32(Vs), BOX);
+      const uint64_t qk = tc5::desc_kmajor(tc5::smem_u32(st + 6 * BOX)), vb = tc5::desc_mnmajor(tc5::smem_u32(Vb), BOX);
       if (lead) {
 #pragma unroll
-        for (int kk = 0; kk < CH / 16; ++kk)
-          tc5::mma_ss(tmem + 64, kt + static_cast<uint64_t>((kk * 2048) >> 4), vb + static_cast<uint64_t>((kk * 2048) >> 4), idesc2, 1u);
+        for (int kk = 0; kk < CH / 16; ++kk)       // S += k^T (sk v_new)
+          tc5::mma_ss(tmem + cS, kt + static_cast<uint64_t>((kk * 2048) >> 4), vs + static_cast<uint64_t>((kk * 2048) >> 4), idesc2, 1u);
         tc5::mma_commit(m2);
+#pragma unroll
+        for (int kk = 0; kk < CH / 16; ++kk)       // D2 = [0 ; qk] v_new
+          tc5::mma_ss(tmem + cD2, qk + static_cast<uint64_t>((kk * 32) >> 4), vb + static_cast<uint64_t>((kk * 2048) >> 4), idesc1, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(m3);
       }
       __syncwarp();
     }
@@ -267,23 +302,25 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     tc5::fence_after_sync();
     if (c + 1 < NC) {
       float sv[64];
-      tmem_ld_row64(tS, sv);                       // S entering chunk c+1, row r
+      tmem_ld_row64(tmem + lane_off + cS, sv);     // S entering chunk c+1, row r
       uint32_t pk[32];
       pack_row(sv, pk);
       write_row_swz(Sb, r, pk);
+      const float g = __expf(gl_next);             // its decay through chunk c + 1
 #pragma unroll
       for (int j = 0; j < 64; ++j) sv[j] *= g;
-      tmem_st_row64(tS, sv);
+      tmem_st_row64(tmem + lane_off + cS, sv);
       tc5::fence_proxy_async();
     }
     tc5::fence_before_sync();
     __syncthreads();
-    if (r == 0 && c + 1 < NC) {
+    if (r == 0 && c + 1 < NC && p.store_states) {
       tc5::tma_store_2d(&tm_sa, Sb, vt * VT, (bh * NC + c + 1) * KD);
       tc5::tma_store_commit();
     }
   }
-  if (r == 0) tc5::tma_store_wait_read<0>();
+  if (ok) finish_output(NC - 1);
+  if (r == 0 || r == CH) tc5::tma_store_wait_read<0>();
   if (!ok && r == 0) {
     // a load for the next chunk may still be in flight: give it a bounded chance to land
     const long long t0 = clock64();
@@ -295,44 +332,35 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
   tc5::fence_before_sync();
   __syncthreads();
-  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 128); }
+  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 256); }
 }
 
 struct BwdParams {
-  const bf16* v_new;     // [BH, NC, 64, V]
-  const bf16* dv_new;    // [BH, NC, 64, V]  gradient arriving at v_new from the intra-chunk output term
-  const bf16* d_o;       // [BH, NC, 64, V]  gradient of o_inter
-  const float* gamma;    // [BH, NC]
-  bf16* du;              // [BH, NC, 64, V]
-  bf16* dw_part;         // [VTILES, BH, NC, 64, KD]
-  bf16* dqd_part;        // [VTILES, BH, NC, 64, KD]
-  bf16* dkt_part;        // [VTILES, BH, NC, 64, KD]
+  const bf16* d_o;       // [B, T, H, V]
+  const float* gc;       // [BH, NC, 64]
   float* dgamma_part;    // [VTILES, BH, NC]
-  int NC, V, BH;
+  int NC, V, BH, H, T;
+  float scale;
   KernelStatus* status;
 };
 
-// stage: k-block kb of [k_tail ; w] (2 x 16 KB), q_dec (2 x 8 KB), S_prev [KD][64] (16 KB)
-constexpr int BWD_STAGE = 2 * 2 * BOX + 2 * BOX + 2 * BOX;                 // 64 KB
-constexpr int BWD_SMEM = 2 * BWD_STAGE + 2 * BOX /*[dv_tot;do]*/ + 2 * BOX /*[v_new;do]*/ + 2 * BOX /*dSb*/ +
-                         2 * BOX /*dk_tail out*/ + 4 * BOX /*dw, dq_dec out*/ + 1024 + 128;
+// stage: k-block kb of [k ; w] (2 x 16 KB), q (16 KB), S_prev [KD][64] (16 KB), [qk | 0] (16 KB, second half zero)
+constexpr int BWD_STAGE = 10 * BOX;                                        // 80 KB
+constexpr int BWD_TX = 9 * BOX;
+constexpr int BWD_SMEM = 2 * BWD_STAGE + BOX /*du*/ + 2 * BOX /*do, sq do*/ + 2 * BOX /*dSb*/ + 1024 + 128;
 
 __global__ void __launch_bounds__(128, 1)
-gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_qd,
-                   const __grid_constant__ CUtensorMap tm_kt, const __grid_constant__ CUtensorMap tm_S,
-                   const __grid_constant__ CUtensorMap tm_du, const __grid_constant__ CUtensorMap tm_dkt,
-                   const __grid_constant__ CUtensorMap tm_dw, const __grid_constant__ CUtensorMap tm_dqd,
-                   const BwdParams p) {
+gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_q,
+                   const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_S,
+                   const __grid_constant__ CUtensorMap tm_qk, const __grid_constant__ CUtensorMap tm_du,
+                   const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* AD = smem + 2 * BWD_STAGE;     // [dv_tot (64 rows) ; do (64 rows)] x 64 cols
-  uint8_t* AV = AD + 2 * BOX;             // [v_new ; do]
-  uint8_t* dSb = AV + 2 * BOX;            // [KD rows][64] bf16 mirror of dS
-  // Outputs leave as TMA stores from swizzled tiles (see the forward kernel): du straight from AD,
-  // the dk_tail partial from Kst, the -dw and dq_dec partials from Wst.
-  uint8_t* Kst = dSb + 2 * BOX;           // [2 k-blocks][64 rows][64]
-  uint8_t* Wst = Kst + 2 * BOX;           // [2 k-blocks][128 rows][64]: rows 0..63 -dw, rows 64..127 dq_dec
-  uint64_t* bars = reinterpret_cast<uint64_t*>(Wst + 4 * BOX);
+  uint8_t* sDU = smem + 2 * BWD_STAGE;    // [64][64] du
+  uint8_t* sDO = sDU + BOX;               // [64][64] do
+  uint8_t* sDOs = sDO + BOX;              // [64][64] sq do
+  uint8_t* dSb = sDOs + BOX;              // [KD rows][64] bf16 mirror of dS
+  uint64_t* bars = reinterpret_cast<uint64_t*>(dSb + 2 * BOX);
   uint64_t* full = bars;
   uint64_t* m1 = bars + 2;
   uint64_t* m2 = bars + 3;
@@ -342,7 +370,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 
   const int r = threadIdx.x;
   const int warp = r >> 5;
-  const int vt = blockIdx.x, bh = blockIdx.y;
+  const int vt = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
   const int NC = p.NC, V = p.V;
 
   if (r == 0) {
@@ -353,12 +381,13 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     tc5::mbar_init(m2, 1);
     tc5::fence_barrier_init();
   }
-  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 512); tc5::tmem_relinquish(); }
+  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
   {
     uint32_t z[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) z[j] = 0u;
     write_row_swz(dSb, r, z);
+    write_row_swz(smem + (r >> 6) * BWD_STAGE + 9 * BOX, r & 63, z);
   }
   tc5::fence_proxy_async();
   tc5::fence_before_sync();
@@ -366,8 +395,8 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_off = static_cast<uint32_t>(warp * 32) << 16;
-  // TMEM columns: Da [0,64)  Dc [64,192)  Db [192,320)  dS [320,384)
-  const uint32_t cDa = 0, cDc = 64, cDb = 192, cDs = 320;
+  // TMEM columns: Da = [k ; w] dS [0,64)   Dd = [qk^T ; 0] do [64,128)   dS [128,192)
+  const uint32_t cDa = 0, cDd = 64, cDs = 128;
   {
     float z[64];
 #pragma unroll
@@ -376,61 +405,71 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
   tc5::fence_before_sync();
   __syncthreads();
+  // outputs leave as TMA stores from swizzled tiles (see the forward kernel); the last chunk's state has no gradient
+  if (r == 0) {
+    tc5::tma_store_2d(&tm_ds, dSb, vt * VT, (bh * NC + NC - 1) * KD);
+    tc5::tma_store_commit();
+  }
 
   auto issue_loads = [&](int c, int it) {
     const int s = it & 1;
     uint8_t* st = smem + s * BWD_STAGE;
     const int row0 = (bh * NC + c) * CH;
-    tc5::mbar_expect_tx(&full[s], BWD_STAGE);
+    tc5::mbar_expect_tx(&full[s], BWD_TX);
 #pragma unroll
     for (int kb = 0; kb < 2; ++kb) {
-      tc5::tma_load_2d(st + kb * 2 * BOX, &tm_kt, &full[s], kb * 64, row0);
+      tc5::tma_load_4d(st + kb * 2 * BOX, &tm_k, &full[s], kb * 64, h, c * CH, b);
       tc5::tma_load_2d(st + kb * 2 * BOX + BOX, &tm_w, &full[s], kb * 64, row0);
-      tc5::tma_load_2d(st + 4 * BOX + kb * BOX, &tm_qd, &full[s], kb * 64, row0);
+      tc5::tma_load_4d(st + 4 * BOX + kb * BOX, &tm_q, &full[s], kb * 64, h, c * CH, b);
     }
     tc5::tma_load_2d(st + 6 * BOX, &tm_S, &full[s], vt * VT, (bh * NC + c) * KD);
+    tc5::tma_load_2d(st + 8 * BOX, &tm_qk, &full[s], 0, row0);
   };
   if (r == 0) issue_loads(NC - 1, 0);
 
-  constexpr uint32_t id_a = tc5::make_idesc_bf16(128, VT, 0, 1);        // [kt;w] (K-major) x dS (MN-major)
-  constexpr uint32_t id_c = tc5::make_idesc_bf16(128, KD, 0, 0);        // [v_new;do] x dS^T  and  [dv_tot;do] x S^T
-  constexpr uint32_t id_d = tc5::make_idesc_bf16(128, VT, 1, 1);        // q_dec^T x do
-  constexpr uint32_t id_dn = tc5::make_idesc_bf16(128, VT, 1, 1, 1);    // (-w)^T x dv_tot
-  const long part_rows = static_cast<long>(p.BH) * NC * CH;      // rows of one V tile's partials
+  constexpr uint32_t id_a = tc5::make_idesc_bf16(128, VT, 0, 1);        // [k;w] (K-major) x dS (MN-major)
+  constexpr uint32_t id_d = tc5::make_idesc_bf16(128, VT, 1, 1);        // q^T x (sq do), [qk^T ; 0] x do
+  constexpr uint32_t id_dn = tc5::make_idesc_bf16(128, VT, 1, 1, 1);    // (-w)^T x du
   bool ok = true;
-  // The chunk loop is one dependent chain: the rows that come straight from global memory (v_new and
-  // dv_new for rows 0..63, do for rows 64..127) and the decay are fetched one chunk ahead, so their
-  // latency is not paid once per chunk.
-  uint32_t row_next[32], dv_next[32];
-  auto fetch_rows = [&](int cc) {
-    const long rr = static_cast<long>(bh * NC + cc) * CH;
-    if (r < CH) {
-      load_row_global(p.v_new + (rr + r) * V + vt * VT, row_next);
-      load_row_global(p.dv_new + (rr + r) * V + vt * VT, dv_next);
-    } else {
-      load_row_global(p.d_o + (rr + r - CH) * V + vt * VT, row_next);
-    }
-  };
+  // The chunk loop is one dependent chain: the do rows (threads 64..127) and the gates are fetched one chunk ahead.
+  const float* gc = p.gc + static_cast<long>(bh) * NC * CH;
+  const bf16* d_o = p.d_o + (static_cast<long>(b) * p.T * p.H + h) * V + vt * VT;
+  uint32_t row_next[32];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) dv_next[j] = 0u;
+  for (int j = 0; j < 32; ++j) row_next[j] = 0u;
+  float gr_next, gl_next;
+  auto fetch_rows = [&](int cc) {
+    const int t = cc * CH + r - CH;
+    if (r >= CH) {
+      if (t < p.T) load_row_global(d_o + static_cast<long>(t) * p.H * V, row_next);
+      else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) row_next[j] = 0u;
+      }
+    }
+    gr_next = gc[cc * CH + (r & 63)];
+    gl_next = gc[cc * CH + CH - 1];
+  };
   fetch_rows(NC - 1);
-  float g_next = p.gamma[bh * NC + NC - 1];
   for (int it = 0; it < NC && ok; ++it) {
     const int c = NC - 1 - it;
     const int s = it & 1;
     uint8_t* st = smem + s * BWD_STAGE;
     const long row0 = static_cast<long>(bh * NC + c) * CH;
-    // stage this chunk's rows (already in registers) and start the next chunk's loads
-    uint32_t dvin[32];
+    const float g_row = gr_next, g_last = gl_next;
+    // stage this chunk's do rows (already in registers) and start the next chunk's loads
+    if (r >= CH) {
+      write_row_swz(sDO, r - CH, row_next);
+      float f[64];
+      unpack_row(row_next, f);
+      const float sq = p.scale * __expf(g_row);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) dvin[j] = dv_next[j];
-    write_row_swz(AV, r, row_next);
-    if (r >= CH) write_row_swz(AD, r, row_next);
-    const float g = g_next;
-    if (c > 0) {
-      fetch_rows(c - 1);
-      g_next = p.gamma[bh * NC + c - 1];
+      for (int j = 0; j < 64; ++j) f[j] *= sq;
+      uint32_t pk[32];
+      pack_row(f, pk);
+      write_row_swz(sDOs, r - CH, pk);
     }
+    if (c > 0) fetch_rows(c - 1);
     tc5::fence_proxy_async();
     tc5::fence_before_sync();
     __syncthreads();
@@ -440,104 +479,79 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       if (__all_sync(0xffffffffu, tc5::mbar_wait(&full[s], (it >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL))) {
         tc5::fence_after_sync();
         const uint64_t a = tc5::desc_kmajor(tc5::smem_u32(st)), dsbm = tc5::desc_mnmajor(tc5::smem_u32(dSb), BOX);
-        const uint64_t dsbk = tc5::desc_kmajor(tc5::smem_u32(dSb)), av = tc5::desc_kmajor(tc5::smem_u32(AV));
+        const uint64_t qk = tc5::desc_mnmajor(tc5::smem_u32(st + 8 * BOX), BOX), dom = tc5::desc_mnmajor(tc5::smem_u32(sDO), BOX);
         if (lead) {
 #pragma unroll
-          for (int kk = 0; kk < KD / 16; ++kk)      // Da = [k_tail ; w] * dS
+          for (int kk = 0; kk < KD / 16; ++kk)      // Da = [k ; w] dS
             tc5::mma_ss(tmem + cDa, a + static_cast<uint64_t>(((kk >> 2) * 2 * BOX + (kk & 3) * 32) >> 4),
                         dsbm + static_cast<uint64_t>((kk * 2048) >> 4), id_a, kk > 0 ? 1u : 0u);
 #pragma unroll
-          for (int kk = 0; kk < VT / 16; ++kk)      // Dc = [v_new ; do] * dS^T
-            tc5::mma_ss(tmem + cDc, av + static_cast<uint64_t>((kk * 32) >> 4), dsbk + static_cast<uint64_t>((kk * 32) >> 4), id_c, kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < CH / 16; ++kk)      // Dd = [qk^T ; 0] do
+            tc5::mma_ss(tmem + cDd, qk + static_cast<uint64_t>((kk * 2048) >> 4), dom + static_cast<uint64_t>((kk * 2048) >> 4), id_d, kk > 0 ? 1u : 0u);
           tc5::mma_commit(m1);
           if (it + 1 < NC) issue_loads(c - 1, it + 1);
         }
       }
       __syncwarp();
     }
-    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous chunk's du / dk_tail tiles have been read
     if (!tc5::mbar_wait(m1, it & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
+    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous du tile has been read (one newer store: the dS tile)
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc5::fence_after_sync();
+    if (r < CH) {
+      float da[64], dd[64];
+      tmem_ld_row64(tmem + lane_off + cDa, da);
+      tmem_ld_row64(tmem + lane_off + cDd, dd);
+      const float sk = __expf(g_last - g_row);
+#pragma unroll
+      for (int j = 0; j < 64; ++j) da[j] = dd[j] + sk * da[j];
+      uint32_t pk[32];
+      pack_row(da, pk);
+      write_row_swz(sDU, r, pk);
+    }
     float part_dg = 0.f;
     {
-      // dS (entering from chunk c+1): dgamma partial with S_prev, then scale by gamma in place
+      // dS: dgamma partial with S_prev, then scaled by gamma in place
       float ds[64], sp[64];
       tmem_ld_row64(tmem + lane_off + cDs, ds);
       read_row_swz(st + 6 * BOX, r, sp);
+      const float g = __expf(g_last);
 #pragma unroll
       for (int j = 0; j < 64; ++j) { part_dg += ds[j] * sp[j]; ds[j] *= g; }
       tmem_st_row64(tmem + lane_off + cDs, ds);
     }
-    if (r < CH) {
-      float da[64], dvf[64];
-      tmem_ld_row64(tmem + lane_off + cDa, da);
-      unpack_row(dvin, dvf);
-#pragma unroll
-      for (int j = 0; j < 64; ++j) da[j] += dvf[j];
-      uint32_t pk[32];
-      pack_row(da, pk);
-      write_row_swz(AD, r, pk);
-      // dk_tail partial: row r of Dc, KD columns
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float dc[64];
-        tmem_ld_row64(tmem + lane_off + cDc + h * 64, dc);
-        uint32_t pk2[32];
-        pack_row(dc, pk2);
-        write_row_swz(Kst + h * BOX, r, pk2);
-      }
-    }
-    // block reduction of the dgamma partial
-    for (int o = 16; o > 0; o >>= 1) part_dg += __shfl_xor_sync(0xffffffffu, part_dg, o);
-    if ((r & 31) == 0) red[warp] = part_dg;
     tc5::fence_proxy_async();
     tc5::fence_before_sync();
     __syncthreads();
     if (r == 0) {
-      p.dgamma_part[(static_cast<long>(vt) * p.BH + bh) * NC + c] = red[0] + red[1] + red[2] + red[3];
-      tc5::tma_store_2d(&tm_du, AD, vt * VT, static_cast<int>(row0));
-      tc5::tma_store_2d(&tm_dkt, Kst, 0, static_cast<int>(vt * part_rows + row0));
-      tc5::tma_store_2d(&tm_dkt, Kst + BOX, 64, static_cast<int>(vt * part_rows + row0));
+      tc5::tma_store_2d(&tm_du, sDU, vt * VT, static_cast<int>(row0));
       tc5::tma_store_commit();
     }
     if (warp == 0) {
       const bool lead = tc5::elect_one();
       tc5::fence_after_sync();
-      const uint64_t adk = tc5::desc_kmajor(tc5::smem_u32(AD)), spk = tc5::desc_kmajor(tc5::smem_u32(st + 6 * BOX));
-      const uint64_t qdm = tc5::desc_mnmajor(tc5::smem_u32(st + 4 * BOX), BOX), dom = tc5::desc_mnmajor(tc5::smem_u32(AD + BOX), BOX);
-      const uint64_t wm = tc5::desc_mnmajor(tc5::smem_u32(st + BOX), 2 * BOX), adm = tc5::desc_mnmajor(tc5::smem_u32(AD), BOX);
+      const uint64_t qdm = tc5::desc_mnmajor(tc5::smem_u32(st + 4 * BOX), BOX), dom = tc5::desc_mnmajor(tc5::smem_u32(sDOs), BOX);
+      const uint64_t wm = tc5::desc_mnmajor(tc5::smem_u32(st + BOX), 2 * BOX), dum = tc5::desc_mnmajor(tc5::smem_u32(sDU), BOX);
       if (lead) {
 #pragma unroll
-        for (int kk = 0; kk < VT / 16; ++kk)        // Db = [dv_tot ; do] * S_prev^T
-          tc5::mma_ss(tmem + cDb, adk + static_cast<uint64_t>((kk * 32) >> 4), spk + static_cast<uint64_t>((kk * 32) >> 4), id_c, kk > 0 ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < CH / 16; ++kk)        // dS += q_dec^T * do      (do = rows 64..127 of AD)
+        for (int kk = 0; kk < CH / 16; ++kk)        // dS += q^T (sq do)
           tc5::mma_ss(tmem + cDs, qdm + static_cast<uint64_t>((kk * 2048) >> 4), dom + static_cast<uint64_t>((kk * 2048) >> 4), id_d, 1u);
 #pragma unroll
-        for (int kk = 0; kk < CH / 16; ++kk)        // dS -= w^T * dv_tot      (w = second half of each k-block)
-          tc5::mma_ss(tmem + cDs, wm + static_cast<uint64_t>((kk * 2048) >> 4), adm + static_cast<uint64_t>((kk * 2048) >> 4), id_dn, 1u);
+        for (int kk = 0; kk < CH / 16; ++kk)        // dS -= w^T du      (w = second half of each k-block)
+          tc5::mma_ss(tmem + cDs, wm + static_cast<uint64_t>((kk * 2048) >> 4), dum + static_cast<uint64_t>((kk * 2048) >> 4), id_dn, 1u);
         tc5::mma_commit(m2);
       }
       __syncwarp();
     }
-    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous chunk's dw / dq_dec tiles have been read
+    // block reduction of the dgamma partial, behind the MMAs
+    for (int o = 16; o > 0; o >>= 1) part_dg += __shfl_xor_sync(0xffffffffu, part_dg, o);
+    if ((r & 31) == 0) red[warp] = part_dg;
+    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous dS tile has been read
     if (!tc5::mbar_wait(m2, it & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc5::fence_after_sync();
-    {
-      // rows 0..63: -dw partial; rows 64..127: dq_dec partial
-      const float sign = r < CH ? -1.f : 1.f;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float db[64];
-        tmem_ld_row64(tmem + lane_off + cDb + h * 64, db);
-#pragma unroll
-        for (int j = 0; j < 64; ++j) db[j] *= sign;
-        uint32_t pk[32];
-        pack_row(db, pk);
-        write_row_swz(Wst + h * 2 * BOX, r, pk);
-      }
+    if (r == 0) p.dgamma_part[(static_cast<long>(vt) * p.BH + bh) * NC + c] = red[0] + red[1] + red[2] + red[3];
+    if (c > 0) {
       float ds[64];
       tmem_ld_row64(tmem + lane_off + cDs, ds);
       uint32_t pk[32];
@@ -547,13 +561,8 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     tc5::fence_proxy_async();
     tc5::fence_before_sync();
     __syncthreads();
-    if (r == 0) {
-      const int prow = static_cast<int>(vt * part_rows + row0);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        tc5::tma_store_2d(&tm_dw, Wst + h * 2 * BOX, h * 64, prow);
-        tc5::tma_store_2d(&tm_dqd, Wst + h * 2 * BOX + BOX, h * 64, prow);
-      }
+    if (r == 0 && c > 0) {
+      tc5::tma_store_2d(&tm_ds, dSb, vt * VT, (bh * NC + c - 1) * KD);
       tc5::tma_store_commit();
     }
   }
@@ -568,71 +577,74 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
   tc5::fence_before_sync();
   __syncthreads();
-  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 512); }
+  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 256); }
 }
 
 int make_rows_map(CUtensorMap* m, const void* base, long rows, int cols, int box_rows) {
   return nsa::make_tmap_2d_bf16(m, base, cols, rows, cols, 64, box_rows);
 }
+// [B, T, H, D] token-major; box: 64 tokens of one head, 64 columns
+int make_token_map(CUtensorMap* m, const void* base, int B, int T, int H, int D) {
+  uint64_t dims[4] = {(uint64_t)D, (uint64_t)H, (uint64_t)T, (uint64_t)B};
+  uint64_t strides[3] = {(uint64_t)D * 2, (uint64_t)H * D * 2, (uint64_t)T * H * D * 2};
+  uint32_t box[4] = {64, 1, (uint32_t)CH, 1};
+  return nsa::make_tmap_bf16(m, base, 4, dims, strides, box, 1);
+}
+template <typename F>
+int set_smem(F* kernel, int bytes, const char* what) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e == cudaSuccess ? 0 : nsa::fail_cuda(e, what);
+}
 }  // namespace
 
-// w, qd, kt: [BH*NC*64, 128] bf16; u: [BH*NC*64, V] bf16; gamma: [BH*NC] fp32.
-// Outputs: v_new [BH*NC*64, V] bf16, o_inter [BH*NC*64, V] bf16, S_all [BH*NC*128, V] bf16.
-extern "C" int nsa_gdn_seq_fwd(const void* w, const void* qd, const void* kt, const void* u, const float* gamma,
-                               void* v_new, void* o_inter, void* S_all, int BH, int NC, int K, int V,
+// q, k [B, T, H, 128] bf16; w [B*H, NC, 64, 128], u [.., 64, V], qk [.., 64, 64] bf16 and gc [B*H, NC, 64] fp32 from
+// nsa_gdn_prep.  o [B, T, H, V]; v_new [B*H, NC, 64, V] and S_all [B*H, NC, 128, V] (states entering the chunks) are
+// written for the backward, or null.
+extern "C" int nsa_gdn_seq_fwd(const void* q, const void* k, const void* w, const void* u, const void* qk, const float* gc,
+                               void* o, void* v_new, void* S_all, int B, int T, int H, int K, int V, float scale,
                                cudaStream_t st) {
   if (K != KD || V % VT) return nsa::fail(NSA_ERR_SHAPE, "gdn: key width must be 128 and value width a multiple of 64");
-  CUtensorMap tw, tq, tk;
+  const int NC = (T + CH - 1) / CH, BH = B * H;
   const long rows = static_cast<long>(BH) * NC * CH;
+  const bool states = v_new != nullptr && S_all != nullptr;
+  CUtensorMap tw, tq, tk, tqk, tvn, to, tsa;
   int rc;
-  if ((rc = make_rows_map(&tw, w, rows, KD, 64))) return rc;
-  if ((rc = make_rows_map(&tq, qd, rows, KD, 64))) return rc;
-  if ((rc = make_rows_map(&tk, kt, rows, KD, 64))) return rc;
-  CUtensorMap tvn, toi, tsa;
-  if ((rc = make_rows_map(&tvn, v_new, rows, V, CH))) return rc;
-  if ((rc = make_rows_map(&toi, o_inter, rows, V, CH))) return rc;
-  if ((rc = make_rows_map(&tsa, S_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
-  FwdParams p{(const bf16*)u, gamma, (bf16*)v_new, (bf16*)o_inter, (bf16*)S_all, NC, V, nsa::status_ptr()};
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gdn_seq_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM);
-    if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn fwd smem attribute");
-    configured = true;
-  }
-  gdn_seq_fwd_kernel<<<dim3(V / VT, BH), 128, FWD_SMEM, st>>>(tw, tq, tk, tvn, toi, tsa, p);
+  if ((rc = make_rows_map(&tw, w, rows, KD, CH))) return rc;
+  if ((rc = make_token_map(&tq, q, B, T, H, KD))) return rc;
+  if ((rc = make_token_map(&tk, k, B, T, H, KD))) return rc;
+  if ((rc = make_rows_map(&tqk, qk, rows, CH, CH))) return rc;
+  if ((rc = make_token_map(&to, o, B, T, H, V))) return rc;
+  tvn = tw; tsa = tw;                              // never used without the states
+  if (states && (rc = make_rows_map(&tvn, v_new, rows, V, CH))) return rc;
+  if (states && (rc = make_rows_map(&tsa, S_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
+  FwdParams p{(const bf16*)u, gc, states, NC, V, H, scale, nsa::status_ptr()};
+  if ((rc = set_smem(gdn_seq_fwd_kernel, FWD_SMEM, "gdn fwd smem attribute"))) return rc;
+  gdn_seq_fwd_kernel<<<dim3(V / VT, BH), 128, FWD_SMEM, st>>>(tw, tq, tk, tqk, tvn, to, tsa, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_seq_fwd launch");
 }
 
-// Partials: dw_part/dqd_part/dkt_part [V/64, BH*NC*64, 128] bf16, dgamma_part [V/64, BH*NC] fp32.
-extern "C" int nsa_gdn_seq_bwd(const void* w, const void* qd, const void* kt, const void* S_all, const void* v_new,
-                               const void* dv_new, const void* d_o, const float* gamma, void* du, void* dw_part,
-                               void* dqd_part, void* dkt_part, float* dgamma_part, int BH, int NC, int K, int V,
-                               cudaStream_t st) {
+// d_o [B, T, H, V] bf16.  Outputs: du [B*H, NC, 64, V], dS_all [B*H, NC, 128, V] (gradients of the states leaving the
+// chunks) bf16, dgamma_part [V/64, B*H, NC] fp32.
+extern "C" int nsa_gdn_seq_bwd(const void* q, const void* k, const void* w, const void* qk, const void* S_all, const void* d_o,
+                               const float* gc, void* du, void* dS_all, float* dgamma_part, int B, int T, int H, int K, int V,
+                               float scale, cudaStream_t st) {
   if (K != KD || V % VT) return nsa::fail(NSA_ERR_SHAPE, "gdn: key width must be 128 and value width a multiple of 64");
-  CUtensorMap tw, tq, tk, ts;
+  const int NC = (T + CH - 1) / CH, BH = B * H;
   const long rows = static_cast<long>(BH) * NC * CH;
+  CUtensorMap tw, tq, tk, tqk, ts, tdu, tds;
   int rc;
-  if ((rc = make_rows_map(&tw, w, rows, KD, 64))) return rc;
-  if ((rc = make_rows_map(&tq, qd, rows, KD, 64))) return rc;
-  if ((rc = make_rows_map(&tk, kt, rows, KD, 64))) return rc;
+  if ((rc = make_rows_map(&tw, w, rows, KD, CH))) return rc;
+  if ((rc = make_token_map(&tq, q, B, T, H, KD))) return rc;
+  if ((rc = make_token_map(&tk, k, B, T, H, KD))) return rc;
+  if ((rc = make_rows_map(&tqk, qk, rows, CH, CH))) return rc;
   if ((rc = make_rows_map(&ts, S_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
-  CUtensorMap tdu, tdkt, tdw, tdqd;
-  const long prows = rows * (V / VT);
   if ((rc = make_rows_map(&tdu, du, rows, V, CH))) return rc;
-  if ((rc = make_rows_map(&tdkt, dkt_part, prows, KD, CH))) return rc;
-  if ((rc = make_rows_map(&tdw, dw_part, prows, KD, CH))) return rc;
-  if ((rc = make_rows_map(&tdqd, dqd_part, prows, KD, CH))) return rc;
-  BwdParams p{(const bf16*)v_new, (const bf16*)dv_new, (const bf16*)d_o, gamma, (bf16*)du, (bf16*)dw_part,
-              (bf16*)dqd_part, (bf16*)dkt_part, dgamma_part, NC, V, BH, nsa::status_ptr()};
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gdn_seq_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
-    if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn bwd smem attribute");
-    configured = true;
-  }
-  gdn_seq_bwd_kernel<<<dim3(V / VT, BH), 128, BWD_SMEM, st>>>(tw, tq, tk, ts, tdu, tdkt, tdw, tdqd, p);
+  if ((rc = make_rows_map(&tds, dS_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
+  BwdParams p{(const bf16*)d_o, gc, dgamma_part, NC, V, BH, H, T, scale, nsa::status_ptr()};
+  if ((rc = set_smem(gdn_seq_bwd_kernel, BWD_SMEM, "gdn bwd smem attribute"))) return rc;
+  gdn_seq_bwd_kernel<<<dim3(V / VT, BH), 128, BWD_SMEM, st>>>(tw, tq, tk, ts, tqk, tdu, tds, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_seq_bwd launch");

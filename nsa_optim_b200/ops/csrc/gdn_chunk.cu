@@ -1,0 +1,630 @@
+// Gated DeltaNet: everything of the chunkwise gated delta rule that is local to a chunk of 64 tokens, one
+// kernel in front of the sequential state kernels of gdn.cu and one behind their backward.
+//
+// With gc the cumulative log-decay inside the chunk, sq_i = scale e^gc_i, sk_i = e^(gc_last - gc_i):
+//     A[i][j]  = beta_i (k_i . k_j) e^(gc_i - gc_j)   (j < i)         X = (I + A)^-1
+//     Tu = X diag(beta), Tw = X diag(beta e^gc)                       u = Tu v, w = Tw k
+//     qk[i][j] = scale (q_i . k_j) e^(gc_i - gc_j)    (j <= i)
+// q, k, v and the gates are read token-major as the caller has them, gradients leave the same way.
+#include "host.cuh"
+#include "mma16.cuh"
+
+namespace {
+using namespace mma16;
+constexpr int CH = 64, KD = 128;
+constexpr int PK = KD + 8, PC = CH + 8;          // tile pitches (elements)
+constexpr int PX = 68;                           // pitch of the fp32 64 x 64 tiles: rows 16-byte aligned, spread over the banks
+
+// Per-chunk gate quantities; 64 threads (two warps) call it, t = token of the row, the caller synchronises.
+// gs: cumulative log-decay, bs: beta.
+__device__ __forceinline__ void load_gates(const float* g, const float* beta, long tok0, int T, int t0, int H, float* gs, float* bs) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    const int ta = t0 + 2 * lane, tb = ta + 1;
+    const float a = ta < T ? g[tok0 + static_cast<long>(ta) * H] : 0.f, b = tb < T ? g[tok0 + static_cast<long>(tb) * H] : 0.f;
+    bs[2 * lane] = ta < T ? beta[tok0 + static_cast<long>(ta) * H] : 0.f;
+    bs[2 * lane + 1] = tb < T ? beta[tok0 + static_cast<long>(tb) * H] : 0.f;
+    float s = a + b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float n = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += n;
+    }
+    gs[2 * lane] = s - b;
+    gs[2 * lane + 1] = s;
+  }
+}
+
+struct PrepParams {
+  const bf16 *q, *k, *v;       // [B, T, H, .]
+  const float *g, *beta;       // [B, T, H]
+  bf16 *w, *u, *qk;            // [BH, NC, 64, 128 / V / 64]
+  float *X, *gc;               // [BH, NC, 64, 64] or null, [BH, NC, 64]
+  int T, H, NC, V;
+  float scale;
+};
+
+// One CTA of eight warps per (chunk, head).  Bound by the memory traffic of q, k, v, u, w (2 KB per token and head)
+// once two CTAs share an SM; the triangular inverse is the longest dependent phase and runs as two
+// 32-column substitutions side by side, joined by two 32 x 32 products over all threads.
+__global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const int V = p.V, PV = V + 8;
+  bf16* sK = reinterpret_cast<bf16*>(smem_raw);            // rows 0..63 k, 64..127 q
+  bf16* sV = sK + 2 * CH * PK;
+  float* As = reinterpret_cast<float*>(sV + CH * PV);      // [64][PX]
+  float* Xs = As + CH * PX;
+  bf16* sTu = reinterpret_cast<bf16*>(Xs + CH * PX);
+  bf16* sTw = sTu + CH * PC;
+  float* gs = reinterpret_cast<float*>(sTw + CH * PC);
+  float* bs = gs + CH;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int c = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
+  const int t0 = c * CH;
+  const long tok0 = static_cast<long>(b) * p.T * p.H + h;  // (b, t, h) = tok0 + t * H
+  for (int i = tid; i < CH * (KD / 8); i += 256) {
+    const int r = i / (KD / 8), cc = (i % (KD / 8)) * 8, t = t0 + r;
+    const bool ok = t < p.T;
+    const long off = (tok0 + static_cast<long>(ok ? t : 0) * p.H) * KD + cc;
+    cp_async16(sK + r * PK + cc, p.k + off, ok);
+    cp_async16(sK + (CH + r) * PK + cc, p.q + off, ok);
+  }
+  cp_async_commit();
+  const int v8 = V / 8;
+  for (int i = tid; i < CH * v8; i += 256) {
+    const int r = i / v8, cc = (i - r * v8) * 8, t = t0 + r;
+    const bool ok = t < p.T;
+    cp_async16(sV + r * PV + cc, p.v + (tok0 + static_cast<long>(ok ? t : 0) * p.H) * V + cc, ok);
+  }
+  cp_async_commit();
+  load_gates(p.g, p.beta, tok0, p.T, t0, p.H, gs, bs);
+  cp_async_wait<1>();
+  __syncthreads();
+  const long chunk = static_cast<long>(bh) * p.NC + c;
+  if (tid < CH) p.gc[chunk * CH + tid] = gs[tid];
+  // ---- [k ; q] k^T: warp w owns rows 16 w .. of the stacked 128
+  {
+    float acc[8][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < KD; kk += 16) {
+      uint32_t a[4];
+      load_a(a, sK, PK, warp * 16, kk);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        uint32_t bb[4];
+        load_b(bb, sK, PK, n * 16, kk);
+        mma2(acc[2 * n], acc[2 * n + 1], a, bb);
+      }
+    }
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int i = (warp & 3) * 16 + (lane >> 2) + 8 * hh;
+      const float gi = gs[i], bi = bs[i];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        const int j = n * 8 + 2 * (lane & 3);
+        // the exponent is zero where the entry is masked, so nothing overflows
+        const float e0 = __expf(j <= i ? gi - gs[j] : 0.f), e1 = __expf(j + 1 <= i ? gi - gs[j + 1] : 0.f);
+        const float x0 = acc[n][2 * hh] * e0, x1 = acc[n][2 * hh + 1] * e1;
+        if (warp < 4) {
+          *reinterpret_cast<float2*>(As + i * PX + j) = make_float2(j < i ? bi * x0 : 0.f, j + 1 < i ? bi * x1 : 0.f);
+        } else {
+          *reinterpret_cast<uint32_t*>(p.qk + (chunk * CH + i) * CH + j) =
+              pack2(j <= i ? p.scale * x0 : 0.f, j + 1 <= i ? p.scale * x1 : 0.f);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // ---- X = (I + A)^-1.  Diagonal 32 x 32 blocks: thread (block, column) substitutes forward
+  if (warp < 2) {
+    const float* Ad = As + warp * 32 * PX + warp * 32;
+    float x[32];
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+      float s[4] = {r == lane ? 1.f : 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < r; j += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(Ad + r * PX + j);   // zero from column r on
+        s[0] = fmaf(-a.x, x[j], s[0]);
+        if (j + 1 < r) s[1] = fmaf(-a.y, x[j + 1], s[1]);
+        if (j + 2 < r) s[2] = fmaf(-a.z, x[j + 2], s[2]);
+        if (j + 3 < r) s[3] = fmaf(-a.w, x[j + 3], s[3]);
+      }
+      x[r] = (s[0] + s[1]) + (s[2] + s[3]);
+    }
+#pragma unroll
+    for (int r = 0; r < 32; ++r) Xs[(warp * 32 + r) * PX + warp * 32 + lane] = x[r];
+  } else if (warp < 4) {
+    for (int r = (warp - 2) * 16; r < (warp - 2) * 16 + 16; ++r) Xs[r * PX + 32 + lane] = 0.f;
+  }
+  __syncthreads();
+  // ---- X21 = -X22 (A21 X11); the product in the middle goes to the unused upper block of As
+  {
+    const int i = tid >> 3, c4 = (tid & 7) * 4;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int j = 0; j < 32; ++j) {
+      const float a = As[(32 + i) * PX + j];
+      const float4 x = *reinterpret_cast<const float4*>(Xs + j * PX + c4);
+      s.x = fmaf(a, x.x, s.x); s.y = fmaf(a, x.y, s.y); s.z = fmaf(a, x.z, s.z); s.w = fmaf(a, x.w, s.w);
+    }
+    *reinterpret_cast<float4*>(As + i * PX + 32 + c4) = s;
+    __syncthreads();
+    s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int j = 0; j < 32; ++j) {
+      const float a = Xs[(32 + i) * PX + 32 + j];
+      const float4 m = *reinterpret_cast<const float4*>(As + j * PX + 32 + c4);
+      s.x = fmaf(-a, m.x, s.x); s.y = fmaf(-a, m.y, s.y); s.z = fmaf(-a, m.z, s.z); s.w = fmaf(-a, m.w, s.w);
+    }
+    *reinterpret_cast<float4*>(Xs + (32 + i) * PX + c4) = s;
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int i = tid; i < CH * CH / 4; i += 256) {
+    const int r = i / (CH / 4), j = (i % (CH / 4)) * 4;
+    const float4 x = *reinterpret_cast<const float4*>(Xs + r * PX + j);
+    if (p.X) *reinterpret_cast<float4*>(p.X + (chunk * CH + r) * CH + j) = x;
+    const float u0 = x.x * bs[j], u1 = x.y * bs[j + 1], u2 = x.z * bs[j + 2], u3 = x.w * bs[j + 3];
+    *reinterpret_cast<uint2*>(sTu + r * PC + j) = make_uint2(pack2(u0, u1), pack2(u2, u3));
+    *reinterpret_cast<uint2*>(sTw + r * PC + j) = make_uint2(pack2(u0 * __expf(gs[j]), u1 * __expf(gs[j + 1])),
+                                                             pack2(u2 * __expf(gs[j + 2]), u3 * __expf(gs[j + 3])));
+  }
+  __syncthreads();
+  // ---- u = Tu v and w = Tw k, 16 columns at a time; a warp is the only reader of its columns and
+  //      puts the result in their place
+  for (int unit = warp; unit < (V + KD) / 16; unit += 8) {
+    const bool is_u = unit < V / 16;
+    bf16* src = is_u ? sV : sK;
+    const bf16* tm = is_u ? sTu : sTw;
+    const int pitch = is_u ? PV : PK, n0 = (is_u ? unit : unit - V / 16) * 16;
+    float acc[4][2][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < CH; kk += 16) {
+      uint32_t bb[4];
+      load_b_t(bb, src, pitch, n0, kk);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        if (kk > m * 16) continue;                 // the matrices are lower triangular
+        uint32_t a[4];
+        load_a(a, tm, PC, m * 16, kk);
+        mma2(acc[m][0], acc[m][1], a, bb);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh)
+          *reinterpret_cast<uint32_t*>(src + (m * 16 + (lane >> 2) + 8 * hh) * pitch + n0 + n * 8 + 2 * (lane & 3)) =
+              pack2(acc[m][n][2 * hh], acc[m][n][2 * hh + 1]);
+  }
+  __syncthreads();
+  for (int i = tid; i < CH * v8; i += 256) {
+    const int r = i / v8, cc = (i - r * v8) * 8;
+    *reinterpret_cast<uint4*>(p.u + (chunk * CH + r) * V + cc) = *reinterpret_cast<const uint4*>(sV + r * PV + cc);
+  }
+  for (int i = tid; i < CH * (KD / 8); i += 256) {
+    const int r = i / (KD / 8), cc = (i % (KD / 8)) * 8;
+    *reinterpret_cast<uint4*>(p.w + (chunk * CH + r) * KD + cc) = *reinterpret_cast<const uint4*>(sK + r * PK + cc);
+  }
+}
+
+struct PostParams {
+  const bf16 *q, *k, *v, *d_o;          // [B, T, H, .]
+  const float* beta;                    // [B, T, H]
+  const float *gc, *X;                  // [BH, NC, 64], [BH, NC, 64, 64]
+  const bf16 *v_new, *du;               // [BH, NC, 64, V]
+  const bf16 *S, *dS;                   // [BH, NC, 128, V]: state entering the chunk, gradient of the state leaving it
+  const float* dgamma;                  // [V / 64, BH, NC]: <state entering, gradient of the state leaving> per V tile
+  bf16 *dq, *dk, *dv;                   // [B, T, H, .]
+  float *dg, *dbeta;                    // [B, T, H]
+  int B, T, H, NC, V;
+  float scale;
+};
+
+constexpr int POST_SLICE = (2 * KD + 4 * CH) * PC * 2;                     // S, dS, do, v_new, du, v: 64 columns each
+constexpr int POST_SMEM = 2 * CH * PK * 2 + 2 * POST_SLICE + CH * PX * 4 + CH * PC * 2 + (2 + 16) * CH * 4;
+
+// One CTA of sixteen warps per (chunk, head): every gradient of the chunk once du (of the sequential pass) and
+// the two states are known.
+//     dw = -du S^T, dqs = do S^T, dks = v_new dS^T, dqk = do v_new^T, dTu = du v^T, dTw = dw k^T
+//     dX = (dTu + dTw e^gc) beta (columns), dA = -(X^T dX X^T), then through the definitions above.
+// The value dimension is walked in slices of 64 columns, the next one in flight; all products that sum over it
+// accumulate in registers.  Memory bound by design: 3.5 KB in and 1 KB out per token and head, against 6 KB
+// alone for the per-V-tile partials of dw, dq and dk that the sequential pass would have to write and re-read.
+__global__ void __launch_bounds__(512, 1) gdn_post_kernel(const PostParams p) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  bf16* sK = reinterpret_cast<bf16*>(smem_raw);
+  bf16* sQ = sK + CH * PK;
+  uint8_t* slices = reinterpret_cast<uint8_t*>(sQ + CH * PK);
+  float* Xs = reinterpret_cast<float*>(slices + 2 * POST_SLICE);
+  bf16* sTu = reinterpret_cast<bf16*>(Xs + CH * PX);
+  float* gs = reinterpret_cast<float*>(sTu + CH * PC);
+  float* bs = gs + CH;
+  float* red = bs + CH;                                    // [16][64]
+  // over the slices once they are done
+  bf16* sW = reinterpret_cast<bf16*>(slices);              // dw   [64][PK]
+  float* sDX = reinterpret_cast<float*>(sW + CH * PK);     // [64][PX], later dA
+  float* sY = sDX + CH * PX;                               // [64][PX]
+  bf16* sTw = reinterpret_cast<bf16*>(sY + CH * PX);
+  bf16* sDK = sTw + CH * PC;                               // d(k k^T)
+  bf16* sDQ = sDK + CH * PC;                               // d(q k^T)
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int c = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
+  const int t0 = c * CH, V = p.V, nvt = V / CH;
+  const long tok0 = static_cast<long>(b) * p.T * p.H + h;
+  const long chunk = static_cast<long>(bh) * p.NC + c;
+  auto load_slice = [&](int s) {
+    bf16* d = reinterpret_cast<bf16*>(slices + (s & 1) * POST_SLICE);
+    for (int i = tid; i < KD * 8; i += 512) {
+      const int r = i >> 3, cc = (i & 7) * 8;
+      const long off = (chunk * KD + r) * V + s * CH + cc;
+      cp_async16(d + r * PC + cc, p.S + off, true);
+      cp_async16(d + (KD + r) * PC + cc, p.dS + off, true);
+    }
+    d += 2 * KD * PC;
+    for (int i = tid; i < CH * 8; i += 512) {
+      const int r = i >> 3, cc = (i & 7) * 8, t = t0 + r;
+      const bool ok = t < p.T;
+      const long tm = (tok0 + static_cast<long>(ok ? t : 0) * p.H) * V + s * CH + cc, cm = (chunk * CH + r) * V + s * CH + cc;
+      cp_async16(d + r * PC + cc, p.d_o + tm, ok);
+      cp_async16(d + (CH + r) * PC + cc, p.v_new + cm, true);
+      cp_async16(d + (2 * CH + r) * PC + cc, p.du + cm, true);
+      cp_async16(d + (3 * CH + r) * PC + cc, p.v + tm, ok);
+    }
+    cp_async_commit();
+  };
+  for (int i = tid; i < CH * (KD / 8); i += 512) {
+    const int r = i / (KD / 8), cc = (i % (KD / 8)) * 8, t = t0 + r;
+    const bool ok = t < p.T;
+    const long off = (tok0 + static_cast<long>(ok ? t : 0) * p.H) * KD + cc;
+    cp_async16(sK + r * PK + cc, p.k + off, ok);
+    cp_async16(sQ + r * PK + cc, p.q + off, ok);
+  }
+  load_slice(0);
+  if (tid < CH) {
+    gs[tid] = p.gc[chunk * CH + tid];
+    bs[tid] = t0 + tid < p.T ? p.beta[tok0 + static_cast<long>(t0 + tid) * p.H] : 0.f;
+  }
+  __syncthreads();
+  for (int i = tid; i < CH * CH / 4; i += 512) {
+    const int r = i / (CH / 4), j = (i % (CH / 4)) * 4;
+    const float4 x = *reinterpret_cast<const float4*>(p.X + (chunk * CH + r) * CH + j);
+    *reinterpret_cast<float4*>(Xs + r * PX + j) = x;
+    *reinterpret_cast<uint2*>(sTu + r * PC + j) = make_uint2(pack2(x.x * bs[j], x.y * bs[j + 1]), pack2(x.z * bs[j + 2], x.w * bs[j + 3]));
+  }
+  const int m0 = (warp & 3) * 16, n32 = (warp >> 2) * 32, n16 = (warp >> 2) * 16;
+  const int r0 = m0 + (lane >> 2), cl = 2 * (lane & 3);    // first row and column offset of this lane's accumulator elements
+  float aW[4][4] = {}, aQ[4][4] = {}, aK[4][4] = {}, aP[2][4] = {}, aT[2][4] = {};
+  for (int s = 0; s < nvt; ++s) {
+    if (s + 1 < nvt) { load_slice(s + 1); cp_async_wait<1>(); }
+    else cp_async_wait<0>();
+    __syncthreads();
+    const bf16* tS = reinterpret_cast<const bf16*>(slices + (s & 1) * POST_SLICE);
+    const bf16 *tD = tS + KD * PC, *tO = tD + KD * PC, *tN = tO + CH * PC, *tU = tN + CH * PC, *tV = tU + CH * PC;
+#pragma unroll
+    for (int kk = 0; kk < CH; kk += 16) {
+      uint32_t au[4], ao[4], an[4], bb[4];
+      load_a(au, tU, PC, m0, kk);
+      load_a(ao, tO, PC, m0, kk);
+      load_a(an, tN, PC, m0, kk);
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        load_b(bb, tS, PC, n32 + n * 16, kk);
+        mma2(aW[2 * n], aW[2 * n + 1], au, bb);
+        mma2(aQ[2 * n], aQ[2 * n + 1], ao, bb);
+        load_b(bb, tD, PC, n32 + n * 16, kk);
+        mma2(aK[2 * n], aK[2 * n + 1], an, bb);
+      }
+      load_b(bb, tN, PC, n16, kk);
+      mma2(aP[0], aP[1], ao, bb);
+      load_b(bb, tV, PC, n16, kk);
+      mma2(aT[0], aT[1], au, bb);
+    }
+    // dv of this slice: Tu^T du (row j needs i >= j only)
+    float dv[2][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < CH; kk += 16) {
+      if (kk < m0) continue;
+      uint32_t a[4], bb[4];
+      load_a_t(a, sTu, PC, m0, kk);
+      load_b_t(bb, tU, PC, n16, kk);
+      mma2(dv[0], dv[1], a, bb);
+    }
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int t = t0 + r0 + 8 * hh;
+      if (t >= p.T) continue;
+      bf16* dst = p.dv + (tok0 + static_cast<long>(t) * p.H) * V + s * CH + n16 + cl;
+#pragma unroll
+      for (int n = 0; n < 2; ++n) *reinterpret_cast<uint32_t*>(dst + n * 8) = pack2(dv[n][2 * hh], dv[n][2 * hh + 1]);
+    }
+    __syncthreads();                                       // the slice's buffer is refilled two slices on
+  }
+  const float g_last = gs[CH - 1];
+  // ---- dw as an operand; row sums q . dqs and k . dks (gates that scale rows of q and k); Tw
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    const int i = r0 + 8 * hh;
+    float dq_s = 0.f, dk_s = 0.f;
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int j = n32 + n * 8 + cl;
+      *reinterpret_cast<uint32_t*>(sW + i * PK + j) = pack2(-aW[n][2 * hh], -aW[n][2 * hh + 1]);
+      const float2 qv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sQ + i * PK + j));
+      const float2 kv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sK + i * PK + j));
+      dq_s += aQ[n][2 * hh] * qv.x + aQ[n][2 * hh + 1] * qv.y;
+      dk_s += aK[n][2 * hh] * kv.x + aK[n][2 * hh + 1] * kv.y;
+    }
+    dq_s += __shfl_xor_sync(0xffffffffu, dq_s, 1);
+    dk_s += __shfl_xor_sync(0xffffffffu, dk_s, 1);
+    dq_s += __shfl_xor_sync(0xffffffffu, dq_s, 2);
+    dk_s += __shfl_xor_sync(0xffffffffu, dk_s, 2);
+    if ((lane & 3) == 0) {
+      red[(warp >> 2) * CH + i] = dq_s;
+      red[(4 + (warp >> 2)) * CH + i] = dk_s;
+    }
+    const float sq = p.scale * __expf(gs[i]), sk = __expf(g_last - gs[i]);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      aQ[n][2 * hh] *= sq; aQ[n][2 * hh + 1] *= sq;
+      aK[n][2 * hh] *= sk; aK[n][2 * hh + 1] *= sk;
+    }
+  }
+  for (int i = tid; i < CH * CH / 4; i += 512) {
+    const int r = i / (CH / 4), j = (i % (CH / 4)) * 4;
+    const float4 x = *reinterpret_cast<const float4*>(Xs + r * PX + j);
+    *reinterpret_cast<uint2*>(sTw + r * PC + j) =
+        make_uint2(pack2(x.x * bs[j] * __expf(gs[j]), x.y * bs[j + 1] * __expf(gs[j + 1])),
+                   pack2(x.z * bs[j + 2] * __expf(gs[j + 2]), x.w * bs[j + 3] * __expf(gs[j + 3])));
+  }
+  __syncthreads();
+  // gradient of gc_i and beta_i, collected by thread i < 64
+  float dgc = 0.f, dbeta = 0.f, dlast = 0.f;
+  if (tid < CH) {
+    float a = 0.f, k_ = 0.f;
+#pragma unroll
+    for (int n = 0; n < 4; ++n) { a += red[n * CH + tid]; k_ += red[(4 + n) * CH + tid]; }
+    dlast = __expf(g_last - gs[tid]) * k_;
+    dgc = p.scale * __expf(gs[tid]) * a - dlast;
+  }
+  // ---- dTw = dw k^T, dX
+  {
+    float aw[2][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < KD; kk += 16) {
+      uint32_t a[4], bb[4];
+      load_a(a, sW, PK, m0, kk);
+      load_b(bb, sK, PK, n16, kk);
+      mma2(aw[0], aw[1], a, bb);
+    }
+    __syncthreads();                                       // red is read
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int j = n16 + n * 8 + cl + e;
+        const float eg = __expf(gs[j]), bj = bs[j];
+        float cb = 0.f, cg = 0.f;
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const int i = r0 + 8 * hh;
+          const float x = Xs[i * PX + j], tw = aw[n][2 * hh + e] * eg, d = aT[n][2 * hh + e] + tw;
+          sDX[i * PX + j] = j <= i ? d * bj : 0.f;
+          cb += d * x;                                     // x is zero above the diagonal
+          cg += tw * x;
+        }
+        cg *= bj;
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) {
+          cb += __shfl_xor_sync(0xffffffffu, cb, o);
+          cg += __shfl_xor_sync(0xffffffffu, cg, o);
+        }
+        if (lane < 4) {
+          red[(warp & 3) * CH + j] = cb;
+          red[(4 + (warp & 3)) * CH + j] = cg;
+        }
+      }
+  }
+  __syncthreads();
+  if (tid < CH)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) { dbeta += red[n * CH + tid]; dgc += red[(4 + n) * CH + tid]; }
+  // ---- dA = -(X^T dX X^T) below the diagonal, fp32; warp w owns rows 4 w .. 4 w + 3
+  {
+    const int ra = (tid >> 4) * 2, ca = (tid & 15) * 4;
+    float4 y0 = make_float4(0.f, 0.f, 0.f, 0.f), y1 = y0;
+#pragma unroll 4
+    for (int i = warp * 4; i < CH; ++i) {
+      const float2 x = *reinterpret_cast<const float2*>(Xs + i * PX + ra);
+      const float4 d = *reinterpret_cast<const float4*>(sDX + i * PX + ca);
+      y0.x = fmaf(x.x, d.x, y0.x); y0.y = fmaf(x.x, d.y, y0.y); y0.z = fmaf(x.x, d.z, y0.z); y0.w = fmaf(x.x, d.w, y0.w);
+      y1.x = fmaf(x.y, d.x, y1.x); y1.y = fmaf(x.y, d.y, y1.y); y1.z = fmaf(x.y, d.z, y1.z); y1.w = fmaf(x.y, d.w, y1.w);
+    }
+    *reinterpret_cast<float4*>(sY + ra * PX + ca) = y0;
+    *reinterpret_cast<float4*>(sY + (ra + 1) * PX + ca) = y1;
+    __syncthreads();
+    const int cb = tid & 15;
+    float s[2][4] = {};
+#pragma unroll 2
+    for (int j = 0; j < warp * 4 + 4; j += 4) {            // X[b][j] is zero for j > b, and b < a
+      const float4 ya = *reinterpret_cast<const float4*>(sY + ra * PX + j), yb = *reinterpret_cast<const float4*>(sY + (ra + 1) * PX + j);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float4 x = *reinterpret_cast<const float4*>(Xs + (cb + 16 * e) * PX + j);
+        s[0][e] += ya.x * x.x + ya.y * x.y + ya.z * x.z + ya.w * x.w;
+        s[1][e] += yb.x * x.x + yb.y * x.y + yb.z * x.z + yb.w * x.w;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      sDX[ra * PX + cb + 16 * e] = -s[0][e];
+      sDX[(ra + 1) * PX + cb + 16 * e] = -s[1][e];
+    }
+  }
+  __syncthreads();
+  // ---- through the definitions of A and qk
+  {
+    float kk_[2][4] = {}, qk_[2][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < KD; kk += 16) {
+      uint32_t a[4], bb[4];
+      load_b(bb, sK, PK, n16, kk);
+      load_a(a, sK, PK, m0, kk);
+      mma2(kk_[0], kk_[1], a, bb);
+      load_a(a, sQ, PK, m0, kk);
+      mma2(qk_[0], qk_[1], a, bb);
+    }
+    float col[2][2] = {};
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int i = r0 + 8 * hh;
+      const float gi = gs[i], bi = bs[i];
+      float rb = 0.f, rg = 0.f;
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        float ok[2], oq[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int j = n16 + n * 8 + cl + e;
+          const float ex = __expf(j <= i ? gi - gs[j] : 0.f);
+          const float d = j < i ? sDX[i * PX + j] : 0.f;
+          const float araw = kk_[n][2 * hh + e] * ex;
+          ok[e] = d * bi * ex;
+          oq[e] = j <= i ? aP[n][2 * hh + e] * p.scale * ex : 0.f;
+          const float t = d * bi * araw + oq[e] * qk_[n][2 * hh + e];
+          rb += d * araw;
+          rg += t;
+          col[n][e] -= t;
+        }
+        *reinterpret_cast<uint32_t*>(sDK + i * PC + n16 + n * 8 + cl) = pack2(ok[0], ok[1]);
+        *reinterpret_cast<uint32_t*>(sDQ + i * PC + n16 + n * 8 + cl) = pack2(oq[0], oq[1]);
+      }
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        rb += __shfl_xor_sync(0xffffffffu, rb, o);
+        rg += __shfl_xor_sync(0xffffffffu, rg, o);
+      }
+      if ((lane & 3) == 0) {
+        red[(warp >> 2) * CH + i] = rb;
+        red[(4 + (warp >> 2)) * CH + i] = rg;
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float s = col[n][e];
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane < 4) red[(8 + (warp & 3)) * CH + n16 + n * 8 + cl + e] = s;
+      }
+  }
+  __syncthreads();
+  if (tid < CH) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      dbeta += red[n * CH + tid];
+      dgc += red[(4 + n) * CH + tid] + red[(8 + n) * CH + tid];
+    }
+    red[12 * CH + tid] = dgc;
+    red[13 * CH + tid] = dlast;
+    if (t0 + tid < p.T) p.dbeta[tok0 + static_cast<long>(t0 + tid) * p.H] = dbeta;
+  }
+  // ---- dq = sq dqs + dqkr k;  dk = sk dks + dkk k + dkk^T k + dqkr^T q + Tw^T dw
+#pragma unroll
+  for (int kk = 0; kk < CH; kk += 16) {
+    uint32_t a1[4], a2[4], a3[4], a4[4], a5[4];
+    load_a(a1, sDQ, PC, m0, kk);
+    load_a(a2, sDK, PC, m0, kk);
+    load_a_t(a3, sDK, PC, m0, kk);
+    load_a_t(a4, sDQ, PC, m0, kk);
+    load_a_t(a5, sTw, PC, m0, kk);
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      uint32_t bb[4];
+      load_b_t(bb, sK, PK, n32 + n * 16, kk);
+      mma2(aQ[2 * n], aQ[2 * n + 1], a1, bb);
+      mma2(aK[2 * n], aK[2 * n + 1], a2, bb);
+      mma2(aK[2 * n], aK[2 * n + 1], a3, bb);
+      load_b_t(bb, sQ, PK, n32 + n * 16, kk);
+      mma2(aK[2 * n], aK[2 * n + 1], a4, bb);
+      load_b_t(bb, sW, PK, n32 + n * 16, kk);
+      mma2(aK[2 * n], aK[2 * n + 1], a5, bb);
+    }
+  }
+  __syncthreads();                                         // the tiles of q and k become those of dq and dk
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int o = (r0 + 8 * hh) * PK + n32 + n * 8 + cl;
+      *reinterpret_cast<uint32_t*>(sQ + o) = pack2(aQ[n][2 * hh], aQ[n][2 * hh + 1]);
+      *reinterpret_cast<uint32_t*>(sK + o) = pack2(aK[n][2 * hh], aK[n][2 * hh + 1]);
+    }
+  // ---- d g_t: sum of d gc_i over i >= t; the chunk's last gc also carries the decay of the state and of k
+  if (warp == 0) {
+    float l2 = red[13 * CH + 2 * lane] + red[13 * CH + 2 * lane + 1];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l2 += __shfl_xor_sync(0xffffffffu, l2, o);
+    float dgam = 0.f;
+    for (int s = 0; s < nvt; ++s) dgam += p.dgamma[(static_cast<long>(s) * gridDim.y + bh) * p.NC + c];
+    l2 += dgam * __expf(g_last);
+    const float a = red[12 * CH + 2 * lane], bq = red[12 * CH + 2 * lane + 1] + (lane == 31 ? l2 : 0.f);
+    float s = a + bq;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float n = __shfl_down_sync(0xffffffffu, s, o);
+      if (lane + o < 32) s += n;
+    }
+    const int ta = t0 + 2 * lane;
+    if (ta < p.T) p.dg[tok0 + static_cast<long>(ta) * p.H] = s;
+    if (ta + 1 < p.T) p.dg[tok0 + static_cast<long>(ta + 1) * p.H] = s - a;
+  }
+  __syncthreads();
+  for (int i = tid; i < CH * (KD / 8); i += 512) {
+    const int r = i / (KD / 8), cc = (i % (KD / 8)) * 8, t = t0 + r;
+    if (t >= p.T) continue;
+    const long off = (tok0 + static_cast<long>(t) * p.H) * KD + cc;
+    *reinterpret_cast<uint4*>(p.dq + off) = *reinterpret_cast<const uint4*>(sQ + r * PK + cc);
+    *reinterpret_cast<uint4*>(p.dk + off) = *reinterpret_cast<const uint4*>(sK + r * PK + cc);
+  }
+}
+}  // namespace
+
+// q, k [B, T, H, 128], v [B, T, H, V] bf16 contiguous, g (log-decay) and beta [B, T, H] fp32 -> w, u, qk, gc and, where
+// X is not null, the fp32 inverse the backward needs.  NC = ceil(T / 64).
+extern "C" int nsa_gdn_prep(const void* q, const void* k, const void* v, const float* g, const float* beta, void* w, void* u,
+                            void* qk, float* X, float* gc, int B, int T, int H, int K, int V, float scale, cudaStream_t st) {
+  if (K != KD || V % 64 || V > 512) return nsa::fail(NSA_ERR_SHAPE, "gdn: key width must be 128, value width a multiple of 64 up to 512");
+  const int NC = (T + CH - 1) / CH;
+  PrepParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, g, beta, (bf16*)w, (bf16*)u, (bf16*)qk, X, gc, T, H, NC, V, scale};
+  const int smem = 2 * CH * PK * 2 + CH * (V + 8) * 2 + 2 * CH * PX * 4 + 2 * CH * PC * 2 + 2 * CH * 4;
+  cudaError_t e = cudaFuncSetAttribute(gdn_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn prep smem attribute");
+  gdn_prep_kernel<<<dim3(NC, B * H), 256, smem, st>>>(p);
+  nsa::count_launch();
+  e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_prep launch");
+}
+
+// d_o [B, T, H, V] bf16; du, v_new [B*H, NC, 64, V]; S, dS [B*H, NC, 128, V]; dgamma [V / 64, B*H, NC] -> dq, dk, dv, dg, dbeta.
+extern "C" int nsa_gdn_post(const void* q, const void* k, const void* v, const void* d_o, const float* beta, const float* gc,
+                            const float* X, const void* v_new, const void* du, const void* S, const void* dS,
+                            const float* dgamma, void* dq, void* dk, void* dv, float* dg, float* dbeta, int B, int T, int H,
+                            int K, int V, float scale, cudaStream_t st) {
+  if (K != KD || V % 64) return nsa::fail(NSA_ERR_SHAPE, "gdn: key width must be 128 and value width a multiple of 64");
+  const int NC = (T + CH - 1) / CH;
+  PostParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, (const bf16*)d_o, beta, gc, X, (const bf16*)v_new, (const bf16*)du,
+               (const bf16*)S, (const bf16*)dS, dgamma, (bf16*)dq, (bf16*)dk, (bf16*)dv, dg, dbeta, B, T, H, NC, V, scale};
+  cudaError_t e = cudaFuncSetAttribute(gdn_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, POST_SMEM);
+  if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn post smem attribute");
+  gdn_post_kernel<<<dim3(NC, B * H), 512, POST_SMEM, st>>>(p);
+  nsa::count_launch();
+  e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_post launch");
+}

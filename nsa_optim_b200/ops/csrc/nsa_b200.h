@@ -45,11 +45,6 @@ int nsa_l2norm_bwd(const void* y, const void* dy, const float* rinv, void* dx, l
 int nsa_swiglu_fwd(const void* g, const void* u, void* y, long rows, int cols, long ldg, long ldu, cudaStream_t st);
 int nsa_swiglu_bwd(const void* g, const void* u, const void* dy, void* dg, void* du, long rows, int cols, long ldg,
                    long ldu, long ldo, cudaStream_t st);
-// bf16 rows between head-major (B, H, Th, D) and token-major (B, Tt, H, D); to_token 1: head -> token (t < Th copied),
-// 0: token -> head (rows t >= Tt zeroed).
-int nsa_permute_rows(const void* src, void* dst, int B, int H, int Th, int Tt, int D, int to_token, cudaStream_t st);
-// out[o][i] = sum over p of in[o][p][i]; bf16 in and out, fp32 sums in ascending p; n a multiple of 8.
-int nsa_sum_parts_bf16(const void* in, void* out, long outer, int parts, long n, cudaStream_t st);
 int nsa_rope(const void* x, const float* cos_t, const float* sin_t, void* y, long batch, int T, int H, int D,
              int backward, cudaStream_t st);
 int nsa_conv1d_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, long ldx, int width,
@@ -121,12 +116,17 @@ int nsa_gate_combine_bwd(const void* o1, const void* o2, const void* o3, const v
     g3, const void* d_o, void* do1, void* do2, void* do3, void* dg1, void* dg2, void* dg3, long rows, int D, cudaStream_t
     st);
 
-/* ---- Gated DeltaNet state recurrence (csrc/gdn.cu) ---- */
-int nsa_gdn_seq_fwd(const void* w, const void* qd, const void* kt, const void* u, const float* gamma, void* v_new,
-    void* o_inter, void* S_all, int BH, int NC, int K, int V, cudaStream_t st);   /* o_inter: bf16 */
-int nsa_gdn_seq_bwd(const void* w, const void* qd, const void* kt, const void* S_all, const void* v_new, const void*
-    dv_new, const void* d_o, const float* gamma, void* du, void* dw_part, void* dqd_part, void* dkt_part, float*
-    dgamma_part, int BH, int NC, int K, int V, cudaStream_t st);
+/* ---- Gated DeltaNet: per-chunk kernels (csrc/gdn_chunk.cu), state recurrence (csrc/gdn.cu) ---- */
+int nsa_gdn_prep(const void* q, const void* k, const void* v, const float* g, const float* beta, void* w, void* u,
+    void* qk, float* X, float* gc, int B, int T, int H, int K, int V, float scale, cudaStream_t st);
+int nsa_gdn_seq_fwd(const void* q, const void* k, const void* w, const void* u, const void* qk, const float* gc, void*
+    o, void* v_new, void* S_all, int B, int T, int H, int K, int V, float scale, cudaStream_t st);
+int nsa_gdn_seq_bwd(const void* q, const void* k, const void* w, const void* qk, const void* S_all, const void* d_o,
+    const float* gc, void* du, void* dS_all, float* dgamma_part, int B, int T, int H, int K, int V, float scale,
+    cudaStream_t st);
+int nsa_gdn_post(const void* q, const void* k, const void* v, const void* d_o, const float* beta, const float* gc,
+    const float* X, const void* v_new, const void* du, const void* S, const void* dS, const float* dgamma, void* dq,
+    void* dk, void* dv, float* dg, float* dbeta, int B, int T, int H, int K, int V, float scale, cudaStream_t st);
 
 /* ---- GEMM (csrc/gemm.cu) ---- */
 int nsa_gemm_bf16_ag(const void* A, void* C, int M, int N, int K, int lda, int ldc, const void* const* shards, void*
@@ -155,20 +155,6 @@ int nsa_ssd_chunk_grad(const void* Cm, long ld_c, const void* Bm, long ld_b, con
 /* ---- further entry points of attention.cu ---- */
 int nsa_select_blocks(const float* imp, int* idx, long rows, int T, int nS, int sel_block, int top_n, cudaStream_t
     st);
-
-/* ---- further entry points of elementwise.cu ---- */
-int nsa_gdn_pack_fwd(const void* q, const void* k, const void* v, const float* sq, const float* sk, void* qh, void*
-    kh, void* vh, void* qd, void* kt, int B, int T, int Tp, int H, int K, int V, cudaStream_t st);
-int nsa_gdn_pack_bwd(const void* q, const void* k, const float* sq, const float* sk, const void* dqh, const void*
-    dkh, const void* dvh, const void* dqd, const void* dkt, void* dq, void* dk, void* dv, float* dsq, float* dsk, int B,
-    int T, int Tp, int H, int K, int V, cudaStream_t st);
-int nsa_gdn_tmat_fwd(const void* kk, const void* qkr, const float* gc, const float* beta, void* Tu, void* Tw, void*
-    qk, float* X, long n_chunks, float scale, cudaStream_t st);
-int nsa_gdn_tmat_dx(const void* dTu, const void* dTw, const float* gc, const float* beta, float* dX, long n_chunks,
-    cudaStream_t st);
-int nsa_gdn_tmat_bwd(const float* dA, const void* kk, const void* qkr, const void* dqk, const void* dTu, const void*
-    dTw, const float* X, const float* gc, const float* beta, void* dkk, void* dqkr, float* dgc, float* dbeta, long
-    n_chunks, float scale, cudaStream_t st);
 
 /* ---- further entry points of optim.cu ---- */
 int nsa_affine_quant(const float* t, uint8_t* q, float* scale, float* zero, long rows, int cols, int q_block, int

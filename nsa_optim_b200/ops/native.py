@@ -885,176 +885,73 @@ def adamw8bit_step(p, g, mq, mabs, vq, vabs, step, lr, b1, b2, eps, wd, grad_sca
 # --------------------------------------------------------------------------------------
 # gated delta rule (chunk 64, key width 128)
 # --------------------------------------------------------------------------------------
-class _GDNSeq(torch.autograd.Function):
-    """Inter-chunk state recurrence of the gated delta rule on tcgen05 (``csrc/gdn.cu``).
-    Inputs are the per-chunk operands of the WY form, (BH, NC, 64, .) contiguous bf16."""
+class _GatedDelta(torch.autograd.Function):
+    """Chunkwise gated delta rule, two kernels each way: per-chunk matrices and operands
+    (``gdn_prep_kernel``), the state recurrence with the output (``csrc/gdn.cu``); backward the reverse recurrence,
+    then every gradient of a chunk (``gdn_post_kernel``).  All tensors token-major, gates fp32."""
 
     @staticmethod
-    def forward(ctx, w, qd, kt, u, gamma):
-        BH, NC, C, K = w.shape
-        V = u.shape[-1]
-        v_new = _empty_like(u)
-        o_inter = _empty(BH, NC, C, V, dtype=torch.bfloat16, device=u.device)
-        S_all = _empty(BH, NC, K, V, dtype=torch.bfloat16, device=u.device)
-        _check(load().nsa_gdn_seq_fwd(_p(w), _p(qd), _p(kt), _p(u), _p(gamma), _p(v_new), _p(o_inter), _p(S_all),
-                                      c_int(BH), c_int(NC), c_int(K), c_int(V), _stream()))
-        ctx.save_for_backward(w, qd, kt, gamma, S_all, v_new)
-        # o_inter leaves the kernel as bf16 (it is added to a bf16 matmul result next), so its gradient
-        # also arrives as bf16 instead of making an fp32 round trip
-        return v_new, o_inter
-
-    @staticmethod
-    def backward(ctx, dv_new, do_inter):
-        w, qd, kt, gamma, S_all, v_new = ctx.saved_tensors
-        BH, NC, C, K = w.shape
-        V = v_new.shape[-1]
-        nvt = V // 64
-        dv = _zeros_like(v_new) if dv_new is None else dv_new.to(torch.bfloat16).contiguous()
-        do = _zeros_like(v_new) if do_inter is None else do_inter.to(torch.bfloat16).contiguous()
-        du = _empty_like(v_new)
-        parts = _empty(3, nvt, BH, NC, C, K, dtype=torch.bfloat16, device=w.device)
-        dgp = _empty(nvt, BH, NC, dtype=torch.float32, device=w.device)
-        _check(load().nsa_gdn_seq_bwd(_p(w), _p(qd), _p(kt), _p(S_all), _p(v_new), _p(dv), _p(do), _p(gamma), _p(du),
-                                      _p(parts[0]), _p(parts[1]), _p(parts[2]), _p(dgp), c_int(BH), c_int(NC),
-                                      c_int(K), c_int(V), _stream()))
-        red = _empty(3, BH, NC, C, K, dtype=torch.bfloat16, device=w.device)
-        _check(load().nsa_sum_parts_bf16(_p(parts), _p(red), c_long(3), c_int(nvt), c_long(BH * NC * C * K), _stream()))
-        return red[0], red[1], red[2], du, dgp.sum(0)
-
-
-class _GDNPack(torch.autograd.Function):
-    """Token-major q, k, v -> head-major chunk rows (B*H, Tp, .): copies qh, kh, vh and the
-    decay-scaled operands qd = q * sq, kt = k * sk in one pass each way (``csrc/elementwise.cu``)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, sq, sk):
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        sq, sk = sq.float().contiguous(), sk.float().contiguous()
+    def forward(ctx, q, k, v, g, beta, scale):
         B, T, H, K = q.shape
         V = v.shape[-1]
-        Tp = sq.shape[-1]
-        mk = lambda w: _empty(B * H, Tp, w, dtype=torch.bfloat16, device=q.device)
-        qh, kh, vh, qd, kt = mk(K), mk(K), mk(V), mk(K), mk(K)
-        _check(load().nsa_gdn_pack_fwd(_p(q), _p(k), _p(v), _p(sq), _p(sk), _p(qh), _p(kh), _p(vh), _p(qd), _p(kt),
-                                       c_int(B), c_int(T), c_int(Tp), c_int(H), c_int(K), c_int(V), _stream()))
-        ctx.save_for_backward(q, k, sq, sk)
-        ctx.V = V
-        return qh, kh, vh, qd, kt
+        BH, nc = B * H, -(-T // 64)
+        dev, bf, f32 = q.device, torch.bfloat16, torch.float32
+        train = any(ctx.needs_input_grad)
+        w, u = _empty(BH, nc, 64, K, dtype=bf, device=dev), _empty(BH, nc, 64, V, dtype=bf, device=dev)
+        qk, gc = _empty(BH, nc, 64, 64, dtype=bf, device=dev), _empty(BH, nc, 64, dtype=f32, device=dev)
+        X = _empty(BH, nc, 64, 64, dtype=f32, device=dev) if train else None
+        o = _empty(B, T, H, V, dtype=bf, device=dev)
+        v_new = _empty(BH, nc, 64, V, dtype=bf, device=dev) if train else None
+        S = _empty(BH, nc, K, V, dtype=bf, device=dev) if train else None
+        lib, st = load(), _stream()
+        dims = (c_int(B), c_int(T), c_int(H), c_int(K), c_int(V), c_float(scale), st)
+        _check(lib.nsa_gdn_prep(_p(q), _p(k), _p(v), _p(g), _p(beta), _p(w), _p(u), _p(qk), _p(X), _p(gc), *dims))
+        _check(lib.nsa_gdn_seq_fwd(_p(q), _p(k), _p(w), _p(u), _p(qk), _p(gc), _p(o), _p(v_new), _p(S), *dims))
+        if train:
+            ctx.save_for_backward(q, k, v, beta, w, qk, gc, X, v_new, S)
+            ctx.scale = scale
+        return o
 
     @staticmethod
-    def backward(ctx, dqh, dkh, dvh, dqd, dkt):
-        q, k, sq, sk = ctx.saved_tensors
+    def backward(ctx, do):
+        q, k, v, beta, w, qk, gc, X, v_new, S = ctx.saved_tensors
         B, T, H, K = q.shape
-        V, Tp = ctx.V, sq.shape[-1]
-        c = lambda t: None if t is None else t.to(torch.bfloat16).contiguous()
-        dqh, dkh, dvh, dqd, dkt = c(dqh), c(dkh), c(dvh), c(dqd), c(dkt)
-        dq, dk = _empty_like(q), _empty_like(k)
-        dv = _empty(B, T, H, V, dtype=torch.bfloat16, device=q.device)
-        dsq, dsk = _empty_like(sq), _empty_like(sk)
-        _check(load().nsa_gdn_pack_bwd(_p(q), _p(k), _p(sq), _p(sk), _p(dqh), _p(dkh), _p(dvh), _p(dqd), _p(dkt), _p(dq), _p(dk),
-                                       _p(dv), _p(dsq), _p(dsk), c_int(B), c_int(T), c_int(Tp), c_int(H), c_int(K), c_int(V),
-                                       _stream()))
-        return dq, dk, dv, dsq, dsk
+        V = v.shape[-1]
+        BH, nc = B * H, gc.shape[1]
+        dev = q.device
+        do = do.to(torch.bfloat16).contiguous()
+        du, dS = _empty_like(v_new), _empty_like(S)
+        dgamma = _empty(V // 64, BH, nc, dtype=torch.float32, device=dev)
+        dq, dk, dv = _empty_like(q), _empty_like(k), _empty_like(v)
+        dg, dbeta = _empty_like(beta), _empty_like(beta)
+        lib, st = load(), _stream()
+        dims = (c_int(B), c_int(T), c_int(H), c_int(K), c_int(V), c_float(ctx.scale), st)
+        _check(lib.nsa_gdn_seq_bwd(_p(q), _p(k), _p(w), _p(qk), _p(S), _p(do), _p(gc), _p(du), _p(dS), _p(dgamma), *dims))
+        _check(lib.nsa_gdn_post(_p(q), _p(k), _p(v), _p(do), _p(beta), _p(gc), _p(X), _p(v_new), _p(du), _p(S), _p(dS), _p(dgamma),
+                                _p(dq), _p(dk), _p(dv), _p(dg), _p(dbeta), *dims))
+        return dq, dk, dv, dg, dbeta, None
 
 
-class _GDNTmat(torch.autograd.Function):
-    """Per-chunk 64 x 64 matrices of the gated delta rule (``gdn_tmat_*`` in ``csrc/elementwise.cu``):
-    from kk = K K^T, qkr = Q K^T (bf16), the cumulative gate gc and beta build
-    Tu = X diag(beta), Tw = X diag(beta e^gc) with X = (I + A)^-1 and the decayed, scaled, causal qk.
-    The backward needs dA = -(X^T dX X^T): two batched fp32 matmuls between two small kernels."""
-
-    @staticmethod
-    def forward(ctx, kk, qkr, gc, bh, scale):
-        kk, qkr = kk.contiguous(), qkr.contiguous()
-        gc, bh = gc.float().contiguous(), bh.float().contiguous()
-        n = gc.numel() // 64
-        Tu, Tw, qk = _empty_like(kk), _empty_like(kk), _empty_like(kk)
-        X = _empty(kk.shape, dtype=torch.float32, device=kk.device)
-        _check(load().nsa_gdn_tmat_fwd(_p(kk), _p(qkr), _p(gc), _p(bh), _p(Tu), _p(Tw), _p(qk), _p(X), c_long(n), c_float(scale),
-                                       _stream()))
-        ctx.save_for_backward(kk, qkr, gc, bh, X)
-        ctx.scale = scale
-        return Tu, Tw, qk
-
-    @staticmethod
-    def backward(ctx, dTu, dTw, dqk):
-        kk, qkr, gc, bh, X = ctx.saved_tensors
-        n = gc.numel() // 64
-        z = lambda t: _zeros_like(kk) if t is None else t.to(torch.bfloat16).contiguous()
-        dTu, dTw, dqk = z(dTu), z(dTw), z(dqk)
-        dX = _empty_like(X)
-        lib = load()
-        _check(lib.nsa_gdn_tmat_dx(_p(dTu), _p(dTw), _p(gc), _p(bh), _p(dX), c_long(n), _stream()))
-        Xt = X.transpose(-1, -2)
-        dA = -torch.matmul(torch.matmul(Xt, dX), Xt)
-        del dX
-        dkk, dqkr = _empty_like(kk), _empty_like(kk)
-        dgc, dbh = _empty_like(gc), _empty_like(bh)
-        _check(lib.nsa_gdn_tmat_bwd(_p(dA.contiguous()), _p(kk), _p(qkr), _p(dqk), _p(dTu), _p(dTw), _p(X), _p(gc), _p(bh), _p(dkk),
-                                    _p(dqkr), _p(dgc), _p(dbh), c_long(n), c_float(ctx.scale), _stream()))
-        return dkk, dqkr, dgc, dbh, None
-
-
-class _HeadToToken(torch.autograd.Function):
-    """(B*H, Tp, D) head-major rows -> (B, T, H, D) token-major (T <= Tp), one coalesced copy each way
-    (``permute_rows_kernel``) instead of a generic strided copy."""
-
-    @staticmethod
-    def forward(ctx, x, B, H, T):
-        Tp, D = x.shape[-2], x.shape[-1]
-        ctx.dims = (B, H, Tp, T, D)
-        x = x.contiguous()
-        y = _empty(B, T, H, D, dtype=x.dtype, device=x.device)
-        _check(load().nsa_permute_rows(_p(x), _p(y), c_int(B), c_int(H), c_int(Tp), c_int(T), c_int(D), c_int(1), _stream()))
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        B, H, Tp, T, D = ctx.dims
-        dy = dy.to(torch.bfloat16).contiguous()
-        dx = _empty(B * H, Tp, D, dtype=dy.dtype, device=dy.device)
-        _check(load().nsa_permute_rows(_p(dy), _p(dx), c_int(B), c_int(H), c_int(Tp), c_int(T), c_int(D), c_int(0), _stream()))
-        return dx, None, None, None
+def _dense16(t: Tensor) -> Tensor:
+    """Contiguous with a 16-byte aligned start, as the copy engine and 16-byte loads need."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
 
 
 def gated_delta_rule(q, k, v, g, beta, scale=None, chunk=64):
-    """Chunkwise gated delta rule.  One layout pass brings q, k, v to head-major chunk rows together
-    with the decay-scaled operands; K K^T, Q K^T and the applications of the per-chunk matrices are
-    batched bf16 matmuls; the 64 x 64 matrices themselves (decay masks, the unit-triangular inverse
-    by substitution, their gradients) come from one small kernel each way; the sequential state
-    pass is the tcgen05 kernel of ``csrc/gdn.cu``."""
+    """Chunkwise gated delta rule (:class:`_GatedDelta`).  Value columns are independent of one another given
+    q, k and the gates, so values wider than one launch's shared memory go in slices."""
     B, T, H, K = q.shape
     V = v.shape[-1]
     if K != 128 or V % 64 or chunk != 64 or q.dtype != torch.bfloat16:
         _fallback("gated_delta_rule")
         return torch_impl.gated_delta_rule(q, k, v, g, beta, scale, chunk)
     scale = K ** -0.5 if scale is None else scale
-    C = 64
-    pad = (-T) % C
-    Tp = T + pad
-    nc = Tp // C
-    f32, bf = torch.float32, torch.bfloat16
-    gh = g.to(f32).permute(0, 2, 1)
-    bh = beta.to(f32).permute(0, 2, 1)
-    if pad:
-        gh, bh = torch.nn.functional.pad(gh, (0, pad)), torch.nn.functional.pad(bh, (0, pad))
-    gh, bh = gh.reshape(B * H, nc, C), bh.reshape(B * H, nc, C)
-    gc = torch.cumsum(gh, -1)
-    eg = torch.exp(gc)
-    sq = (scale * eg).reshape(B * H, Tp)
-    sk = torch.exp(gc[..., -1:] - gc).reshape(B * H, Tp)
-    qh, kh, vh, qd, kt = (t.view(B * H, nc, C, -1) for t in _GDNPack.apply(q, k, v.to(bf), sq, sk))
-    kT = kh.transpose(-1, -2)
-    Tu, Tw, qk = _GDNTmat.apply(torch.matmul(kh, kT), torch.matmul(qh, kT), gc, bh, float(scale))
-    u = torch.matmul(Tu, vh)
-    w = torch.matmul(Tw, kh)
-    gamma = eg[..., -1].contiguous()
-    v_new, o_inter = _GDNSeq.apply(w, qd, kt, u, gamma)
-    # o = o_inter + qk v_new in one batched GEMM with fp32 accumulation
-    o = torch.baddbmm(o_inter.view(-1, C, V), qk.view(-1, C, C), v_new.view(-1, C, V))
-    if o.dtype == torch.bfloat16 and V % 8 == 0:
-        return _HeadToToken.apply(o.view(B * H, Tp, V), B, H, T).to(v.dtype)
-    o = o.view(B, H, Tp, V).permute(0, 2, 1, 3)[:, :T]
+    bf = torch.bfloat16
+    args = [_dense16(q), _dense16(k.to(bf)), v.to(bf), g.float().contiguous(), beta.float().contiguous()]
+    outs = [_GatedDelta.apply(args[0], args[1], _dense16(part), args[3], args[4], float(scale))
+            for part in (args[2].split(512, -1) if V > 512 else (args[2],))]
+    o = outs[0] if len(outs) == 1 else torch.cat(outs, -1)
     return o.to(v.dtype)
 
 
