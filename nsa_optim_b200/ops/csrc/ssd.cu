@@ -46,6 +46,44 @@ __device__ __forceinline__ void ld_row64(const uint8_t* kblock, int row, float (
     }
   }
 }
+// 32 columns col0.. of a tile of [128][64] boxes; the row's 16-byte pieces are swizzled as above
+__device__ __forceinline__ void st_row32(uint8_t* tile, int row, int col0, const uint32_t (&pk)[16]) {
+  uint8_t* base = tile + (col0 >> 6) * BOXB + row * 128;
+  const int j0 = (col0 & 63) >> 3;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    *reinterpret_cast<uint4*>(base + (((j0 + j) ^ (row & 7)) << 4)) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+}
+template <int N>
+__device__ __forceinline__ void ld_row(const uint8_t* tile, int row, int col0, float (&out)[N]) {
+  const uint8_t* base = tile + (col0 >> 6) * BOXB + row * 128;
+  const int j0 = (col0 & 63) >> 3;
+#pragma unroll
+  for (int j = 0; j < N / 8; ++j) {
+    const uint4 v = *reinterpret_cast<const uint4*>(base + (((j0 + j) ^ (row & 7)) << 4));
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 f = __bfloat1622float2(h[k]);
+      out[8 * j + 2 * k] = f.x;
+      out[8 * j + 2 * k + 1] = f.y;
+    }
+  }
+}
+__device__ __forceinline__ void tld32(uint32_t taddr, float (&out)[32]) {
+  uint32_t a[32];
+  tc5::tmem_ld_x32(taddr, a);
+  tc5::tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < 32; ++j) out[j] = __uint_as_float(a[j]);
+}
+__device__ __forceinline__ void tld16(uint32_t taddr, float (&out)[16]) {
+  uint32_t a[16];
+  tc5::tmem_ld_x16(taddr, a);
+  tc5::tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < 16; ++j) out[j] = __uint_as_float(a[j]);
+}
 __device__ __forceinline__ void tld64(uint32_t taddr, float (&out)[64]) {
   uint32_t a[32], b[32];
   tc5::tmem_ld_x32(taddr, a);
@@ -55,23 +93,25 @@ __device__ __forceinline__ void tld64(uint32_t taddr, float (&out)[64]) {
   for (int j = 0; j < 32; ++j) { out[j] = __uint_as_float(a[j]); out[32 + j] = __uint_as_float(b[j]); }
 }
 
-// Inclusive scan of `a` over the 128 threads of the CTA; cum[] and dts[] (shared, 128 floats
-// each) receive every row's value.  Returns this thread's inclusive sum.
+// Inclusive scan of `a` over the 128 rows of the chunk, by every group of 128 threads of the CTA (with the same
+// result); cum[] and dts[] (shared, 128 floats each) receive every row's value.  Returns this row's inclusive sum.
 __device__ __forceinline__ float chunk_scan(float a, float dt, float* cum, float* dts, float* warp_tot) {
-  const int r = threadIdx.x, lane = r & 31, w = r >> 5;
+  const int r = threadIdx.x & 127, lane = r & 31, w = r >> 5;
   float v = a;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const float n = __shfl_up_sync(0xffffffffu, v, o);
     if (lane >= o) v += n;
   }
-  if (lane == 31) warp_tot[w] = v;
+  if (lane == 31 && threadIdx.x < 128) warp_tot[w] = v;
   __syncthreads();
   float off = 0.f;
   for (int k = 0; k < w; ++k) off += warp_tot[k];
   v += off;
-  cum[r] = v;
-  dts[r] = dt;
+  if (threadIdx.x < 128) {
+    cum[r] = v;
+    dts[r] = dt;
+  }
   __syncthreads();
   return v;
 }
@@ -125,7 +165,7 @@ ssd_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_c
   float* warp_tot = dts + L;
 
   const int r = threadIdx.x, warp = r >> 5;
-  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int h = blockIdx.x, c = blockIdx.y, b = blockIdx.z;    // heads fastest: see the launches
   const int t0 = c * L;
   if (r == 0) {
     *abort_flag = 0;
@@ -183,9 +223,18 @@ ssd_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_c
     tc5::fence_after_sync();
     float o[64];
     tld64(tmem + (static_cast<uint32_t>(warp * 32) << 16), o);
-    float4* dst = reinterpret_cast<float4*>(p.S_out + (((static_cast<long>(b) * p.nc + c) * p.H + h) * NS + r) * PD);
+    // The tile is contiguous in memory but a thread owns a row of it, and direct stores would put 16 bytes into
+    // 32 rows per instruction: it is turned through the operand tile (free now), pieces swizzled by row.
+    float4* stage = reinterpret_cast<float4*>(sBC);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) dst[j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+    for (int j = 0; j < 16; ++j) stage[r * 16 + (j ^ (r & 15))] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+    __syncthreads();
+    float4* dst = reinterpret_cast<float4*>(p.S_out + ((static_cast<long>(b) * p.nc + c) * p.H + h) * NS * PD);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int i = j * 128 + r;
+      dst[i] = stage[(i & ~15) + ((i ^ (i >> 4)) & 15)];
+    }
     if (MODE == 0 && r == 0 && p.gamma_out) p.gamma_out[(static_cast<long>(b) * p.nc + c) * p.H + h] = exp2f(tot * LOG2E);
   }
   tc5::fence_before_sync();
@@ -196,7 +245,7 @@ ssd_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_c
 // ---------------------------------------------------------------------------------------
 // chunk_out: y = P x + exp(cum) (C H) + D x  for one (chunk, head, batch).
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(256, 2)
 ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_b,
                      const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_h,
                      const __grid_constant__ CUtensorMap tm_y, const SsdParams p) {
@@ -206,8 +255,8 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   uint8_t* sB = sC + 2 * BOXB;
   uint8_t* sX = sB + 2 * BOXB;         // [128 t][64]
   uint8_t* sH = sX + BOXB;             // [128 n][64]
-  uint8_t* sP = sH + BOXB;             // [2 k-blocks][128][64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + 2 * BOXB);
+  uint8_t* sP = sB;                    // [2 k-blocks][128][64], over B once C B^T is complete
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sH + BOXB);
   uint64_t* full = bars;
   uint64_t* m1 = bars + 1;
   uint64_t* m2 = bars + 2;
@@ -217,10 +266,10 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   float* dts = cum + L;
   float* warp_tot = dts + L;
 
-  const int r = threadIdx.x, warp = r >> 5;
-  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int r = threadIdx.x & 127, half = threadIdx.x >> 7, warp = threadIdx.x >> 5;   // row, column half
+  const int h = blockIdx.x, c = blockIdx.y, b = blockIdx.z;    // heads fastest: see the launches
   const int t0 = c * L;
-  if (r == 0) {
+  if (threadIdx.x == 0) {
     *abort_flag = 0;
     tc5::mbar_init(full, 1);
     tc5::mbar_init(m1, 1);
@@ -243,7 +292,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_off = static_cast<uint32_t>(warp * 32) << 16;
+  const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
   const uint32_t cS = 0, cYi = 128, cYo = 192;
   constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);
   constexpr uint32_t id_y = tc5::make_idesc_bf16(128, PD, 0, 1);
@@ -275,8 +324,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   if (ok) {
     tc5::fence_after_sync();
     const float ci = cm * LOG2E;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    {
       float s[64];
       tld64(tmem + lane_off + cS + half * 64, s);
       uint32_t pk[32];
@@ -315,23 +363,23 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
     tc5::fence_after_sync();
     // y leaves through shared memory and one TMA store (a thread owns a token row, so direct stores
     // would write 16 bytes per thread into 32 different rows per instruction); x comes from its tile
-    float yo[64], yi[64];
-    tld64(tmem + lane_off + cYo, yo);
-    tld64(tmem + lane_off + cYi, yi);
+    float yo[32], yi[32];
+    tld32(tmem + lane_off + cYo + half * 32, yo);
+    tld32(tmem + lane_off + cYi + half * 32, yi);
     const float e = exp2f(cm * LOG2E);
     const float dsk = p.Dskip ? p.Dskip[h] : 0.f;
-    uint32_t o[32];
+    uint32_t o[16];
     {
-      float xf[64];
-      ld_row64(sX, r, xf);
+      float xf[32];
+      ld_row(sX, r, half * 32, xf);
 #pragma unroll
-      for (int i = 0; i < 64; i += 2)
+      for (int i = 0; i < 32; i += 2)
         o[i / 2] = tc5::pack_bf16(yo[i] + e * yi[i] + dsk * xf[i], yo[i + 1] + e * yi[i + 1] + dsk * xf[i + 1]);
     }
-    st_row64(sP, r, o);                 // the P tile is free once the second MMA is complete
+    st_row32(sP, r, half * 32, o);      // the P tile is free once the second MMA is complete
     tc5::fence_proxy_async();
     __syncthreads();
-    if (r == 0) {                       // rows past T are clipped by the copy engine
+    if (threadIdx.x == 0) {             // rows past T are clipped by the copy engine
       tc5::tma_store_4d(&tm_y, sP, 0, h, t0, b);
       tc5::tma_store_commit();
       tc5::tma_store_wait_read<0>();
@@ -351,7 +399,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
 //   dB_j  = sum_i dS_ij C_i + s_j x_j dHn^T
 // dB / dC are summed over heads with fp32 vector reductions.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(512, 1)
 ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_b,
                       const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_dy,
                       const __grid_constant__ CUtensorMap tm_h, const __grid_constant__ CUtensorMap tm_dh,
@@ -376,12 +424,13 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* cum = reinterpret_cast<float*>(bars + 4);
   float* dts = cum + L;
-  float* warp_tot = dts + L;
+  float* warp_tot = dts + L;           // [4], padded to 8
+  float* part = warp_tot + 8;          // [4 groups][128] row sums on their way to one
 
-  const int r = threadIdx.x, warp = r >> 5;
-  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int r = threadIdx.x & 127, grp = threadIdx.x >> 7, warp = threadIdx.x >> 5;    // row, column group
+  const int h = blockIdx.x, c = blockIdx.y, b = blockIdx.z;    // heads fastest: see the launches
   const int t0 = c * L;
-  if (r == 0) {
+  if (threadIdx.x == 0) {
     *abort_flag = 0;
     tc5::mbar_init(full, 1);
     tc5::mbar_init(m1, 1);
@@ -409,7 +458,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_off = static_cast<uint32_t>(warp * 32) << 16;
+  const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
   // TMEM columns: S / dC [0,128)  R / dB [128,256)  dX [256,320)  dXi [320,384)  dCi [384,512)
   const uint32_t cS = 0, cR = 128, cDX = 256, cDXI = 320, cDCI = 384;
   constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);     // K-major x K-major -> [128 x 128]
@@ -450,12 +499,14 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
   // x rows scaled by s_j (operand of the state-path part of dB) while the MMAs run
   bool landed = tc5::mbar_wait(full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL);
   if (landed) {
-    float xv[64];
-    ld_row64(sX, r, xv);
-    uint32_t pk[32];
+    if (grp < 2) {
+      float xv[32];
+      ld_row(sX, r, grp * 32, xv);
+      uint32_t pk[16];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) pk[j] = tc5::pack_bf16(xv[2 * j] * s_row, xv[2 * j + 1] * s_row);
-    st_row64(sXS, r, pk);
+      for (int j = 0; j < 16; ++j) pk[j] = tc5::pack_bf16(xv[2 * j] * s_row, xv[2 * j + 1] * s_row);
+      st_row32(sXS, r, grp * 32, pk);
+    }
   } else ok = false;
   if (!tc5::mbar_wait(m1, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
   if (__syncthreads_or(!ok)) ok = false;
@@ -463,28 +514,25 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
   if (ok) {
     tc5::fence_after_sync();
     const float ci = cm * LOG2E;
+    float s[32], rr[32];
+    tld32(tmem + lane_off + cS + grp * 32, s);
+    tld32(tmem + lane_off + cR + grp * 32, rr);
+    uint32_t pp[16], ds[16];
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      float s[64], rr[64];
-      tld64(tmem + lane_off + cS + half * 64, s);
-      tld64(tmem + lane_off + cR + half * 64, rr);
-      uint32_t pp[32], ds[32];
-#pragma unroll
-      for (int j = 0; j < 64; j += 2) {
-        // operands fetched and the weight computed for every j, then selected (no branch per element)
-        const int j0 = half * 64 + j;
-        const float2 cj = *reinterpret_cast<const float2*>(cum + j0), dj = *reinterpret_cast<const float2*>(dts + j0);
-        const float e0 = exp2f(fminf(ci - cj.x * LOG2E, 0.f)) * dj.x, e1 = exp2f(fminf(ci - cj.y * LOG2E, 0.f)) * dj.y;
-        const float w0 = j0 <= r ? e0 : 0.f;
-        const float w1 = j0 + 1 <= r ? e1 : 0.f;
-        pp[j / 2] = tc5::pack_bf16(s[j] * w0, s[j + 1] * w1);
-        ds[j / 2] = tc5::pack_bf16(rr[j] * w0, rr[j + 1] * w1);
-        const float2 pr = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pp[j / 2]));
-        q_intra += pr.x * rr[j] + pr.y * rr[j + 1];
-      }
-      st_row64(sP + half * BOXB, r, pp);
-      st_row64(sDS + half * BOXB, r, ds);
+    for (int j = 0; j < 32; j += 2) {
+      // operands fetched and the weight computed for every j, then selected (no branch per element)
+      const int j0 = grp * 32 + j;
+      const float2 cj = *reinterpret_cast<const float2*>(cum + j0), dj = *reinterpret_cast<const float2*>(dts + j0);
+      const float e0 = exp2f(fminf(ci - cj.x * LOG2E, 0.f)) * dj.x, e1 = exp2f(fminf(ci - cj.y * LOG2E, 0.f)) * dj.y;
+      const float w0 = j0 <= r ? e0 : 0.f;
+      const float w1 = j0 + 1 <= r ? e1 : 0.f;
+      pp[j / 2] = tc5::pack_bf16(s[j] * w0, s[j + 1] * w1);
+      ds[j / 2] = tc5::pack_bf16(rr[j] * w0, rr[j + 1] * w1);
+      const float2 pr = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pp[j / 2]));
+      q_intra += pr.x * rr[j] + pr.y * rr[j + 1];
     }
+    st_row32(sP, r, grp * 32, pp);
+    st_row32(sDS, r, grp * 32, ds);
   }
   tc5::fence_proxy_async();
   tc5::fence_before_sync();
@@ -524,67 +572,67 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
     const long tok = static_cast<long>(b) * p.T + t;
     const float e = exp2f(cm * LOG2E);
     const bool heads = p.dB_heads != nullptr;
+    const int col = grp * 32;           // this thread's columns of dB and dC; half as many of dx
+    float kacc = 0.f, racc = 0.f, q_inter = 0.f;
     {
-      float dxa[64], dxi[64];
-      tld64(tmem + lane_off + cDX, dxa);
-      tld64(tmem + lane_off + cDXI, dxi);
+      float dxa[16], dxi[16], xf[16], df[16];
+      tld16(tmem + lane_off + cDX + grp * 16, dxa);
+      tld16(tmem + lane_off + cDXI + grp * 16, dxi);
       const float dsk = p.Dskip ? p.Dskip[h] : 0.f;
-      float kacc = 0.f, racc = 0.f;
-      uint32_t o[32];
-      {
-        float xf[64], df[64];
-        ld_row64(sX, r, xf);
-        ld_row64(sDY, r, df);
+      ld_row(sX, r, grp * 16, xf);
+      ld_row(sDY, r, grp * 16, df);
+      uint32_t o[8];
 #pragma unroll
-        for (int i = 0; i < 64; i += 2) {
-          const float g0 = dxa[i] + s_row * dxi[i], g1 = dxa[i + 1] + s_row * dxi[i + 1];
-          kacc += xf[i] * g0 + xf[i + 1] * g1;
-          racc += xf[i] * df[i] + xf[i + 1] * df[i + 1];
-          o[i / 2] = tc5::pack_bf16(g0 + dsk * df[i], g1 + dsk * df[i + 1]);
-        }
+      for (int i = 0; i < 16; i += 2) {
+        const float g0 = dxa[i] + s_row * dxi[i], g1 = dxa[i + 1] + s_row * dxi[i + 1];
+        kacc += xf[i] * g0 + xf[i + 1] * g1;
+        racc += xf[i] * df[i] + xf[i + 1] * df[i + 1];
+        o[i / 2] = tc5::pack_bf16(g0 + dsk * df[i], g1 + dsk * df[i + 1]);
       }
-      st_row64(sXS, r, o);
-      if (row_ok) {
-        p.k_out[tok * p.H + h] = kacc;
-        if (p.r_out) p.r_out[tok * p.H + h] = racc;
-      }
+      uint8_t* base = sXS + r * 128;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        *reinterpret_cast<uint4*>(base + (((grp * 2 + j) ^ (r & 7)) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
     }
-    float q_inter = 0.f;    // C_i . (dy_i H^T): the state-path part of dy.(y - D x), before exp(cum_i)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      float dc[64], dci[64], db[64];
-      tld64(tmem + lane_off + cS + half * 64, dc);
-      tld64(tmem + lane_off + cDCI + half * 64, dci);
-      tld64(tmem + lane_off + cR + half * 64, db);
+    {                       // q_inter = C_i . (dy_i H^T): the state-path part of dy.(y - D x), before exp(cum_i)
+      float dc[32], dci[32], db[32];
+      tld32(tmem + lane_off + cS + col, dc);
+      tld32(tmem + lane_off + cDCI + col, dci);
+      tld32(tmem + lane_off + cR + col, db);
       {
-        float cv[64];
-        ld_row64(sC + half * BOXB, r, cv);
+        float cv[32];
+        ld_row(sC, r, col, cv);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) q_inter += cv[j] * dci[j];
+        for (int j = 0; j < 32; ++j) q_inter += cv[j] * dci[j];
       }
       if (heads) {
-        uint32_t vc[32], vb[32];
+        uint32_t vc[16], vb[16];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < 16; ++j) {
           vc[j] = tc5::pack_bf16(dc[2 * j] + e * dci[2 * j], dc[2 * j + 1] + e * dci[2 * j + 1]);
           vb[j] = tc5::pack_bf16(db[2 * j], db[2 * j + 1]);
         }
-        st_row64(sP + half * BOXB, r, vc);
-        st_row64(sDS + half * BOXB, r, vb);
+        st_row32(sP, r, col, vc);
+        st_row32(sDS, r, col, vb);
       } else if (row_ok) {
-        float4* pc = reinterpret_cast<float4*>(p.dC_acc + tok * NS + half * 64);
-        float4* pb = reinterpret_cast<float4*>(p.dB_acc + tok * NS + half * 64);
+        float4* pc = reinterpret_cast<float4*>(p.dC_acc + tok * NS + col);
+        float4* pb = reinterpret_cast<float4*>(p.dB_acc + tok * NS + col);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
+        for (int j = 0; j < 8; ++j) {
           atomicAdd(pc + j, make_float4(dc[4 * j] + e * dci[4 * j], dc[4 * j + 1] + e * dci[4 * j + 1],
                                         dc[4 * j + 2] + e * dci[4 * j + 2], dc[4 * j + 3] + e * dci[4 * j + 3]));
           atomicAdd(pb + j, make_float4(db[4 * j], db[4 * j + 1], db[4 * j + 2], db[4 * j + 3]));
         }
       }
     }
+    // row sums: groups add up in a fixed order
+    part[grp * L + r] = kacc;
+    part[(4 + grp) * L + r] = racc;
+    part[(8 + grp) * L + r] = q_intra;
+    part[(12 + grp) * L + r] = q_inter;
     tc5::fence_proxy_async();
     __syncthreads();
-    if (r == 0) {                       // rows past T are clipped by the copy engine
+    if (threadIdx.x == 0) {             // rows past T are clipped by the copy engine
       tc5::tma_store_4d(&tm_dx, sXS, 0, h, t0, b);
       if (heads) {
         tc5::tma_store_4d(&tm_dch, sP, 0, h, t0, b);
@@ -595,7 +643,12 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
       tc5::tma_store_commit();
       tc5::tma_store_wait_read<0>();    // shared memory must outlive the copies' reads
     }
-    if (row_ok) p.q_out[tok * p.H + h] = q_intra + e * q_inter;
+    if (grp > 0 && row_ok) {            // group g finishes sum g (thread 0 is busy with the stores)
+      auto row_sum = [&](int k) { return (part[k * L + r] + part[(k + 1) * L + r]) + (part[(k + 2) * L + r] + part[(k + 3) * L + r]); };
+      if (grp == 1) p.k_out[tok * p.H + h] = row_sum(0);
+      else if (grp == 2) { if (p.r_out) p.r_out[tok * p.H + h] = row_sum(4); }
+      else p.q_out[tok * p.H + h] = row_sum(8) + e * row_sum(12);
+    }
   }
   tc5::fence_before_sync();
   __syncthreads();
@@ -605,33 +658,192 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
 // ---------------------------------------------------------------------------------------
 // State passing over chunks (elementwise).  Layout [B, nc, H, E], E = NS * PD.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) ssd_state_fwd_kernel(const float* __restrict__ S, const float* __restrict__ gamma,
-                                                            float* __restrict__ Hprev, bf16* __restrict__ Hprev_bf,
-                                                            float* __restrict__ Hlast, int nc, int H, long E) {
-  const long e = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= E) return;
-  const int h = blockIdx.y, b = blockIdx.z;
-  float st = 0.f;
-  for (int c = 0; c < nc; ++c) {
-    const long bch = (static_cast<long>(b) * nc + c) * H + h;
-    if (Hprev) Hprev[bch * E + e] = st;
-    if (Hprev_bf) Hprev_bf[bch * E + e] = __float2bfloat16(st);
-    st = gamma[bch] * st + S[bch * E + e];
-  }
-  if (Hlast) Hlast[(static_cast<long>(b) * H + h) * E + e] = st;
+// A thread walks the chunks of VEC neighbouring elements.  The recurrence itself is one FMA per chunk; what takes time is
+// memory, so the terms of the next eight chunks are always in flight.
+template <int VEC>
+struct Elems { float v[VEC]; };
+template <int VEC>
+__device__ __forceinline__ void st_bf16(bf16* p, const Elems<VEC>& x) {
+  if constexpr (VEC == 4) *reinterpret_cast<uint2*>(p) = make_uint2(tc5::pack_bf16(x.v[0], x.v[1]), tc5::pack_bf16(x.v[2], x.v[3]));
+  else *p = __float2bfloat16(x.v[0]);
 }
-__global__ void __launch_bounds__(256) ssd_state_bwd_kernel(const float* __restrict__ dHprev, const float* __restrict__ gamma,
-                                                            float* __restrict__ dS, bf16* __restrict__ dS_bf, int nc, int H, long E) {
-  const long e = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+template <int VEC>
+__device__ __forceinline__ Elems<VEC> ld_f32(const float* p) {
+  Elems<VEC> e;
+  if constexpr (VEC == 4) { const float4 f = *reinterpret_cast<const float4*>(p); e.v[0] = f.x; e.v[1] = f.y; e.v[2] = f.z; e.v[3] = f.w; }
+  else e.v[0] = *p;
+  return e;
+}
+template <int VEC>
+__device__ __forceinline__ void st_f32(float* p, const Elems<VEC>& x) {
+  if constexpr (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(x.v[0], x.v[1], x.v[2], x.v[3]);
+  else *p = x.v[0];
+}
+// out[c] = state entering chunk c; step: state <- gamma[c] state + in[c].  BACK walks the chunks in reverse.
+template <int VEC, bool BACK>
+__global__ void __launch_bounds__(256) ssd_state_kernel(const float* __restrict__ in, const float* __restrict__ gamma,
+                                                        float* __restrict__ out, bf16* __restrict__ out_bf,
+                                                        float* __restrict__ last, int nc, int H, long E) {
+  constexpr int U = 8;
+  const long e = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * VEC;
   if (e >= E) return;
   const int h = blockIdx.y, b = blockIdx.z;
-  float g = 0.f;
-  for (int c = nc - 1; c >= 0; --c) {
-    const long bch = (static_cast<long>(b) * nc + c) * H + h;
-    if (dS) dS[bch * E + e] = g;
-    if (dS_bf) dS_bf[bch * E + e] = __float2bfloat16(g);
-    g = dHprev[bch * E + e] + gamma[bch] * g;
+  auto at = [&](int i) { return (static_cast<long>(b) * nc + (BACK ? nc - 1 - i : i)) * H + h; };
+  Elems<VEC> st{}, next[U];
+  float g_next[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (u < nc) { next[u] = ld_f32<VEC>(in + at(u) * E + e); g_next[u] = gamma[at(u)]; }
+  for (int i0 = 0; i0 < nc; i0 += U) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u;
+      if (i >= nc) break;
+      const long o = at(i) * E + e;
+      if (out) st_f32<VEC>(out + o, st);
+      if (out_bf) st_bf16<VEC>(out_bf + o, st);
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) st.v[k] = g_next[u] * st.v[k] + next[u].v[k];
+      if (i + U < nc) { next[u] = ld_f32<VEC>(in + at(i + U) * E + e); g_next[u] = gamma[at(i + U)]; }
+    }
   }
+  if (last) st_f32<VEC>(last + (static_cast<long>(b) * H + h) * E + e, st);
+}
+template <bool BACK>
+int launch_state(const float* in, const float* gamma, float* out, void* out_bf, float* last, int B, int nc, int H, long E,
+                 cudaStream_t st) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(last) |
+                        (reinterpret_cast<uintptr_t>(out_bf) << 1);
+  if (E % 4 == 0 && all % 16 == 0)
+    ssd_state_kernel<4, BACK><<<dim3((unsigned)((E / 4 + 255) / 256), H, B), 256, 0, st>>>(in, gamma, out, (bf16*)out_bf, last, nc, H, E);
+  else
+    ssd_state_kernel<1, BACK><<<dim3((unsigned)((E + 255) / 256), H, B), 256, 0, st>>>(in, gamma, out, (bf16*)out_bf, last, nc, H, E);
+  nsa::count_launch();
+  return 0;
+}
+
+// ---------------------------------------------------------------------------------------
+// What follows the chunk gradients: sums over heads and over time.
+// ---------------------------------------------------------------------------------------
+// out[row][:] = sum over heads of in[row][h][:] for dB (z = 0) and dC (z = 1), fp32 sums in a fixed order, bf16 out.  A warp owns a
+// token: its rows are contiguous, 16 bytes per lane, two heads per instruction.
+__global__ void __launch_bounds__(256) ssd_sum_heads_kernel(const bf16* __restrict__ dBh, const bf16* __restrict__ dCh,
+                                                            bf16* __restrict__ dB, bf16* __restrict__ dC, long rows, int H) {
+  const long row = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
+  const uint4* src = reinterpret_cast<const uint4*>((blockIdx.y ? dCh : dBh) + row * H * NS) + lane;
+  float acc[8] = {};
+#pragma unroll 8
+  for (int h = lane >> 4; h < H; h += 2) {
+    const uint4 v = src[(h - (lane >> 4)) * (NS / 8)];
+    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 f = __bfloat1622float2(p[k]);
+      acc[2 * k] += f.x;
+      acc[2 * k + 1] += f.y;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);
+  if (lane < 16)
+    reinterpret_cast<uint4*>((blockIdx.y ? dC : dB) + row * NS)[lane] =
+        make_uint4(tc5::pack_bf16(acc[0], acc[1]), tc5::pack_bf16(acc[2], acc[3]), tc5::pack_bf16(acc[4], acc[5]), tc5::pack_bf16(acc[6], acc[7]));
+}
+
+// With da_t = sum over t' >= t of (q - k)_t' :  ddt = da A + k / dt,  dA = sum da dt,  dD = sum r  (sums over tokens and batch).
+// Chunks of 128 tokens in parallel: one kernel leaves each chunk's totals, the next adds up the totals of the chunks
+// behind its own (a few KB from L2) and walks the chunk from its end, a third sums the per-chunk dA and dD.
+// Thread = (head of 64, quarter of the chunk).  totals, pA, pD: [B * nc][H].
+__global__ void __launch_bounds__(256) ssd_totals_kernel(const float* __restrict__ q, const float* __restrict__ k,
+                                                         const float* __restrict__ r, float* __restrict__ totals,
+                                                         float* __restrict__ pD, int T, int H, int nc) {
+  __shared__ float ss[4][64], sd[4][64];
+  const int hl = threadIdx.x & 63, part = threadIdx.x >> 6, c = blockIdx.x, b = blockIdx.y;
+  const int t0 = c * L + part * 32, t1 = min(t0 + 32, T);
+  for (int h0 = 0; h0 < H; h0 += 64) {
+    const int h = h0 + hl;
+    float s = 0.f, d = 0.f;
+    if (h < H) {
+#pragma unroll 8
+      for (int t = t0; t < t1; ++t) {
+        const long i = (static_cast<long>(b) * T + t) * H + h;
+        s += q[i] - k[i];
+        if (r) d += r[i];
+      }
+    }
+    ss[part][hl] = s;
+    sd[part][hl] = d;
+    __syncthreads();
+    if (part == 0 && h < H) {
+      const long o = (static_cast<long>(b) * nc + c) * H + h;
+      totals[o] = (ss[0][hl] + ss[1][hl]) + (ss[2][hl] + ss[3][hl]);
+      if (r) pD[o] = (sd[0][hl] + sd[1][hl]) + (sd[2][hl] + sd[3][hl]);
+    }
+    __syncthreads();
+  }
+}
+__global__ void __launch_bounds__(256) ssd_ddt_kernel(const float* __restrict__ q, const float* __restrict__ k,
+                                                      const float* __restrict__ dt, const float* __restrict__ A,
+                                                      const float* __restrict__ totals, float* __restrict__ ddt,
+                                                      float* __restrict__ pA, int T, int H, int nc) {
+  __shared__ float ss[4][64], sb[4][64], sa[4][64];
+  const int hl = threadIdx.x & 63, part = threadIdx.x >> 6, c = blockIdx.x, b = blockIdx.y;
+  const int t0 = c * L + part * 32, t1 = min(t0 + 32, T);
+  for (int h0 = 0; h0 < H; h0 += 64) {
+    const int h = h0 + hl;
+    const bool live = h < H;
+    float s = 0.f, behind = 0.f;
+    if (live) {
+#pragma unroll 8
+      for (int t = t0; t < t1; ++t) {
+        const long i = (static_cast<long>(b) * T + t) * H + h;
+        s += q[i] - k[i];
+      }
+#pragma unroll 8
+      for (int cc = c + 1 + part; cc < nc; cc += 4) behind += totals[(static_cast<long>(b) * nc + cc) * H + h];
+    }
+    ss[part][hl] = s;
+    sb[part][hl] = behind;
+    __syncthreads();
+    float da = (sb[0][hl] + sb[1][hl]) + (sb[2][hl] + sb[3][hl]), acc = 0.f;
+    for (int p = 3; p > part; --p) da += ss[p][hl];
+    if (live) {
+      const float a = A[h];
+#pragma unroll 8
+      for (int t = t1 - 1; t >= t0; --t) {
+        const long i = (static_cast<long>(b) * T + t) * H + h;
+        const float kv = k[i], dv = dt[i];
+        da += q[i] - kv;
+        ddt[i] = da * a + kv / fmaxf(dv, 1e-20f);
+        acc += da * dv;
+      }
+    }
+    sa[part][hl] = acc;
+    __syncthreads();
+    if (part == 0 && live) pA[(static_cast<long>(b) * nc + c) * H + h] = (sa[0][hl] + sa[1][hl]) + (sa[2][hl] + sa[3][hl]);
+    __syncthreads();
+  }
+}
+// dA[h], dD[h] = sums over the rows of pA, pD in a fixed order.  CTA: 32 heads x 32 groups of rows.
+__global__ void __launch_bounds__(1024) ssd_head_sums_kernel(const float* __restrict__ pA, const float* __restrict__ pD,
+                                                             float* __restrict__ dA, float* __restrict__ dD, int rows, int H) {
+  __shared__ float sums[32][33];
+  const int l = threadIdx.x & 31, g = threadIdx.x >> 5, h = blockIdx.x * 32 + l;
+  const float* src = blockIdx.y ? pD : pA;
+  float s = 0.f;
+  if (h < H) {
+#pragma unroll 4
+    for (int i = g; i < rows; i += 32) s += src[static_cast<long>(i) * H + h];
+  }
+  sums[g][l] = s;
+  __syncthreads();
+  s = sums[l][g];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  const int hg = blockIdx.x * 32 + g;
+  if (l == 0 && hg < H) (blockIdx.y ? dD : dA)[hg] = s;
 }
 
 int map_bc(CUtensorMap* m, const void* base, int B, int T, long ld) {
@@ -670,17 +882,30 @@ int check_dims(int N, int P, long ld_bc, long ld_v) {
 
 extern "C" int nsa_ssd_state_fwd(const float* S, const float* gamma, float* Hprev, void* Hprev_bf16, float* Hlast, int B,
                                  int nc, int H, long E, cudaStream_t st) {
-  dim3 grid((unsigned)((E + 255) / 256), H, B);
-  ssd_state_fwd_kernel<<<grid, 256, 0, st>>>(S, gamma, Hprev, (bf16*)Hprev_bf16, Hlast, nc, H, E);
-  nsa::count_launch();
-  return 0;
+  return launch_state<false>(S, gamma, Hprev, Hprev_bf16, Hlast, B, nc, H, E, st);
 }
 extern "C" int nsa_ssd_state_bwd(const float* dHprev, const float* gamma, float* dS, void* dS_bf16, int B, int nc, int H,
                                  long E, cudaStream_t st) {
-  dim3 grid((unsigned)((E + 255) / 256), H, B);
-  ssd_state_bwd_kernel<<<grid, 256, 0, st>>>(dHprev, gamma, dS, (bf16*)dS_bf16, nc, H, E);
-  nsa::count_launch();
-  return 0;
+  return launch_state<true>(dHprev, gamma, dS, dS_bf16, nullptr, B, nc, H, E, st);
+}
+
+// dB_heads, dC_heads [B, T, H, 128] bf16 -> dB, dC [B, T, 128] bf16; q, k, r (or null), dt [B, T, H], A [H] fp32 ->
+// ddt [B, T, H], dA [H], dD [H] (or null).  scratch: 3 * B * ceil(T / 128) * H floats.
+extern "C" int nsa_ssd_finish(const void* dB_heads, const void* dC_heads, const float* q, const float* k, const float* r,
+                              const float* dt, const float* A, float* scratch, void* dB, void* dC, float* ddt, float* dA,
+                              float* dD, int B, int T, int H, cudaStream_t st) {
+  if (B <= 0 || T <= 0 || H <= 0 || (r == nullptr) != (dD == nullptr)) return nsa::fail(NSA_ERR_SHAPE, "ssd_finish: bad arguments");
+  const long rows = static_cast<long>(B) * T;
+  const int nc = (T + L - 1) / L;
+  float *totals = scratch, *pA = totals + static_cast<long>(B) * nc * H, *pD = pA + static_cast<long>(B) * nc * H;
+  ssd_sum_heads_kernel<<<dim3((unsigned)((rows + 7) / 8), 2), 256, 0, st>>>((const bf16*)dB_heads, (const bf16*)dC_heads, (bf16*)dB,
+                                                                           (bf16*)dC, rows, H);
+  ssd_totals_kernel<<<dim3(nc, B), 256, 0, st>>>(q, k, r, totals, pD, T, H, nc);
+  ssd_ddt_kernel<<<dim3(nc, B), 256, 0, st>>>(q, k, dt, A, totals, ddt, pA, T, H, nc);
+  ssd_head_sums_kernel<<<dim3((H + 31) / 32, dD ? 2 : 1), 1024, 0, st>>>(pA, pD, dA, dD, B * nc, H);
+  nsa::count_launch(4);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_finish launch");
 }
 
 // mode 0: bc = B rows, v = x -> chunk end states and gamma.  mode 1: bc = C rows, v = dy -> G.
@@ -697,7 +922,9 @@ extern "C" int nsa_ssd_chunk_state(int mode, const void* bc, long ld_bc, const v
   p.dt = dt; p.A = A; p.B = B; p.T = T; p.H = H; p.nc = (T + L - 1) / L;
   p.S_out = S_out; p.gamma_out = gamma_out; p.status = nsa::status_ptr();
   const int smem = 3 * BOXB + 1024 + 2048;
-  const dim3 grid(p.nc, H, B);
+  // Heads vary fastest in all three chunk kernels: a head's row of a token is 128 bytes, so CTAs that run together read
+  // and write neighbouring pieces of the same rows, and share the chunk's B and C tiles in L2.
+  const dim3 grid(H, p.nc, B);
   if (mode == 0) {
     static bool cfg = false;
     if (!cfg) { if ((rc = smem_attr(ssd_chunk_state_kernel<0>, smem))) return rc; cfg = true; }
@@ -727,11 +954,11 @@ extern "C" int nsa_ssd_chunk_out(const void* Cm, long ld_c, const void* Bm, long
   SsdParams p{};
   p.dt = dt; p.A = A; p.Dskip = Dskip; p.B = B; p.T = T; p.H = H; p.nc = nc;
   p.y = (bf16*)y; p.x_raw = (const bf16*)x; p.ldx = ld_x; p.status = nsa::status_ptr();
-  const int smem = 8 * BOXB + 1024 + 2048;
+  const int smem = 6 * BOXB + 1024 + 2048;
   static bool cfg = false;
   if (!cfg) { if ((rc = smem_attr(ssd_chunk_out_kernel, smem))) return rc; cfg = true; }
   if ((rc = map_v(&ty, y, B, T, H, static_cast<long>(H) * PD))) return rc;
-  ssd_chunk_out_kernel<<<dim3(nc, H, B), 128, smem, st>>>(tc, tb, tx, th, ty, p);
+  ssd_chunk_out_kernel<<<dim3(H, nc, B), 256, smem, st>>>(tc, tb, tx, th, ty, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_chunk_out launch");
@@ -763,10 +990,10 @@ static int ssd_chunk_grad_impl(const void* Cm, long ld_c, const void* Bm, long l
   p.x_raw = (const bf16*)x; p.ldx = ld_x; p.y_in = (const bf16*)y; p.dy_raw = (const bf16*)dy; p.dx = (bf16*)dx;
   p.dB_acc = dB_acc; p.dC_acc = dC_acc; p.q_out = q_out; p.k_out = k_out; p.status = nsa::status_ptr();
   p.dB_heads = (bf16*)dB_heads; p.dC_heads = (bf16*)dC_heads; p.r_out = r_out;
-  const int smem = 13 * BOXB + 1024 + 2048;
+  const int smem = 13 * BOXB + 1024 + 2048 + 16 * L * 4;
   static bool cfg = false;
   if (!cfg) { if ((rc = smem_attr(ssd_chunk_grad_kernel, smem))) return rc; cfg = true; }
-  ssd_chunk_grad_kernel<<<dim3(nc, H, B), 128, smem, st>>>(tc, tb, tx, tdy, th, tdh, tdx, tdbh, tdch, p);
+  ssd_chunk_grad_kernel<<<dim3(H, nc, B), 512, smem, st>>>(tc, tb, tx, tdy, th, tdh, tdx, tdbh, tdch, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_chunk_grad launch");

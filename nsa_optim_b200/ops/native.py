@@ -1370,20 +1370,20 @@ class _SSD(torch.autograd.Function):
         y = _empty(Bsz, T, H, P, dtype=torch.bfloat16, device=dev)
         _check(lib.nsa_ssd_chunk_out(_p(Cm), c_long(ldc), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(Hb), _p(dt), _p(A),
                                      _p(Df), _p(y), c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream()))
-        ctx.save_for_backward(x, dt, A, Bm, Cm, Df if Df is not None else _empty(0, device=dev), y, gamma, Hb)
+        ctx.save_for_backward(x, dt, A, Bm, Cm, Df if Df is not None else _empty(0, device=dev), gamma, Hb)
         ctx.lds = (ldx, ldb, ldc)
         ctx.has_D = D is not None
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, dt, A, Bm, Cm, Df, y, gamma, Hb = ctx.saved_tensors
+        x, dt, A, Bm, Cm, Df, gamma, Hb = ctx.saved_tensors
         ldx, ldb, ldc = ctx.lds
         Df = Df if ctx.has_D else None
-        Bsz, T, H, P = y.shape
+        Bsz, T, H, P = x.shape
         N = Bm.shape[-1]
         nc = gamma.shape[1]
-        dev = y.device
+        dev = x.device
         dy = dy.contiguous()
         lib = load()
         G = _empty(Bsz, nc, H, N, P, dtype=torch.float32, device=dev)
@@ -1401,21 +1401,18 @@ class _SSD(torch.autograd.Function):
         q = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
         k = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
         rdx = _empty(Bsz, T, H, dtype=torch.float32, device=dev) if ctx.has_D else None
-        _check(lib.nsa_ssd_chunk_grad_heads(_p(Cm), c_long(ldc), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(dy), _p(y), _p(Hb),
+        _check(lib.nsa_ssd_chunk_grad_heads(_p(Cm), c_long(ldc), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(dy), c_void_p(0), _p(Hb),
                                             _p(dHn), _p(dt), _p(A), _p(Df), _p(dx), _p(dBh), _p(dCh), _p(q), _p(k), _p(rdx),
                                             c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream()))
-        dB = dBh.sum(2, dtype=torch.float32)
-        dC = dCh.sum(2, dtype=torch.float32)
-        del dBh, dCh
         # d(cum_t) = dy_t.(y_t - D x_t) - x_t.dx_t ;  a_k = dt_k A enters every cum_t with t >= k
-        # (suffix sum over time, taken with time innermost: a scan along an outer dimension is slow)
-        dcum = (q - k).transpose(1, 2).contiguous()
-        pre = torch.cumsum(dcum, -1)
-        da = (pre[..., -1:] - pre + dcum).transpose(1, 2)
-        ddt = da * A[None, None, :] + k / dt.clamp_min(1e-20)
-        dA = (da * dt).sum((0, 1))
-        dD = rdx.sum((0, 1)) if ctx.has_D else None
-        return (dx, ddt, dA, dB.view(Bsz, T, 1, N).to(torch.bfloat16), dC.view(Bsz, T, 1, N).to(torch.bfloat16), dD)
+        dB, dC = (_empty(Bsz, T, 1, N, dtype=torch.bfloat16, device=dev) for _ in range(2))
+        ddt = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
+        dA = _empty(H, dtype=torch.float32, device=dev)
+        dD = _empty(H, dtype=torch.float32, device=dev) if ctx.has_D else None
+        scratch = _empty(3 * Bsz * nc * H, dtype=torch.float32, device=dev)
+        _check(lib.nsa_ssd_finish(_p(dBh), _p(dCh), _p(q), _p(k), _p(rdx), _p(dt), _p(A), _p(scratch), _p(dB), _p(dC), _p(ddt),
+                                  _p(dA), _p(dD), c_int(Bsz), c_int(T), c_int(H), _stream()))
+        return dx, ddt, dA, dB, dC, dD
 
 
 def copy_columns(dst: Tensor, src: Tensor) -> bool:

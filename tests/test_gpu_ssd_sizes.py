@@ -1,0 +1,59 @@
+"""Mamba-2 scan forward and backward where the chunk, state and head-sum kernels can go wrong: shorter than a chunk, around chunk
+ends, head counts off the eight heads of a summation block and odd, two sequences, no skip weight, strided inputs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(x, dt, A, Bm, Cm, D):
+    """The recurrence in 64 bits, one step at a time."""
+    h = x.new_zeros(x.shape[0], x.shape[2], x.shape[3], Bm.shape[-1])
+    ys = []
+    for t in range(x.shape[1]):
+        h = h * torch.exp(dt[:, t] * A)[..., None, None] + (dt[:, t, :, None] * x[:, t])[..., None] * Bm[:, t, 0][:, None, None, :]
+        ys.append(torch.einsum("bhpn,bn->bhp", h, Cm[:, t, 0]))
+    y = torch.stack(ys, 1)
+    return y if D is None else y + x * D[:, None]
+
+
+@pytest.mark.parametrize("B,T,H,skip", [(1, 1, 1, True), (2, 100, 3, False), (1, 128, 8, True), (2, 129, 9, True), (1, 300, 24, False)])
+def test_ssd_sizes(native, B, T, H, skip):
+    torch.manual_seed(T)
+    xbc = torch.nn.functional.silu(torch.randn(B, T, H * 64 + 256, device="cuda")).bfloat16()
+    dt = torch.nn.functional.softplus(torch.randn(B, T, H, device="cuda") - 3)
+    leaves = [xbc[..., :H * 64].view(B, T, H, 64), dt, -torch.rand(H, device="cuda") * 15 - 1, xbc[..., H * 64:H * 64 + 128].view(B, T, 1, 128),
+              xbc[..., H * 64 + 128:].view(B, T, 1, 128)] + ([torch.rand(H, device="cuda") + 0.5] if skip else [])
+    leaves = [t.detach().requires_grad_() for t in leaves]
+    dy = (torch.randn(B, T, H, 64, device="cuda") + 0.5).bfloat16()
+    y = native.ssd_scan(*leaves)
+    got = [y.detach()] + list(torch.autograd.grad(y, leaves, dy))
+    ref = [t.detach().double().requires_grad_() for t in leaves]
+    r = _reference(*ref, *([] if skip else [None]))
+    want = [r.detach()] + list(torch.autograd.grad(r, ref, dy.double()))
+    for name, a, b in zip(("y", "dx", "ddt", "dA", "dB", "dC", "dD"), got, want):
+        assert a.shape == b.shape
+        # bf16 operands and per-head terms: 2^-9 each, a few of them, averaged over the sums
+        assert (a.double() - b).norm() < 1e-2 * b.norm() + 1e-6, name
+
+
+@pytest.mark.parametrize("nc,E", [(1, 7), (7, 12), (8, 64), (9, 1000), (30, 8192)])
+@pytest.mark.parametrize("back", [False, True])
+def test_state_pass(native, nc, E, back):
+    from ctypes import c_int, c_long, c_void_p
+    torch.manual_seed(nc)
+    B, H = 2, 3
+    S, gamma = torch.randn(B, nc, H, E, device="cuda"), torch.rand(B, nc, H, device="cuda")
+    out, out_bf = torch.empty_like(S), torch.empty(S.shape, device="cuda", dtype=torch.bfloat16)
+    p = lambda t: c_void_p(t.data_ptr())                                            # noqa: E731
+    dims = (c_int(B), c_int(nc), c_int(H), c_long(E), native._stream())
+    if back:
+        native._check(native.load().nsa_ssd_state_bwd(p(S), p(gamma), p(out), p(out_bf), *dims))
+    else:
+        native._check(native.load().nsa_ssd_state_fwd(p(S), p(gamma), p(out), p(out_bf), c_void_p(0), *dims))
+    st, want = torch.zeros(B, H, E, device="cuda", dtype=torch.float64), torch.empty(S.shape, device="cuda", dtype=torch.float64)
+    for c in (reversed(range(nc)) if back else range(nc)):
+        want[:, c] = st
+        st = gamma[:, c, :, None].double() * st + S[:, c].double()
+    assert (out.double() - want).abs().max() <= 1e-5 * want.abs().max() + 1e-12     # one fp32 rounding per chunk, decaying
+    assert torch.equal(out_bf, out.to(torch.bfloat16))
