@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256) rmsnorm_add_fwd_kernel(const bf16* __rest
 // input by another route (the residual stream); it is added into dx here instead of by a
 // separate pass over both tensors.
 template <int TPR, int NV, int MODE>
-__global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g,
+__global__ void __launch_bounds__(256, NV == 1 ? (MODE == 0 && TPR == 256 ? 4 : 2) : 1) rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g,
                                                           const bf16* __restrict__ w, const bf16* __restrict__ dy,
                                                           const float* __restrict__ rstd_in, bf16* __restrict__ dx,
                                                           bf16* __restrict__ dg, float* __restrict__ partial,
@@ -191,10 +191,30 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
     if (c < d) load8(w + c, wv[i]);
   }
-  for (long base = static_cast<long>(blockIdx.x) * rows_per_cta; base < rows; base += static_cast<long>(gridDim.x) * rows_per_cta) {
+  // The next row's operands are in flight while this row is reduced (the reduction is two barriers long); rows of 8192
+  // would need too many registers for that and load when they are used.
+  constexpr bool AHEAD = NV <= 2;
+  uint4 nx[NV], ndy[NV], ng[NV], nr[NV];
+  auto fetch = [&](long row) {
+    if (row >= rows) return;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (t + i * TPR) * 8;
+      if (c >= d) continue;
+      nx[i] = *reinterpret_cast<const uint4*>(x + row * d + c);
+      ndy[i] = *reinterpret_cast<const uint4*>(dy + row * d + c);
+      if (MODE != 0) ng[i] = *reinterpret_cast<const uint4*>(g + row * (ldg ? ldg : d) + c);
+      if (dres != nullptr) nr[i] = *reinterpret_cast<const uint4*>(dres + row * d + c);
+    }
+  };
+  const long stride = static_cast<long>(gridDim.x) * rows_per_cta;
+  if (AHEAD) fetch(static_cast<long>(blockIdx.x) * rows_per_cta + sub);
+  for (long base = static_cast<long>(blockIdx.x) * rows_per_cta; base < rows; base += stride) {
     const long row = base + sub;
     const bool active = row < rows;
     const float rstd = active ? rstd_in[row] : 0.f;
+    if (!AHEAD) fetch(row);
+    uint4 cx[NV], cr[NV];
     float xn[NV][8], wdy[NV][8], gv[NV][8], sg[NV][8];
     float dot = 0.f;
 #pragma unroll
@@ -202,9 +222,11 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
       const int c = (t + i * TPR) * 8;
       if (active && c < d) {
         float xv[8], dv[8];
-        load8(x + row * d + c, xv);
-        load8(dy + row * d + c, dv);
-        if (MODE != 0) load8(g + row * (ldg ? ldg : d) + c, gv[i]);
+        cx[i] = nx[i];
+        cr[i] = nr[i];
+        unpack8(nx[i], xv);
+        unpack8(ndy[i], dv);
+        if (MODE != 0) unpack8(ng[i], gv[i]);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           float xin = xv[j];
@@ -223,6 +245,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
         }
       }
     }
+    if (AHEAD) fetch(row + stride);
     dot = row_sum<TPR>(dot, red) / d;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -234,7 +257,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
         if (MODE == 2) {
           // norm input u = x*silu(g): dx = du*silu(g), dg = du*x*dsilu(g)
           float xv[8], og[8];
-          load8(x + row * d + c, xv);
+          unpack8(cx[i], xv);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             og[j] = o[j] * xv[j] * dsilu_f(gv[i][j]);
@@ -246,7 +269,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
         }
         if (dres != nullptr) {
           float rv[8];
-          load8(dres + row * d + c, rv);
+          unpack8(cr[i], rv);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += rv[j];
         }
@@ -281,15 +304,26 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
   }
 }
 
-// out[c] = sum_p partial[p][c], p ascending (deterministic); bf16 or fp32 output.
-__global__ void reduce_partials_kernel(const float* __restrict__ partial, int parts, int width,
-                                       bf16* __restrict__ out_bf16, float* __restrict__ out_f32) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= width) return;
+// out[c] = sum_p partial[p][c] in a fixed order; bf16 or fp32 output.  CTA: 32 columns x 32 groups of parts (a thread per
+// column walking all parts took 25 us for 592 x 2048: one dependent stream of reads on eight CTAs).
+__global__ void __launch_bounds__(1024) reduce_partials_kernel(const float* __restrict__ partial, int parts, int width,
+                                                               bf16* __restrict__ out_bf16, float* __restrict__ out_f32) {
+  __shared__ float sums[32][33];
+  const int l = threadIdx.x & 31, g = threadIdx.x >> 5, c = blockIdx.x * 32 + l;
   float s = 0.f;
-  for (int p = 0; p < parts; ++p) s += partial[static_cast<long>(p) * width + c];
-  if (out_bf16) out_bf16[c] = __float2bfloat16(s);
-  if (out_f32) out_f32[c] = s;
+  if (c < width) {
+#pragma unroll 4
+    for (int p = g; p < parts; p += 32) s += partial[static_cast<long>(p) * width + c];
+  }
+  sums[g][l] = s;
+  __syncthreads();
+  // warp g finishes column g of the tile: 32 group sums meet by shuffles
+  s = warp_sum(sums[l][g]);
+  const int cg = blockIdx.x * 32 + g;
+  if (l == 0 && cg < width) {
+    if (out_bf16) out_bf16[cg] = __float2bfloat16(s);
+    if (out_f32) out_f32[cg] = s;
+  }
 }
 
 // ------------------------------------------------------------------------------------
@@ -815,14 +849,14 @@ int launch_rms_fwd(const void* x, const void* g, const void* w, void* y, float* 
 
 template <int MODE>
 int launch_rms_bwd(const void* x, const void* g, const void* w, const void* dy, const float* rstd, void* dx, void* dg,
-                   float* partial, int grid, long rows, int d, cudaStream_t st, const void* dres = nullptr, long ldg = 0) {
+                   float* partial, int& grid, long rows, int d, cudaStream_t st, const void* dres = nullptr, long ldg = 0) {
   const bf16 *X = (const bf16*)x, *G = (const bf16*)g, *Wt = (const bf16*)w, *DY = (const bf16*)dy, *DR = (const bf16*)dres;
   bf16 *DX = (bf16*)dx, *DG = (bf16*)dg;
-  if (d <= 256) rmsnorm_bwd_kernel<32, 1, MODE><<<grid, 256, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
-  else if (d <= 512) rmsnorm_bwd_kernel<32, 2, MODE><<<grid, 256, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
-  else if (d <= 2048) rmsnorm_bwd_kernel<256, 1, MODE><<<grid, 256, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
-  else if (d <= 4096) rmsnorm_bwd_kernel<256, 2, MODE><<<grid, 256, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
-  else if (d <= 8192) rmsnorm_bwd_kernel<256, 4, MODE><<<grid, 256, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
+  if (d <= 256) run_rms_bwd<32, 1, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
+  else if (d <= 512) run_rms_bwd<32, 2, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
+  else if (d <= 2048) run_rms_bwd<256, 1, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
+  else if (d <= 4096) run_rms_bwd<256, 2, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
+  else if (d <= 8192) run_rms_bwd<256, 4, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
   else return nsa::fail(NSA_ERR_SHAPE, "rmsnorm: width above 8192 is not supported");
   nsa::count_launch();
   return 0;
@@ -841,6 +875,25 @@ int launch_rms_add_fwd(const void* x, const void* r, const void* w, void* h, voi
   else return nsa::fail(NSA_ERR_SHAPE, "rmsnorm: width above 8192 is not supported");
   nsa::count_launch();
   return 0;
+// CTAs of the persistent backward: all resident at once (a partial second round would idle most SMs), at most `parts`.
+template <int TPR, int NV, int MODE>
+int bwd_grid(int parts) {
+  static int per_sm = 0;
+  if (per_sm == 0) {
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rmsnorm_bwd_kernel<TPR, NV, MODE>, 256, 0);
+    per_sm = n > 0 ? n : 1;
+  }
+  const int all = per_sm * nsa::sm_count();
+  return parts < all ? parts : all;
+}
+template <int TPR, int NV, int MODE>
+void run_rms_bwd(const bf16* X, const bf16* G, const bf16* Wt, const bf16* DY, const float* rstd, bf16* DX, bf16* DG, float* partial,
+                 int& grid, long rows, int d, const bf16* DR, long ldg, cudaStream_t st) {
+  grid = bwd_grid<TPR, NV, MODE>(grid);
+  rmsnorm_bwd_kernel<TPR, NV, MODE><<<grid, 256, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
+}
+// `grid` holds the number of partial rows the caller has room for and receives the number written.
 }
 
 }  // namespace
@@ -867,13 +920,13 @@ extern "C" int nsa_rmsnorm_bwd(const void* x, const void* gate, const void* w, c
                                void* dx, void* dgate, void* dw_bf16, float* dw_f32, float* partial, long rows, int d,
                                int mode, cudaStream_t st) {
   if (d % 8) return nsa::fail(NSA_ERR_SHAPE, "rmsnorm: width must be a multiple of 8");
-  const int parts = nsa_rmsnorm_bwd_parts(rows, d);
+  int parts = nsa_rmsnorm_bwd_parts(rows, d);
   int rc;
   if (mode == 0) rc = launch_rms_bwd<0>(x, gate, w, dy, rstd, dx, dgate, partial, parts, rows, d, st);
   else if (mode == 1) rc = launch_rms_bwd<1>(x, gate, w, dy, rstd, dx, dgate, partial, parts, rows, d, st);
   else rc = launch_rms_bwd<2>(x, gate, w, dy, rstd, dx, dgate, partial, parts, rows, d, st);
   if (rc) return rc;
-  reduce_partials_kernel<<<(d + 255) / 256, 256, 0, st>>>(partial, parts, d, (bf16*)dw_bf16, dw_f32);
+  reduce_partials_kernel<<<(d + 31) / 32, 1024, 0, st>>>(partial, parts, d, (bf16*)dw_bf16, dw_f32);
   nsa::count_launch();
   return 0;
 }
@@ -892,13 +945,13 @@ extern "C" int nsa_rmsnorm_bwd_ldg(const void* x, const void* gate, long ldg, co
                                    int mode, cudaStream_t st) {
   if (d % 8 || ldg % 8 || (reinterpret_cast<uintptr_t>(gate) & 15))
     return nsa::fail(NSA_ERR_ALIGNMENT, "rmsnorm: widths multiples of 8 and 16-byte aligned gate rows required");
-  const int parts = nsa_rmsnorm_bwd_parts(rows, d);
+  int parts = nsa_rmsnorm_bwd_parts(rows, d);
   int rc;
   if (mode == 1) rc = launch_rms_bwd<1>(x, gate, w, dy, rstd, dx, dgate, partial, parts, rows, d, st, nullptr, ldg);
   else if (mode == 2) rc = launch_rms_bwd<2>(x, gate, w, dy, rstd, dx, dgate, partial, parts, rows, d, st, nullptr, ldg);
   else return nsa::fail(NSA_ERR_SHAPE, "nsa_rmsnorm_bwd_ldg: gated modes only");
   if (rc) return rc;
-  reduce_partials_kernel<<<(d + 255) / 256, 256, 0, st>>>(partial, parts, d, (bf16*)dw_bf16, dw_f32);
+  reduce_partials_kernel<<<(d + 31) / 32, 1024, 0, st>>>(partial, parts, d, (bf16*)dw_bf16, dw_f32);
   nsa::count_launch();
   return 0;
 }
@@ -915,10 +968,10 @@ extern "C" int nsa_rmsnorm_bwd_res(const void* x, const void* w, const void* dy,
                                    void* dx, void* dw_bf16, float* dw_f32, float* partial, long rows, int d,
                                    cudaStream_t st) {
   if (d % 8) return nsa::fail(NSA_ERR_SHAPE, "rmsnorm: width must be a multiple of 8");
-  const int parts = nsa_rmsnorm_bwd_parts(rows, d);
+  int parts = nsa_rmsnorm_bwd_parts(rows, d);
   const int rc = launch_rms_bwd<0>(x, nullptr, w, dy, rstd, dx, nullptr, partial, parts, rows, d, st, dres);
   if (rc) return rc;
-  reduce_partials_kernel<<<(d + 255) / 256, 256, 0, st>>>(partial, parts, d, (bf16*)dw_bf16, dw_f32);
+  reduce_partials_kernel<<<(d + 31) / 32, 1024, 0, st>>>(partial, parts, d, (bf16*)dw_bf16, dw_f32);
   nsa::count_launch();
   return 0;
 }

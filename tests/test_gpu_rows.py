@@ -1,0 +1,53 @@
+"""Row kernels around the sizes their launches choose by: cross-entropy rows that fit in registers or stream, norm
+backward with fewer rows than CTAs, several rows per CTA and each register layout, against 64-bit results."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N,V", [(1, 8), (5, 4096), (3, 4104), (130, 32000), (7, 32768), (7, 32776)])
+def test_linear_cross_entropy_rows(native, N, V):
+    torch.manual_seed(V)
+    d = 64
+    h = (torch.randn(N, d, device="cuda") * 2).bfloat16().requires_grad_()
+    w = (torch.randn(V, d, device="cuda") * 0.2).bfloat16().requires_grad_()
+    labels = torch.randint(0, V, (N,), device="cuda")
+    if N > 4:
+        labels[3] = -100
+    loss = native.linear_cross_entropy(h, w, labels)
+    got = torch.autograd.grad(loss * 3.0, [h, w])
+    hr, wr = h.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    ref = F.cross_entropy(hr @ wr.t(), labels, ignore_index=-100)
+    want = torch.autograd.grad(ref * 3.0, [hr, wr])
+    assert abs(float(loss) - float(ref)) <= 2e-3 * abs(float(ref)) + 2e-3          # logits are rounded to bf16
+    for a, b in zip(got, want):
+        assert a.dtype == torch.bfloat16 and (a.double() - b).norm() <= 1.5e-2 * b.norm()
+
+
+@pytest.mark.parametrize("mode", ["plain", "add", "before", "after"])
+@pytest.mark.parametrize("rows,d", [(1, 256), (7, 512), (3000, 256), (6000, 264), (1, 2048), (593, 2048), (1300, 1000), (700, 4096), (600, 8192)])
+def test_norm_backward_rows(native, mode, rows, d):
+    torch.manual_seed(d)
+    x, r, dy, dh = (torch.randn(rows, d, device="cuda").bfloat16() for _ in range(4))
+    w = (1 + 0.1 * torch.randn(d, device="cuda")).bfloat16()
+    leaves = [t.requires_grad_() for t in ([x, w] if mode == "plain" else [x, r, w])]
+    ref = [t.detach().double().requires_grad_() for t in leaves]
+    norm = lambda u, v: u * (u.square().mean(-1, keepdim=True) + 1e-6).rsqrt() * v     # noqa: E731
+    if mode == "add":
+        h, y = native.add_rms_norm(*leaves)
+        got = torch.autograd.grad([h, y], leaves, [dh, dy])
+        # the kernel's statistics are those of the rounded sum
+        s = ref[0] + ref[1]
+        s = s + (s.to(torch.bfloat16).double() - s).detach()
+        want = torch.autograd.grad([s, norm(s, ref[2])], ref, [dh.double(), dy.double()])
+    elif mode == "plain":
+        got = torch.autograd.grad(native.rms_norm(*leaves), leaves, dy)
+        want = torch.autograd.grad(norm(*ref), ref, dy.double())
+    else:
+        got = torch.autograd.grad(native.gated_rms_norm(*leaves, norm_before_gate=mode == "before"), leaves, dy)
+        y = norm(ref[0], ref[2]) * F.silu(ref[1]) if mode == "before" else norm(ref[0] * F.silu(ref[1]), ref[2])
+        want = torch.autograd.grad(y, ref, dy.double())
+    for a, b in zip(got, want):
+        assert (a.double() - b).norm() <= 5e-3 * b.norm() + 1e-6                      # one rounding to bf16, fp32 inside
