@@ -594,12 +594,20 @@ __global__ void __launch_bounds__(256) rope_kernel(const bf16* __restrict__ x, c
 // Causal depthwise conv1d, width 4, channel-last (B, T, C), optional bias and SiLU.
 // Bound by memory when the arithmetic stays out of the way: a lane owns four channels (8-byte
 // accesses, a warp covers 256 contiguous bytes of a row) and walks `rows` consecutive time steps
-// with the last three rows in registers, so every element is read and widened once and no row
-// passes through shared memory; the next four rows are in flight while four are computed.  The
-// taps are packed fp32 FMAs (two channels per instruction).  The eight warps of a CTA own eight
-// consecutive time segments.
+// with the last three rows in registers, so every element is read and widened once.  The rows ahead
+// travel through a ring of shared memory that a lane fills (cp.async) and reads for itself alone: no barriers,
+// and 12 rows of a warp stay in flight without holding registers.  The taps are packed fp32 FMAs (two channels per
+// instruction).  A CTA is four channel tiles (1 KB of a row) by two time segments.
 // ------------------------------------------------------------------------------------
-constexpr int CT_WARPS = 8, CT_C = 128, CT_U = 4;
+constexpr int CT_CW = 4, CT_TW = 2, CT_WARPS = CT_CW * CT_TW, CT_C = 128, CT_U = 4, CT_RING = 4;
+
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pred) {   // zero fill when !pred
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gmem), "r"(pred ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Two fp32 lanes per instruction; each lane rounds as the scalar instruction does.
 __device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c) {
@@ -643,37 +651,46 @@ __device__ __forceinline__ void conv_taps(const bf16* __restrict__ w, const bf16
   bv = Quad{make_float2(s[0], s[1]), make_float2(s[2], s[3])};
 }
 
-__global__ void __launch_bounds__(CT_WARPS * 32) conv1d_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                                                   const bf16* __restrict__ bias, bf16* __restrict__ y,
-                                                                   int T, int C, long ldx, int act, int rows) {
-  const int c = blockIdx.x * CT_C + (threadIdx.x & 31) * 4;
-  const int t0 = (blockIdx.y * CT_WARPS + (threadIdx.x >> 5)) * rows;
+__global__ void __launch_bounds__(CT_WARPS * 32, 4) conv1d_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
+                                                                      const bf16* __restrict__ bias, bf16* __restrict__ y,
+                                                                      int T, int C, long ldx, int act, int rows) {
+  __shared__ uint2 ring_all[CT_WARPS][CT_RING * CT_U][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = (blockIdx.x * CT_CW + warp % CT_CW) * CT_C + lane * 4;
+  const int t0 = (blockIdx.y * CT_TW + warp / CT_CW) * rows;
   if (c >= C || t0 >= T) return;
+  uint2(*ring)[32] = ring_all[warp];
   const bf16* xp = x + static_cast<long>(blockIdx.z) * T * ldx + c;
-  bf16* yp = y + static_cast<long>(blockIdx.z) * T * C + c;
-  const int t1 = min(t0 + rows, T);
-  auto load = [&](int t) {
-    return t >= 0 && t < t1 ? *reinterpret_cast<const uint2*>(xp + t * ldx) : make_uint2(0u, 0u);
-  };
-  uint2 next[CT_U];
-#pragma unroll
-  for (int u = 0; u < CT_U; ++u) next[u] = load(t0 + u);
-  Quad x0 = quad_unpack(load(t0 - 3)), x1 = quad_unpack(load(t0 - 2)), x2 = quad_unpack(load(t0 - 1));
-  Quad wv[4], bv;
-  conv_taps(w, bias, c, true, wv, bv);
-  for (int t = t0; t < t1; t += CT_U) {
-    uint2 cur[CT_U];
-#pragma unroll
-    for (int u = 0; u < CT_U; ++u) cur[u] = next[u];
-#pragma unroll
-    for (int u = 0; u < CT_U; ++u) next[u] = load(t + CT_U + u);
+  bf16* yp = y + (static_cast<long>(blockIdx.z) * T + t0) * C + c;
+  const int n = min(rows, T - t0);                  // rows of this segment
+  const bf16* xs = xp + static_cast<long>(t0) * ldx;
+  auto issue = [&](int g) {                         // rows g * CT_U .. of the segment
 #pragma unroll
     for (int u = 0; u < CT_U; ++u) {
-      const Quad x3 = quad_unpack(cur[u]);
+      const int r = g * CT_U + u;
+      cp_async8(&ring[(g % CT_RING) * CT_U + u][lane], r < n ? xs + r * ldx : xs, r < n);
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int g = 0; g < CT_RING - 1; ++g) issue(g);
+  auto before = [&](int k) {
+    return quad_unpack(t0 >= k ? *reinterpret_cast<const uint2*>(xs - k * ldx) : make_uint2(0u, 0u));
+  };
+  Quad x0 = before(3), x1 = before(2), x2 = before(1);
+  Quad wv[4], bv;
+  conv_taps(w, bias, c, true, wv, bv);
+  for (int g = 0; g * CT_U < n; ++g) {
+    issue(g + CT_RING - 1);
+    cp_async_wait<CT_RING - 1>();
+#pragma unroll
+    for (int u = 0; u < CT_U; ++u) {
+      const Quad x3 = quad_unpack(ring[(g % CT_RING) * CT_U + u][lane]);
       Quad o = quad_fma(wv[3], x3, quad_fma(wv[2], x2, quad_fma(wv[1], x1, quad_fma(wv[0], x0, bv))));
       x0 = x1; x1 = x2; x2 = x3;
       if (act) o = Quad{make_float2(silu_f(o.a.x), silu_f(o.a.y)), make_float2(silu_f(o.b.x), silu_f(o.b.y))};
-      if (t + u < t1) *reinterpret_cast<uint2*>(yp + static_cast<long>(t + u) * C) = quad_pack(o);
+      if (g * CT_U + u < n) *reinterpret_cast<uint2*>(yp) = quad_pack(o);
+      yp += C;
     }
   }
 }
@@ -681,50 +698,58 @@ __global__ void __launch_bounds__(CT_WARPS * 32) conv1d_fwd_kernel(const bf16* _
 // Backward: dpre[t] = dy[t] (times SiLU'(pre[t]), pre recomputed from x), dx[s] = sum_j w[j] dpre[s + 3 - j],
 // dw[j] = sum_t dpre[t] x[t - 3 + j], db = sum_t dpre[t].  The walk of the forward with dx three rows
 // behind: a segment also computes dpre on the three rows after its end, which the next one counts.
-// Weight and bias gradients stay in registers, the warps of a CTA meet through shared memory in a
+// Weight and bias gradients stay in registers, the CTA's time segments meet through shared memory in a
 // fixed order, and one partial sum leaves per (CTA in time, batch): partial layout [chunk][5][C]
 // (row 4 = bias gradient), chunk = blockIdx.z * gridDim.y + blockIdx.y.
+struct ConvBwdSmem {
+  uint2 x[CT_WARPS][CT_RING * CT_U][32], g[CT_WARPS][CT_RING * CT_U][32];
+};
 __global__ void __launch_bounds__(CT_WARPS * 32, 2) conv1d_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                                       const bf16* __restrict__ bias, const bf16* __restrict__ dy,
                                                                       bf16* __restrict__ dx, float* __restrict__ partial,
                                                                       int T, int C, long ldx, int act, int rows) {
-  __shared__ __align__(16) float sred[CT_WARPS][5][CT_C];
+  extern __shared__ __align__(16) uint8_t conv_smem[];
+  ConvBwdSmem& sm = *reinterpret_cast<ConvBwdSmem*>(conv_smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = blockIdx.x * CT_C + lane * 4;
-  const bool c_ok = c < C;
-  const int t0 = (blockIdx.y * CT_WARPS + warp) * rows;
-  const int t1 = min(t0 + rows, T);
+  const int c = (blockIdx.x * CT_CW + warp % CT_CW) * CT_C + lane * 4;
+  const int t0 = (blockIdx.y * CT_TW + warp / CT_CW) * rows;
   Quad dw[4], db = quad_zero();
 #pragma unroll
   for (int j = 0; j < 4; ++j) dw[j] = quad_zero();
-  if (c_ok && t0 < T) {
-    const bf16* xp = x + static_cast<long>(blockIdx.z) * T * ldx + c;
-    const bf16* gp = dy + static_cast<long>(blockIdx.z) * T * C + c;
-    bf16* dp = dx + static_cast<long>(blockIdx.z) * T * C + c;
-    const int te = min(t1 + 3, T);               // dpre is needed on [t0, te); rows past T count as zero
-    auto load_x = [&](int t) {
-      return t >= 0 && t < te ? *reinterpret_cast<const uint2*>(xp + t * ldx) : make_uint2(0u, 0u);
-    };
-    auto load_g = [&](int t) {
-      return t < te ? *reinterpret_cast<const uint2*>(gp + static_cast<long>(t) * C) : make_uint2(0u, 0u);
-    };
-    uint2 nx[CT_U], ng[CT_U];
+  if (c < C && t0 < T) {
+    uint2 (*rx)[32] = sm.x[warp], (*rg)[32] = sm.g[warp];
+    const bf16* xs = x + (static_cast<long>(blockIdx.z) * T + t0) * ldx + c;
+    const bf16* gs = dy + (static_cast<long>(blockIdx.z) * T + t0) * C + c;
+    bf16* dp = dx + (static_cast<long>(blockIdx.z) * T + t0) * C + c;
+    const int n = min(rows, T - t0);             // rows of this segment
+    const int ne = min(n + 3, T - t0);           // dpre is needed on [0, ne); rows past T count as zero
+    auto issue = [&](int g) {
 #pragma unroll
-    for (int u = 0; u < CT_U; ++u) { nx[u] = load_x(t0 + u); ng[u] = load_g(t0 + u); }
-    Quad x0 = quad_unpack(load_x(t0 - 3)), x1 = quad_unpack(load_x(t0 - 2)), x2 = quad_unpack(load_x(t0 - 1));
+      for (int u = 0; u < CT_U; ++u) {
+        const int r = g * CT_U + u, slot = (g % CT_RING) * CT_U + u;
+        cp_async8(&rx[slot][lane], r < ne ? xs + r * ldx : xs, r < ne);
+        cp_async8(&rg[slot][lane], r < ne ? gs + static_cast<long>(r) * C : gs, r < ne);
+      }
+      cp_async_commit();
+    };
+#pragma unroll
+    for (int g = 0; g < CT_RING - 1; ++g) issue(g);
+    auto before = [&](int k) {
+      return quad_unpack(t0 >= k ? *reinterpret_cast<const uint2*>(xs - k * ldx) : make_uint2(0u, 0u));
+    };
+    Quad x0 = before(3), x1 = before(2), x2 = before(1);
     Quad wv[4], bv;
     conv_taps(w, bias, c, true, wv, bv);
     Quad d0 = quad_zero(), d1 = quad_zero(), d2 = quad_zero();
-    for (int t = t0; t < t1 + 3; t += CT_U) {
-      uint2 cx[CT_U], cg[CT_U];
-#pragma unroll
-      for (int u = 0; u < CT_U; ++u) { cx[u] = nx[u]; cg[u] = ng[u]; }
-#pragma unroll
-      for (int u = 0; u < CT_U; ++u) { nx[u] = load_x(t + CT_U + u); ng[u] = load_g(t + CT_U + u); }
+    dp -= 3L * C;
+    for (int g = 0; g * CT_U < n + 3; ++g) {
+      issue(g + CT_RING - 1);
+      cp_async_wait<CT_RING - 1>();
 #pragma unroll
       for (int u = 0; u < CT_U; ++u) {
-        const Quad x3 = quad_unpack(cx[u]);
-        Quad d3 = quad_unpack(cg[u]);            // zero past T, and so is dpre
+        const int r = g * CT_U + u, slot = (g % CT_RING) * CT_U + u;
+        const Quad x3 = quad_unpack(rx[slot][lane]);
+        Quad d3 = quad_unpack(rg[slot][lane]);   // zero past T, and so is dpre
         if (act) {
           const Quad p = quad_fma(wv[3], x3, quad_fma(wv[2], x2, quad_fma(wv[1], x1, quad_fma(wv[0], x0, bv))));
           d3.a.x *= dsilu_f(p.a.x); d3.a.y *= dsilu_f(p.a.y);
@@ -1170,25 +1195,27 @@ extern "C" int nsa_rope(const void* x, const float* cos_t, const float* sin_t, v
 }
 
 // Time steps per warp: 64 keeps the rows read twice (3 of x ahead of a segment, 3 of dpre behind it) under
-// a tenth; short sequences take 32, 16 or 8 so that four CTAs per SM still find work.
+// a tenth; short sequences take 32, 16 or 8 so that every SM still finds 32 warps.
 static int conv_rows(int B, int T, int C) {
   int rows = 64;
-  auto ctas = [&](int r) { return static_cast<long>(B) * ((C + CT_C - 1) / CT_C) * ((T + CT_WARPS * r - 1) / (CT_WARPS * r)); };
-  while (rows > 8 && ctas(rows) < 4L * nsa::sm_count()) rows >>= 1;
+  auto warps = [&](int r) { return static_cast<long>(B) * ((C + CT_C - 1) / CT_C) * ((T + r - 1) / r); };
+  while (rows > 8 && warps(rows) < 32L * nsa::sm_count()) rows >>= 1;
   return rows;
 }
 extern "C" int nsa_conv1d_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, long ldx,
                               int width, int act, cudaStream_t st) {
   if (C % 8 || ldx % 8 || width != 4) return nsa::fail(NSA_ERR_SHAPE, "conv1d: channels multiple of 8 and width 4 required");
+static dim3 conv_grid(int B, int T, int C, int rows) {
+  return dim3((C + CT_CW * CT_C - 1) / (CT_CW * CT_C), (T + CT_TW * rows - 1) / (CT_TW * rows), B);
+}
   const int rows = conv_rows(B, T, C);
-  dim3 grid((C + CT_C - 1) / CT_C, (T + CT_WARPS * rows - 1) / (CT_WARPS * rows), B);
+  const dim3 grid = conv_grid(B, T, C, rows);
   conv1d_fwd_kernel<<<grid, CT_WARPS * 32, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)y, T, C, ldx, act, rows);
   nsa::count_launch();
   return 0;
 }
 extern "C" long nsa_conv1d_bwd_parts(int B, int T, int C) {
-  const int span = CT_WARPS * conv_rows(B, T, C);
-  return static_cast<long>(B) * ((T + span - 1) / span);
+  return static_cast<long>(B) * conv_grid(B, T, C, conv_rows(B, T, C)).y;
 }
 // partial: scratch of nsa_conv1d_bwd_parts(B, T, C) * 5 * C floats.  dw: [C][4]; db: [C] or null; both fp32
 // (dw_fp32 = 1) or bf16.
@@ -1196,8 +1223,15 @@ extern "C" int nsa_conv1d_bwd(const void* x, const void* w, const void* bias, co
                               void* dw, void* db, int dw_fp32, int B, int T, int C, long ldx, int width, int act, cudaStream_t st) {
   if (C % 8 || ldx % 8 || width != 4) return nsa::fail(NSA_ERR_SHAPE, "conv1d: channels multiple of 8 and width 4 required");
   const int rows = conv_rows(B, T, C);
-  dim3 grid((C + CT_C - 1) / CT_C, (T + CT_WARPS * rows - 1) / (CT_WARPS * rows), B);
-  conv1d_bwd_kernel<<<grid, CT_WARPS * 32, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (const bf16*)dy, (bf16*)dx,
+  const dim3 grid = conv_grid(B, T, C, rows);
+  static_assert(sizeof(ConvBwdSmem) >= CT_WARPS * 5 * CT_C * 4, "conv1d: reduction buffer");
+  static bool cfg = false;
+  if (!cfg) {
+    cudaError_t e = cudaFuncSetAttribute(conv1d_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ConvBwdSmem));
+    if (e != cudaSuccess) return nsa::fail_cuda(e, "conv1d_bwd: shared memory attribute");
+    cfg = true;
+  }
+  conv1d_bwd_kernel<<<grid, CT_WARPS * 32, sizeof(ConvBwdSmem), st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (const bf16*)dy, (bf16*)dx,
                                                     partial, T, C, ldx, act, rows);
   const int parts = static_cast<int>(nsa_conv1d_bwd_parts(B, T, C));
   if (dw_fp32) conv1d_dw_kernel<float><<<(C + 31) / 32, 256, 0, st>>>(partial, parts, C, (float*)dw, (float*)db);
