@@ -72,6 +72,8 @@ int nsa_sumsq_parts(void);
 int nsa_sumsq(const void* g, long n, int g_fp32, float* partial, float* out, int accumulate, cudaStream_t st);
 int nsa_cross_entropy(void* logits, const long* labels, float* loss_rows, const float* inv_count, long rows, int V,
                       long ld, long ignore_index, int write_grad, cudaStream_t st);
+/* dst (bf16) = src (fp32 or bf16) * (*scale); 16-byte aligned bases. */
+int nsa_scale_bf16(const void* src, void* dst, const float* scale, long n, int src_fp32, cudaStream_t st);
 
 /* ---- attention family: (B, T, H, D) bf16 tensors, L = log2-sum-exp per row (csrc/attention.cu) ---- */
 int nsa_attn_fwd(const void* q, const void* k, const void* v, void* o, float* L, int B, int T, int S, int Hq, int

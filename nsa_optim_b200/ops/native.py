@@ -794,7 +794,9 @@ class _LinearCE(torch.autograd.Function):
         inv = (1.0 / n_valid).reshape(1)
         loss_rows = _empty(N, dtype=torch.float32, device=hidden.device)
         dh = _empty_like(h) if need_h else None
-        dw = _zeros(V, d, dtype=torch.float32, device=hidden.device) if need_w else None
+        dw = None
+        if need_w:                                   # the first chunk's GEMM writes it whole
+            dw = (_empty if N > 0 else _zeros)(V, d, dtype=torch.float32, device=hidden.device)
         logits = _empty(min(chunk, N), V, dtype=torch.bfloat16, device=hidden.device)
         for s0 in range(0, N, chunk):
             s1 = min(N, s0 + chunk)
@@ -814,8 +816,18 @@ class _LinearCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gout):
         dh, dw = ctx.saved_tensors
-        return (None if dh is None else dh * gout.to(dh.dtype),
-                None if dw is None else (dw * gout).to(ctx.wdtype), None, None, None)
+        return (None if dh is None else _scaled_by(dh, gout.to(dh.dtype), dh.dtype),
+                None if dw is None else _scaled_by(dw, gout, ctx.wdtype), None, None, None)
+
+
+def _scaled_by(t: Tensor, s: Tensor, dtype: torch.dtype) -> Tensor:
+    """t * s rounded once to ``dtype``, s a one-element tensor: one pass for bf16 results."""
+    if dtype != torch.bfloat16 or t.dtype not in (torch.float32, torch.bfloat16) or not t.is_contiguous() or t.data_ptr() % 16:
+        return (t * s).to(dtype)
+    out = _empty(t.shape, dtype=dtype, device=t.device)
+    sf = s.reshape(1).float()
+    _check(load().nsa_scale_bf16(_p(t), _p(out), _p(sf), c_long(t.numel()), c_int(int(t.dtype == torch.float32)), _stream()))
+    return out
 
 
 def linear_cross_entropy(hidden, weight, labels, ignore_index=-100, chunk=4096):
