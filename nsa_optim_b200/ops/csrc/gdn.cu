@@ -6,7 +6,8 @@
 // cumulative log-decay gc from gdn_chunk.cu, and q, k as the caller has them:
 //     v_new   = u - w S                 o = sq (q S) + qk v_new            sq_i = scale e^gc_i
 //     S_next  = e^gc_last S + k^T (sk v_new)                               sk_i = e^(gc_last - gc_i)
-// One CTA owns one (head, 64-wide V tile) and walks the chunks in order.  The loop is one dependent
+// One CTA owns one (head, 64-wide V tile) and walks the chunks in order, two threads per accumulator row
+// (half the conversions in the chain: 256 instead of 128 threads).  The loop is one dependent
 // chain and there are fewer CTAs than SMs at the usual head counts, so its length is what a call
 // takes: row scalings are applied to accumulator rows in registers instead of to operands, the
 // output's part of a chunk (its second product, the read-back, the store) runs behind the
@@ -26,17 +27,19 @@ constexpr int VT = 64;    // V tile per CTA
 constexpr int CH = 64;    // chunk length
 constexpr int BOX = 8192; // bytes of one [64 rows][64 bf16] swizzled box
 
-__device__ __forceinline__ void write_row_swz(uint8_t* tile, int row, const uint32_t (&packed)[32]) {
+// A thread handles half a row: HC columns from column half * HC on.
+constexpr int HC = 32;
+__device__ __forceinline__ void write_half(uint8_t* tile, int row, int half, const uint32_t (&packed)[HC / 2]) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    uint4 v = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
-    *reinterpret_cast<uint4*>(tile + row * 128 + ((j ^ (row & 7)) << 4)) = v;
+  for (int j = 0; j < HC / 8; ++j) {
+    const uint4 v = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+    *reinterpret_cast<uint4*>(tile + row * 128 + (((half * (HC / 8) + j) ^ (row & 7)) << 4)) = v;
   }
 }
-__device__ __forceinline__ void read_row_swz(const uint8_t* tile, int row, float (&out)[64]) {
+__device__ __forceinline__ void read_half(const uint8_t* tile, int row, int half, float (&out)[HC]) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    uint4 v = *reinterpret_cast<const uint4*>(tile + row * 128 + ((j ^ (row & 7)) << 4));
+  for (int j = 0; j < HC / 8; ++j) {
+    const uint4 v = *reinterpret_cast<const uint4*>(tile + row * 128 + (((half * (HC / 8) + j) ^ (row & 7)) << 4));
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -46,41 +49,39 @@ __device__ __forceinline__ void read_row_swz(const uint8_t* tile, int row, float
     }
   }
 }
-__device__ __forceinline__ void load_row_global(const bf16* src, uint32_t (&packed)[32]) {
+__device__ __forceinline__ void load_global(const bf16* src, uint32_t (&packed)[HC / 2]) {
   const uint4* s4 = reinterpret_cast<const uint4*>(src);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    uint4 v = s4[j];
+  for (int j = 0; j < HC / 8; ++j) {
+    const uint4 v = s4[j];
     packed[4 * j] = v.x; packed[4 * j + 1] = v.y; packed[4 * j + 2] = v.z; packed[4 * j + 3] = v.w;
   }
 }
-__device__ __forceinline__ void unpack_row(const uint32_t (&packed)[32], float (&out)[64]) {
+__device__ __forceinline__ void unpack_half(const uint32_t (&packed)[HC / 2], float (&out)[HC]) {
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
+  for (int j = 0; j < HC / 2; ++j) {
     float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&packed[j]));
     out[2 * j] = f.x;
     out[2 * j + 1] = f.y;
   }
 }
-__device__ __forceinline__ void tmem_ld_row64(uint32_t taddr, float (&out)[64]) {
-  uint32_t a[32], b[32];
+__device__ __forceinline__ void tmem_ld_half(uint32_t taddr, float (&out)[HC]) {
+  uint32_t a[HC];
   tc5::tmem_ld_x32(taddr, a);
-  tc5::tmem_ld_x32(taddr + 32, b);
   tc5::tmem_ld_wait();
 #pragma unroll
-  for (int j = 0; j < 32; ++j) { out[j] = __uint_as_float(a[j]); out[32 + j] = __uint_as_float(b[j]); }
+  for (int j = 0; j < HC; ++j) out[j] = __uint_as_float(a[j]);
 }
-__device__ __forceinline__ void tmem_st_row64(uint32_t taddr, const float (&in)[64]) {
-  uint32_t a[32], b[32];
+__device__ __forceinline__ void tmem_st_half(uint32_t taddr, const float (&in)[HC]) {
+  uint32_t a[HC];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) { a[j] = __float_as_uint(in[j]); b[j] = __float_as_uint(in[32 + j]); }
+  for (int j = 0; j < HC; ++j) a[j] = __float_as_uint(in[j]);
   tc5::tmem_st_x32(taddr, a);
-  tc5::tmem_st_x32(taddr + 32, b);
   tc5::tmem_st_wait();
 }
-__device__ __forceinline__ void pack_row(const float (&in)[64], uint32_t (&packed)[32]) {
+__device__ __forceinline__ void pack_half(const float (&in)[HC], uint32_t (&packed)[HC / 2]) {
 #pragma unroll
-  for (int j = 0; j < 32; ++j) packed[j] = tc5::pack_bf16(in[2 * j], in[2 * j + 1]);
+  for (int j = 0; j < HC / 2; ++j) packed[j] = tc5::pack_bf16(in[2 * j], in[2 * j + 1]);
 }
 
 struct FwdParams {
@@ -97,7 +98,7 @@ constexpr int FWD_STAGE = 8 * BOX;
 constexpr int FWD_TX = 7 * BOX;                                                       // bytes that arrive per chunk
 constexpr int FWD_SMEM = 2 * FWD_STAGE + 2 * BOX /*Sb*/ + 2 * BOX /*Vb, Vs*/ + BOX /*Ob*/ + 1024 + 128;
 
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(256, 1)
 gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_qk,
                    const __grid_constant__ CUtensorMap tm_vn, const __grid_constant__ CUtensorMap tm_o,
@@ -116,12 +117,13 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int r = threadIdx.x;               // TMEM lane / tile row owned by this thread
-  const int warp = r >> 5;
+  const int r = threadIdx.x & 127, half = threadIdx.x >> 7;   // TMEM lane / tile row, half of its columns
+  const int warp = threadIdx.x >> 5;
+  const bool boss = threadIdx.x == 0;
   const int vt = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
   const int NC = p.NC, V = p.V;
 
-  if (r == 0) {
+  if (boss) {
     *abort_flag = 0;
     tc5::mbar_init(&full[0], 1);
     tc5::mbar_init(&full[1], 1);
@@ -133,32 +135,32 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   if (warp == 0) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
   // S = 0: bf16 mirror in shared memory; the constant zero half of both [0 ; qk] operands
   {
-    uint32_t z[32];
+    uint32_t z[HC / 2];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) z[j] = 0u;
-    write_row_swz(Sb, r, z);
-    write_row_swz(smem + (r >> 6) * FWD_STAGE + 6 * BOX, r & 63, z);
+    for (int j = 0; j < HC / 2; ++j) z[j] = 0u;
+    write_half(Sb, r, half, z);
+    write_half(smem + (r >> 6) * FWD_STAGE + 6 * BOX, r & 63, half, z);
   }
   tc5::fence_proxy_async();
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_off = static_cast<uint32_t>(warp * 32) << 16;
+  const uint32_t lane_off = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * HC;   // lanes and columns of this thread
   // TMEM columns: D1 = [w ; q] S [0, 64)   S [64, 128)   D2 = [0 ; qk] v_new [128, 192)
   const uint32_t cD1 = 0, cS = 64, cD2 = 128;
   {
-    float z[64];
+    float z[HC];
 #pragma unroll
-    for (int j = 0; j < 64; ++j) z[j] = 0.f;
-    tmem_st_row64(tmem + lane_off + cS, z);
+    for (int j = 0; j < HC; ++j) z[j] = 0.f;
+    tmem_st_half(tmem + lane_off + cS, z);
   }
   tc5::fence_before_sync();
   __syncthreads();
   // Outputs leave as TMA stores from the swizzled tiles they are in anyway.  Thread 0 stores v_new and the
   // state, thread 64 the output; each waits until its earlier store has read a tile before that tile is
   // rewritten.  Chunk 0 enters with the zero state that Sb holds now.
-  if (r == 0 && p.store_states) {
+  if (boss && p.store_states) {
     tc5::tma_store_2d(&tm_sa, Sb, vt * VT, bh * NC * KD);
     tc5::tma_store_commit();
   }
@@ -176,37 +178,37 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     }
     tc5::tma_load_2d(st + 7 * BOX, &tm_qk, &full[s], 0, row0);
   };
-  if (r == 0) issue_loads(0);
+  if (boss) issue_loads(0);
 
   constexpr uint32_t idesc1 = tc5::make_idesc_bf16(128, VT, 0, 1);   // A K-major, B MN-major
   constexpr uint32_t idesc2 = tc5::make_idesc_bf16(128, VT, 1, 1);   // A MN-major (k^T), B MN-major
   bool ok = true;
   // Global loads of the chain (u row, gates) are fetched one chunk ahead.
   const float* gc = p.gc + static_cast<long>(bh) * NC * CH;
-  uint32_t upk_next[32];
+  uint32_t upk_next[HC / 2];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) upk_next[j] = 0u;
-  if (r < CH) load_row_global(p.u + (static_cast<long>(bh * NC) * CH + r) * V + vt * VT, upk_next);
+  for (int j = 0; j < HC / 2; ++j) upk_next[j] = 0u;
+  if (r < CH) load_global(p.u + (static_cast<long>(bh * NC) * CH + r) * V + vt * VT + half * HC, upk_next);
   float gr_next = gc[r & 63], gl_next = gc[CH - 1];
-  float oi[64];                                    // sq (q S) of the chunk whose output is still open (rows 64..127)
+  float oi[HC];                                    // sq (q S) of the chunk whose output is still open (rows 64..127)
   // Output of chunk c: D2 joins oi; runs while the tensor core works on chunk c + 1.
   auto finish_output = [&](int c) {
     if (!tc5::mbar_wait(m3, c & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
     __syncwarp();
     tc5::fence_after_sync();
-    if (r < CH) return;                            // warps 2 and 3 stay together, also after a wait that gave up
-    float d2[64];
-    tmem_ld_row64(tmem + lane_off + cD2, d2);
+    if (r < CH) return;                            // the other warps stay together, also after a wait that gave up
+    float d2[HC];
+    tmem_ld_half(tmem + lane_off + cD2, d2);
 #pragma unroll
-    for (int j = 0; j < 64; ++j) d2[j] += oi[j];
-    uint32_t pk[32];
-    pack_row(d2, pk);
-    if (r == CH) tc5::tma_store_wait_read<0>();    // the previous output tile has been read
-    asm volatile("bar.sync 1, 64;" ::: "memory");
-    write_row_swz(Ob, r - CH, pk);
+    for (int j = 0; j < HC; ++j) d2[j] += oi[j];
+    uint32_t pk[HC / 2];
+    pack_half(d2, pk);
+    if (threadIdx.x == CH) tc5::tma_store_wait_read<0>();    // the previous output tile has been read
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    write_half(Ob, r - CH, half, pk);
     tc5::fence_proxy_async();
-    asm volatile("bar.sync 1, 64;" ::: "memory");
-    if (r == CH && ok) {                           // rows past T are clipped by the copy engine
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (threadIdx.x == CH && ok) {                           // rows past T are clipped by the copy engine
       tc5::tma_store_4d(&tm_o, Ob, vt * VT, h, c * CH, b);
       tc5::tma_store_commit();
     }
@@ -215,9 +217,9 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const int s = c & 1;
     uint8_t* st = smem + s * FWD_STAGE;
     const long row0 = static_cast<long>(bh * NC + c) * CH;
-    uint32_t upk[32];
+    uint32_t upk[HC / 2];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) upk[j] = upk_next[j];
+    for (int j = 0; j < HC / 2; ++j) upk[j] = upk_next[j];
     const float g_row = gr_next, g_last = gl_next;
     if (warp == 0) {
       // The issuing warp stays converged and one elected lane issues: descriptors then live in
@@ -239,43 +241,43 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     }
     // next chunk's u row (rows 0..63 only) and gates, in flight while this chunk computes
     if (c + 1 < NC) {
-      if (r < CH) load_row_global(p.u + (row0 + CH + r) * V + vt * VT, upk_next);
+      if (r < CH) load_global(p.u + (row0 + CH + r) * V + vt * VT + half * HC, upk_next);
       gr_next = gc[(c + 1) * CH + (r & 63)];
       gl_next = gc[(c + 1) * CH + CH - 1];
     }
     if (c > 0) finish_output(c - 1);
     // the stage of chunk c + 1 was last read by chunk c - 1's second group of MMAs, complete since finish_output
-    if (r == 0 && ok && c + 1 < NC) issue_loads(c + 1);
-    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous v_new tile has been read
+    if (boss && ok && c + 1 < NC) issue_loads(c + 1);
+    if (boss) tc5::tma_store_wait_read<1>();     // the previous v_new tile has been read
     if (ok && !tc5::mbar_wait(m1, c & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc5::fence_after_sync();
     {
-      float d1[64];
-      tmem_ld_row64(tmem + lane_off + cD1, d1);
+      float d1[HC];
+      tmem_ld_half(tmem + lane_off + cD1, d1);
       if (r < CH) {
-        float uf[64];
-        unpack_row(upk, uf);
+        float uf[HC];
+        unpack_half(upk, uf);
         const float sk = __expf(g_last - g_row);
-        uint32_t pk[32], ps[32];
+        uint32_t pk[HC / 2], ps[HC / 2];
 #pragma unroll
-        for (int j = 0; j < 64; ++j) d1[j] = uf[j] - d1[j];
-        pack_row(d1, pk);
+        for (int j = 0; j < HC; ++j) d1[j] = uf[j] - d1[j];
+        pack_half(d1, pk);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) d1[j] *= sk;
-        pack_row(d1, ps);
-        write_row_swz(Vb, r, pk);
-        write_row_swz(Vs, r, ps);
+        for (int j = 0; j < HC; ++j) d1[j] *= sk;
+        pack_half(d1, ps);
+        write_half(Vb, r, half, pk);
+        write_half(Vs, r, half, ps);
       } else {
         const float sq = p.scale * __expf(g_row);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) oi[j] = sq * d1[j];
+        for (int j = 0; j < HC; ++j) oi[j] = sq * d1[j];
       }
     }
     tc5::fence_proxy_async();
     tc5::fence_before_sync();
     __syncthreads();
-    if (r == 0 && p.store_states) {
+    if (boss && p.store_states) {
       tc5::tma_store_2d(&tm_vn, Vb, vt * VT, static_cast<int>(row0));
       tc5::tma_store_commit();
     }
@@ -296,32 +298,32 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       }
       __syncwarp();
     }
-    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous state tile has been read
+    if (boss) tc5::tma_store_wait_read<1>();     // the previous state tile has been read
     if (!tc5::mbar_wait(m2, c & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc5::fence_after_sync();
     if (c + 1 < NC) {
-      float sv[64];
-      tmem_ld_row64(tmem + lane_off + cS, sv);     // S entering chunk c+1, row r
-      uint32_t pk[32];
-      pack_row(sv, pk);
-      write_row_swz(Sb, r, pk);
+      float sv[HC];
+      tmem_ld_half(tmem + lane_off + cS, sv);     // S entering chunk c+1, row r
+      uint32_t pk[HC / 2];
+      pack_half(sv, pk);
+      write_half(Sb, r, half, pk);
       const float g = __expf(gl_next);             // its decay through chunk c + 1
 #pragma unroll
-      for (int j = 0; j < 64; ++j) sv[j] *= g;
-      tmem_st_row64(tmem + lane_off + cS, sv);
+      for (int j = 0; j < HC; ++j) sv[j] *= g;
+      tmem_st_half(tmem + lane_off + cS, sv);
       tc5::fence_proxy_async();
     }
     tc5::fence_before_sync();
     __syncthreads();
-    if (r == 0 && c + 1 < NC && p.store_states) {
+    if (boss && c + 1 < NC && p.store_states) {
       tc5::tma_store_2d(&tm_sa, Sb, vt * VT, (bh * NC + c + 1) * KD);
       tc5::tma_store_commit();
     }
   }
   if (ok) finish_output(NC - 1);
-  if (r == 0 || r == CH) tc5::tma_store_wait_read<0>();
-  if (!ok && r == 0) {
+  if (boss || threadIdx.x == CH) tc5::tma_store_wait_read<0>();
+  if (!ok && boss) {
     // a load for the next chunk may still be in flight: give it a bounded chance to land
     const long long t0 = clock64();
     for (int s = 0; s < 2; ++s)
@@ -349,7 +351,7 @@ constexpr int BWD_STAGE = 10 * BOX;                                        // 80
 constexpr int BWD_TX = 9 * BOX;
 constexpr int BWD_SMEM = 2 * BWD_STAGE + BOX /*du*/ + 2 * BOX /*do, sq do*/ + 2 * BOX /*dSb*/ + 1024 + 128;
 
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(256, 1)
 gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_S,
                    const __grid_constant__ CUtensorMap tm_qk, const __grid_constant__ CUtensorMap tm_du,
@@ -366,14 +368,15 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   uint64_t* m2 = bars + 3;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* red = reinterpret_cast<float*>(tmem_slot + 2);     // [4]
+  float* red = reinterpret_cast<float*>(tmem_slot + 2);     // [8]
 
-  const int r = threadIdx.x;
-  const int warp = r >> 5;
+  const int r = threadIdx.x & 127, half = threadIdx.x >> 7;
+  const int warp = threadIdx.x >> 5;
+  const bool boss = threadIdx.x == 0;
   const int vt = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
   const int NC = p.NC, V = p.V;
 
-  if (r == 0) {
+  if (boss) {
     *abort_flag = 0;
     tc5::mbar_init(&full[0], 1);
     tc5::mbar_init(&full[1], 1);
@@ -383,30 +386,30 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
   if (warp == 0) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
   {
-    uint32_t z[32];
+    uint32_t z[HC / 2];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) z[j] = 0u;
-    write_row_swz(dSb, r, z);
-    write_row_swz(smem + (r >> 6) * BWD_STAGE + 9 * BOX, r & 63, z);
+    for (int j = 0; j < HC / 2; ++j) z[j] = 0u;
+    write_half(dSb, r, half, z);
+    write_half(smem + (r >> 6) * BWD_STAGE + 9 * BOX, r & 63, half, z);
   }
   tc5::fence_proxy_async();
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_off = static_cast<uint32_t>(warp * 32) << 16;
+  const uint32_t lane_off = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * HC;   // lanes and columns of this thread
   // TMEM columns: Da = [k ; w] dS [0,64)   Dd = [qk^T ; 0] do [64,128)   dS [128,192)
   const uint32_t cDa = 0, cDd = 64, cDs = 128;
   {
-    float z[64];
+    float z[HC];
 #pragma unroll
-    for (int j = 0; j < 64; ++j) z[j] = 0.f;
-    tmem_st_row64(tmem + lane_off + cDs, z);
+    for (int j = 0; j < HC; ++j) z[j] = 0.f;
+    tmem_st_half(tmem + lane_off + cDs, z);
   }
   tc5::fence_before_sync();
   __syncthreads();
   // outputs leave as TMA stores from swizzled tiles (see the forward kernel); the last chunk's state has no gradient
-  if (r == 0) {
+  if (boss) {
     tc5::tma_store_2d(&tm_ds, dSb, vt * VT, (bh * NC + NC - 1) * KD);
     tc5::tma_store_commit();
   }
@@ -425,7 +428,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     tc5::tma_load_2d(st + 6 * BOX, &tm_S, &full[s], vt * VT, (bh * NC + c) * KD);
     tc5::tma_load_2d(st + 8 * BOX, &tm_qk, &full[s], 0, row0);
   };
-  if (r == 0) issue_loads(NC - 1, 0);
+  if (boss) issue_loads(NC - 1, 0);
 
   constexpr uint32_t id_a = tc5::make_idesc_bf16(128, VT, 0, 1);        // [k;w] (K-major) x dS (MN-major)
   constexpr uint32_t id_d = tc5::make_idesc_bf16(128, VT, 1, 1);        // q^T x (sq do), [qk^T ; 0] x do
@@ -433,18 +436,18 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   bool ok = true;
   // The chunk loop is one dependent chain: the do rows (threads 64..127) and the gates are fetched one chunk ahead.
   const float* gc = p.gc + static_cast<long>(bh) * NC * CH;
-  const bf16* d_o = p.d_o + (static_cast<long>(b) * p.T * p.H + h) * V + vt * VT;
-  uint32_t row_next[32];
+  const bf16* d_o = p.d_o + (static_cast<long>(b) * p.T * p.H + h) * V + vt * VT + half * HC;
+  uint32_t row_next[HC / 2];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) row_next[j] = 0u;
+  for (int j = 0; j < HC / 2; ++j) row_next[j] = 0u;
   float gr_next, gl_next;
   auto fetch_rows = [&](int cc) {
     const int t = cc * CH + r - CH;
     if (r >= CH) {
-      if (t < p.T) load_row_global(d_o + static_cast<long>(t) * p.H * V, row_next);
+      if (t < p.T) load_global(d_o + static_cast<long>(t) * p.H * V, row_next);
       else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) row_next[j] = 0u;
+        for (int j = 0; j < HC / 2; ++j) row_next[j] = 0u;
       }
     }
     gr_next = gc[cc * CH + (r & 63)];
@@ -459,15 +462,15 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const float g_row = gr_next, g_last = gl_next;
     // stage this chunk's do rows (already in registers) and start the next chunk's loads
     if (r >= CH) {
-      write_row_swz(sDO, r - CH, row_next);
-      float f[64];
-      unpack_row(row_next, f);
+      write_half(sDO, r - CH, half, row_next);
+      float f[HC];
+      unpack_half(row_next, f);
       const float sq = p.scale * __expf(g_row);
 #pragma unroll
-      for (int j = 0; j < 64; ++j) f[j] *= sq;
-      uint32_t pk[32];
-      pack_row(f, pk);
-      write_row_swz(sDOs, r - CH, pk);
+      for (int j = 0; j < HC; ++j) f[j] *= sq;
+      uint32_t pk[HC / 2];
+      pack_half(f, pk);
+      write_half(sDOs, r - CH, half, pk);
     }
     if (c > 0) fetch_rows(c - 1);
     tc5::fence_proxy_async();
@@ -495,35 +498,35 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       __syncwarp();
     }
     if (!tc5::mbar_wait(m1, it & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
-    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous du tile has been read (one newer store: the dS tile)
+    if (boss) tc5::tma_store_wait_read<1>();     // the previous du tile has been read (one newer store: the dS tile)
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc5::fence_after_sync();
     if (r < CH) {
-      float da[64], dd[64];
-      tmem_ld_row64(tmem + lane_off + cDa, da);
-      tmem_ld_row64(tmem + lane_off + cDd, dd);
+      float da[HC], dd[HC];
+      tmem_ld_half(tmem + lane_off + cDa, da);
+      tmem_ld_half(tmem + lane_off + cDd, dd);
       const float sk = __expf(g_last - g_row);
 #pragma unroll
-      for (int j = 0; j < 64; ++j) da[j] = dd[j] + sk * da[j];
-      uint32_t pk[32];
-      pack_row(da, pk);
-      write_row_swz(sDU, r, pk);
+      for (int j = 0; j < HC; ++j) da[j] = dd[j] + sk * da[j];
+      uint32_t pk[HC / 2];
+      pack_half(da, pk);
+      write_half(sDU, r, half, pk);
     }
     float part_dg = 0.f;
     {
       // dS: dgamma partial with S_prev, then scaled by gamma in place
-      float ds[64], sp[64];
-      tmem_ld_row64(tmem + lane_off + cDs, ds);
-      read_row_swz(st + 6 * BOX, r, sp);
+      float ds[HC], sp[HC];
+      tmem_ld_half(tmem + lane_off + cDs, ds);
+      read_half(st + 6 * BOX, r, half, sp);
       const float g = __expf(g_last);
 #pragma unroll
-      for (int j = 0; j < 64; ++j) { part_dg += ds[j] * sp[j]; ds[j] *= g; }
-      tmem_st_row64(tmem + lane_off + cDs, ds);
+      for (int j = 0; j < HC; ++j) { part_dg += ds[j] * sp[j]; ds[j] *= g; }
+      tmem_st_half(tmem + lane_off + cDs, ds);
     }
     tc5::fence_proxy_async();
     tc5::fence_before_sync();
     __syncthreads();
-    if (r == 0) {
+    if (boss) {
       tc5::tma_store_2d(&tm_du, sDU, vt * VT, static_cast<int>(row0));
       tc5::tma_store_commit();
     }
@@ -545,29 +548,30 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     }
     // block reduction of the dgamma partial, behind the MMAs
     for (int o = 16; o > 0; o >>= 1) part_dg += __shfl_xor_sync(0xffffffffu, part_dg, o);
-    if ((r & 31) == 0) red[warp] = part_dg;
-    if (r == 0) tc5::tma_store_wait_read<1>();     // the previous dS tile has been read
+    if ((threadIdx.x & 31) == 0) red[warp] = part_dg;
+    if (boss) tc5::tma_store_wait_read<1>();     // the previous dS tile has been read
     if (!tc5::mbar_wait(m2, it & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc5::fence_after_sync();
-    if (r == 0) p.dgamma_part[(static_cast<long>(vt) * p.BH + bh) * NC + c] = red[0] + red[1] + red[2] + red[3];
+    if (boss) p.dgamma_part[(static_cast<long>(vt) * p.BH + bh) * NC + c] =
+        ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
     if (c > 0) {
-      float ds[64];
-      tmem_ld_row64(tmem + lane_off + cDs, ds);
-      uint32_t pk[32];
-      pack_row(ds, pk);
-      write_row_swz(dSb, r, pk);
+      float ds[HC];
+      tmem_ld_half(tmem + lane_off + cDs, ds);
+      uint32_t pk[HC / 2];
+      pack_half(ds, pk);
+      write_half(dSb, r, half, pk);
     }
     tc5::fence_proxy_async();
     tc5::fence_before_sync();
     __syncthreads();
-    if (r == 0 && c > 0) {
+    if (boss && c > 0) {
       tc5::tma_store_2d(&tm_ds, dSb, vt * VT, (bh * NC + c - 1) * KD);
       tc5::tma_store_commit();
     }
   }
-  if (r == 0) tc5::tma_store_wait_read<0>();
-  if (!ok && r == 0) {
+  if (boss) tc5::tma_store_wait_read<0>();
+  if (!ok && boss) {
     const long long t0 = clock64();
     for (int s = 0; s < 2; ++s)
       for (uint32_t i = 0; i < (1u << 16); ++i) {
@@ -619,7 +623,7 @@ extern "C" int nsa_gdn_seq_fwd(const void* q, const void* k, const void* w, cons
   if (states && (rc = make_rows_map(&tsa, S_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
   FwdParams p{(const bf16*)u, gc, states, NC, V, H, scale, nsa::status_ptr()};
   if ((rc = set_smem(gdn_seq_fwd_kernel, FWD_SMEM, "gdn fwd smem attribute"))) return rc;
-  gdn_seq_fwd_kernel<<<dim3(V / VT, BH), 128, FWD_SMEM, st>>>(tw, tq, tk, tqk, tvn, to, tsa, p);
+  gdn_seq_fwd_kernel<<<dim3(V / VT, BH), 256, FWD_SMEM, st>>>(tw, tq, tk, tqk, tvn, to, tsa, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_seq_fwd launch");
@@ -644,7 +648,7 @@ extern "C" int nsa_gdn_seq_bwd(const void* q, const void* k, const void* w, cons
   if ((rc = make_rows_map(&tds, dS_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
   BwdParams p{(const bf16*)d_o, gc, dgamma_part, NC, V, BH, H, T, scale, nsa::status_ptr()};
   if ((rc = set_smem(gdn_seq_bwd_kernel, BWD_SMEM, "gdn bwd smem attribute"))) return rc;
-  gdn_seq_bwd_kernel<<<dim3(V / VT, BH), 128, BWD_SMEM, st>>>(tw, tq, tk, ts, tqk, tdu, tds, p);
+  gdn_seq_bwd_kernel<<<dim3(V / VT, BH), 256, BWD_SMEM, st>>>(tw, tq, tk, ts, tqk, tdu, tds, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_seq_bwd launch");

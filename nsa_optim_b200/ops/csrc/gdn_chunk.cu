@@ -8,6 +8,7 @@
 // q, k, v and the gates are read token-major as the caller has them, gradients leave the same way.
 #include "host.cuh"
 #include "mma16.cuh"
+#include "tc5.cuh"
 
 namespace {
 using namespace mma16;
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
   float* gs = reinterpret_cast<float*>(sTw + CH * PC);
   float* bs = gs + CH;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int c = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
+  const int bh = blockIdx.x, c = blockIdx.y, h = bh % p.H, b = bh / p.H;   // heads fastest: neighbouring pieces of token rows together
   const int t0 = c * CH;
   const long tok0 = static_cast<long>(b) * p.T * p.H + h;  // (b, t, h) = tok0 + t * H
   for (int i = tid; i < CH * (KD / 8); i += 256) {
@@ -214,70 +215,117 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
 }
 
 struct PostParams {
-  const bf16 *q, *k, *v, *d_o;          // [B, T, H, .]
+  const bf16 *q, *k;                    // [B, T, H, 128]
   const float* beta;                    // [B, T, H]
   const float *gc, *X;                  // [BH, NC, 64], [BH, NC, 64, 64]
-  const bf16 *v_new, *du;               // [BH, NC, 64, V]
-  const bf16 *S, *dS;                   // [BH, NC, 128, V]: state entering the chunk, gradient of the state leaving it
   const float* dgamma;                  // [V / 64, BH, NC]: <state entering, gradient of the state leaving> per V tile
   bf16 *dq, *dk, *dv;                   // [B, T, H, .]
   float *dg, *dbeta;                    // [B, T, H]
   int B, T, H, NC, V;
   float scale;
+  KernelStatus* status;
 };
 
-constexpr int POST_SLICE = (2 * KD + 4 * CH) * PC * 2;                     // S, dS, do, v_new, du, v: 64 columns each
-constexpr int POST_SMEM = 2 * CH * PK * 2 + 2 * POST_SLICE + CH * PX * 4 + CH * PC * 2 + (2 + 16) * CH * 4;
+// Stage: 64 columns of [du ; do], [v_new ; v] (128 rows each), S, dS, as 128-byte-swizzled TMA tiles.
+constexpr int TILE = 128 * 128;
+constexpr int POST_STAGE = 4 * TILE;
+constexpr int PF = KD + 4;                                                 // pitch of the fp32 [64][128] tiles
+constexpr int POST_SMEM = 2 * POST_STAGE + 2 * CH * PK * 2 + CH * PX * 4 + CH * PC * 2 + (2 + 16) * CH * 4 + 64 + 1024;
+static_assert(4 * CH * PX * 4 + CH * PK * 2 + 3 * CH * PC * 2 <= 2 * POST_STAGE, "gdn post: tail tiles");
+static_assert(2 * CH * PF * 4 <= 4 * CH * PX * 4, "gdn post: result tiles");
+
+// B fragments of 16 columns n0.. from a swizzled tile stored [k][64 n]
+__device__ __forceinline__ void load_b_t_swz(uint32_t (&r)[4], const uint8_t* tile, int n0, int k0) {
+  const int l = threadIdx.x & 31, i = l >> 3, row = k0 + (i & 1) * 8 + (l & 7), chunk = (n0 >> 3) + (i >> 1);
+  ldsm4_t(r, reinterpret_cast<const bf16*>(tile + row * 128 + ((chunk ^ (row & 7)) << 4)));
+}
+__device__ __forceinline__ float dot32(const float (&a)[32], const bf16* b) {
+  float s = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint4 u = *reinterpret_cast<const uint4*>(b + 8 * j);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = __bfloat1622float2(h[e]);
+      s += a[8 * j + 2 * e] * f.x + a[8 * j + 2 * e + 1] * f.y;
+    }
+  }
+  return s;
+}
+template <int N>
+__device__ __forceinline__ void tmem_cols(uint32_t taddr, float (&out)[N]) {
+  uint32_t a[N];
+  if constexpr (N == 32) tc5::tmem_ld_x32(taddr, a);
+  else tc5::tmem_ld_x16(taddr, a);
+  tc5::tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < N; ++j) out[j] = __uint_as_float(a[j]);
+}
 
 // One CTA of sixteen warps per (chunk, head): every gradient of the chunk once du (of the sequential pass) and
 // the two states are known.
 //     dw = -du S^T, dqs = do S^T, dks = v_new dS^T, dqk = do v_new^T, dTu = du v^T, dTw = dw k^T
 //     dX = (dTu + dTw e^gc) beta (columns), dA = -(X^T dX X^T), then through the definitions above.
-// The value dimension is walked in slices of 64 columns, the next one in flight; all products that sum over it
-// accumulate in registers.  Memory bound by design: 3.5 KB in and 1 KB out per token and head, against 6 KB
-// alone for the per-V-tile partials of dw, dq and dk that the sequential pass would have to write and re-read.
-__global__ void __launch_bounds__(512, 1) gdn_post_kernel(const PostParams p) {
-  extern __shared__ __align__(16) uint8_t smem_raw[];
-  bf16* sK = reinterpret_cast<bf16*>(smem_raw);
+// The five products that sum over the value dimension are three full tcgen05 tiles of the stacked operands,
+// [du ; do] S^T, [v_new ; v] dS^T and [du ; do] [v_new ; v]^T, accumulated in tensor memory while slices of 64 value
+// columns stream through two TMA stages (as warp products with register accumulators they were two thirds of the
+// kernel: 700 us at 16384 tokens x 16 heads).  What is left are 64-row products, done by warps.  Per token and head
+// 3.5 KB come in and 1 KB goes out, against 6 KB alone for the per-V-tile partials of dw, dq and dk that the sequential
+// pass would otherwise write and re-read.
+__global__ void __launch_bounds__(512, 1)
+gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant__ CUtensorMap tm_do,
+                const __grid_constant__ CUtensorMap tm_vn, const __grid_constant__ CUtensorMap tm_v,
+                const __grid_constant__ CUtensorMap tm_S, const __grid_constant__ CUtensorMap tm_dS, const PostParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  bf16* sK = reinterpret_cast<bf16*>(stages + 2 * POST_STAGE);
   bf16* sQ = sK + CH * PK;
-  uint8_t* slices = reinterpret_cast<uint8_t*>(sQ + CH * PK);
-  float* Xs = reinterpret_cast<float*>(slices + 2 * POST_SLICE);
+  float* Xs = reinterpret_cast<float*>(sQ + CH * PK);
   bf16* sTu = reinterpret_cast<bf16*>(Xs + CH * PX);
   float* gs = reinterpret_cast<float*>(sTu + CH * PC);
   float* bs = gs + CH;
   float* red = bs + CH;                                    // [16][64]
-  // over the slices once they are done
-  bf16* sW = reinterpret_cast<bf16*>(slices);              // dw   [64][PK]
-  float* sDX = reinterpret_cast<float*>(sW + CH * PK);     // [64][PX], later dA
-  float* sY = sDX + CH * PX;                               // [64][PX]
-  bf16* sTw = reinterpret_cast<bf16*>(sY + CH * PX);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(red + 16 * CH);
+  uint64_t *full = bars, *done = bars + 2;                 // [2] each
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  // over the stages once they are done
+  float* sDX = reinterpret_cast<float*>(stages);           // [64][PX], later dA
+  float* sY = sDX + CH * PX;
+  float* sT = sY + CH * PX;                                // dTu
+  float* sP = sT + CH * PX;                                // dqk
+  float* sFQ = sDX;                                        // [64][PF] over the four above, at the very end
+  float* sFK = sFQ + CH * PF;
+  bf16* sW = reinterpret_cast<bf16*>(sP + CH * PX);        // dw [64][PK]
+  bf16* sTw = sW + CH * PK;
   bf16* sDK = sTw + CH * PC;                               // d(k k^T)
   bf16* sDQ = sDK + CH * PC;                               // d(q k^T)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int c = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
+  const int bh = blockIdx.x, c = blockIdx.y, h = bh % p.H, b = bh / p.H;   // heads fastest: neighbouring pieces of token rows together
   const int t0 = c * CH, V = p.V, nvt = V / CH;
   const long tok0 = static_cast<long>(b) * p.T * p.H + h;
   const long chunk = static_cast<long>(bh) * p.NC + c;
-  auto load_slice = [&](int s) {
-    bf16* d = reinterpret_cast<bf16*>(slices + (s & 1) * POST_SLICE);
-    for (int i = tid; i < KD * 8; i += 512) {
-      const int r = i >> 3, cc = (i & 7) * 8;
-      const long off = (chunk * KD + r) * V + s * CH + cc;
-      cp_async16(d + r * PC + cc, p.S + off, true);
-      cp_async16(d + (KD + r) * PC + cc, p.dS + off, true);
-    }
-    d += 2 * KD * PC;
-    for (int i = tid; i < CH * 8; i += 512) {
-      const int r = i >> 3, cc = (i & 7) * 8, t = t0 + r;
-      const bool ok = t < p.T;
-      const long tm = (tok0 + static_cast<long>(ok ? t : 0) * p.H) * V + s * CH + cc, cm = (chunk * CH + r) * V + s * CH + cc;
-      cp_async16(d + r * PC + cc, p.d_o + tm, ok);
-      cp_async16(d + (CH + r) * PC + cc, p.v_new + cm, true);
-      cp_async16(d + (2 * CH + r) * PC + cc, p.du + cm, true);
-      cp_async16(d + (3 * CH + r) * PC + cc, p.v + tm, ok);
-    }
-    cp_async_commit();
+  auto load_slice = [&](int s) {                           // one thread
+    uint8_t* d = stages + (s & 1) * POST_STAGE;
+    uint64_t* bar = full + (s & 1);
+    const int row = static_cast<int>(chunk) * CH, x = s * CH;
+    tc5::mbar_expect_tx(bar, POST_STAGE);
+    tc5::tma_load_2d(d, &tm_du, bar, x, row);
+    tc5::tma_load_4d(d + TILE / 2, &tm_do, bar, x, h, t0, b);
+    tc5::tma_load_2d(d + TILE, &tm_vn, bar, x, row);
+    tc5::tma_load_4d(d + TILE + TILE / 2, &tm_v, bar, x, h, t0, b);
+    tc5::tma_load_2d(d + 2 * TILE, &tm_S, bar, x, static_cast<int>(chunk) * KD);
+    tc5::tma_load_2d(d + 3 * TILE, &tm_dS, bar, x, static_cast<int>(chunk) * KD);
   };
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < 2; ++i) { tc5::mbar_init(full + i, 1); tc5::mbar_init(done + i, 1); }
+    tc5::fence_barrier_init();
+    load_slice(0);
+    if (nvt > 1) load_slice(1);
+  }
+  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 512); tc5::tmem_relinquish(); }
   for (int i = tid; i < CH * (KD / 8); i += 512) {
     const int r = i / (KD / 8), cc = (i % (KD / 8)) * 8, t = t0 + r;
     const bool ok = t < p.T;
@@ -285,54 +333,63 @@ __global__ void __launch_bounds__(512, 1) gdn_post_kernel(const PostParams p) {
     cp_async16(sK + r * PK + cc, p.k + off, ok);
     cp_async16(sQ + r * PK + cc, p.q + off, ok);
   }
-  load_slice(0);
+  cp_async_commit();
   if (tid < CH) {
     gs[tid] = p.gc[chunk * CH + tid];
     bs[tid] = t0 + tid < p.T ? p.beta[tok0 + static_cast<long>(t0 + tid) * p.H] : 0.f;
   }
+  tc5::fence_before_sync();
   __syncthreads();
+  tc5::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
   for (int i = tid; i < CH * CH / 4; i += 512) {
     const int r = i / (CH / 4), j = (i % (CH / 4)) * 4;
     const float4 x = *reinterpret_cast<const float4*>(p.X + (chunk * CH + r) * CH + j);
     *reinterpret_cast<float4*>(Xs + r * PX + j) = x;
     *reinterpret_cast<uint2*>(sTu + r * PC + j) = make_uint2(pack2(x.x * bs[j], x.y * bs[j + 1]), pack2(x.z * bs[j + 2], x.w * bs[j + 3]));
   }
+  cp_async_wait<0>();
+  __syncthreads();
+  // fragment view of warp products: rows m0.., 32 (of 128) or 16 (of 64) columns
   const int m0 = (warp & 3) * 16, n32 = (warp >> 2) * 32, n16 = (warp >> 2) * 16;
   const int r0 = m0 + (lane >> 2), cl = 2 * (lane & 3);    // first row and column offset of this lane's accumulator elements
-  float aW[4][4] = {}, aQ[4][4] = {}, aK[4][4] = {}, aP[2][4] = {}, aT[2][4] = {};
+  // tensor-memory view: lane row (0..63 the upper operand of a stack, 64..127 the lower), 32 columns from n32
+  const int row = (warp & 3) * 32 + lane, ri = row & 63;
+  const bool upper = row < CH;                             // uniform in a warp
+  const uint32_t trow = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  constexpr uint32_t cWQ = 0, cKS = 128, cPT = 256;        // accumulator columns of the three products
+  constexpr uint32_t idesc = tc5::make_idesc_bf16(128, 128, 0, 0);
+  bool ok = true;
   for (int s = 0; s < nvt; ++s) {
-    if (s + 1 < nvt) { load_slice(s + 1); cp_async_wait<1>(); }
-    else cp_async_wait<0>();
-    __syncthreads();
-    const bf16* tS = reinterpret_cast<const bf16*>(slices + (s & 1) * POST_SLICE);
-    const bf16 *tD = tS + KD * PC, *tO = tD + KD * PC, *tN = tO + CH * PC, *tU = tN + CH * PC, *tV = tU + CH * PC;
+    const uint8_t* st = stages + (s & 1) * POST_STAGE;
+    if (!tc5::mbar_wait(full + (s & 1), (s >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL)) ok = false;
+    if (__syncthreads_or(!ok)) { ok = false; break; }
+    if (warp == 0) {
+      const bool lead = tc5::elect_one();                  // converged warp, elected lane issues
+      tc5::fence_after_sync();
+      const uint64_t uo = tc5::desc_kmajor(tc5::smem_u32(st)), nv = tc5::desc_kmajor(tc5::smem_u32(st + TILE));
+      const uint64_t S = tc5::desc_kmajor(tc5::smem_u32(st + 2 * TILE)), dS = tc5::desc_kmajor(tc5::smem_u32(st + 3 * TILE));
+      if (lead) {
 #pragma unroll
-    for (int kk = 0; kk < CH; kk += 16) {
-      uint32_t au[4], ao[4], an[4], bb[4];
-      load_a(au, tU, PC, m0, kk);
-      load_a(ao, tO, PC, m0, kk);
-      load_a(an, tN, PC, m0, kk);
-#pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        load_b(bb, tS, PC, n32 + n * 16, kk);
-        mma2(aW[2 * n], aW[2 * n + 1], au, bb);
-        mma2(aQ[2 * n], aQ[2 * n + 1], ao, bb);
-        load_b(bb, tD, PC, n32 + n * 16, kk);
-        mma2(aK[2 * n], aK[2 * n + 1], an, bb);
+        for (int kk = 0; kk < CH / 16; ++kk) {
+          const uint64_t off = static_cast<uint64_t>((kk * 32) >> 4);
+          const uint32_t acc = s > 0 || kk > 0 ? 1u : 0u;
+          tc5::mma_ss(tmem + cWQ, uo + off, S + off, idesc, acc);
+          tc5::mma_ss(tmem + cKS, nv + off, dS + off, idesc, acc);
+          tc5::mma_ss(tmem + cPT, uo + off, nv + off, idesc, acc);
+        }
+        tc5::mma_commit(done + (s & 1));
       }
-      load_b(bb, tN, PC, n16, kk);
-      mma2(aP[0], aP[1], ao, bb);
-      load_b(bb, tV, PC, n16, kk);
-      mma2(aT[0], aT[1], au, bb);
+      __syncwarp();
     }
-    // dv of this slice: Tu^T du (row j needs i >= j only)
+    // dv of this slice behind the MMAs: Tu^T du (row j needs i >= j only)
     float dv[2][4] = {};
 #pragma unroll
     for (int kk = 0; kk < CH; kk += 16) {
       if (kk < m0) continue;
       uint32_t a[4], bb[4];
       load_a_t(a, sTu, PC, m0, kk);
-      load_b_t(bb, tU, PC, n16, kk);
+      load_b_t_swz(bb, st, n16, kk);
       mma2(dv[0], dv[1], a, bb);
     }
 #pragma unroll
@@ -343,37 +400,53 @@ __global__ void __launch_bounds__(512, 1) gdn_post_kernel(const PostParams p) {
 #pragma unroll
       for (int n = 0; n < 2; ++n) *reinterpret_cast<uint32_t*>(dst + n * 8) = pack2(dv[n][2 * hh], dv[n][2 * hh + 1]);
     }
-    __syncthreads();                                       // the slice's buffer is refilled two slices on
+    if (s + 2 < nvt) {
+      __syncthreads();                                     // du of this stage has been read by every warp
+      if (tid == 0) {
+        if (tc5::mbar_wait(done + (s & 1), (s >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) load_slice(s + 2);
+        else ok = false;
+      }
+    }
   }
+  // the last two commits cover every product
+  if (ok) {
+    const int s = nvt - 1;
+    if (!tc5::mbar_wait(done + (s & 1), (s >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
+  }
+  if (__syncthreads_or(!ok)) {
+    if (tid == 0) {                                        // copies in flight get a bounded chance to land
+      const long long start = clock64();
+      for (int s = 0; s < 2; ++s)
+        while (!tc5::mbar_try_wait(full + s, 0) && !tc5::mbar_try_wait(full + s, 1) && clock64() - start < tc5::kMaxWaitCycles) {}
+    }
+    __syncthreads();
+    if (warp == 0) tc5::tmem_dealloc(tmem, 512);
+    return;
+  }
+  tc5::fence_after_sync();
   const float g_last = gs[CH - 1];
-  // ---- dw as an operand; row sums q . dqs and k . dks (gates that scale rows of q and k); Tw
+  // ---- out of tensor memory: dw as an operand, dTu and dqk as fp32 tiles, and the row sums q . dqs and k . dks (gates
+  //      that scale rows of q and k); dqs and dks stay where they are until the end
+  {
+    float a[32], t16[16];
+    tmem_cols(trow + cWQ + n32, a);
+    float dot;
+    if (upper) {
 #pragma unroll
-  for (int hh = 0; hh < 2; ++hh) {
-    const int i = r0 + 8 * hh;
-    float dq_s = 0.f, dk_s = 0.f;
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<uint4*>(sW + ri * PK + n32 + 8 * j) =
+            make_uint4(pack2(-a[8 * j], -a[8 * j + 1]), pack2(-a[8 * j + 2], -a[8 * j + 3]), pack2(-a[8 * j + 4], -a[8 * j + 5]),
+                       pack2(-a[8 * j + 6], -a[8 * j + 7]));
+      tmem_cols(trow + cKS + n32, a);
+      dot = dot32(a, sK + ri * PK + n32);
+    } else {
+      dot = dot32(a, sQ + ri * PK + n32);
+    }
+    red[((upper ? 4 : 0) + (warp >> 2)) * CH + ri] = dot;
+    tmem_cols(trow + cPT + (upper ? CH : 0) + n16, t16);
+    float* dst = (upper ? sT : sP) + ri * PX + n16;
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int j = n32 + n * 8 + cl;
-      *reinterpret_cast<uint32_t*>(sW + i * PK + j) = pack2(-aW[n][2 * hh], -aW[n][2 * hh + 1]);
-      const float2 qv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sQ + i * PK + j));
-      const float2 kv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sK + i * PK + j));
-      dq_s += aQ[n][2 * hh] * qv.x + aQ[n][2 * hh + 1] * qv.y;
-      dk_s += aK[n][2 * hh] * kv.x + aK[n][2 * hh + 1] * kv.y;
-    }
-    dq_s += __shfl_xor_sync(0xffffffffu, dq_s, 1);
-    dk_s += __shfl_xor_sync(0xffffffffu, dk_s, 1);
-    dq_s += __shfl_xor_sync(0xffffffffu, dq_s, 2);
-    dk_s += __shfl_xor_sync(0xffffffffu, dk_s, 2);
-    if ((lane & 3) == 0) {
-      red[(warp >> 2) * CH + i] = dq_s;
-      red[(4 + (warp >> 2)) * CH + i] = dk_s;
-    }
-    const float sq = p.scale * __expf(gs[i]), sk = __expf(g_last - gs[i]);
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      aQ[n][2 * hh] *= sq; aQ[n][2 * hh + 1] *= sq;
-      aK[n][2 * hh] *= sk; aK[n][2 * hh + 1] *= sk;
-    }
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(dst + 4 * j) = make_float4(t16[4 * j], t16[4 * j + 1], t16[4 * j + 2], t16[4 * j + 3]);
   }
   for (int i = tid; i < CH * CH / 4; i += 512) {
     const int r = i / (CH / 4), j = (i % (CH / 4)) * 4;
@@ -413,7 +486,7 @@ __global__ void __launch_bounds__(512, 1) gdn_post_kernel(const PostParams p) {
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           const int i = r0 + 8 * hh;
-          const float x = Xs[i * PX + j], tw = aw[n][2 * hh + e] * eg, d = aT[n][2 * hh + e] + tw;
+          const float x = Xs[i * PX + j], tw = aw[n][2 * hh + e] * eg, d = sT[i * PX + j] + tw;
           sDX[i * PX + j] = j <= i ? d * bj : 0.f;
           cb += d * x;                                     // x is zero above the diagonal
           cg += tw * x;
@@ -495,7 +568,7 @@ __global__ void __launch_bounds__(512, 1) gdn_post_kernel(const PostParams p) {
           const float d = j < i ? sDX[i * PX + j] : 0.f;
           const float araw = kk_[n][2 * hh + e] * ex;
           ok[e] = d * bi * ex;
-          oq[e] = j <= i ? aP[n][2 * hh + e] * p.scale * ex : 0.f;
+          oq[e] = j <= i ? sP[i * PX + j] * p.scale * ex : 0.f;
           const float t = d * bi * araw + oq[e] * qk_[n][2 * hh + e];
           rb += d * araw;
           rg += t;
@@ -536,43 +609,59 @@ __global__ void __launch_bounds__(512, 1) gdn_post_kernel(const PostParams p) {
     if (t0 + tid < p.T) p.dbeta[tok0 + static_cast<long>(t0 + tid) * p.H] = dbeta;
   }
   // ---- dq = sq dqs + dqkr k;  dk = sk dks + dkk k + dkk^T k + dqkr^T q + Tw^T dw
+  {
+    float aQ[4][4] = {}, aK[4][4] = {};
 #pragma unroll
-  for (int kk = 0; kk < CH; kk += 16) {
-    uint32_t a1[4], a2[4], a3[4], a4[4], a5[4];
-    load_a(a1, sDQ, PC, m0, kk);
-    load_a(a2, sDK, PC, m0, kk);
-    load_a_t(a3, sDK, PC, m0, kk);
-    load_a_t(a4, sDQ, PC, m0, kk);
-    load_a_t(a5, sTw, PC, m0, kk);
+    for (int kk = 0; kk < CH; kk += 16) {
+      uint32_t a1[4], a2[4], a3[4], a4[4], a5[4];
+      load_a(a1, sDQ, PC, m0, kk);
+      load_a(a2, sDK, PC, m0, kk);
+      load_a_t(a3, sDK, PC, m0, kk);
+      load_a_t(a4, sDQ, PC, m0, kk);
+      load_a_t(a5, sTw, PC, m0, kk);
 #pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      uint32_t bb[4];
-      load_b_t(bb, sK, PK, n32 + n * 16, kk);
-      mma2(aQ[2 * n], aQ[2 * n + 1], a1, bb);
-      mma2(aK[2 * n], aK[2 * n + 1], a2, bb);
-      mma2(aK[2 * n], aK[2 * n + 1], a3, bb);
-      load_b_t(bb, sQ, PK, n32 + n * 16, kk);
-      mma2(aK[2 * n], aK[2 * n + 1], a4, bb);
-      load_b_t(bb, sW, PK, n32 + n * 16, kk);
-      mma2(aK[2 * n], aK[2 * n + 1], a5, bb);
+      for (int n = 0; n < 2; ++n) {
+        uint32_t bb[4];
+        load_b_t(bb, sK, PK, n32 + n * 16, kk);
+        mma2(aQ[2 * n], aQ[2 * n + 1], a1, bb);
+        mma2(aK[2 * n], aK[2 * n + 1], a2, bb);
+        mma2(aK[2 * n], aK[2 * n + 1], a3, bb);
+        load_b_t(bb, sQ, PK, n32 + n * 16, kk);
+        mma2(aK[2 * n], aK[2 * n + 1], a4, bb);
+        load_b_t(bb, sW, PK, n32 + n * 16, kk);
+        mma2(aK[2 * n], aK[2 * n + 1], a5, bb);
+      }
     }
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const int o = (r0 + 8 * hh) * PF + n32 + n * 8 + cl;
+        *reinterpret_cast<float2*>(sFQ + o) = make_float2(aQ[n][2 * hh], aQ[n][2 * hh + 1]);
+        *reinterpret_cast<float2*>(sFK + o) = make_float2(aK[n][2 * hh], aK[n][2 * hh + 1]);
+      }
   }
   __syncthreads();                                         // the tiles of q and k become those of dq and dk
+  {
+    float a[32];
+    tmem_cols(trow + (upper ? cKS : cWQ) + n32, a);
+    const float sc = upper ? __expf(g_last - gs[ri]) : p.scale * __expf(gs[ri]);
+    const float* add = (upper ? sFK : sFQ) + ri * PF + n32;
+    bf16* dst = (upper ? sK : sQ) + ri * PK + n32;
 #pragma unroll
-  for (int hh = 0; hh < 2; ++hh)
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int o = (r0 + 8 * hh) * PK + n32 + n * 8 + cl;
-      *reinterpret_cast<uint32_t*>(sQ + o) = pack2(aQ[n][2 * hh], aQ[n][2 * hh + 1]);
-      *reinterpret_cast<uint32_t*>(sK + o) = pack2(aK[n][2 * hh], aK[n][2 * hh + 1]);
+    for (int j = 0; j < 8; ++j) {
+      const float4 f = *reinterpret_cast<const float4*>(add + 4 * j);
+      *reinterpret_cast<uint2*>(dst + 4 * j) = make_uint2(pack2(sc * a[4 * j] + f.x, sc * a[4 * j + 1] + f.y),
+                                                          pack2(sc * a[4 * j + 2] + f.z, sc * a[4 * j + 3] + f.w));
     }
+  }
   // ---- d g_t: sum of d gc_i over i >= t; the chunk's last gc also carries the decay of the state and of k
   if (warp == 0) {
     float l2 = red[13 * CH + 2 * lane] + red[13 * CH + 2 * lane + 1];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l2 += __shfl_xor_sync(0xffffffffu, l2, o);
     float dgam = 0.f;
-    for (int s = 0; s < nvt; ++s) dgam += p.dgamma[(static_cast<long>(s) * gridDim.y + bh) * p.NC + c];
+    for (int s = 0; s < nvt; ++s) dgam += p.dgamma[(static_cast<long>(s) * gridDim.x + bh) * p.NC + c];
     l2 += dgam * __expf(g_last);
     const float a = red[12 * CH + 2 * lane], bq = red[12 * CH + 2 * lane + 1] + (lane == 31 ? l2 : 0.f);
     float s = a + bq;
@@ -585,6 +674,7 @@ __global__ void __launch_bounds__(512, 1) gdn_post_kernel(const PostParams p) {
     if (ta < p.T) p.dg[tok0 + static_cast<long>(ta) * p.H] = s;
     if (ta + 1 < p.T) p.dg[tok0 + static_cast<long>(ta + 1) * p.H] = s - a;
   }
+  tc5::fence_before_sync();
   __syncthreads();
   for (int i = tid; i < CH * (KD / 8); i += 512) {
     const int r = i / (KD / 8), cc = (i % (KD / 8)) * 8, t = t0 + r;
@@ -593,6 +683,7 @@ __global__ void __launch_bounds__(512, 1) gdn_post_kernel(const PostParams p) {
     *reinterpret_cast<uint4*>(p.dq + off) = *reinterpret_cast<const uint4*>(sQ + r * PK + cc);
     *reinterpret_cast<uint4*>(p.dk + off) = *reinterpret_cast<const uint4*>(sK + r * PK + cc);
   }
+  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 512); }
 }
 }  // namespace
 
@@ -606,7 +697,7 @@ extern "C" int nsa_gdn_prep(const void* q, const void* k, const void* v, const f
   const int smem = 2 * CH * PK * 2 + CH * (V + 8) * 2 + 2 * CH * PX * 4 + 2 * CH * PC * 2 + 2 * CH * 4;
   cudaError_t e = cudaFuncSetAttribute(gdn_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn prep smem attribute");
-  gdn_prep_kernel<<<dim3(NC, B * H), 256, smem, st>>>(p);
+  gdn_prep_kernel<<<dim3(B * H, NC), 256, smem, st>>>(p);
   nsa::count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_prep launch");
@@ -619,11 +710,26 @@ extern "C" int nsa_gdn_post(const void* q, const void* k, const void* v, const v
                             int K, int V, float scale, cudaStream_t st) {
   if (K != KD || V % 64) return nsa::fail(NSA_ERR_SHAPE, "gdn: key width must be 128 and value width a multiple of 64");
   const int NC = (T + CH - 1) / CH;
-  PostParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, (const bf16*)d_o, beta, gc, X, (const bf16*)v_new, (const bf16*)du,
-               (const bf16*)S, (const bf16*)dS, dgamma, (bf16*)dq, (bf16*)dk, (bf16*)dv, dg, dbeta, B, T, H, NC, V, scale};
+  const long chunks = static_cast<long>(B) * H * NC;
+  CUtensorMap tdu, tdo, tvn, tv, tS, tdS;
+  int rc;
+  auto token_map = [&](CUtensorMap* m, const void* base) {
+    const uint64_t dims[4] = {(uint64_t)V, (uint64_t)H, (uint64_t)T, (uint64_t)B};
+    const uint64_t strides[3] = {(uint64_t)V * 2, (uint64_t)H * V * 2, (uint64_t)T * H * V * 2};
+    const uint32_t box[4] = {64, 1, (uint32_t)CH, 1};
+    return nsa::make_tmap_bf16(m, base, 4, dims, strides, box, 1);
+  };
+  if ((rc = nsa::make_tmap_2d_bf16(&tdu, du, V, chunks * CH, V, 64, CH))) return rc;
+  if ((rc = token_map(&tdo, d_o))) return rc;
+  if ((rc = nsa::make_tmap_2d_bf16(&tvn, v_new, V, chunks * CH, V, 64, CH))) return rc;
+  if ((rc = token_map(&tv, v))) return rc;
+  if ((rc = nsa::make_tmap_2d_bf16(&tS, S, V, chunks * KD, V, 64, KD))) return rc;
+  if ((rc = nsa::make_tmap_2d_bf16(&tdS, dS, V, chunks * KD, V, 64, KD))) return rc;
+  PostParams p{(const bf16*)q, (const bf16*)k, beta, gc, X, dgamma, (bf16*)dq, (bf16*)dk, (bf16*)dv, dg, dbeta, B, T, H, NC, V, scale,
+               nsa::status_ptr()};
   cudaError_t e = cudaFuncSetAttribute(gdn_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, POST_SMEM);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn post smem attribute");
-  gdn_post_kernel<<<dim3(NC, B * H), 512, POST_SMEM, st>>>(p);
+  gdn_post_kernel<<<dim3(B * H, NC), 512, POST_SMEM, st>>>(tdu, tdo, tvn, tv, tS, tdS, p);
   nsa::count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_post launch");
