@@ -214,9 +214,8 @@ class HybridModel(CausalLMBase):
 
     def forward(self, input_ids: Tensor, attention_mask: Optional[Tensor] = None,
                 labels: Optional[Tensor] = None, position_ids: Optional[Tensor] = None, **_):
-        T = input_ids.shape[1]
-        if position_ids is None:
-            position_ids = torch.arange(T, device=input_ids.device)
+        # without position_ids the rotary tables are sliced by length: explicit ids cost each attention block a
+        # device synchronisation (their maximum) and two gathers
         h = self.embed_tokens(input_ids)
         for layer in self.layers:
             h = self.run_layer(layer, h, attention_mask, position_ids)

@@ -221,7 +221,7 @@ class TransformerModel(CausalLMBase):
                 labels: Optional[Tensor] = None, use_cache: bool = False):
         B, T = input_ids.shape
         past_len = 0 if past_key_values is None else past_key_values[0][0].shape[1]
-        if position_ids is None:
+        if position_ids is None and past_len > 0:    # from position 0 the rotary tables are sliced by length
             position_ids = torch.arange(past_len, past_len + T, device=input_ids.device)
         h = self.embed_tokens(input_ids)
         caches = [] if use_cache else None

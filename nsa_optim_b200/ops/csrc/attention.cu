@@ -191,7 +191,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int r = tid & 127, ch = tid >> 7;
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
   const int q0 = qt * p.R;
   const int tok_local = r / p.G, g = r % p.G;
   const int t = q0 + tok_local;
@@ -478,7 +478,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -831,7 +831,7 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -1058,7 +1058,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -1368,7 +1368,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int r = tid & 127, ch = tid >> 7;
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
   const int q0 = qt * p.R;
   const int tok_local = r / p.G, g = r % p.G;
   const int t = q0 + tok_local;
@@ -1614,7 +1614,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -1918,7 +1918,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -2571,21 +2571,37 @@ __global__ void __launch_bounds__(256) nsa_select_kernel(const float* __restrict
 // --------------------------------------------------------------------------------------
 // Helper kernels
 // --------------------------------------------------------------------------------------
-// delta[row] = sum_d dO[row, d] * O[row, d]; one warp per row.
+// delta[row] = sum_d dO[row, d] * O[row, d].  D / 8 lanes share a row and load 16 bytes each (4-byte loads kept
+// too little in flight: 74 us for 512 K rows of 128, 40 us of memory traffic).
+template <int D>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const bf16* __restrict__ O, const bf16* __restrict__ dO,
-                                                         float* __restrict__ delta, long rows, int D) {
-  const long row = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  float s = 0.f;
-  for (int c = lane * 2; c < D; c += 64) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(O + row * D + c));
-    const float2 d = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dO + row * D + c));
-    s += a.x * d.x + a.y * d.y;
+                                                         float* __restrict__ delta, long rows) {
+  constexpr int LANES = D / 8, U = 2;               // U rows per group of lanes, loads first
+  const long group = (static_cast<long>(blockIdx.x) * 256 + threadIdx.x) / LANES;
+  const int c = (threadIdx.x % LANES) * 8;
+  uint4 a[U], d[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long row = group * U + u;
+    a[u] = d[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (row < rows) {
+      a[u] = *reinterpret_cast<const uint4*>(O + row * D + c);
+      d[u] = *reinterpret_cast<const uint4*>(dO + row * D + c);
+    }
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) delta[row] = s;
+  for (int u = 0; u < U; ++u) {
+    const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&a[u]), *y = reinterpret_cast<const __nv_bfloat162*>(&d[u]);
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 f = __bfloat1622float2(x[k]), g = __bfloat1622float2(y[k]);
+      s += f.x * g.x + f.y * g.y;
+    }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (c == 0 && group * U + u < rows) delta[group * U + u] = s;
+  }
 }
 
 // Union of the selection blocks chosen by the R tokens of each query tile.
@@ -2593,14 +2609,17 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const bf16* __restrict_
 // Inverse of the selection map: for every (batch, kv head, block) the ascending list of tokens that
 // selected the block (what the key-stationary dK/dV pass walks).  Counting, scanning and filling,
 // with no sort and no atomics on global memory, so the lists are the same on every run:
-//   1. one warp per (b*h, chunk of INV_CHUNK tokens) builds the chunk's histogram over blocks;
+//   1. one warp per (b*h, chunk of tokens) builds the chunk's histogram over blocks;
 //   2. per list, an exclusive scan of the histograms along the chunks gives each chunk's offset
 //      inside the list, and the total gives the list's length;
 //   3. one thread block scans the lengths into list starts (and the CTA counts per list);
 //   4. the warps of step 1 walk their tokens again in the same order and write them.
 // An entry is dropped if it is negative, out of range or repeats an earlier entry of the same token.
 // --------------------------------------------------------------------------------------
-constexpr int INV_CHUNK = 256;
+// A walk is one warp stepping through its tokens, so short chunks are what spreads it over the GPU (chunks of 256 left 128 warps
+// for 16384 tokens x 2 heads and took 106 us per walk).  Above 131072 tokens there are warps enough, and the
+// histograms (one row of counts per chunk) stay as small as they were.
+inline int inverse_chunk(int T) { return T <= 131072 ? 64 : 256; }
 
 // mode 0: hist[(bh * chunks + chunk) * nS + blk] = entries of the chunk; mode 1: fill tok_list.
 // The warp takes the chunk's tokens one after the other, lane j looking at entry j of the token's
@@ -2609,16 +2628,16 @@ constexpr int INV_CHUNK = 256;
 __global__ void __launch_bounds__(32) nsa_inverse_walk_kernel(const int* __restrict__ idx, int* __restrict__ hist,
                                                               const int* __restrict__ chunk_off,
                                                               const int* __restrict__ list_start, int* __restrict__ tok_list,
-                                                              int T, int n, int nS, int chunks, int mode) {
+                                                              int T, int n, int nS, int chunks, int len, int mode) {
   extern __shared__ int bins[];                   // nS running counts of this chunk
   const int chunk = blockIdx.x, lane = threadIdx.x;
   const long bh = blockIdx.y;
   for (int i = lane; i < nS; i += 32) bins[i] = 0;
   __syncwarp();
   const long slot = (bh * chunks + chunk) * nS;
-  const int t_end = min(T, (chunk + 1) * INV_CHUNK);
-  int v_next = (lane < n && chunk * INV_CHUNK < t_end) ? idx[(bh * T + chunk * INV_CHUNK) * n + lane] : -1;
-  for (int t = chunk * INV_CHUNK; t < t_end; ++t) {
+  const int t_end = min(T, (chunk + 1) * len);
+  int v_next = (lane < n && chunk * len < t_end) ? idx[(bh * T + chunk * len) * n + lane] : -1;
+  for (int t = chunk * len; t < t_end; ++t) {
     const int v = v_next;
     if (t + 1 < t_end && lane < n) v_next = idx[(bh * T + t + 1) * n + lane];      // next token's entry, ahead of use
     const bool in_range = lane < n && v >= 0 && v < nS;
@@ -2635,21 +2654,35 @@ __global__ void __launch_bounds__(32) nsa_inverse_walk_kernel(const int* __restr
     for (int i = lane; i < nS; i += 32) hist[slot + i] = bins[i];
 }
 
-// one thread per list: offsets of the chunks inside the list (in place over hist) and the length
+// offsets of the chunks inside each list (in place over hist) and the list's length
 __global__ void __launch_bounds__(256) nsa_inverse_offsets_kernel(int* __restrict__ hist, int* __restrict__ count, long lists,
                                                                  int nS, int chunks) {
-  const long l = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (l >= lists) return;
-  const long bh = l / nS;
-  const int blk = static_cast<int>(l - bh * nS);
+  // CTA: 32 neighbouring lists x 8 chunk groups, so that a row of hist is read in one piece
+  __shared__ int part[8][32];
+  const int l = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const long list = static_cast<long>(blockIdx.x) * 32 + l;
+  const bool live = list < lists;
+  const long bh = live ? list / nS : 0;
+  const int blk = live ? static_cast<int>(list - bh * nS) : 0;
+  const int per = (chunks + 7) / 8, c0 = g * per, c1 = min(c0 + per, chunks);
+  int sum = 0;
+  if (live)
+#pragma unroll 4
+    for (int c = c0; c < c1; ++c) sum += hist[(bh * chunks + c) * nS + blk];
+  part[g][l] = sum;
+  __syncthreads();
   int run = 0;
-  for (int c = 0; c < chunks; ++c) {
-    int* p = hist + (bh * chunks + c) * nS + blk;
-    const int v = *p;
-    *p = run;
-    run += v;
+  for (int k = 0; k < g; ++k) run += part[k][l];
+  if (live) {
+#pragma unroll 4
+    for (int c = c0; c < c1; ++c) {
+      int* p = hist + (bh * chunks + c) * nS + blk;
+      const int v = *p;
+      *p = run;
+      run += v;
+    }
+    if (g == 7) count[list] = run;
   }
-  count[l] = run;
 }
 
 // single CTA: list_start[l] = sum of count[< l]; item_start[l] = sum of ceil(ceil(count / R) / vpc)
@@ -2739,6 +2772,13 @@ __global__ void __launch_bounds__(128) nsa_union_kernel(const int* __restrict__ 
     const unsigned int pos = prefix[blk >> 5] + __popc(below);
     if (pos < static_cast<unsigned>(max_u)) atomicOr(&om[pos], 1ull << tl);
   }
+}
+
+void launch_delta(const void* o, const void* d_o, float* delta, long rows, int D, cudaStream_t st) {
+  const long per_cta = 256 / (D / 8) * 2;
+  const unsigned grid = static_cast<unsigned>((rows + per_cta - 1) / per_cta);
+  if (D == 128) attn_delta_kernel<128><<<grid, 256, 0, st>>>((const bf16*)o, (const bf16*)d_o, delta, rows);
+  else attn_delta_kernel<64><<<grid, 256, 0, st>>>((const bf16*)o, (const bf16*)d_o, delta, rows);
 }
 
 // box_tokens 0: a whole query tile (128 / G tokens); otherwise that many tokens per box
@@ -2874,7 +2914,7 @@ extern "C" int nsa_attn_bwd(const void* q, const void* k, const void* v, const v
   if ((rc = make_kv_map(&tk, k, B, S, Hkv, D))) return rc;
   if ((rc = make_kv_map(&tv, v, B, S, Hkv, D))) return rc;
   const long rows = static_cast<long>(B) * T * Hq;
-  attn_delta_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const bf16*)o, (const bf16*)d_o, delta, rows, D);
+  launch_delta(o, d_o, delta, rows, D, st);
   AttnParams p;
   fill_params(p, B, T, S, Hq, Hkv, D, scale, causal, window, kp_stride, kp_off, tile_blocks, tile_masks, tile_counts, max_u);
   p.L = const_cast<float*>(L); p.delta = delta; p.dQb = (bf16*)dq; p.dK = dk; p.dV = dv;
@@ -2921,7 +2961,7 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
   if ((rc = make_kv_map(&tk, k, B, S, Hkv, D))) return rc;
   if ((rc = make_kv_map(&tv, v, B, S, Hkv, D))) return rc;
   const long rows = static_cast<long>(B) * T * Hq;
-  attn_delta_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const bf16*)o, (const bf16*)d_o, delta, rows, D);
+  launch_delta(o, d_o, delta, rows, D, st);
   AttnParams p;
   fill_params(p, B, T, S, Hq, Hkv, D, scale, causal, window, kp_stride, kp_off, tile_blocks, tile_masks, tile_counts, max_u);
   p.L = const_cast<float*>(L); p.delta = delta; p.dQb = (bf16*)dq; p.dK = nullptr; p.dV = nullptr;
@@ -2992,19 +3032,21 @@ extern "C" int nsa_union_blocks(const int* idx, int* tile_blocks, unsigned long 
 
 // Inverse selection map (see nsa_inverse_walk_kernel).  idx: [B*Hkv, T, n] int32.  Outputs: tok_list
 // (capacity B*Hkv*T*n), list_start and item_start (lists + 1 entries, lists = B*Hkv*nS).  Scratch:
-// hist with B*Hkv*chunks*nS ints (chunks = ceil(T / 256)) and count with `lists` ints.
+// hist with B*Hkv*nsa_inverse_chunks(T)*nS ints and count with `lists` ints.
+// Rows of counts per (batch, KV head) in `hist` of nsa_inverse_blocks.
+extern "C" int nsa_inverse_chunks(int T) { return (T + inverse_chunk(T) - 1) / inverse_chunk(T); }
 extern "C" int nsa_inverse_blocks(const int* idx, int* tok_list, int* list_start, int* item_start, int* hist, int* count,
                                   int BH, int T, int n, int nS, int R, int visits_per_cta, cudaStream_t st) {
   if (BH <= 0 || T <= 0 || n <= 0 || nS <= 0 || R <= 0 || visits_per_cta <= 0)
     return nsa::fail(NSA_ERR_SHAPE, "nsa_inverse_blocks: empty problem");
   if (nS * 4 > 48 * 1024 || n > 32) return nsa::fail(NSA_ERR_SHAPE, "nsa_inverse_blocks: at most 12288 selection blocks and 32 entries per token");
-  const int chunks = (T + INV_CHUNK - 1) / INV_CHUNK;
+  const int len = inverse_chunk(T), chunks = nsa_inverse_chunks(T);
   const long lists = static_cast<long>(BH) * nS;
   const dim3 grid(chunks, BH);
-  nsa_inverse_walk_kernel<<<grid, 32, nS * 4, st>>>(idx, hist, nullptr, nullptr, nullptr, T, n, nS, chunks, 0);
-  nsa_inverse_offsets_kernel<<<(unsigned)((lists + 255) / 256), 256, 0, st>>>(hist, count, lists, nS, chunks);
+  nsa_inverse_walk_kernel<<<grid, 32, nS * 4, st>>>(idx, hist, nullptr, nullptr, nullptr, T, n, nS, chunks, len, 0);
+  nsa_inverse_offsets_kernel<<<(unsigned)((lists + 31) / 32), 256, 0, st>>>(hist, count, lists, nS, chunks);
   nsa_inverse_scan_kernel<<<1, 1024, 0, st>>>(count, list_start, item_start, lists, R, visits_per_cta);
-  nsa_inverse_walk_kernel<<<grid, 32, nS * 4, st>>>(idx, nullptr, hist, list_start, tok_list, T, n, nS, chunks, 1);
+  nsa_inverse_walk_kernel<<<grid, 32, nS * 4, st>>>(idx, nullptr, hist, list_start, tok_list, T, n, nS, chunks, len, 1);
   nsa::count_launch(4);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_inverse_blocks launch");

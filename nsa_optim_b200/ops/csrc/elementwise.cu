@@ -755,34 +755,37 @@ __global__ void __launch_bounds__(CT_WARPS * 32, 2) conv1d_bwd_kernel(const bf16
           d3.a.x *= dsilu_f(p.a.x); d3.a.y *= dsilu_f(p.a.y);
           d3.b.x *= dsilu_f(p.b.x); d3.b.y *= dsilu_f(p.b.y);
         }
-        if (t + u < t1) {
+        if (r < n) {
           dw[0] = quad_fma(d3, x0, dw[0]);
           dw[1] = quad_fma(d3, x1, dw[1]);
           dw[2] = quad_fma(d3, x2, dw[2]);
           dw[3] = quad_fma(d3, x3, dw[3]);
           db.a.x += d3.a.x; db.a.y += d3.a.y; db.b.x += d3.b.x; db.b.y += d3.b.y;
         }
-        const int s = t + u - 3;
-        if (s >= t0 && s < t1)
-          *reinterpret_cast<uint2*>(dp + static_cast<long>(s) * C) =
+        if (r >= 3 && r < n + 3)
+          *reinterpret_cast<uint2*>(dp) =
               quad_pack(quad_fma(wv[3], d0, quad_fma(wv[2], d1, quad_fma(wv[1], d2, quad_fma(wv[0], d3, quad_zero())))));
+        dp += C;
         x0 = x1; x1 = x2; x2 = x3;
         d0 = d1; d1 = d2; d2 = d3;
       }
     }
+    cp_async_wait<0>();
   }
+  __syncthreads();                               // the rings become the reduction buffer
+  float(*sred)[5][CT_C] = reinterpret_cast<float(*)[5][CT_C]>(conv_smem);
 #pragma unroll
   for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&sred[warp][j][lane * 4]) = make_float4(dw[j].a.x, dw[j].a.y, dw[j].b.x, dw[j].b.y);
   *reinterpret_cast<float4*>(&sred[warp][4][lane * 4]) = make_float4(db.a.x, db.a.y, db.b.x, db.b.y);
   __syncthreads();
   float* pp = partial + (static_cast<long>(blockIdx.z) * gridDim.y + blockIdx.y) * 5 * C;
-  for (int e = threadIdx.x; e < 5 * CT_C; e += CT_WARPS * 32) {
-    const int j = e / CT_C, cc = e - j * CT_C;
-    const int cg = blockIdx.x * CT_C + cc;
+  for (int e = threadIdx.x; e < 5 * CT_CW * CT_C; e += CT_WARPS * 32) {
+    const int j = e / (CT_CW * CT_C), cc = e - j * (CT_CW * CT_C);
+    const int cg = blockIdx.x * CT_CW * CT_C + cc;
     if (cg >= C) continue;
     float acc = 0.f;
 #pragma unroll
-    for (int wi = 0; wi < CT_WARPS; ++wi) acc += sred[wi][j][cc];
+    for (int ti = 0; ti < CT_TW; ++ti) acc += sred[ti * CT_CW + cc / CT_C][j][cc % CT_C];
     pp[static_cast<long>(j) * C + cg] = acc;
   }
 }
@@ -872,6 +875,25 @@ int launch_rms_fwd(const void* x, const void* g, const void* w, void* y, float* 
   return 0;
 }
 
+// CTAs of the persistent backward: all resident at once (a partial second round would idle most SMs), at most `parts`.
+template <int TPR, int NV, int MODE>
+int bwd_grid(int parts) {
+  static int per_sm = 0;
+  if (per_sm == 0) {
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rmsnorm_bwd_kernel<TPR, NV, MODE>, 256, 0);
+    per_sm = n > 0 ? n : 1;
+  }
+  const int all = per_sm * nsa::sm_count();
+  return parts < all ? parts : all;
+}
+template <int TPR, int NV, int MODE>
+void run_rms_bwd(const bf16* X, const bf16* G, const bf16* Wt, const bf16* DY, const float* rstd, bf16* DX, bf16* DG, float* partial,
+                 int& grid, long rows, int d, const bf16* DR, long ldg, cudaStream_t st) {
+  grid = bwd_grid<TPR, NV, MODE>(grid);
+  rmsnorm_bwd_kernel<TPR, NV, MODE><<<grid, 256, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
+}
+// `grid` holds the number of partial rows the caller has room for and receives the number written.
 template <int MODE>
 int launch_rms_bwd(const void* x, const void* g, const void* w, const void* dy, const float* rstd, void* dx, void* dg,
                    float* partial, int& grid, long rows, int d, cudaStream_t st, const void* dres = nullptr, long ldg = 0) {
@@ -900,25 +922,6 @@ int launch_rms_add_fwd(const void* x, const void* r, const void* w, void* h, voi
   else return nsa::fail(NSA_ERR_SHAPE, "rmsnorm: width above 8192 is not supported");
   nsa::count_launch();
   return 0;
-// CTAs of the persistent backward: all resident at once (a partial second round would idle most SMs), at most `parts`.
-template <int TPR, int NV, int MODE>
-int bwd_grid(int parts) {
-  static int per_sm = 0;
-  if (per_sm == 0) {
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rmsnorm_bwd_kernel<TPR, NV, MODE>, 256, 0);
-    per_sm = n > 0 ? n : 1;
-  }
-  const int all = per_sm * nsa::sm_count();
-  return parts < all ? parts : all;
-}
-template <int TPR, int NV, int MODE>
-void run_rms_bwd(const bf16* X, const bf16* G, const bf16* Wt, const bf16* DY, const float* rstd, bf16* DX, bf16* DG, float* partial,
-                 int& grid, long rows, int d, const bf16* DR, long ldg, cudaStream_t st) {
-  grid = bwd_grid<TPR, NV, MODE>(grid);
-  rmsnorm_bwd_kernel<TPR, NV, MODE><<<grid, 256, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
-}
-// `grid` holds the number of partial rows the caller has room for and receives the number written.
 }
 
 }  // namespace
@@ -1202,12 +1205,12 @@ static int conv_rows(int B, int T, int C) {
   while (rows > 8 && warps(rows) < 32L * nsa::sm_count()) rows >>= 1;
   return rows;
 }
-extern "C" int nsa_conv1d_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, long ldx,
-                              int width, int act, cudaStream_t st) {
-  if (C % 8 || ldx % 8 || width != 4) return nsa::fail(NSA_ERR_SHAPE, "conv1d: channels multiple of 8 and width 4 required");
 static dim3 conv_grid(int B, int T, int C, int rows) {
   return dim3((C + CT_CW * CT_C - 1) / (CT_CW * CT_C), (T + CT_TW * rows - 1) / (CT_TW * rows), B);
 }
+extern "C" int nsa_conv1d_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, long ldx,
+                              int width, int act, cudaStream_t st) {
+  if (C % 8 || ldx % 8 || width != 4) return nsa::fail(NSA_ERR_SHAPE, "conv1d: channels multiple of 8 and width 4 required");
   const int rows = conv_rows(B, T, C);
   const dim3 grid = conv_grid(B, T, C, rows);
   conv1d_fwd_kernel<<<grid, CT_WARPS * 32, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)y, T, C, ldx, act, rows);

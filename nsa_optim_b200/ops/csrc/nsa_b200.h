@@ -144,11 +144,11 @@ int nsa_ssd_state_fwd(const float* S, const float* gamma, float* Hprev, void* Hp
     nc, int H, long E, cudaStream_t st);
 int nsa_ssd_state_bwd(const float* dHprev, const float* gamma, float* dS, void* dS_bf16, int B, int nc, int H, long
     E, cudaStream_t st);
-int nsa_ssd_chunk_state(int mode, const void* bc, long ld_bc, const void* v, long ld_v, const float* dt, const float*
-    A, float* S_out, float* gamma_out, int B, int T, int H, int N, int P, cudaStream_t st);
 int nsa_ssd_finish(const void* dB_heads, const void* dC_heads, const float* q, const float* k, const float* r, const
     float* dt, const float* A, float* scratch, void* dB, void* dC, float* ddt, float* dA, float* dD, int B, int T, int H,
     cudaStream_t st);
+int nsa_ssd_chunk_state(int mode, const void* bc, long ld_bc, const void* v, long ld_v, const float* dt, const float*
+    A, float* S_out, float* gamma_out, int B, int T, int H, int N, int P, cudaStream_t st);
 int nsa_ssd_chunk_out(const void* Cm, long ld_c, const void* Bm, long ld_b, const void* x, long ld_x, const void*
     Hprev_bf16, const float* dt, const float* A, const float* Dskip, void* y, int B, int T, int H, int N, int P,
     cudaStream_t st);

@@ -94,7 +94,8 @@ def _check(rc: int) -> None:
 
 
 def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the raw handle of the current stream; torch.cuda.current_stream() builds a Stream object for it each time
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _p(t: Optional[Tensor]) -> c_void_p:
@@ -203,7 +204,7 @@ def check_status(sync: bool = True) -> None:
 # GEMM
 # --------------------------------------------------------------------------------------
 def _as_2d(x: Tensor) -> Tensor:
-    x2 = x.reshape(-1, x.shape[-1])
+    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     if x2.stride(-1) != 1 or (x2.stride(0) % 8) or (x2.data_ptr() % 16):
         x2 = x2.contiguous()
     return x2
@@ -219,8 +220,10 @@ def split_k_choice(M: int, N: int, K: int, clusters: int = 74) -> int:
     is mostly empty, and splitting the reduction fills it.  Two parts added into a zeroed fp32 C
     give the same bits in either order, so the default limit of 2 keeps results reproducible;
     ``NSA_B200_SPLITK_MAX`` raises it."""
+    if K < 8192 or M <= 128:
+        return 1
     tiles = -(-M // 256) * -(-N // 256)
-    if K < 8192 or M <= 128 or tiles >= 6 * clusters:
+    if tiles >= 6 * clusters:
         return 1
 
     def eff(S):
@@ -276,14 +279,20 @@ def gemm_select(which: str = "default") -> None:
     load().nsa_gemm_select(c_int({"default": 0, "single": 1, "pair": 2}[which]))
 
 
+def _project(x2: Tensor, w: Tensor, lead) -> Tensor:
+    """x2 w^T in the shape (*lead, out features): the output is allocated as the caller wants it."""
+    y = _empty(*lead, w.shape[0], dtype=torch.bfloat16, device=x2.device)
+    gemm(x2, w, False, False, out=y if y.dim() == 2 else y.view(-1, w.shape[0]))
+    return y
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x: Tensor, w: Tensor):
         x2 = _as_2d(x)
         ctx.save_for_backward(x2, w)
         ctx.xshape = x.shape
-        y = gemm(x2, w, False, False)
-        return y.view(*x.shape[:-1], w.shape[0])
+        return _project(x2, w, x.shape[:-1])
 
     @staticmethod
     def backward(ctx, dy: Tensor):
@@ -309,8 +318,10 @@ class _MultiLinear(torch.autograd.Function):
         ctx.xshape = x.shape
         ys = []
         for i, w in enumerate(ws):
-            y = run_first(x2, w) if (i == 0 and run_first is not None) else gemm(x2, w, False, False)
-            ys.append(y.view(*x.shape[:-1], w.shape[0]))
+            if i == 0 and run_first is not None:
+                ys.append(run_first(x2, w).view(*x.shape[:-1], w.shape[0]))
+            else:
+                ys.append(_project(x2, w, x.shape[:-1]))
         return tuple(ys)
 
     @staticmethod
@@ -847,21 +858,28 @@ def _require_numel(what: str, t: Optional[Tensor], n: int) -> None:
         raise ValueError(f"optimizer state '{what}' has {t.numel()} elements, the kernel needs {n}")
 
 
-def _adamw_words(items, states) -> ctypes.Array:
-    """Seven 64-bit words per tensor, (p, g, m, v, a, b, n); every state tensor is checked against n."""
+def _adamw_words(items, block: int) -> ctypes.Array:
+    """Seven 64-bit words per tensor, (p, g, m, v, a, b, n).  Every state tensor is checked against n; with ``block``
+    the last two are the scales of the quantised moments, else an fp32 master copy (or None) and nothing."""
     words = []
-    for it in items:
-        n = it[0].numel()
-        for (name, div), t in zip(states, it[1:]):
-            _require_numel(name, t, n // div)
-        words += [0 if t is None else t.data_ptr() for t in it] + [n]
+    for p, g, m, v, a, b in items:
+        n = p.numel()
+        na = n // block if block else n
+        if (g.numel() != n or m.numel() != n or v.numel() != n or (a is not None and a.numel() != na)
+                or (b is not None and b.numel() != na)):
+            for what, t in (("grad", g), ("exp_avg", m), ("exp_avg_sq", v)):
+                _require_numel(what, t, n)
+            _require_numel("exp_avg_absmax" if block else "master", a, na)
+            _require_numel("exp_avg_sq_absmax", b, na)
+        words += (p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), 0 if a is None else a.data_ptr(),
+                  0 if b is None else b.data_ptr(), n)
     return (c_longlong * len(words))(*words)
 
 
 def adamw_multi(items, step, lr, b1, b2, eps, wd, grad_scale) -> None:
     """AdamW over (p, g, exp_avg, exp_avg_sq, master or None, None) tuples that share a device, dtypes and step."""
     p, g = items[0][:2]
-    words = _adamw_words(items, (("grad", 1), ("exp_avg", 1), ("exp_avg_sq", 1), ("master", 1), ("", 1)))
+    words = _adamw_words(items, 0)
     gs = None if grad_scale is None else grad_scale.reshape(1).float()
     _check(load().nsa_adamw_multi(words, c_int(len(items)), _p(gs), c_int(int(p.dtype == torch.float32)),
                                   c_int(int(g.dtype == torch.float32)), c_int(step), c_float(lr), c_float(b1), c_float(b2),
@@ -876,8 +894,7 @@ def adamw8bit_multi(items, step, lr, b1, b2, eps, wd, grad_scale, block) -> None
         if it[0].numel() % block:
             raise ValueError(f"8-bit AdamW needs a multiple of {block} elements, got {it[0].numel()}")
     p, g = items[0][:2]
-    words = _adamw_words(items, (("grad", 1), ("exp_avg", 1), ("exp_avg_sq", 1), ("exp_avg_absmax", block),
-                                 ("exp_avg_sq_absmax", block)))
+    words = _adamw_words(items, block)
     gs = None if grad_scale is None else grad_scale.reshape(1).float()
     cs = quant.codebook(8, True, p.device)
     cu = quant.codebook(8, False, p.device)
@@ -1068,7 +1085,7 @@ def inverse_blocks(idx: Tensor, nS: int, R: int, visits_per_cta: int):
     dev = idx.device
     idx = idx.to(torch.int32).contiguous()
     lists = B * Hkv * nS
-    chunks = -(-T // 256)
+    chunks = int(load().nsa_inverse_chunks(c_int(T)))
     tok = _empty(B * Hkv * T * n, dtype=torch.int32, device=dev)
     list_start = _empty(lists + 1, dtype=torch.int32, device=dev)
     item_start = _empty(lists + 1, dtype=torch.int32, device=dev)

@@ -34,6 +34,7 @@ import torch.nn as nn
 from torch import Tensor
 from torch.optim import Optimizer
 
+from . import ops
 from .config import OptimizerConfig, OptimizerType
 from .ops import quant
 
@@ -74,10 +75,7 @@ def get_param_groups(model_or_named, weight_decay: float) -> List[Dict[str, Any]
 
 
 def _native_for(t: Tensor):
-    if not t.is_cuda:
-        return None
-    from . import ops
-    if ops.get_backend() == "torch":
+    if not t.is_cuda or ops.get_backend() == "torch":
         return None
     return ops.native_module()
 
@@ -102,7 +100,6 @@ class _NativeBatch:
     def run(self, lr, b1, b2, eps, wd, grad_scale, block: int = 256) -> None:
         if not self.lists:
             return
-        from . import ops
         nat = ops.native_module()
         for (quantised, step, *_), items in self.lists.items():
             if quantised:
