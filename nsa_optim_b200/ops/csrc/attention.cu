@@ -56,6 +56,7 @@ struct AttnParams {
   const float* delta;               // [B, T, Hq]  rowsum(dO * O)
   float* dQ;                        // unused (dQ written as bf16 below)
   bf16* dQb;                        // [B, T, Hq, D]
+  int add_dq;                       // dQ is added to what dQb holds (fp32 sum, one rounding)
   float* dK;                        // [B, S, Hkv, D] fp32, pre-zeroed
   float* dV;
   KernelStatus* status;
@@ -151,6 +152,26 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&v)[64]) {
   tc5::tmem_ld_wait();
 #pragma unroll
   for (int i = 0; i < 32; ++i) { v[i] = a[i]; v[32 + i] = b[i]; }
+}
+
+// 32 accumulator columns of one row -> bf16 row of dQ, on top of what the row holds when `add` is set
+__device__ __forceinline__ void store_dq32(bf16* dst, const uint32_t (&a)[32], int add) {
+  uint4* d = reinterpret_cast<uint4*>(dst);
+  uint4 old[4] = {};
+  if (add) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) old[i] = d[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t w[4] = {old[i].x, old[i].y, old[i].z, old[i].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)          // a bf16 is the upper half of its fp32
+      o[j] = tc5::pack_bf16(__uint_as_float(a[8 * i + 2 * j]) + __uint_as_float(w[j] << 16),
+                            __uint_as_float(a[8 * i + 2 * j + 1]) + __uint_as_float(w[j] & 0xffff0000u));
+    d[i] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
 }
 
 // write 64 bf16 (32 packed pairs) as row `row` of a [128][64] swizzled k-block
@@ -1865,17 +1886,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
         for (int i = 0; i < 32; ++i) a[i] = 0u;
       }
-      if (row_ok) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint4 o4;
-          o4.x = tc5::pack_bf16(__uint_as_float(a[8 * i]), __uint_as_float(a[8 * i + 1]));
-          o4.y = tc5::pack_bf16(__uint_as_float(a[8 * i + 2]), __uint_as_float(a[8 * i + 3]));
-          o4.z = tc5::pack_bf16(__uint_as_float(a[8 * i + 4]), __uint_as_float(a[8 * i + 5]));
-          o4.w = tc5::pack_bf16(__uint_as_float(a[8 * i + 6]), __uint_as_float(a[8 * i + 7]));
-          reinterpret_cast<uint4*>(dst + q4 * 32)[i] = o4;
-        }
-      }
+      if (row_ok) store_dq32(dst + q4 * 32, a, p.add_dq);
     }
   }
   tc5::fence_before_sync();
@@ -2144,17 +2155,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 32; ++i) a[i] = 0u;
       }
-      if (row_ok) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint4 o4;
-          o4.x = tc5::pack_bf16(__uint_as_float(a[8 * i]), __uint_as_float(a[8 * i + 1]));
-          o4.y = tc5::pack_bf16(__uint_as_float(a[8 * i + 2]), __uint_as_float(a[8 * i + 3]));
-          o4.z = tc5::pack_bf16(__uint_as_float(a[8 * i + 4]), __uint_as_float(a[8 * i + 5]));
-          o4.w = tc5::pack_bf16(__uint_as_float(a[8 * i + 6]), __uint_as_float(a[8 * i + 7]));
-          reinterpret_cast<uint4*>(dst + q4 * 32)[i] = o4;
-        }
-      }
+      if (row_ok) store_dq32(dst + q4 * 32, a, p.add_dq);
     }
   }
   tc5::fence_before_sync();
@@ -2940,12 +2941,15 @@ extern "C" int nsa_attn_bwd(const void* q, const void* k, const void* v, const v
 // (b, h, block), ascending), list_start / item_start ([B*Hkv*nS + 1] exclusive prefixes of list
 // lengths and of CTAs per list, a CTA covering visits_per_cta * (128 / G) tokens) and
 // item_bound >= item_start[last].  head_dim 128 only; selected mode needs G >= 8.
+// delta_given: delta holds rowsum(dO * O) already (the gated combine's backward has both tensors in registers).
+// add_dq: dQ is added to what dq holds; dK / dV always add to what the caller put there.
 extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                                   const float* L, float* delta, void* dq, float* dk, float* dv, int B, int T, int S,
                                   int Hq, int Hkv, int D, float scale, int causal, int window, int kp_stride, int kp_off,
                                   const int* tile_blocks, const unsigned long long* tile_masks, const int* tile_counts,
                                   int max_u, const int* tok_list, const int* list_start, const int* item_start, int nS,
-                                  int item_bound, int visits_per_cta, cudaStream_t st) {
+                                  int item_bound, int visits_per_cta, int delta_given, int add_dq,
+                                  cudaStream_t st) {
   int rc = check_shape(Hq, Hkv, D, tile_blocks);
   if (rc) return rc;
   const int G = Hq / Hkv;
@@ -2961,10 +2965,10 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
   if ((rc = make_kv_map(&tk, k, B, S, Hkv, D))) return rc;
   if ((rc = make_kv_map(&tv, v, B, S, Hkv, D))) return rc;
   const long rows = static_cast<long>(B) * T * Hq;
-  launch_delta(o, d_o, delta, rows, D, st);
+  if (!delta_given) launch_delta(o, d_o, delta, rows, D, st);
   AttnParams p;
   fill_params(p, B, T, S, Hq, Hkv, D, scale, causal, window, kp_stride, kp_off, tile_blocks, tile_masks, tile_counts, max_u);
-  p.L = const_cast<float*>(L); p.delta = delta; p.dQb = (bf16*)dq; p.dK = nullptr; p.dV = nullptr;
+  p.L = const_cast<float*>(L); p.delta = delta; p.dQb = (bf16*)dq; p.add_dq = add_dq; p.dK = nullptr; p.dV = nullptr;
   {
     const dim3 grid((T + p.R - 1) / p.R, Hkv, B);
     static const bool smem_operands = [] { const char* e = getenv("NSA_B200_ATTN_DQ"); return e && !strcmp(e, "smem"); }();
@@ -3000,7 +3004,7 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
     if (!cfg) { if ((rc = set_smem(attn_bwd_kv_kernel, smem))) return rc; cfg = true; }
     attn_bwd_kv_kernel<<<grid, KV_THREADS, smem, st>>>(tq, tdo, tq1, tdo1, tk, tv, p, w, scale);
   }
-  nsa::count_launch(3);
+  nsa::count_launch(delta_given ? 2 : 3);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_attn_bwd_split launch");
 }

@@ -459,12 +459,14 @@ __global__ void __launch_bounds__(256) gate_combine_bwd_kernel(const bf16* __res
                                                                const bf16* __restrict__ d_o, bf16* __restrict__ do1,
                                                                bf16* __restrict__ do2, bf16* __restrict__ do3,
                                                                bf16* __restrict__ dg1, bf16* __restrict__ dg2,
-                                                               bf16* __restrict__ dg3, long n8, int Hq, long ldg, int sig) {
+                                                               bf16* __restrict__ dg3, float* __restrict__ e1,
+                                                               float* __restrict__ e2, float* __restrict__ e3, long n8, int Hq,
+                                                               long ldg, int sig) {
   // the grid is sized so that every thread handles exactly one vector (rows stay inside a warp)
   const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool live = i < n8;
   const long row = (live ? i : 0) / LANES;
-  float s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  float s1 = 0.f, s2 = 0.f, s3 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
   const long gi = (row / Hq) * ldg + row % Hq;
   float a = 0.f, b = 0.f, c = 0.f;
   if (live) {
@@ -478,13 +480,13 @@ __global__ void __launch_bounds__(256) gate_combine_bwd_kernel(const bf16* __res
 #pragma unroll
     for (int j = 0; j < 8; ++j) { s1 += d[j] * x[j]; s2 += d[j] * y[j]; s3 += d[j] * z[j]; }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) r[j] = a * d[j];
+    for (int j = 0; j < 8; ++j) { r[j] = __bfloat162float(__float2bfloat16(a * d[j])); t1 += r[j] * x[j]; }
     store8(do1 + i * 8, r);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) r[j] = b * d[j];
+    for (int j = 0; j < 8; ++j) { r[j] = __bfloat162float(__float2bfloat16(b * d[j])); t2 += r[j] * y[j]; }
     store8(do2 + i * 8, r);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) r[j] = c * d[j];
+    for (int j = 0; j < 8; ++j) { r[j] = __bfloat162float(__float2bfloat16(c * d[j])); t3 += r[j] * z[j]; }
     store8(do3 + i * 8, r);
   }
 #pragma unroll
@@ -492,6 +494,15 @@ __global__ void __launch_bounds__(256) gate_combine_bwd_kernel(const bf16* __res
     s1 += __shfl_xor_sync(0xffffffffu, s1, o);
     s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+  }
+  if (e1 != nullptr) {
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
+      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+      t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+      t3 += __shfl_xor_sync(0xffffffffu, t3, o);
+    }
+    if (live && (threadIdx.x % LANES) == 0) { e1[row] = t1; e2[row] = t2; e3[row] = t3; }
   }
   if (live && (threadIdx.x % LANES) == 0) {
     // gates given as logits: the gradient goes back through the sigmoid here
@@ -1127,7 +1138,7 @@ extern "C" int nsa_gate_combine_bwd(const void* o1, const void* o2, const void* 
   if (blocks > 2147483647L) return nsa::fail(NSA_ERR_SHAPE, "gate_combine: problem too large for one launch");
 #define NSA_GC_BWD(L) gate_combine_bwd_kernel<L><<<(unsigned)blocks, 256, 0, st>>>((const bf16*)o1, (const bf16*)o2, \
     (const bf16*)o3, (const bf16*)g1, (const bf16*)g2, (const bf16*)g3, (const bf16*)d_o, (bf16*)do1, (bf16*)do2, (bf16*)do3, \
-    (bf16*)dg1, (bf16*)dg2, (bf16*)dg3, n8, 1, 1L, 0)
+    (bf16*)dg1, (bf16*)dg2, (bf16*)dg3, nullptr, nullptr, nullptr, n8, 1, 1L, 0)
   if (D == 64) NSA_GC_BWD(8); else if (D == 128) NSA_GC_BWD(16); else NSA_GC_BWD(32);
 #undef NSA_GC_BWD
   nsa::count_launch();
@@ -1136,7 +1147,7 @@ extern "C" int nsa_gate_combine_bwd(const void* o1, const void* o2, const void* 
 
 // The same with the three gates as columns of one [tokens, >= 3*Hq] bf16 matrix (row pitch ldg, the
 // gate projection's output as it stands) and, with sig != 0, given as logits: the sigmoid and its
-// derivative are applied here.  rows = tokens * Hq.  dg1..dg3 use the same pitch.
+// derivative are applied here.  rows = tokens * Hq.  dg1..dg3 use the same pitch.  e1..e3 (all or none): fp32 [rows].
 extern "C" int nsa_gate_combine_fwd_ex(const void* o1, const void* o2, const void* o3, const void* g1, const void* g2,
                                        const void* g3, long ldg, int Hq, int sig, void* o, long rows, int D, cudaStream_t st) {
   if (D != 64 && D != 128 && D != 256) return nsa::fail(NSA_ERR_SHAPE, "gate_combine: head_dim must be 64, 128 or 256");
@@ -1152,7 +1163,8 @@ extern "C" int nsa_gate_combine_fwd_ex(const void* o1, const void* o2, const voi
 }
 extern "C" int nsa_gate_combine_bwd_ex(const void* o1, const void* o2, const void* o3, const void* g1, const void* g2,
                                        const void* g3, long ldg, int Hq, int sig, const void* d_o, void* do1, void* do2,
-                                       void* do3, void* dg1, void* dg2, void* dg3, long rows, int D, cudaStream_t st) {
+                                       void* do3, void* dg1, void* dg2, void* dg3, float* e1, float* e2, float* e3,
+                                       long rows, int D, cudaStream_t st) {
   if (D != 64 && D != 128 && D != 256) return nsa::fail(NSA_ERR_SHAPE, "gate_combine: head_dim must be 64, 128 or 256");
   if (Hq <= 0 || rows % Hq) return nsa::fail(NSA_ERR_SHAPE, "gate_combine: rows must be tokens * heads");
   const long n8 = rows * (D / 8);
@@ -1160,7 +1172,7 @@ extern "C" int nsa_gate_combine_bwd_ex(const void* o1, const void* o2, const voi
   if (blocks > 2147483647L) return nsa::fail(NSA_ERR_SHAPE, "gate_combine: problem too large for one launch");
 #define NSA_GC_BWD(L) gate_combine_bwd_kernel<L><<<(unsigned)blocks, 256, 0, st>>>((const bf16*)o1, (const bf16*)o2, \
     (const bf16*)o3, (const bf16*)g1, (const bf16*)g2, (const bf16*)g3, (const bf16*)d_o, (bf16*)do1, (bf16*)do2, (bf16*)do3, \
-    (bf16*)dg1, (bf16*)dg2, (bf16*)dg3, n8, Hq, ldg, sig)
+    (bf16*)dg1, (bf16*)dg2, (bf16*)dg3, e1, e2, e3, n8, Hq, ldg, sig)
   if (D == 64) NSA_GC_BWD(8); else if (D == 128) NSA_GC_BWD(16); else NSA_GC_BWD(32);
 #undef NSA_GC_BWD
   nsa::count_launch();

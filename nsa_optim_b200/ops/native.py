@@ -987,6 +987,51 @@ def gated_delta_rule(q, k, v, g, beta, scale=None, chunk=64):
 # --------------------------------------------------------------------------------------
 # attention family (csrc/attention.cu)
 # --------------------------------------------------------------------------------------
+def _attn_forward(q, k, v, causal, window, scale, kp_stride, kp_off, tiles):
+    """(output, L) of contiguous q, k, v; see :class:`_Attn`."""
+    B, T, Hq, D = q.shape
+    S, Hkv = k.shape[1], k.shape[2]
+    o = _empty_like(q)
+    L = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
+    tb, tm, tc, mu = tiles[:4] if tiles is not None else (None, None, None, 0)
+    _check(load().nsa_attn_fwd(_p(q), _p(k), _p(v), _p(o), _p(L), c_int(B), c_int(T), c_int(S), c_int(Hq),
+                               c_int(Hkv), c_int(D), c_float(scale), c_int(int(causal)), c_int(window),
+                               c_int(kp_stride), c_int(kp_off), _p(tb), _p(tm), _p(tc), c_int(mu), _stream()))
+    return o, L
+
+
+def _attn_backward_split(q, k, v, o, do, L, dq, dk, dv, causal, window, scale, kp_stride, kp_off, tiles, delta=None, add_dq=False):
+    """dQ from the query-tile-outer kernel, dK / dV from the key-block-stationary kernel.  dk and dv (fp32) are added
+    to, dq (bf16) is written or, with ``add_dq``, added to; ``delta`` is rowsum(do * o) where the caller has it."""
+    B, T, Hq, D = q.shape
+    S, Hkv = k.shape[1], k.shape[2]
+    given = delta is not None
+    if not given:
+        delta = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
+    tb, tm, tc, mu = tiles[:4] if tiles is not None else (None, None, None, 0)
+    inv = (None, None, None, 0, 0)
+    visits = _kv_visits()
+    if tiles is not None:
+        idx, nS = tiles[4], tiles[5]
+        visits = int(os.environ.get('NSA_B200_KV_VISITS_SEL', '64'))
+        inv = inverse_blocks(idx, nS, 128 // (Hq // Hkv), visits)
+    _check(load().nsa_attn_bwd_split(_p(q), _p(k), _p(v), _p(o), _p(do), _p(L), _p(delta), _p(dq), _p(dk), _p(dv),
+                                     c_int(B), c_int(T), c_int(S), c_int(Hq), c_int(Hkv), c_int(D), c_float(scale),
+                                     c_int(int(causal)), c_int(window), c_int(kp_stride), c_int(kp_off),
+                                     _p(tb), _p(tm), _p(tc), c_int(mu), _p(inv[0]), _p(inv[1]), _p(inv[2]),
+                                     c_int(inv[3]), c_int(inv[4]), c_int(visits), c_int(int(given)), c_int(int(add_dq)),
+                                     _stream()))
+
+
+def _kv_visits() -> int:
+    """Query tiles per CTA of the dK / dV kernel over a contiguous key range."""
+    return int(os.environ.get('NSA_B200_KV_VISITS', '128'))
+
+
+def _bwd_is_split(D: int, G: int, selected: bool) -> bool:
+    return D == 128 and os.environ.get("NSA_B200_ATTN_BWD", "split") == "split" and (not selected or G >= 8)
+
+
 class _Attn(torch.autograd.Function):
     """Softmax attention on (B, T, H, D) tensors through the tcgen05 kernels.  ``tiles`` is
     ``None`` (contiguous key range bounded by causality / window) or the per-query-tile block
@@ -996,14 +1041,7 @@ class _Attn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, causal, window, scale, kp_stride, kp_off, tiles):
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        B, T, Hq, D = q.shape
-        S, Hkv = k.shape[1], k.shape[2]
-        o = _empty_like(q)
-        L = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
-        tb, tm, tc, mu = tiles[:4] if tiles is not None else (None, None, None, 0)
-        _check(load().nsa_attn_fwd(_p(q), _p(k), _p(v), _p(o), _p(L), c_int(B), c_int(T), c_int(S), c_int(Hq),
-                                   c_int(Hkv), c_int(D), c_float(scale), c_int(int(causal)), c_int(window),
-                                   c_int(kp_stride), c_int(kp_off), _p(tb), _p(tm), _p(tc), c_int(mu), _stream()))
+        o, L = _attn_forward(q, k, v, causal, window, scale, kp_stride, kp_off, tiles)
         ctx.save_for_backward(q, k, v, o, L)
         ctx.cfg = (causal, window, scale, kp_stride, kp_off)
         ctx.tiles = tiles
@@ -1020,25 +1058,11 @@ class _Attn(torch.autograd.Function):
         dq = _empty_like(q)
         dk = _zeros(k.shape, dtype=torch.float32, device=q.device)
         dv = _zeros(v.shape, dtype=torch.float32, device=q.device)
-        delta = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
-        tb, tm, tc, mu = ctx.tiles[:4] if ctx.tiles is not None else (None, None, None, 0)
-        G = Hq // Hkv
-        split = D == 128 and os.environ.get("NSA_B200_ATTN_BWD", "split") == "split" and (ctx.tiles is None or G >= 8)
-        if split:
-            # dQ from the query-tile-outer kernel, dK / dV from the key-block-stationary kernel
-            R = 128 // G
-            inv = (None, None, None, 0, 0)
-            visits = int(os.environ.get('NSA_B200_KV_VISITS', '128'))
-            if ctx.tiles is not None:
-                idx, nS = ctx.tiles[4], ctx.tiles[5]
-                visits = int(os.environ.get('NSA_B200_KV_VISITS_SEL', '64'))
-                inv = inverse_blocks(idx, nS, R, visits)
-            _check(load().nsa_attn_bwd_split(_p(q), _p(k), _p(v), _p(o), _p(do), _p(L), _p(delta), _p(dq), _p(dk), _p(dv),
-                                             c_int(B), c_int(T), c_int(S), c_int(Hq), c_int(Hkv), c_int(D), c_float(scale),
-                                             c_int(int(causal)), c_int(window), c_int(kp_stride), c_int(kp_off),
-                                             _p(tb), _p(tm), _p(tc), c_int(mu), _p(inv[0]), _p(inv[1]), _p(inv[2]),
-                                             c_int(inv[3]), c_int(inv[4]), c_int(visits), _stream()))
+        if _bwd_is_split(D, Hq // Hkv, ctx.tiles is not None):
+            _attn_backward_split(q, k, v, o, do, L, dq, dk, dv, *ctx.cfg, ctx.tiles)
         else:
+            tb, tm, tc, mu = ctx.tiles[:4] if ctx.tiles is not None else (None, None, None, 0)
+            delta = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
             _check(load().nsa_attn_bwd(_p(q), _p(k), _p(v), _p(o), _p(do), _p(L), _p(delta), _p(dq), _p(dk), _p(dv),
                                        c_int(B), c_int(T), c_int(S), c_int(Hq), c_int(Hkv), c_int(D), c_float(scale),
                                        c_int(int(causal)), c_int(window), c_int(kp_stride), c_int(kp_off),
@@ -1215,46 +1239,99 @@ class _GateCombine(torch.autograd.Function):
         return d1, d2, d3, e1, e2, e3
 
 
+def _gate_logits_forward(o1, o2, o3, gates):
+    """(combined output, bf16 logits) with the three gates as logits straight from the gate projection: ``gates`` is
+    (B, T, 3*Hq) (or wider; columns [0, Hq) compressed, [Hq, 2Hq) selected, [2Hq, 3Hq) window)."""
+    Hq, D = o1.shape[-2], o1.shape[-1]
+    gl = gates.to(torch.bfloat16)
+    if gl.stride(-1) != 1 or not gl.is_contiguous():
+        gl = gl.contiguous()
+    g0, step = gl.data_ptr(), Hq * gl.element_size()
+    o = _empty_like(o1)
+    _check(load().nsa_gate_combine_fwd_ex(_p(o1), _p(o2), _p(o3), c_void_p(g0), c_void_p(g0 + step), c_void_p(g0 + 2 * step),
+                                          c_long(gl.shape[-1]), c_int(Hq), c_int(1), _p(o), c_long(o1.numel() // D), c_int(D),
+                                          _stream()))
+    return o, gl
+
+
+def _gate_logits_backward(o1, o2, o3, gl, do, sums=(None, None, None)):
+    """(do1, do2, do3, d logits); ``sums``, three fp32 tensors of one value per row, receive rowsum(do_i * o_i)."""
+    do = do.contiguous()
+    Hq, D, ldg = o1.shape[-2], o1.shape[-1], gl.shape[-1]
+    step = Hq * gl.element_size()
+    d1, d2, d3 = _empty_like(o1), _empty_like(o1), _empty_like(o1)
+    dgl = _zeros_like(gl) if ldg > 3 * Hq else _empty_like(gl)
+    g0, dg0 = gl.data_ptr(), dgl.data_ptr()
+    _check(load().nsa_gate_combine_bwd_ex(_p(o1), _p(o2), _p(o3), c_void_p(g0), c_void_p(g0 + step), c_void_p(g0 + 2 * step),
+                                          c_long(ldg), c_int(Hq), c_int(1), _p(do), _p(d1), _p(d2), _p(d3), c_void_p(dg0),
+                                          c_void_p(dg0 + step), c_void_p(dg0 + 2 * step), _p(sums[0]), _p(sums[1]), _p(sums[2]),
+                                          c_long(o1.numel() // D), c_int(D), _stream()))
+    return d1, d2, d3, dgl
+
+
 class _GateCombineLogits(torch.autograd.Function):
-    """The same combine with the three gates taken as logits straight from the gate projection:
-    ``gates`` is (B, T, 3*Hq) (or wider; columns [0, Hq) compressed, [Hq, 2Hq) selected, [2Hq, 3Hq)
-    window).  The sigmoid runs inside the combine kernel and its derivative inside the backward
-    kernel, which writes d(logits) in the projection's own layout."""
+    """The same combine with the gates given as logits.  The sigmoid runs inside the combine kernel and its
+    derivative inside the backward kernel, which writes d(logits) in the projection's own layout."""
 
     @staticmethod
     def forward(ctx, o1, o2, o3, gates):
         o1, o2, o3 = o1.contiguous(), o2.contiguous(), o3.contiguous()
-        Hq, D = o1.shape[-2], o1.shape[-1]
-        gl = gates.to(torch.bfloat16)
-        if gl.stride(-1) != 1 or not gl.is_contiguous():
-            gl = gl.contiguous()
-        ldg = gl.shape[-1]
-        rows = o1.numel() // D
-        o = _empty_like(o1)
-        es = gl.element_size()
-        _check(load().nsa_gate_combine_fwd_ex(_p(o1), _p(o2), _p(o3), c_void_p(gl.data_ptr()), c_void_p(gl.data_ptr() + Hq * es),
-                                              c_void_p(gl.data_ptr() + 2 * Hq * es), c_long(ldg), c_int(Hq), c_int(1), _p(o),
-                                              c_long(rows), c_int(D), _stream()))
+        o, gl = _gate_logits_forward(o1, o2, o3, gates)
         ctx.save_for_backward(o1, o2, o3, gl)
         ctx.gdtype = gates.dtype
         return o
 
     @staticmethod
     def backward(ctx, do):
-        o1, o2, o3, gl = ctx.saved_tensors
-        do = do.contiguous()
-        Hq, D = o1.shape[-2], o1.shape[-1]
-        ldg = gl.shape[-1]
-        rows = o1.numel() // D
-        es = gl.element_size()
-        d1, d2, d3 = _empty_like(o1), _empty_like(o1), _empty_like(o1)
-        dgl = _zeros_like(gl) if ldg > 3 * Hq else _empty_like(gl)
-        g0, dg0 = gl.data_ptr(), dgl.data_ptr()
-        _check(load().nsa_gate_combine_bwd_ex(_p(o1), _p(o2), _p(o3), c_void_p(g0), c_void_p(g0 + Hq * es),
-                                              c_void_p(g0 + 2 * Hq * es), c_long(ldg), c_int(Hq), c_int(1), _p(do), _p(d1), _p(d2),
-                                              _p(d3), c_void_p(dg0), c_void_p(dg0 + Hq * es), c_void_p(dg0 + 2 * Hq * es),
-                                              c_long(rows), c_int(D), _stream()))
+        d1, d2, d3, dgl = _gate_logits_backward(*ctx.saved_tensors, do)
         return d1, d2, d3, dgl.to(ctx.gdtype)
+
+
+def _nsa_select_tiles(q, kc, L_cmp, nS, stride, block, sel_block, top_n, scale):
+    """Importance of the selection blocks, the top_n of each token, and the per-tile lists of :class:`_Attn`."""
+    idx = nsa_select(nsa_importance(q, kc, L_cmp, nS, stride, block, scale), sel_block, top_n)
+    return union_blocks(idx, q.shape[2] // kc.shape[2], nS) + (idx, nS)
+
+
+class _NSA(torch.autograd.Function):
+    """The three branches and their gated combine as one node.  With separate nodes the backward read every do_i and
+    o_i again for rowsum(do_i * o_i) and added the branches' dq, dk and dv in passes of their own (16384 tokens x 32
+    heads: 280 of 6810 us); here the combine's backward leaves the sums, and each branch adds to the gradients of the one
+    before it: dq in the kernel's epilogue, dk and dv of the selected and window branches in one fp32 buffer."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, kc, vc, gates, stride, block, sel_block, top_n, window, scale):
+        q, k, v, kc, vc = (t.contiguous() for t in (q, k, v, kc, vc))
+        o1, L1 = _attn_forward(q, kc, vc, True, 0, scale, stride, block - 1, None)
+        tiles = _nsa_select_tiles(q, kc, L1, -(-q.shape[1] // sel_block), stride, block, sel_block, top_n, scale)
+        o2, L2 = _attn_forward(q, k, v, True, 0, scale, 1, 0, tiles)
+        o3, L3 = _attn_forward(q, k, v, True, window, scale, 1, 0, None)
+        o, gl = _gate_logits_forward(o1, o2, o3, gates)
+        ctx.save_for_backward(q, k, v, kc, vc, gl, o1, o2, o3, L1, L2, L3)
+        ctx.cfg, ctx.tiles, ctx.gdtype = (stride, block, window, scale), tiles, gates.dtype
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, kc, vc, gl, o1, o2, o3, L1, L2, L3 = ctx.saved_tensors
+        stride, block, window, scale = ctx.cfg
+        f32 = torch.float32
+        sums = [_empty_like(L1) for _ in range(3)]
+        d1, d2, d3, dgl = _gate_logits_backward(o1, o2, o3, gl, do, sums)
+        dq = _empty_like(q)
+        dkc, dvc, dk, dv = (_zeros(t.shape, dtype=f32, device=q.device) for t in (kc, vc, k, v))
+        _attn_backward_split(q, kc, vc, o1, d1, L1, dq, dkc, dvc, True, 0, scale, stride, block - 1, None, sums[0])
+        _attn_backward_split(q, k, v, o2, d2, L2, dq, dk, dv, True, 0, scale, 1, 0, ctx.tiles, sums[1], True)
+        # The window branch shares dk / dv while one CTA covers a key block: one more addition to what is there gives
+        # the same bits on every run, two in either order would not.
+        R = 128 // (q.shape[2] // k.shape[2])
+        shared = (63 + window - 1) // R + 2 <= _kv_visits()
+        dk3, dv3 = (dk, dv) if shared else (_zeros(t.shape, dtype=f32, device=q.device) for t in (k, v))
+        _attn_backward_split(q, k, v, o3, d3, L3, dq, dk3, dv3, True, window, scale, 1, 0, None, sums[2], True)
+        if not shared:
+            dk, dv = dk + dk3, dv + dv3
+        return (dq, dk.to(k.dtype), dv.to(v.dtype), dkc.to(kc.dtype), dvc.to(vc.dtype), dgl.to(ctx.gdtype),
+                None, None, None, None, None, None)
 
 
 class _Pool(torch.autograd.Function):
@@ -1310,13 +1387,11 @@ def nsa_attention(q, k, v, g_cmp, g_slc, g_swa, cmp_block=32, cmp_stride=16, sel
     scale = D ** -0.5 if scale is None else scale
     kc = nsa_compress(k, cmp_block, cmp_stride)
     vc = nsa_compress(v, cmp_block, cmp_stride)
+    if gate_logits is not None and window > 0 and q.dtype == torch.bfloat16 and _bwd_is_split(D, G, True):
+        return _NSA.apply(q, k, v, kc, vc, gate_logits, cmp_stride, cmp_block, sel_block, top_n, int(window), float(scale))
     o_cmp, L_cmp = _Attn.apply(q, kc, vc, True, 0, float(scale), cmp_stride, cmp_block - 1, None)
-    nS = -(-T // sel_block)
     with torch.no_grad():
-        imp = nsa_importance(q, kc, L_cmp, nS, cmp_stride, cmp_block, float(scale))
-        idx = nsa_select(imp, sel_block, top_n)
-        del imp
-        tiles = union_blocks(idx, G, nS) + (idx, nS)
+        tiles = _nsa_select_tiles(q, kc, L_cmp, -(-T // sel_block), cmp_stride, cmp_block, sel_block, top_n, float(scale))
     o_slc = _Attn.apply(q, k, v, True, 0, float(scale), 1, 0, tiles)[0]
     o_swa = _Attn.apply(q, k, v, True, int(window), float(scale), 1, 0, None)[0]
     if gate_logits is not None:
