@@ -1296,7 +1296,7 @@ def _nsa_select_tiles(q, kc, L_cmp, nS, stride, block, sel_block, top_n, scale):
 class _NSA(torch.autograd.Function):
     """The three branches and their gated combine as one node.  With separate nodes the backward read every do_i and
     o_i again for rowsum(do_i * o_i) and added the branches' dq, dk and dv in passes of their own (16384 tokens x 32
-    heads: 280 of 6810 us); here the combine's backward leaves the sums, and each branch adds to the gradients of the one
+    heads: 280 of 6810 us; 6400 in all now); here the combine's backward leaves the sums, and each branch adds to the gradients of the one
     before it: dq in the kernel's epilogue, dk and dv of the selected and window branches in one fp32 buffer."""
 
     @staticmethod
