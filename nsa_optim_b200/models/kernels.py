@@ -109,7 +109,10 @@ class RotaryEmbedding(nn.Module):
         self._initial = max_position_embeddings
 
     def _set_cos_sin_cache(self, seq_len: int, device=None):
-        cos, sin = ops.oracle.rope_tables(self.dim, seq_len, self.base, device=device)
+        # ordinary tensors also when the first call is an evaluation under inference mode: a later training
+        # step saves slices of them for its backward
+        with torch.inference_mode(False):
+            cos, sin = ops.oracle.rope_tables(self.dim, seq_len, self.base, device=device)
         self.cos_cached, self.sin_cached = cos, sin
         self.max_seq_len_cached = seq_len
 

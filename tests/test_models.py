@@ -43,6 +43,22 @@ def test_transformer_forward_backward(attn):
     assert logits.shape == (2, 32, 100) and loss is None
 
 
+@pytest.mark.parametrize("family", ["transformer", "hybrid"])
+def test_training_after_evaluation_under_inference_mode(family):
+    # the rotary tables are first built by the evaluation and saved for backward by the training step
+    torch.manual_seed(0)
+    m = create_model(small_cfg()) if family == "transformer" else create_hybrid_model(HybridConfig(
+        d_model=64, vocab_size=100, block_pattern="A", block_repeats=1, num_attention_heads=4, num_key_value_heads=2,
+        head_dim=16, max_position_embeddings=64))
+    ids = torch.randint(0, 100, (2, 32))
+    with torch.inference_mode():
+        before = m(ids)[0].clone()
+    logits, loss = m(ids, labels=ids)[:2]
+    loss.backward()
+    assert all(p.grad is not None for p in m.parameters())
+    assert torch.equal(m(ids)[0].detach(), before)
+
+
 def test_transformer_state_dict_keys():
     keys = set(create_model(small_cfg(AttentionType.NSA)).state_dict())
     for k in ("embed_tokens.weight", "norm.weight", "lm_head.weight", "layers.0.input_layernorm.weight",
