@@ -170,13 +170,23 @@ __global__ void __launch_bounds__(256) rmsnorm_add_fwd_kernel(const bf16* __rest
 // dw into `partial[gridDim.x][d]`.  `dres` (may be null) is a gradient that reaches the norm's
 // input by another route (the residual stream); it is added into dx here instead of by a
 // separate pass over both tensors.
+//
+// Bound by memory traffic, so by the bytes in flight per SM.  A row that a CTA shares (TPR 256) ends in two barriers: what
+// helps is the next row's operands in flight behind them, though that costs resident CTAs (gate first, 8192 x 4096: 136 -> 107 us
+// with one CTA per SM instead of two), and above 4096 columns all loads of the row issued together, though that spills (gate first,
+// 4096 x 8192: 195 -> 139 us with 328 bytes spilled).  A row of one warp (TPR 32, up to 512 columns) meets no barrier: its
+// warps run apart and hide each other's loads, so the registers go to more warps, and x and dres are read again where
+// they are used.  1048576 x 128: 260 us plain and 407 norm first (516 and 604 with the next row in registers: two CTAs
+// instead of four and three); 262144 x 512: 169 plain, 320 gate first (311 and 415).
+// CTAs per SM that the registers leave room for:
 template <int TPR, int NV, int MODE>
-__global__ void __launch_bounds__(256, NV == 1 ? (MODE == 0 && TPR == 256 ? 4 : 2) : 1) rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g,
-                                                          const bf16* __restrict__ w, const bf16* __restrict__ dy,
-                                                          const float* __restrict__ rstd_in, bf16* __restrict__ dx,
-                                                          bf16* __restrict__ dg, float* __restrict__ partial,
-                                                          long rows, int d, const bf16* __restrict__ dres = nullptr,
-                                                          long ldg = 0) {
+constexpr int rms_bwd_ctas = TPR == 32 ? (NV == 1 ? (MODE == 0 ? 4 : 3) : (MODE == 0 ? 3 : 2))
+                                       : (NV == 1 ? (MODE == 0 ? 4 : 2) : 1);
+template <int TPR, int NV, int MODE>
+__global__ void __launch_bounds__(256, rms_bwd_ctas<TPR, NV, MODE>)
+rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, const bf16* __restrict__ w, const bf16* __restrict__ dy,
+                   const float* __restrict__ rstd_in, bf16* __restrict__ dx, bf16* __restrict__ dg, float* __restrict__ partial,
+                   long rows, int d, const bf16* __restrict__ dres = nullptr, long ldg = 0) {
   __shared__ float red[8];
   __shared__ float dw_sh[(TPR == 32) ? 512 : 1];
   const int rows_per_cta = 256 / TPR;
@@ -191,9 +201,9 @@ __global__ void __launch_bounds__(256, NV == 1 ? (MODE == 0 && TPR == 256 ? 4 : 
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
     if (c < d) load8(w + c, wv[i]);
   }
-  // The next row's operands are in flight while this row is reduced (the reduction is two barriers long); rows of 8192
-  // would need too many registers for that and load when they are used.
-  constexpr bool AHEAD = NV <= 2;
+  // HELD: a row's operands are loaded together and kept as they came; AHEAD: one row early (rows of 8192 would need too
+  // many registers for that).
+  constexpr bool HELD = TPR == 256, AHEAD = HELD && NV <= 2;
   uint4 nx[NV], ndy[NV], ng[NV], nr[NV];
   auto fetch = [&](long row) {
     if (row >= rows) return;
@@ -213,7 +223,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? (MODE == 0 && TPR == 256 ? 4 : 
     const long row = base + sub;
     const bool active = row < rows;
     const float rstd = active ? rstd_in[row] : 0.f;
-    if (!AHEAD) fetch(row);
+    if (HELD && !AHEAD) fetch(row);
     uint4 cx[NV], cr[NV];
     float xn[NV][8], wdy[NV][8], gv[NV][8], sg[NV][8];
     float dot = 0.f;
@@ -222,11 +232,17 @@ __global__ void __launch_bounds__(256, NV == 1 ? (MODE == 0 && TPR == 256 ? 4 : 
       const int c = (t + i * TPR) * 8;
       if (active && c < d) {
         float xv[8], dv[8];
-        cx[i] = nx[i];
-        cr[i] = nr[i];
-        unpack8(nx[i], xv);
-        unpack8(ndy[i], dv);
-        if (MODE != 0) unpack8(ng[i], gv[i]);
+        if (HELD) {
+          cx[i] = nx[i];
+          cr[i] = nr[i];
+          unpack8(nx[i], xv);
+          unpack8(ndy[i], dv);
+          if (MODE != 0) unpack8(ng[i], gv[i]);
+        } else {
+          load8(x + row * d + c, xv);
+          load8(dy + row * d + c, dv);
+          if (MODE != 0) load8(g + row * (ldg ? ldg : d) + c, gv[i]);
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           float xin = xv[j];
@@ -257,7 +273,8 @@ __global__ void __launch_bounds__(256, NV == 1 ? (MODE == 0 && TPR == 256 ? 4 : 
         if (MODE == 2) {
           // norm input u = x*silu(g): dx = du*silu(g), dg = du*x*dsilu(g)
           float xv[8], og[8];
-          unpack8(cx[i], xv);
+          if (HELD) unpack8(cx[i], xv);
+          else load8(x + row * d + c, xv);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             og[j] = o[j] * xv[j] * dsilu_f(gv[i][j]);
@@ -269,7 +286,8 @@ __global__ void __launch_bounds__(256, NV == 1 ? (MODE == 0 && TPR == 256 ? 4 : 
         }
         if (dres != nullptr) {
           float rv[8];
-          unpack8(cr[i], rv);
+          if (HELD) unpack8(cr[i], rv);
+          else load8(dres + row * d + c, rv);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += rv[j];
         }

@@ -51,3 +51,43 @@ def test_norm_backward_rows(native, mode, rows, d):
         want = torch.autograd.grad(y, ref, dy.double())
     for a, b in zip(got, want):
         assert (a.double() - b).norm() <= 5e-3 * b.norm() + 1e-6                      # one rounding to bf16, fp32 inside
+
+
+@pytest.mark.parametrize("mode", ["before", "after"])
+@pytest.mark.parametrize("rows,d,pitch", [(3000, 128, 136), (1200, 512, 1024), (900, 4096, 8512), (500, 8192, 8200)])
+def test_gated_norm_backward_pitched_gate(native, mode, rows, d, pitch):
+    torch.manual_seed(pitch)
+    x, dy = (torch.randn(rows, d, device="cuda").bfloat16() for _ in range(2))
+    gate = torch.randn(rows, pitch, device="cuda").bfloat16()[:, pitch - d:]
+    w = (1 + 0.1 * torch.randn(d, device="cuda")).bfloat16()
+    leaves = [x.requires_grad_(), gate.requires_grad_(), w.requires_grad_()]
+    ref = [t.detach().double().requires_grad_() for t in leaves]
+    norm = lambda u, v: u * (u.square().mean(-1, keepdim=True) + 1e-6).rsqrt() * v     # noqa: E731
+    got = torch.autograd.grad(native.gated_rms_norm(*leaves, norm_before_gate=mode == "before"), leaves, dy)
+    y = norm(ref[0], ref[2]) * F.silu(ref[1]) if mode == "before" else norm(ref[0] * F.silu(ref[1]), ref[2])
+    for a, b in zip(got, torch.autograd.grad(y, ref, dy.double())):
+        assert (a.double() - b).norm() <= 5e-3 * b.norm() + 1e-6                      # one rounding to bf16, fp32 inside
+
+
+def test_norm_backward_of_many_narrow_rows_is_memory_bound(native):
+    # Rows of one warp live on resident warps.  Three tensors pass through memory; a copy kernel of as many bytes is the
+    # yardstick: 2.1 times its time with four CTAs per SM, 4.1 times with two.
+    rows, d = 1 << 20, 128
+    x, dy = (torch.randn(rows, d, device="cuda").bfloat16().requires_grad_(i == 0) for i in range(2))
+    w = torch.ones(d, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    y = native.rms_norm(x, w)
+    src, dst = (torch.empty(rows * d * 3 // 2, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+
+    def fastest(call):
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            call()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times[2:])
+
+    copy = fastest(lambda: dst.copy_(src))
+    assert fastest(lambda: torch.autograd.grad(y, [x, w], dy, retain_graph=True)) <= 3.1 * copy
