@@ -832,7 +832,10 @@ class _LinearCE(torch.autograd.Function):
 
 
 def _scaled_by(t: Tensor, s: Tensor, dtype: torch.dtype) -> Tensor:
-    """t * s rounded once to ``dtype``, s a one-element tensor: one pass for bf16 results."""
+    """t * s rounded once to ``dtype``, s a one-element tensor: one pass for bf16 results.  Tensor arithmetic where the
+    product is differentiated again with respect to s, or s stands for a batch of factors."""
+    if (torch.is_grad_enabled() and s.requires_grad) or not torch._C._has_storage(s):     # a batch under vmap has none
+        return (t * s).to(dtype)
     if dtype != torch.bfloat16 or t.dtype not in (torch.float32, torch.bfloat16) or not t.is_contiguous() or t.data_ptr() % 16:
         return (t * s).to(dtype)
     out = _empty(t.shape, dtype=dtype, device=t.device)

@@ -26,6 +26,30 @@ def test_linear_cross_entropy_rows(native, N, V):
         assert a.dtype == torch.bfloat16 and (a.double() - b).norm() <= 1.5e-2 * b.norm()
 
 
+def test_linear_cross_entropy_gradient_of_the_upstream_factor(native):
+    torch.manual_seed(0)
+    h = torch.randn(40, 64, device="cuda").bfloat16().requires_grad_()
+    w = (torch.randn(512, 64, device="cuda") * 0.2).bfloat16().requires_grad_()
+    labels = torch.randint(0, 512, (40,), device="cuda")
+    loss = native.linear_cross_entropy(h, w, labels)
+    plain = torch.autograd.grad(loss, [h, w], retain_graph=True)
+    # a batch of factors
+    factors = torch.tensor([1.0, -2.0, 0.5], device="cuda")
+    many = torch.autograd.grad(loss, [h, w], factors, is_grads_batched=True, retain_graph=True)
+    for m, g in zip(many, plain):
+        assert m.dtype == g.dtype and torch.equal(m, torch.stack([g, -2.0 * g, 0.5 * g]))     # powers of two: exact
+    # the gradient is linear in the factor, and its derivative with respect to the factor is the plain gradient
+    a = torch.tensor(1.0, device="cuda", requires_grad=True)
+    got = torch.autograd.grad(loss * a, [h, w], create_graph=True)
+    for g, ref in zip(got, plain):
+        assert torch.equal(g, ref)
+        c = torch.randn_like(ref, dtype=torch.float32)
+        slope, = torch.autograd.grad((g.float() * c).sum(), a, retain_graph=True)
+        want = (ref.float() * c).sum()
+        # bf16 products (dh) enter the sum: one rounding of 2^-9 per term at most
+        assert abs(float(slope - want)) <= 2 ** -8 * float((ref.float() * c).abs().sum())
+
+
 @pytest.mark.parametrize("mode", ["plain", "add", "before", "after"])
 @pytest.mark.parametrize("rows,d", [(1, 256), (7, 512), (3000, 256), (6000, 264), (1, 2048), (593, 2048), (1300, 1000), (700, 4096), (600, 8192)])
 def test_norm_backward_rows(native, mode, rows, d):
