@@ -60,7 +60,8 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
   float* gs = reinterpret_cast<float*>(sTw + CH * PC);
   float* bs = gs + CH;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int bh = blockIdx.x, c = blockIdx.y, h = bh % p.H, b = bh / p.H;   // heads fastest: neighbouring pieces of token rows together
+  const int bh = blockIdx.x, h = bh % p.H, b = bh / p.H, c = blockIdx.z * gridDim.y + blockIdx.y;   // see chunk_grid
+  if (c >= p.NC) return;
   const int t0 = c * CH;
   const long tok0 = static_cast<long>(b) * p.T * p.H + h;  // (b, t, h) = tok0 + t * H
   for (int i = tid; i < CH * (KD / 8); i += 256) {
@@ -302,7 +303,8 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
   bf16* sDK = sTw + CH * PC;                               // d(k k^T)
   bf16* sDQ = sDK + CH * PC;                               // d(q k^T)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int bh = blockIdx.x, c = blockIdx.y, h = bh % p.H, b = bh / p.H;   // heads fastest: neighbouring pieces of token rows together
+  const int bh = blockIdx.x, h = bh % p.H, b = bh / p.H, c = blockIdx.z * gridDim.y + blockIdx.y;   // see chunk_grid
+  if (c >= p.NC) return;
   const int t0 = c * CH, V = p.V, nvt = V / CH;
   const long tok0 = static_cast<long>(b) * p.T * p.H + h;
   const long chunk = static_cast<long>(bh) * p.NC + c;
@@ -685,6 +687,9 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
   }
   if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 512); }
 }
+// One CTA per (chunk, head), heads fastest so that CTAs that run together touch neighbouring pieces of the same token rows.
+// y ends at 65535 chunks (4.2 M tokens); longer sequences go on in z, whose last layer may reach past the end.
+dim3 chunk_grid(int BH, int NC) { return dim3(BH, NC < 65535 ? NC : 65535, (NC + 65534) / 65535); }
 }  // namespace
 
 // q, k [B, T, H, 128], v [B, T, H, V] bf16 contiguous, g (log-decay) and beta [B, T, H] fp32 -> w, u, qk, gc and, where
@@ -697,7 +702,7 @@ extern "C" int nsa_gdn_prep(const void* q, const void* k, const void* v, const f
   const int smem = 2 * CH * PK * 2 + CH * (V + 8) * 2 + 2 * CH * PX * 4 + 2 * CH * PC * 2 + 2 * CH * 4;
   cudaError_t e = cudaFuncSetAttribute(gdn_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn prep smem attribute");
-  gdn_prep_kernel<<<dim3(B * H, NC), 256, smem, st>>>(p);
+  gdn_prep_kernel<<<chunk_grid(B * H, NC), 256, smem, st>>>(p);
   nsa::count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_prep launch");
@@ -729,7 +734,7 @@ extern "C" int nsa_gdn_post(const void* q, const void* k, const void* v, const v
                nsa::status_ptr()};
   cudaError_t e = cudaFuncSetAttribute(gdn_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, POST_SMEM);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn post smem attribute");
-  gdn_post_kernel<<<dim3(B * H, NC), 512, POST_SMEM, st>>>(tdu, tdo, tvn, tv, tS, tdS, p);
+  gdn_post_kernel<<<chunk_grid(B * H, NC), 512, POST_SMEM, st>>>(tdu, tdo, tvn, tv, tS, tdS, p);
   nsa::count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_post launch");

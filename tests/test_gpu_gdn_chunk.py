@@ -53,3 +53,24 @@ def test_gdn_strided_unaligned_bf16_gates(native):
     with torch.no_grad():
         b = native.gated_delta_rule(q, k, v, g, beta)
     assert torch.equal(a, b)
+
+
+def test_gdn_more_chunks_than_a_second_grid_dimension_holds(native):
+    # 65540 chunks of 64 tokens.  Decays of e^-3 per chunk at least: what is more than a hundred chunks away is gone, so both ends
+    # equal runs over the ends alone.
+    T, n, keep = 65540 * 64, 128 * 64, 16 * 64
+    inputs = _inputs(1, T, 1, 64, 0.2)
+    inputs[3] -= 0.05
+
+    def run(ts, dy):
+        leaves = [t.detach().requires_grad_() for t in ts]
+        o = native.gated_delta_rule(*leaves)
+        return [o.detach()] + list(torch.autograd.grad(o, leaves, dy))
+
+    dy = torch.randn(1, T, 1, 64, device="cuda").bfloat16()
+    whole = run(inputs, dy)
+    for part, kept in ((slice(0, n), slice(0, keep)), (slice(T - n, T), slice(n - keep, n))):
+        ends = run([t[:, part] for t in inputs], dy[:, part])
+        for a, b in zip(whole, ends):
+            a, b = a[:, part][:, kept].double(), b[:, kept].double()
+            assert b.norm() > 0 and (a - b).norm() <= 2 ** -8 * b.norm()
