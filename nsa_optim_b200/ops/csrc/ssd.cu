@@ -120,7 +120,7 @@ struct SsdParams {
   const float* dt;     // [B, T, H] (after softplus)
   const float* A;      // [H] (negative)
   const float* Dskip;  // [H] or null
-  int B, T, H, nc;
+  int B, T, H, nc, c0; // c0: first chunk of the launch
   // chunk_state
   float* S_out;        // [B, nc, H, NS, PD] fp32
   float* gamma_out;    // [B, nc, H] or null
@@ -165,7 +165,7 @@ ssd_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_c
   float* warp_tot = dts + L;
 
   const int r = threadIdx.x, warp = r >> 5;
-  const int h = blockIdx.x, c = blockIdx.y, b = blockIdx.z;    // heads fastest: see the launches
+  const int h = blockIdx.x, c = p.c0 + blockIdx.y, b = blockIdx.z;    // see each_slab
   const int t0 = c * L;
   if (r == 0) {
     *abort_flag = 0;
@@ -267,7 +267,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   float* warp_tot = dts + L;
 
   const int r = threadIdx.x & 127, half = threadIdx.x >> 7, warp = threadIdx.x >> 5;   // row, column half
-  const int h = blockIdx.x, c = blockIdx.y, b = blockIdx.z;    // heads fastest: see the launches
+  const int h = blockIdx.x, c = p.c0 + blockIdx.y, b = blockIdx.z;    // see each_slab
   const int t0 = c * L;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -428,7 +428,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
   float* part = warp_tot + 8;          // [4 groups][128] row sums on their way to one
 
   const int r = threadIdx.x & 127, grp = threadIdx.x >> 7, warp = threadIdx.x >> 5;    // row, column group
-  const int h = blockIdx.x, c = blockIdx.y, b = blockIdx.z;    // heads fastest: see the launches
+  const int h = blockIdx.x, c = p.c0 + blockIdx.y, b = blockIdx.z;    // see each_slab
   const int t0 = c * L;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -846,6 +846,19 @@ __global__ void __launch_bounds__(1024) ssd_head_sums_kernel(const float* __rest
   if (l == 0 && hg < H) (blockIdx.y ? dD : dA)[hg] = s;
 }
 
+// Launches of one CTA per (chunk, head, sequence).  Heads vary fastest: a head's row of a token is 128 bytes, so CTAs that run
+// together read and write neighbouring pieces of the same rows, and share the chunk's B and C tiles in L2.  A grid's second
+// dimension ends at 65535, so chunks go in slabs of that many (8.4 M tokens).
+template <typename F>
+void each_slab(SsdParams& p, F launch) {
+  p.c0 = 0;
+  do {                                             // no tokens: the launch reports an empty grid
+    launch(dim3(p.H, p.nc - p.c0 < 65535 ? p.nc - p.c0 : 65535, p.B));
+    nsa::count_launch();
+    p.c0 += 65535;
+  } while (p.c0 < p.nc);
+}
+
 int map_bc(CUtensorMap* m, const void* base, int B, int T, long ld) {
   uint64_t dims[3] = {(uint64_t)NS, (uint64_t)T, (uint64_t)B};
   uint64_t strides[2] = {(uint64_t)ld * 2, (uint64_t)T * ld * 2};
@@ -922,19 +935,15 @@ extern "C" int nsa_ssd_chunk_state(int mode, const void* bc, long ld_bc, const v
   p.dt = dt; p.A = A; p.B = B; p.T = T; p.H = H; p.nc = (T + L - 1) / L;
   p.S_out = S_out; p.gamma_out = gamma_out; p.status = nsa::status_ptr();
   const int smem = 3 * BOXB + 1024 + 2048;
-  // Heads vary fastest in all three chunk kernels: a head's row of a token is 128 bytes, so CTAs that run together read
-  // and write neighbouring pieces of the same rows, and share the chunk's B and C tiles in L2.
-  const dim3 grid(H, p.nc, B);
   if (mode == 0) {
     static bool cfg = false;
     if (!cfg) { if ((rc = smem_attr(ssd_chunk_state_kernel<0>, smem))) return rc; cfg = true; }
-    ssd_chunk_state_kernel<0><<<grid, 128, smem, st>>>(tb, tv, p);
+    each_slab(p, [&](dim3 grid) { ssd_chunk_state_kernel<0><<<grid, 128, smem, st>>>(tb, tv, p); });
   } else {
     static bool cfg = false;
     if (!cfg) { if ((rc = smem_attr(ssd_chunk_state_kernel<1>, smem))) return rc; cfg = true; }
-    ssd_chunk_state_kernel<1><<<grid, 128, smem, st>>>(tb, tv, p);
+    each_slab(p, [&](dim3 grid) { ssd_chunk_state_kernel<1><<<grid, 128, smem, st>>>(tb, tv, p); });
   }
-  nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_chunk_state launch");
 }
@@ -958,8 +967,7 @@ extern "C" int nsa_ssd_chunk_out(const void* Cm, long ld_c, const void* Bm, long
   static bool cfg = false;
   if (!cfg) { if ((rc = smem_attr(ssd_chunk_out_kernel, smem))) return rc; cfg = true; }
   if ((rc = map_v(&ty, y, B, T, H, static_cast<long>(H) * PD))) return rc;
-  ssd_chunk_out_kernel<<<dim3(H, nc, B), 256, smem, st>>>(tc, tb, tx, th, ty, p);
-  nsa::count_launch();
+  each_slab(p, [&](dim3 grid) { ssd_chunk_out_kernel<<<grid, 256, smem, st>>>(tc, tb, tx, th, ty, p); });
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_chunk_out launch");
 }
@@ -993,8 +1001,7 @@ static int ssd_chunk_grad_impl(const void* Cm, long ld_c, const void* Bm, long l
   const int smem = 13 * BOXB + 1024 + 2048 + 16 * L * 4;
   static bool cfg = false;
   if (!cfg) { if ((rc = smem_attr(ssd_chunk_grad_kernel, smem))) return rc; cfg = true; }
-  ssd_chunk_grad_kernel<<<dim3(H, nc, B), 512, smem, st>>>(tc, tb, tx, tdy, th, tdh, tdx, tdbh, tdch, p);
-  nsa::count_launch();
+  each_slab(p, [&](dim3 grid) { ssd_chunk_grad_kernel<<<grid, 512, smem, st>>>(tc, tb, tx, tdy, th, tdh, tdx, tdbh, tdch, p); });
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_chunk_grad launch");
 }

@@ -57,3 +57,31 @@ def test_state_pass(native, nc, E, back):
         st = gamma[:, c, :, None].double() * st + S[:, c].double()
     assert (out.double() - want).abs().max() <= 1e-5 * want.abs().max() + 1e-12     # one fp32 rounding per chunk, decaying
     assert torch.equal(out_bf, out.to(torch.bfloat16))
+
+
+def test_ssd_more_chunks_than_a_second_grid_dimension_holds(native):
+    # 65540 chunks of 128 tokens, one head.  Decays of e^-6 per chunk at least: what is more than fifty chunks away is gone, so
+    # both ends equal runs over the ends alone.
+    torch.manual_seed(0)
+    T, n, keep = 65540 * 128 - 28, 100 * 128, 16 * 128
+    xbc = torch.randn(1, T, 320, device="cuda", dtype=torch.bfloat16)
+    dy = torch.randn(1, T, 1, 64, device="cuda", dtype=torch.bfloat16)
+    dt, A, D = torch.rand(1, T, 1, device="cuda") * 0.05 + 0.05, -torch.ones(1, device="cuda"), torch.ones(1, device="cuda")
+
+    def run(part):
+        x = xbc[:, part]
+        leaves = [t.detach().requires_grad_() for t in (x[..., :64].unflatten(-1, (1, 64)), dt[:, part], A,
+                                                        x[..., 64:192].unsqueeze(2), x[..., 192:].unsqueeze(2), D)]
+        y = native.ssd_scan(*leaves)
+        dx, ddt, _, dB, dC, dD = torch.autograd.grad(y, leaves, dy[:, part])
+        return [y.detach(), dx, dB, dC, ddt], dD
+
+    whole, dD = run(slice(0, T))
+    want = (xbc[..., :64].double() * dy[:, :, 0].double()).sum()
+    assert abs(float(dD - want)) <= 1e-3 * T ** 0.5 * 8                              # a sum of 64 T products of size one
+    tail = T - n + 28                                                                # on a chunk boundary
+    for part, kept, outputs in ((slice(0, n), slice(0, keep), 4), (slice(tail, T), slice(n - keep - 128, None), 5)):
+        # ddt is a sum over all later tokens, whose rounding is not that of a shorter run's: compared at the end only
+        for a, b in list(zip(whole, run(part)[0]))[:outputs]:
+            a, b = a[:, part][:, kept].double(), b[:, kept].double()
+            assert b.shape[1] >= 1 and b.norm() > 0 and (a - b).norm() <= 2 ** -8 * b.norm()
