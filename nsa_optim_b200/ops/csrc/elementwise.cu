@@ -1228,9 +1228,11 @@ extern "C" int nsa_rope(const void* x, const float* cos_t, const float* sin_t, v
 }
 
 // Time steps per warp: 64 keeps the rows read twice (3 of x ahead of a segment, 3 of dpre behind it) under
-// a tenth; short sequences take 32, 16 or 8 so that every SM still finds 32 warps.
+// a tenth; short sequences take 32, 16 or 8 so that every SM still finds 32 warps; beyond 8.4 M steps 128 or 256, so that the
+// grid's second dimension (at most 65535) reaches as far as 33.5 M.
 static int conv_rows(int B, int T, int C) {
   int rows = 64;
+  while (rows < 256 && static_cast<long>(rows) * CT_TW * 65535 < T) rows <<= 1;
   auto warps = [&](int r) { return static_cast<long>(B) * ((C + CT_C - 1) / CT_C) * ((T + r - 1) / r); };
   while (rows > 8 && warps(rows) < 32L * nsa::sm_count()) rows >>= 1;
   return rows;

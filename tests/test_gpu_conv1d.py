@@ -32,3 +32,7 @@ def test_conv1d_segments(native, B, T, C, act, bias, wdt):
         assert (a.double() - r).abs().max() <= 5e-3 * r.abs().max() + 1e-5
     short = oracle.causal_conv1d(x.detach(), w.detach().to(torch.bfloat16), None if b is None else b.detach().to(torch.bfloat16), act)
     assert (got[0].float() - short.float()).abs().max() <= 2 ** -7 * short.float().abs().max() + 1e-5
+
+
+def test_conv1d_past_65535_segments(native):
+    test_conv1d_segments(native, 1, 8388500, 8, True, True, torch.bfloat16)
