@@ -80,3 +80,21 @@ def test_list_of_8bit_updates_equals_single_calls(native, pdt, gdt):
         assert all(torch.equal(s, t) for s, t in zip(x, y))
     with pytest.raises(ValueError):
         native.adamw8bit_multi([(torch.zeros(100, device="cuda"),) * 6], 1, *HYPER, None, 256)
+
+
+def test_unaligned_update_keeps_its_accesses_coalesced(native):
+    # one element off, 2^26 bf16 parameters: 315 us against 241 aligned; 473 where a thread takes four neighbours one by one
+    def fastest(off):
+        p, g = (torch.randn((1 << 26) + off, device="cuda").bfloat16()[off:] for _ in range(2))
+        m, v = torch.zeros(p.numel(), device="cuda"), torch.zeros(p.numel(), device="cuda")
+        times = []
+        for t in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            native.adamw_step(p, g, m, v, None, t + 1, *HYPER, None)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times[2:])
+
+    assert fastest(1) <= 1.55 * fastest(0)
