@@ -626,9 +626,11 @@ __global__ void __launch_bounds__(256) rope_kernel(const bf16* __restrict__ x, c
 // with the last three rows in registers, so every element is read and widened once.  The rows ahead
 // travel through a ring of shared memory that a lane fills (cp.async) and reads for itself alone: no barriers,
 // and 12 rows of a warp stay in flight without holding registers.  The taps are packed fp32 FMAs (two channels per
-// instruction).  A CTA is four channel tiles (1 KB of a row) by two time segments.
+// instruction).  A CTA is CW channel tiles by 8 / CW time segments: four tiles (1 KB of a row) where there are as many, one or
+// two for tensors of up to 128 or 256 channels, whose warps would otherwise have nothing to do (524288 x 128,
+// forward and backward: 565 us with six idle warps in eight, 181 now).
 // ------------------------------------------------------------------------------------
-constexpr int CT_CW = 4, CT_TW = 2, CT_WARPS = CT_CW * CT_TW, CT_C = 128, CT_U = 4, CT_RING = 4;
+constexpr int CT_WARPS = 8, CT_C = 128, CT_U = 4, CT_RING = 4;
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pred) {   // zero fill when !pred
   const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -680,13 +682,14 @@ __device__ __forceinline__ void conv_taps(const bf16* __restrict__ w, const bf16
   bv = Quad{make_float2(s[0], s[1]), make_float2(s[2], s[3])};
 }
 
+template <int CW>
 __global__ void __launch_bounds__(CT_WARPS * 32, 4) conv1d_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                                       const bf16* __restrict__ bias, bf16* __restrict__ y,
                                                                       int T, int C, long ldx, int act, int rows) {
   __shared__ uint2 ring_all[CT_WARPS][CT_RING * CT_U][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = (blockIdx.x * CT_CW + warp % CT_CW) * CT_C + lane * 4;
-  const int t0 = (blockIdx.y * CT_TW + warp / CT_CW) * rows;
+  const int c = (blockIdx.x * CW + warp % CW) * CT_C + lane * 4;
+  const int t0 = (blockIdx.y * (CT_WARPS / CW) + warp / CW) * rows;
   if (c >= C || t0 >= T) return;
   uint2(*ring)[32] = ring_all[warp];
   const bf16* xp = x + static_cast<long>(blockIdx.z) * T * ldx + c;
@@ -733,6 +736,7 @@ __global__ void __launch_bounds__(CT_WARPS * 32, 4) conv1d_fwd_kernel(const bf16
 struct ConvBwdSmem {
   uint2 x[CT_WARPS][CT_RING * CT_U][32], g[CT_WARPS][CT_RING * CT_U][32];
 };
+template <int CW>
 __global__ void __launch_bounds__(CT_WARPS * 32, 2) conv1d_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                                       const bf16* __restrict__ bias, const bf16* __restrict__ dy,
                                                                       bf16* __restrict__ dx, float* __restrict__ partial,
@@ -740,8 +744,8 @@ __global__ void __launch_bounds__(CT_WARPS * 32, 2) conv1d_bwd_kernel(const bf16
   extern __shared__ __align__(16) uint8_t conv_smem[];
   ConvBwdSmem& sm = *reinterpret_cast<ConvBwdSmem*>(conv_smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = (blockIdx.x * CT_CW + warp % CT_CW) * CT_C + lane * 4;
-  const int t0 = (blockIdx.y * CT_TW + warp / CT_CW) * rows;
+  const int c = (blockIdx.x * CW + warp % CW) * CT_C + lane * 4;
+  const int t0 = (blockIdx.y * (CT_WARPS / CW) + warp / CW) * rows;
   Quad dw[4], db = quad_zero();
 #pragma unroll
   for (int j = 0; j < 4; ++j) dw[j] = quad_zero();
@@ -808,35 +812,38 @@ __global__ void __launch_bounds__(CT_WARPS * 32, 2) conv1d_bwd_kernel(const bf16
   *reinterpret_cast<float4*>(&sred[warp][4][lane * 4]) = make_float4(db.a.x, db.a.y, db.b.x, db.b.y);
   __syncthreads();
   float* pp = partial + (static_cast<long>(blockIdx.z) * gridDim.y + blockIdx.y) * 5 * C;
-  for (int e = threadIdx.x; e < 5 * CT_CW * CT_C; e += CT_WARPS * 32) {
-    const int j = e / (CT_CW * CT_C), cc = e - j * (CT_CW * CT_C);
-    const int cg = blockIdx.x * CT_CW * CT_C + cc;
+  for (int e = threadIdx.x; e < 5 * CW * CT_C; e += CT_WARPS * 32) {
+    const int j = e / (CW * CT_C), cc = e - j * (CW * CT_C);
+    const int cg = blockIdx.x * CW * CT_C + cc;
     if (cg >= C) continue;
     float acc = 0.f;
 #pragma unroll
-    for (int ti = 0; ti < CT_TW; ++ti) acc += sred[ti * CT_CW + cc / CT_C][j][cc % CT_C];
+    for (int ti = 0; ti < CT_WARPS / CW; ++ti) acc += sred[ti * CW + cc / CT_C][j][cc % CT_C];
     pp[static_cast<long>(j) * C + cg] = acc;
   }
 }
 
-// partial [parts][5][C] -> dw (C, 4) and db (C), fp32 or bf16, in a fixed order.  CTA: 32 channels, 8 groups of parts.
-template <typename OT>
-__global__ void __launch_bounds__(256) conv1d_dw_kernel(const float* __restrict__ partial, int parts, int C,
-                                                        OT* __restrict__ dw, OT* __restrict__ db) {
-  __shared__ float s[8][5][32];
+// partial [parts][5][C] -> dw (C, 4) and db (C), fp32 or bf16, in a fixed order.  CTA: 32 channels, G groups of parts: 8 warps for
+// the few hundred parts of wide tensors, 32 where few channels leave thousands of parts to few CTAs.
+template <typename OT, int G>
+__global__ void __launch_bounds__(G * 32) conv1d_dw_kernel(const float* __restrict__ partial, int parts, int C,
+                                                           OT* __restrict__ dw, OT* __restrict__ db) {
+  __shared__ float s[G][5][32];
   const int cl = threadIdx.x & 31, g = threadIdx.x >> 5, c = blockIdx.x * 32 + cl;
   float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  if (c < C)
-    for (int p = g; p < parts; p += 8)
+  if (c < C) {
+#pragma unroll 4
+    for (int p = g; p < parts; p += G)
 #pragma unroll
       for (int j = 0; j < 5; ++j) acc[j] += partial[(static_cast<long>(p) * 5 + j) * C + c];
+  }
 #pragma unroll
   for (int j = 0; j < 5; ++j) s[g][j][cl] = acc[j];
   __syncthreads();
   if (g >= 5 || c >= C) return;
   float v = 0.f;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) v += s[k][g][cl];
+  for (int k = 0; k < G; ++k) v += s[k][g][cl];
   if (g < 4) dw[static_cast<long>(c) * 4 + g] = static_cast<OT>(v);
   else if (db) db[c] = static_cast<OT>(v);
 }
@@ -1227,25 +1234,32 @@ extern "C" int nsa_rope(const void* x, const float* cos_t, const float* sin_t, v
   return 0;
 }
 
+// Channel tiles of a CTA.
+static int conv_tiles(int C) { return C <= CT_C ? 1 : C <= 2 * CT_C ? 2 : 4; }
 // Time steps per warp: 64 keeps the rows read twice (3 of x ahead of a segment, 3 of dpre behind it) under
-// a tenth; short sequences take 32, 16 or 8 so that every SM still finds 32 warps; beyond 8.4 M steps 128 or 256, so that the
-// grid's second dimension (at most 65535) reaches as far as 33.5 M.
+// a tenth; short sequences take 32, 16 or 8 so that every SM still finds 32 warps; beyond 8.4 M steps (of two segments
+// a CTA) 128 or 256, so that the grid's second dimension (at most 65535) reaches as far as 33.5 M.
 static int conv_rows(int B, int T, int C) {
   int rows = 64;
-  while (rows < 256 && static_cast<long>(rows) * CT_TW * 65535 < T) rows <<= 1;
+  while (rows < 256 && static_cast<long>(rows) * (CT_WARPS / conv_tiles(C)) * 65535 < T) rows <<= 1;
   auto warps = [&](int r) { return static_cast<long>(B) * ((C + CT_C - 1) / CT_C) * ((T + r - 1) / r); };
   while (rows > 8 && warps(rows) < 32L * nsa::sm_count()) rows >>= 1;
   return rows;
 }
 static dim3 conv_grid(int B, int T, int C, int rows) {
-  return dim3((C + CT_CW * CT_C - 1) / (CT_CW * CT_C), (T + CT_TW * rows - 1) / (CT_TW * rows), B);
+  const int cw = conv_tiles(C), steps = CT_WARPS / cw * rows;
+  return dim3((C + cw * CT_C - 1) / (cw * CT_C), static_cast<unsigned>((static_cast<long>(T) + steps - 1) / steps), B);
 }
 extern "C" int nsa_conv1d_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, long ldx,
                               int width, int act, cudaStream_t st) {
   if (C % 8 || ldx % 8 || width != 4) return nsa::fail(NSA_ERR_SHAPE, "conv1d: channels multiple of 8 and width 4 required");
   const int rows = conv_rows(B, T, C);
   const dim3 grid = conv_grid(B, T, C, rows);
-  conv1d_fwd_kernel<<<grid, CT_WARPS * 32, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)y, T, C, ldx, act, rows);
+#define NSA_CONV_FWD(CW) \
+  conv1d_fwd_kernel<CW><<<grid, CT_WARPS * 32, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)y, T, C, ldx, act, rows)
+  const int cw = conv_tiles(C);
+  if (cw == 1) NSA_CONV_FWD(1); else if (cw == 2) NSA_CONV_FWD(2); else NSA_CONV_FWD(4);
+#undef NSA_CONV_FWD
   nsa::count_launch();
   return 0;
 }
@@ -1260,17 +1274,21 @@ extern "C" int nsa_conv1d_bwd(const void* x, const void* w, const void* bias, co
   const int rows = conv_rows(B, T, C);
   const dim3 grid = conv_grid(B, T, C, rows);
   static_assert(sizeof(ConvBwdSmem) >= CT_WARPS * 5 * CT_C * 4, "conv1d: reduction buffer");
-  static bool cfg = false;
-  if (!cfg) {
-    cudaError_t e = cudaFuncSetAttribute(conv1d_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ConvBwdSmem));
+  const int cw = conv_tiles(C);
+  auto* kernel = cw == 1 ? conv1d_bwd_kernel<1> : cw == 2 ? conv1d_bwd_kernel<2> : conv1d_bwd_kernel<4>;
+  static bool cfg[3] = {};
+  if (!cfg[cw / 2]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ConvBwdSmem));
     if (e != cudaSuccess) return nsa::fail_cuda(e, "conv1d_bwd: shared memory attribute");
-    cfg = true;
+    cfg[cw / 2] = true;
   }
-  conv1d_bwd_kernel<<<grid, CT_WARPS * 32, sizeof(ConvBwdSmem), st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (const bf16*)dy, (bf16*)dx,
+  kernel<<<grid, CT_WARPS * 32, sizeof(ConvBwdSmem), st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (const bf16*)dy, (bf16*)dx,
                                                     partial, T, C, ldx, act, rows);
   const int parts = static_cast<int>(nsa_conv1d_bwd_parts(B, T, C));
-  if (dw_fp32) conv1d_dw_kernel<float><<<(C + 31) / 32, 256, 0, st>>>(partial, parts, C, (float*)dw, (float*)db);
-  else conv1d_dw_kernel<bf16><<<(C + 31) / 32, 256, 0, st>>>(partial, parts, C, (bf16*)dw, (bf16*)db);
+#define NSA_CONV_DW(OT, G) conv1d_dw_kernel<OT, G><<<(C + 31) / 32, G * 32, 0, st>>>(partial, parts, C, (OT*)dw, (OT*)db)
+  if (parts <= 256) { if (dw_fp32) NSA_CONV_DW(float, 8); else NSA_CONV_DW(bf16, 8); }
+  else { if (dw_fp32) NSA_CONV_DW(float, 32); else NSA_CONV_DW(bf16, 32); }
+#undef NSA_CONV_DW
   nsa::count_launch(2);
   return 0;
 }

@@ -35,4 +35,49 @@ def test_conv1d_segments(native, B, T, C, act, bias, wdt):
 
 
 def test_conv1d_past_65535_segments(native):
-    test_conv1d_segments(native, 1, 8388500, 8, True, True, torch.bfloat16)
+    # both ends against runs over the ends alone, the weight gradient against sums of pieces in 64 bits
+    torch.manual_seed(0)
+    T, C, n = 8388500, 264, 1000
+    x, dy = (torch.randn(1, T, C, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    w = (torch.randn(C, 4, device="cuda") * 0.4).requires_grad_()
+
+    def run(part):
+        xs = x[:, part].detach().requires_grad_()
+        y = native.causal_conv1d(xs, w, None, False)
+        return [y.detach()] + list(torch.autograd.grad(y, [xs, w], dy[:, part]))
+
+    y, dx, dw = run(slice(0, T))
+    ys, dxs, _ = run(slice(0, n + 3))
+    assert torch.equal(y[:, :n], ys[:, :n]) and torch.equal(dx[:, :n], dxs[:, :n])
+    ys, dxs, _ = run(slice(T - n, T))
+    assert torch.equal(y[:, T - n + 3:], ys[:, 3:]) and torch.equal(dx[:, T - n:], dxs)
+    want = torch.zeros(C, 4, device="cuda", dtype=torch.float64)
+    for s in range(0, T, 1 << 18):
+        e = min(T, s + (1 << 18))
+        xs = torch.nn.functional.pad(x[0, max(0, s - 3):e].double(), (0, 0, 3 - min(s, 3), 0))
+        want += torch.stack([(dy[0, s:e].double() * xs[j:j + e - s]).sum(0) for j in range(4)], 1)
+    assert (dw.double() - want).norm() <= 1e-5 * T ** 0.5 * want.numel() ** 0.5    # sums of T products of size one, in fp32
+
+
+def test_conv1d_backward_of_few_channels_fills_the_sms(native):
+    # 128 channels are one tile: all eight warps of a CTA take time segments.  A copy of as many bytes is the yardstick
+    T, C = 1 << 19, 128
+    x, dy = (torch.randn(1, T, C, device="cuda").bfloat16().requires_grad_(i == 0) for i in range(2))
+    w = torch.randn(C, 4, device="cuda").bfloat16().requires_grad_()
+    y = native.causal_conv1d(x, w, None, True)
+    src, dst = (torch.empty(3 * T * C // 2, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+
+    def fastest(call):
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            call()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times[2:])
+
+    copy = fastest(lambda: dst.copy_(src))
+    back = fastest(lambda: torch.autograd.grad(y, [x, w], dy, retain_graph=True))
+    assert back <= 4.5 * copy, (back, copy)
