@@ -308,79 +308,6 @@ __global__ void __launch_bounds__(256) cross_entropy_kernel(bf16* __restrict__ l
   }
 }
 
-// The same for rows of at most 32768 logits, a multiple of 8: the row is read once and stays in registers as bf16 (eight
-// 16-byte pieces per thread) between the maximum, the sum and the gradient, so memory sees one read and one write.
-constexpr int CE_THREADS = 512, CE_PIECES = 8;
-__global__ void __launch_bounds__(CE_THREADS, 2) cross_entropy_row_kernel(bf16* __restrict__ logits, const long* __restrict__ labels,
-                                                                          float* __restrict__ loss_out, const float* __restrict__ inv_count,
-                                                                          int V, long ld, long ignore_index, int write_grad,
-                                                                          KernelStatus* status) {
-  __shared__ float red[CE_THREADS / 32], red2[CE_THREADS / 32], at_label;
-  const long row = blockIdx.x;
-  bf16* lp = logits + row * ld;
-  const long label = labels[row];
-  const bool ignored = (label == ignore_index) || label < 0 || label >= V;
-  if (threadIdx.x == 0) {
-    NSA_CHECK_INDEX(label == ignore_index || (label >= 0 && label < V), status, label);
-    at_label = ignored ? 0.f : __bfloat162float(lp[label]);
-  }
-  const int V8 = V / 8;
-  uint4 u[CE_PIECES];
-  float mx = -INFINITY;
-#pragma unroll
-  for (int k = 0; k < CE_PIECES; ++k) {
-    const int i = threadIdx.x + k * CE_THREADS;
-    // absent pieces hold -inf, which adds nothing anywhere
-    u[k] = i < V8 ? *reinterpret_cast<const uint4*>(lp + i * 8) : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);
-  }
-#pragma unroll
-  for (int k = 0; k < CE_PIECES; ++k) {
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[k]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(h[j]); mx = fmaxf(mx, fmaxf(f.x, f.y)); }
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  mx = warp_max(mx);
-  if (l == 0) red[w] = mx;
-  __syncthreads();
-  mx = red[0];
-#pragma unroll
-  for (int k = 1; k < CE_THREADS / 32; ++k) mx = fmaxf(mx, red[k]);
-  float s = 0.f;
-#pragma unroll
-  for (int k = 0; k < CE_PIECES; ++k) {
-    if (threadIdx.x + k * CE_THREADS >= V8) break;
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[k]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(h[j]); s += __expf(f.x - mx) + __expf(f.y - mx); }
-  }
-  s = warp_sum(s);
-  if (l == 0) red2[w] = s;
-  __syncthreads();
-  s = 0.f;
-#pragma unroll
-  for (int k = 0; k < CE_THREADS / 32; ++k) s += red2[k];
-  const float lse = mx + __logf(s);
-  if (threadIdx.x == 0) loss_out[row] = ignored ? 0.f : lse - at_label;
-  if (!write_grad) return;
-  const float scale = ignored ? 0.f : *inv_count;
-#pragma unroll
-  for (int k = 0; k < CE_PIECES; ++k) {
-    const int i = threadIdx.x + k * CE_THREADS;
-    if (i >= V8) break;
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u[k]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 f = __bfloat1622float2(h[j]);
-      const int c = i * 8 + 2 * j;
-      f.x = (__expf(f.x - lse) - (c == label ? 1.f : 0.f)) * scale;
-      f.y = (__expf(f.y - lse) - (c + 1 == label ? 1.f : 0.f)) * scale;
-      h[j] = __floats2bfloat162_rn(f.x, f.y);
-    }
-    *reinterpret_cast<uint4*>(lp + i * 8) = u[k];
-  }
-}
-
 // dst = src * (*scale), rounded once to bf16; 8 elements per thread and iteration.
 template <typename ST>
 __global__ void __launch_bounds__(256) scale_kernel(const ST* __restrict__ src, bf16* __restrict__ dst, const float* __restrict__ scale, long n) {
@@ -563,13 +490,8 @@ extern "C" int nsa_cross_entropy(void* logits, const long* labels, float* loss_r
                                  int V, long ld, long ignore_index, int write_grad, cudaStream_t st) {
   if (rows <= 0) return 0;
   if (ld % 8) return nsa::fail(NSA_ERR_SHAPE, "cross_entropy: row pitch must be a multiple of 8");
-  // 8192 x 32000: 117 us a chunk of 4096 rows through the streaming kernel (two reads, the second from L2)
-  if (V % 8 == 0 && V <= CE_THREADS * CE_PIECES * 8)
-    cross_entropy_row_kernel<<<(unsigned)rows, CE_THREADS, 0, st>>>((bf16*)logits, labels, loss_rows, inv_count, V, ld, ignore_index,
-                                                                    write_grad, nsa::status_ptr());
-  else
-    cross_entropy_kernel<<<(unsigned)rows, 256, 0, st>>>((bf16*)logits, labels, loss_rows, inv_count, V, ld, ignore_index, write_grad,
-                                                         nsa::status_ptr());
+  cross_entropy_kernel<<<(unsigned)rows, 256, 0, st>>>((bf16*)logits, labels, loss_rows, inv_count, V, ld, ignore_index, write_grad,
+                                                       nsa::status_ptr());
   nsa::count_launch();
   return 0;
 }

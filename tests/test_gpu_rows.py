@@ -1,4 +1,4 @@
-"""Row kernels around the sizes their launches choose by: cross-entropy rows that fit in registers or stream, norm
+"""Row kernels around the sizes their launches choose by: cross-entropy rows of few and many vectors per thread, norm
 backward with fewer rows than CTAs, several rows per CTA and each register layout, against 64-bit results."""
 import pytest
 import torch
@@ -24,6 +24,29 @@ def test_linear_cross_entropy_rows(native, N, V):
     assert abs(float(loss) - float(ref)) <= 2e-3 * abs(float(ref)) + 2e-3          # logits are rounded to bf16
     for a, b in zip(got, want):
         assert a.dtype == torch.bfloat16 and (a.double() - b).norm() <= 1.5e-2 * b.norm()
+
+
+def test_cross_entropy_of_short_rows_costs_little(native):
+    # 16384 rows of 512 logits against as many of 32000: 0.09 of the time; 0.33 with CTAs sized for the long rows
+    from ctypes import c_int, c_long, c_void_p
+    p = lambda t: c_void_p(t.data_ptr())                                            # noqa: E731
+    rows = 16384
+    labels, losses, inv = torch.zeros(rows, device="cuda", dtype=torch.long), torch.empty(rows, device="cuda"), torch.ones(1, device="cuda")
+
+    def fastest(V):
+        logits = torch.randn(rows, V, device="cuda", dtype=torch.bfloat16)
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            native._check(native.load().nsa_cross_entropy(p(logits), p(labels), p(losses), p(inv), c_long(rows), c_int(V), c_long(V),
+                                                          c_long(-100), c_int(1), native._stream()))
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times[2:])
+
+    assert fastest(512) <= 0.2 * fastest(32000)
 
 
 def test_linear_cross_entropy_gradient_of_the_upstream_factor(native):
