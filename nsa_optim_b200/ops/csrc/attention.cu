@@ -62,6 +62,12 @@ struct AttnParams {
   KernelStatus* status;
 };
 
+// Query tile of a CTA.  Causal: the longest tiles first, so that the last CTAs to start are short (8192 tokens x 32 heads, forward:
+// 668 -> 640 us).  Tiles of one length (a window, no causality) go in the order of the keys they share (65536 tokens x 32 heads,
+// window 512: 1225 us, 1237 backwards).
+__host__ __device__ __forceinline__ bool longest_first(const AttnParams& p) { return p.causal && (p.window == 0 || p.window >= p.T); }
+__device__ __forceinline__ int query_tile(const AttnParams& p) { return longest_first(p) ? gridDim.x - 1 - blockIdx.x : blockIdx.x; }
+
 // Which key tiles a query tile visits, for contiguous-range modes.
 __device__ __forceinline__ void key_tile_range(const AttnParams& p, int t_lo, int t_hi, int& j0, int& j1) {
   // keys with pos <= t_hi (causal) and pos > t_lo - window (window)
@@ -206,7 +212,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int r = tid & 127, ch = tid >> 7;
-  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
+  const int qt = query_tile(p), h = blockIdx.y, b = blockIdx.z;
   const int q0 = qt * p.R;
   const int tok_local = r / p.G, g = r % p.G;
   const int t = q0 + tok_local;
@@ -469,6 +475,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // --------------------------------------------------------------------------------------
 constexpr int FWT_STAGES = 5;
 
+// The order of the tiles is a template argument here: chosen at run time it costs registers and 2 % without causality.
+template <bool LONGEST_FIRST>
 __global__ void __launch_bounds__(352, 1)
 attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
@@ -493,7 +501,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
+  const int qt = LONGEST_FIRST ? gridDim.x - 1 - blockIdx.x : blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -846,7 +854,7 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
+  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // always causal: longest tiles first
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -1073,7 +1081,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
+  const int qt = query_tile(p), h = blockIdx.y, b = blockIdx.z;
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -1383,7 +1391,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int r = tid & 127, ch = tid >> 7;
-  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
+  const int qt = query_tile(p), h = blockIdx.y, b = blockIdx.z;
   const int q0 = qt * p.R;
   const int tok_local = r / p.G, g = r % p.G;
   const int t = q0 + tok_local;
@@ -1630,7 +1638,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
+  const int qt = query_tile(p), h = blockIdx.y, b = blockIdx.z;
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -1929,7 +1937,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // causal: longest tiles first
+  const int qt = query_tile(p), h = blockIdx.y, b = blockIdx.z;
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
@@ -2849,9 +2857,11 @@ extern "C" int nsa_attn_fwd(const void* q, const void* k, const void* v, void* o
   static const bool smem_operands = [] { const char* e = getenv("NSA_B200_ATTN_FWD"); return e && !strcmp(e, "smem"); }();
   if (D == 128 && !legacy && !smem_operands) {
     const int smem_ts = (4 + 4 * FWT_STAGES) * HALF + 1024 + 1024 + 256;
-    static bool cfg = false;
-    if (!cfg) { if ((rc = set_smem(attn_fwd_ts_kernel, smem_ts))) return rc; cfg = true; }
-    attn_fwd_ts_kernel<<<grid, 352, smem_ts, st>>>(tq, tk, tv, p);
+    auto* kernel = longest_first(p) ? attn_fwd_ts_kernel<true> : attn_fwd_ts_kernel<false>;
+    static bool cfg[2] = {};
+    bool& ready = cfg[longest_first(p)];
+    if (!ready) { if ((rc = set_smem(kernel, smem_ts))) return rc; ready = true; }
+    kernel<<<grid, 352, smem_ts, st>>>(tq, tk, tv, p);
   } else if (D == 128 && !legacy) {
     const int smem_ws = (4 + 4 * FW_STAGES + 4) * HALF + 1024 + 1024 + 256;
     static bool cfg = false;
