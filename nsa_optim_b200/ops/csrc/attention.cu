@@ -444,13 +444,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
   }
   if (!ok && tid == 0) {
-    const long long t0 = clock64();
     uint64_t* pend[5] = {qbar, &kfull[0], &kfull[1], &vfull[0], &vfull[1]};
-    for (int i = 0; i < 5; ++i)
-      for (uint32_t n = 0; n < (1u << 16); ++n) {
-        if (tc5::mbar_try_wait(pend[i], 0) || tc5::mbar_try_wait(pend[i], 1)) break;
-        if (clock64() - t0 > tc5::kMaxWaitCycles) break;
-      }
+    for (int i = 0; i < 5; ++i) tc5::mbar_drain(pend[i]);
   }
   tc5::fence_before_sync();
   __syncthreads();
@@ -1581,13 +1576,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
   }
   if (!ok && tid == 0) {
-    const long long t0 = clock64();
     uint64_t* pend[2] = {qbar, kvbar};
-    for (int i = 0; i < 2; ++i)
-      for (uint32_t n = 0; n < (1u << 16); ++n) {
-        if (tc5::mbar_try_wait(pend[i], 0) || tc5::mbar_try_wait(pend[i], 1)) break;
-        if (clock64() - t0 > tc5::kMaxWaitCycles) break;
-      }
+    for (int i = 0; i < 2; ++i) tc5::mbar_drain(pend[i]);
   }
   tc5::fence_before_sync();
   __syncthreads();

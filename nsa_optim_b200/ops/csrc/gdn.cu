@@ -323,14 +323,9 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
   if (ok) finish_output(NC - 1);
   if (boss || threadIdx.x == CH) tc5::tma_store_wait_read<0>();
-  if (!ok && boss) {
-    // a load for the next chunk may still be in flight: give it a bounded chance to land
-    const long long t0 = clock64();
-    for (int s = 0; s < 2; ++s)
-      for (uint32_t i = 0; i < (1u << 16); ++i) {
-        if (tc5::mbar_try_wait(&full[s], 0) || tc5::mbar_try_wait(&full[s], 1)) break;
-        if (clock64() - t0 > tc5::kMaxWaitCycles) break;
-      }
+  if (!ok && boss) {                               // a load for the next chunk may still be in flight
+    tc5::mbar_drain(&full[0]);
+    tc5::mbar_drain(&full[1]);
   }
   tc5::fence_before_sync();
   __syncthreads();
@@ -571,13 +566,9 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     }
   }
   if (boss) tc5::tma_store_wait_read<0>();
-  if (!ok && boss) {
-    const long long t0 = clock64();
-    for (int s = 0; s < 2; ++s)
-      for (uint32_t i = 0; i < (1u << 16); ++i) {
-        if (tc5::mbar_try_wait(&full[s], 0) || tc5::mbar_try_wait(&full[s], 1)) break;
-        if (clock64() - t0 > tc5::kMaxWaitCycles) break;
-      }
+  if (!ok && boss) {                               // a load for the next chunk may still be in flight
+    tc5::mbar_drain(&full[0]);
+    tc5::mbar_drain(&full[1]);
   }
   tc5::fence_before_sync();
   __syncthreads();

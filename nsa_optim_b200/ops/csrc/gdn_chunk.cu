@@ -416,10 +416,9 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
     if (!tc5::mbar_wait(done + (s & 1), (s >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
   }
   if (__syncthreads_or(!ok)) {
-    if (tid == 0) {                                        // copies in flight get a bounded chance to land
-      const long long start = clock64();
-      for (int s = 0; s < 2; ++s)
-        while (!tc5::mbar_try_wait(full + s, 0) && !tc5::mbar_try_wait(full + s, 1) && clock64() - start < tc5::kMaxWaitCycles) {}
+    if (tid == 0) {                                        // slices may still be in flight
+      tc5::mbar_drain(full);
+      tc5::mbar_drain(full + 1);
     }
     __syncthreads();
     if (warp == 0) tc5::tmem_dealloc(tmem, 512);

@@ -87,6 +87,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// After a wait that gave up: gives a copy that may still be in flight towards `bar` a bounded chance (10 ms) to land before the
+// CTA's shared memory goes to another CTA.  The open phase is read from the barrier (waiting for either parity would not
+// wait at all: one of the two is always complete); where no copy is on its way, the limit passes.
+constexpr long long kDrainCycles = 20000000ll;
+__device__ __forceinline__ void mbar_drain(uint64_t* bar) {
+  const uint32_t open = mbar_try_wait(bar, 0) ? 1u : 0u;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, open) && clock64() - t0 < kDrainCycles) {}
+}
+
 // The same wait with a caller-chosen cycle budget (no poll-count limit): for consumers whose
 // producer may itself legitimately wait on another GPU for up to `max_cycles`.
 __device__ __forceinline__ bool mbar_wait_cycles(uint64_t* bar, uint32_t parity, volatile int* abort_flag,

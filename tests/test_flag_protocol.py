@@ -115,3 +115,14 @@ def test_checker_catches_a_missing_wait(mutation):
     gather reads a shard of the previous step."""
     caught = sum(1 for seed in range(300) if run(seed, **{mutation: False}))
     assert caught > 0
+
+
+def test_no_wait_accepts_either_parity_of_a_barrier():
+    """One of the two parities of an mbarrier is always complete, so polling for either of them returns at once: a kernel that
+    gives up would leave its shared memory to the next CTA with copies still on their way."""
+    import pathlib
+    import re
+    csrc = pathlib.Path(__file__).parent.parent / "nsa_optim_b200" / "ops" / "csrc"
+    both = re.compile(r"mbar_try_wait\((.+?), 0\)\s*(?:\|\||&&)\s*!?\s*(?:tc5::)?mbar_try_wait\(\1, 1\)")
+    found = [f"{f.name}: {m.group(0)}" for f in sorted(csrc.glob("*.cu*")) for m in both.finditer(f.read_text())]
+    assert not found, found
