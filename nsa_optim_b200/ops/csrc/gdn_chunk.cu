@@ -16,7 +16,7 @@ constexpr int CH = 64, KD = 128;
 constexpr int PK = KD + 8, PC = CH + 8;          // tile pitches (elements)
 constexpr int PX = 68;                           // pitch of the fp32 64 x 64 tiles: rows 16-byte aligned, spread over the banks
 
-// Per-chunk gate quantities; 64 threads (two warps) call it, t = token of the row, the caller synchronises.
+// Per-chunk gate quantities: the CTA's first warp does the work, two tokens a lane; the caller synchronises.
 // gs: cumulative log-decay, bs: beta.
 __device__ __forceinline__ void load_gates(const float* g, const float* beta, long tok0, int T, int t0, int H, float* gs, float* bs) {
   const int lane = threadIdx.x & 31;
@@ -45,9 +45,10 @@ struct PrepParams {
   float scale;
 };
 
-// One CTA of eight warps per (chunk, head).  Bound by the memory traffic of q, k, v, u, w (2 KB per token and head)
-// once two CTAs share an SM; the triangular inverse is the longest dependent phase and runs as two
-// 32-column substitutions side by side, joined by two 32 x 32 products over all threads.
+// One CTA of eight warps per (chunk, head).  Two CTAs share an SM for values up to 192 wide; at 256 one needs 122 KB and runs alone,
+// and what bounds the kernel there is its chain of phases, not the memory traffic of q, k, v, u, w (2 KB per token and
+// head: 282 us at 16384 tokens x 16 heads, 87 us of it at the copy rate).  The triangular inverse is the longest
+// dependent phase and runs as two 32-column substitutions side by side, joined by two 32 x 32 products over all threads.
 __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const int V = p.V, PV = V + 8;

@@ -1,8 +1,8 @@
 // Warp-level bf16 matrix products (mma.sync m16n8k16, fp32 accumulation) on padded shared-memory tiles.
 //
-// For per-chunk products of 64-row tiles.  A tcgen05 tile of 128 rows would be half empty, its accumulators
-// cap a CTA's neighbours through tensor memory, and these kernels are bound by memory traffic and by
-// dependent phases: several small CTAs per SM with accumulators in registers hide those.
+// For per-chunk products of 64-row tiles, of which a tcgen05 tile of 128 rows would be half empty.  The kernels that use
+// them are chains of dependent phases with products of a few thousand cycles at most between them; accumulators in
+// registers go straight into the next phase's arithmetic, without a trip through tensor memory.
 // Tiles are row-major with a pitch that is an odd multiple of 16 bytes, so ldmatrix is free of bank conflicts.
 #pragma once
 #include <cuda_bf16.h>

@@ -124,14 +124,7 @@ struct SsdParams {
   // chunk_state
   float* S_out;        // [B, nc, H, NS, PD] fp32
   float* gamma_out;    // [B, nc, H] or null
-  // chunk_out
-  bf16* y;             // [B, T, H, PD]
-  const bf16* x_raw;   // x for the D skip and row scalars (token stride ldx elements, head offset h*PD)
-  long ldx;
-  // chunk_grad
-  const bf16* y_in;    // [B, T, H, PD]
-  const bf16* dy_raw;  // [B, T, H, PD]
-  bf16* dx;            // [B, T, H, PD]
+  // chunk_grad (y and dx leave through their tensor maps)
   float* dB_acc;       // [B, T, NS] fp32 (pre-zeroed, summed over heads)
   float* dC_acc;       // [B, T, NS]
   bf16* dB_heads;      // [B, T, H, NS] per-head results written with plain stores (null: use the fp32 reductions above);
@@ -397,7 +390,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
 //   dx_j  = sum_i P_ij dy_i + s_j B_j dHn + D dy_j          (s_j = exp(tot - cum_j) dt_j)
 //   dC_i  = sum_j dS_ij B_j + exp(cum_i) dy_i H^T
 //   dB_j  = sum_i dS_ij C_i + s_j x_j dHn^T
-// dB / dC are summed over heads with fp32 vector reductions.
+// dB / dC leave per head as bf16 tiles that nsa_ssd_finish sums, or (nsa_ssd_chunk_grad) by fp32 vector reductions over heads.
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(512, 1)
 ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_b,
@@ -962,7 +955,7 @@ extern "C" int nsa_ssd_chunk_out(const void* Cm, long ld_c, const void* Bm, long
   if ((rc = map_state(&th, Hprev_bf16, static_cast<long>(B) * nc * H * NS))) return rc;
   SsdParams p{};
   p.dt = dt; p.A = A; p.Dskip = Dskip; p.B = B; p.T = T; p.H = H; p.nc = nc;
-  p.y = (bf16*)y; p.x_raw = (const bf16*)x; p.ldx = ld_x; p.status = nsa::status_ptr();
+  p.status = nsa::status_ptr();
   const int smem = 6 * BOXB + 1024 + 2048;
   static bool cfg = false;
   if (!cfg) { if ((rc = smem_attr(ssd_chunk_out_kernel, smem))) return rc; cfg = true; }
@@ -974,10 +967,9 @@ extern "C" int nsa_ssd_chunk_out(const void* Cm, long ld_c, const void* Bm, long
 
 // dB_acc / dC_acc: fp32 [B, T, N], zeroed by the caller.  q_out / k_out: fp32 [B, T, H].
 static int ssd_chunk_grad_impl(const void* Cm, long ld_c, const void* Bm, long ld_b, const void* x, long ld_x,
-                               const void* dy, const void* y, const void* Hprev_bf16, const void* dHn_bf16,
-                               const float* dt, const float* A, const float* Dskip, void* dx, float* dB_acc,
-                               float* dC_acc, void* dB_heads, void* dC_heads, float* q_out, float* k_out, float* r_out,
-                               int B, int T, int H, int N, int P, cudaStream_t st) {
+                               const void* dy, const void* Hprev_bf16, const void* dHn_bf16, const float* dt, const float* A,
+                               const float* Dskip, void* dx, float* dB_acc, float* dC_acc, void* dB_heads, void* dC_heads,
+                               float* q_out, float* k_out, float* r_out, int B, int T, int H, int N, int P, cudaStream_t st) {
   int rc = check_dims(N, P, ld_c | ld_b, ld_x);
   if (rc) return rc;
   const int nc = (T + L - 1) / L;
@@ -995,7 +987,6 @@ static int ssd_chunk_grad_impl(const void* Cm, long ld_c, const void* Bm, long l
   if ((rc = map_heads(&tdch, dC_heads ? dC_heads : dx, B, T, H, dC_heads != nullptr))) return rc;
   SsdParams p{};
   p.dt = dt; p.A = A; p.Dskip = Dskip; p.B = B; p.T = T; p.H = H; p.nc = nc;
-  p.x_raw = (const bf16*)x; p.ldx = ld_x; p.y_in = (const bf16*)y; p.dy_raw = (const bf16*)dy; p.dx = (bf16*)dx;
   p.dB_acc = dB_acc; p.dC_acc = dC_acc; p.q_out = q_out; p.k_out = k_out; p.status = nsa::status_ptr();
   p.dB_heads = (bf16*)dB_heads; p.dC_heads = (bf16*)dC_heads; p.r_out = r_out;
   const int smem = 13 * BOXB + 1024 + 2048 + 16 * L * 4;
@@ -1006,12 +997,13 @@ static int ssd_chunk_grad_impl(const void* Cm, long ld_c, const void* Bm, long l
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_chunk_grad launch");
 }
 
+// y is not read (the sums that used it come from the products themselves); callers may pass null.
 extern "C" int nsa_ssd_chunk_grad(const void* Cm, long ld_c, const void* Bm, long ld_b, const void* x, long ld_x,
                                   const void* dy, const void* y, const void* Hprev_bf16, const void* dHn_bf16,
                                   const float* dt, const float* A, const float* Dskip, void* dx, float* dB_acc,
                                   float* dC_acc, float* q_out, float* k_out, int B, int T, int H, int N, int P,
                                   cudaStream_t st) {
-  return ssd_chunk_grad_impl(Cm, ld_c, Bm, ld_b, x, ld_x, dy, y, Hprev_bf16, dHn_bf16, dt, A, Dskip, dx, dB_acc, dC_acc,
+  return ssd_chunk_grad_impl(Cm, ld_c, Bm, ld_b, x, ld_x, dy, Hprev_bf16, dHn_bf16, dt, A, Dskip, dx, dB_acc, dC_acc,
                              nullptr, nullptr, q_out, k_out, nullptr, B, T, H, N, P, st);
 }
 // Same, with dB / dC written per head as bf16 [B, T, H, N] (plain stores); the caller sums over heads.
@@ -1022,6 +1014,6 @@ extern "C" int nsa_ssd_chunk_grad_heads(const void* Cm, long ld_c, const void* B
                                         void* dC_heads, float* q_out, float* k_out, float* r_out, int B, int T, int H,
                                         int N, int P, cudaStream_t st) {
   if (dB_heads == nullptr || dC_heads == nullptr) return nsa::fail(NSA_ERR_SHAPE, "ssd_chunk_grad_heads: null output");
-  return ssd_chunk_grad_impl(Cm, ld_c, Bm, ld_b, x, ld_x, dy, y, Hprev_bf16, dHn_bf16, dt, A, Dskip, dx, nullptr, nullptr,
+  return ssd_chunk_grad_impl(Cm, ld_c, Bm, ld_b, x, ld_x, dy, Hprev_bf16, dHn_bf16, dt, A, Dskip, dx, nullptr, nullptr,
                              dB_heads, dC_heads, q_out, k_out, r_out, B, T, H, N, P, st);
 }
