@@ -251,3 +251,9 @@ def test_inverse_selection_map_kernels_match_the_sort_based_form(native, T, nS, 
 def test_both_orders_of_the_query_tiles(native, D, T, W, causal):
     run_pair(lambda q, k, v: native.attention(q, k, v, causal, W),
              lambda q, k, v: oracle.attention(q, k, v, causal, W), mk(1, T, 8, 2, D))
+
+
+@pytest.mark.parametrize("T", [131072, 131073])
+def test_inverse_selection_map_on_both_sides_of_the_chunk_length_rule(native, T):
+    # chunks of 64 tokens up to 131072, of 256 above
+    test_inverse_selection_map_kernels_match_the_sort_based_form(native, T, 300, 4)
