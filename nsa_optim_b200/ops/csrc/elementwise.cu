@@ -2,8 +2,8 @@
 // SwiGLU, rotary embedding, causal depthwise conv1d (+SiLU), embedding gather and its
 // deterministic scatter-add backward.  bf16 storage, fp32 arithmetic, 16-byte accesses.
 //
-// Row kernels keep a whole row in registers (one global read per element).  Rows up to 512
-// elements use one warp per row, longer rows (up to 8192) use one 256-thread CTA per row.
+// Row kernels keep a whole row in registers.  Rows up to 512 elements use one warp per row, longer
+// rows (up to 8192) one CTA of 256 threads per row, or of 512 in the norm backward's wider forms.
 // Weight gradients of the norms and the convolution are reduced deterministically:
 // a persistent grid accumulates per-CTA partial sums into a scratch buffer
 // [grid, width] (fp32) that a second kernel adds up in a fixed order.
@@ -171,25 +171,31 @@ __global__ void __launch_bounds__(256) rmsnorm_add_fwd_kernel(const bf16* __rest
 // input by another route (the residual stream); it is added into dx here instead of by a
 // separate pass over both tensors.
 //
-// Bound by memory traffic, so by the bytes in flight per SM.  A row that a CTA shares (TPR 256) ends in two barriers: what
-// helps is the next row's operands in flight behind them, though that costs resident CTAs (gate first, 8192 x 4096: 136 -> 107 us
-// with one CTA per SM instead of two), and above 4096 columns all loads of the row issued together, though that spills (gate first,
-// 4096 x 8192: 195 -> 139 us with 328 bytes spilled).  A row of one warp (TPR 32, up to 512 columns) meets no barrier: its
-// warps run apart and hide each other's loads, so the registers go to more warps, and x and dres are read again where
-// they are used.  1048576 x 128: 260 us plain and 407 norm first (516 and 604 with the next row in registers: two CTAs
-// instead of four and three); 262144 x 512: 169 plain, 320 gate first (311 and 415).
+// Bound by memory traffic, so by the bytes in flight per SM.  A row that a CTA shares ends in two barriers: what helps is the
+// next row's operands in flight behind them, as long as a thread's part of a row is one 16-byte piece: TPR 256 up to 2048
+// columns, 512 up to 4096 (two pieces a thread ahead leave one CTA of 256 threads per SM: 65536 x 4096, gate first, 757 us,
+// 732 without looking ahead, 603 with 512 threads; plain 545, 502, 300).  Above 4096 columns all loads of a row are issued
+// together and held (32768 x 8192, plain: 408 us, 752 read where they are used), but with the gate first that
+// spills, and 512 threads that read x again take 765 us instead of 1045.  A row of one warp (TPR 32, up to 512 columns) meets
+// no barrier: its warps run apart and hide each other's loads, so the registers go to more warps, and x and dres are read
+// again where they are used.  1048576 x 128: 260 us plain and 407 norm first (516 and 604 with the next row in registers:
+// two CTAs instead of four and three); 262144 x 512: 169 plain, 320 gate first (311 and 415).
 // CTAs per SM that the registers leave room for:
 template <int TPR, int NV, int MODE>
-constexpr int rms_bwd_ctas = TPR == 32 ? (NV == 1 ? (MODE == 0 ? 4 : 3) : (MODE == 0 ? 3 : 2))
-                                       : (NV == 1 ? (MODE == 0 ? 4 : 2) : 1);
+constexpr int rms_bwd_ctas = TPR == 32    ? (NV == 1 ? (MODE == 0 ? 4 : 3) : (MODE == 0 ? 3 : 2))
+                             : NV > 1     ? 1
+                             : TPR == 256 ? (MODE == 0 ? 4 : 2)
+                                          : (MODE == 0 ? 2 : 1);
+template <int TPR>
+constexpr int rms_bwd_threads = TPR > 256 ? TPR : 256;
 template <int TPR, int NV, int MODE>
-__global__ void __launch_bounds__(256, rms_bwd_ctas<TPR, NV, MODE>)
+__global__ void __launch_bounds__(rms_bwd_threads<TPR>, rms_bwd_ctas<TPR, NV, MODE>)
 rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, const bf16* __restrict__ w, const bf16* __restrict__ dy,
                    const float* __restrict__ rstd_in, bf16* __restrict__ dx, bf16* __restrict__ dg, float* __restrict__ partial,
                    long rows, int d, const bf16* __restrict__ dres = nullptr, long ldg = 0) {
-  __shared__ float red[8];
+  __shared__ float red[rms_bwd_threads<TPR> / 32];
   __shared__ float dw_sh[(TPR == 32) ? 512 : 1];
-  const int rows_per_cta = 256 / TPR;
+  const int rows_per_cta = rms_bwd_threads<TPR> / TPR;
   const int sub = threadIdx.x / TPR;
   const int t = threadIdx.x % TPR;
   float dwacc[NV][8];
@@ -201,9 +207,8 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, const
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
     if (c < d) load8(w + c, wv[i]);
   }
-  // HELD: a row's operands are loaded together and kept as they came; AHEAD: one row early (rows of 8192 would need too
-  // many registers for that).
-  constexpr bool HELD = TPR == 256, AHEAD = HELD && NV <= 2;
+  // HELD: a row's operands are loaded together and kept as they came; AHEAD: one row early.
+  constexpr bool AHEAD = TPR > 32 && NV == 1, HELD = AHEAD || NV == 4;
   uint4 nx[NV], ndy[NV], ng[NV], nr[NV];
   auto fetch = [&](long row) {
     if (row >= rows) return;
@@ -917,7 +922,7 @@ int bwd_grid(int parts) {
   static int per_sm = 0;
   if (per_sm == 0) {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rmsnorm_bwd_kernel<TPR, NV, MODE>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rmsnorm_bwd_kernel<TPR, NV, MODE>, rms_bwd_threads<TPR>, 0);
     per_sm = n > 0 ? n : 1;
   }
   const int all = per_sm * nsa::sm_count();
@@ -927,7 +932,7 @@ template <int TPR, int NV, int MODE>
 void run_rms_bwd(const bf16* X, const bf16* G, const bf16* Wt, const bf16* DY, const float* rstd, bf16* DX, bf16* DG, float* partial,
                  int& grid, long rows, int d, const bf16* DR, long ldg, cudaStream_t st) {
   grid = bwd_grid<TPR, NV, MODE>(grid);
-  rmsnorm_bwd_kernel<TPR, NV, MODE><<<grid, 256, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
+  rmsnorm_bwd_kernel<TPR, NV, MODE><<<grid, rms_bwd_threads<TPR>, 0, st>>>(X, G, Wt, DY, rstd, DX, DG, partial, rows, d, DR, ldg);
 }
 // `grid` holds the number of partial rows the caller has room for and receives the number written.
 template <int MODE>
@@ -938,8 +943,11 @@ int launch_rms_bwd(const void* x, const void* g, const void* w, const void* dy, 
   if (d <= 256) run_rms_bwd<32, 1, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
   else if (d <= 512) run_rms_bwd<32, 2, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
   else if (d <= 2048) run_rms_bwd<256, 1, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
-  else if (d <= 4096) run_rms_bwd<256, 2, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
-  else if (d <= 8192) run_rms_bwd<256, 4, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
+  else if (d <= 4096) run_rms_bwd<512, 1, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
+  else if (d <= 8192) {
+    if constexpr (MODE == 2) run_rms_bwd<512, 2, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
+    else run_rms_bwd<256, 4, MODE>(X, G, Wt, DY, rstd, DX, DG, partial, grid, rows, d, DR, ldg, st);
+  }
   else return nsa::fail(NSA_ERR_SHAPE, "rmsnorm: width above 8192 is not supported");
   nsa::count_launch();
   return 0;

@@ -116,10 +116,10 @@ def test_gated_norm_backward_pitched_gate(native, mode, rows, d, pitch):
         assert (a.double() - b).norm() <= 5e-3 * b.norm() + 1e-6                      # one rounding to bf16, fp32 inside
 
 
-def test_norm_backward_of_many_narrow_rows_is_memory_bound(native):
-    # Rows of one warp live on resident warps.  Three tensors pass through memory; a copy kernel of as many bytes is the
-    # yardstick: 2.1 times its time with four CTAs per SM, 4.1 times with two.
-    rows, d = 1 << 20, 128
+# 2.1 times the copy at 128 columns with four CTAs per SM, 4.1 with two; 1.2 at 4096 columns with 512 threads a row, 2.2 with 256
+@pytest.mark.parametrize("rows,d,limit", [(1 << 20, 128, 3.1), (1 << 16, 4096, 1.7)])
+def test_norm_backward_of_many_rows_is_memory_bound(native, rows, d, limit):
+    # Three tensors pass through memory; a copy of as many bytes is the yardstick
     x, dy = (torch.randn(rows, d, device="cuda").bfloat16().requires_grad_(i == 0) for i in range(2))
     w = torch.ones(d, device="cuda", dtype=torch.bfloat16, requires_grad=True)
     y = native.rms_norm(x, w)
@@ -137,4 +137,4 @@ def test_norm_backward_of_many_narrow_rows_is_memory_bound(native):
         return min(times[2:])
 
     copy = fastest(lambda: dst.copy_(src))
-    assert fastest(lambda: torch.autograd.grad(y, [x, w], dy, retain_graph=True)) <= 3.1 * copy
+    assert fastest(lambda: torch.autograd.grad(y, [x, w], dy, retain_graph=True)) <= limit * copy
