@@ -652,7 +652,10 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
 // State passing over chunks (elementwise).  Layout [B, nc, H, E], E = NS * PD.
 // ---------------------------------------------------------------------------------------
 // A thread walks the chunks of VEC neighbouring elements.  The recurrence itself is one FMA per chunk; what takes time is
-// memory, so the terms of the next eight chunks are always in flight.
+// memory, so the terms of the next eight chunks are always in flight (512 chunks x 64 heads x 8192, bf16 out: 348 us without,
+// 268 now).  Few elements leave one warp per scheduler, and then a step is as long as its instructions: pointers move by a
+// step, and the bounds are tested outside the unrolled walk (1000 chunks x 3 heads x 63: 87 us with an address computed per
+// access, 53 without chunks in flight, 32 now).
 template <int VEC>
 struct Elems { float v[VEC]; };
 template <int VEC>
@@ -674,32 +677,41 @@ __device__ __forceinline__ void st_f32(float* p, const Elems<VEC>& x) {
 }
 // out[c] = state entering chunk c; step: state <- gamma[c] state + in[c].  BACK walks the chunks in reverse.
 template <int VEC, bool BACK>
-__global__ void __launch_bounds__(256) ssd_state_kernel(const float* __restrict__ in, const float* __restrict__ gamma,
+__global__ void __launch_bounds__(256, 3) ssd_state_kernel(const float* __restrict__ in, const float* __restrict__ gamma,
                                                         float* __restrict__ out, bf16* __restrict__ out_bf,
                                                         float* __restrict__ last, int nc, int H, long E) {
   constexpr int U = 8;
   const long e = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * VEC;
   if (e >= E) return;
   const int h = blockIdx.y, b = blockIdx.z;
-  auto at = [&](int i) { return (static_cast<long>(b) * nc + (BACK ? nc - 1 - i : i)) * H + h; };
+  const long first = (static_cast<long>(b) * nc + (BACK ? nc - 1 : 0)) * H + h;
+  const long gstep = BACK ? -H : H, step = gstep * E;              // from one chunk to the next
+  in += first * E + e;
+  gamma += first;
+  if (out) out += first * E + e;
+  if (out_bf) out_bf += first * E + e;
   Elems<VEC> st{}, next[U];
   float g_next[U];
 #pragma unroll
   for (int u = 0; u < U; ++u)
-    if (u < nc) { next[u] = ld_f32<VEC>(in + at(u) * E + e); g_next[u] = gamma[at(u)]; }
-  for (int i0 = 0; i0 < nc; i0 += U) {
+    if (u < nc) { next[u] = ld_f32<VEC>(in + u * step); g_next[u] = gamma[u * gstep]; }
+  in += U * step;
+  gamma += U * gstep;
+  auto advance = [&](int u, bool more) {
+    if (out) { st_f32<VEC>(out, st); out += step; }
+    if (out_bf) { st_bf16<VEC>(out_bf, st); out_bf += step; }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = i0 + u;
-      if (i >= nc) break;
-      const long o = at(i) * E + e;
-      if (out) st_f32<VEC>(out + o, st);
-      if (out_bf) st_bf16<VEC>(out_bf + o, st);
+    for (int k = 0; k < VEC; ++k) st.v[k] = g_next[u] * st.v[k] + next[u].v[k];
+    if (more) { next[u] = ld_f32<VEC>(in); g_next[u] = *gamma; in += step; gamma += gstep; }
+  };
+  int i = 0;
+  for (; i + 2 * U <= nc; i += U)
 #pragma unroll
-      for (int k = 0; k < VEC; ++k) st.v[k] = g_next[u] * st.v[k] + next[u].v[k];
-      if (i + U < nc) { next[u] = ld_f32<VEC>(in + at(i + U) * E + e); g_next[u] = gamma[at(i + U)]; }
-    }
-  }
+    for (int u = 0; u < U; ++u) advance(u, true);
+  for (; i < nc; i += U)
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u < nc) advance(u, i + u + U < nc);
   if (last) st_f32<VEC>(last + (static_cast<long>(b) * H + h) * E + e, st);
 }
 template <bool BACK>

@@ -85,3 +85,23 @@ def test_ssd_more_chunks_than_a_second_grid_dimension_holds(native):
         for a, b in list(zip(whole, run(part)[0]))[:outputs]:
             a, b = a[:, part][:, kept].double(), b[:, kept].double()
             assert b.shape[1] >= 1 and b.norm() > 0 and (a - b).norm() <= 2 ** -8 * b.norm()
+
+
+def test_state_pass_of_few_elements_is_a_short_chain(native):
+    # 1000 chunks of 3 x 63 elements: what one step takes. 32 us; 87 with addresses computed per access
+    from ctypes import c_int, c_long, c_void_p
+    p = lambda t: c_void_p(t.data_ptr())                                            # noqa: E731
+    B, nc, H, E = 1, 1000, 3, 63
+    S, gamma = torch.randn(B, nc, H, E, device="cuda"), torch.rand(B, nc, H, device="cuda")
+    out = torch.empty(S.shape, device="cuda", dtype=torch.bfloat16)
+    times = []
+    for _ in range(8):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(20):
+            native._check(native.load().nsa_ssd_state_fwd(p(S), p(gamma), c_void_p(0), p(out), c_void_p(0), c_int(B), c_int(nc), c_int(H),
+                                                          c_long(E), native._stream()))
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b) / 20 * 1e3)
+    assert min(times[2:]) <= 60, times
