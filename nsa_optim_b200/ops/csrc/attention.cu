@@ -2623,9 +2623,10 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const bf16* __restrict_
 // An entry is dropped if it is negative, out of range or repeats an earlier entry of the same token.
 // --------------------------------------------------------------------------------------
 // A walk is one warp stepping through its tokens, so short chunks are what spreads it over the GPU (chunks of 256 left 128 warps
-// for 16384 tokens x 2 heads and took 106 us per walk).  Above 131072 tokens there are warps enough, and the
-// histograms (one row of counts per chunk) stay as small as they were.
-inline int inverse_chunk(int T) { return T <= 131072 ? 64 : 256; }
+// for 16384 tokens x 2 heads and took 106 us per walk).  The histograms, one row of counts per chunk, pass through memory four
+// times; beyond 25 MB long chunks are the faster ones (100000 tokens, 1563 blocks: x 2 heads, 20 MB with chunks of 64, 235 us and
+// 265 with 256; x 4 heads 404 and 312; 131072 tokens x 8 heads 2045 and 886).
+inline int inverse_chunk(int BH, int T, int nS) { return static_cast<long>(BH) * ((T + 63) / 64) * nS <= 6l << 20 ? 64 : 256; }
 
 // mode 0: hist[(bh * chunks + chunk) * nS + blk] = entries of the chunk; mode 1: fill tok_list.
 // The warp takes the chunk's tokens one after the other, lane j looking at entry j of the token's
@@ -3050,15 +3051,18 @@ extern "C" int nsa_union_blocks(const int* idx, int* tile_blocks, unsigned long 
 
 // Inverse selection map (see nsa_inverse_walk_kernel).  idx: [B*Hkv, T, n] int32.  Outputs: tok_list
 // (capacity B*Hkv*T*n), list_start and item_start (lists + 1 entries, lists = B*Hkv*nS).  Scratch:
-// hist with B*Hkv*nsa_inverse_chunks(T)*nS ints and count with `lists` ints.
+// hist with B*Hkv*nsa_inverse_chunks(B*Hkv, T, nS)*nS ints and count with `lists` ints.
 // Rows of counts per (batch, KV head) in `hist` of nsa_inverse_blocks.
-extern "C" int nsa_inverse_chunks(int T) { return (T + inverse_chunk(T) - 1) / inverse_chunk(T); }
+extern "C" int nsa_inverse_chunks(int BH, int T, int nS) {
+  const int len = inverse_chunk(BH, T, nS);
+  return (T + len - 1) / len;
+}
 extern "C" int nsa_inverse_blocks(const int* idx, int* tok_list, int* list_start, int* item_start, int* hist, int* count,
                                   int BH, int T, int n, int nS, int R, int visits_per_cta, cudaStream_t st) {
   if (BH <= 0 || T <= 0 || n <= 0 || nS <= 0 || R <= 0 || visits_per_cta <= 0)
     return nsa::fail(NSA_ERR_SHAPE, "nsa_inverse_blocks: empty problem");
   if (nS * 4 > 48 * 1024 || n > 32) return nsa::fail(NSA_ERR_SHAPE, "nsa_inverse_blocks: at most 12288 selection blocks and 32 entries per token");
-  const int len = inverse_chunk(T), chunks = nsa_inverse_chunks(T);
+  const int len = inverse_chunk(BH, T, nS), chunks = nsa_inverse_chunks(BH, T, nS);
   const long lists = static_cast<long>(BH) * nS;
   const dim3 grid(chunks, BH);
   nsa_inverse_walk_kernel<<<grid, 32, nS * 4, st>>>(idx, hist, nullptr, nullptr, nullptr, T, n, nS, chunks, len, 0);

@@ -1112,7 +1112,7 @@ def inverse_blocks(idx: Tensor, nS: int, R: int, visits_per_cta: int):
     dev = idx.device
     idx = idx.to(torch.int32).contiguous()
     lists = B * Hkv * nS
-    chunks = int(load().nsa_inverse_chunks(c_int(T)))
+    chunks = int(load().nsa_inverse_chunks(c_int(B * Hkv), c_int(T), c_int(nS)))
     tok = _empty(B * Hkv * T * n, dtype=torch.int32, device=dev)
     list_start = _empty(lists + 1, dtype=torch.int32, device=dev)
     item_start = _empty(lists + 1, dtype=torch.int32, device=dev)

@@ -253,7 +253,27 @@ def test_both_orders_of_the_query_tiles(native, D, T, W, causal):
              lambda q, k, v: oracle.attention(q, k, v, causal, W), mk(1, T, 8, 2, D))
 
 
-@pytest.mark.parametrize("T", [131072, 131073])
+@pytest.mark.parametrize("T", [335488, 335489])
 def test_inverse_selection_map_on_both_sides_of_the_chunk_length_rule(native, T):
-    # chunks of 64 tokens up to 131072, of 256 above
+    # 4 heads x 300 blocks: chunks of 64 tokens while the counts fit in 25 MB, of 256 above
     test_inverse_selection_map_kernels_match_the_sort_based_form(native, T, 300, 4)
+
+
+def test_inverse_selection_map_of_more_heads_costs_in_proportion(native):
+    # 131072 tokens: 8 lists of heads against 2 take 3.6 times as long; 8 with counts that leave L2
+    T, nS = 131072, 2048
+
+    def fastest(heads):
+        own = (torch.arange(T, device="cuda") // 64).view(1, 1, T, 1)
+        idx = (torch.rand(1, heads, T, 16, device="cuda") * (own + 1)).int()
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            native.inverse_blocks(idx, nS, 8, 64)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times[2:])
+
+    assert fastest(8) <= 5.5 * fastest(2)
