@@ -565,6 +565,12 @@ def _gate_rows(gate: Tensor):
     return g2, d
 
 
+def _row_pitch(t: Tensor) -> int:
+    """Elements from one row (last dimension) to the next.  Read from a saved tensor as it comes back: saved-tensor
+    hooks (activations kept on the host) return a pitched view as a dense tensor."""
+    return t.shape[-1] if t.is_contiguous() else t.stride(-2)
+
+
 class _GatedRMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gate, w, eps, norm_before_gate):
@@ -578,7 +584,7 @@ class _GatedRMSNorm(torch.autograd.Function):
         _check(load().nsa_rmsnorm_fwd_ldg(_p(x2), _p(g2), c_long(ldg), _p(wb), _p(y), _p(rstd), c_long(rows), c_int(d),
                                           c_float(eps), c_int(mode), _stream()))
         ctx.save_for_backward(x2, g2, wb, rstd)
-        ctx.mode, ctx.wdtype, ctx.gshape, ctx.ldg = mode, w.dtype, gate.shape, ldg
+        ctx.mode, ctx.wdtype, ctx.gshape = mode, w.dtype, gate.shape
         return y.view(x.shape)
 
     @staticmethod
@@ -590,7 +596,7 @@ class _GatedRMSNorm(torch.autograd.Function):
         dw = _empty(d, dtype=torch.bfloat16, device=x2.device)
         parts = int(load().nsa_rmsnorm_bwd_parts(c_long(rows), c_int(d)))
         partial = _empty(parts * d, dtype=torch.float32, device=x2.device)
-        _check(load().nsa_rmsnorm_bwd_ldg(_p(x2), _p(g2), c_long(ctx.ldg), _p(wb), _p(dy2), _p(rstd), _p(dx), _p(dg), _p(dw),
+        _check(load().nsa_rmsnorm_bwd_ldg(_p(x2), _p(g2), c_long(_row_pitch(g2)), _p(wb), _p(dy2), _p(rstd), _p(dx), _p(dg), _p(dw),
                                           c_void_p(0), _p(partial), c_long(rows), c_int(d), c_int(ctx.mode), _stream()))
         return dx.view(dy.shape), dg.view(ctx.gshape), dw.to(ctx.wdtype), None, None
 
@@ -1478,14 +1484,13 @@ class _SSD(torch.autograd.Function):
         _check(lib.nsa_ssd_chunk_out(_p(Cm), c_long(ldc), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(Hb), _p(dt), _p(A),
                                      _p(Df), _p(y), c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream()))
         ctx.save_for_backward(x, dt, A, Bm, Cm, Df if Df is not None else _empty(0, device=dev), gamma, Hb)
-        ctx.lds = (ldx, ldb, ldc)
         ctx.has_D = D is not None
         return y
 
     @staticmethod
     def backward(ctx, dy):
         x, dt, A, Bm, Cm, Df, gamma, Hb = ctx.saved_tensors
-        ldx, ldb, ldc = ctx.lds
+        ldx, ldb, ldc = (_row_pitch(t.flatten(2)) for t in (x, Bm, Cm))
         Df = Df if ctx.has_D else None
         Bsz, T, H, P = x.shape
         N = Bm.shape[-1]
