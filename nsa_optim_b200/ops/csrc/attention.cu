@@ -63,9 +63,12 @@ struct AttnParams {
 };
 
 // Query tile of a CTA.  Causal: the longest tiles first, so that the last CTAs to start are short (8192 tokens x 32 heads, forward:
-// 668 -> 640 us).  Tiles of one length (a window, no causality) go in the order of the keys they share (65536 tokens x 32 heads,
-// window 512: 1225 us, 1237 backwards).
-__host__ __device__ __forceinline__ bool longest_first(const AttnParams& p) { return p.causal && (p.window == 0 || p.window >= p.T); }
+// 668 -> 640 us).  A window leaves the tiles of its first tokens shorter than the rest, which pays in the same way while
+// they are a sixteenth of all or more (window 512, forward: 4359 tokens 82.8 us, 84.8 in order; 8192 equal); beyond that,
+// and without causality, tiles go in the order of the keys they share (65536 tokens 1225 us, 1237 backwards).
+__host__ __device__ __forceinline__ bool longest_first(const AttnParams& p) {
+  return p.causal && (p.window == 0 || p.T <= 16l * p.window);
+}
 __device__ __forceinline__ int query_tile(const AttnParams& p) { return longest_first(p) ? gridDim.x - 1 - blockIdx.x : blockIdx.x; }
 
 // Which key tiles a query tile visits, for contiguous-range modes.
