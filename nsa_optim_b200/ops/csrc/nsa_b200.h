@@ -144,7 +144,8 @@ int nsa_ssd_state_fwd(const float* S, const float* gamma, float* Hprev, void* Hp
     nc, int H, long E, cudaStream_t st);
 int nsa_ssd_state_bwd(const float* dHprev, const float* gamma, float* dS, void* dS_bf16, int B, int nc, int H, long
     E, cudaStream_t st);
-int nsa_ssd_finish(const void* dB_heads, const void* dC_heads, const float* q, const float* k, const float* r, const
+int nsa_ssd_grad_slots(int B, int T, int H);
+int nsa_ssd_finish(const float* dB_part, const float* dC_part, const float* q, const float* k, const float* r, const
     float* dt, const float* A, float* scratch, void* dB, void* dC, float* ddt, float* dA, float* dD, int B, int T, int H,
     cudaStream_t st);
 int nsa_ssd_chunk_state(int mode, const void* bc, long ld_bc, const void* v, long ld_v, const float* dt, const float*
@@ -153,9 +154,8 @@ int nsa_ssd_chunk_out(const void* Cm, long ld_c, const void* Bm, long ld_b, cons
     Hprev_bf16, const float* dt, const float* A, const float* Dskip, void* y, int B, int T, int H, int N, int P,
     cudaStream_t st);
 int nsa_ssd_chunk_grad(const void* Cm, long ld_c, const void* Bm, long ld_b, const void* x, long ld_x, const void*
-    dy, const void* y, const void* Hprev_bf16, const void* dHn_bf16, const float* dt, const float* A, const float* Dskip,
-    void* dx, float* dB_acc, float* dC_acc, float* q_out, float* k_out, int B, int T, int H, int N, int P, cudaStream_t
-    st);
+    dy, const void* Hprev_bf16, const void* dHn_bf16, const float* dt, const float* A, const float* Dskip, void* dx, float*
+    dB_part, float* dC_part, float* q_out, float* k_out, float* r_out, int B, int T, int H, int N, int P, cudaStream_t st);
 
 /* ---- further entry points of attention.cu ---- */
 int nsa_select_blocks(const float* imp, int* idx, long rows, int T, int nS, int sel_block, int top_n, cudaStream_t
@@ -170,12 +170,6 @@ int nsa_affine_dequant(const uint8_t* q, const float* scale, const float* zero, 
 /* ---- further entry points of runtime.cu ---- */
 int nsa_copy2d(void* dst, long dst_pitch_bytes, const void* src, long src_pitch_bytes, long width_bytes, long rows,
     cudaStream_t st);
-
-/* ---- further entry points of ssd.cu ---- */
-int nsa_ssd_chunk_grad_heads(const void* Cm, long ld_c, const void* Bm, long ld_b, const void* x, long ld_x, const
-    void* dy, const void* y, const void* Hprev_bf16, const void* dHn_bf16, const float* dt, const float* A, const float*
-    Dskip, void* dx, void* dB_heads, void* dC_heads, float* q_out, float* k_out, float* r_out, int B, int T, int H, int
-    N, int P, cudaStream_t st);
 
 #ifdef __cplusplus
 }

@@ -6,15 +6,16 @@
 //     P_ij    = (C_i . B_j) exp(cum_i - cum_j) dt_j   (j <= i)          "decayed scores"
 //     y_i     = sum_j P_ij x_j + exp(cum_i) C_i H + D x_i
 //     H_next  = exp(tot) H + sum_j exp(tot - cum_j) dt_j B_j (outer) x_j
-// Kernels (one CTA per (chunk, head, batch), no loops over tiles):
+// Kernels (chunk_state: one CTA per (chunk, head, batch)):
 //   chunk_state : the sum in H_next (mode 0), or G = sum_i exp(cum_i) C_i (outer) dy_i (mode 1,
 //                 the per-chunk term of the state gradient);   fp32 [.., N, P]
 //   state pass  : the recurrence over chunks (forward) / its reverse (backward), elementwise
 //   chunk_out   : y for the chunk (three MMAs: C B^T, P x, C H)
-//   chunk_grad  : dx, per-head dB / dC contributions (added to fp32 buffers), and the two row
+//   chunk_grad  : dx, dB / dC summed over the heads that a CTA has of a chunk, and the two row
 //                 scalars dy.(y - D x) and x.dx from which d(dt) and dA follow by a suffix sum.
+// chunk_out and chunk_grad are persistent: a CTA walks a run of (chunk, head) items.
 // Decay factors are formed per element in registers (exp2 of a difference that is <= 0), never
-// stored; the [128 x 128] P and dS tiles live only in shared memory as bf16 MMA operands.
+// stored; the [128 x 128] P and dS tiles live only on chip, as bf16 MMA operands.
 #include "host.cuh"
 #include "tc5.cuh"
 
@@ -116,6 +117,14 @@ __device__ __forceinline__ float chunk_scan(float a, float dt, float* cum, float
   return v;
 }
 
+// OR over the sixteen computing warps of a kernel that has one more
+__device__ __forceinline__ bool compute_any(bool bad) {
+  int any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, 1, 512, p;\n\tselp.s32 %0, 1, 0, q;\n\t}\n"
+               : "=r"(any) : "r"(static_cast<int>(bad)) : "memory");
+  return any != 0;
+}
+
 struct SsdParams {
   const float* dt;     // [B, T, H] (after softplus)
   const float* A;      // [H] (negative)
@@ -124,11 +133,11 @@ struct SsdParams {
   // chunk_state
   float* S_out;        // [B, nc, H, NS, PD] fp32
   float* gamma_out;    // [B, nc, H] or null
-  // chunk_grad (y and dx leave through their tensor maps)
-  float* dB_acc;       // [B, T, NS] fp32 (pre-zeroed, summed over heads)
-  float* dC_acc;       // [B, T, NS]
-  bf16* dB_heads;      // [B, T, H, NS] per-head results written with plain stores (null: use the fp32 reductions above);
-  bf16* dC_heads;      //   the caller sums over heads: 64 heads adding into one row contend for the same L2 lines otherwise
+  // chunk_out, chunk_grad (y and dx leave through their tensor maps)
+  int quota;           // (chunk, head) items per CTA
+  int slots;           // partial tiles of dB and dC per chunk: one per CTA that has heads of it
+  float* dB_part;      // [B, T, slots, NS] sums over a CTA's heads of the chunk
+  float* dC_part;
   float* q_out;        // [B, T, H]  dy . (y - D x)
   float* k_out;        // [B, T, H]  x . dx (without the D term)
   float* r_out;        // [B, T, H]  dy . x (gradient of the skip weight D before the sum over tokens), or null
@@ -236,9 +245,80 @@ ssd_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_c
 }
 
 // ---------------------------------------------------------------------------------------
-// chunk_out: y = P x + exp(cum) (C H) + D x  for one (chunk, head, batch).
+// Items (chunk, head), heads fastest, in runs of p.quota per CTA: what a chunk's heads share (B, C and the scores C B^T)
+// is loaded and computed once per run of one chunk ("segment"), and the next items' tiles are in flight meanwhile.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256, 2)
+struct Items {
+  int first, end, H, nc;
+  __device__ Items(const SsdParams& p) : H(p.H), nc(p.nc) {
+    const int total = p.B * p.nc * p.H;
+    first = blockIdx.x * p.quota;
+    end = min(first + p.quota, total);
+  }
+  __device__ int head(int it) const { return it % H; }
+  __device__ int chunk(int it) const { return (it / H) % nc; }
+  __device__ int batch(int it) const { return it / H / nc; }
+  __device__ bool opens(int it) const { return it == first || it % H == 0; }              // first item of a segment
+  __device__ bool closes(int it) const { return it + 1 == end || (it + 1) % H == 0; }     // last one
+};
+
+// dt of four neighbouring rows of the item's chunk, for chunk_scan_warp
+__device__ __forceinline__ float4 load_dt4(const SsdParams& p, const Items& items, int it) {
+  const int t = items.chunk(it) * L + 4 * (threadIdx.x & 31), h = items.head(it);
+  const float* src = p.dt + (static_cast<long>(items.batch(it)) * p.T + t) * p.H + h;
+  return make_float4(t < p.T ? src[0] : 0.f, t + 1 < p.T ? src[p.H] : 0.f, t + 2 < p.T ? src[2 * p.H] : 0.f,
+                     t + 3 < p.T ? src[3 * p.H] : 0.f);
+}
+// One warp: cum[] = inclusive sums of dt A in units of log 2, dts[] = dt, for 128 rows.  Pairs of rows in different blocks of
+// 32 need no exponential of their own: with m the sum at the end of an earlier block, exp(c_i - c_j) = exp(c_i - m)
+// exp(m - c_j), and both exponents are <= 0.  colf[] receives the factors that belong to columns:
+//   FWD  (columns j, rows i): for row block q = 1..3, m = end of block q - 1: exp(m - c_j) dt_j, j < 32 q, at 16 q (q - 1) + j
+//   !FWD (columns i, rows j): for row block q = 0..2, m = end of block q:     exp(c_i - m), i >= 32 (q + 1), at later_block(q) + i
+__device__ __forceinline__ int later_block(int q) { return 16 * q * (7 - q) - 32 * (q + 1); }   // 0, 96, 160 at the block's first row
+template <bool FWD>
+__device__ __forceinline__ void chunk_scan_warp(float4 dt, float a, float* cum, float* dts, float* colf) {
+  const int lane = threadIdx.x & 31, blk = lane >> 3;
+  float4 v = make_float4(dt.x * a, dt.y * a, dt.z * a, dt.w * a);
+  v.y += v.x;
+  v.z += v.y;
+  v.w += v.z;
+  float run = v.w;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float n = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run += n;
+  }
+  const float off = run - v.w;
+  v = make_float4((off + v.x) * LOG2E, (off + v.y) * LOG2E, (off + v.z) * LOG2E, run * LOG2E);
+  *reinterpret_cast<float4*>(cum + 4 * lane) = v;
+  *reinterpret_cast<float4*>(dts + 4 * lane) = dt;
+  auto ex = [](float x) { return exp2f(fminf(x, 0.f)); };
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {                      // m = sum at the end of block q
+    const float m = __shfl_sync(0xffffffffu, v.w, 8 * q + 7);
+    if (FWD) {
+      if (blk <= q)
+        *reinterpret_cast<float4*>(colf + 16 * q * (q + 1) + 4 * lane) =
+            make_float4(ex(m - v.x) * dt.x, ex(m - v.y) * dt.y, ex(m - v.z) * dt.z, ex(m - v.w) * dt.w);
+    } else if (blk > q) {
+      *reinterpret_cast<float4*>(colf + later_block(q) + 4 * lane) = make_float4(ex(v.x - m), ex(v.y - m), ex(v.z - m), ex(v.w - m));
+    }
+  }
+}
+__device__ __forceinline__ void arrive_warp(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) tc5::mbar_arrive(bar);
+}
+
+// ---------------------------------------------------------------------------------------
+// chunk_out: y = P x + exp(cum) (C H) + D x.
+// Sixteen warps compute the weights of one item, then finish the rows of the item before, whose products ran meanwhile;
+// the seventeenth loads, scans, issues and stores.  C B^T stays in registers for all heads of a segment, P goes to tensor
+// memory as the A operand, y leaves from the place of x.
+// ---------------------------------------------------------------------------------------
+constexpr int OUT_ST = 4;                             // stages of (x, H)
+constexpr int OUT_SMEM = 1024 + (4 + 2 * OUT_ST) * BOXB + 2 * (2 * L + 192) * 4 + 256;
+__global__ void __launch_bounds__(544, 1)
 ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_b,
                      const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_h,
                      const __grid_constant__ CUtensorMap tm_y, const SsdParams p) {
@@ -246,141 +326,224 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sC = smem;                  // [2 k-blocks][128][64]
   uint8_t* sB = sC + 2 * BOXB;
-  uint8_t* sX = sB + 2 * BOXB;         // [128 t][64]
-  uint8_t* sH = sX + BOXB;             // [128 n][64]
-  uint8_t* sP = sB;                    // [2 k-blocks][128][64], over B once C B^T is complete
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sH + BOXB);
-  uint64_t* full = bars;
-  uint64_t* m1 = bars + 1;
-  uint64_t* m2 = bars + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3);
+  uint8_t* stages = sB + 2 * BOXB;     // x [128 t][64], H [128 n][64]
+  float* scan = reinterpret_cast<float*>(stages + 2 * OUT_ST * BOXB);   // even and odd items: cum, dts, colf
+  uint64_t* bars = reinterpret_cast<uint64_t*>(scan + 2 * (2 * L + 192));
+  uint64_t *full = bars, *cb = bars + OUT_ST, *ms = cb + 1, *sread = cb + 2;
+  uint64_t *scanned = cb + 3, *ready = cb + 5, *done = cb + 7, *left = cb + 9;    // even and odd items
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(cb + 11);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* cum = reinterpret_cast<float*>(bars + 4);
-  float* dts = cum + L;
-  float* warp_tot = dts + L;
 
-  const int r = threadIdx.x & 127, half = threadIdx.x >> 7, warp = threadIdx.x >> 5;   // row, column half
-  const int h = blockIdx.x, c = p.c0 + blockIdx.y, b = blockIdx.z;    // see each_slab
-  const int t0 = c * L;
+  const int warp = threadIdx.x >> 5;
+  const Items items(p);
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    tc5::mbar_init(full, 1);
-    tc5::mbar_init(m1, 1);
-    tc5::mbar_init(m2, 1);
+    for (int i = 0; i < OUT_ST; ++i) tc5::mbar_init(full + i, 1);
+    tc5::mbar_init(cb, 1);
+    tc5::mbar_init(ms, 1);
+    tc5::mbar_init(sread, 16);
+    for (int i = 0; i < 2; ++i) {
+      tc5::mbar_init(scanned + i, 1);
+      tc5::mbar_init(ready + i, 16);
+      tc5::mbar_init(done + i, 1);
+      tc5::mbar_init(left + i, 16);
+    }
     tc5::fence_barrier_init();
-    tc5::mbar_expect_tx(full, 6 * BOXB);
-    tc5::tma_load_3d(sC, &tm_c, full, 0, t0, b);
-    tc5::tma_load_3d(sC + BOXB, &tm_c, full, 64, t0, b);
-    tc5::tma_load_3d(sB, &tm_b, full, 0, t0, b);
-    tc5::tma_load_3d(sB + BOXB, &tm_b, full, 64, t0, b);
-    tc5::tma_load_4d(sX, &tm_x, full, 0, h, t0, b);
-    tc5::tma_load_2d(sH, &tm_h, full, 0, ((b * p.nc + c) * p.H + h) * NS);
   }
-  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
-  const int t = t0 + r;
-  const bool row_ok = t < p.T;
-  const float dt = row_ok ? p.dt[(static_cast<long>(b) * p.T + t) * p.H + h] : 0.f;
-  const float cm = chunk_scan(dt * p.A[h], dt, cum, dts, warp_tot);
+  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 512); tc5::tmem_relinquish(); }
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-  const uint32_t cS = 0, cYi = 128, cYo = 192;
-  constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);
-  constexpr uint32_t id_y = tc5::make_idesc_bf16(128, PD, 0, 1);
-  bool ok = true;
-  if (warp == 0) {
-    // converged warp, elected lane issues (see ssd_chunk_state_kernel)
-    const bool lead = tc5::elect_one();
-    if (__all_sync(0xffffffffu, tc5::mbar_wait(full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL))) {
-      tc5::fence_after_sync();
-      const uint64_t cc = tc5::desc_kmajor(tc5::smem_u32(sC)), bb = tc5::desc_kmajor(tc5::smem_u32(sB));
-      const uint64_t hh = tc5::desc_mnmajor(tc5::smem_u32(sH), BOXB);
-      if (lead) {
-#pragma unroll
-        for (int kk = 0; kk < NS / 16; ++kk) {
-          const uint64_t off = static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4);
-          tc5::mma_ss(tmem + cS, cc + off, bb + off, id_s, kk > 0 ? 1u : 0u);
+  const uint32_t cS = 0, cP = 128, cYi = 256, cYo = 384;     // the last three: 64 columns for even and odd items each
+  const int n = items.end - items.first;
+  if (warp == 16) {
+    constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);
+    constexpr uint32_t id_y = tc5::make_idesc_bf16(128, PD, 0, 1);
+    const bool lead = tc5::elect_one();                // converged warp, elected lane issues (see ssd_chunk_state_kernel)
+    auto wait = [&](uint64_t* bar, int phase, int code) {
+      return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+    };
+    auto load = [&](int k) {
+      const int it = items.first + k, s = k % OUT_ST;
+      uint8_t* st = stages + s * 2 * BOXB;
+      tc5::mbar_expect_tx(full + s, 2 * BOXB);
+      tc5::tma_load_4d(st, &tm_x, full + s, 0, items.head(it), items.chunk(it) * L, items.batch(it));
+      tc5::tma_load_2d(st + BOXB, &tm_h, full + s, 0, it * NS);
+    };
+    auto load_bc = [&](int it) {
+      const int t0 = items.chunk(it) * L, b = items.batch(it);
+      tc5::mbar_expect_tx(cb, 4 * BOXB);
+      tc5::tma_load_3d(sC, &tm_c, cb, 0, t0, b);
+      tc5::tma_load_3d(sC + BOXB, &tm_c, cb, 64, t0, b);
+      tc5::tma_load_3d(sB, &tm_b, cb, 0, t0, b);
+      tc5::tma_load_3d(sB + BOXB, &tm_b, cb, 64, t0, b);
+    };
+    auto store = [&](int k) {                          // rows past T are clipped by the copy engine
+      const int it = items.first + k;
+      tc5::tma_store_4d(&tm_y, stages + (k % OUT_ST) * 2 * BOXB, 0, items.head(it), items.chunk(it) * L, items.batch(it));
+      tc5::tma_store_commit();
+    };
+    auto scan_item = [&](int k, float4 dt) {
+      float* at = scan + (k & 1) * (2 * L + 192);
+      chunk_scan_warp<true>(dt, p.A[items.head(items.first + k)], at, at + L, at + 2 * L);
+      arrive_warp(scanned + (k & 1));
+    };
+    if (lead) {
+      load_bc(items.first);
+      load(0);
+      if (n > 1) load(1);
+    }
+    scan_item(0, load_dt4(p, items, items.first));
+    if (n > 1) scan_item(1, load_dt4(p, items, items.first + 1));
+    const uint64_t cc = tc5::desc_kmajor(tc5::smem_u32(sC)), bb = tc5::desc_kmajor(tc5::smem_u32(sB));
+    bool ok = true;
+    int seg = 0;
+    for (int k = 0; k < n; ++k) {
+      const int buf = k & 1, s = k % OUT_ST;
+      float4 dt_next = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (k + 2 < n) dt_next = load_dt4(p, items, items.first + k + 2);
+      if (items.opens(items.first + k)) {
+        if (k > 0) {                                   // C is read by the products of item k - 1
+          if (!(ok = wait(done + (buf ^ 1), (k - 1) >> 1, STATUS_TIMEOUT_TMEM_FULL))) break;
+          if (lead) load_bc(items.first + k);
+          if (!(ok = wait(sread, seg - 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
         }
+        if (!(ok = wait(cb, seg, STATUS_TIMEOUT_SMEM_FULL))) break;
+        tc5::fence_after_sync();
+        if (lead) {
+#pragma unroll
+          for (int kk = 0; kk < NS / 16; ++kk) {
+            const uint64_t off = static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4);
+            tc5::mma_ss(tmem + cS, cc + off, bb + off, id_s, kk > 0 ? 1u : 0u);
+          }
+          tc5::mma_commit(ms);
+        }
+        __syncwarp();
+        ++seg;
+      }
+      if (!(ok = wait(full + s, k / OUT_ST, STATUS_TIMEOUT_SMEM_FULL))) break;
+      const uint64_t xx = tc5::desc_mnmajor(tc5::smem_u32(stages + s * 2 * BOXB), BOXB);
+      const uint64_t hh = tc5::desc_mnmajor(tc5::smem_u32(stages + s * 2 * BOXB + BOXB), BOXB);
+      if (lead) {                                      // rows of item k - 2 have left these columns (see below)
 #pragma unroll
         for (int kk = 0; kk < NS / 16; ++kk)
-          tc5::mma_ss(tmem + cYi, cc + static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4),
+          tc5::mma_ss(tmem + cYi + buf * 64, cc + static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4),
                       hh + static_cast<uint64_t>((kk * 2048) >> 4), id_y, kk > 0 ? 1u : 0u);
-        tc5::mma_commit(m1);
       }
-    }
-    __syncwarp();
-  }
-  if (!tc5::mbar_wait(m1, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
-  if (__syncthreads_or(!ok)) ok = false;
-  if (ok) {
-    tc5::fence_after_sync();
-    const float ci = cm * LOG2E;
-    {
-      float s[64];
-      tld64(tmem + lane_off + cS + half * 64, s);
-      uint32_t pk[32];
+      __syncwarp();
+      if (!(ok = wait(ready + buf, k >> 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+      tc5::fence_after_sync();
+      if (lead) {
 #pragma unroll
-      for (int j = 0; j < 64; j += 2) {
-        // operands fetched and the weight computed for every j, then selected: a conditional around
-        // the loads costs a branch per element
-        const int j0 = half * 64 + j;
-        const float2 cj = *reinterpret_cast<const float2*>(cum + j0), dj = *reinterpret_cast<const float2*>(dts + j0);
-        const float w0 = exp2f(fminf(ci - cj.x * LOG2E, 0.f)) * dj.x, w1 = exp2f(fminf(ci - cj.y * LOG2E, 0.f)) * dj.y;
-        const float p0 = j0 <= r ? s[j] * w0 : 0.f;
-        const float p1 = j0 + 1 <= r ? s[j + 1] * w1 : 0.f;
-        pk[j / 2] = tc5::pack_bf16(p0, p1);
+        for (int kk = 0; kk < L / 16; ++kk)
+          tc5::mma_ts(tmem + cYo + buf * 64, tmem + cP + buf * 64 + kk * 8, xx + static_cast<uint64_t>((kk * 2048) >> 4), id_y, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(done + buf);
       }
-      st_row64(sP + half * BOXB, r, pk);
+      __syncwarp();
+      if (k + 2 < n) scan_item(k + 2, dt_next);        // this item's sums have been read
+      if (k > 0) {
+        if (!(ok = wait(left + (buf ^ 1), (k - 1) >> 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+        tc5::fence_after_sync();
+        if (lead) store(k - 1);
+      }
+      if (lead && k + 2 < n) {                         // over the stage of item k - 2, stored one step ago
+        tc5::tma_store_wait_read<1>();
+        load(k + 2);
+      }
+      __syncwarp();
+    }
+    if (ok && wait(left + ((n - 1) & 1), (n - 1) >> 1, STATUS_TIMEOUT_TMEM_EMPTY)) {
+      if (lead) store(n - 1);
+    } else if (lead) {                                 // loads may still be in flight
+      for (int i = 0; i < OUT_ST; ++i) tc5::mbar_drain(full + i);
+      tc5::mbar_drain(cb);
+    }
+    if (lead) tc5::tma_store_wait_read<0>();
+    __syncwarp();
+  } else {
+    const int r = threadIdx.x & 127, lane = r & 31, quad = warp & 3, grp = warp >> 2;    // row, its block of 32, column block
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+    auto wait = [&](uint64_t* bar, int phase, int code) {
+      return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+    };
+    float s[32];                                       // C_i . B_j of the segment: row i = r, columns j = 32 grp ..
+    float e_open = 0.f;                                // exp(cum) of the item whose rows are still open
+    bool ok = true;
+    int seg = 0;
+    for (int k = 0; k <= n; ++k) {
+      float e = 0.f;
+      if (k < n) {
+        const int buf = k & 1;
+        if (items.opens(items.first + k)) {
+          if (!(ok = wait(ms, seg, STATUS_TIMEOUT_TMEM_FULL))) break;
+          tc5::fence_after_sync();
+          tld32(lanes + cS + grp * 32, s);
+          tc5::fence_before_sync();
+          arrive_warp(sread);
+          ++seg;
+        }
+        if (!(ok = wait(scanned + buf, k >> 1, STATUS_TIMEOUT_SMEM_FULL))) break;
+        const float* cum = scan + buf * (2 * L + 192);
+        const float *dts = cum + L + grp * 32, *cols = cum + grp * 32;
+        const float ci = cum[r];
+        e = exp2f(ci);
+        uint32_t pk[16];
+        if (grp < quad) {                              // every column is before every row
+          const float rowf = exp2f(fminf(ci - cum[32 * quad - 1], 0.f));
+          const float* f = cum + 2 * L + 16 * quad * (quad - 1) + grp * 32;          // see chunk_scan_warp
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            const float4 w = *reinterpret_cast<const float4*>(f + j);
+            pk[j / 2] = tc5::pack_bf16(s[j] * (rowf * w.x), s[j + 1] * (rowf * w.y));
+            pk[j / 2 + 1] = tc5::pack_bf16(s[j + 2] * (rowf * w.z), s[j + 3] * (rowf * w.w));
+          }
+        } else if (grp == quad) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            // operands fetched and the weight computed for every j, then selected: a conditional around
+            // the loads costs a branch per element
+            const float2 c = *reinterpret_cast<const float2*>(cols + j), d = *reinterpret_cast<const float2*>(dts + j);
+            const float w0 = exp2f(fminf(ci - c.x, 0.f)) * d.x, w1 = exp2f(fminf(ci - c.y, 0.f)) * d.y;
+            pk[j / 2] = tc5::pack_bf16(j <= lane ? s[j] * w0 : 0.f, j + 1 <= lane ? s[j + 1] * w1 : 0.f);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) pk[j] = 0u;
+        }
+        tc5::tmem_st_x16(lanes + cP + buf * 64 + grp * 16, pk);
+        tc5::tmem_st_wait();
+        tc5::fence_before_sync();
+        arrive_warp(ready + buf);
+      }
+      if (k > 0) {                                     // rows of the item before, whose products ran meanwhile
+        const int q = k - 1, buf = q & 1;
+        if (!(ok = wait(full + q % OUT_ST, q / OUT_ST, STATUS_TIMEOUT_SMEM_FULL) && wait(done + buf, q >> 1, STATUS_TIMEOUT_TMEM_FULL))) break;
+        tc5::fence_after_sync();
+        const float dsk = p.Dskip ? p.Dskip[items.head(items.first + q)] : 0.f;
+        uint8_t* sX = stages + (q % OUT_ST) * 2 * BOXB;
+        float xf[16], yo[16], yi[16];
+        ld_row(sX, r, grp * 16, xf);
+        tld16(lanes + cYo + buf * 64 + grp * 16, yo);
+        tld16(lanes + cYi + buf * 64 + grp * 16, yi);
+        uint32_t o[8];
+#pragma unroll
+        for (int i = 0; i < 16; i += 2)
+          o[i / 2] = tc5::pack_bf16(yo[i] + e_open * yi[i] + dsk * xf[i], yo[i + 1] + e_open * yi[i + 1] + dsk * xf[i + 1]);
+        uint8_t* base = sX + r * 128;                  // the thread's own piece of x, which the products have read
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          *reinterpret_cast<uint4*>(base + (((grp * 2 + j) ^ (r & 7)) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+        tc5::fence_proxy_async();
+        tc5::fence_before_sync();
+        arrive_warp(left + buf);
+      }
+      e_open = e;
     }
   }
-  tc5::fence_proxy_async();
   tc5::fence_before_sync();
   __syncthreads();
-  if (ok && warp == 0) {
-    const bool lead = tc5::elect_one();
-    tc5::fence_after_sync();
-    const uint64_t pp = tc5::desc_kmajor(tc5::smem_u32(sP)), xx = tc5::desc_mnmajor(tc5::smem_u32(sX), BOXB);
-    if (lead) {
-#pragma unroll
-      for (int kk = 0; kk < L / 16; ++kk)
-        tc5::mma_ss(tmem + cYo, pp + static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4),
-                    xx + static_cast<uint64_t>((kk * 2048) >> 4), id_y, kk > 0 ? 1u : 0u);
-      tc5::mma_commit(m2);
-    }
-    __syncwarp();
-  }
-  if (ok && !tc5::mbar_wait(m2, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
-  if (!__syncthreads_or(!ok)) {
-    tc5::fence_after_sync();
-    // y leaves through shared memory and one TMA store (a thread owns a token row, so direct stores
-    // would write 16 bytes per thread into 32 different rows per instruction); x comes from its tile
-    float yo[32], yi[32];
-    tld32(tmem + lane_off + cYo + half * 32, yo);
-    tld32(tmem + lane_off + cYi + half * 32, yi);
-    const float e = exp2f(cm * LOG2E);
-    const float dsk = p.Dskip ? p.Dskip[h] : 0.f;
-    uint32_t o[16];
-    {
-      float xf[32];
-      ld_row(sX, r, half * 32, xf);
-#pragma unroll
-      for (int i = 0; i < 32; i += 2)
-        o[i / 2] = tc5::pack_bf16(yo[i] + e * yi[i] + dsk * xf[i], yo[i + 1] + e * yi[i + 1] + dsk * xf[i + 1]);
-    }
-    st_row32(sP, r, half * 32, o);      // the P tile is free once the second MMA is complete
-    tc5::fence_proxy_async();
-    __syncthreads();
-    if (threadIdx.x == 0) {             // rows past T are clipped by the copy engine
-      tc5::tma_store_4d(&tm_y, sP, 0, h, t0, b);
-      tc5::tma_store_commit();
-      tc5::tma_store_wait_read<0>();
-    }
-  }
-  tc5::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 256); }
+  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 512); }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -388,259 +551,364 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
 // the gradient of the state leaving it (dHn):
 //   S = C B^T, R = dy x^T;  P = S w, dS = R w  with w_ij = exp(cum_i - cum_j) dt_j (j <= i)
 //   dx_j  = sum_i P_ij dy_i + s_j B_j dHn + D dy_j          (s_j = exp(tot - cum_j) dt_j)
-//   dC_i  = sum_j dS_ij B_j + exp(cum_i) dy_i H^T
-//   dB_j  = sum_i dS_ij C_i + s_j x_j dHn^T
-// dB / dC leave per head as bf16 tiles that nsa_ssd_finish sums, or (nsa_ssd_chunk_grad) by fp32 vector reductions over heads.
+//   dC_i  = sum_j dS_ij B_j + (exp(cum_i) dy_i) H^T         summed over the heads of a segment in tensor memory
+//   dB_j  = sum_i dS_ij C_i + (s_j x_j) dHn^T               likewise
+//   q_i   = dy_i . (y_i - D x_i) = sum_j P_ij R_ij + exp(cum_i) dy_i . (C_i H),   k_j = x_j . (dx_j - D dy_j),   r = dy . x
+// Scores are held transposed (lanes j, columns i): P^T, dS^T and the scaled rows of x and dy are A operands in tensor memory, and
+// only dS needs a tile in shared memory.  Sixteen warps compute, a quarter of the columns each; the seventeenth loads the
+// next item (64 KB in flight during a whole item), scans its step sizes, issues the products and stores.
+// The sums over heads leave once per segment, as fp32 tiles that nsa_ssd_finish adds up.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(512, 1)
+constexpr int GRAD_SMEM = 1024 + 14 * BOXB + (2 * L + 192) * 4 + 128;
+__global__ void __launch_bounds__(544, 1)
 ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_b,
                       const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_dy,
                       const __grid_constant__ CUtensorMap tm_h, const __grid_constant__ CUtensorMap tm_dh,
-                      const __grid_constant__ CUtensorMap tm_dx, const __grid_constant__ CUtensorMap tm_dbh,
-                      const __grid_constant__ CUtensorMap tm_dch, const SsdParams p) {
+                      const __grid_constant__ CUtensorMap tm_dx, const SsdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sC = smem;                  // 2 boxes
   uint8_t* sB = sC + 2 * BOXB;         // 2 boxes
-  uint8_t* sX = sB + 2 * BOXB;         // 1
-  uint8_t* sDY = sX + BOXB;            // 1
-  uint8_t* sH = sDY + BOXB;            // 1   [n][p]
-  uint8_t* sDH = sH + BOXB;            // 1   [n][p]
-  uint8_t* sP = sDH + BOXB;            // 2
-  uint8_t* sDS = sP + 2 * BOXB;        // 2
-  uint8_t* sXS = sDS + 2 * BOXB;       // 1   x rows scaled by s_j
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sXS + BOXB);
-  uint64_t* full = bars;
-  uint64_t* m1 = bars + 1;
-  uint64_t* m2 = bars + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* cum = reinterpret_cast<float*>(bars + 4);
+  uint8_t* sDS = sB + 2 * BOXB;        // 2 boxes: dS^T [j][i]; row sums once the products have read it
+  uint8_t* stages = sDS + 2 * BOXB;    // 2 x (x, dy, H [n][p], dHn [n][p])
+  float* cum = reinterpret_cast<float*>(stages + 8 * BOXB);
   float* dts = cum + L;
-  float* warp_tot = dts + L;           // [4], padded to 8
-  float* part = warp_tot + 8;          // [4 groups][128] row sums on their way to one
+  float* colf = dts + L;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(colf + 192);
+  uint64_t *full = bars, *cb = bars + 2, *ms = bars + 3, *sread = bars + 4, *scanned = bars + 5;
+  uint64_t *m0 = bars + 6, *m1 = bars + 7, *ready = bars + 8, *m2 = bars + 9, *left = bars + 10;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* part = reinterpret_cast<float*>(sDS);         // [16][128]
 
-  const int r = threadIdx.x & 127, grp = threadIdx.x >> 7, warp = threadIdx.x >> 5;    // row, column group
-  const int h = blockIdx.x, c = p.c0 + blockIdx.y, b = blockIdx.z;    // see each_slab
-  const int t0 = c * L;
+  const int warp = threadIdx.x >> 5;
+  const Items items(p);
+  const int n = items.end - items.first;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     tc5::mbar_init(full, 1);
+    tc5::mbar_init(full + 1, 1);
+    tc5::mbar_init(cb, 1);
+    tc5::mbar_init(ms, 1);
+    tc5::mbar_init(sread, 16);
+    tc5::mbar_init(scanned, 1);
+    tc5::mbar_init(m0, 1);
     tc5::mbar_init(m1, 1);
+    tc5::mbar_init(ready, 16);
     tc5::mbar_init(m2, 1);
+    tc5::mbar_init(left, 16);
     tc5::fence_barrier_init();
-    tc5::mbar_expect_tx(full, 8 * BOXB);
-    tc5::tma_load_3d(sC, &tm_c, full, 0, t0, b);
-    tc5::tma_load_3d(sC + BOXB, &tm_c, full, 64, t0, b);
-    tc5::tma_load_3d(sB, &tm_b, full, 0, t0, b);
-    tc5::tma_load_3d(sB + BOXB, &tm_b, full, 64, t0, b);
-    tc5::tma_load_4d(sX, &tm_x, full, 0, h, t0, b);
-    tc5::tma_load_4d(sDY, &tm_dy, full, 0, h, t0, b);
-    const int srow = ((b * p.nc + c) * p.H + h) * NS;
-    tc5::tma_load_2d(sH, &tm_h, full, 0, srow);
-    tc5::tma_load_2d(sDH, &tm_dh, full, 0, srow);
   }
   if (warp == 0) { tc5::tmem_alloc(tmem_slot, 512); tc5::tmem_relinquish(); }
-  const int t = t0 + r;
-  const bool row_ok = t < p.T;
-  const float dt = row_ok ? p.dt[(static_cast<long>(b) * p.T + t) * p.H + h] : 0.f;
-  const float cm = chunk_scan(dt * p.A[h], dt, cum, dts, warp_tot);
-  const float tot = cum[L - 1];
-  const float s_row = exp2f((tot - cm) * LOG2E) * dt;
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-  // TMEM columns: S / dC [0,128)  R / dB [128,256)  dX [256,320)  dXi [320,384)  dCi [384,512)
-  const uint32_t cS = 0, cR = 128, cDX = 256, cDXI = 320, cDCI = 384;
-  constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);     // K-major x K-major -> [128 x 128]
-  constexpr uint32_t id_kn64 = tc5::make_idesc_bf16(128, PD, 0, 1);   // K-major A, MN-major B -> [128 x 64]
-  constexpr uint32_t id_tn64 = tc5::make_idesc_bf16(128, PD, 1, 1);   // MN-major A, MN-major B -> [128 x 64]
-  constexpr uint32_t id_kn128 = tc5::make_idesc_bf16(128, NS, 0, 1);  // K-major A, MN-major B -> [128 x 128]
-  constexpr uint32_t id_tn128 = tc5::make_idesc_bf16(128, NS, 1, 1);  // MN-major A, MN-major B -> [128 x 128]
-  bool ok = true;
-  if (warp == 0) {
-    // converged warp, elected lane issues (see ssd_chunk_state_kernel)
-    const bool lead = tc5::elect_one();
-    if (__all_sync(0xffffffffu, tc5::mbar_wait(full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL))) {
+  // TMEM columns.  R^T [0, 128): of each 16 columns, the first 8 become P^T and the others dS^T (bf16 pairs, 16 i).
+  // B dHn, then dx [128, 192).  C H [192, 256): of each 16, 8 become exp(cum) dy and 8 s x (16 p).  dB, dC [256, 512).
+  const uint32_t cR = 0, cX = 128, cY = 192, cDB = 256, cDC = 384;
+  auto wait = [&](uint64_t* bar, int phase, int code) {
+    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+  };
+  if (warp == 16) {
+    constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);     // K-major x K-major -> [128 x 128]
+    constexpr uint32_t id_kn64 = tc5::make_idesc_bf16(128, PD, 0, 1);   // K-major A, MN-major B -> [128 x 64]
+    constexpr uint32_t id_kn128 = tc5::make_idesc_bf16(128, NS, 0, 1);  // K-major A, MN-major B -> [128 x 128]
+    constexpr uint32_t id_tn128 = tc5::make_idesc_bf16(128, NS, 1, 1);  // MN-major A, MN-major B -> [128 x 128]
+    const bool lead = tc5::elect_one();                // converged warp, elected lane issues (see ssd_chunk_state_kernel)
+    auto load = [&](int k) {
+      const int it = items.first + k, h = items.head(it), t0 = items.chunk(it) * L, b = items.batch(it);
+      uint8_t* st = stages + (k & 1) * 4 * BOXB;
+      uint64_t* bar = full + (k & 1);
+      tc5::mbar_expect_tx(bar, 4 * BOXB);
+      tc5::tma_load_4d(st, &tm_x, bar, 0, h, t0, b);
+      tc5::tma_load_4d(st + BOXB, &tm_dy, bar, 0, h, t0, b);
+      tc5::tma_load_2d(st + 2 * BOXB, &tm_h, bar, 0, it * NS);
+      tc5::tma_load_2d(st + 3 * BOXB, &tm_dh, bar, 0, it * NS);
+    };
+    auto load_bc = [&](int it) {
+      const int t0 = items.chunk(it) * L, b = items.batch(it);
+      tc5::mbar_expect_tx(cb, 4 * BOXB);
+      tc5::tma_load_3d(sC, &tm_c, cb, 0, t0, b);
+      tc5::tma_load_3d(sC + BOXB, &tm_c, cb, 64, t0, b);
+      tc5::tma_load_3d(sB, &tm_b, cb, 0, t0, b);
+      tc5::tma_load_3d(sB + BOXB, &tm_b, cb, 64, t0, b);
+    };
+    auto store = [&](int k) {                          // dx from the place of x; rows past T are clipped by the copy engine
+      const int it = items.first + k;
+      tc5::tma_store_4d(&tm_dx, stages + (k & 1) * 4 * BOXB, 0, items.head(it), items.chunk(it) * L, items.batch(it));
+      tc5::tma_store_commit();
+      tc5::tma_store_wait_read<0>();                   // the next item but one goes there
+    };
+    auto scan_item = [&](int k, float4 dt) {
+      chunk_scan_warp<false>(dt, p.A[items.head(items.first + k)], cum, dts, colf);
+      arrive_warp(scanned);
+    };
+    if (lead) {
+      load_bc(items.first);
+      load(0);
+    }
+    scan_item(0, load_dt4(p, items, items.first));
+    const uint64_t ck = tc5::desc_kmajor(tc5::smem_u32(sC)), bk = tc5::desc_kmajor(tc5::smem_u32(sB));
+    const uint64_t cm = tc5::desc_mnmajor(tc5::smem_u32(sC), BOXB), bm = tc5::desc_mnmajor(tc5::smem_u32(sB), BOXB);
+    const uint64_t dsm = tc5::desc_mnmajor(tc5::smem_u32(sDS), BOXB);
+    auto kblock = [](int kk) { return static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4); };
+    auto krow = [](int kk) { return static_cast<uint64_t>((kk * 2048) >> 4); };
+    bool ok = true;
+    int seg = 0;
+    for (int k = 0; k < n; ++k) {
+      const int s = k & 1;
+      const uint8_t* st = stages + s * 4 * BOXB;
+      const bool opens = items.opens(items.first + k);
+      if (opens) {
+        if (k > 0) {                                   // every product and every reader of the segment before is through
+          if (!(ok = wait(left, k - 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+          if (lead) load_bc(items.first + k);
+        }
+        if (!(ok = wait(cb, seg, STATUS_TIMEOUT_SMEM_FULL))) break;
+        tc5::fence_after_sync();
+        if (lead) {
+#pragma unroll
+          for (int kk = 0; kk < NS / 16; ++kk)         // S^T = B C^T
+            tc5::mma_ss(tmem + cR, bk + kblock(kk), ck + kblock(kk), id_s, kk > 0 ? 1u : 0u);
+          tc5::mma_commit(ms);
+        }
+        __syncwarp();
+        if (!(ok = wait(sread, seg, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+        tc5::fence_after_sync();
+        ++seg;
+      }
+      if (!(ok = wait(full + s, k >> 1, STATUS_TIMEOUT_SMEM_FULL))) break;
       tc5::fence_after_sync();
-      const uint64_t cc = tc5::desc_kmajor(tc5::smem_u32(sC)), bb = tc5::desc_kmajor(tc5::smem_u32(sB));
-      const uint64_t xx = tc5::desc_kmajor(tc5::smem_u32(sX)), dy = tc5::desc_kmajor(tc5::smem_u32(sDY));
-      const uint64_t hh = tc5::desc_kmajor(tc5::smem_u32(sH)), dhm = tc5::desc_mnmajor(tc5::smem_u32(sDH), BOXB);
+      const uint64_t xk = tc5::desc_kmajor(tc5::smem_u32(st)), dyk = tc5::desc_kmajor(tc5::smem_u32(st + BOXB));
+      const uint64_t dym = tc5::desc_mnmajor(tc5::smem_u32(st + BOXB), BOXB);
+      const uint64_t hk = tc5::desc_kmajor(tc5::smem_u32(st + 2 * BOXB)), hm = tc5::desc_mnmajor(tc5::smem_u32(st + 2 * BOXB), BOXB);
+      const uint64_t dhk = tc5::desc_kmajor(tc5::smem_u32(st + 3 * BOXB)), dhm = tc5::desc_mnmajor(tc5::smem_u32(st + 3 * BOXB), BOXB);
+      if (lead) {                                      // behind the products of the item before, which read these columns as operands
+#pragma unroll
+        for (int kk = 0; kk < PD / 16; ++kk)           // R^T = x dy^T
+          tc5::mma_ss(tmem + cR, xk + static_cast<uint64_t>((kk * 32) >> 4), dyk + static_cast<uint64_t>((kk * 32) >> 4), id_s, kk > 0 ? 1u : 0u);
+#pragma unroll
+        for (int kk = 0; kk < NS / 16; ++kk)           // C H
+          tc5::mma_ss(tmem + cY, ck + kblock(kk), hm + krow(kk), id_kn64, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(m0);
+      }
+      __syncwarp();
+      if (k > 0 && !opens && !(ok = wait(left, k - 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+      tc5::fence_after_sync();
       if (lead) {
 #pragma unroll
-        for (int kk = 0; kk < NS / 16; ++kk) {             // S = C B^T
-          const uint64_t off = static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4);
-          tc5::mma_ss(tmem + cS, cc + off, bb + off, id_s, kk > 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int kk = 0; kk < PD / 16; ++kk)               // R = dy x^T
-          tc5::mma_ss(tmem + cR, dy + static_cast<uint64_t>((kk * 32) >> 4), xx + static_cast<uint64_t>((kk * 32) >> 4), id_s, kk > 0 ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < NS / 16; ++kk)               // dXi = B dHn   (row scale s_j applied later)
-          tc5::mma_ss(tmem + cDXI, bb + static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4),
-                      dhm + static_cast<uint64_t>((kk * 2048) >> 4), id_kn64, kk > 0 ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < PD / 16; ++kk)               // dCi = dy H^T  (row scale exp(cum_i) applied later)
-          tc5::mma_ss(tmem + cDCI, dy + static_cast<uint64_t>((kk * 32) >> 4), hh + static_cast<uint64_t>((kk * 32) >> 4), id_s, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < NS / 16; ++kk)           // B dHn
+          tc5::mma_ss(tmem + cX, bk + kblock(kk), dhm + krow(kk), id_kn64, kk > 0 ? 1u : 0u);
         tc5::mma_commit(m1);
+        if (k > 0) store(k - 1);
+        if (k + 1 < n) load(k + 1);
       }
+      __syncwarp();
+      float4 dt_next = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (k + 1 < n) dt_next = load_dt4(p, items, items.first + k + 1);
+      if (!(ok = wait(ready, k, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+      tc5::fence_after_sync();
+      if (lead) {
+        const uint32_t sum = opens ? 0u : 1u;
+#pragma unroll
+        for (int kk = 0; kk < L / 16; ++kk)            // dx += P^T dy
+          tc5::mma_ts(tmem + cX, tmem + cR + 16 * kk, dym + krow(kk), id_kn64, 1u);
+#pragma unroll
+        for (int kk = 0; kk < L / 16; ++kk)            // dC += dS B
+          tc5::mma_ss(tmem + cDC, dsm + krow(kk), bm + krow(kk), id_tn128, kk > 0 ? 1u : sum);
+#pragma unroll
+        for (int kk = 0; kk < L / 16; ++kk)            // dB += dS^T C
+          tc5::mma_ts(tmem + cDB, tmem + cR + 16 * kk + 8, cm + krow(kk), id_kn128, kk > 0 ? 1u : sum);
+#pragma unroll
+        for (int kk = 0; kk < PD / 16; ++kk)           // dC += (exp(cum) dy) H^T
+          tc5::mma_ts(tmem + cDC, tmem + cY + 16 * kk, hk + static_cast<uint64_t>((kk * 32) >> 4), id_s, 1u);
+#pragma unroll
+        for (int kk = 0; kk < PD / 16; ++kk)           // dB += (s x) dHn^T
+          tc5::mma_ts(tmem + cDB, tmem + cY + 16 * kk + 8, dhk + static_cast<uint64_t>((kk * 32) >> 4), id_s, 1u);
+        tc5::mma_commit(m2);
+      }
+      __syncwarp();
+      if (k + 1 < n) scan_item(k + 1, dt_next);        // this item's sums have been read
+    }
+    if (ok && wait(left, n - 1, STATUS_TIMEOUT_TMEM_EMPTY)) {
+      if (lead) store(n - 1);
+    } else if (lead) {                                 // copies may still be in flight
+      tc5::mbar_drain(full);
+      tc5::mbar_drain(full + 1);
+      tc5::mbar_drain(cb);
+      tc5::tma_store_wait_read<0>();
     }
     __syncwarp();
-  }
-  // x rows scaled by s_j (operand of the state-path part of dB) while the MMAs run
-  bool landed = tc5::mbar_wait(full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL);
-  if (landed) {
-    if (grp < 2) {
-      float xv[32];
-      ld_row(sX, r, grp * 32, xv);
-      uint32_t pk[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) pk[j] = tc5::pack_bf16(xv[2 * j] * s_row, xv[2 * j + 1] * s_row);
-      st_row32(sXS, r, grp * 32, pk);
-    }
-  } else ok = false;
-  if (!tc5::mbar_wait(m1, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
-  if (__syncthreads_or(!ok)) ok = false;
-  float q_intra = 0.f;      // sum_j P_ij R_ij with P as rounded for the MMA: pairs exactly with x.dx
-  if (ok) {
-    tc5::fence_after_sync();
-    const float ci = cm * LOG2E;
-    float s[32], rr[32];
-    tld32(tmem + lane_off + cS + grp * 32, s);
-    tld32(tmem + lane_off + cR + grp * 32, rr);
-    uint32_t pp[16], ds[16];
-#pragma unroll
-    for (int j = 0; j < 32; j += 2) {
-      // operands fetched and the weight computed for every j, then selected (no branch per element)
-      const int j0 = grp * 32 + j;
-      const float2 cj = *reinterpret_cast<const float2*>(cum + j0), dj = *reinterpret_cast<const float2*>(dts + j0);
-      const float e0 = exp2f(fminf(ci - cj.x * LOG2E, 0.f)) * dj.x, e1 = exp2f(fminf(ci - cj.y * LOG2E, 0.f)) * dj.y;
-      const float w0 = j0 <= r ? e0 : 0.f;
-      const float w1 = j0 + 1 <= r ? e1 : 0.f;
-      pp[j / 2] = tc5::pack_bf16(s[j] * w0, s[j + 1] * w1);
-      ds[j / 2] = tc5::pack_bf16(rr[j] * w0, rr[j + 1] * w1);
-      const float2 pr = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pp[j / 2]));
-      q_intra += pr.x * rr[j] + pr.y * rr[j + 1];
-    }
-    st_row32(sP, r, grp * 32, pp);
-    st_row32(sDS, r, grp * 32, ds);
-  }
-  tc5::fence_proxy_async();
-  tc5::fence_before_sync();
-  __syncthreads();
-  if (ok && warp == 0) {
-    const bool lead = tc5::elect_one();
-    tc5::fence_after_sync();
-    const uint64_t ccm = tc5::desc_mnmajor(tc5::smem_u32(sC), BOXB), bbm = tc5::desc_mnmajor(tc5::smem_u32(sB), BOXB);
-    const uint64_t dym = tc5::desc_mnmajor(tc5::smem_u32(sDY), BOXB), dh = tc5::desc_kmajor(tc5::smem_u32(sDH));
-    const uint64_t ppm = tc5::desc_mnmajor(tc5::smem_u32(sP), BOXB), ds = tc5::desc_kmajor(tc5::smem_u32(sDS));
-    const uint64_t dsm = tc5::desc_mnmajor(tc5::smem_u32(sDS), BOXB), xs = tc5::desc_kmajor(tc5::smem_u32(sXS));
-    if (lead) {
-#pragma unroll
-      for (int kk = 0; kk < L / 16; ++kk)                  // dX = P^T dy
-        tc5::mma_ss(tmem + cDX, ppm + static_cast<uint64_t>((kk * 2048) >> 4), dym + static_cast<uint64_t>((kk * 2048) >> 4), id_tn64, kk > 0 ? 1u : 0u);
-#pragma unroll
-      for (int kk = 0; kk < L / 16; ++kk)                  // dC = dS B
-        tc5::mma_ss(tmem + cS, ds + static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4),
-                    bbm + static_cast<uint64_t>((kk * 2048) >> 4), id_kn128, kk > 0 ? 1u : 0u);
-#pragma unroll
-      for (int kk = 0; kk < L / 16; ++kk)                  // dB = dS^T C
-        tc5::mma_ss(tmem + cR, dsm + static_cast<uint64_t>((kk * 2048) >> 4), ccm + static_cast<uint64_t>((kk * 2048) >> 4), id_tn128, kk > 0 ? 1u : 0u);
-#pragma unroll
-      for (int kk = 0; kk < PD / 16; ++kk)                 // dB += (s x) dHn^T
-        tc5::mma_ss(tmem + cR, xs + static_cast<uint64_t>((kk * 32) >> 4), dh + static_cast<uint64_t>((kk * 32) >> 4), id_s, 1u);
-      tc5::mma_commit(m2);
-    }
-    __syncwarp();
-  }
-  if (ok && !tc5::mbar_wait(m2, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
-  if (!__syncthreads_or(!ok)) {
-    tc5::fence_after_sync();
-    // Outputs leave through shared memory and TMA stores: a thread owns a token row, so direct
-    // stores would write 16 bytes per thread into 32 different rows per instruction.  The operand
-    // tiles are free once the second group of MMAs is complete: dx goes to the x-scaled tile, dC
-    // to the P tile, dB to the dS tile.  x and dy are read back from their own tiles.
-    const long tok = static_cast<long>(b) * p.T + t;
-    const float e = exp2f(cm * LOG2E);
-    const bool heads = p.dB_heads != nullptr;
-    const int col = grp * 32;           // this thread's columns of dB and dC; half as many of dx
-    float kacc = 0.f, racc = 0.f, q_inter = 0.f;
-    {
-      float dxa[16], dxi[16], xf[16], df[16];
-      tld16(tmem + lane_off + cDX + grp * 16, dxa);
-      tld16(tmem + lane_off + cDXI + grp * 16, dxi);
-      const float dsk = p.Dskip ? p.Dskip[h] : 0.f;
-      ld_row(sX, r, grp * 16, xf);
-      ld_row(sDY, r, grp * 16, df);
-      uint32_t o[8];
-#pragma unroll
-      for (int i = 0; i < 16; i += 2) {
-        const float g0 = dxa[i] + s_row * dxi[i], g1 = dxa[i + 1] + s_row * dxi[i + 1];
-        kacc += xf[i] * g0 + xf[i + 1] * g1;
-        racc += xf[i] * df[i] + xf[i + 1] * df[i + 1];
-        o[i / 2] = tc5::pack_bf16(g0 + dsk * df[i], g1 + dsk * df[i + 1]);
-      }
-      uint8_t* base = sXS + r * 128;
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        *reinterpret_cast<uint4*>(base + (((grp * 2 + j) ^ (r & 7)) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-    }
-    {                       // q_inter = C_i . (dy_i H^T): the state-path part of dy.(y - D x), before exp(cum_i)
-      float dc[32], dci[32], db[32];
-      tld32(tmem + lane_off + cS + col, dc);
-      tld32(tmem + lane_off + cDCI + col, dci);
-      tld32(tmem + lane_off + cR + col, db);
-      {
-        float cv[32];
-        ld_row(sC, r, col, cv);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) q_inter += cv[j] * dci[j];
-      }
-      if (heads) {
-        uint32_t vc[16], vb[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          vc[j] = tc5::pack_bf16(dc[2 * j] + e * dci[2 * j], dc[2 * j + 1] + e * dci[2 * j + 1]);
-          vb[j] = tc5::pack_bf16(db[2 * j], db[2 * j + 1]);
+  } else {
+    const int r = threadIdx.x & 127, lane = r & 31, quad = warp & 3, grp = warp >> 2;    // row, its block of 32, column block
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+    float s[32];                                       // B_j . C_i of the segment: row j = r, columns i = 32 grp ..
+    bool ok = true;
+    int seg = 0;
+    for (int k = 0; k < n; ++k) {
+      const int it = items.first + k, h = items.head(it), b = items.batch(it), t = items.chunk(it) * L + r;
+      uint8_t* sX = stages + (k & 1) * 4 * BOXB;
+      const uint8_t* sDY = sX + BOXB;
+      if (items.opens(it)) {
+        ok = ok && wait(ms, seg, STATUS_TIMEOUT_TMEM_FULL);
+        if (ok) {
+          tc5::fence_after_sync();
+          tld32(lanes + cR + grp * 32, s);
+          tc5::fence_before_sync();
+          arrive_warp(sread);
         }
-        st_row32(sP, r, col, vc);
-        st_row32(sDS, r, col, vb);
-      } else if (row_ok) {
-        float4* pc = reinterpret_cast<float4*>(p.dC_acc + tok * NS + col);
-        float4* pb = reinterpret_cast<float4*>(p.dB_acc + tok * NS + col);
+        ++seg;
+      }
+      ok = ok && wait(scanned, k, STATUS_TIMEOUT_SMEM_FULL) && wait(full + (k & 1), k >> 1, STATUS_TIMEOUT_SMEM_FULL) &&
+           wait(m0, k, STATUS_TIMEOUT_TMEM_FULL);
+      float q_intra = 0.f;      // sum_j P_ij R_ij with P as rounded for the MMA (pairs exactly with x.dx): of column i = 32 grp + lane
+      float q_inter = 0.f, e = 0.f;
+      if (ok) {
+        tc5::fence_after_sync();
+        const float cj = cum[r], dtj = dts[r];
+        const float s_row = exp2f(cum[L - 1] - cj) * dtj;
+        e = exp2f(cj);
+        // 16 columns: weights -> P^T, dS^T and the column sums of P^T R^T over this warp's 32 rows
+        auto sixteen = [&](const int hf, auto weight) {
+          float rr[16], g[16];
+          tld16(lanes + cR + grp * 32 + hf * 16, rr);
+          uint32_t pk[8], ds[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          atomicAdd(pc + j, make_float4(dc[4 * j] + e * dci[4 * j], dc[4 * j + 1] + e * dci[4 * j + 1],
-                                        dc[4 * j + 2] + e * dci[4 * j + 2], dc[4 * j + 3] + e * dci[4 * j + 3]));
-          atomicAdd(pb + j, make_float4(db[4 * j], db[4 * j + 1], db[4 * j + 2], db[4 * j + 3]));
+          for (int i = 0; i < 16; i += 2) {
+            const float2 w = weight(hf * 16 + i);
+            pk[i / 2] = tc5::pack_bf16(s[hf * 16 + i] * w.x, s[hf * 16 + i + 1] * w.y);
+            ds[i / 2] = tc5::pack_bf16(rr[i] * w.x, rr[i + 1] * w.y);
+            const float2 pr = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[i / 2]));
+            g[i] = pr.x * rr[i];
+            g[i + 1] = pr.y * rr[i + 1];
+          }
+          tc5::tmem_st_x8(lanes + cR + grp * 32 + hf * 16, pk);
+          tc5::tmem_st_x8(lanes + cR + grp * 32 + hf * 16 + 8, ds);
+          tc5::tmem_st_wait();
+          if (hf == 0) ok = wait(m1, k, STATUS_TIMEOUT_TMEM_FULL);      // row sums of the item before have been read
+          const int c0 = grp * 32 + hf * 16, j0 = (c0 & 63) >> 3;
+          uint8_t* base = sDS + (c0 >> 6) * BOXB + r * 128;
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            *reinterpret_cast<uint4*>(base + (((j0 + j) ^ (r & 7)) << 4)) = make_uint4(ds[4 * j], ds[4 * j + 1], ds[4 * j + 2], ds[4 * j + 3]);
+          // halves of the columns change hands between lanes until a lane holds the sum of one column
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) {
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < o; ++i) {
+              const float send = up ? g[i] : g[i + o];
+              g[i] = (up ? g[i + o] : g[i]) + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+          }
+          g[0] += __shfl_xor_sync(0xffffffffu, g[0], 16);
+          if ((lane >> 4) == hf) q_intra = g[0];
+        };
+        if (grp > quad) {                              // every column i is behind every row j
+          const float rowf = exp2f(fminf(cum[32 * quad + 31] - cj, 0.f)) * dtj;
+          const float* f = colf + later_block(quad) + grp * 32;
+          auto weight = [&](int i) {
+            const float2 c = *reinterpret_cast<const float2*>(f + i);
+            return make_float2(rowf * c.x, rowf * c.y);
+          };
+          sixteen(0, weight);
+          sixteen(1, weight);
+        } else if (grp == quad) {
+          auto weight = [&](int i) {                   // computed for every i, then selected (no branch per element)
+            const float2 c = *reinterpret_cast<const float2*>(cum + grp * 32 + i);
+            const float w0 = exp2f(fminf(c.x - cj, 0.f)) * dtj, w1 = exp2f(fminf(c.y - cj, 0.f)) * dtj;
+            return make_float2(i >= lane ? w0 : 0.f, i + 1 >= lane ? w1 : 0.f);
+          };
+          sixteen(0, weight);
+          sixteen(1, weight);
+        } else {                                       // masked: zero operands
+          uint32_t z[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) z[i] = 0u;
+          tc5::tmem_st_x16(lanes + cR + grp * 32, z);
+          tc5::tmem_st_x16(lanes + cR + grp * 32 + 16, z);
+          tc5::tmem_st_wait();
+          ok = wait(m1, k, STATUS_TIMEOUT_TMEM_FULL);
+          st_row32(sDS, r, grp * 32, z);
+        }
+        if (ok) {
+          tc5::fence_after_sync();
+          // dx starts from s_j B_j dHn; rows of dy and x, scaled, take the place of C H.  (The sources of a tcgen05.st must
+          // stay as they are until it is waited for: all three leave together.)
+          float v[16], u[16];
+          uint32_t w[16], a[8], c[8];
+          tld16(lanes + cX + grp * 16, v);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(s_row * v[i]);
+          tld16(lanes + cY + grp * 16, v);
+          ld_row(sDY, r, grp * 16, u);
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            q_inter += u[i] * v[i] + u[i + 1] * v[i + 1];
+            a[i / 2] = tc5::pack_bf16(e * u[i], e * u[i + 1]);
+          }
+          ld_row(sX, r, grp * 16, u);
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) c[i / 2] = tc5::pack_bf16(s_row * u[i], s_row * u[i + 1]);
+          tc5::tmem_st_x16(lanes + cX + grp * 16, w);
+          tc5::tmem_st_x8(lanes + cY + grp * 16, a);
+          tc5::tmem_st_x8(lanes + cY + grp * 16 + 8, c);
+          tc5::tmem_st_wait();
+          tc5::fence_proxy_async();
+          tc5::fence_before_sync();
+          arrive_warp(ready);
         }
       }
-    }
-    // row sums: groups add up in a fixed order
-    part[grp * L + r] = kacc;
-    part[(4 + grp) * L + r] = racc;
-    part[(8 + grp) * L + r] = q_intra;
-    part[(12 + grp) * L + r] = q_inter;
-    tc5::fence_proxy_async();
-    __syncthreads();
-    if (threadIdx.x == 0) {             // rows past T are clipped by the copy engine
-      tc5::tma_store_4d(&tm_dx, sXS, 0, h, t0, b);
-      if (heads) {
-        tc5::tma_store_4d(&tm_dch, sP, 0, h, t0, b);
-        tc5::tma_store_4d(&tm_dch, sP + BOXB, 64, h, t0, b);
-        tc5::tma_store_4d(&tm_dbh, sDS, 0, h, t0, b);
-        tc5::tma_store_4d(&tm_dbh, sDS + BOXB, 64, h, t0, b);
+      ok = ok && wait(m2, k, STATUS_TIMEOUT_TMEM_FULL);
+      const long tok = static_cast<long>(b) * p.T + t;
+      if (ok) {
+        tc5::fence_after_sync();
+        float kacc = 0.f, racc = 0.f;
+        float g[16], xf[16], df[16];
+        tld16(lanes + cX + grp * 16, g);
+        const float dsk = p.Dskip ? p.Dskip[h] : 0.f;
+        ld_row(sX, r, grp * 16, xf);
+        ld_row(sDY, r, grp * 16, df);
+        uint32_t o[8];
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          kacc += xf[i] * g[i] + xf[i + 1] * g[i + 1];
+          racc += xf[i] * df[i] + xf[i + 1] * df[i + 1];
+          o[i / 2] = tc5::pack_bf16(g[i] + dsk * df[i], g[i + 1] + dsk * df[i + 1]);
+        }
+        uint8_t* base = sX + r * 128;                  // the thread's own piece of x, which the products have read
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          *reinterpret_cast<uint4*>(base + (((grp * 2 + j) ^ (r & 7)) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+        part[grp * L + r] = kacc;
+        part[(4 + grp) * L + r] = racc;
+        part[(8 + grp) * L + r] = q_inter;
+        part[(12 + quad) * L + grp * 32 + lane] = q_intra;
       }
-      tc5::tma_store_commit();
-      tc5::tma_store_wait_read<0>();    // shared memory must outlive the copies' reads
-    }
-    if (grp > 0 && row_ok) {            // group g finishes sum g (thread 0 is busy with the stores)
-      auto row_sum = [&](int k) { return (part[k * L + r] + part[(k + 1) * L + r]) + (part[(k + 2) * L + r] + part[(k + 3) * L + r]); };
-      if (grp == 1) p.k_out[tok * p.H + h] = row_sum(0);
-      else if (grp == 2) { if (p.r_out) p.r_out[tok * p.H + h] = row_sum(4); }
-      else p.q_out[tok * p.H + h] = row_sum(8) + e * row_sum(12);
+      if (compute_any(!ok)) { ok = false; break; }     // all sixteen warps leave together
+      if (t < p.T) {                                   // groups add up in a fixed order; group g finishes sum g
+        auto row_sum = [&](int i) { return (part[i * L + r] + part[(i + 1) * L + r]) + (part[(i + 2) * L + r] + part[(i + 3) * L + r]); };
+        if (grp == 0) p.k_out[tok * p.H + h] = row_sum(0);
+        else if (grp == 1) { if (p.r_out) p.r_out[tok * p.H + h] = row_sum(4); }
+        else if (grp == 2) p.q_out[tok * p.H + h] = row_sum(12) + e * row_sum(8);
+      }
+      if (items.closes(it)) {                          // the segment's sums over heads
+        const int chunk = it / p.H, slot = blockIdx.x - static_cast<int>(static_cast<long>(chunk) * p.H / p.quota);
+        const long o = (tok * p.slots + slot) * NS + grp * 32;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float v[32];
+          tld32(lanes + (q ? cDC : cDB) + grp * 32, v);
+          float* dst = (q ? p.dC_part : p.dB_part) + o;
+          if (t < p.T)
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        }
+      }
+      tc5::fence_proxy_async();
+      tc5::fence_before_sync();
+      arrive_warp(left);
     }
   }
   tc5::fence_before_sync();
@@ -730,31 +998,24 @@ int launch_state(const float* in, const float* gamma, float* out, void* out_bf, 
 // ---------------------------------------------------------------------------------------
 // What follows the chunk gradients: sums over heads and over time.
 // ---------------------------------------------------------------------------------------
-// out[row][:] = sum over heads of in[row][h][:] for dB (z = 0) and dC (z = 1), fp32 sums in a fixed order, bf16 out.  A warp owns a
-// token: its rows are contiguous, 16 bytes per lane, two heads per instruction.
-__global__ void __launch_bounds__(256) ssd_sum_heads_kernel(const bf16* __restrict__ dBh, const bf16* __restrict__ dCh,
-                                                            bf16* __restrict__ dB, bf16* __restrict__ dC, long rows, int H) {
+// dB (blockIdx.y = 0) and dC: a token's partial rows, fp32 sums in a fixed order, bf16 out.  A chunk has one partial per CTA of the
+// gradient kernel that had heads of it.  A warp owns a token, 16 bytes per lane.
+__global__ void __launch_bounds__(256) ssd_sum_parts_kernel(const float* __restrict__ dB_part, const float* __restrict__ dC_part,
+                                                            bf16* __restrict__ dB, bf16* __restrict__ dC, long rows, int T, int H,
+                                                            int nc, int quota, int slots) {
   const long row = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
-  const uint4* src = reinterpret_cast<const uint4*>((blockIdx.y ? dCh : dBh) + row * H * NS) + lane;
-  float acc[8] = {};
-#pragma unroll 8
-  for (int h = lane >> 4; h < H; h += 2) {
-    const uint4 v = src[(h - (lane >> 4)) * (NS / 8)];
-    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 f = __bfloat1622float2(p[k]);
-      acc[2 * k] += f.x;
-      acc[2 * k + 1] += f.y;
-    }
+  const long first = (row / T * nc + (row % T) / L) * H;           // the chunk's first item
+  const int n = static_cast<int>((first + H - 1) / quota - first / quota) + 1;
+  const float4* src = reinterpret_cast<const float4*>((blockIdx.y ? dC_part : dB_part) + row * slots * NS) + lane;
+  float4 acc = src[0];
+#pragma unroll 4
+  for (int i = 1; i < n; ++i) {
+    const float4 v = src[i * (NS / 4)];
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
   }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);
-  if (lane < 16)
-    reinterpret_cast<uint4*>((blockIdx.y ? dC : dB) + row * NS)[lane] =
-        make_uint4(tc5::pack_bf16(acc[0], acc[1]), tc5::pack_bf16(acc[2], acc[3]), tc5::pack_bf16(acc[4], acc[5]), tc5::pack_bf16(acc[6], acc[7]));
+  reinterpret_cast<uint2*>((blockIdx.y ? dC : dB) + row * NS)[lane] = make_uint2(tc5::pack_bf16(acc.x, acc.y), tc5::pack_bf16(acc.z, acc.w));
 }
 
 // With da_t = sum over t' >= t of (q - k)_t' :  ddt = da A + k / dt,  dA = sum da dt,  dD = sum r  (sums over tokens and batch).
@@ -864,6 +1125,19 @@ void each_slab(SsdParams& p, F launch) {
   } while (p.c0 < p.nc);
 }
 
+// (chunk, head) items are dealt out in equal runs, one per SM (one CTA fills an SM)
+int items_per_cta(int B, int T, int H) {
+  const long total = static_cast<long>(B) * ((T + L - 1) / L) * H, sms = nsa::sm_count();
+  return static_cast<int>((total + sms - 1) / sms);
+}
+// Sets the runs of a launch and returns its CTAs (0: nothing to do)
+unsigned deal_items(SsdParams& p) {
+  p.quota = items_per_cta(p.B, p.T, p.H);
+  if (p.quota == 0) return 0;
+  const long total = static_cast<long>(p.B) * p.nc * p.H;
+  return static_cast<unsigned>((total + p.quota - 1) / p.quota);
+}
+
 int map_bc(CUtensorMap* m, const void* base, int B, int T, long ld) {
   uint64_t dims[3] = {(uint64_t)NS, (uint64_t)T, (uint64_t)B};
   uint64_t strides[2] = {(uint64_t)ld * 2, (uint64_t)T * ld * 2};
@@ -873,13 +1147,6 @@ int map_bc(CUtensorMap* m, const void* base, int B, int T, long ld) {
 int map_v(CUtensorMap* m, const void* base, int B, int T, int H, long ld) {
   uint64_t dims[4] = {(uint64_t)PD, (uint64_t)H, (uint64_t)T, (uint64_t)B};
   uint64_t strides[3] = {(uint64_t)PD * 2, (uint64_t)ld * 2, (uint64_t)T * ld * 2};
-  uint32_t box[4] = {64, 1, (uint32_t)L, 1};
-  return nsa::make_tmap_bf16(m, base, 4, dims, strides, box, 1);
-}
-int map_heads(CUtensorMap* m, const void* base, int B, int T, int H, bool real) {
-  if (!real) return map_v(m, base, B, T, H, static_cast<long>(H) * PD);
-  uint64_t dims[4] = {(uint64_t)NS, (uint64_t)H, (uint64_t)T, (uint64_t)B};
-  uint64_t strides[3] = {(uint64_t)NS * 2, (uint64_t)H * NS * 2, (uint64_t)T * H * NS * 2};
   uint32_t box[4] = {64, 1, (uint32_t)L, 1};
   return nsa::make_tmap_bf16(m, base, 4, dims, strides, box, 1);
 }
@@ -907,17 +1174,24 @@ extern "C" int nsa_ssd_state_bwd(const float* dHprev, const float* gamma, float*
   return launch_state<true>(dHprev, gamma, dS, dS_bf16, nullptr, B, nc, H, E, st);
 }
 
-// dB_heads, dC_heads [B, T, H, 128] bf16 -> dB, dC [B, T, 128] bf16; q, k, r (or null), dt [B, T, H], A [H] fp32 ->
-// ddt [B, T, H], dA [H], dD [H] (or null).  scratch: 3 * B * ceil(T / 128) * H floats.
-extern "C" int nsa_ssd_finish(const void* dB_heads, const void* dC_heads, const float* q, const float* k, const float* r,
+// Partial tiles of dB and dC per chunk that nsa_ssd_chunk_grad writes: the runs of (chunk, head) items that the heads of one
+// chunk can fall into.
+extern "C" int nsa_ssd_grad_slots(int B, int T, int H) {
+  const int quota = items_per_cta(B, T, H);
+  return H < 2 ? 1 : (H - 2) / quota + 2;
+}
+
+// dB_part, dC_part [B, T, slots, 128] fp32 of nsa_ssd_chunk_grad -> dB, dC [B, T, 128] bf16; q, k, r (or null), dt [B, T, H], A [H]
+// fp32 -> ddt [B, T, H], dA [H], dD [H] (or null).  scratch: 3 * B * ceil(T / 128) * H floats.
+extern "C" int nsa_ssd_finish(const float* dB_part, const float* dC_part, const float* q, const float* k, const float* r,
                               const float* dt, const float* A, float* scratch, void* dB, void* dC, float* ddt, float* dA,
                               float* dD, int B, int T, int H, cudaStream_t st) {
   if (B <= 0 || T <= 0 || H <= 0 || (r == nullptr) != (dD == nullptr)) return nsa::fail(NSA_ERR_SHAPE, "ssd_finish: bad arguments");
   const long rows = static_cast<long>(B) * T;
   const int nc = (T + L - 1) / L;
   float *totals = scratch, *pA = totals + static_cast<long>(B) * nc * H, *pD = pA + static_cast<long>(B) * nc * H;
-  ssd_sum_heads_kernel<<<dim3((unsigned)((rows + 7) / 8), 2), 256, 0, st>>>((const bf16*)dB_heads, (const bf16*)dC_heads, (bf16*)dB,
-                                                                           (bf16*)dC, rows, H);
+  ssd_sum_parts_kernel<<<dim3((unsigned)((rows + 7) / 8), 2), 256, 0, st>>>(dB_part, dC_part, (bf16*)dB, (bf16*)dC, rows, T, H, nc,
+                                                                           items_per_cta(B, T, H), nsa_ssd_grad_slots(B, T, H));
   ssd_totals_kernel<<<dim3(nc, B), 256, 0, st>>>(q, k, r, totals, pD, T, H, nc);
   ssd_ddt_kernel<<<dim3(nc, B), 256, 0, st>>>(q, k, dt, A, totals, ddt, pA, T, H, nc);
   ssd_head_sums_kernel<<<dim3((H + 31) / 32, dD ? 2 : 1), 1024, 0, st>>>(pA, pD, dA, dD, B * nc, H);
@@ -968,25 +1242,26 @@ extern "C" int nsa_ssd_chunk_out(const void* Cm, long ld_c, const void* Bm, long
   SsdParams p{};
   p.dt = dt; p.A = A; p.Dskip = Dskip; p.B = B; p.T = T; p.H = H; p.nc = nc;
   p.status = nsa::status_ptr();
-  const int smem = 6 * BOXB + 1024 + 2048;
   static bool cfg = false;
-  if (!cfg) { if ((rc = smem_attr(ssd_chunk_out_kernel, smem))) return rc; cfg = true; }
+  if (!cfg) { if ((rc = smem_attr(ssd_chunk_out_kernel, OUT_SMEM))) return rc; cfg = true; }
   if ((rc = map_v(&ty, y, B, T, H, static_cast<long>(H) * PD))) return rc;
-  each_slab(p, [&](dim3 grid) { ssd_chunk_out_kernel<<<grid, 256, smem, st>>>(tc, tb, tx, th, ty, p); });
+  ssd_chunk_out_kernel<<<deal_items(p), 544, OUT_SMEM, st>>>(tc, tb, tx, th, ty, p);
+  nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_chunk_out launch");
 }
 
-// dB_acc / dC_acc: fp32 [B, T, N], zeroed by the caller.  q_out / k_out: fp32 [B, T, H].
-static int ssd_chunk_grad_impl(const void* Cm, long ld_c, const void* Bm, long ld_b, const void* x, long ld_x,
-                               const void* dy, const void* Hprev_bf16, const void* dHn_bf16, const float* dt, const float* A,
-                               const float* Dskip, void* dx, float* dB_acc, float* dC_acc, void* dB_heads, void* dC_heads,
-                               float* q_out, float* k_out, float* r_out, int B, int T, int H, int N, int P, cudaStream_t st) {
+// dx [B, T, H, P]; dB_part, dC_part [B, T, nsa_ssd_grad_slots, N] fp32; q_out, k_out and r_out (or null) fp32 [B, T, H]: dy . (y - D x),
+// x . (dx - D dy) and dy . x per token and head.
+extern "C" int nsa_ssd_chunk_grad(const void* Cm, long ld_c, const void* Bm, long ld_b, const void* x, long ld_x,
+                                  const void* dy, const void* Hprev_bf16, const void* dHn_bf16, const float* dt, const float* A,
+                                  const float* Dskip, void* dx, float* dB_part, float* dC_part, float* q_out, float* k_out,
+                                  float* r_out, int B, int T, int H, int N, int P, cudaStream_t st) {
   int rc = check_dims(N, P, ld_c | ld_b, ld_x);
   if (rc) return rc;
   const int nc = (T + L - 1) / L;
   const long rows = static_cast<long>(B) * nc * H * NS;
-  CUtensorMap tc, tb, tx, tdy, th, tdh, tdx, tdbh, tdch;
+  CUtensorMap tc, tb, tx, tdy, th, tdh, tdx;
   if ((rc = map_bc(&tc, Cm, B, T, ld_c))) return rc;
   if ((rc = map_bc(&tb, Bm, B, T, ld_b))) return rc;
   if ((rc = map_v(&tx, x, B, T, H, ld_x))) return rc;
@@ -994,38 +1269,14 @@ static int ssd_chunk_grad_impl(const void* Cm, long ld_c, const void* Bm, long l
   if ((rc = map_state(&th, Hprev_bf16, rows))) return rc;
   if ((rc = map_state(&tdh, dHn_bf16, rows))) return rc;
   if ((rc = map_v(&tdx, dx, B, T, H, static_cast<long>(H) * PD))) return rc;
-  // per-head dB / dC [B, T, H, N]; without them the maps point at dx and are never used
-  if ((rc = map_heads(&tdbh, dB_heads ? dB_heads : dx, B, T, H, dB_heads != nullptr))) return rc;
-  if ((rc = map_heads(&tdch, dC_heads ? dC_heads : dx, B, T, H, dC_heads != nullptr))) return rc;
   SsdParams p{};
   p.dt = dt; p.A = A; p.Dskip = Dskip; p.B = B; p.T = T; p.H = H; p.nc = nc;
-  p.dB_acc = dB_acc; p.dC_acc = dC_acc; p.q_out = q_out; p.k_out = k_out; p.status = nsa::status_ptr();
-  p.dB_heads = (bf16*)dB_heads; p.dC_heads = (bf16*)dC_heads; p.r_out = r_out;
-  const int smem = 13 * BOXB + 1024 + 2048 + 16 * L * 4;
+  p.dB_part = dB_part; p.dC_part = dC_part; p.q_out = q_out; p.k_out = k_out; p.r_out = r_out; p.status = nsa::status_ptr();
+  p.slots = nsa_ssd_grad_slots(B, T, H);
   static bool cfg = false;
-  if (!cfg) { if ((rc = smem_attr(ssd_chunk_grad_kernel, smem))) return rc; cfg = true; }
-  each_slab(p, [&](dim3 grid) { ssd_chunk_grad_kernel<<<grid, 512, smem, st>>>(tc, tb, tx, tdy, th, tdh, tdx, tdbh, tdch, p); });
+  if (!cfg) { if ((rc = smem_attr(ssd_chunk_grad_kernel, GRAD_SMEM))) return rc; cfg = true; }
+  ssd_chunk_grad_kernel<<<deal_items(p), 544, GRAD_SMEM, st>>>(tc, tb, tx, tdy, th, tdh, tdx, p);
+  nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_chunk_grad launch");
-}
-
-// y is not read (the sums that used it come from the products themselves); callers may pass null.
-extern "C" int nsa_ssd_chunk_grad(const void* Cm, long ld_c, const void* Bm, long ld_b, const void* x, long ld_x,
-                                  const void* dy, const void* y, const void* Hprev_bf16, const void* dHn_bf16,
-                                  const float* dt, const float* A, const float* Dskip, void* dx, float* dB_acc,
-                                  float* dC_acc, float* q_out, float* k_out, int B, int T, int H, int N, int P,
-                                  cudaStream_t st) {
-  return ssd_chunk_grad_impl(Cm, ld_c, Bm, ld_b, x, ld_x, dy, Hprev_bf16, dHn_bf16, dt, A, Dskip, dx, dB_acc, dC_acc,
-                             nullptr, nullptr, q_out, k_out, nullptr, B, T, H, N, P, st);
-}
-// Same, with dB / dC written per head as bf16 [B, T, H, N] (plain stores); the caller sums over heads.
-// r_out (optional, fp32 [B, T, H]) receives dy . x per token and head.
-extern "C" int nsa_ssd_chunk_grad_heads(const void* Cm, long ld_c, const void* Bm, long ld_b, const void* x, long ld_x,
-                                        const void* dy, const void* y, const void* Hprev_bf16, const void* dHn_bf16,
-                                        const float* dt, const float* A, const float* Dskip, void* dx, void* dB_heads,
-                                        void* dC_heads, float* q_out, float* k_out, float* r_out, int B, int T, int H,
-                                        int N, int P, cudaStream_t st) {
-  if (dB_heads == nullptr || dC_heads == nullptr) return nsa::fail(NSA_ERR_SHAPE, "ssd_chunk_grad_heads: null output");
-  return ssd_chunk_grad_impl(Cm, ld_c, Bm, ld_b, x, ld_x, dy, Hprev_bf16, dHn_bf16, dt, A, Dskip, dx, nullptr, nullptr,
-                             dB_heads, dC_heads, q_out, k_out, r_out, B, T, H, N, P, st);
 }

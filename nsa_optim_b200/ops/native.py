@@ -1506,23 +1506,22 @@ class _SSD(torch.autograd.Function):
                                      _stream()))
         del G
         dx = _empty(Bsz, T, H, P, dtype=torch.bfloat16, device=dev)
-        # dB / dC: every head writes its own bf16 rows, summed afterwards (64 heads reducing into the
-        # same fp32 rows with vector atomics was the slowest part of the kernel)
-        dBh = _empty(Bsz, T, H, N, dtype=torch.bfloat16, device=dev)
-        dCh = _empty(Bsz, T, H, N, dtype=torch.bfloat16, device=dev)
+        # dB / dC: fp32 sums over the heads that one CTA has of a chunk, added up afterwards
+        slots = lib.nsa_ssd_grad_slots(c_int(Bsz), c_int(T), c_int(H))
+        dB_part, dC_part = (_empty(Bsz, T, slots, N, dtype=torch.float32, device=dev) for _ in range(2))
         q = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
         k = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
         rdx = _empty(Bsz, T, H, dtype=torch.float32, device=dev) if ctx.has_D else None
-        _check(lib.nsa_ssd_chunk_grad_heads(_p(Cm), c_long(ldc), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(dy), c_void_p(0), _p(Hb),
-                                            _p(dHn), _p(dt), _p(A), _p(Df), _p(dx), _p(dBh), _p(dCh), _p(q), _p(k), _p(rdx),
-                                            c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream()))
+        _check(lib.nsa_ssd_chunk_grad(_p(Cm), c_long(ldc), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(dy), _p(Hb), _p(dHn), _p(dt),
+                                      _p(A), _p(Df), _p(dx), _p(dB_part), _p(dC_part), _p(q), _p(k), _p(rdx), c_int(Bsz), c_int(T),
+                                      c_int(H), c_int(N), c_int(P), _stream()))
         # d(cum_t) = dy_t.(y_t - D x_t) - x_t.dx_t ;  a_k = dt_k A enters every cum_t with t >= k
         dB, dC = (_empty(Bsz, T, 1, N, dtype=torch.bfloat16, device=dev) for _ in range(2))
         ddt = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
         dA = _empty(H, dtype=torch.float32, device=dev)
         dD = _empty(H, dtype=torch.float32, device=dev) if ctx.has_D else None
         scratch = _empty(3 * Bsz * nc * H, dtype=torch.float32, device=dev)
-        _check(lib.nsa_ssd_finish(_p(dBh), _p(dCh), _p(q), _p(k), _p(rdx), _p(dt), _p(A), _p(scratch), _p(dB), _p(dC), _p(ddt),
+        _check(lib.nsa_ssd_finish(_p(dB_part), _p(dC_part), _p(q), _p(k), _p(rdx), _p(dt), _p(A), _p(scratch), _p(dB), _p(dC), _p(ddt),
                                   _p(dA), _p(dD), c_int(Bsz), c_int(T), c_int(H), _stream()))
         return dx, ddt, dA, dB, dC, dD
 
