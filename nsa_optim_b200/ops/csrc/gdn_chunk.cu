@@ -45,10 +45,11 @@ struct PrepParams {
   float scale;
 };
 
-// One CTA of eight warps per (chunk, head).  Two CTAs share an SM for values up to 192 wide; at 256 one needs 122 KB and runs alone,
-// and what bounds the kernel there is its chain of phases, not the memory traffic of q, k, v, u, w (2 KB per token and
-// head: 282 us at 16384 tokens x 16 heads, 87 us of it at the copy rate).  The triangular inverse is the longest
-// dependent phase and runs as two 32-column substitutions side by side, joined by two 32 x 32 products over all threads.
+// One CTA of eight warps per (chunk, head).  What bounds it is its chain of phases, not the memory traffic of q, k, v, u, w (2 KB
+// per token and head, 87 us at the copy rate for 16384 tokens x 16 heads), so two CTAs have to share an SM: the operands
+// of the last products take the places of q and A, which are through by then (values 256 wide: 101 KB; with tiles of their
+// own, 122 KB and one CTA per SM, 283 us; now 198).  The triangular inverse is the longest dependent phase and runs as
+// two 32-column substitutions side by side, joined by two 32 x 32 products over all threads.
 __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const int V = p.V, PV = V + 8;
@@ -56,9 +57,9 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
   bf16* sV = sK + 2 * CH * PK;
   float* As = reinterpret_cast<float*>(sV + CH * PV);      // [64][PX]
   float* Xs = As + CH * PX;
-  bf16* sTu = reinterpret_cast<bf16*>(Xs + CH * PX);
-  bf16* sTw = sTu + CH * PC;
-  float* gs = reinterpret_cast<float*>(sTw + CH * PC);
+  float* gs = Xs + CH * PX;
+  bf16* sTu = sK + CH * PK;                                // over q once q k^T is done
+  bf16* sTw = reinterpret_cast<bf16*>(As);                 // over A once its inverse is known
   float* bs = gs + CH;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bh = blockIdx.x, h = bh % p.H, b = bh / p.H, c = blockIdx.z * gridDim.y + blockIdx.y;   // see chunk_grid
@@ -233,6 +234,7 @@ constexpr int TILE = 128 * 128;
 constexpr int POST_STAGE = 4 * TILE;
 constexpr int PF = KD + 4;                                                 // pitch of the fp32 [64][128] tiles
 constexpr int POST_SMEM = 2 * POST_STAGE + 2 * CH * PK * 2 + CH * PX * 4 + CH * PC * 2 + (2 + 16) * CH * 4 + 64 + 1024;
+static_assert(PC <= PK && CH * PC * 2 <= CH * PX * 4, "gdn prep: operand tiles");
 static_assert(4 * CH * PX * 4 + CH * PK * 2 + 3 * CH * PC * 2 <= 2 * POST_STAGE, "gdn post: tail tiles");
 static_assert(2 * CH * PF * 4 <= 4 * CH * PX * 4, "gdn post: result tiles");
 
@@ -699,7 +701,7 @@ extern "C" int nsa_gdn_prep(const void* q, const void* k, const void* v, const f
   if (K != KD || V % 64 || V > 512) return nsa::fail(NSA_ERR_SHAPE, "gdn: key width must be 128, value width a multiple of 64 up to 512");
   const int NC = (T + CH - 1) / CH;
   PrepParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, g, beta, (bf16*)w, (bf16*)u, (bf16*)qk, X, gc, T, H, NC, V, scale};
-  const int smem = 2 * CH * PK * 2 + CH * (V + 8) * 2 + 2 * CH * PX * 4 + 2 * CH * PC * 2 + 2 * CH * 4;
+  const int smem = 2 * CH * PK * 2 + CH * (V + 8) * 2 + 2 * CH * PX * 4 + 2 * CH * 4;
   cudaError_t e = cudaFuncSetAttribute(gdn_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn prep smem attribute");
   gdn_prep_kernel<<<chunk_grid(B * H, NC), 256, smem, st>>>(p);
