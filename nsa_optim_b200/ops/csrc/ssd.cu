@@ -249,23 +249,28 @@ ssd_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_c
 // is loaded and computed once per run of one chunk ("segment"), and the next items' tiles are in flight meanwhile.
 // ---------------------------------------------------------------------------------------
 struct Items {
-  int first, end, H, nc;
-  __device__ Items(const SsdParams& p) : H(p.H), nc(p.nc) {
-    const int total = p.B * p.nc * p.H;
-    first = blockIdx.x * p.quota;
-    end = min(first + p.quota, total);
+  int n, h, t0, b, H, rows;            // items of the run; head, first token and sequence of the current one; padded length
+  __device__ explicit Items(const SsdParams& p) : H(p.H), rows(p.nc * L) {
+    const int total = p.B * p.nc * p.H, first = blockIdx.x * p.quota;
+    n = min(p.quota, total - first);
+    h = first % H;
+    t0 = first / H % p.nc * L;
+    b = first / H / p.nc;
   }
-  __device__ int head(int it) const { return it % H; }
-  __device__ int chunk(int it) const { return (it / H) % nc; }
-  __device__ int batch(int it) const { return it / H / nc; }
-  __device__ bool opens(int it) const { return it == first || it % H == 0; }              // first item of a segment
-  __device__ bool closes(int it) const { return it + 1 == end || (it + 1) % H == 0; }     // last one
+  __device__ void next() {
+    if (++h < H) return;
+    h = 0;
+    t0 += L;
+    if (t0 == rows) { t0 = 0; ++b; }
+  }
+  __device__ bool opens(int k) const { return k == 0 || h == 0; }              // first item of a segment
+  __device__ bool closes(int k) const { return k + 1 == n || h + 1 == H; }     // last one
 };
 
 // dt of four neighbouring rows of the item's chunk, for chunk_scan_warp
-__device__ __forceinline__ float4 load_dt4(const SsdParams& p, const Items& items, int it) {
-  const int t = items.chunk(it) * L + 4 * (threadIdx.x & 31), h = items.head(it);
-  const float* src = p.dt + (static_cast<long>(items.batch(it)) * p.T + t) * p.H + h;
+__device__ __forceinline__ float4 load_dt4(const SsdParams& p, const Items& at) {
+  const int t = at.t0 + 4 * (threadIdx.x & 31);
+  const float* src = p.dt + (static_cast<long>(at.b) * p.T + t) * p.H + at.h;
   return make_float4(t < p.T ? src[0] : 0.f, t + 1 < p.T ? src[p.H] : 0.f, t + 2 < p.T ? src[2 * p.H] : 0.f,
                      t + 3 < p.T ? src[3 * p.H] : 0.f);
 }
@@ -335,7 +340,6 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
-  const Items items(p);
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int i = 0; i < OUT_ST; ++i) tc5::mbar_init(full + i, 1);
@@ -356,7 +360,6 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const uint32_t cS = 0, cP = 128, cYi = 256, cYo = 384;     // the last three: 64 columns for even and odd items each
-  const int n = items.end - items.first;
   if (warp == 16) {
     constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);
     constexpr uint32_t id_y = tc5::make_idesc_bf16(128, PD, 0, 1);
@@ -364,49 +367,48 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
     auto wait = [&](uint64_t* bar, int phase, int code) {
       return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
     };
-    auto load = [&](int k) {
-      const int it = items.first + k, s = k % OUT_ST;
+    Items cur(p), ahead(p), behind(p);                 // the item of a step, the next to be loaded and scanned, the next to be stored
+    const int n = cur.n, item0 = blockIdx.x * p.quota;
+    auto load = [&](int k) {                           // item k, which is `ahead`
+      const int s = k % OUT_ST;
       uint8_t* st = stages + s * 2 * BOXB;
       tc5::mbar_expect_tx(full + s, 2 * BOXB);
-      tc5::tma_load_4d(st, &tm_x, full + s, 0, items.head(it), items.chunk(it) * L, items.batch(it));
-      tc5::tma_load_2d(st + BOXB, &tm_h, full + s, 0, it * NS);
+      tc5::tma_load_4d(st, &tm_x, full + s, 0, ahead.h, ahead.t0, ahead.b);
+      tc5::tma_load_2d(st + BOXB, &tm_h, full + s, 0, (item0 + k) * NS);
     };
-    auto load_bc = [&](int it) {
-      const int t0 = items.chunk(it) * L, b = items.batch(it);
+    auto load_bc = [&]() {                             // of the chunk of `cur`
       tc5::mbar_expect_tx(cb, 4 * BOXB);
-      tc5::tma_load_3d(sC, &tm_c, cb, 0, t0, b);
-      tc5::tma_load_3d(sC + BOXB, &tm_c, cb, 64, t0, b);
-      tc5::tma_load_3d(sB, &tm_b, cb, 0, t0, b);
-      tc5::tma_load_3d(sB + BOXB, &tm_b, cb, 64, t0, b);
+      tc5::tma_load_3d(sC, &tm_c, cb, 0, cur.t0, cur.b);
+      tc5::tma_load_3d(sC + BOXB, &tm_c, cb, 64, cur.t0, cur.b);
+      tc5::tma_load_3d(sB, &tm_b, cb, 0, cur.t0, cur.b);
+      tc5::tma_load_3d(sB + BOXB, &tm_b, cb, 64, cur.t0, cur.b);
     };
-    auto store = [&](int k) {                          // rows past T are clipped by the copy engine
-      const int it = items.first + k;
-      tc5::tma_store_4d(&tm_y, stages + (k % OUT_ST) * 2 * BOXB, 0, items.head(it), items.chunk(it) * L, items.batch(it));
+    auto store = [&](int k) {                          // item k, which is `behind`; rows past T are clipped by the copy engine
+      tc5::tma_store_4d(&tm_y, stages + (k % OUT_ST) * 2 * BOXB, 0, behind.h, behind.t0, behind.b);
       tc5::tma_store_commit();
     };
-    auto scan_item = [&](int k, float4 dt) {
+    auto scan_item = [&](int k, float4 dt, float a) {
       float* at = scan + (k & 1) * (2 * L + 192);
-      chunk_scan_warp<true>(dt, p.A[items.head(items.first + k)], at, at + L, at + 2 * L);
+      chunk_scan_warp<true>(dt, a, at, at + L, at + 2 * L);
       arrive_warp(scanned + (k & 1));
     };
-    if (lead) {
-      load_bc(items.first);
-      load(0);
-      if (n > 1) load(1);
+    if (lead) load_bc();
+    for (int k = 0; k < 2 && k < n; ++k, ahead.next()) {
+      if (lead) load(k);
+      scan_item(k, load_dt4(p, ahead), p.A[ahead.h]);
     }
-    scan_item(0, load_dt4(p, items, items.first));
-    if (n > 1) scan_item(1, load_dt4(p, items, items.first + 1));
     const uint64_t cc = tc5::desc_kmajor(tc5::smem_u32(sC)), bb = tc5::desc_kmajor(tc5::smem_u32(sB));
     bool ok = true;
     int seg = 0;
-    for (int k = 0; k < n; ++k) {
+    for (int k = 0; k < n; ++k, cur.next()) {
       const int buf = k & 1, s = k % OUT_ST;
       float4 dt_next = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (k + 2 < n) dt_next = load_dt4(p, items, items.first + k + 2);
-      if (items.opens(items.first + k)) {
+      float a_next = 0.f;
+      if (k + 2 < n) { dt_next = load_dt4(p, ahead); a_next = p.A[ahead.h]; }
+      if (cur.opens(k)) {
         if (k > 0) {                                   // C is read by the products of item k - 1
           if (!(ok = wait(done + (buf ^ 1), (k - 1) >> 1, STATUS_TIMEOUT_TMEM_FULL))) break;
-          if (lead) load_bc(items.first + k);
+          if (lead) load_bc();
           if (!(ok = wait(sread, seg - 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
         }
         if (!(ok = wait(cb, seg, STATUS_TIMEOUT_SMEM_FULL))) break;
@@ -441,16 +443,18 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
         tc5::mma_commit(done + buf);
       }
       __syncwarp();
-      if (k + 2 < n) scan_item(k + 2, dt_next);        // this item's sums have been read
+      if (k + 2 < n) scan_item(k + 2, dt_next, a_next);        // this item's sums have been read
       if (k > 0) {
         if (!(ok = wait(left + (buf ^ 1), (k - 1) >> 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
         tc5::fence_after_sync();
         if (lead) store(k - 1);
+        behind.next();
       }
       if (lead && k + 2 < n) {                         // over the stage of item k - 2, stored one step ago
         tc5::tma_store_wait_read<1>();
         load(k + 2);
       }
+      ahead.next();
       __syncwarp();
     }
     if (ok && wait(left + ((n - 1) & 1), (n - 1) >> 1, STATUS_TIMEOUT_TMEM_EMPTY)) {
@@ -468,14 +472,17 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
       return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
     };
     float s[32];                                       // C_i . B_j of the segment: row i = r, columns j = 32 grp ..
-    float e_open = 0.f;                                // exp(cum) of the item whose rows are still open
+    float e_open = 0.f, dsk_open = 0.f;                // exp(cum) and skip weight of the item whose rows are still open
+    Items cur(p);
+    const int n = cur.n;
     bool ok = true;
     int seg = 0;
-    for (int k = 0; k <= n; ++k) {
-      float e = 0.f;
+    for (int k = 0; k <= n; ++k, cur.next()) {
+      float e = 0.f, dsk = 0.f;
       if (k < n) {
         const int buf = k & 1;
-        if (items.opens(items.first + k)) {
+        if (p.Dskip) dsk = p.Dskip[cur.h];             // in flight until the item's rows are finished
+        if (cur.opens(k)) {
           if (!(ok = wait(ms, seg, STATUS_TIMEOUT_TMEM_FULL))) break;
           tc5::fence_after_sync();
           tld32(lanes + cS + grp * 32, s);
@@ -520,7 +527,6 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
         const int q = k - 1, buf = q & 1;
         if (!(ok = wait(full + q % OUT_ST, q / OUT_ST, STATUS_TIMEOUT_SMEM_FULL) && wait(done + buf, q >> 1, STATUS_TIMEOUT_TMEM_FULL))) break;
         tc5::fence_after_sync();
-        const float dsk = p.Dskip ? p.Dskip[items.head(items.first + q)] : 0.f;
         uint8_t* sX = stages + (q % OUT_ST) * 2 * BOXB;
         float xf[16], yo[16], yi[16];
         ld_row(sX, r, grp * 16, xf);
@@ -529,7 +535,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
         uint32_t o[8];
 #pragma unroll
         for (int i = 0; i < 16; i += 2)
-          o[i / 2] = tc5::pack_bf16(yo[i] + e_open * yi[i] + dsk * xf[i], yo[i + 1] + e_open * yi[i + 1] + dsk * xf[i + 1]);
+          o[i / 2] = tc5::pack_bf16(yo[i] + e_open * yi[i] + dsk_open * xf[i], yo[i + 1] + e_open * yi[i + 1] + dsk_open * xf[i + 1]);
         uint8_t* base = sX + r * 128;                  // the thread's own piece of x, which the products have read
 #pragma unroll
         for (int j = 0; j < 2; ++j)
@@ -539,6 +545,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
         arrive_warp(left + buf);
       }
       e_open = e;
+      dsk_open = dsk;
     }
   }
   tc5::fence_before_sync();
@@ -569,21 +576,18 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sC = smem;                  // 2 boxes
   uint8_t* sB = sC + 2 * BOXB;         // 2 boxes
-  uint8_t* sDS = sB + 2 * BOXB;        // 2 boxes: dS^T [j][i]; row sums once the products have read it
+  uint8_t* sDS = sB + 2 * BOXB;        // 2 boxes: dS^T [j][i]
   uint8_t* stages = sDS + 2 * BOXB;    // 2 x (x, dy, H [n][p], dHn [n][p])
   float* cum = reinterpret_cast<float*>(stages + 8 * BOXB);
   float* dts = cum + L;
   float* colf = dts + L;
   uint64_t* bars = reinterpret_cast<uint64_t*>(colf + 192);
   uint64_t *full = bars, *cb = bars + 2, *ms = bars + 3, *sread = bars + 4, *scanned = bars + 5;
-  uint64_t *m0 = bars + 6, *m1 = bars + 7, *ready = bars + 8, *m2 = bars + 9, *left = bars + 10;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  uint64_t *m0 = bars + 6, *m1 = bars + 7, *ready = bars + 8, *m2 = bars + 9, *m3 = bars + 10, *sums = bars + 11, *left = bars + 12;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* part = reinterpret_cast<float*>(sDS);         // [16][128]
 
   const int warp = threadIdx.x >> 5;
-  const Items items(p);
-  const int n = items.end - items.first;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     tc5::mbar_init(full, 1);
@@ -596,6 +600,8 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
     tc5::mbar_init(m1, 1);
     tc5::mbar_init(ready, 16);
     tc5::mbar_init(m2, 1);
+    tc5::mbar_init(m3, 1);
+    tc5::mbar_init(sums, 1);
     tc5::mbar_init(left, 16);
     tc5::fence_barrier_init();
   }
@@ -616,120 +622,156 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
     constexpr uint32_t id_kn128 = tc5::make_idesc_bf16(128, NS, 0, 1);  // K-major A, MN-major B -> [128 x 128]
     constexpr uint32_t id_tn128 = tc5::make_idesc_bf16(128, NS, 1, 1);  // MN-major A, MN-major B -> [128 x 128]
     const bool lead = tc5::elect_one();                // converged warp, elected lane issues (see ssd_chunk_state_kernel)
-    auto load = [&](int k) {
-      const int it = items.first + k, h = items.head(it), t0 = items.chunk(it) * L, b = items.batch(it);
+    Items cur(p), ahead(p), behind(p);                 // the item of a step, the next to be loaded and scanned, the next to be stored
+    const int n = cur.n, item0 = blockIdx.x * p.quota;
+    auto load = [&](int k) {                           // item k, which is `ahead`
       uint8_t* st = stages + (k & 1) * 4 * BOXB;
       uint64_t* bar = full + (k & 1);
       tc5::mbar_expect_tx(bar, 4 * BOXB);
-      tc5::tma_load_4d(st, &tm_x, bar, 0, h, t0, b);
-      tc5::tma_load_4d(st + BOXB, &tm_dy, bar, 0, h, t0, b);
-      tc5::tma_load_2d(st + 2 * BOXB, &tm_h, bar, 0, it * NS);
-      tc5::tma_load_2d(st + 3 * BOXB, &tm_dh, bar, 0, it * NS);
+      tc5::tma_load_4d(st, &tm_x, bar, 0, ahead.h, ahead.t0, ahead.b);
+      tc5::tma_load_4d(st + BOXB, &tm_dy, bar, 0, ahead.h, ahead.t0, ahead.b);
+      tc5::tma_load_2d(st + 2 * BOXB, &tm_h, bar, 0, (item0 + k) * NS);
+      tc5::tma_load_2d(st + 3 * BOXB, &tm_dh, bar, 0, (item0 + k) * NS);
     };
-    auto load_bc = [&](int it) {
-      const int t0 = items.chunk(it) * L, b = items.batch(it);
-      tc5::mbar_expect_tx(cb, 4 * BOXB);
-      tc5::tma_load_3d(sC, &tm_c, cb, 0, t0, b);
-      tc5::tma_load_3d(sC + BOXB, &tm_c, cb, 64, t0, b);
-      tc5::tma_load_3d(sB, &tm_b, cb, 0, t0, b);
-      tc5::tma_load_3d(sB + BOXB, &tm_b, cb, 64, t0, b);
-    };
-    auto store = [&](int k) {                          // dx from the place of x; rows past T are clipped by the copy engine
-      const int it = items.first + k;
-      tc5::tma_store_4d(&tm_dx, stages + (k & 1) * 4 * BOXB, 0, items.head(it), items.chunk(it) * L, items.batch(it));
+    auto store = [&](int k) {                          // dx of item k, `behind`, from the place of x; rows past T are clipped by the copy engine
+      tc5::tma_store_4d(&tm_dx, stages + (k & 1) * 4 * BOXB, 0, behind.h, behind.t0, behind.b);
       tc5::tma_store_commit();
       tc5::tma_store_wait_read<0>();                   // the next item but one goes there
     };
-    auto scan_item = [&](int k, float4 dt) {
-      chunk_scan_warp<false>(dt, p.A[items.head(items.first + k)], cum, dts, colf);
-      arrive_warp(scanned);
-    };
-    if (lead) {
-      load_bc(items.first);
-      load(0);
-    }
-    scan_item(0, load_dt4(p, items, items.first));
     const uint64_t ck = tc5::desc_kmajor(tc5::smem_u32(sC)), bk = tc5::desc_kmajor(tc5::smem_u32(sB));
     const uint64_t cm = tc5::desc_mnmajor(tc5::smem_u32(sC), BOXB), bm = tc5::desc_mnmajor(tc5::smem_u32(sB), BOXB);
     const uint64_t dsm = tc5::desc_mnmajor(tc5::smem_u32(sDS), BOXB);
     auto kblock = [](int kk) { return static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4); };
+    auto kcols = [](int kk) { return static_cast<uint64_t>((kk * 32) >> 4); };
     auto krow = [](int kk) { return static_cast<uint64_t>((kk * 2048) >> 4); };
-    bool ok = true;
+    auto box = [&](int k, int i) { return tc5::smem_u32(stages + ((k & 1) * 4 + i) * BOXB); };      // x, dy, H, dHn of item k
     int seg = 0;
-    for (int k = 0; k < n; ++k) {
-      const int s = k & 1;
-      const uint8_t* st = stages + s * 4 * BOXB;
-      const bool opens = items.opens(items.first + k);
-      if (opens) {
-        if (k > 0) {                                   // every product and every reader of the segment before is through
-          if (!(ok = wait(left, k - 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
-          if (lead) load_bc(items.first + k);
-        }
-        if (!(ok = wait(cb, seg, STATUS_TIMEOUT_SMEM_FULL))) break;
-        tc5::fence_after_sync();
-        if (lead) {
-#pragma unroll
-          for (int kk = 0; kk < NS / 16; ++kk)         // S^T = B C^T
-            tc5::mma_ss(tmem + cR, bk + kblock(kk), ck + kblock(kk), id_s, kk > 0 ? 1u : 0u);
-          tc5::mma_commit(ms);
-        }
-        __syncwarp();
-        if (!(ok = wait(sread, seg, STATUS_TIMEOUT_TMEM_EMPTY))) break;
-        tc5::fence_after_sync();
-        ++seg;
+    auto open_segment = [&]() {                        // C and B of the chunk of `cur`, S^T = B C^T
+      if (lead) {
+        tc5::mbar_expect_tx(cb, 4 * BOXB);
+        tc5::tma_load_3d(sC, &tm_c, cb, 0, cur.t0, cur.b);
+        tc5::tma_load_3d(sC + BOXB, &tm_c, cb, 64, cur.t0, cur.b);
+        tc5::tma_load_3d(sB, &tm_b, cb, 0, cur.t0, cur.b);
+        tc5::tma_load_3d(sB + BOXB, &tm_b, cb, 64, cur.t0, cur.b);
       }
-      if (!(ok = wait(full + s, k >> 1, STATUS_TIMEOUT_SMEM_FULL))) break;
+      __syncwarp();
+      if (!wait(cb, seg, STATUS_TIMEOUT_SMEM_FULL)) return false;
       tc5::fence_after_sync();
-      const uint64_t xk = tc5::desc_kmajor(tc5::smem_u32(st)), dyk = tc5::desc_kmajor(tc5::smem_u32(st + BOXB));
-      const uint64_t dym = tc5::desc_mnmajor(tc5::smem_u32(st + BOXB), BOXB);
-      const uint64_t hk = tc5::desc_kmajor(tc5::smem_u32(st + 2 * BOXB)), hm = tc5::desc_mnmajor(tc5::smem_u32(st + 2 * BOXB), BOXB);
-      const uint64_t dhk = tc5::desc_kmajor(tc5::smem_u32(st + 3 * BOXB)), dhm = tc5::desc_mnmajor(tc5::smem_u32(st + 3 * BOXB), BOXB);
-      if (lead) {                                      // behind the products of the item before, which read these columns as operands
+      if (lead) {
 #pragma unroll
-        for (int kk = 0; kk < PD / 16; ++kk)           // R^T = x dy^T
-          tc5::mma_ss(tmem + cR, xk + static_cast<uint64_t>((kk * 32) >> 4), dyk + static_cast<uint64_t>((kk * 32) >> 4), id_s, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < NS / 16; ++kk) tc5::mma_ss(tmem + cR, bk + kblock(kk), ck + kblock(kk), id_s, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(ms);
+      }
+      __syncwarp();
+      if (!wait(sread, seg, STATUS_TIMEOUT_TMEM_EMPTY)) return false;
+      tc5::fence_after_sync();
+      ++seg;
+      return true;
+    };
+    auto scores = [&](int k) {                         // R^T = x dy^T, over P^T and dS^T of the item before
+      if (lead) {
+        const uint64_t xk = tc5::desc_kmajor(box(k, 0)), dyk = tc5::desc_kmajor(box(k, 1));
 #pragma unroll
-        for (int kk = 0; kk < NS / 16; ++kk)           // C H
-          tc5::mma_ss(tmem + cY, ck + kblock(kk), hm + krow(kk), id_kn64, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < PD / 16; ++kk) tc5::mma_ss(tmem + cR, xk + kcols(kk), dyk + kcols(kk), id_s, kk > 0 ? 1u : 0u);
         tc5::mma_commit(m0);
       }
       __syncwarp();
-      if (k > 0 && !opens && !(ok = wait(left, k - 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
-      tc5::fence_after_sync();
+    };
+    auto state_rows = [&](int k) {                     // C H, over the scaled rows of the item before
       if (lead) {
+        const uint64_t hm = tc5::desc_mnmajor(box(k, 2), BOXB);
 #pragma unroll
-        for (int kk = 0; kk < NS / 16; ++kk)           // B dHn
+        for (int kk = 0; kk < NS / 16; ++kk) tc5::mma_ss(tmem + cY, ck + kblock(kk), hm + krow(kk), id_kn64, kk > 0 ? 1u : 0u);
+      }
+      __syncwarp();
+    };
+    if (lead) load(0);
+    chunk_scan_warp<false>(load_dt4(p, ahead), p.A[ahead.h], cum, dts, colf);
+    arrive_warp(scanned);
+    ahead.next();
+    // A step issues the rest of item k and the first products of item k + 1 between them, so that the scores of k + 1 are
+    // there when the warps have finished the rows of k, and the sums over heads run behind their work.
+    bool ok = open_segment() && wait(full, 0, STATUS_TIMEOUT_SMEM_FULL);
+    if (ok) {
+      tc5::fence_after_sync();
+      scores(0);
+      state_rows(0);
+    }
+    for (int k = 0; k < n && ok; ++k) {
+      const bool opens = cur.opens(k), closes = cur.closes(k), more = k + 1 < n;
+      if (k > 0) {
+        if (!(ok = wait(left, k - 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+        tc5::fence_after_sync();
+      }
+      if (lead) {
+        const uint64_t dhm = tc5::desc_mnmajor(box(k, 3), BOXB);
+#pragma unroll
+        for (int kk = 0; kk < NS / 16; ++kk)           // B dHn, over dx of the item before
           tc5::mma_ss(tmem + cX, bk + kblock(kk), dhm + krow(kk), id_kn64, kk > 0 ? 1u : 0u);
         tc5::mma_commit(m1);
         if (k > 0) store(k - 1);
-        if (k + 1 < n) load(k + 1);
       }
+      if (k > 0) behind.next();
       __syncwarp();
+      if (more) {                                      // over item k - 1, whose last products are complete when these are
+        if (!(ok = wait(m1, k, STATUS_TIMEOUT_TMEM_FULL))) break;
+        if (lead) load(k + 1);
+        __syncwarp();
+      }
       float4 dt_next = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (k + 1 < n) dt_next = load_dt4(p, items, items.first + k + 1);
+      float a_next = 0.f;
+      if (more) { dt_next = load_dt4(p, ahead); a_next = p.A[ahead.h]; }
+      ahead.next();
       if (!(ok = wait(ready, k, STATUS_TIMEOUT_TMEM_EMPTY))) break;
       tc5::fence_after_sync();
+      const uint32_t sum = opens ? 0u : 1u;
       if (lead) {
-        const uint32_t sum = opens ? 0u : 1u;
+        const uint64_t dym = tc5::desc_mnmajor(box(k, 1), BOXB);
 #pragma unroll
         for (int kk = 0; kk < L / 16; ++kk)            // dx += P^T dy
           tc5::mma_ts(tmem + cX, tmem + cR + 16 * kk, dym + krow(kk), id_kn64, 1u);
-#pragma unroll
-        for (int kk = 0; kk < L / 16; ++kk)            // dC += dS B
-          tc5::mma_ss(tmem + cDC, dsm + krow(kk), bm + krow(kk), id_tn128, kk > 0 ? 1u : sum);
+        tc5::mma_commit(m2);
 #pragma unroll
         for (int kk = 0; kk < L / 16; ++kk)            // dB += dS^T C
           tc5::mma_ts(tmem + cDB, tmem + cR + 16 * kk + 8, cm + krow(kk), id_kn128, kk > 0 ? 1u : sum);
-#pragma unroll
-        for (int kk = 0; kk < PD / 16; ++kk)           // dC += (exp(cum) dy) H^T
-          tc5::mma_ts(tmem + cDC, tmem + cY + 16 * kk, hk + static_cast<uint64_t>((kk * 32) >> 4), id_s, 1u);
-#pragma unroll
-        for (int kk = 0; kk < PD / 16; ++kk)           // dB += (s x) dHn^T
-          tc5::mma_ts(tmem + cDB, tmem + cY + 16 * kk + 8, dhk + static_cast<uint64_t>((kk * 32) >> 4), id_s, 1u);
-        tc5::mma_commit(m2);
       }
       __syncwarp();
-      if (k + 1 < n) scan_item(k + 1, dt_next);        // this item's sums have been read
+      const bool same = more && !closes;               // item k + 1 is of the same chunk
+      if (same) {
+        if (!(ok = wait(full + ((k + 1) & 1), (k + 1) >> 1, STATUS_TIMEOUT_SMEM_FULL))) break;
+        tc5::fence_after_sync();
+        scores(k + 1);
+      }
+      if (lead) {
+        const uint64_t hk = tc5::desc_kmajor(box(k, 2)), dhk = tc5::desc_kmajor(box(k, 3));
+#pragma unroll
+        for (int kk = 0; kk < L / 16; ++kk)            // dC += dS B
+          tc5::mma_ss(tmem + cDC, dsm + krow(kk), bm + krow(kk), id_tn128, kk > 0 ? 1u : sum);
+        tc5::mma_commit(m3);
+#pragma unroll
+        for (int kk = 0; kk < PD / 16; ++kk)           // dC += (exp(cum) dy) H^T
+          tc5::mma_ts(tmem + cDC, tmem + cY + 16 * kk, hk + kcols(kk), id_s, 1u);
+#pragma unroll
+        for (int kk = 0; kk < PD / 16; ++kk)           // dB += (s x) dHn^T
+          tc5::mma_ts(tmem + cDB, tmem + cY + 16 * kk + 8, dhk + kcols(kk), id_s, 1u);
+        if (closes) tc5::mma_commit(sums);
+      }
+      __syncwarp();
+      if (more) {                                      // this item's sums of step sizes have been read
+        chunk_scan_warp<false>(dt_next, a_next, cum, dts, colf);
+        arrive_warp(scanned);
+      }
+      cur.next();
+      if (same) {
+        state_rows(k + 1);
+      } else if (more) {                               // every product and every reader of the segment is through: C and B may go
+        ok = wait(left, k, STATUS_TIMEOUT_TMEM_EMPTY) && open_segment() &&
+             wait(full + ((k + 1) & 1), (k + 1) >> 1, STATUS_TIMEOUT_SMEM_FULL);
+        if (!ok) break;
+        tc5::fence_after_sync();
+        scores(k + 1);
+        state_rows(k + 1);
+      }
     }
     if (ok && wait(left, n - 1, STATUS_TIMEOUT_TMEM_EMPTY)) {
       if (lead) store(n - 1);
@@ -746,11 +788,14 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
     float s[32];                                       // B_j . C_i of the segment: row j = r, columns i = 32 grp ..
     bool ok = true;
     int seg = 0;
-    for (int k = 0; k < n; ++k) {
-      const int it = items.first + k, h = items.head(it), b = items.batch(it), t = items.chunk(it) * L + r;
+    Items cur(p);
+    const int n = cur.n;
+    for (int k = 0; k < n; ++k, cur.next()) {
+      const int t = cur.t0 + r;
+      const float dsk = p.Dskip ? p.Dskip[cur.h] : 0.f;          // in flight until the item's last phase
       uint8_t* sX = stages + (k & 1) * 4 * BOXB;
-      const uint8_t* sDY = sX + BOXB;
-      if (items.opens(it)) {
+      uint8_t* sDY = sX + BOXB;
+      if (cur.opens(k)) {
         ok = ok && wait(ms, seg, STATUS_TIMEOUT_TMEM_FULL);
         if (ok) {
           tc5::fence_after_sync();
@@ -786,7 +831,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
           tc5::tmem_st_x8(lanes + cR + grp * 32 + hf * 16, pk);
           tc5::tmem_st_x8(lanes + cR + grp * 32 + hf * 16 + 8, ds);
           tc5::tmem_st_wait();
-          if (hf == 0) ok = wait(m1, k, STATUS_TIMEOUT_TMEM_FULL);      // row sums of the item before have been read
+          if (hf == 0 && k > 0) ok = wait(m3, k - 1, STATUS_TIMEOUT_TMEM_FULL);     // dS of the item before has been read
           const int c0 = grp * 32 + hf * 16, j0 = (c0 & 63) >> 3;
           uint8_t* base = sDS + (c0 >> 6) * BOXB + r * 128;
 #pragma unroll
@@ -829,9 +874,10 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
           tc5::tmem_st_x16(lanes + cR + grp * 32, z);
           tc5::tmem_st_x16(lanes + cR + grp * 32 + 16, z);
           tc5::tmem_st_wait();
-          ok = wait(m1, k, STATUS_TIMEOUT_TMEM_FULL);
+          if (k > 0) ok = wait(m3, k - 1, STATUS_TIMEOUT_TMEM_FULL);
           st_row32(sDS, r, grp * 32, z);
         }
+        ok = ok && wait(m1, k, STATUS_TIMEOUT_TMEM_FULL);
         if (ok) {
           tc5::fence_after_sync();
           // dx starts from s_j B_j dHn; rows of dy and x, scaled, take the place of C H.  (The sources of a tcgen05.st must
@@ -861,13 +907,11 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
         }
       }
       ok = ok && wait(m2, k, STATUS_TIMEOUT_TMEM_FULL);
-      const long tok = static_cast<long>(b) * p.T + t;
       if (ok) {
         tc5::fence_after_sync();
         float kacc = 0.f, racc = 0.f;
         float g[16], xf[16], df[16];
         tld16(lanes + cX + grp * 16, g);
-        const float dsk = p.Dskip ? p.Dskip[h] : 0.f;
         ld_row(sX, r, grp * 16, xf);
         ld_row(sDY, r, grp * 16, df);
         uint32_t o[8];
@@ -881,31 +925,39 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
 #pragma unroll
         for (int j = 0; j < 2; ++j)
           *reinterpret_cast<uint4*>(base + (((grp * 2 + j) ^ (r & 7)) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-        part[grp * L + r] = kacc;
-        part[(4 + grp) * L + r] = racc;
-        part[(8 + grp) * L + r] = q_inter;
-        part[(12 + quad) * L + grp * 32 + lane] = q_intra;
+        // the sums of its row and column on their way to one: over its own piece of dy
+        *reinterpret_cast<float4*>(sDY + r * 128 + (((grp * 2) ^ (r & 7)) << 4)) = make_float4(kacc, racc, q_inter, q_intra);
       }
       if (compute_any(!ok)) { ok = false; break; }     // all sixteen warps leave together
-      if (t < p.T) {                                   // groups add up in a fixed order; group g finishes sum g
-        auto row_sum = [&](int i) { return (part[i * L + r] + part[(i + 1) * L + r]) + (part[(i + 2) * L + r] + part[(i + 3) * L + r]); };
-        if (grp == 0) p.k_out[tok * p.H + h] = row_sum(0);
-        else if (grp == 1) { if (p.r_out) p.r_out[tok * p.H + h] = row_sum(4); }
-        else if (grp == 2) p.q_out[tok * p.H + h] = row_sum(12) + e * row_sum(8);
+      const long tok = static_cast<long>(cur.b) * p.T + t;
+      if (t < p.T && grp < 3) {                        // the four pieces add up in a fixed order; group g finishes sum g
+        auto piece = [&](int row, int g) { return reinterpret_cast<const float*>(sDY + row * 128 + (((g * 2) ^ (row & 7)) << 4)); };
+        auto row_sum = [&](int i) { return (piece(r, 0)[i] + piece(r, 1)[i]) + (piece(r, 2)[i] + piece(r, 3)[i]); };
+        const long o = tok * p.H + cur.h;
+        if (grp == 0) p.k_out[o] = row_sum(0);
+        else if (grp == 1) { if (p.r_out) p.r_out[o] = row_sum(1); }
+        else p.q_out[o] = ((piece(lane, quad)[3] + piece(32 + lane, quad)[3]) + (piece(64 + lane, quad)[3] + piece(96 + lane, quad)[3])) +
+                          e * row_sum(2);
       }
-      if (items.closes(it)) {                          // the segment's sums over heads
-        const int chunk = it / p.H, slot = blockIdx.x - static_cast<int>(static_cast<long>(chunk) * p.H / p.quota);
-        const long o = (tok * p.slots + slot) * NS + grp * 32;
+      if (cur.closes(k)) {                             // the segment's sums over heads
+        ok = wait(sums, seg - 1, STATUS_TIMEOUT_TMEM_FULL);
+        if (ok) {
+          tc5::fence_after_sync();
+          const long chunk = static_cast<long>(cur.b) * p.nc + cur.t0 / L;
+          const int slot = blockIdx.x - static_cast<int>(chunk * p.H / p.quota);
+          const long o = (tok * p.slots + slot) * NS + grp * 32;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          float v[32];
-          tld32(lanes + (q ? cDC : cDB) + grp * 32, v);
-          float* dst = (q ? p.dC_part : p.dB_part) + o;
-          if (t < p.T)
+          for (int q = 0; q < 2; ++q) {
+            float v[32];
+            tld32(lanes + (q ? cDC : cDB) + grp * 32, v);
+            float* dst = (q ? p.dC_part : p.dB_part) + o;
+            if (t < p.T)
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+              for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+          }
         }
       }
+      if (!ok) continue;                               // the next item's vote ends the walk
       tc5::fence_proxy_async();
       tc5::fence_before_sync();
       arrive_warp(left);
