@@ -49,22 +49,6 @@ __device__ __forceinline__ void read_half(const uint8_t* tile, int row, int half
     }
   }
 }
-__device__ __forceinline__ void load_global(const bf16* src, uint32_t (&packed)[HC / 2]) {
-  const uint4* s4 = reinterpret_cast<const uint4*>(src);
-#pragma unroll
-  for (int j = 0; j < HC / 8; ++j) {
-    const uint4 v = s4[j];
-    packed[4 * j] = v.x; packed[4 * j + 1] = v.y; packed[4 * j + 2] = v.z; packed[4 * j + 3] = v.w;
-  }
-}
-__device__ __forceinline__ void unpack_half(const uint32_t (&packed)[HC / 2], float (&out)[HC]) {
-#pragma unroll
-  for (int j = 0; j < HC / 2; ++j) {
-    float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&packed[j]));
-    out[2 * j] = f.x;
-    out[2 * j + 1] = f.y;
-  }
-}
 __device__ __forceinline__ void tmem_ld_half(uint32_t taddr, float (&out)[HC]) {
   uint32_t a[HC];
   tc5::tmem_ld_x32(taddr, a);
@@ -85,7 +69,6 @@ __device__ __forceinline__ void pack_half(const float (&in)[HC], uint32_t (&pack
 }
 
 struct FwdParams {
-  const bf16* u;        // [BH, NC, 64, V]
   const float* gc;      // [BH, NC, 64]
   int store_states;     // also write v_new and S_all (the backward needs them)
   int NC, V, H;
@@ -93,172 +76,118 @@ struct FwdParams {
   KernelStatus* status;
 };
 
+// Roles of both kernels: warps 0..7 compute, warp 8 issues the products, warp 9 loads, the last one stores.  The chunk loop is one
+// dependent chain (product, accumulator rows, product, state rows), so everything that is not on it is kept off the
+// warps that are: a thread that also copies and issues costs its whole CTA 1400 of 3500 cycles a chunk at the barriers.
+constexpr int WARP_MMA = 8, WARP_LOAD = 9;
+// A chunk's tiles are asked for into L2 this many chunks ahead: two stages alone leave a load from memory one chunk's time,
+// and the chain then waits for it.  256 chunks x 64 CTAs, forward and backward: 472 and 526 us with one thread for copies,
+// stores and products, 455 and 597 with warps for each, 395 and 492 with the prefetch and operands released where their last
+// product is issued, 356 and 365 with u and do as tiles too (rows of their own per thread are 32 lines an instruction).
+constexpr int AHEAD = 6;
+__device__ __forceinline__ void arrive_warp(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) tc5::mbar_arrive(bar);
+}
+
 // stage: k-block kb of [w ; q] (2 x 16 KB), k (16 KB), [0 ; qk] (16 KB, first half zero)
 constexpr int FWD_STAGE = 8 * BOX;
-constexpr int FWD_TX = 7 * BOX;                                                       // bytes that arrive per chunk
-constexpr int FWD_SMEM = 2 * FWD_STAGE + 2 * BOX /*Sb*/ + 2 * BOX /*Vb, Vs*/ + BOX /*Ob*/ + 1024 + 128;
+constexpr int FWD_TX_A = 4 * BOX, FWD_TX_B = 3 * BOX;    // bytes that arrive per chunk: [w ; q], free after the first product, and the rest
+constexpr int FWD_SMEM = 2 * FWD_STAGE + 2 * BOX /*u*/ + 4 * BOX /*Sb*/ + 3 * BOX /*Vb, Vs*/ + 2 * BOX /*Ob*/ + 1024 + 256;
 
-__global__ void __launch_bounds__(256, 1)
-gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_q,
+__global__ void __launch_bounds__(352, 1)
+gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_qk,
                    const __grid_constant__ CUtensorMap tm_vn, const __grid_constant__ CUtensorMap tm_o,
                    const __grid_constant__ CUtensorMap tm_sa, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* Sb = smem + 2 * FWD_STAGE;           // [KD rows][64] bf16 state, B operand
-  uint8_t* Vb = Sb + 2 * BOX;                   // [64 rows][64] v_new
-  uint8_t* Vs = Vb + BOX;                       // [64 rows][64] sk v_new
-  uint8_t* Ob = Vs + BOX;                       // [64 rows][64] o on its way out
-  uint64_t* bars = reinterpret_cast<uint64_t*>(Ob + BOX);
-  uint64_t* full = bars;        // [2]
-  uint64_t* m1 = bars + 2;
-  uint64_t* m2 = bars + 3;
-  uint64_t* m3 = bars + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
+  uint8_t* Sb = smem + 2 * FWD_STAGE;           // 2 x [KD rows][64] bf16 state, B operand
+  uint8_t* Vb = Sb + 4 * BOX;                   // 2 x [64 rows][64] v_new
+  uint8_t* Ob = Vb + 2 * BOX;                   // 2 x [64 rows][64] o on its way out
+  uint8_t* Vs = Ob + 2 * BOX;                   // [64 rows][64] sk v_new
+  uint8_t* Us = Vs + BOX;                       // 2 x [64 rows][64] u
+  uint64_t* bars = reinterpret_cast<uint64_t*>(Us + 2 * BOX);
+  uint64_t *full_a = bars, *empty_a = bars + 2, *full_b = bars + 4, *empty_b = bars + 6;     // [2] each: the stages
+  uint64_t *full_u = bars + 8, *empty_u = bars + 10;                  // [2] each
+  uint64_t *m1 = bars + 12, *m2 = bars + 13, *m3 = bars + 14;         // products complete: D1, S, D2
+  uint64_t *sready = bars + 15, *scaled = bars + 16, *vready = bars + 17, *oready = bars + 18;   // rows written: Sb, S, Vb and Vs, Ob
+  uint64_t* freed = bars + 19;                  // stores of the chunk before have read their tiles
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int r = threadIdx.x & 127, half = threadIdx.x >> 7;   // TMEM lane / tile row, half of its columns
+  const int r = threadIdx.x & 127, half = (threadIdx.x >> 7) & 1;   // TMEM lane / tile row, half of its columns
   const int warp = threadIdx.x >> 5;
-  const bool boss = threadIdx.x == 0;
   const int vt = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
-  const int NC = p.NC, V = p.V;
+  const int NC = p.NC;
 
-  if (boss) {
+  if (threadIdx.x == 0) {
     *abort_flag = 0;
-    tc5::mbar_init(&full[0], 1);
-    tc5::mbar_init(&full[1], 1);
+    for (int i = 0; i < 10; ++i) tc5::mbar_init(bars + i, 1);
+    tc5::mbar_init(empty_u, 4);
+    tc5::mbar_init(empty_u + 1, 4);
     tc5::mbar_init(m1, 1);
     tc5::mbar_init(m2, 1);
     tc5::mbar_init(m3, 1);
+    tc5::mbar_init(sready, 8);
+    tc5::mbar_init(scaled, 8);
+    tc5::mbar_init(vready, 4);
+    tc5::mbar_init(oready, 4);
+    tc5::mbar_init(freed, 1);
     tc5::fence_barrier_init();
   }
   if (warp == 0) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
-  // S = 0: bf16 mirror in shared memory; the constant zero half of both [0 ; qk] operands
-  {
+  if (warp < 8) {
+    // S = 0: bf16 mirror in shared memory; the constant zero half of both [0 ; qk] operands
     uint32_t z[HC / 2];
 #pragma unroll
     for (int j = 0; j < HC / 2; ++j) z[j] = 0u;
     write_half(Sb, r, half, z);
     write_half(smem + (r >> 6) * FWD_STAGE + 6 * BOX, r & 63, half, z);
+    tc5::fence_proxy_async();
   }
-  tc5::fence_proxy_async();
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_off = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * HC;   // lanes and columns of this thread
   // TMEM columns: D1 = [w ; q] S [0, 64)   S [64, 128)   D2 = [0 ; qk] v_new [128, 192)
   const uint32_t cD1 = 0, cS = 64, cD2 = 128;
-  {
-    float z[HC];
-#pragma unroll
-    for (int j = 0; j < HC; ++j) z[j] = 0.f;
-    tmem_st_half(tmem + lane_off + cS, z);
-  }
-  tc5::fence_before_sync();
-  __syncthreads();
-  // Outputs leave as TMA stores from the swizzled tiles they are in anyway.  Thread 0 stores v_new and the
-  // state, thread 64 the output; each waits until its earlier store has read a tile before that tile is
-  // rewritten.  Chunk 0 enters with the zero state that Sb holds now.
-  if (boss && p.store_states) {
-    tc5::tma_store_2d(&tm_sa, Sb, vt * VT, bh * NC * KD);
-    tc5::tma_store_commit();
-  }
-
-  auto issue_loads = [&](int c) {
-    const int s = c & 1;
-    uint8_t* st = smem + s * FWD_STAGE;
-    const int row0 = (bh * NC + c) * CH;
-    tc5::mbar_expect_tx(&full[s], FWD_TX);
-#pragma unroll
-    for (int kb = 0; kb < 2; ++kb) {
-      tc5::tma_load_2d(st + kb * 2 * BOX, &tm_w, &full[s], kb * 64, row0);
-      tc5::tma_load_4d(st + kb * 2 * BOX + BOX, &tm_q, &full[s], kb * 64, h, c * CH, b);
-      tc5::tma_load_4d(st + 4 * BOX + kb * BOX, &tm_k, &full[s], kb * 64, h, c * CH, b);
-    }
-    tc5::tma_load_2d(st + 7 * BOX, &tm_qk, &full[s], 0, row0);
+  auto wait = [&](uint64_t* bar, int phase, int code) {
+    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
   };
-  if (boss) issue_loads(0);
-
-  constexpr uint32_t idesc1 = tc5::make_idesc_bf16(128, VT, 0, 1);   // A K-major, B MN-major
-  constexpr uint32_t idesc2 = tc5::make_idesc_bf16(128, VT, 1, 1);   // A MN-major (k^T), B MN-major
-  bool ok = true;
-  // Global loads of the chain (u row, gates) are fetched one chunk ahead.
   const float* gc = p.gc + static_cast<long>(bh) * NC * CH;
-  uint32_t upk_next[HC / 2];
-#pragma unroll
-  for (int j = 0; j < HC / 2; ++j) upk_next[j] = 0u;
-  if (r < CH) load_global(p.u + (static_cast<long>(bh * NC) * CH + r) * V + vt * VT + half * HC, upk_next);
-  float gr_next = gc[r & 63], gl_next = gc[CH - 1];
-  float oi[HC];                                    // sq (q S) of the chunk whose output is still open (rows 64..127)
-  // Output of chunk c: D2 joins oi; runs while the tensor core works on chunk c + 1.
-  auto finish_output = [&](int c) {
-    if (!tc5::mbar_wait(m3, c & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
-    __syncwarp();
-    tc5::fence_after_sync();
-    if (r < CH) return;                            // the other warps stay together, also after a wait that gave up
-    float d2[HC];
-    tmem_ld_half(tmem + lane_off + cD2, d2);
-#pragma unroll
-    for (int j = 0; j < HC; ++j) d2[j] += oi[j];
-    uint32_t pk[HC / 2];
-    pack_half(d2, pk);
-    if (threadIdx.x == CH) tc5::tma_store_wait_read<0>();    // the previous output tile has been read
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    write_half(Ob, r - CH, half, pk);
-    tc5::fence_proxy_async();
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (threadIdx.x == CH && ok) {                           // rows past T are clipped by the copy engine
-      tc5::tma_store_4d(&tm_o, Ob, vt * VT, h, c * CH, b);
-      tc5::tma_store_commit();
-    }
-  };
-  for (int c = 0; c < NC && ok; ++c) {
-    const int s = c & 1;
-    uint8_t* st = smem + s * FWD_STAGE;
-    const long row0 = static_cast<long>(bh * NC + c) * CH;
-    uint32_t upk[HC / 2];
-#pragma unroll
-    for (int j = 0; j < HC / 2; ++j) upk[j] = upk_next[j];
-    const float g_row = gr_next, g_last = gl_next;
-    if (warp == 0) {
-      // The issuing warp stays converged and one elected lane issues: descriptors then live in
-      // uniform registers and an MMA costs the issuing thread a few cycles instead of 70 to 100,
-      // which matters in a loop that is one dependent chain.
-      const bool lead = tc5::elect_one();
-      if (__all_sync(0xffffffffu, tc5::mbar_wait(&full[s], (c >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL))) {
-        tc5::fence_after_sync();
-        const uint64_t a1 = tc5::desc_kmajor(tc5::smem_u32(st)), sb = tc5::desc_mnmajor(tc5::smem_u32(Sb), BOX);
-        if (lead) {
-#pragma unroll
-          for (int kk = 0; kk < KD / 16; ++kk)
-            tc5::mma_ss(tmem + cD1, a1 + static_cast<uint64_t>(((kk >> 2) * 2 * BOX + (kk & 3) * 32) >> 4),
-                        sb + static_cast<uint64_t>((kk * 2048) >> 4), idesc1, kk > 0 ? 1u : 0u);
-          tc5::mma_commit(m1);
-        }
-      }
-      __syncwarp();
-    }
-    // next chunk's u row (rows 0..63 only) and gates, in flight while this chunk computes
-    if (c + 1 < NC) {
-      if (r < CH) load_global(p.u + (row0 + CH + r) * V + vt * VT + half * HC, upk_next);
-      gr_next = gc[(c + 1) * CH + (r & 63)];
-      gl_next = gc[(c + 1) * CH + CH - 1];
-    }
-    if (c > 0) finish_output(c - 1);
-    // the stage of chunk c + 1 was last read by chunk c - 1's second group of MMAs, complete since finish_output
-    if (boss && ok && c + 1 < NC) issue_loads(c + 1);
-    if (boss) tc5::tma_store_wait_read<1>();     // the previous v_new tile has been read
-    if (ok && !tc5::mbar_wait(m1, c & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
-    if (__syncthreads_or(!ok)) { ok = false; break; }
-    tc5::fence_after_sync();
+  if (warp < 8) {
+    const uint32_t lane_off = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * HC;   // lanes and columns of this thread
     {
+      float z[HC];
+#pragma unroll
+      for (int j = 0; j < HC; ++j) z[j] = 0.f;
+      tmem_st_half(tmem + lane_off + cS, z);
+    }
+    tc5::fence_before_sync();
+    arrive_warp(sready);
+    arrive_warp(scaled);
+    const bool upper = r < CH;                     // rows of w S and v_new; the others hold q S and the output
+    // The gates are in flight for a whole chunk.
+    float g_row = gc[r & 63], g_last = gc[CH - 1];
+    for (int c = 0; c < NC; ++c) {
+      float g_row_next = 0.f, g_last_next = 0.f;
+      if (c + 1 < NC) {
+        g_row_next = gc[(c + 1) * CH + (r & 63)];
+        g_last_next = gc[(c + 1) * CH + CH - 1];
+      }
+      const float sk = __expf(g_last - g_row), sq = p.scale * __expf(g_row);
+      float uf[HC];
+      if (upper) {
+        if (!wait(full_u + (c & 1), c >> 1, STATUS_TIMEOUT_SMEM_FULL)) break;
+        read_half(Us + (c & 1) * BOX, r, half, uf);
+        arrive_warp(empty_u + (c & 1));
+      }
+      if (!wait(m1, c, STATUS_TIMEOUT_TMEM_FULL)) break;
+      tc5::fence_after_sync();
       float d1[HC];
       tmem_ld_half(tmem + lane_off + cD1, d1);
-      if (r < CH) {
-        float uf[HC];
-        unpack_half(upk, uf);
-        const float sk = __expf(g_last - g_row);
+      if (upper) {
         uint32_t pk[HC / 2], ps[HC / 2];
 #pragma unroll
         for (int j = 0; j < HC; ++j) d1[j] = uf[j] - d1[j];
@@ -266,26 +195,79 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 #pragma unroll
         for (int j = 0; j < HC; ++j) d1[j] *= sk;
         pack_half(d1, ps);
-        write_half(Vb, r, half, pk);
-        write_half(Vs, r, half, ps);
+        write_half(Vs, r, half, ps);               // read by the products of chunk c - 1, complete since m2
+        write_half(Vb + (c & 1) * BOX, r, half, pk);
+        tc5::fence_proxy_async();
+        arrive_warp(vready);
       } else {
-        const float sq = p.scale * __expf(g_row);
 #pragma unroll
-        for (int j = 0; j < HC; ++j) oi[j] = sq * d1[j];
+        for (int j = 0; j < HC; ++j) d1[j] *= sq;
       }
+      if (c + 1 < NC) {
+        const float g = __expf(g_last_next);       // decay of the state through chunk c + 1
+        if (!wait(m2, c, STATUS_TIMEOUT_TMEM_FULL)) break;
+        tc5::fence_after_sync();
+        float sv[HC];
+        tmem_ld_half(tmem + lane_off + cS, sv);    // S entering chunk c + 1, row r
+        uint32_t pk[HC / 2];
+        pack_half(sv, pk);
+        if (!wait(freed, c, STATUS_TIMEOUT_SMEM_EMPTY)) break;
+        write_half(Sb + ((c + 1) & 1) * 2 * BOX, r, half, pk);
+        tc5::fence_proxy_async();
+        tc5::fence_before_sync();
+        arrive_warp(sready);
+#pragma unroll
+        for (int j = 0; j < HC; ++j) sv[j] *= g;
+        tmem_st_half(tmem + lane_off + cS, sv);
+        tc5::fence_before_sync();
+        arrive_warp(scaled);
+      } else if (!wait(freed, c, STATUS_TIMEOUT_SMEM_EMPTY)) {
+        break;
+      }
+      if (!upper) {                                // output rows, behind the next chunk's first product
+        if (!wait(m3, c, STATUS_TIMEOUT_TMEM_FULL)) break;
+        tc5::fence_after_sync();
+        float d2[HC];
+        tmem_ld_half(tmem + lane_off + cD2, d2);
+#pragma unroll
+        for (int j = 0; j < HC; ++j) d2[j] += d1[j];
+        uint32_t pk[HC / 2];
+        pack_half(d2, pk);
+        write_half(Ob + (c & 1) * BOX, r - CH, half, pk);
+        tc5::fence_proxy_async();
+        tc5::fence_before_sync();
+        arrive_warp(oready);
+      }
+      g_row = g_row_next;
+      g_last = g_last_next;
     }
-    tc5::fence_proxy_async();
-    tc5::fence_before_sync();
-    __syncthreads();
-    if (boss && p.store_states) {
-      tc5::tma_store_2d(&tm_vn, Vb, vt * VT, static_cast<int>(row0));
-      tc5::tma_store_commit();
-    }
-    if (warp == 0) {
-      const bool lead = tc5::elect_one();
+  } else if (warp == WARP_MMA) {
+    constexpr uint32_t idesc1 = tc5::make_idesc_bf16(128, VT, 0, 1);   // A K-major, B MN-major
+    constexpr uint32_t idesc2 = tc5::make_idesc_bf16(128, VT, 1, 1);   // A MN-major (k^T), B MN-major
+    // The issuing warp stays converged and one elected lane issues: descriptors then live in uniform
+    // registers and an MMA costs the issuing thread a few cycles instead of 70 to 100.
+    const bool lead = tc5::elect_one();
+    const uint64_t vs = tc5::desc_mnmajor(tc5::smem_u32(Vs), BOX);
+    for (int c = 0; c < NC; ++c) {
+      const int s = c & 1;
+      const uint32_t st = tc5::smem_u32(smem + s * FWD_STAGE);
+      const uint64_t a1 = tc5::desc_kmajor(st), sb = tc5::desc_mnmajor(tc5::smem_u32(Sb + s * 2 * BOX), BOX);
+      const uint64_t kt = tc5::desc_mnmajor(st + 4 * BOX, BOX), qk = tc5::desc_kmajor(st + 6 * BOX);
+      const uint64_t vb = tc5::desc_mnmajor(tc5::smem_u32(Vb + s * BOX), BOX);
+      if (!wait(full_a + s, c >> 1, STATUS_TIMEOUT_SMEM_FULL) || !wait(sready, c, STATUS_TIMEOUT_TMEM_EMPTY)) break;
       tc5::fence_after_sync();
-      const uint64_t kt = tc5::desc_mnmajor(tc5::smem_u32(st + 4 * BOX), BOX), vs = tc5::desc_mnmajor(tc5::smem_u32(Vs), BOX);
-      const uint64_t qk = tc5::desc_kmajor(tc5::smem_u32(st + 6 * BOX)), vb = tc5::desc_mnmajor(tc5::smem_u32(Vb), BOX);
+      if (lead) {
+#pragma unroll
+        for (int kk = 0; kk < KD / 16; ++kk)
+          tc5::mma_ss(tmem + cD1, a1 + static_cast<uint64_t>(((kk >> 2) * 2 * BOX + (kk & 3) * 32) >> 4),
+                      sb + static_cast<uint64_t>((kk * 2048) >> 4), idesc1, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(m1);
+        tc5::mma_commit(empty_a + s);
+      }
+      __syncwarp();
+      if (!wait(full_b + s, c >> 1, STATUS_TIMEOUT_SMEM_FULL) || !wait(scaled, c, STATUS_TIMEOUT_TMEM_EMPTY) || (c > 0 && !wait(oready, c - 1, STATUS_TIMEOUT_TMEM_EMPTY)) ||
+          !wait(vready, c, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      tc5::fence_after_sync();
       if (lead) {
 #pragma unroll
         for (int kk = 0; kk < CH / 16; ++kk)       // S += k^T (sk v_new)
@@ -295,37 +277,96 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         for (int kk = 0; kk < CH / 16; ++kk)       // D2 = [0 ; qk] v_new
           tc5::mma_ss(tmem + cD2, qk + static_cast<uint64_t>((kk * 32) >> 4), vb + static_cast<uint64_t>((kk * 2048) >> 4), idesc1, kk > 0 ? 1u : 0u);
         tc5::mma_commit(m3);
+        tc5::mma_commit(empty_b + s);
       }
       __syncwarp();
     }
-    if (boss) tc5::tma_store_wait_read<1>();     // the previous state tile has been read
-    if (!tc5::mbar_wait(m2, c & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
-    if (__syncthreads_or(!ok)) { ok = false; break; }
-    tc5::fence_after_sync();
-    if (c + 1 < NC) {
-      float sv[HC];
-      tmem_ld_half(tmem + lane_off + cS, sv);     // S entering chunk c+1, row r
-      uint32_t pk[HC / 2];
-      pack_half(sv, pk);
-      write_half(Sb, r, half, pk);
-      const float g = __expf(gl_next);             // its decay through chunk c + 1
+  } else if (warp == WARP_LOAD) {
+    const bool lead = tc5::elect_one();
+    bool ok = true;
+    // The CTAs of a head's V tiles share the chunk's tiles; each asks for those of every nvt-th chunk.
+    const int nvt = gridDim.x;
+    auto prefetch = [&](int c) {
+      if (c >= NC || !lead) return;
+      const int row0 = (bh * NC + c) * CH;
+      tc5::tma_prefetch_2d(&tm_u, vt * VT, row0);
+      if (c % nvt != vt) return;
 #pragma unroll
-      for (int j = 0; j < HC; ++j) sv[j] *= g;
-      tmem_st_half(tmem + lane_off + cS, sv);
-      tc5::fence_proxy_async();
+      for (int kb = 0; kb < 2; ++kb) {
+        tc5::tma_prefetch_2d(&tm_w, kb * 64, row0);
+        tc5::tma_prefetch_4d(&tm_q, kb * 64, h, c * CH, b);
+        tc5::tma_prefetch_4d(&tm_k, kb * 64, h, c * CH, b);
+      }
+      tc5::tma_prefetch_2d(&tm_qk, 0, row0);
+    };
+    for (int c = 2; c < AHEAD; ++c) prefetch(c);
+    for (int c = 0; c < NC; ++c) {
+      const int s = c & 1, row0 = (bh * NC + c) * CH;
+      uint8_t* st = smem + s * FWD_STAGE;
+      if (c >= 2 && !(ok = wait(empty_a + s, (c >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
+      if (lead) {
+        tc5::mbar_expect_tx(full_a + s, FWD_TX_A);
+#pragma unroll
+        for (int kb = 0; kb < 2; ++kb) {
+          tc5::tma_load_2d(st + kb * 2 * BOX, &tm_w, full_a + s, kb * 64, row0);
+          tc5::tma_load_4d(st + kb * 2 * BOX + BOX, &tm_q, full_a + s, kb * 64, h, c * CH, b);
+        }
+      }
+      __syncwarp();
+      if (c >= 2 && !(ok = wait(empty_u + s, (c >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
+      if (lead) {
+        tc5::mbar_expect_tx(full_u + s, BOX);
+        tc5::tma_load_2d(Us + s * BOX, &tm_u, full_u + s, vt * VT, row0);
+      }
+      __syncwarp();
+      if (c >= 2 && !(ok = wait(empty_b + s, (c >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
+      if (lead) {
+        tc5::mbar_expect_tx(full_b + s, FWD_TX_B);
+#pragma unroll
+        for (int kb = 0; kb < 2; ++kb) tc5::tma_load_4d(st + 4 * BOX + kb * BOX, &tm_k, full_b + s, kb * 64, h, c * CH, b);
+        tc5::tma_load_2d(st + 7 * BOX, &tm_qk, full_b + s, 0, row0);
+      }
+      prefetch(c + AHEAD);
+      __syncwarp();
     }
-    tc5::fence_before_sync();
-    __syncthreads();
-    if (boss && c + 1 < NC && p.store_states) {
-      tc5::tma_store_2d(&tm_sa, Sb, vt * VT, (bh * NC + c + 1) * KD);
+    for (int c = NC > 2 ? NC - 2 : 0; c < NC && ok; ++c)
+      ok = wait(empty_a + (c & 1), c >> 1, STATUS_TIMEOUT_SMEM_EMPTY) && wait(empty_b + (c & 1), c >> 1, STATUS_TIMEOUT_SMEM_EMPTY);
+    if (!ok && lead) {                             // loads may still be in flight
+      for (int i = 0; i < 2; ++i) {
+        tc5::mbar_drain(full_a + i);
+        tc5::mbar_drain(full_b + i);
+        tc5::mbar_drain(full_u + i);
+      }
+    }
+    __syncwarp();
+  } else {
+    // Outputs leave as TMA stores from the swizzled tiles they are in anyway; chunk 0 enters with the zero state.
+    const bool lead = tc5::elect_one();
+    auto store_o = [&](int c) {                    // rows past T are clipped by the copy engine
+      if (lead) tc5::tma_store_4d(&tm_o, Ob + (c & 1) * BOX, vt * VT, h, c * CH, b);
+    };
+    bool ok = true;
+    for (int c = 0; c < NC; ++c) {
+      if (!(ok = wait(sready, c, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+      if (lead && p.store_states) tc5::tma_store_2d(&tm_sa, Sb + (c & 1) * 2 * BOX, vt * VT, (bh * NC + c) * KD);
+      if (c > 0) {
+        if (!(ok = wait(oready, c - 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+        store_o(c - 1);
+      }
+      if (!(ok = wait(vready, c, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+      if (lead) {
+        if (p.store_states) tc5::tma_store_2d(&tm_vn, Vb + (c & 1) * BOX, vt * VT, (bh * NC + c) * CH);
+        tc5::tma_store_commit();
+        tc5::tma_store_wait_read<1>();
+      }
+      arrive_warp(freed);
+    }
+    if (ok && wait(oready, NC - 1, STATUS_TIMEOUT_TMEM_EMPTY)) store_o(NC - 1);
+    if (lead) {
       tc5::tma_store_commit();
+      tc5::tma_store_wait_read<0>();
     }
-  }
-  if (ok) finish_output(NC - 1);
-  if (boss || threadIdx.x == CH) tc5::tma_store_wait_read<0>();
-  if (!ok && boss) {                               // a load for the next chunk may still be in flight
-    tc5::mbar_drain(&full[0]);
-    tc5::mbar_drain(&full[1]);
+    __syncwarp();
   }
   tc5::fence_before_sync();
   __syncthreads();
@@ -333,7 +374,6 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 }
 
 struct BwdParams {
-  const bf16* d_o;       // [B, T, H, V]
   const float* gc;       // [BH, NC, 64]
   float* dgamma_part;    // [VTILES, BH, NC]
   int NC, V, BH, H, T;
@@ -343,232 +383,293 @@ struct BwdParams {
 
 // stage: k-block kb of [k ; w] (2 x 16 KB), q (16 KB), S_prev [KD][64] (16 KB), [qk | 0] (16 KB, second half zero)
 constexpr int BWD_STAGE = 10 * BOX;                                        // 80 KB
-constexpr int BWD_TX = 9 * BOX;
-constexpr int BWD_SMEM = 2 * BWD_STAGE + BOX /*du*/ + 2 * BOX /*do, sq do*/ + 2 * BOX /*dSb*/ + 1024 + 128;
+constexpr int BWD_TX = 8 * BOX, BWD_TX_S = 2 * BOX;                        // with do; S_prev is free much earlier than the others
+constexpr int BWD_SMEM = 2 * BWD_STAGE + 2 * BOX /*du*/ + 3 * BOX /*do, sq do*/ + 2 * BOX /*dSb*/ + 1024 + 256;
 
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(352, 1)
 gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_S,
-                   const __grid_constant__ CUtensorMap tm_qk, const __grid_constant__ CUtensorMap tm_du,
+                   const __grid_constant__ CUtensorMap tm_qk, const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_du,
                    const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sDU = smem + 2 * BWD_STAGE;    // [64][64] du
-  uint8_t* sDO = sDU + BOX;               // [64][64] do
-  uint8_t* sDOs = sDO + BOX;              // [64][64] sq do
+  uint8_t* sDU = smem + 2 * BWD_STAGE;    // 2 x [64][64] du
+  uint8_t* sDO = sDU + 2 * BOX;           // 2 x [64][64] do, of the stages
+  uint8_t* sDOs = sDO + 2 * BOX;          // [64][64] sq do
   uint8_t* dSb = sDOs + BOX;              // [KD rows][64] bf16 mirror of dS
   uint64_t* bars = reinterpret_cast<uint64_t*>(dSb + 2 * BOX);
-  uint64_t* full = bars;
-  uint64_t* m1 = bars + 2;
-  uint64_t* m2 = bars + 3;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
+  uint64_t *full = bars, *empty = bars + 2;     // [2] each: the stages without S_prev
+  uint64_t *full_s = bars + 4, *empty_s = bars + 6;   // [2] each: S_prev
+  uint64_t *m1 = bars + 8, *m2 = bars + 9;      // products complete: Da and Dd, dS
+  uint64_t *sready = bars + 10, *scaled = bars + 11, *uready = bars + 12, *oready = bars + 13;    // rows written: dSb, dS, du, do and sq do
+  uint64_t *gready = bars + 14, *freed = bars + 15;   // sums of dgamma are there; dSb and the other tile of du have been read by their stores
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* red = reinterpret_cast<float*>(tmem_slot + 2);     // [8]
+  float* red = reinterpret_cast<float*>(tmem_slot + 2);     // [2][8]
 
-  const int r = threadIdx.x & 127, half = threadIdx.x >> 7;
+  const int r = threadIdx.x & 127, half = (threadIdx.x >> 7) & 1;
   const int warp = threadIdx.x >> 5;
-  const bool boss = threadIdx.x == 0;
   const int vt = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
-  const int NC = p.NC, V = p.V;
+  const int NC = p.NC;
 
-  if (boss) {
+  if (threadIdx.x == 0) {
     *abort_flag = 0;
-    tc5::mbar_init(&full[0], 1);
-    tc5::mbar_init(&full[1], 1);
+    for (int i = 0; i < 6; ++i) tc5::mbar_init(bars + i, 1);
+    tc5::mbar_init(empty_s, 8);
+    tc5::mbar_init(empty_s + 1, 8);
     tc5::mbar_init(m1, 1);
     tc5::mbar_init(m2, 1);
+    tc5::mbar_init(sready, 8);
+    tc5::mbar_init(scaled, 8);
+    tc5::mbar_init(uready, 4);
+    tc5::mbar_init(oready, 4);
+    tc5::mbar_init(gready, 8);
+    tc5::mbar_init(freed, 1);
     tc5::fence_barrier_init();
   }
   if (warp == 0) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
-  {
+  if (warp < 8) {
     uint32_t z[HC / 2];
 #pragma unroll
     for (int j = 0; j < HC / 2; ++j) z[j] = 0u;
     write_half(dSb, r, half, z);
     write_half(smem + (r >> 6) * BWD_STAGE + 9 * BOX, r & 63, half, z);
+    tc5::fence_proxy_async();
   }
-  tc5::fence_proxy_async();
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_off = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * HC;   // lanes and columns of this thread
   // TMEM columns: Da = [k ; w] dS [0,64)   Dd = [qk^T ; 0] do [64,128)   dS [128,192)
   const uint32_t cDa = 0, cDd = 64, cDs = 128;
-  {
-    float z[HC];
-#pragma unroll
-    for (int j = 0; j < HC; ++j) z[j] = 0.f;
-    tmem_st_half(tmem + lane_off + cDs, z);
-  }
-  tc5::fence_before_sync();
-  __syncthreads();
-  // outputs leave as TMA stores from swizzled tiles (see the forward kernel); the last chunk's state has no gradient
-  if (boss) {
-    tc5::tma_store_2d(&tm_ds, dSb, vt * VT, (bh * NC + NC - 1) * KD);
-    tc5::tma_store_commit();
-  }
-
-  auto issue_loads = [&](int c, int it) {
-    const int s = it & 1;
-    uint8_t* st = smem + s * BWD_STAGE;
-    const int row0 = (bh * NC + c) * CH;
-    tc5::mbar_expect_tx(&full[s], BWD_TX);
-#pragma unroll
-    for (int kb = 0; kb < 2; ++kb) {
-      tc5::tma_load_4d(st + kb * 2 * BOX, &tm_k, &full[s], kb * 64, h, c * CH, b);
-      tc5::tma_load_2d(st + kb * 2 * BOX + BOX, &tm_w, &full[s], kb * 64, row0);
-      tc5::tma_load_4d(st + 4 * BOX + kb * BOX, &tm_q, &full[s], kb * 64, h, c * CH, b);
-    }
-    tc5::tma_load_2d(st + 6 * BOX, &tm_S, &full[s], vt * VT, (bh * NC + c) * KD);
-    tc5::tma_load_2d(st + 8 * BOX, &tm_qk, &full[s], 0, row0);
+  auto wait = [&](uint64_t* bar, int phase, int code) {
+    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
   };
-  if (boss) issue_loads(NC - 1, 0);
-
-  constexpr uint32_t id_a = tc5::make_idesc_bf16(128, VT, 0, 1);        // [k;w] (K-major) x dS (MN-major)
-  constexpr uint32_t id_d = tc5::make_idesc_bf16(128, VT, 1, 1);        // q^T x (sq do), [qk^T ; 0] x do
-  constexpr uint32_t id_dn = tc5::make_idesc_bf16(128, VT, 1, 1, 1);    // (-w)^T x du
-  bool ok = true;
-  // The chunk loop is one dependent chain: the do rows (threads 64..127) and the gates are fetched one chunk ahead.
   const float* gc = p.gc + static_cast<long>(bh) * NC * CH;
-  const bf16* d_o = p.d_o + (static_cast<long>(b) * p.T * p.H + h) * V + vt * VT + half * HC;
-  uint32_t row_next[HC / 2];
+  if (warp < 8) {
+    const uint32_t lane_off = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * HC;   // lanes and columns of this thread
+    const bool upper = r < CH;                     // rows of k dS and du; the others bring do
+    {
+      float z[HC];
 #pragma unroll
-  for (int j = 0; j < HC / 2; ++j) row_next[j] = 0u;
-  float gr_next, gl_next;
-  auto fetch_rows = [&](int cc) {
-    const int t = cc * CH + r - CH;
-    if (r >= CH) {
-      if (t < p.T) load_global(d_o + static_cast<long>(t) * p.H * V, row_next);
-      else {
-#pragma unroll
-        for (int j = 0; j < HC / 2; ++j) row_next[j] = 0u;
-      }
+      for (int j = 0; j < HC; ++j) z[j] = 0.f;
+      tmem_st_half(tmem + lane_off + cDs, z);
     }
-    gr_next = gc[cc * CH + (r & 63)];
-    gl_next = gc[cc * CH + CH - 1];
-  };
-  fetch_rows(NC - 1);
-  for (int it = 0; it < NC && ok; ++it) {
-    const int c = NC - 1 - it;
-    const int s = it & 1;
-    uint8_t* st = smem + s * BWD_STAGE;
-    const long row0 = static_cast<long>(bh * NC + c) * CH;
-    const float g_row = gr_next, g_last = gl_next;
-    // stage this chunk's do rows (already in registers) and start the next chunk's loads
-    if (r >= CH) {
-      write_half(sDO, r - CH, half, row_next);
+    tc5::fence_before_sync();
+    arrive_warp(sready);
+    arrive_warp(scaled);
+    auto stage_row = [&](int it, float g_row) {    // sq do of step `it`
+      if (!wait(full + (it & 1), it >> 1, STATUS_TIMEOUT_SMEM_FULL)) return false;
       float f[HC];
-      unpack_half(row_next, f);
+      read_half(sDO + (it & 1) * BOX, r - CH, half, f);
       const float sq = p.scale * __expf(g_row);
 #pragma unroll
       for (int j = 0; j < HC; ++j) f[j] *= sq;
       uint32_t pk[HC / 2];
       pack_half(f, pk);
       write_half(sDOs, r - CH, half, pk);
+      tc5::fence_proxy_async();
+      arrive_warp(oready);
+      return true;
+    };
+    // dgamma of step `it`, whose leaving gradient is ds: partial per warp; the last use of the entering state in the stage
+    auto gamma_part = [&](int it, const float (&ds)[HC]) {
+      const int s = it & 1;
+      if (!wait(full_s + s, it >> 1, STATUS_TIMEOUT_SMEM_FULL)) return false;
+      float sp[HC], part = 0.f;
+      read_half(smem + s * BWD_STAGE + 6 * BOX, r, half, sp);
+#pragma unroll
+      for (int j = 0; j < HC; ++j) part += ds[j] * sp[j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      if ((threadIdx.x & 31) == 0) red[s * 8 + warp] = part;
+      arrive_warp(gready);
+      arrive_warp(empty_s + s);
+      return true;
+    };
+    float g_row = gc[(NC - 1) * CH + (r & 63)], g_last = gc[(NC - 1) * CH + CH - 1];
+    bool ok = upper || stage_row(0, g_row);
+    if (ok) {
+      float z[HC];
+#pragma unroll
+      for (int j = 0; j < HC; ++j) z[j] = 0.f;
+      ok = gamma_part(0, z);                       // nothing follows the last chunk
     }
-    if (c > 0) fetch_rows(c - 1);
-    tc5::fence_proxy_async();
-    tc5::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) {
-      // converged issuing warp, one elected lane issues (see the forward kernel)
-      const bool lead = tc5::elect_one();
-      if (__all_sync(0xffffffffu, tc5::mbar_wait(&full[s], (it >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL))) {
+    for (int it = 0; it < NC && ok; ++it) {
+      const int c = NC - 1 - it;
+      float g_row_next = 0.f, g_last_next = 0.f;
+      if (c > 0) {
+        g_row_next = gc[(c - 1) * CH + (r & 63)];
+        g_last_next = gc[(c - 1) * CH + CH - 1];
+      }
+      const float sk = __expf(g_last - g_row);
+      if (upper) {
+        if (!wait(m1, it, STATUS_TIMEOUT_TMEM_FULL)) break;
         tc5::fence_after_sync();
-        const uint64_t a = tc5::desc_kmajor(tc5::smem_u32(st)), dsbm = tc5::desc_mnmajor(tc5::smem_u32(dSb), BOX);
-        const uint64_t qk = tc5::desc_mnmajor(tc5::smem_u32(st + 8 * BOX), BOX), dom = tc5::desc_mnmajor(tc5::smem_u32(sDO), BOX);
-        if (lead) {
+        float da[HC], dd[HC];
+        tmem_ld_half(tmem + lane_off + cDa, da);
+        tmem_ld_half(tmem + lane_off + cDd, dd);
 #pragma unroll
-          for (int kk = 0; kk < KD / 16; ++kk)      // Da = [k ; w] dS
-            tc5::mma_ss(tmem + cDa, a + static_cast<uint64_t>(((kk >> 2) * 2 * BOX + (kk & 3) * 32) >> 4),
-                        dsbm + static_cast<uint64_t>((kk * 2048) >> 4), id_a, kk > 0 ? 1u : 0u);
+        for (int j = 0; j < HC; ++j) da[j] = dd[j] + sk * da[j];
+        uint32_t pk[HC / 2];
+        pack_half(da, pk);
+        write_half(sDU + (it & 1) * BOX, r, half, pk);
+        tc5::fence_proxy_async();
+        tc5::fence_before_sync();
+        arrive_warp(uready);
+      }
+      if (c == 0) break;
+      const float g = __expf(g_last_next);
+      if (!wait(m2, it, STATUS_TIMEOUT_TMEM_FULL)) break;
+      tc5::fence_after_sync();
+      float ds[HC];
+      tmem_ld_half(tmem + lane_off + cDs, ds);     // gradient of the state leaving chunk c - 1
+      uint32_t pk[HC / 2];
+      pack_half(ds, pk);
+      if (!wait(freed, it, STATUS_TIMEOUT_SMEM_EMPTY)) break;
+      write_half(dSb, r, half, pk);
+      tc5::fence_proxy_async();
+      tc5::fence_before_sync();
+      arrive_warp(sready);
+      if (!upper && !stage_row(it + 1, g_row_next)) break;
+      {
+        float sv[HC];
 #pragma unroll
-          for (int kk = 0; kk < CH / 16; ++kk)      // Dd = [qk^T ; 0] do
-            tc5::mma_ss(tmem + cDd, qk + static_cast<uint64_t>((kk * 2048) >> 4), dom + static_cast<uint64_t>((kk * 2048) >> 4), id_d, kk > 0 ? 1u : 0u);
-          tc5::mma_commit(m1);
-          if (it + 1 < NC) issue_loads(c - 1, it + 1);
-        }
+        for (int j = 0; j < HC; ++j) sv[j] = g * ds[j];
+        tmem_st_half(tmem + lane_off + cDs, sv);
+      }
+      tc5::fence_before_sync();
+      arrive_warp(scaled);
+      ok = gamma_part(it + 1, ds);
+      g_row = g_row_next;
+      g_last = g_last_next;
+    }
+  } else if (warp == WARP_MMA) {
+    constexpr uint32_t id_a = tc5::make_idesc_bf16(128, VT, 0, 1);        // [k;w] (K-major) x dS (MN-major)
+    constexpr uint32_t id_d = tc5::make_idesc_bf16(128, VT, 1, 1);        // q^T x (sq do), [qk^T ; 0] x do
+    constexpr uint32_t id_dn = tc5::make_idesc_bf16(128, VT, 1, 1, 1);    // (-w)^T x du
+    const bool lead = tc5::elect_one();            // converged issuing warp, one elected lane issues (see the forward kernel)
+    const uint64_t dsbm = tc5::desc_mnmajor(tc5::smem_u32(dSb), BOX), dos = tc5::desc_mnmajor(tc5::smem_u32(sDOs), BOX);
+    for (int it = 0; it < NC; ++it) {
+      const int s = it & 1;
+      const uint32_t st = tc5::smem_u32(smem + s * BWD_STAGE);
+      const uint64_t a = tc5::desc_kmajor(st), dom = tc5::desc_mnmajor(tc5::smem_u32(sDO + s * BOX), BOX);
+      const uint64_t qk = tc5::desc_mnmajor(st + 8 * BOX, BOX), qdm = tc5::desc_mnmajor(st + 4 * BOX, BOX);
+      const uint64_t wm = tc5::desc_mnmajor(st + BOX, 2 * BOX), dum = tc5::desc_mnmajor(tc5::smem_u32(sDU + s * BOX), BOX);
+      if (!wait(full + s, it >> 1, STATUS_TIMEOUT_SMEM_FULL) || !wait(sready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      tc5::fence_after_sync();
+      if (lead) {
+#pragma unroll
+        for (int kk = 0; kk < KD / 16; ++kk)      // Da = [k ; w] dS
+          tc5::mma_ss(tmem + cDa, a + static_cast<uint64_t>(((kk >> 2) * 2 * BOX + (kk & 3) * 32) >> 4),
+                      dsbm + static_cast<uint64_t>((kk * 2048) >> 4), id_a, kk > 0 ? 1u : 0u);
       }
       __syncwarp();
-    }
-    if (!tc5::mbar_wait(m1, it & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
-    if (boss) tc5::tma_store_wait_read<1>();     // the previous du tile has been read (one newer store: the dS tile)
-    if (__syncthreads_or(!ok)) { ok = false; break; }
-    tc5::fence_after_sync();
-    if (r < CH) {
-      float da[HC], dd[HC];
-      tmem_ld_half(tmem + lane_off + cDa, da);
-      tmem_ld_half(tmem + lane_off + cDd, dd);
-      const float sk = __expf(g_last - g_row);
-#pragma unroll
-      for (int j = 0; j < HC; ++j) da[j] = dd[j] + sk * da[j];
-      uint32_t pk[HC / 2];
-      pack_half(da, pk);
-      write_half(sDU, r, half, pk);
-    }
-    float part_dg = 0.f;
-    {
-      // dS: dgamma partial with S_prev, then scaled by gamma in place
-      float ds[HC], sp[HC];
-      tmem_ld_half(tmem + lane_off + cDs, ds);
-      read_half(st + 6 * BOX, r, half, sp);
-      const float g = __expf(g_last);
-#pragma unroll
-      for (int j = 0; j < HC; ++j) { part_dg += ds[j] * sp[j]; ds[j] *= g; }
-      tmem_st_half(tmem + lane_off + cDs, ds);
-    }
-    tc5::fence_proxy_async();
-    tc5::fence_before_sync();
-    __syncthreads();
-    if (boss) {
-      tc5::tma_store_2d(&tm_du, sDU, vt * VT, static_cast<int>(row0));
-      tc5::tma_store_commit();
-    }
-    if (warp == 0) {
-      const bool lead = tc5::elect_one();
+      if (!wait(oready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
       tc5::fence_after_sync();
-      const uint64_t qdm = tc5::desc_mnmajor(tc5::smem_u32(st + 4 * BOX), BOX), dom = tc5::desc_mnmajor(tc5::smem_u32(sDOs), BOX);
-      const uint64_t wm = tc5::desc_mnmajor(tc5::smem_u32(st + BOX), 2 * BOX), dum = tc5::desc_mnmajor(tc5::smem_u32(sDU), BOX);
+      if (lead) {
+#pragma unroll
+        for (int kk = 0; kk < CH / 16; ++kk)      // Dd = [qk^T ; 0] do
+          tc5::mma_ss(tmem + cDd, qk + static_cast<uint64_t>((kk * 2048) >> 4), dom + static_cast<uint64_t>((kk * 2048) >> 4), id_d, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(m1);
+      }
+      __syncwarp();
+      if (!wait(scaled, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      tc5::fence_after_sync();
       if (lead) {
 #pragma unroll
         for (int kk = 0; kk < CH / 16; ++kk)        // dS += q^T (sq do)
-          tc5::mma_ss(tmem + cDs, qdm + static_cast<uint64_t>((kk * 2048) >> 4), dom + static_cast<uint64_t>((kk * 2048) >> 4), id_d, 1u);
+          tc5::mma_ss(tmem + cDs, qdm + static_cast<uint64_t>((kk * 2048) >> 4), dos + static_cast<uint64_t>((kk * 2048) >> 4), id_d, 1u);
+      }
+      __syncwarp();
+      if (!wait(uready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      tc5::fence_after_sync();
+      if (lead) {
 #pragma unroll
         for (int kk = 0; kk < CH / 16; ++kk)        // dS -= w^T du      (w = second half of each k-block)
           tc5::mma_ss(tmem + cDs, wm + static_cast<uint64_t>((kk * 2048) >> 4), dum + static_cast<uint64_t>((kk * 2048) >> 4), id_dn, 1u);
         tc5::mma_commit(m2);
+        tc5::mma_commit(empty + s);
       }
       __syncwarp();
     }
-    // block reduction of the dgamma partial, behind the MMAs
-    for (int o = 16; o > 0; o >>= 1) part_dg += __shfl_xor_sync(0xffffffffu, part_dg, o);
-    if ((threadIdx.x & 31) == 0) red[warp] = part_dg;
-    if (boss) tc5::tma_store_wait_read<1>();     // the previous dS tile has been read
-    if (!tc5::mbar_wait(m2, it & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) { ok = false; }
-    if (__syncthreads_or(!ok)) { ok = false; break; }
-    tc5::fence_after_sync();
-    if (boss) p.dgamma_part[(static_cast<long>(vt) * p.BH + bh) * NC + c] =
-        ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
-    if (c > 0) {
-      float ds[HC];
-      tmem_ld_half(tmem + lane_off + cDs, ds);
-      uint32_t pk[HC / 2];
-      pack_half(ds, pk);
-      write_half(dSb, r, half, pk);
+  } else if (warp == WARP_LOAD) {
+    const bool lead = tc5::elect_one();
+    bool ok = true;
+    const int nvt = gridDim.x;
+    auto prefetch = [&](int it) {                    // see the forward kernel; S_prev is this CTA's own
+      const int c = NC - 1 - it, row0 = (bh * NC + c) * CH;
+      if (c < 0 || !lead) return;
+      tc5::tma_prefetch_2d(&tm_S, vt * VT, (bh * NC + c) * KD);
+      tc5::tma_prefetch_4d(&tm_do, vt * VT, h, c * CH, b);
+      if (c % nvt != vt) return;
+#pragma unroll
+      for (int kb = 0; kb < 2; ++kb) {
+        tc5::tma_prefetch_4d(&tm_k, kb * 64, h, c * CH, b);
+        tc5::tma_prefetch_2d(&tm_w, kb * 64, row0);
+        tc5::tma_prefetch_4d(&tm_q, kb * 64, h, c * CH, b);
+      }
+      tc5::tma_prefetch_2d(&tm_qk, 0, row0);
+    };
+    for (int it = 2; it < AHEAD; ++it) prefetch(it);
+    for (int it = 0; it < NC; ++it) {
+      const int s = it & 1, c = NC - 1 - it, row0 = (bh * NC + c) * CH;
+      uint8_t* st = smem + s * BWD_STAGE;
+      if (it >= 2 && !(ok = wait(empty_s + s, (it >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
+      if (lead) {
+        tc5::mbar_expect_tx(full_s + s, BWD_TX_S);
+        tc5::tma_load_2d(st + 6 * BOX, &tm_S, full_s + s, vt * VT, (bh * NC + c) * KD);
+      }
+      __syncwarp();
+      if (it >= 2 && !(ok = wait(empty + s, (it >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
+      if (lead) {
+        tc5::mbar_expect_tx(full + s, BWD_TX);
+#pragma unroll
+        for (int kb = 0; kb < 2; ++kb) {
+          tc5::tma_load_4d(st + kb * 2 * BOX, &tm_k, full + s, kb * 64, h, c * CH, b);
+          tc5::tma_load_2d(st + kb * 2 * BOX + BOX, &tm_w, full + s, kb * 64, row0);
+          tc5::tma_load_4d(st + 4 * BOX + kb * BOX, &tm_q, full + s, kb * 64, h, c * CH, b);
+        }
+        tc5::tma_load_2d(st + 8 * BOX, &tm_qk, full + s, 0, row0);
+        tc5::tma_load_4d(sDO + s * BOX, &tm_do, full + s, vt * VT, h, c * CH, b);
+      }
+      prefetch(it + AHEAD);
+      __syncwarp();
     }
-    tc5::fence_proxy_async();
-    tc5::fence_before_sync();
-    __syncthreads();
-    if (boss && c > 0) {
-      tc5::tma_store_2d(&tm_ds, dSb, vt * VT, (bh * NC + c - 1) * KD);
-      tc5::tma_store_commit();
+    for (int it = NC > 2 ? NC - 2 : 0; it < NC && ok; ++it)
+      ok = wait(empty + (it & 1), it >> 1, STATUS_TIMEOUT_SMEM_EMPTY) && wait(empty_s + (it & 1), it >> 1, STATUS_TIMEOUT_SMEM_EMPTY);
+    if (!ok && lead) {                               // loads may still be in flight
+      for (int i = 0; i < 2; ++i) {
+        tc5::mbar_drain(full + i);
+        tc5::mbar_drain(full_s + i);
+      }
     }
-  }
-  if (boss) tc5::tma_store_wait_read<0>();
-  if (!ok && boss) {                               // a load for the next chunk may still be in flight
-    tc5::mbar_drain(&full[0]);
-    tc5::mbar_drain(&full[1]);
+    __syncwarp();
+  } else {
+    // outputs leave as TMA stores from swizzled tiles; the last chunk's state has no gradient
+    const bool lead = tc5::elect_one();
+    for (int it = 0; it < NC; ++it) {
+      const int s = it & 1, c = NC - 1 - it;
+      if (!wait(sready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      if (lead) {
+        tc5::tma_store_2d(&tm_ds, dSb, vt * VT, (bh * NC + c) * KD);
+        tc5::tma_store_commit();
+      }
+      if (!wait(gready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      if (lead) {
+        const float* g = red + s * 8;
+        p.dgamma_part[(static_cast<long>(vt) * p.BH + bh) * NC + c] = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7]));
+      }
+      if (!wait(uready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      if (lead) {
+        tc5::tma_store_2d(&tm_du, sDU + s * BOX, vt * VT, (bh * NC + c) * CH);
+        tc5::tma_store_commit();
+        tc5::tma_store_wait_read<1>();             // dS of this chunk and du of the one before have been read
+      }
+      arrive_warp(freed);
+    }
+    if (lead) tc5::tma_store_wait_read<0>();
+    __syncwarp();
   }
   tc5::fence_before_sync();
   __syncthreads();
@@ -602,9 +703,10 @@ extern "C" int nsa_gdn_seq_fwd(const void* q, const void* k, const void* w, cons
   const int NC = (T + CH - 1) / CH, BH = B * H;
   const long rows = static_cast<long>(BH) * NC * CH;
   const bool states = v_new != nullptr && S_all != nullptr;
-  CUtensorMap tw, tq, tk, tqk, tvn, to, tsa;
+  CUtensorMap tw, tu, tq, tk, tqk, tvn, to, tsa;
   int rc;
   if ((rc = make_rows_map(&tw, w, rows, KD, CH))) return rc;
+  if ((rc = make_rows_map(&tu, u, rows, V, CH))) return rc;
   if ((rc = make_token_map(&tq, q, B, T, H, KD))) return rc;
   if ((rc = make_token_map(&tk, k, B, T, H, KD))) return rc;
   if ((rc = make_rows_map(&tqk, qk, rows, CH, CH))) return rc;
@@ -612,9 +714,9 @@ extern "C" int nsa_gdn_seq_fwd(const void* q, const void* k, const void* w, cons
   tvn = tw; tsa = tw;                              // never used without the states
   if (states && (rc = make_rows_map(&tvn, v_new, rows, V, CH))) return rc;
   if (states && (rc = make_rows_map(&tsa, S_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
-  FwdParams p{(const bf16*)u, gc, states, NC, V, H, scale, nsa::status_ptr()};
+  FwdParams p{gc, states, NC, V, H, scale, nsa::status_ptr()};
   if ((rc = set_smem(gdn_seq_fwd_kernel, FWD_SMEM, "gdn fwd smem attribute"))) return rc;
-  gdn_seq_fwd_kernel<<<dim3(V / VT, BH), 256, FWD_SMEM, st>>>(tw, tq, tk, tqk, tvn, to, tsa, p);
+  gdn_seq_fwd_kernel<<<dim3(V / VT, BH), 352, FWD_SMEM, st>>>(tw, tu, tq, tk, tqk, tvn, to, tsa, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_seq_fwd launch");
@@ -628,18 +730,19 @@ extern "C" int nsa_gdn_seq_bwd(const void* q, const void* k, const void* w, cons
   if (K != KD || V % VT) return nsa::fail(NSA_ERR_SHAPE, "gdn: key width must be 128 and value width a multiple of 64");
   const int NC = (T + CH - 1) / CH, BH = B * H;
   const long rows = static_cast<long>(BH) * NC * CH;
-  CUtensorMap tw, tq, tk, tqk, ts, tdu, tds;
+  CUtensorMap tw, tq, tk, tqk, ts, tdo, tdu, tds;
   int rc;
   if ((rc = make_rows_map(&tw, w, rows, KD, CH))) return rc;
   if ((rc = make_token_map(&tq, q, B, T, H, KD))) return rc;
   if ((rc = make_token_map(&tk, k, B, T, H, KD))) return rc;
   if ((rc = make_rows_map(&tqk, qk, rows, CH, CH))) return rc;
   if ((rc = make_rows_map(&ts, S_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
+  if ((rc = make_token_map(&tdo, d_o, B, T, H, V))) return rc;
   if ((rc = make_rows_map(&tdu, du, rows, V, CH))) return rc;
   if ((rc = make_rows_map(&tds, dS_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
-  BwdParams p{(const bf16*)d_o, gc, dgamma_part, NC, V, BH, H, T, scale, nsa::status_ptr()};
+  BwdParams p{gc, dgamma_part, NC, V, BH, H, T, scale, nsa::status_ptr()};
   if ((rc = set_smem(gdn_seq_bwd_kernel, BWD_SMEM, "gdn bwd smem attribute"))) return rc;
-  gdn_seq_bwd_kernel<<<dim3(V / VT, BH), 256, BWD_SMEM, st>>>(tw, tq, tk, ts, tqk, tdu, tds, p);
+  gdn_seq_bwd_kernel<<<dim3(V / VT, BH), 352, BWD_SMEM, st>>>(tw, tq, tk, ts, tqk, tdo, tdu, tds, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_gdn_seq_bwd launch");
