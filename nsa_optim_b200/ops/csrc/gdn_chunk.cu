@@ -16,6 +16,16 @@ constexpr int CH = 64, KD = 128;
 constexpr int PK = KD + 8, PC = CH + 8;          // tile pitches (elements)
 constexpr int PX = 68;                           // pitch of the fp32 64 x 64 tiles: rows 16-byte aligned, spread over the banks
 
+// Two fp32 lanes per instruction; each lane rounds as the scalar instruction does.
+__device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+        "l"(reinterpret_cast<const unsigned long long&>(c)));
+  return d;
+}
+
 // Per-chunk gate quantities: the CTA's first warp does the work, two tokens a lane; the caller synchronises.
 // gs: cumulative log-decay, bs: beta.
 __device__ __forceinline__ void load_gates(const float* g, const float* beta, long tok0, int T, int t0, int H, float* gs, float* bs) {
@@ -36,6 +46,16 @@ __device__ __forceinline__ void load_gates(const float* g, const float* beta, lo
   }
 }
 
+// The inputs of the CTA that will run on this SM next are asked for into L2 (resident: CTAs that run together): a chunk's loads
+// then wait for L2 and not for memory.
+__device__ __forceinline__ bool next_chunk(int resident, int H, int NC, int& bh, int& c) {
+  const long next = (static_cast<long>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x + resident;
+  bh = static_cast<int>(next % gridDim.x);
+  c = static_cast<int>(next / gridDim.x);
+  return c < NC;
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 struct PrepParams {
   const bf16 *q, *k, *v;       // [B, T, H, .]
   const float *g, *beta;       // [B, T, H]
@@ -43,6 +63,7 @@ struct PrepParams {
   float *X, *gc;               // [BH, NC, 64, 64] or null, [BH, NC, 64]
   int T, H, NC, V;
   float scale;
+  int resident;
 };
 
 // One CTA of eight warps per (chunk, head).  What bounds it is its chain of phases, not the memory traffic of q, k, v, u, w (2 KB
@@ -82,6 +103,13 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
   }
   cp_async_commit();
   load_gates(p.g, p.beta, tok0, p.T, t0, p.H, gs, bs);
+  int nbh, nc;
+  if (next_chunk(p.resident, p.H, p.NC, nbh, nc) && nc * CH + (tid & 63) < p.T) {        // a row each, 128 bytes at a time
+    const long row = (static_cast<long>(nbh / p.H) * p.T + nc * CH + (tid & 63)) * p.H + nbh % p.H;
+    const bf16* src = tid < 64 ? p.k + row * KD : tid < 128 ? p.q + row * KD : p.v + row * V + (tid < 192 ? 0 : 64);
+    const int step = tid < 128 ? 64 : 128, end = tid < 128 ? KD : V - (tid < 192 ? 0 : 64);
+    for (int x = 0; x < end; x += step) prefetch_l2(src + x);
+  }
   cp_async_wait<1>();
   __syncthreads();
   const long chunk = static_cast<long>(bh) * p.NC + c;
@@ -226,6 +254,7 @@ struct PostParams {
   float *dg, *dbeta;                    // [B, T, H]
   int B, T, H, NC, V;
   float scale;
+  int resident;
   KernelStatus* status;
 };
 
@@ -274,7 +303,9 @@ __device__ __forceinline__ void tmem_cols(uint32_t taddr, float (&out)[N]) {
 // The five products that sum over the value dimension are three full tcgen05 tiles of the stacked operands,
 // [du ; do] S^T, [v_new ; v] dS^T and [du ; do] [v_new ; v]^T, accumulated in tensor memory while slices of 64 value
 // columns stream through two TMA stages (as warp products with register accumulators they were two thirds of the
-// kernel: 700 us at 16384 tokens x 16 heads).  What is left are 64-row products, done by warps.  Per token and head
+// kernel: 700 us at 16384 tokens x 16 heads).  What is left are 64-row products, done by warps; they are two thirds of a CTA's 42000 cycles,
+// and one CTA fills an SM, so the next chunk's tiles are asked for into L2 meanwhile (670 us without that and with
+// 2 x 4 tiles for dA, 641 now).  Per token and head
 // 3.5 KB come in and 1 KB goes out, against 6 KB alone for the per-V-tile partials of dw, dq and dk that the sequential
 // pass would otherwise write and re-read.
 __global__ void __launch_bounds__(512, 1)
@@ -413,6 +444,27 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
       }
     }
   }
+  {
+    int nbh, nc;
+    if (next_chunk(p.resident, p.H, p.NC, nbh, nc)) {
+      const int nb = nbh / p.H, nh = nbh % p.H, nt = nc * CH;
+      const long nchunk = static_cast<long>(nbh) * p.NC + nc;
+      if (tid < nvt) {                                     // a slice each
+        const int x = tid * CH, row = static_cast<int>(nchunk) * CH;
+        tc5::tma_prefetch_2d(&tm_du, x, row);
+        tc5::tma_prefetch_4d(&tm_do, x, nh, nt, nb);
+        tc5::tma_prefetch_2d(&tm_vn, x, row);
+        tc5::tma_prefetch_4d(&tm_v, x, nh, nt, nb);
+        tc5::tma_prefetch_2d(&tm_S, x, static_cast<int>(nchunk) * KD);
+        tc5::tma_prefetch_2d(&tm_dS, x, static_cast<int>(nchunk) * KD);
+      } else if (tid >= 128 && tid < 256) {                // 64 rows of 256 bytes
+        prefetch_l2(p.X + nchunk * CH * CH + (tid - 128) * 32);
+      } else if (tid >= 256 && nt + (tid & 63) < p.T) {    // q and k, 128 bytes at a time
+        const bf16* src = tid < 384 ? p.q : p.k;
+        prefetch_l2(src + ((static_cast<long>(nb) * p.T + nt + (tid & 63)) * p.H + nh) * KD + (tid & 64));
+      }
+    }
+  }
   // the last two commits cover every product
   if (ok) {
     const int s = nvt - 1;
@@ -511,36 +563,49 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
   if (tid < CH)
 #pragma unroll
     for (int n = 0; n < 4; ++n) { dbeta += red[n * CH + tid]; dgc += red[(4 + n) * CH + tid]; }
-  // ---- dA = -(X^T dX X^T) below the diagonal, fp32; warp w owns rows 4 w .. 4 w + 3
+  // ---- dA = -(X^T dX X^T) below the diagonal, fp32; 4 x 4 tiles of eight warps (2 x 4 of sixteen read shared memory twice as
+  //      often as they multiply).  Warp w owns rows 8 w .. 8 w + 7.
   {
-    const int ra = (tid >> 4) * 2, ca = (tid & 15) * 4;
-    float4 y0 = make_float4(0.f, 0.f, 0.f, 0.f), y1 = y0;
+    const int ra = (tid >> 4) * 4, cc = tid & 15;
+    if (tid < 256) {
+      float2 y[4][2] = {};
 #pragma unroll 4
-    for (int i = warp * 4; i < CH; ++i) {
-      const float2 x = *reinterpret_cast<const float2*>(Xs + i * PX + ra);
-      const float4 d = *reinterpret_cast<const float4*>(sDX + i * PX + ca);
-      y0.x = fmaf(x.x, d.x, y0.x); y0.y = fmaf(x.x, d.y, y0.y); y0.z = fmaf(x.x, d.z, y0.z); y0.w = fmaf(x.x, d.w, y0.w);
-      y1.x = fmaf(x.y, d.x, y1.x); y1.y = fmaf(x.y, d.y, y1.y); y1.z = fmaf(x.y, d.z, y1.z); y1.w = fmaf(x.y, d.w, y1.w);
-    }
-    *reinterpret_cast<float4*>(sY + ra * PX + ca) = y0;
-    *reinterpret_cast<float4*>(sY + (ra + 1) * PX + ca) = y1;
-    __syncthreads();
-    const int cb = tid & 15;
-    float s[2][4] = {};
-#pragma unroll 2
-    for (int j = 0; j < warp * 4 + 4; j += 4) {            // X[b][j] is zero for j > b, and b < a
-      const float4 ya = *reinterpret_cast<const float4*>(sY + ra * PX + j), yb = *reinterpret_cast<const float4*>(sY + (ra + 1) * PX + j);
+      for (int i = warp * 8; i < CH; ++i) {                // X[i][a] is zero for i < a
+        const float4 x = *reinterpret_cast<const float4*>(Xs + i * PX + ra), d = *reinterpret_cast<const float4*>(sDX + i * PX + cc * 4);
+        const float2 d0 = make_float2(d.x, d.y), d1 = make_float2(d.z, d.w);
+        const float xa[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float4 x = *reinterpret_cast<const float4*>(Xs + (cb + 16 * e) * PX + j);
-        s[0][e] += ya.x * x.x + ya.y * x.y + ya.z * x.z + ya.w * x.w;
-        s[1][e] += yb.x * x.x + yb.y * x.y + yb.z * x.z + yb.w * x.w;
+        for (int e = 0; e < 4; ++e) {
+          y[e][0] = fma2(make_float2(xa[e], xa[e]), d0, y[e][0]);
+          y[e][1] = fma2(make_float2(xa[e], xa[e]), d1, y[e][1]);
+        }
       }
-    }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      sDX[ra * PX + cb + 16 * e] = -s[0][e];
-      sDX[(ra + 1) * PX + cb + 16 * e] = -s[1][e];
+      for (int e = 0; e < 4; ++e)
+        *reinterpret_cast<float4*>(sY + (ra + e) * PX + cc * 4) = make_float4(y[e][0].x, y[e][0].y, y[e][1].x, y[e][1].y);
+    }
+    __syncthreads();
+    if (tid < 256) {
+      float2 s[4][4] = {};                                 // even and odd j
+#pragma unroll 2
+      for (int j = 0; j < warp * 8 + 8; j += 4) {          // X[b][j] is zero for j > b, and b < a
+        float4 ya[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ya[e] = *reinterpret_cast<const float4*>(sY + (ra + e) * PX + j);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float4 x = *reinterpret_cast<const float4*>(Xs + (cc + 16 * k) * PX + j);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            s[e][k] = fma2(make_float2(ya[e].x, ya[e].y), make_float2(x.x, x.y), s[e][k]);
+            s[e][k] = fma2(make_float2(ya[e].z, ya[e].w), make_float2(x.z, x.w), s[e][k]);
+          }
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sDX[(ra + e) * PX + cc + 16 * k] = -(s[e][k].x + s[e][k].y);
     }
   }
   __syncthreads();
@@ -700,10 +765,13 @@ extern "C" int nsa_gdn_prep(const void* q, const void* k, const void* v, const f
                             void* qk, float* X, float* gc, int B, int T, int H, int K, int V, float scale, cudaStream_t st) {
   if (K != KD || V % 64 || V > 512) return nsa::fail(NSA_ERR_SHAPE, "gdn: key width must be 128, value width a multiple of 64 up to 512");
   const int NC = (T + CH - 1) / CH;
-  PrepParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, g, beta, (bf16*)w, (bf16*)u, (bf16*)qk, X, gc, T, H, NC, V, scale};
+  PrepParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, g, beta, (bf16*)w, (bf16*)u, (bf16*)qk, X, gc, T, H, NC, V, scale, 0};
   const int smem = 2 * CH * PK * 2 + CH * (V + 8) * 2 + 2 * CH * PX * 4 + 2 * CH * 4;
   cudaError_t e = cudaFuncSetAttribute(gdn_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn prep smem attribute");
+  int per_sm = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gdn_prep_kernel, 256, smem);
+  p.resident = per_sm * nsa::sm_count();
   gdn_prep_kernel<<<chunk_grid(B * H, NC), 256, smem, st>>>(p);
   nsa::count_launch();
   e = cudaGetLastError();
@@ -733,7 +801,7 @@ extern "C" int nsa_gdn_post(const void* q, const void* k, const void* v, const v
   if ((rc = nsa::make_tmap_2d_bf16(&tS, S, V, chunks * KD, V, 64, KD))) return rc;
   if ((rc = nsa::make_tmap_2d_bf16(&tdS, dS, V, chunks * KD, V, 64, KD))) return rc;
   PostParams p{(const bf16*)q, (const bf16*)k, beta, gc, X, dgamma, (bf16*)dq, (bf16*)dk, (bf16*)dv, dg, dbeta, B, T, H, NC, V, scale,
-               nsa::status_ptr()};
+               nsa::sm_count(), nsa::status_ptr()};
   cudaError_t e = cudaFuncSetAttribute(gdn_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, POST_SMEM);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn post smem attribute");
   gdn_post_kernel<<<chunk_grid(B * H, NC), 512, POST_SMEM, st>>>(tdu, tdo, tvn, tv, tS, tdS, p);
