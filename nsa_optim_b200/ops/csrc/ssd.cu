@@ -16,6 +16,7 @@
 // chunk_out and chunk_grad are persistent: a CTA walks a run of (chunk, head) items.
 // Decay factors are formed per element in registers (exp2 of a difference that is <= 0), never
 // stored; the [128 x 128] P and dS tiles live only on chip, as bf16 MMA operands.
+#include <algorithm>
 #include "host.cuh"
 #include "tc5.cuh"
 
@@ -116,6 +117,24 @@ __device__ __forceinline__ float chunk_scan(float a, float dt, float* cum, float
   __syncthreads();
   return v;
 }
+
+// Two fp32 lanes per instruction; each lane rounds as the scalar instruction does.
+__device__ __forceinline__ float2 mul2(const float2& a, const float2& b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+        "l"(reinterpret_cast<const unsigned long long&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); }
 
 // OR over the sixteen computing warps of a kernel that has one more
 __device__ __forceinline__ bool compute_any(bool bad) {
@@ -475,7 +494,6 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
     float e_open = 0.f, dsk_open = 0.f;                // exp(cum) and skip weight of the item whose rows are still open
     Items cur(p);
     const int n = cur.n;
-    bool ok = true;
     int seg = 0;
     for (int k = 0; k <= n; ++k, cur.next()) {
       float e = 0.f, dsk = 0.f;
@@ -483,14 +501,14 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
         const int buf = k & 1;
         if (p.Dskip) dsk = p.Dskip[cur.h];             // in flight until the item's rows are finished
         if (cur.opens(k)) {
-          if (!(ok = wait(ms, seg, STATUS_TIMEOUT_TMEM_FULL))) break;
+          if (!wait(ms, seg, STATUS_TIMEOUT_TMEM_FULL)) break;
           tc5::fence_after_sync();
           tld32(lanes + cS + grp * 32, s);
           tc5::fence_before_sync();
           arrive_warp(sread);
           ++seg;
         }
-        if (!(ok = wait(scanned + buf, k >> 1, STATUS_TIMEOUT_SMEM_FULL))) break;
+        if (!wait(scanned + buf, k >> 1, STATUS_TIMEOUT_SMEM_FULL)) break;
         const float* cum = scan + buf * (2 * L + 192);
         const float *dts = cum + L + grp * 32, *cols = cum + grp * 32;
         const float ci = cum[r];
@@ -525,7 +543,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
       }
       if (k > 0) {                                     // rows of the item before, whose products ran meanwhile
         const int q = k - 1, buf = q & 1;
-        if (!(ok = wait(full + q % OUT_ST, q / OUT_ST, STATUS_TIMEOUT_SMEM_FULL) && wait(done + buf, q >> 1, STATUS_TIMEOUT_TMEM_FULL))) break;
+        if (!wait(full + q % OUT_ST, q / OUT_ST, STATUS_TIMEOUT_SMEM_FULL) || !wait(done + buf, q >> 1, STATUS_TIMEOUT_TMEM_FULL)) break;
         tc5::fence_after_sync();
         uint8_t* sX = stages + (q % OUT_ST) * 2 * BOXB;
         float xf[16], yo[16], yi[16];
@@ -969,6 +987,192 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
 }
 
 // ---------------------------------------------------------------------------------------
+// States entering the chunks (BACK: gradients of the states leaving them) in one pass: one CTA per (head, sequence) walks the
+// chunks, the state in registers; only its bf16 copies reach memory, where chunk_state and the state pass move 20 bytes per element
+// of it.  Eight warps scale a chunk's rows of B (C) in place, eight add the product of the chunk before to the state; the others
+// issue, load with the scan of the step sizes, and store.  (Rows of x are half as many elements, but scaled x rounds
+// differently from what the gradients pair it with: dA was a quarter further from its 64-bit value.)
+// ---------------------------------------------------------------------------------------
+constexpr int WALK_ST = 4;                             // stages of B (C) and x (dy)
+constexpr int WALK_SMEM = 1024 + (3 * WALK_ST + 1) * BOXB + WALK_ST * (L + 4) * 4 + 256;
+template <bool BACK>
+__global__ void __launch_bounds__(608, 1)
+ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant__ CUtensorMap tm_v,
+                const __grid_constant__ CUtensorMap tm_out, const SsdParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sOut = smem + 3 * WALK_ST * BOXB;           // [128 n][64 p]
+  float* scale = reinterpret_cast<float*>(sOut + BOXB);      // per stage: row scales, decay of the chunk
+  uint64_t* bars = reinterpret_cast<uint64_t*>(scale + WALK_ST * (L + 4));
+  uint64_t *full = bars, *empty = bars + WALK_ST, *ready = bars + 2 * WALK_ST, *done = ready + 2, *taken = ready + 4;   // [2] each: even and odd chunks
+  uint64_t *oready = ready + 6, *freed = ready + 7;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ready + 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* decay = reinterpret_cast<float*>(tmem_slot + 2);        // [2]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.x, b = blockIdx.y, nc = p.nc;
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < WALK_ST; ++i) { tc5::mbar_init(full + i, 2); tc5::mbar_init(empty + i, 1); }
+    for (int i = 0; i < 2; ++i) { tc5::mbar_init(ready + i, 8); tc5::mbar_init(done + i, 1); tc5::mbar_init(taken + i, 8); }
+    tc5::mbar_init(oready, 8);
+    tc5::mbar_init(freed, 1);
+    tc5::fence_barrier_init();
+  }
+  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 128); tc5::tmem_relinquish(); }
+  tc5::fence_before_sync();
+  __syncthreads();
+  tc5::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  auto wait = [&](uint64_t* bar, int phase, int code) {
+    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+  };
+  auto chunk_of = [&](int i) { return BACK ? nc - 1 - i : i; };
+  const int r = threadIdx.x & 127, half = (warp >> 2) & 1;      // row and half of its columns, for the first sixteen warps
+  if (warp < 8) {                                      // state: row n, columns p = 32 half ..
+    const uint32_t acc = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * 32;
+    float2 st[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) st[j] = make_float2(0.f, 0.f);
+    for (int i = 0; i < nc; ++i) {
+      if (i > 0) {
+        float a[32];
+        if (!wait(done + ((i - 1) & 1), (i - 1) >> 1, STATUS_TIMEOUT_TMEM_FULL)) break;
+        tc5::fence_after_sync();
+        const float g = decay[(i - 1) & 1];            // of the chunk before
+        tld32(acc + ((i - 1) & 1) * 64, a);
+        tc5::fence_before_sync();
+        arrive_warp(taken + ((i - 1) & 1));
+        const float2 g2 = make_float2(g, g);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) st[j] = fma2(g2, st[j], make_float2(a[2 * j], a[2 * j + 1]));
+      }
+      uint32_t pk[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) pk[j] = tc5::pack_bf16(st[j].x, st[j].y);
+      if (i > 0 && !wait(freed, i - 1, STATUS_TIMEOUT_SMEM_EMPTY)) break;
+      st_row32(sOut, r, half * 32, pk);
+      tc5::fence_proxy_async();
+      arrive_warp(oready);
+    }
+  } else if (warp < 16) {                              // row t of B (C), 64 columns
+    for (int i = 0; i + 1 < nc; ++i) {
+      const int s = i % WALK_ST;
+      if (!wait(full + s, i / WALK_ST, STATUS_TIMEOUT_SMEM_FULL)) break;
+      const float sc = scale[s * (L + 4) + r];
+      const float2 f = make_float2(sc, sc);
+      uint8_t* row = smem + (s * 3 + half) * BOXB + r * 128;
+      uint4 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const uint4*>(row + ((j ^ (r & 7)) << 4));
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 a = mul2(unpack2(v[j].x), f), c = mul2(unpack2(v[j].y), f), d = mul2(unpack2(v[j].z), f), e = mul2(unpack2(v[j].w), f);
+        *reinterpret_cast<uint4*>(row + ((j ^ (r & 7)) << 4)) =
+            make_uint4(tc5::pack_bf16(a.x, a.y), tc5::pack_bf16(c.x, c.y), tc5::pack_bf16(d.x, d.y), tc5::pack_bf16(e.x, e.y));
+      }
+      tc5::fence_proxy_async();
+      // the decay goes along to the product's readers, who have taken the one two chunks back
+      if (i > 1 && !wait(taken + (i & 1), (i >> 1) - 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      if (threadIdx.x == 256) decay[i & 1] = scale[s * (L + 4) + L];
+      arrive_warp(ready + (i & 1));
+    }
+  } else if (warp == 16) {
+    constexpr uint32_t idesc = tc5::make_idesc_bf16(128, PD, 1, 1);
+    const bool lead = tc5::elect_one();                // converged warp, elected lane issues (see ssd_chunk_state_kernel)
+    for (int i = 0; i + 1 < nc; ++i) {                 // nothing follows the last chunk
+      const int s = i % WALK_ST;
+      const uint64_t a0 = tc5::desc_mnmajor(tc5::smem_u32(smem + s * 3 * BOXB), BOXB);
+      const uint64_t v0 = tc5::desc_mnmajor(tc5::smem_u32(smem + (s * 3 + 2) * BOXB), BOXB);
+      if (!wait(ready + (i & 1), i >> 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;       // also: the product two chunks back has been taken
+      tc5::fence_after_sync();
+      if (lead) {
+#pragma unroll
+        for (int kk = 0; kk < L / 16; ++kk)
+          tc5::mma_ss(tmem + (i & 1) * 64, a0 + static_cast<uint64_t>((kk * 2048) >> 4), v0 + static_cast<uint64_t>((kk * 2048) >> 4), idesc, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(done + (i & 1));
+        tc5::mma_commit(empty + s);
+      }
+      __syncwarp();
+    }
+  } else if (warp == 17) {
+    const bool lead = tc5::elect_one();
+    const float a = p.A[h];
+    auto load_dt = [&](int i) {
+      const int t = chunk_of(i) * L + 4 * lane;
+      const float* src = p.dt + (static_cast<long>(b) * p.T + t) * p.H + h;
+      return make_float4(t < p.T ? src[0] : 0.f, t + 1 < p.T ? src[p.H] : 0.f, t + 2 < p.T ? src[2 * p.H] : 0.f,
+                         t + 3 < p.T ? src[3 * p.H] : 0.f);
+    };
+    // into L2 a few chunks ahead: the stages alone leave a load from memory less time than it takes
+    constexpr int AHEAD = 8;
+    auto prefetch = [&](int i) {
+      if (i + 1 >= nc || !lead) return;
+      const int t0 = chunk_of(i) * L;
+      tc5::tma_prefetch_4d(&tm_v, 0, h, t0, b);
+      if (i % p.H != h) return;                        // shared by all heads
+      tc5::tma_prefetch_3d(&tm_bc, 0, t0, b);
+      tc5::tma_prefetch_3d(&tm_bc, 64, t0, b);
+    };
+    for (int i = WALK_ST; i < AHEAD; ++i) prefetch(i);
+    bool ok = true;
+    float4 dt = load_dt(0);
+    for (int i = 0; i + 1 < nc; ++i) {
+      const int s = i % WALK_ST, t0 = chunk_of(i) * L;
+      uint8_t* st = smem + s * 3 * BOXB;
+      const float4 dt_next = load_dt(i + 1);
+      if (i >= WALK_ST && !(ok = wait(empty + s, i / WALK_ST - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
+      if (lead) {
+        tc5::mbar_expect_tx(full + s, 3 * BOXB);
+        tc5::tma_load_3d(st, &tm_bc, full + s, 0, t0, b);
+        tc5::tma_load_3d(st + BOXB, &tm_bc, full + s, 64, t0, b);
+        tc5::tma_load_4d(st + 2 * BOXB, &tm_v, full + s, 0, h, t0, b);
+      }
+      prefetch(i + AHEAD);
+      __syncwarp();
+      float4 c = make_float4(dt.x * a, dt.y * a, dt.z * a, dt.w * a);
+      c.y += c.x;
+      c.z += c.y;
+      c.w += c.z;
+      float run = c.w;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float n = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += n;
+      }
+      const float off = run - c.w, tot = __shfl_sync(0xffffffffu, run, 31);
+      auto weight = [&](float cum, float d) { return BACK ? exp2f(cum * LOG2E) : exp2f((tot - cum) * LOG2E) * d; };
+      float* sc = scale + s * (L + 4);
+      *reinterpret_cast<float4*>(sc + 4 * lane) =
+          make_float4(weight(off + c.x, dt.x), weight(off + c.y, dt.y), weight(off + c.z, dt.z), weight(run, dt.w));
+      if (lane == 0) sc[L] = exp2f(tot * LOG2E);
+      arrive_warp(full + s);
+      dt = dt_next;
+    }
+    // stages whose last use was not waited for above
+    for (int i = nc > WALK_ST + 1 ? nc - WALK_ST : 0; i + 1 < nc && ok; ++i) ok = wait(empty + i % WALK_ST, i / WALK_ST, STATUS_TIMEOUT_SMEM_EMPTY);
+    if (!ok && lead)                                   // loads may still be in flight
+      for (int i = 0; i < WALK_ST; ++i) tc5::mbar_drain(full + i);
+    __syncwarp();
+  } else {
+    const bool lead = tc5::elect_one();
+    for (int i = 0; i < nc; ++i) {
+      if (!wait(oready, i, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      if (lead) {
+        tc5::tma_store_2d(&tm_out, sOut, 0, ((b * nc + chunk_of(i)) * p.H + h) * NS);
+        tc5::tma_store_commit();
+        tc5::tma_store_wait_read<0>();
+      }
+      arrive_warp(freed);
+    }
+    if (lead) tc5::tma_store_wait_read<0>();
+    __syncwarp();
+  }
+  tc5::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 128); }
+}
+
+// ---------------------------------------------------------------------------------------
 // State passing over chunks (elementwise).  Layout [B, nc, H, E], E = NS * PD.
 // ---------------------------------------------------------------------------------------
 // A thread walks the chunks of VEC neighbouring elements.  The recurrence itself is one FMA per chunk; what takes time is
@@ -1250,6 +1454,38 @@ extern "C" int nsa_ssd_finish(const float* dB_part, const float* dC_part, const 
   nsa::count_launch(4);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_finish launch");
+}
+
+// One pass over the chunks (nsa_ssd_states) or chunk_state and the state pass.  The walk takes 1.15 us a chunk for up to one head per
+// SM; the two kernels 0.0205 us per (chunk, head), 17 us for two launches at least.  16384 tokens, 64 heads: 141 us
+// against 169; 48: 141 and 121; 24: 140 and 69; two sequences of 8192 x 64: 82 and 162; 1000 tokens x 32: 14 and 19.
+extern "C" int nsa_ssd_states_in_one(int B, int T, int H) {
+  const long heads = static_cast<long>(B) * H, chunks = (T + L - 1) / L, sms = nsa::sm_count();
+  return 1.15 * chunks * ((heads + sms - 1) / sms) + 4. <= std::max(17., 0.0205 * heads * chunks);
+}
+
+// back = 0: bc = B rows, v = x -> states entering the chunks; back = 1: bc = C rows, v = dy -> gradients of the states leaving them.
+// out: bf16 [B, nc, H, N, P].
+extern "C" int nsa_ssd_states(int back, const void* bc, long ld_bc, const void* v, long ld_v, const float* dt, const float* A,
+                              void* out, int B, int T, int H, int N, int P, cudaStream_t st) {
+  int rc = check_dims(N, P, ld_bc, ld_v);
+  if (rc) return rc;
+  SsdParams p{};
+  p.dt = dt; p.A = A; p.B = B; p.T = T; p.H = H; p.nc = (T + L - 1) / L; p.status = nsa::status_ptr();
+  CUtensorMap tb, tv, to;
+  if ((rc = map_bc(&tb, bc, B, T, ld_bc))) return rc;
+  if ((rc = map_v(&tv, v, B, T, H, ld_v))) return rc;
+  if ((rc = map_state(&to, out, static_cast<long>(B) * p.nc * H * NS))) return rc;
+  static bool cfg = false;
+  if (!cfg) {
+    if ((rc = smem_attr(ssd_walk_kernel<true>, WALK_SMEM)) || (rc = smem_attr(ssd_walk_kernel<false>, WALK_SMEM))) return rc;
+    cfg = true;
+  }
+  if (back) ssd_walk_kernel<true><<<dim3(H, B), 608, WALK_SMEM, st>>>(tb, tv, to, p);
+  else ssd_walk_kernel<false><<<dim3(H, B), 608, WALK_SMEM, st>>>(tb, tv, to, p);
+  nsa::count_launch();
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_states launch");
 }
 
 // mode 0: bc = B rows, v = x -> chunk end states and gamma.  mode 1: bc = C rows, v = dy -> G.

@@ -1471,15 +1471,8 @@ class _SSD(torch.autograd.Function):
         A = A.float().contiguous()
         Df = None if D is None else D.float().contiguous()
         dev = x.device
-        S_loc = _empty(Bsz, nc, H, N, P, dtype=torch.float32, device=dev)
-        gamma = _empty(Bsz, nc, H, dtype=torch.float32, device=dev)
         lib = load()
-        _check(lib.nsa_ssd_chunk_state(c_int(0), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(dt), _p(A), _p(S_loc), _p(gamma),
-                                       c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream()))
-        Hb = _empty(Bsz, nc, H, N, P, dtype=torch.bfloat16, device=dev)
-        _check(lib.nsa_ssd_state_fwd(_p(S_loc), _p(gamma), c_void_p(0), _p(Hb), c_void_p(0), c_int(Bsz), c_int(nc), c_int(H),
-                                     c_long(N * P), _stream()))
-        del S_loc
+        Hb, gamma = _SSD.states(lib, False, Bm, ldb, x, ldx, dt, A, None)
         y = _empty(Bsz, T, H, P, dtype=torch.bfloat16, device=dev)
         _check(lib.nsa_ssd_chunk_out(_p(Cm), c_long(ldc), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(Hb), _p(dt), _p(A),
                                      _p(Df), _p(y), c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream()))
@@ -1488,23 +1481,41 @@ class _SSD(torch.autograd.Function):
         return y
 
     @staticmethod
+    def states(lib, back, rows, ld_rows, v, ld_v, dt, A, gamma):
+        """bf16 states entering the chunks (back: gradients of those leaving them), and the chunks' decays where the two-kernel
+        form needs them."""
+        Bsz, T, H, P = v.shape
+        N, nc, dev = rows.shape[-1], -(-T // 128), v.device
+        dims = (c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream())
+        out = _empty(Bsz, nc, H, N, P, dtype=torch.bfloat16, device=dev)
+        if lib.nsa_ssd_states_in_one(c_int(Bsz), c_int(T), c_int(H)):
+            _check(lib.nsa_ssd_states(c_int(back), _p(rows), c_long(ld_rows), _p(v), c_long(ld_v), _p(dt), _p(A), _p(out), *dims))
+            return out, _empty(0, device=dev)
+        if not back:
+            gamma = _empty(Bsz, nc, H, dtype=torch.float32, device=dev)
+        local = _empty(Bsz, nc, H, N, P, dtype=torch.float32, device=dev)
+        _check(lib.nsa_ssd_chunk_state(c_int(back), _p(rows), c_long(ld_rows), _p(v), c_long(ld_v), _p(dt), _p(A), _p(local),
+                                       c_void_p(0) if back else _p(gamma), *dims))
+        if back:
+            _check(lib.nsa_ssd_state_bwd(_p(local), _p(gamma), c_void_p(0), _p(out), c_int(Bsz), c_int(nc), c_int(H), c_long(N * P),
+                                         _stream()))
+        else:
+            _check(lib.nsa_ssd_state_fwd(_p(local), _p(gamma), c_void_p(0), _p(out), c_void_p(0), c_int(Bsz), c_int(nc), c_int(H),
+                                         c_long(N * P), _stream()))
+        return out, gamma
+
+    @staticmethod
     def backward(ctx, dy):
         x, dt, A, Bm, Cm, Df, gamma, Hb = ctx.saved_tensors
         ldx, ldb, ldc = (_row_pitch(t.flatten(2)) for t in (x, Bm, Cm))
         Df = Df if ctx.has_D else None
         Bsz, T, H, P = x.shape
         N = Bm.shape[-1]
-        nc = gamma.shape[1]
+        nc = Hb.shape[1]
         dev = x.device
         dy = dy.contiguous()
         lib = load()
-        G = _empty(Bsz, nc, H, N, P, dtype=torch.float32, device=dev)
-        _check(lib.nsa_ssd_chunk_state(c_int(1), _p(Cm), c_long(ldc), _p(dy), c_long(H * P), _p(dt), _p(A), _p(G), c_void_p(0),
-                                       c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream()))
-        dHn = _empty(Bsz, nc, H, N, P, dtype=torch.bfloat16, device=dev)
-        _check(lib.nsa_ssd_state_bwd(_p(G), _p(gamma), c_void_p(0), _p(dHn), c_int(Bsz), c_int(nc), c_int(H), c_long(N * P),
-                                     _stream()))
-        del G
+        dHn, _ = _SSD.states(lib, True, Cm, ldc, dy, H * P, dt, A, gamma)
         dx = _empty(Bsz, T, H, P, dtype=torch.bfloat16, device=dev)
         # dB / dC: fp32 sums over the heads that one CTA has of a chunk, added up afterwards
         slots = lib.nsa_ssd_grad_slots(c_int(Bsz), c_int(T), c_int(H))

@@ -37,6 +37,14 @@ def test_ssd_sizes(native, B, T, H, skip):
         assert (a.double() - b).norm() < 1e-2 * b.norm() + 1e-6, name
 
 
+# 32 sequences x heads and more: the states come from one walk over the chunks (one chunk, as many as it has stages, more); runs of
+# (chunk, head) items that end inside a chunk, at its end, and go over several
+@pytest.mark.parametrize("B,T,H,skip", [(32, 5, 1, True), (1, 256, 32, True), (2, 384, 16, False), (1, 513, 48, True), (2, 700, 70, True),
+                                        (1, 1100, 33, False)])
+def test_ssd_walk_and_runs(native, B, T, H, skip):
+    test_ssd_sizes(native, B, T, H, skip)
+
+
 @pytest.mark.parametrize("nc,E", [(1, 7), (7, 12), (8, 64), (9, 1000), (30, 8192)])
 @pytest.mark.parametrize("back", [False, True])
 def test_state_pass(native, nc, E, back):
