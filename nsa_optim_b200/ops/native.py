@@ -13,13 +13,14 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import c_float, c_int, c_long, c_longlong, c_void_p
 from typing import Optional, Tuple
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
 
 from . import quant, torch_impl
+from .signatures import declare
 
 _LIB_PATH = os.environ.get("NSA_B200_LIB") or os.path.join(os.path.dirname(os.path.abspath(__file__)), "libnsa_b200.so")
 _lib: Optional[ctypes.CDLL] = None
@@ -71,10 +72,9 @@ def load() -> ctypes.CDLL:
     if _lib is None:
         if not os.path.exists(_LIB_PATH):
             raise FileNotFoundError(f"{_LIB_PATH} is missing; run `python -m nsa_optim_b200.ops.build`")
-        _lib = ctypes.CDLL(_LIB_PATH)
-        _lib.nsa_last_error.restype = ctypes.c_char_p
-        _lib.nsa_launch_count.restype = c_longlong
-        _lib.nsa_conv1d_bwd_parts.restype = c_long
+        lib = ctypes.CDLL(_LIB_PATH)
+        declare(lib)
+        _lib = lib
     return _lib
 
 
@@ -93,17 +93,40 @@ def _check(rc: int) -> None:
         raise RuntimeError(f"nsa_optim_b200 native call failed ({rc}): {load().nsa_last_error().decode()}")
 
 
-def _stream() -> c_void_p:
+def _stream() -> int:
     # the raw handle of the current stream; torch.cuda.current_stream() builds a Stream object for it each time
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _p(t: Optional[Tensor]) -> c_void_p:
-    return c_void_p(0 if t is None else t.data_ptr())
+def _p(t: Optional[Tensor]) -> Optional[int]:
+    return None if t is None else t.data_ptr()
+
+
+class _NoRecord:
+    """Stands in for an autograd context where nothing will be differentiated."""
+    needs_input_grad = (False,) * 32
+
+    def save_for_backward(self, *tensors):
+        pass
+
+    mark_non_differentiable = save_for_backward
+
+
+def _run(fn, *args):
+    """fn.apply(*args); where autograd has nothing to record, the forward alone (a third of the host time of a small op).
+    Transforms, forward-mode derivatives and tracers see the function as before."""
+    if torch.is_grad_enabled():
+        for a in args:
+            if isinstance(a, Tensor) and a.requires_grad:
+                return fn.apply(*args)
+    if (torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0 or torch._C._is_tracing()
+            or torch.compiler.is_compiling()):
+        return fn.apply(*args)
+    return fn.forward(_NoRecord(), *args)
 
 
 def launch_count() -> int:
-    return int(load().nsa_launch_count())
+    return load().nsa_launch_count()
 
 
 def reset_launch_count() -> None:
@@ -111,8 +134,8 @@ def reset_launch_count() -> None:
 
 
 def read_status(reset: bool = True) -> Tuple[int, int, int, int]:
-    out = (c_int * 4)()
-    _check(load().nsa_status_read(out, c_int(1 if reset else 0)))
+    out = (ctypes.c_int * 4)()
+    _check(load().nsa_status_read(out, 1 if reset else 0))
     return tuple(int(v) for v in out)
 
 
@@ -205,7 +228,8 @@ def check_status(sync: bool = True) -> None:
 # --------------------------------------------------------------------------------------
 def _as_2d(x: Tensor) -> Tensor:
     x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
-    if x2.stride(-1) != 1 or (x2.stride(0) % 8) or (x2.data_ptr() % 16):
+    pitch, step = x2.stride()
+    if step != 1 or pitch % 8 or x2.data_ptr() % 16:
         x2 = x2.contiguous()
     return x2
 
@@ -258,15 +282,15 @@ def gemm(a: Tensor, b: Tensor, a_mn: bool, b_mn: bool, out: Optional[Tensor] = N
                 ws.zero_()
         else:
             ws = out.float() if accumulate else _zeros(M, N, dtype=torch.float32, device=a.device)
-        _check(load().nsa_gemm_bf16_splitk(_p(a), _p(b), _p(ws), c_int(M), c_int(N), c_int(K), c_int(a.stride(0)),
-                                           c_int(b.stride(0)), c_int(ws.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)),
-                                           c_int(split_k), _stream()))
+        _check(load().nsa_gemm_bf16_splitk(_p(a), _p(b), _p(ws), M, N, K, a.stride(0),
+                                           b.stride(0), ws.stride(0), int(a_mn), int(b_mn),
+                                           split_k, _stream()))
         if not direct:
             out.copy_(ws)
         return out
-    _check(load().nsa_gemm_bf16(_p(a), _p(b), _p(out), c_int(M), c_int(N), c_int(K), c_int(a.stride(0)),
-                                c_int(b.stride(0)), c_int(out.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)),
-                                c_int(int(out.dtype == torch.float32)), c_int(int(accumulate)), c_int(max_ctas),
+    _check(load().nsa_gemm_bf16(_p(a), _p(b), _p(out), M, N, K, a.stride(0),
+                                b.stride(0), out.stride(0), int(a_mn), int(b_mn),
+                                int(out.dtype == torch.float32), int(accumulate), max_ctas,
                                 _stream()))
     return out
 
@@ -276,7 +300,7 @@ def gemm_select(which: str = "default") -> None:
     (one CTA per 128 x 256 tile) or "default" (pair unless NSA_B200_GEMM=single)."""
     global _gemm_which
     _gemm_which = which
-    load().nsa_gemm_select(c_int({"default": 0, "single": 1, "pair": 2}[which]))
+    load().nsa_gemm_select({"default": 0, "single": 1, "pair": 2}[which])
 
 
 def _project(x2: Tensor, w: Tensor, lead) -> Tensor:
@@ -360,7 +384,7 @@ def multi_linear(x: Tensor, ws) -> tuple:
             run = pg[2]
         else:
             flush_pending_gather()
-    return _MultiLinear.apply(x, run, *ws)
+    return _run(_MultiLinear, x, run, *ws)
 
 
 # A sharded unit may defer its all-gather to the first matmul that touches one of its weights:
@@ -417,9 +441,9 @@ def linear(x: Tensor, w: Tensor) -> Tensor:
     pg = _pending_gather
     if pg is not None:
         if pg[0] <= w.data_ptr() < pg[1] and w.is_contiguous():
-            return _LinearGather.apply(x, w, pg[2])
+            return _run(_LinearGather, x, w, pg[2])
         flush_pending_gather()
-    return _Linear.apply(x, w)
+    return _run(_Linear, x, w)
 
 
 # --------------------------------------------------------------------------------------
@@ -429,8 +453,8 @@ def _rms_fwd(x2, gate2, w, eps, mode):
     rows, d = x2.shape
     y = _empty_like(x2)
     rstd = _empty(rows, dtype=torch.float32, device=x2.device)
-    _check(load().nsa_rmsnorm_fwd(_p(x2), _p(gate2), _p(w), _p(y), _p(rstd), c_long(rows), c_int(d),
-                                  c_float(eps), c_int(mode), _stream()))
+    _check(load().nsa_rmsnorm_fwd(_p(x2), _p(gate2), _p(w), _p(y), _p(rstd), rows, d,
+                                  eps, mode, _stream()))
     return y, rstd
 
 
@@ -439,10 +463,10 @@ def _rms_bwd(x2, gate2, w, dy2, rstd, mode):
     dx = _empty_like(x2)
     dg = _empty_like(x2) if mode != 0 else None
     dw = _empty(d, dtype=torch.bfloat16, device=x2.device)
-    parts = int(load().nsa_rmsnorm_bwd_parts(c_long(rows), c_int(d)))
+    parts = load().nsa_rmsnorm_bwd_parts(rows, d)
     partial = _empty(parts * d, dtype=torch.float32, device=x2.device)
-    _check(load().nsa_rmsnorm_bwd(_p(x2), _p(gate2), _p(w), _p(dy2), _p(rstd), _p(dx), _p(dg), _p(dw), c_void_p(0),
-                                  _p(partial), c_long(rows), c_int(d), c_int(mode), _stream()))
+    _check(load().nsa_rmsnorm_bwd(_p(x2), _p(gate2), _p(w), _p(dy2), _p(rstd), _p(dx), _p(dg), _p(dw), None,
+                                  _p(partial), rows, d, mode, _stream()))
     return dx, dg, dw
 
 
@@ -467,10 +491,10 @@ def _rms_bwd_res(x2, w, dy2, rstd, dres2):
     rows, d = x2.shape
     dx = _empty_like(x2)
     dw = _empty(d, dtype=torch.bfloat16, device=x2.device)
-    parts = int(load().nsa_rmsnorm_bwd_parts(c_long(rows), c_int(d)))
+    parts = load().nsa_rmsnorm_bwd_parts(rows, d)
     partial = _empty(parts * d, dtype=torch.float32, device=x2.device)
-    _check(load().nsa_rmsnorm_bwd_res(_p(x2), _p(w), _p(dy2), _p(rstd), _p(dres2), _p(dx), _p(dw), c_void_p(0),
-                                      _p(partial), c_long(rows), c_int(d), _stream()))
+    _check(load().nsa_rmsnorm_bwd_res(_p(x2), _p(w), _p(dy2), _p(rstd), _p(dres2), _p(dx), _p(dw), None,
+                                      _p(partial), rows, d, _stream()))
     return dx, dw
 
 
@@ -520,8 +544,8 @@ class _AddRMSNorm(torch.autograd.Function):
         h = _empty_like(x2)
         y = _empty_like(x2)
         rstd = _empty(rows, dtype=torch.float32, device=x2.device)
-        _check(load().nsa_rmsnorm_add_fwd(_p(x2), _p(r2), _p(wb), _p(h), _p(y), _p(rstd), c_long(rows), c_int(d),
-                                          c_float(eps), _stream()))
+        _check(load().nsa_rmsnorm_add_fwd(_p(x2), _p(r2), _p(wb), _p(h), _p(y), _p(rstd), rows, d,
+                                          eps, _stream()))
         ctx.save_for_backward(h, wb, rstd)
         ctx.wdtype = w.dtype
         return h.view(x.shape), y.view(x.shape)
@@ -537,14 +561,14 @@ def rms_norm_skip(x, w, eps=1e-6):
     if x.shape[-1] % 8 or x.shape[-1] > 8192:
         _fallback("rms_norm_skip")
         return torch_impl.rms_norm_skip(x, w, eps)
-    return _RMSNormSkip.apply(x, w, eps)
+    return _run(_RMSNormSkip, x, w, eps)
 
 
 def add_rms_norm(x, r, w, eps=1e-6):
     if x.shape[-1] % 8 or x.shape[-1] > 8192 or x.shape != r.shape:
         _fallback("add_rms_norm")
         return torch_impl.add_rms_norm(x, r, w, eps)
-    return _AddRMSNorm.apply(x, r, w, eps)
+    return _run(_AddRMSNorm, x, r, w, eps)
 
 
 def _gate_rows(gate: Tensor):
@@ -581,8 +605,8 @@ class _GatedRMSNorm(torch.autograd.Function):
         rows, d = x2.shape
         y = _empty_like(x2)
         rstd = _empty(rows, dtype=torch.float32, device=x2.device)
-        _check(load().nsa_rmsnorm_fwd_ldg(_p(x2), _p(g2), c_long(ldg), _p(wb), _p(y), _p(rstd), c_long(rows), c_int(d),
-                                          c_float(eps), c_int(mode), _stream()))
+        _check(load().nsa_rmsnorm_fwd_ldg(_p(x2), _p(g2), ldg, _p(wb), _p(y), _p(rstd), rows, d,
+                                          eps, mode, _stream()))
         ctx.save_for_backward(x2, g2, wb, rstd)
         ctx.mode, ctx.wdtype, ctx.gshape = mode, w.dtype, gate.shape
         return y.view(x.shape)
@@ -594,10 +618,10 @@ class _GatedRMSNorm(torch.autograd.Function):
         dy2 = dy.reshape(x2.shape).contiguous()
         dx, dg = _empty_like(x2), _empty_like(x2)
         dw = _empty(d, dtype=torch.bfloat16, device=x2.device)
-        parts = int(load().nsa_rmsnorm_bwd_parts(c_long(rows), c_int(d)))
+        parts = load().nsa_rmsnorm_bwd_parts(rows, d)
         partial = _empty(parts * d, dtype=torch.float32, device=x2.device)
-        _check(load().nsa_rmsnorm_bwd_ldg(_p(x2), _p(g2), c_long(_row_pitch(g2)), _p(wb), _p(dy2), _p(rstd), _p(dx), _p(dg), _p(dw),
-                                          c_void_p(0), _p(partial), c_long(rows), c_int(d), c_int(ctx.mode), _stream()))
+        _check(load().nsa_rmsnorm_bwd_ldg(_p(x2), _p(g2), _row_pitch(g2), _p(wb), _p(dy2), _p(rstd), _p(dx), _p(dg), _p(dw),
+                                          None, _p(partial), rows, d, ctx.mode, _stream()))
         return dx.view(dy.shape), dg.view(ctx.gshape), dw.to(ctx.wdtype), None, None
 
 
@@ -606,7 +630,7 @@ def rms_norm(x, w, eps=1e-6):
     if d % 8 or d > 8192:
         _fallback("rms_norm")
         return torch_impl.rms_norm(x, w, eps)
-    return _RMSNorm.apply(x, w, eps)
+    return _run(_RMSNorm, x, w, eps)
 
 
 def gated_rms_norm(x, gate, w, eps=1e-6, norm_before_gate=True):
@@ -614,7 +638,7 @@ def gated_rms_norm(x, gate, w, eps=1e-6, norm_before_gate=True):
     if d % 8 or d > 8192:
         _fallback("gated_rms_norm")
         return torch_impl.gated_rms_norm(x, gate, w, eps, norm_before_gate)
-    return _GatedRMSNorm.apply(x, gate, w, eps, norm_before_gate)
+    return _run(_GatedRMSNorm, x, gate, w, eps, norm_before_gate)
 
 
 class _L2Norm(torch.autograd.Function):
@@ -624,7 +648,7 @@ class _L2Norm(torch.autograd.Function):
         rows, d = x2.shape
         y = _empty_like(x2)
         rinv = _empty(rows, dtype=torch.float32, device=x.device)
-        _check(load().nsa_l2norm_fwd(_p(x2), _p(y), _p(rinv), c_long(rows), c_int(d), c_float(eps), _stream()))
+        _check(load().nsa_l2norm_fwd(_p(x2), _p(y), _p(rinv), rows, d, eps, _stream()))
         ctx.save_for_backward(y, rinv)
         return y.view(x.shape)
 
@@ -633,7 +657,7 @@ class _L2Norm(torch.autograd.Function):
         y, rinv = ctx.saved_tensors
         dy2 = dy.reshape(y.shape).contiguous()
         dx = _empty_like(y)
-        _check(load().nsa_l2norm_bwd(_p(y), _p(dy2), _p(rinv), _p(dx), c_long(y.shape[0]), c_int(y.shape[1]), _stream()))
+        _check(load().nsa_l2norm_bwd(_p(y), _p(dy2), _p(rinv), _p(dx), y.shape[0], y.shape[1], _stream()))
         return dx.view(dy.shape), None
 
 
@@ -642,7 +666,7 @@ def l2_norm(x, eps=1e-6):
     if d % 8 or d > 512:
         _fallback("l2_norm")
         return torch_impl.l2_norm(x, eps)
-    return _L2Norm.apply(x, eps)
+    return _run(_L2Norm, x, eps)
 
 
 # --------------------------------------------------------------------------------------
@@ -661,8 +685,8 @@ class _SwiGLU(torch.autograd.Function):
         g2, u2 = _rows_view(gate), _rows_view(up)
         rows, cols = g2.shape
         y = _empty(rows, cols, dtype=gate.dtype, device=gate.device)
-        _check(load().nsa_swiglu_fwd(_p(g2), _p(u2), _p(y), c_long(rows), c_int(cols), c_long(g2.stride(0)),
-                                     c_long(u2.stride(0)), _stream()))
+        _check(load().nsa_swiglu_fwd(_p(g2), _p(u2), _p(y), rows, cols, g2.stride(0),
+                                     u2.stride(0), _stream()))
         ctx.save_for_backward(g2, u2)
         return y.view(gate.shape)
 
@@ -673,8 +697,8 @@ class _SwiGLU(torch.autograd.Function):
         dy2 = dy.reshape(rows, cols).contiguous()
         dg = _empty(rows, cols, dtype=dy.dtype, device=dy.device)
         du = _empty(rows, cols, dtype=dy.dtype, device=dy.device)
-        _check(load().nsa_swiglu_bwd(_p(g2), _p(u2), _p(dy2), _p(dg), _p(du), c_long(rows), c_int(cols),
-                                     c_long(g2.stride(0)), c_long(u2.stride(0)), c_long(cols), _stream()))
+        _check(load().nsa_swiglu_bwd(_p(g2), _p(u2), _p(dy2), _p(dg), _p(du), rows, cols,
+                                     g2.stride(0), u2.stride(0), cols, _stream()))
         return dg.view(dy.shape), du.view(dy.shape)
 
 
@@ -682,15 +706,15 @@ def swiglu(gate, up):
     if gate.shape[-1] % 8:
         _fallback("swiglu")
         return torch_impl.swiglu(gate, up)
-    return _SwiGLU.apply(gate, up)
+    return _run(_SwiGLU, gate, up)
 
 
 def _rope_call(x: Tensor, cos: Tensor, sin: Tensor, backward: bool) -> Tensor:
     B, T, H, D = x.shape
     xc = x.contiguous()
     y = _empty_like(xc)
-    _check(load().nsa_rope(_p(xc), _p(cos), _p(sin), _p(y), c_long(B), c_int(T), c_int(H), c_int(D),
-                           c_int(int(backward)), _stream()))
+    _check(load().nsa_rope(_p(xc), _p(cos), _p(sin), _p(y), B, T, H, D,
+                           int(backward), _stream()))
     return y
 
 
@@ -712,7 +736,7 @@ def rope(x, cos, sin):
     if x.shape[-1] % 16 or cos.shape[0] != x.shape[1]:
         _fallback("rope")
         return torch_impl.rope(x, cos, sin)
-    return _RoPE.apply(x, cos, sin)
+    return _run(_RoPE, x, cos, sin)
 
 
 # --------------------------------------------------------------------------------------
@@ -727,8 +751,8 @@ class _Conv1d(torch.autograd.Function):
         wb = weight.to(torch.bfloat16).contiguous()
         bb = None if bias is None else bias.to(torch.bfloat16).contiguous()
         y = _empty(B, T, C, dtype=x.dtype, device=x.device)
-        _check(load().nsa_conv1d_fwd(_p(xv), _p(wb), _p(bb), _p(y), c_int(B), c_int(T), c_int(C),
-                                     c_long(xv.stride(1)), c_int(weight.shape[-1]), c_int(int(activation)), _stream()))
+        _check(load().nsa_conv1d_fwd(_p(xv), _p(wb), _p(bb), _p(y), B, T, C,
+                                     xv.stride(1), weight.shape[-1], int(activation), _stream()))
         ctx.save_for_backward(xv, wb, bb)
         ctx.activation, ctx.wdtype = activation, weight.dtype
         ctx.has_bias = bias is not None
@@ -741,14 +765,14 @@ class _Conv1d(torch.autograd.Function):
         W = wb.shape[-1]
         dyc = dy.contiguous()
         dx = _empty(B, T, C, dtype=dy.dtype, device=dy.device)
-        parts = int(load().nsa_conv1d_bwd_parts(c_int(B), c_int(T), c_int(C)))
+        parts = load().nsa_conv1d_bwd_parts(B, T, C)
         partial = _empty(parts * (W + 1) * C, dtype=torch.float32, device=dy.device)
         out = ctx.wdtype if ctx.wdtype == torch.bfloat16 else torch.float32
         dw = _empty(C, W, dtype=out, device=dy.device)
         db = _empty(C, dtype=out, device=dy.device) if ctx.has_bias else None
         _check(load().nsa_conv1d_bwd(_p(xv), _p(wb), _p(bb), _p(dyc), _p(dx), _p(partial), _p(dw), _p(db),
-                                     c_int(int(out == torch.float32)), c_int(B), c_int(T), c_int(C), c_long(xv.stride(1)),
-                                     c_int(W), c_int(int(ctx.activation)), _stream()))
+                                     int(out == torch.float32), B, T, C, xv.stride(1),
+                                     W, int(ctx.activation), _stream()))
         dw = dw.to(ctx.wdtype)
         db = db.to(ctx.wdtype) if ctx.has_bias else None
         return dx, dw, db, None
@@ -758,7 +782,7 @@ def causal_conv1d(x, weight, bias, activation=True):
     if x.shape[-1] % 8 or weight.shape[-1] != 4:
         _fallback("causal_conv1d")
         return torch_impl.causal_conv1d(x, weight, bias, activation)
-    return _Conv1d.apply(x, weight, bias, activation)
+    return _run(_Conv1d, x, weight, bias, activation)
 
 
 # --------------------------------------------------------------------------------------
@@ -770,7 +794,7 @@ class _Embedding(torch.autograd.Function):
         flat = ids.reshape(-1).contiguous()
         n, d = flat.numel(), weight.shape[1]
         y = _empty(n, d, dtype=weight.dtype, device=weight.device)
-        _check(load().nsa_embedding_fwd(_p(flat), _p(weight), _p(y), c_long(n), c_int(d), c_long(weight.shape[0]), _stream()))
+        _check(load().nsa_embedding_fwd(_p(flat), _p(weight), _p(y), n, d, weight.shape[0], _stream()))
         ctx.save_for_backward(flat)
         ctx.wshape, ctx.wdtype = weight.shape, weight.dtype
         return y.view(*ids.shape, d)
@@ -782,7 +806,7 @@ class _Embedding(torch.autograd.Function):
         sorted_ids, perm = torch.sort(flat, stable=True)
         dw = _zeros(ctx.wshape, dtype=torch.float32, device=dy.device)
         dy2 = dy.reshape(n, d).contiguous()
-        _check(load().nsa_embedding_bwd(_p(sorted_ids), _p(perm), _p(dy2), _p(dw), c_long(n), c_int(d), _stream()))
+        _check(load().nsa_embedding_bwd(_p(sorted_ids), _p(perm), _p(dy2), _p(dw), n, d, _stream()))
         return None, dw.to(ctx.wdtype)
 
 
@@ -790,7 +814,7 @@ def embedding(ids, weight):
     if weight.shape[1] % 8 or ids.dtype != torch.long:
         _fallback("embedding")
         return torch_impl.embedding(ids, weight)
-    return _Embedding.apply(ids, weight)
+    return _run(_Embedding, ids, weight)
 
 
 # --------------------------------------------------------------------------------------
@@ -819,9 +843,9 @@ class _LinearCE(torch.autograd.Function):
             s1 = min(N, s0 + chunk)
             lg = logits[: s1 - s0]
             gemm(h[s0:s1], weight, False, False, out=lg)
-            _check(load().nsa_cross_entropy(_p(lg), _p(labels[s0:s1]), _p(loss_rows[s0:s1]), _p(inv), c_long(s1 - s0),
-                                            c_int(V), c_long(lg.stride(0)), c_long(ignore_index),
-                                            c_int(int(need_h or need_w)), _stream()))
+            _check(load().nsa_cross_entropy(_p(lg), _p(labels[s0:s1]), _p(loss_rows[s0:s1]), _p(inv), s1 - s0,
+                                            V, lg.stride(0), ignore_index,
+                                            int(need_h or need_w), _stream()))
             if need_h:
                 gemm(lg, weight, False, True, out=dh[s0:s1])                   # dlogits (n,V) @ W (V,d)
             if need_w:
@@ -846,7 +870,7 @@ def _scaled_by(t: Tensor, s: Tensor, dtype: torch.dtype) -> Tensor:
         return (t * s).to(dtype)
     out = _empty(t.shape, dtype=dtype, device=t.device)
     sf = s.reshape(1).float()
-    _check(load().nsa_scale_bf16(_p(t), _p(out), _p(sf), c_long(t.numel()), c_int(int(t.dtype == torch.float32)), _stream()))
+    _check(load().nsa_scale_bf16(_p(t), _p(out), _p(sf), t.numel(), int(t.dtype == torch.float32), _stream()))
     return out
 
 
@@ -854,7 +878,7 @@ def linear_cross_entropy(hidden, weight, labels, ignore_index=-100, chunk=4096):
     if hidden.shape[-1] % 8 or weight.shape[0] % 8:
         _fallback("linear_cross_entropy")
         return torch_impl.linear_cross_entropy(hidden, weight, labels, ignore_index, chunk)
-    return _LinearCE.apply(hidden, weight, labels, ignore_index, chunk)
+    return _run(_LinearCE, hidden, weight, labels, ignore_index, chunk)
 
 
 # --------------------------------------------------------------------------------------
@@ -882,7 +906,7 @@ def _adamw_words(items, block: int) -> ctypes.Array:
             _require_numel("exp_avg_sq_absmax", b, na)
         words += (p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), 0 if a is None else a.data_ptr(),
                   0 if b is None else b.data_ptr(), n)
-    return (c_longlong * len(words))(*words)
+    return (ctypes.c_longlong * len(words))(*words)
 
 
 def adamw_multi(items, step, lr, b1, b2, eps, wd, grad_scale) -> None:
@@ -890,9 +914,9 @@ def adamw_multi(items, step, lr, b1, b2, eps, wd, grad_scale) -> None:
     p, g = items[0][:2]
     words = _adamw_words(items, 0)
     gs = None if grad_scale is None else grad_scale.reshape(1).float()
-    _check(load().nsa_adamw_multi(words, c_int(len(items)), _p(gs), c_int(int(p.dtype == torch.float32)),
-                                  c_int(int(g.dtype == torch.float32)), c_int(step), c_float(lr), c_float(b1), c_float(b2),
-                                  c_float(eps), c_float(wd), _stream()))
+    _check(load().nsa_adamw_multi(words, len(items), _p(gs), int(p.dtype == torch.float32),
+                                  int(g.dtype == torch.float32), step, lr, b1, b2,
+                                  eps, wd, _stream()))
 
 
 def adamw8bit_multi(items, step, lr, b1, b2, eps, wd, grad_scale, block) -> None:
@@ -907,9 +931,9 @@ def adamw8bit_multi(items, step, lr, b1, b2, eps, wd, grad_scale, block) -> None
     gs = None if grad_scale is None else grad_scale.reshape(1).float()
     cs = quant.codebook(8, True, p.device)
     cu = quant.codebook(8, False, p.device)
-    _check(load().nsa_adamw8bit_multi(words, c_int(len(items)), _p(cs), _p(cu), _p(gs), c_int(int(p.dtype == torch.float32)),
-                                      c_int(int(g.dtype == torch.float32)), c_int(step), c_float(lr), c_float(b1),
-                                      c_float(b2), c_float(eps), c_float(wd), _stream()))
+    _check(load().nsa_adamw8bit_multi(words, len(items), _p(cs), _p(cu), _p(gs), int(p.dtype == torch.float32),
+                                      int(g.dtype == torch.float32), step, lr, b1,
+                                      b2, eps, wd, _stream()))
 
 
 def adamw_step(p, g, m, v, master, step, lr, b1, b2, eps, wd, grad_scale):
@@ -942,7 +966,7 @@ class _GatedDelta(torch.autograd.Function):
         v_new = _empty(BH, nc, 64, V, dtype=bf, device=dev) if train else None
         S = _empty(BH, nc, K, V, dtype=bf, device=dev) if train else None
         lib, st = load(), _stream()
-        dims = (c_int(B), c_int(T), c_int(H), c_int(K), c_int(V), c_float(scale), st)
+        dims = (B, T, H, K, V, scale, st)
         _check(lib.nsa_gdn_prep(_p(q), _p(k), _p(v), _p(g), _p(beta), _p(w), _p(u), _p(qk), _p(X), _p(gc), *dims))
         _check(lib.nsa_gdn_seq_fwd(_p(q), _p(k), _p(w), _p(u), _p(qk), _p(gc), _p(o), _p(v_new), _p(S), *dims))
         if train:
@@ -963,7 +987,7 @@ class _GatedDelta(torch.autograd.Function):
         dq, dk, dv = _empty_like(q), _empty_like(k), _empty_like(v)
         dg, dbeta = _empty_like(beta), _empty_like(beta)
         lib, st = load(), _stream()
-        dims = (c_int(B), c_int(T), c_int(H), c_int(K), c_int(V), c_float(ctx.scale), st)
+        dims = (B, T, H, K, V, ctx.scale, st)
         _check(lib.nsa_gdn_seq_bwd(_p(q), _p(k), _p(w), _p(qk), _p(S), _p(do), _p(gc), _p(du), _p(dS), _p(dgamma), *dims))
         _check(lib.nsa_gdn_post(_p(q), _p(k), _p(v), _p(do), _p(beta), _p(gc), _p(X), _p(v_new), _p(du), _p(S), _p(dS), _p(dgamma),
                                 _p(dq), _p(dk), _p(dv), _p(dg), _p(dbeta), *dims))
@@ -987,7 +1011,7 @@ def gated_delta_rule(q, k, v, g, beta, scale=None, chunk=64):
     scale = K ** -0.5 if scale is None else scale
     bf = torch.bfloat16
     args = [_dense16(q), _dense16(k.to(bf)), v.to(bf), g.float().contiguous(), beta.float().contiguous()]
-    outs = [_GatedDelta.apply(args[0], args[1], _dense16(part), args[3], args[4], float(scale))
+    outs = [_run(_GatedDelta, args[0], args[1], _dense16(part), args[3], args[4], float(scale))
             for part in (args[2].split(512, -1) if V > 512 else (args[2],))]
     o = outs[0] if len(outs) == 1 else torch.cat(outs, -1)
     return o.to(v.dtype)
@@ -1003,9 +1027,9 @@ def _attn_forward(q, k, v, causal, window, scale, kp_stride, kp_off, tiles):
     o = _empty_like(q)
     L = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
     tb, tm, tc, mu = tiles[:4] if tiles is not None else (None, None, None, 0)
-    _check(load().nsa_attn_fwd(_p(q), _p(k), _p(v), _p(o), _p(L), c_int(B), c_int(T), c_int(S), c_int(Hq),
-                               c_int(Hkv), c_int(D), c_float(scale), c_int(int(causal)), c_int(window),
-                               c_int(kp_stride), c_int(kp_off), _p(tb), _p(tm), _p(tc), c_int(mu), _stream()))
+    _check(load().nsa_attn_fwd(_p(q), _p(k), _p(v), _p(o), _p(L), B, T, S, Hq,
+                               Hkv, D, scale, int(causal), window,
+                               kp_stride, kp_off, _p(tb), _p(tm), _p(tc), mu, _stream()))
     return o, L
 
 
@@ -1025,10 +1049,10 @@ def _attn_backward_split(q, k, v, o, do, L, dq, dk, dv, causal, window, scale, k
         visits = int(os.environ.get('NSA_B200_KV_VISITS_SEL', '64'))
         inv = inverse_blocks(idx, nS, 128 // (Hq // Hkv), visits)
     _check(load().nsa_attn_bwd_split(_p(q), _p(k), _p(v), _p(o), _p(do), _p(L), _p(delta), _p(dq), _p(dk), _p(dv),
-                                     c_int(B), c_int(T), c_int(S), c_int(Hq), c_int(Hkv), c_int(D), c_float(scale),
-                                     c_int(int(causal)), c_int(window), c_int(kp_stride), c_int(kp_off),
-                                     _p(tb), _p(tm), _p(tc), c_int(mu), _p(inv[0]), _p(inv[1]), _p(inv[2]),
-                                     c_int(inv[3]), c_int(inv[4]), c_int(visits), c_int(int(given)), c_int(int(add_dq)),
+                                     B, T, S, Hq, Hkv, D, scale,
+                                     int(causal), window, kp_stride, kp_off,
+                                     _p(tb), _p(tm), _p(tc), mu, _p(inv[0]), _p(inv[1]), _p(inv[2]),
+                                     inv[3], inv[4], visits, int(given), int(add_dq),
                                      _stream()))
 
 
@@ -1073,9 +1097,9 @@ class _Attn(torch.autograd.Function):
             tb, tm, tc, mu = ctx.tiles[:4] if ctx.tiles is not None else (None, None, None, 0)
             delta = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
             _check(load().nsa_attn_bwd(_p(q), _p(k), _p(v), _p(o), _p(do), _p(L), _p(delta), _p(dq), _p(dk), _p(dv),
-                                       c_int(B), c_int(T), c_int(S), c_int(Hq), c_int(Hkv), c_int(D), c_float(scale),
-                                       c_int(int(causal)), c_int(window), c_int(kp_stride), c_int(kp_off),
-                                       _p(tb), _p(tm), _p(tc), c_int(mu), _stream()))
+                                       B, T, S, Hq, Hkv, D, scale,
+                                       int(causal), window, kp_stride, kp_off,
+                                       _p(tb), _p(tm), _p(tc), mu, _stream()))
         return dq, dk.to(k.dtype), dv.to(v.dtype), None, None, None, None, None, None
 
 
@@ -1090,7 +1114,7 @@ def attention(q, k, v, causal=True, window=0, scale=None):
         _fallback("attention")
         return torch_impl.attention(q, k, v, causal, window, scale)
     scale = q.shape[-1] ** -0.5 if scale is None else scale
-    return _Attn.apply(q, k, v, causal, int(window), float(scale), 1, 0, None)[0]
+    return _run(_Attn, q, k, v, causal, int(window), float(scale), 1, 0, None)[0]
 
 
 def union_blocks(idx: Tensor, G: int, nS: int):
@@ -1104,8 +1128,8 @@ def union_blocks(idx: Tensor, G: int, nS: int):
     tb = _empty(B, Hkv, nqt, max_u, dtype=torch.int32, device=idx.device)
     tm = _empty(B, Hkv, nqt, max_u, dtype=torch.int64, device=idx.device)
     tc = _empty(B, Hkv, nqt, dtype=torch.int32, device=idx.device)
-    _check(load().nsa_union_blocks(_p(idx), _p(tb), _p(tm), _p(tc), c_int(B), c_int(T), c_int(Hkv), c_int(G),
-                                   c_int(top_n), c_int(nS), c_int(max_u), _stream()))
+    _check(load().nsa_union_blocks(_p(idx), _p(tb), _p(tm), _p(tc), B, T, Hkv, G,
+                                   top_n, nS, max_u, _stream()))
     return tb, tm, tc, max_u
 
 
@@ -1118,14 +1142,14 @@ def inverse_blocks(idx: Tensor, nS: int, R: int, visits_per_cta: int):
     dev = idx.device
     idx = idx.to(torch.int32).contiguous()
     lists = B * Hkv * nS
-    chunks = int(load().nsa_inverse_chunks(c_int(B * Hkv), c_int(T), c_int(nS)))
+    chunks = load().nsa_inverse_chunks(B * Hkv, T, nS)
     tok = _empty(B * Hkv * T * n, dtype=torch.int32, device=dev)
     list_start = _empty(lists + 1, dtype=torch.int32, device=dev)
     item_start = _empty(lists + 1, dtype=torch.int32, device=dev)
     hist = _empty(B * Hkv * chunks * nS, dtype=torch.int32, device=dev)
     count = _empty(lists, dtype=torch.int32, device=dev)
-    _check(load().nsa_inverse_blocks(_p(idx), _p(tok), _p(list_start), _p(item_start), _p(hist), _p(count), c_int(B * Hkv),
-                                     c_int(T), c_int(n), c_int(nS), c_int(R), c_int(visits_per_cta), _stream()))
+    _check(load().nsa_inverse_blocks(_p(idx), _p(tok), _p(list_start), _p(item_start), _p(hist), _p(count), B * Hkv,
+                                     T, n, nS, R, visits_per_cta, _stream()))
     bound = (B * Hkv * T * n) // (R * visits_per_cta) + lists
     return tok, list_start, item_start, nS, bound
 
@@ -1164,7 +1188,7 @@ def selected_attention(q, k, v, idx, scale=None):
     nS = -(-k.shape[1] // 64)
     idx = idx.to(torch.int32).contiguous()
     tiles = union_blocks(idx, G, nS) + (idx, nS)
-    return _Attn.apply(q, k, v, True, 0, float(scale), 1, 0, tiles)[0]
+    return _run(_Attn, q, k, v, True, 0, float(scale), 1, 0, tiles)[0]
 
 
 def nsa_attention_indexed(q, k, v, idx, g_slc, g_swa, sel_block=64, window=512, scale=None):
@@ -1177,7 +1201,7 @@ def nsa_attention_indexed(q, k, v, idx, g_slc, g_swa, sel_block=64, window=512, 
         return torch_impl.nsa_attention_indexed(q, k, v, idx, g_slc, g_swa, sel_block, window, scale)
     scale = D ** -0.5 if scale is None else scale
     o_slc = selected_attention(q, k, v, idx, scale)
-    o_swa = _Attn.apply(q, k, v, True, int(window), float(scale), 1, 0, None)[0]
+    o_swa = _run(_Attn, q, k, v, True, int(window), float(scale), 1, 0, None)[0]
     return g_slc.unsqueeze(-1) * o_slc + g_swa.unsqueeze(-1) * o_swa
 
 
@@ -1185,9 +1209,9 @@ def nsa_importance(q, k_cmp, L_cmp, nS, stride, block, scale):
     B, T, Hq, D = q.shape
     Hkv = k_cmp.shape[2]
     imp = _zeros(B, Hkv, T, nS, dtype=torch.float32, device=q.device)
-    _check(load().nsa_attn_importance(_p(q.contiguous()), _p(k_cmp.contiguous()), _p(L_cmp), _p(imp), c_int(B), c_int(T),
-                                      c_int(k_cmp.shape[1]), c_int(Hq), c_int(Hkv), c_int(D), c_float(scale),
-                                      c_int(stride), c_int(block - 1), c_int(nS), _stream()))
+    _check(load().nsa_attn_importance(_p(q.contiguous()), _p(k_cmp.contiguous()), _p(L_cmp), _p(imp), B, T,
+                                      k_cmp.shape[1], Hq, Hkv, D, scale,
+                                      stride, block - 1, nS, _stream()))
     return imp
 
 
@@ -1199,8 +1223,8 @@ def nsa_select(imp: Tensor, sel_block: int, top_n: int) -> Tensor:
     if imp.is_cuda and nS <= 2048 and imp.dtype == torch.float32:
         imp = imp.contiguous()
         idx = _empty(B, H, T, top_n, dtype=torch.int32, device=imp.device)
-        _check(load().nsa_select_blocks(_p(imp), _p(idx), c_long(B * H * T), c_int(T), c_int(nS), c_int(sel_block),
-                                        c_int(top_n), _stream()))
+        _check(load().nsa_select_blocks(_p(imp), _p(idx), B * H * T, T, nS, sel_block,
+                                        top_n, _stream()))
         return idx
     return _nsa_select_torch(imp, sel_block, top_n)
 
@@ -1230,7 +1254,7 @@ class _GateCombine(torch.autograd.Function):
         D = o1.shape[-1]
         rows = o1.numel() // D
         o = _empty_like(o1)
-        _check(load().nsa_gate_combine_fwd(_p(o1), _p(o2), _p(o3), _p(g1), _p(g2), _p(g3), _p(o), c_long(rows), c_int(D),
+        _check(load().nsa_gate_combine_fwd(_p(o1), _p(o2), _p(o3), _p(g1), _p(g2), _p(g3), _p(o), rows, D,
                                            _stream()))
         ctx.save_for_backward(o1, o2, o3, g1, g2, g3)
         return o
@@ -1244,7 +1268,7 @@ class _GateCombine(torch.autograd.Function):
         d1, d2, d3 = _empty_like(o1), _empty_like(o1), _empty_like(o1)
         e1, e2, e3 = _empty_like(g1), _empty_like(g1), _empty_like(g1)
         _check(load().nsa_gate_combine_bwd(_p(o1), _p(o2), _p(o3), _p(g1), _p(g2), _p(g3), _p(do), _p(d1), _p(d2), _p(d3),
-                                           _p(e1), _p(e2), _p(e3), c_long(rows), c_int(D), _stream()))
+                                           _p(e1), _p(e2), _p(e3), rows, D, _stream()))
         return d1, d2, d3, e1, e2, e3
 
 
@@ -1257,8 +1281,8 @@ def _gate_logits_forward(o1, o2, o3, gates):
         gl = gl.contiguous()
     g0, step = gl.data_ptr(), Hq * gl.element_size()
     o = _empty_like(o1)
-    _check(load().nsa_gate_combine_fwd_ex(_p(o1), _p(o2), _p(o3), c_void_p(g0), c_void_p(g0 + step), c_void_p(g0 + 2 * step),
-                                          c_long(gl.shape[-1]), c_int(Hq), c_int(1), _p(o), c_long(o1.numel() // D), c_int(D),
+    _check(load().nsa_gate_combine_fwd_ex(_p(o1), _p(o2), _p(o3), g0, g0 + step, g0 + 2 * step,
+                                          gl.shape[-1], Hq, 1, _p(o), o1.numel() // D, D,
                                           _stream()))
     return o, gl
 
@@ -1271,10 +1295,10 @@ def _gate_logits_backward(o1, o2, o3, gl, do, sums=(None, None, None)):
     d1, d2, d3 = _empty_like(o1), _empty_like(o1), _empty_like(o1)
     dgl = _zeros_like(gl) if ldg > 3 * Hq else _empty_like(gl)
     g0, dg0 = gl.data_ptr(), dgl.data_ptr()
-    _check(load().nsa_gate_combine_bwd_ex(_p(o1), _p(o2), _p(o3), c_void_p(g0), c_void_p(g0 + step), c_void_p(g0 + 2 * step),
-                                          c_long(ldg), c_int(Hq), c_int(1), _p(do), _p(d1), _p(d2), _p(d3), c_void_p(dg0),
-                                          c_void_p(dg0 + step), c_void_p(dg0 + 2 * step), _p(sums[0]), _p(sums[1]), _p(sums[2]),
-                                          c_long(o1.numel() // D), c_int(D), _stream()))
+    _check(load().nsa_gate_combine_bwd_ex(_p(o1), _p(o2), _p(o3), g0, g0 + step, g0 + 2 * step,
+                                          ldg, Hq, 1, _p(do), _p(d1), _p(d2), _p(d3), dg0,
+                                          dg0 + step, dg0 + 2 * step, _p(sums[0]), _p(sums[1]), _p(sums[2]),
+                                          o1.numel() // D, D, _stream()))
     return d1, d2, d3, dgl
 
 
@@ -1357,8 +1381,8 @@ class _Pool(torch.autograd.Function):
         xv = x if ok else x.contiguous()
         nC = (T - block) // stride + 1
         y = _empty(B, nC, H, D, dtype=x.dtype, device=x.device)
-        _check(load().nsa_pool_fwd(_p(xv), _p(y), c_int(B), c_int(T), c_int(width), c_long(xv.stride(1)), c_int(block),
-                                   c_int(stride), _stream()))
+        _check(load().nsa_pool_fwd(_p(xv), _p(y), B, T, width, xv.stride(1), block,
+                                   stride, _stream()))
         ctx.shape, ctx.block, ctx.stride = (B, T, H, D), block, stride
         return y
 
@@ -1367,7 +1391,7 @@ class _Pool(torch.autograd.Function):
         B, T, H, D = ctx.shape
         dy = dy.contiguous()
         dx = _empty(B, T, H, D, dtype=dy.dtype, device=dy.device)
-        _check(load().nsa_pool_bwd(_p(dy), _p(dx), c_int(B), c_int(T), c_int(H * D), c_int(ctx.block), c_int(ctx.stride),
+        _check(load().nsa_pool_bwd(_p(dy), _p(dx), B, T, H * D, ctx.block, ctx.stride,
                                    _stream()))
         return dx, None, None
 
@@ -1376,7 +1400,7 @@ def nsa_compress(x, block, stride):
     if x.dtype != torch.bfloat16 or (x.shape[2] * x.shape[3]) % 8 or x.shape[1] < block:
         _fallback("nsa_compress")
         return torch_impl.nsa_compress(x, block, stride)
-    return _Pool.apply(x, int(block), int(stride))
+    return _run(_Pool, x, int(block), int(stride))
 
 
 def nsa_attention(q, k, v, g_cmp, g_slc, g_swa, cmp_block=32, cmp_stride=16, sel_block=64, top_n=16,
@@ -1397,18 +1421,18 @@ def nsa_attention(q, k, v, g_cmp, g_slc, g_swa, cmp_block=32, cmp_stride=16, sel
     kc = nsa_compress(k, cmp_block, cmp_stride)
     vc = nsa_compress(v, cmp_block, cmp_stride)
     if gate_logits is not None and window > 0 and q.dtype == torch.bfloat16 and _bwd_is_split(D, G, True):
-        return _NSA.apply(q, k, v, kc, vc, gate_logits, cmp_stride, cmp_block, sel_block, top_n, int(window), float(scale))
-    o_cmp, L_cmp = _Attn.apply(q, kc, vc, True, 0, float(scale), cmp_stride, cmp_block - 1, None)
+        return _run(_NSA, q, k, v, kc, vc, gate_logits, cmp_stride, cmp_block, sel_block, top_n, int(window), float(scale))
+    o_cmp, L_cmp = _run(_Attn, q, kc, vc, True, 0, float(scale), cmp_stride, cmp_block - 1, None)
     with torch.no_grad():
         tiles = _nsa_select_tiles(q, kc, L_cmp, -(-T // sel_block), cmp_stride, cmp_block, sel_block, top_n, float(scale))
-    o_slc = _Attn.apply(q, k, v, True, 0, float(scale), 1, 0, tiles)[0]
-    o_swa = _Attn.apply(q, k, v, True, int(window), float(scale), 1, 0, None)[0]
+    o_slc = _run(_Attn, q, k, v, True, 0, float(scale), 1, 0, tiles)[0]
+    o_swa = _run(_Attn, q, k, v, True, int(window), float(scale), 1, 0, None)[0]
     if gate_logits is not None:
         if q.dtype == torch.bfloat16 and D in (64, 128, 256):
-            return _GateCombineLogits.apply(o_cmp, o_slc, o_swa, gate_logits)
+            return _run(_GateCombineLogits, o_cmp, o_slc, o_swa, gate_logits)
         g_cmp, g_slc, g_swa = torch.sigmoid(gate_logits.float()).to(q.dtype)[..., :3 * Hq].split(Hq, dim=-1)
     if q.dtype == torch.bfloat16 and D in (64, 128, 256):
-        return _GateCombine.apply(o_cmp, o_slc, o_swa, g_cmp, g_slc, g_swa)
+        return _run(_GateCombine, o_cmp, o_slc, o_swa, g_cmp, g_slc, g_swa)
     return g_cmp.unsqueeze(-1) * o_cmp + g_slc.unsqueeze(-1) * o_slc + g_swa.unsqueeze(-1) * o_swa
 
 
@@ -1425,8 +1449,8 @@ class _SSDStatePass(torch.autograd.Function):
         B, nc, H = gamma.shape
         E = S[0, 0, 0].numel()
         Hprev = _empty_like(S)
-        _check(load().nsa_ssd_state_fwd(_p(S), _p(gamma), _p(Hprev), c_void_p(0), c_void_p(0), c_int(B), c_int(nc),
-                                        c_int(H), c_long(E), _stream()))
+        _check(load().nsa_ssd_state_fwd(_p(S), _p(gamma), _p(Hprev), None, None, B, nc,
+                                        H, E, _stream()))
         ctx.save_for_backward(gamma, Hprev)
         return Hprev
 
@@ -1437,7 +1461,7 @@ class _SSDStatePass(torch.autograd.Function):
         E = Hprev[0, 0, 0].numel()
         dHprev = dHprev.contiguous().float()
         dS = _empty_like(Hprev)
-        _check(load().nsa_ssd_state_bwd(_p(dHprev), _p(gamma), _p(dS), c_void_p(0), c_int(B), c_int(nc), c_int(H), c_long(E),
+        _check(load().nsa_ssd_state_bwd(_p(dHprev), _p(gamma), _p(dS), None, B, nc, H, E,
                                         _stream()))
         dgamma = (Hprev * dS).sum((-1, -2))
         return dS, dgamma
@@ -1474,8 +1498,8 @@ class _SSD(torch.autograd.Function):
         lib = load()
         Hb, gamma = _SSD.states(lib, False, Bm, ldb, x, ldx, dt, A, None)
         y = _empty(Bsz, T, H, P, dtype=torch.bfloat16, device=dev)
-        _check(lib.nsa_ssd_chunk_out(_p(Cm), c_long(ldc), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(Hb), _p(dt), _p(A),
-                                     _p(Df), _p(y), c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream()))
+        _check(lib.nsa_ssd_chunk_out(_p(Cm), ldc, _p(Bm), ldb, _p(x), ldx, _p(Hb), _p(dt), _p(A),
+                                     _p(Df), _p(y), Bsz, T, H, N, P, _stream()))
         ctx.save_for_backward(x, dt, A, Bm, Cm, Df if Df is not None else _empty(0, device=dev), gamma, Hb)
         ctx.has_D = D is not None
         return y
@@ -1486,22 +1510,22 @@ class _SSD(torch.autograd.Function):
         form needs them."""
         Bsz, T, H, P = v.shape
         N, nc, dev = rows.shape[-1], -(-T // 128), v.device
-        dims = (c_int(Bsz), c_int(T), c_int(H), c_int(N), c_int(P), _stream())
+        dims = (Bsz, T, H, N, P, _stream())
         out = _empty(Bsz, nc, H, N, P, dtype=torch.bfloat16, device=dev)
-        if lib.nsa_ssd_states_in_one(c_int(Bsz), c_int(T), c_int(H)):
-            _check(lib.nsa_ssd_states(c_int(back), _p(rows), c_long(ld_rows), _p(v), c_long(ld_v), _p(dt), _p(A), _p(out), *dims))
+        if lib.nsa_ssd_states_in_one(Bsz, T, H):
+            _check(lib.nsa_ssd_states(back, _p(rows), ld_rows, _p(v), ld_v, _p(dt), _p(A), _p(out), *dims))
             return out, _empty(0, device=dev)
         if not back:
             gamma = _empty(Bsz, nc, H, dtype=torch.float32, device=dev)
         local = _empty(Bsz, nc, H, N, P, dtype=torch.float32, device=dev)
-        _check(lib.nsa_ssd_chunk_state(c_int(back), _p(rows), c_long(ld_rows), _p(v), c_long(ld_v), _p(dt), _p(A), _p(local),
-                                       c_void_p(0) if back else _p(gamma), *dims))
+        _check(lib.nsa_ssd_chunk_state(back, _p(rows), ld_rows, _p(v), ld_v, _p(dt), _p(A), _p(local),
+                                       None if back else _p(gamma), *dims))
         if back:
-            _check(lib.nsa_ssd_state_bwd(_p(local), _p(gamma), c_void_p(0), _p(out), c_int(Bsz), c_int(nc), c_int(H), c_long(N * P),
+            _check(lib.nsa_ssd_state_bwd(_p(local), _p(gamma), None, _p(out), Bsz, nc, H, N * P,
                                          _stream()))
         else:
-            _check(lib.nsa_ssd_state_fwd(_p(local), _p(gamma), c_void_p(0), _p(out), c_void_p(0), c_int(Bsz), c_int(nc), c_int(H),
-                                         c_long(N * P), _stream()))
+            _check(lib.nsa_ssd_state_fwd(_p(local), _p(gamma), None, _p(out), None, Bsz, nc, H,
+                                         N * P, _stream()))
         return out, gamma
 
     @staticmethod
@@ -1518,14 +1542,14 @@ class _SSD(torch.autograd.Function):
         dHn, _ = _SSD.states(lib, True, Cm, ldc, dy, H * P, dt, A, gamma)
         dx = _empty(Bsz, T, H, P, dtype=torch.bfloat16, device=dev)
         # dB / dC: fp32 sums over the heads that one CTA has of a chunk, added up afterwards
-        slots = lib.nsa_ssd_grad_slots(c_int(Bsz), c_int(T), c_int(H))
+        slots = lib.nsa_ssd_grad_slots(Bsz, T, H)
         dB_part, dC_part = (_empty(Bsz, T, slots, N, dtype=torch.float32, device=dev) for _ in range(2))
         q = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
         k = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
         rdx = _empty(Bsz, T, H, dtype=torch.float32, device=dev) if ctx.has_D else None
-        _check(lib.nsa_ssd_chunk_grad(_p(Cm), c_long(ldc), _p(Bm), c_long(ldb), _p(x), c_long(ldx), _p(dy), _p(Hb), _p(dHn), _p(dt),
-                                      _p(A), _p(Df), _p(dx), _p(dB_part), _p(dC_part), _p(q), _p(k), _p(rdx), c_int(Bsz), c_int(T),
-                                      c_int(H), c_int(N), c_int(P), _stream()))
+        _check(lib.nsa_ssd_chunk_grad(_p(Cm), ldc, _p(Bm), ldb, _p(x), ldx, _p(dy), _p(Hb), _p(dHn), _p(dt),
+                                      _p(A), _p(Df), _p(dx), _p(dB_part), _p(dC_part), _p(q), _p(k), _p(rdx), Bsz, T,
+                                      H, N, P, _stream()))
         # d(cum_t) = dy_t.(y_t - D x_t) - x_t.dx_t ;  a_k = dt_k A enters every cum_t with t >= k
         dB, dC = (_empty(Bsz, T, 1, N, dtype=torch.bfloat16, device=dev) for _ in range(2))
         ddt = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
@@ -1533,7 +1557,7 @@ class _SSD(torch.autograd.Function):
         dD = _empty(H, dtype=torch.float32, device=dev) if ctx.has_D else None
         scratch = _empty(3 * Bsz * nc * H, dtype=torch.float32, device=dev)
         _check(lib.nsa_ssd_finish(_p(dB_part), _p(dC_part), _p(q), _p(k), _p(rdx), _p(dt), _p(A), _p(scratch), _p(dB), _p(dC), _p(ddt),
-                                  _p(dA), _p(dD), c_int(Bsz), c_int(T), c_int(H), _stream()))
+                                  _p(dA), _p(dD), Bsz, T, H, _stream()))
         return dx, ddt, dA, dB, dC, dD
 
 
@@ -1560,7 +1584,7 @@ def copy_columns(dst: Tensor, src: Tensor) -> bool:
         return False
     es = dst.element_size()
     rows = dst.numel() // dst.shape[-1]
-    _check(load().nsa_copy2d(_p(dst), c_long(dp * es), _p(src), c_long(sp * es), c_long(dst.shape[-1] * es), c_long(rows),
+    _check(load().nsa_copy2d(_p(dst), dp * es, _p(src), sp * es, dst.shape[-1] * es, rows,
                              _stream()))
     return True
 
@@ -1574,7 +1598,7 @@ def sumsq(tensors) -> Tensor:
     for g in tensors:
         if g.dtype not in (torch.bfloat16, torch.float32) or not g.is_contiguous():
             g = g.float().contiguous()
-        _check(lib.nsa_sumsq(_p(g), c_long(g.numel()), c_int(int(g.dtype == torch.float32)), _p(partial), _p(out), c_int(1),
+        _check(lib.nsa_sumsq(_p(g), g.numel(), int(g.dtype == torch.float32), _p(partial), _p(out), 1,
                              _stream()))
     return out
 
@@ -1587,7 +1611,7 @@ def affine_quantize(t: Tensor, bits: int, q_block: int):
     q = _empty(rows, nblk * q_block, dtype=torch.uint8, device=t.device)
     scale = _empty(rows, nblk, dtype=torch.float32, device=t.device)
     zero = _empty(rows, nblk, dtype=torch.float32, device=t.device)
-    _check(load().nsa_affine_quant(_p(t), _p(q), _p(scale), _p(zero), c_long(rows), c_int(cols), c_int(q_block), c_int(bits),
+    _check(load().nsa_affine_quant(_p(t), _p(q), _p(scale), _p(zero), rows, cols, q_block, bits,
                                    _stream()))
     return q, scale, zero, cols
 
@@ -1596,8 +1620,8 @@ def affine_dequantize(q: Tensor, scale: Tensor, zero: Tensor, orig_cols: int) ->
     rows = q.shape[0]
     q_block = q.shape[1] // scale.shape[1]
     out = _empty(rows, orig_cols, dtype=torch.float32, device=q.device)
-    _check(load().nsa_affine_dequant(_p(q.contiguous()), _p(scale.contiguous()), _p(zero.contiguous()), _p(out), c_long(rows),
-                                     c_int(orig_cols), c_int(q_block), _stream()))
+    _check(load().nsa_affine_dequant(_p(q.contiguous()), _p(scale.contiguous()), _p(zero.contiguous()), _p(out), rows,
+                                     orig_cols, q_block, _stream()))
     return out
 
 
@@ -1610,8 +1634,8 @@ def mamba3_gate(u: Tensor, dt: Tensor, A: Tensor, Bc: Tensor, Cc: Tensor, D: Ten
     f = lambda t: t.detach().float().contiguous()
     u, dt, A, Bc, Cc, D = f(u), f(dt), f(A), f(Bc), f(Cc), f(D)
     gate = _empty(B, L, H, dtype=torch.float32, device=u.device)
-    _check(load().nsa_mamba3_scan(_p(u), _p(dt), _p(A), _p(Bc), _p(Cc), _p(D), _p(gate), c_int(B), c_int(L), c_int(H),
-                                  c_int(N), _stream()))
+    _check(load().nsa_mamba3_scan(_p(u), _p(dt), _p(A), _p(Bc), _p(Cc), _p(D), _p(gate), B, L, H,
+                                  N, _stream()))
     return gate
 
 
@@ -1621,7 +1645,7 @@ def ssd_scan(x, dt, A, Bm, Cm, D=None, chunk=256):
     inter-chunk state pass."""
     if (x.shape[-1] == 64 and Bm.shape[-1] == 128 and Bm.shape[2] == 1 and x.dtype == torch.bfloat16
             and Bm.dtype == torch.bfloat16 and Cm.dtype == torch.bfloat16):
-        return _SSD.apply(x, dt, A, Bm, Cm, D)
+        return _run(_SSD, x, dt, A, Bm, Cm, D)
     return _ssd_scan_batched(x, dt, A, Bm, Cm, D, chunk)
 
 
@@ -1659,7 +1683,7 @@ def _ssd_scan_batched(x, dt, A, Bm, Cm, D=None, chunk=256):
     w_end = torch.exp(total[:, :, None, :] - cum)
     Bh = Br.repeat_interleave(rep, dim=3) if rep > 1 else Br
     S_loc = torch.einsum("bclhp,bclhn->bchpn", (xdt.float() * w_end[..., None]).to(cdt), Bh).float()
-    Hprev = _SSDStatePass.apply(S_loc, torch.exp(total))                 # (B,nc,H,P,N) fp32
+    Hprev = _run(_SSDStatePass, S_loc, torch.exp(total))                 # (B,nc,H,P,N) fp32
     Ch = Cr.repeat_interleave(rep, dim=3) if rep > 1 else Cr
     y_inter = torch.einsum("bclhn,bchpn->bclhp", (Ch.float() * torch.exp(cum)[..., None]).to(cdt), Hprev.to(cdt))
     y = (y + y_inter).reshape(Bsz, Tp, H, P)[:, :T]
