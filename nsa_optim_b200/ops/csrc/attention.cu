@@ -2172,13 +2172,371 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 }
 
 // --------------------------------------------------------------------------------------
-// Backward for dK / dV, key-block stationary.  A CTA owns one 64-key block of one KV head and
-// walks over "visits": query tiles of 128 rows (R tokens x G heads) that can see the block.
-//   contiguous modes: the visits are the query tiles of an analytic range (causality, window),
-//     split into chunks of `visits_per_cta` along grid.x;
-//   selected mode: the visits come from the inverse selection map: for every (batch, KV head,
-//     block) the ascending list of tokens that selected it, R tokens per visit, each token's
-//     G query rows fetched by its own TMA box.
+// Backward for dK / dV over contiguous key ranges, key-block stationary.  A CTA owns 128 keys of one KV head and walks over
+// "visits", the query tiles of 128 rows (R tokens x G heads) of an analytic range (causality, window), split into walks
+// along grid.y.  Scores are held transposed (lanes = keys, columns = query rows):
+//     S^T = K Q^T, dP^T = V dO^T;  P^T, dS^T (bf16) take their places and are the A operands of
+//     dV += P^T dO, dK += dS^T Q, which stay in tensor memory for the whole walk.
+// So P and dS never pass through shared memory, which holds K and V, three tiles of Q and two of dO.  One warp issues all products,
+// in the order dV(v), S(v+1), dK(v), dP(v+1): each overwrites columns that the one before has read.  Scores, exponentials, dV and
+// the next scores are a chain (dS, dK and dP run beside it), so dV starts on the first half of P.  The sums leave as bulk
+// reductions of whole rows.
+// (64 keys a CTA and P, dS through shared memory: every product had 64 columns, which costs the tensor pipe as much as 128 when
+// both operands come from shared memory.  8192 tokens x 32 query and 2 KV heads: 1390 us; now 884.  A visit is 3100 cycles here:
+// exponentials 1200, dV and S 1100, the rest signals between them.  S for half tiles costs its products twice, 3250.)
+// Roles: warps 0-7 softmax (key lane, 64 query rows each), warp 8 TMA producer, warp 9 MMA issuer, warp 10 row statistics.
+// --------------------------------------------------------------------------------------
+struct KeyWalks {
+  int visits;                // query tiles per walk
+  int walks;                 // walks per key block
+  float* part;               // [walks][2][B, S, Hkv, D] sums of a walk, added up in order afterwards; null: added to dV and dK
+};
+// Query tiles of walk y of the 128 keys from s0 on: v0 and how many (none: <= 0)
+__device__ __forceinline__ int key_walk(const AttnParams& p, int visits, int s0, int y, int& v0) {
+  const int s_hi = min(s0 + 127, p.S - 1), n_qt = (p.T + p.R - 1) / p.R;
+  const int qt_lo = p.causal ? max(0, (s0 * p.kp_stride + p.kp_off) / p.R) : 0;
+  if (p.window > 0) {                          // short ranges: chunks counted from the block's first tile
+    v0 = qt_lo + y * visits;
+    return min(visits, min(n_qt, (s_hi * p.kp_stride + p.kp_off + p.window - 1) / p.R + 1) - v0);
+  }
+  v0 = max(qt_lo, y * visits);                 // long ranges: absolute chunks, the same Q/dO range for every key block
+  return min(n_qt, (y + 1) * visits) - v0;
+}
+// dV, dK += the walks' sums, in order.  A warp owns a (key, head) row of D = 128.
+__global__ void __launch_bounds__(256) attn_sum_walks_kernel(const AttnParams p, const KeyWalks w, const long rows) {
+  const long row = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const long i = row * 32 + (threadIdx.x & 31), n = rows * 32;               // in float4
+  const int s0 = static_cast<int>(row / p.Hkv % p.S) & ~127;
+  float4* out = reinterpret_cast<float4*>(blockIdx.y ? p.dK : p.dV) + i;
+  const float4* part = reinterpret_cast<const float4*>(w.part) + blockIdx.y * n + i;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int y = 0; y < w.walks; ++y) {
+    int v0;
+    if (key_walk(p, w.visits, s0, y, v0) <= 0) continue;
+    const float4 v = part[2 * n * y];
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  }
+  const float4 old = *out;
+  *out = make_float4(old.x + acc.x, old.y + acc.y, old.z + acc.z, old.w + acc.w);
+}
+
+constexpr int KVC_THREADS = 352;
+constexpr int KVC_SMEM = 28 * HALF + 2 * 2 * 128 * 4 + 256;
+__device__ __forceinline__ void arrive_warp(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) tc5::mbar_arrive(bar);
+}
+
+__global__ void __launch_bounds__(KVC_THREADS, 1)
+attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
+                         const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                         const AttnParams p, const KeyWalks w, const float scale) {
+  constexpr int D = 128, KEYS = 128;
+  constexpr int TILE = 4 * HALF;                 // [128 rows][128] bf16: two 64-column k-blocks
+  constexpr int ROW = D * 4 + 16;                // bytes from one key's sums to the next on their way out
+  static_assert(2 * KEYS * ROW <= 5 * TILE, "attention: dK and dV on their way out");
+  extern __shared__ __align__(1024) uint8_t smem_kvc[];
+  uint8_t* sK = smem_kvc;                        // tiles fill the SM's shared memory: no room to align by hand
+  uint8_t* sV = sK + TILE;
+  uint8_t* sQ = sV + TILE;                       // [3]
+  uint8_t* sDO = sQ + 3 * TILE;                  // [2]
+  float* stats = reinterpret_cast<float*>(sDO + 2 * TILE);       // [2]: -L, -delta scale of 128 rows
+  uint64_t* bars = reinterpret_cast<uint64_t*>(stats + 2 * 256);
+  uint64_t *kv_full = bars, *acc_done = bars + 1;
+  uint64_t *q_full = bars + 2, *q_empty = bars + 5;              // [3]
+  uint64_t *do_full = bars + 8, *do_empty = bars + 10;           // [2]
+  uint64_t *st_full = bars + 12, *st_empty = bars + 14;          // [2]
+  uint64_t *s_full = bars + 16, *dp_full = bars + 17, *ds_full = bars + 18;
+  uint64_t* p_full = bars + 19;                                  // [2]: the first and last 32 of each thread's 64 rows
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = blockIdx.z / p.Hkv, h = blockIdx.z - b * p.Hkv;
+  const int s0 = blockIdx.x * KEYS;              // key block fastest: concurrent CTAs share a Q/dO range in L2
+  int v0;
+  const int n_vis = key_walk(p, w.visits, s0, blockIdx.y, v0);
+  if (n_vis <= 0) return;
+  if (tc5::smem_u32(smem_kvc) & 1023u) {         // the swizzle needs it; never seen otherwise
+    if (tid == 0) status_report(p.status, STATUS_BAD_ARGUMENT, blockIdx.x, static_cast<int>(tc5::smem_u32(smem_kvc)));
+    return;
+  }
+
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < 14; ++i) tc5::mbar_init(bars + i, 1);
+    for (int i = 0; i < 2; ++i) {
+      tc5::mbar_init(st_empty + i, 8);
+      tc5::mbar_init(p_full + i, 8);
+    }
+    tc5::mbar_init(s_full, 1);
+    tc5::mbar_init(dp_full, 1);
+    tc5::mbar_init(ds_full, 8);
+    tc5::fence_barrier_init();
+  }
+  if (warp == 9) { tc5::tmem_alloc(tmem_slot, 512); tc5::tmem_relinquish(); }
+  tc5::fence_before_sync();
+  __syncthreads();
+  tc5::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  constexpr uint32_t cS = 0, cDP = 128, cDV = 256, cDK = 384;
+  auto wait = [&](uint64_t* bar, int phase, int code) {
+    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+  };
+
+  if (warp == 8) {
+    // ------------------------------------------------------------------ TMA producer
+    const bool lead = tc5::elect_one();
+    if (lead) {
+      tc5::mbar_expect_tx(kv_full, 2 * TILE);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {              // k-block i / 2, 64 keys; keys past the end read zero
+        tc5::tma_load_4d(sK + i * HALF, &tm_k, kv_full, (i >> 1) * 64, h, s0 + (i & 1) * 64, b);
+        tc5::tma_load_4d(sV + i * HALF, &tm_v, kv_full, (i >> 1) * 64, h, s0 + (i & 1) * 64, b);
+      }
+    }
+    bool ok = true;
+    for (int v = 0; v < n_vis; ++v) {
+      const int q0 = (v0 + v) * p.R, qb = v % 3, ob = v & 1;
+      if (v >= 3 && !(ok = wait(q_empty + qb, v / 3 - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
+      if (lead) {
+        tc5::mbar_expect_tx(q_full + qb, TILE);
+        tc5::tma_load_5d(sQ + qb * TILE, &tm_q, q_full + qb, 0, 0, h, q0, b);
+        tc5::tma_load_5d(sQ + qb * TILE + 2 * HALF, &tm_q, q_full + qb, 64, 0, h, q0, b);
+      }
+      __syncwarp();
+      if (v >= 2 && !(ok = wait(do_empty + ob, (v >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
+      if (lead) {
+        tc5::mbar_expect_tx(do_full + ob, TILE);
+        tc5::tma_load_5d(sDO + ob * TILE, &tm_do, do_full + ob, 0, 0, h, q0, b);
+        tc5::tma_load_5d(sDO + ob * TILE + 2 * HALF, &tm_do, do_full + ob, 64, 0, h, q0, b);
+      }
+      __syncwarp();
+    }
+    if (ok) ok = wait(acc_done, 0, STATUS_TIMEOUT_TMEM_FULL);
+    if (!ok && lead) {                           // copies may still be in flight
+      tc5::mbar_drain(kv_full);
+      for (int i = 0; i < 3; ++i) tc5::mbar_drain(q_full + i);
+      for (int i = 0; i < 2; ++i) tc5::mbar_drain(do_full + i);
+    }
+    __syncwarp();
+  } else if (warp == 9) {
+    // ------------------------------------------------------------------ MMA issuer (converged warp, elected lane issues)
+    const bool lead = tc5::elect_one();
+    constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0), id_t = tc5::make_idesc_bf16(128, 128, 0, 1);
+    const uint64_t aK = tc5::desc_kmajor(tc5::smem_u32(sK)), aV = tc5::desc_kmajor(tc5::smem_u32(sV));
+    const uint64_t bQ0 = tc5::desc_kmajor(tc5::smem_u32(sQ)), bDO0 = tc5::desc_kmajor(tc5::smem_u32(sDO));
+    const uint64_t tQ0 = tc5::desc_mnmajor(tc5::smem_u32(sQ), 2 * HALF), tDO0 = tc5::desc_mnmajor(tc5::smem_u32(sDO), 2 * HALF);
+    auto kblock = [](int kk) { return static_cast<uint64_t>(((kk >> 2) * 2 * HALF + (kk & 3) * 32) >> 4); };
+    auto at = [](int buf) { return static_cast<uint64_t>((buf * TILE) >> 4); };
+    auto scores = [&](int v) {                   // S^T of visit v
+      if (!wait(q_full + v % 3, v / 3, STATUS_TIMEOUT_SMEM_FULL)) return false;
+      tc5::fence_after_sync();
+      if (lead) {
+        const uint64_t bQ = bQ0 + at(v % 3);
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) tc5::mma_ss(tmem + cS, aK + kblock(kk), bQ + kblock(kk), id_s, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(s_full);
+      }
+      __syncwarp();
+      return true;
+    };
+    auto grads = [&](int v) {                    // dP^T of visit v
+      if (!wait(do_full + (v & 1), v >> 1, STATUS_TIMEOUT_SMEM_FULL)) return false;
+      tc5::fence_after_sync();
+      if (lead) {
+        const uint64_t bDO = bDO0 + at(v & 1);
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) tc5::mma_ss(tmem + cDP, aV + kblock(kk), bDO + kblock(kk), id_s, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(dp_full);
+      }
+      __syncwarp();
+      return true;
+    };
+    // columns of 16 query rows of P^T or dS^T (see the softmax warps)
+    auto rows16 = [](int kk) { return static_cast<uint32_t>((kk >> 2) * 64 + (kk & 3) * 8); };
+    bool ok = wait(kv_full, 0, STATUS_TIMEOUT_SMEM_FULL) && scores(0) && grads(0);
+    for (int v = 0; v < n_vis && ok; ++v) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (ok) ok = wait(p_full + half, v, STATUS_TIMEOUT_TMEM_EMPTY);
+        if (!ok) break;
+        tc5::fence_after_sync();
+        if (lead) {
+          const uint64_t tDO = tDO0 + at(v & 1);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {          // dV += P^T dO; rows 32 half .. of both threads' 64
+            const int kk = (i >> 1) * 4 + half * 2 + (i & 1);
+            tc5::mma_ts(tmem + cDV, tmem + cS + rows16(kk), tDO + static_cast<uint64_t>((kk * 2048) >> 4), id_t,
+                        (v > 0 || half > 0 || i > 0) ? 1u : 0u);
+          }
+          if (half) tc5::mma_commit(do_empty + (v & 1));
+        }
+        __syncwarp();
+      }
+      if (!ok || (v + 1 < n_vis && !(ok = scores(v + 1)))) break;
+      if (!(ok = wait(ds_full, v, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+      tc5::fence_after_sync();
+      if (lead) {
+        const uint64_t tQ = tQ0 + at(v % 3);
+#pragma unroll
+        for (int kk = 0; kk < BM / 16; ++kk)     // dK += dS^T Q
+          tc5::mma_ts(tmem + cDK, tmem + cDP + rows16(kk), tQ + static_cast<uint64_t>((kk * 2048) >> 4), id_t, (v > 0 || kk > 0) ? 1u : 0u);
+        tc5::mma_commit(q_empty + v % 3);
+      }
+      __syncwarp();
+      if (v + 1 < n_vis) ok = grads(v + 1);
+    }
+    if (ok && lead) tc5::mma_commit(acc_done);
+    __syncwarp();
+  } else if (warp == 10) {
+    // ------------------------------------------------------------------ -L and -delta scale of the rows, two visits ahead
+    for (int v = 0; v < n_vis; ++v) {
+      float* st = stats + (v & 1) * 256;
+      float negL[4], nds[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = 4 * lane + i, t = (v0 + v) * p.R + r / p.G;
+        negL[i] = -INFINITY;                     // rows past the end, and rows that see no key (L = -inf): probability 0
+        nds[i] = 0.f;
+        if (t < p.T) {
+          const long rowi = (static_cast<long>(b) * p.T + t) * p.Hq + h * p.G + r % p.G;
+          const float L = p.L[rowi];
+          negL[i] = L == -INFINITY ? -INFINITY : -L;
+          nds[i] = -p.delta[rowi] * scale;
+        }
+      }
+      if (v >= 2 && !wait(st_empty + (v & 1), (v >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY)) break;
+      *reinterpret_cast<float4*>(st + 4 * lane) = make_float4(negL[0], negL[1], negL[2], negL[3]);
+      *reinterpret_cast<float4*>(st + 128 + 4 * lane) = make_float4(nds[0], nds[1], nds[2], nds[3]);
+      arrive_warp(st_full + (v & 1));
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax warps: key lane, query rows 64 ch ..
+    const int ch = warp >> 2, key = s0 + (warp & 3) * 32 + lane;
+    const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + ch * 64;
+    const float sc = p.scale_log2;
+    const int kpos = key * p.kp_stride + p.kp_off;
+    const int w_lo = s0 + (warp & 3) * 32, w_hi = w_lo + 31;     // keys of this warp
+    bool ok = true;
+    for (int v = 0; v < n_vis; ++v) {
+      const int t0 = (v0 + v) * p.R;             // the tile's first token; row c belongs to token t0 + c / G
+      const float* st = stats + (v & 1) * 256 + ch * 64;
+      // rows that see the key are an interval [lo, hi) of the tile's
+      bool check = w_hi >= p.S || t0 + p.R > p.T;
+      if (p.causal) check = check || w_hi * p.kp_stride + p.kp_off > t0;
+      if (p.window > 0) check = check || w_lo * p.kp_stride + p.kp_off <= t0 + p.R - 1 - p.window;
+      int lo = 0, hi = 64;
+      if (check) {
+        if (p.causal) lo = max(0, min(64, max(0, min(p.R, kpos - t0)) * p.G - ch * 64));
+        if (p.window > 0) hi = max(0, min(64, max(0, min(p.R, kpos + p.window - t0)) * p.G - ch * 64));
+        hi = min(hi, max(0, min(64, (p.T - t0) * p.G - ch * 64)));
+        if (key >= p.S) hi = 0;
+      }
+      if (!(ok = wait(st_full + (v & 1), v >> 1, STATUS_TIMEOUT_SMEM_FULL) && wait(s_full, v, STATUS_TIMEOUT_TMEM_FULL))) break;
+      tc5::fence_after_sync();
+      float pr[64];
+      {
+        uint32_t a[32], c[32];
+        tc5::tmem_ld_x32(lanes + cS, a);
+        tc5::tmem_ld_x32(lanes + cS + 32, c);
+        tc5::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          pr[i] = __uint_as_float(a[i]);
+          pr[32 + i] = __uint_as_float(c[i]);
+        }
+      }
+      if (check) {                               // invisible scores are -inf: their probability is 0
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (i < lo || i >= hi) pr[i] = -INFINITY;
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const int i = q * 32 + j;
+          const float4 nl = *reinterpret_cast<const float4*>(st + i);
+          pr[i] = exp2f(fmaf(pr[i], sc, nl.x));
+          pr[i + 1] = exp2f(fmaf(pr[i + 1], sc, nl.y));
+          pr[i + 2] = exp2f(fmaf(pr[i + 2], sc, nl.z));
+          pr[i + 3] = exp2f(fmaf(pr[i + 3], sc, nl.w));
+          pk[j / 2] = tc5::pack_bf16(pr[i], pr[i + 1]);
+          pk[j / 2 + 1] = tc5::pack_bf16(pr[i + 2], pr[i + 3]);
+        }
+        tc5::tmem_st_x16(lanes + cS + q * 16, pk);
+        tc5::tmem_st_wait();
+        tc5::fence_before_sync();
+        arrive_warp(p_full + q);
+      }
+      if (!(ok = wait(dp_full, v, STATUS_TIMEOUT_TMEM_FULL))) break;
+      tc5::fence_after_sync();
+      uint32_t pk[32];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t a[32];
+        tc5::tmem_ld_x32(lanes + cDP + q * 32, a);
+        tc5::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          const float4 nd = *reinterpret_cast<const float4*>(st + 128 + q * 32 + i);
+          const float* pi = pr + q * 32 + i;
+          pk[q * 16 + i / 2] = tc5::pack_bf16(pi[0] * fmaf(__uint_as_float(a[i]), scale, nd.x), pi[1] * fmaf(__uint_as_float(a[i + 1]), scale, nd.y));
+          pk[q * 16 + i / 2 + 1] = tc5::pack_bf16(pi[2] * fmaf(__uint_as_float(a[i + 2]), scale, nd.z), pi[3] * fmaf(__uint_as_float(a[i + 3]), scale, nd.w));
+        }
+      }
+      tc5::tmem_st_x32(lanes + cDP, pk);
+      tc5::tmem_st_wait();
+      tc5::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        tc5::mbar_arrive(ds_full);
+        tc5::mbar_arrive(st_empty + (v & 1));
+      }
+    }
+    // ---- accumulators -> global.  A thread holds half a key's row; rows go through shared memory (free now, pitch spread over
+    //      the banks) and are added to global memory by one bulk reduction each: scattered 16-byte reductions were most of a CTA's
+    //      fixed cost of 14 us.
+    const bool have = ok && wait(acc_done, 0, STATUS_TIMEOUT_TMEM_FULL);
+    if (have) {
+      tc5::fence_after_sync();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t a[32];
+        tc5::tmem_ld_x32(lanes + (q < 2 ? cDV : cDK) + (q & 1) * 32, a);
+        tc5::tmem_ld_wait();
+        float4* dst = reinterpret_cast<float4*>(sQ + (q < 2 ? 0 : KEYS * ROW) + (tid & 127) * ROW + (ch * 64 + (q & 1) * 32) * 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          dst[i] = make_float4(__uint_as_float(a[4 * i]), __uint_as_float(a[4 * i + 1]), __uint_as_float(a[4 * i + 2]),
+                               __uint_as_float(a[4 * i + 3]));
+      }
+      tc5::fence_proxy_async();
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    const int row = tid & 127;                   // warps 0-3 send dV, 4-7 dK
+    if (have && s0 + row < p.S) {
+      const long o = ((static_cast<long>(b) * p.S + s0 + row) * p.Hkv + h) * D;
+      const uint8_t* src = sQ + ch * KEYS * ROW + row * ROW;
+      if (w.part) tc5::bulk_store(w.part + (blockIdx.y * 2 + ch) * (static_cast<long>(p.B) * p.S * p.Hkv * D) + o, src, D * 4);
+      else tc5::bulk_reduce_add_f32((ch ? p.dK : p.dV) + o, src, D * 4);
+      tc5::tma_store_commit();
+      tc5::tma_store_wait_read<0>();
+    }
+  }
+  tc5::fence_before_sync();
+  __syncthreads();
+  if (warp == 9) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 512); }
+}
+
+// --------------------------------------------------------------------------------------
+// Backward for dK / dV of selected blocks, key-block stationary.  A CTA owns one 64-key block of one KV head and
+// walks over "visits" of 128 rows (R tokens x G heads) that come from the inverse selection map: for every (batch, KV head,
+// block) the ascending list of tokens that selected it, R tokens per visit, each token's G query rows fetched
+// by its own TMA box.
 // dV^T (D x 64) += dO^T P and dK^T (D x 64) += Q^T dS stay in TMEM for the whole walk, so global
 // memory sees one fp32 reduction per CTA instead of one per (query tile, key tile) pair.
 // Roles: warps 0-7 softmax (thread (r, ch) = row r, 32 key columns), warp 8 TMA producer,
@@ -2188,7 +2546,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // --------------------------------------------------------------------------------------
 struct KvWalk {
   int visits_per_cta;
-  const int* tok_list;      // selected mode: tokens grouped by (b, h, block), ascending inside a group
+  const int* tok_list;      // tokens grouped by (b, h, block), ascending inside a group
   const int* list_start;    // [n_lists + 1]
   const int* item_start;    // [n_lists + 1] exclusive prefix of CTAs per list
   int n_lists, nS;
@@ -2197,8 +2555,7 @@ struct KvWalk {
 constexpr int KV_THREADS = 384;
 
 __global__ void __launch_bounds__(KV_THREADS, 1)
-attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
-                   const __grid_constant__ CUtensorMap tm_q1, const __grid_constant__ CUtensorMap tm_do1,
+attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_constant__ CUtensorMap tm_do1,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const AttnParams p, const KvWalk w, const float scale) {
   constexpr int D = 128;
@@ -2224,42 +2581,18 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool selected = w.tok_list != nullptr;
   // ---- which block, which visits (uniform over the CTA; CTAs without work leave before any setup)
-  int b, h, s0, v0, n_vis, lst0 = 0, cnt = 0;
-  if (selected) {
-    const int item = blockIdx.x;
-    if (item >= w.item_start[w.n_lists]) return;
-    int lo = 0, hi = w.n_lists;                  // largest l with item_start[l] <= item
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (w.item_start[mid] <= item) lo = mid; else hi = mid;
-    }
-    const int l = lo;
-    const int bh = l / w.nS;
-    b = bh / p.Hkv; h = bh - b * p.Hkv;
-    s0 = (l - bh * w.nS) * 64;
-    lst0 = w.list_start[l];
-    cnt = w.list_start[l + 1] - lst0;
-    v0 = (item - w.item_start[l]) * w.visits_per_cta;
-    n_vis = min(w.visits_per_cta, (cnt + p.R - 1) / p.R - v0);
-  } else {
-    const int bh = blockIdx.z;
-    b = bh / p.Hkv; h = bh - b * p.Hkv;
-    s0 = blockIdx.x * 64;                         // key block fastest: concurrent CTAs share a Q/dO range in L2
-    const int s_hi = min(s0 + 63, p.S - 1);
-    const int n_qt = (p.T + p.R - 1) / p.R;
-    int qt_lo = 0, qt_hi = n_qt;
-    if (p.causal) qt_lo = max(0, (s0 * p.kp_stride + p.kp_off) / p.R);
-    if (p.window > 0) qt_hi = min(n_qt, (s_hi * p.kp_stride + p.kp_off + p.window - 1) / p.R + 1);
-    if (p.window > 0) {                          // short ranges: chunks counted from the block's first tile
-      v0 = qt_lo + blockIdx.y * w.visits_per_cta;
-      n_vis = min(w.visits_per_cta, qt_hi - v0);
-    } else {                                     // long ranges: absolute chunks, the same Q/dO range for every key block
-      v0 = max(qt_lo, static_cast<int>(blockIdx.y) * w.visits_per_cta);
-      n_vis = min(qt_hi, (static_cast<int>(blockIdx.y) + 1) * w.visits_per_cta) - v0;
-    }
+  const int item = blockIdx.x;
+  if (item >= w.item_start[w.n_lists]) return;
+  int lst = 0;                                   // largest list with item_start[list] <= item
+  for (int hi = w.n_lists; hi - lst > 1;) {
+    const int mid = (lst + hi) >> 1;
+    if (w.item_start[mid] <= item) lst = mid; else hi = mid;
   }
+  const int bh = lst / w.nS, b = bh / p.Hkv, h = bh - b * p.Hkv, s0 = (lst - bh * w.nS) * 64;
+  const int lst0 = w.list_start[lst], cnt = w.list_start[lst + 1] - lst0;
+  const int v0 = (item - w.item_start[lst]) * w.visits_per_cta;
+  const int n_vis = min(w.visits_per_cta, (cnt + p.R - 1) / p.R - v0);
   if (n_vis <= 0) return;
 
   if (tid == 0) {
@@ -2305,25 +2638,14 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (!ok) break;
       uint8_t* dq_ = sQ + buf * QT;
       uint8_t* dd_ = sDO + buf * QT;
-      if (!selected) {
-        if (lane == 0) {
-          const int q0 = (v0 + v) * p.R;
+      for (int j = lane; j < p.R; j += 32) {
+        const int li = (v0 + v) * p.R + j;
+        const int tok = li < cnt ? __ldg(w.tok_list + lst0 + li) : 0;   // rows past the list read token 0 and are masked
+        const int off = j * p.G * 128;
 #pragma unroll
-          for (int kb = 0; kb < 2; ++kb) {
-            tc5::tma_load_5d(dq_ + kb * 2 * HALF, &tm_q, q_full + buf, kb * 64, 0, h, q0, b);
-            tc5::tma_load_5d(dd_ + kb * 2 * HALF, &tm_do, q_full + buf, kb * 64, 0, h, q0, b);
-          }
-        }
-      } else {
-        for (int j = lane; j < p.R; j += 32) {
-          const int li = (v0 + v) * p.R + j;
-          const int tok = li < cnt ? __ldg(w.tok_list + lst0 + li) : 0;   // rows past the list read token 0 and are masked
-          const int off = j * p.G * 128;
-#pragma unroll
-          for (int kb = 0; kb < 2; ++kb) {
-            tc5::tma_load_5d(dq_ + kb * 2 * HALF + off, &tm_q1, q_full + buf, kb * 64, 0, h, tok, b);
-            tc5::tma_load_5d(dd_ + kb * 2 * HALF + off, &tm_do1, q_full + buf, kb * 64, 0, h, tok, b);
-          }
+        for (int kb = 0; kb < 2; ++kb) {
+          tc5::tma_load_5d(dq_ + kb * 2 * HALF + off, &tm_q1, q_full + buf, kb * 64, 0, h, tok, b);
+          tc5::tma_load_5d(dd_ + kb * 2 * HALF + off, &tm_do1, q_full + buf, kb * 64, 0, h, tok, b);
         }
       }
       __syncwarp();
@@ -2416,16 +2738,12 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const float sc = p.scale_log2;
     const int sb = s0 + ch * 32;                   // this thread's first key
     bool ok = true;
-    // The row's token (selected mode: from the inverse list) and its L / delta are fetched one and
+    // The row's token (from the inverse list) and its L / delta are fetched one and
     // two visits ahead, so the two dependent global loads are off the per-visit critical path.
     auto token_of = [&](int v) -> int {
       if (v >= n_vis) return -1;
-      if (selected) {
-        const int li = (v0 + v) * p.R + tok_local;
-        return li < cnt ? w.tok_list[lst0 + li] : -1;
-      }
-      const int tt = (v0 + v) * p.R + tok_local;
-      return tt < p.T ? tt : -1;
+      const int li = (v0 + v) * p.R + tok_local;
+      return li < cnt ? w.tok_list[lst0 + li] : -1;
     };
     int t_cur = token_of(0), t_nxt = token_of(1);
     float L_cur = 0.f, d_cur = 0.f;
@@ -2946,6 +3264,26 @@ extern "C" int nsa_attn_bwd(const void* q, const void* k, const void* v, const v
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_attn_bwd launch");
 }
 
+// Query tiles that one 128-key block can be visited by, at most
+static int key_visits(int T, int R, int window, int kp_stride) {
+  const int n_qt = (T + R - 1) / R;
+  return window > 0 ? std::min(n_qt, (127 * kp_stride + window - 1) / R + 2) : n_qt;
+}
+// Walks per 128-key block for nsa_attn_bwd_split over contiguous ranges, whose sums it wants room for (`part`, floats: walks x 2 x
+// B S Hkv D) if they are more than one; 0: walks of `visits_per_cta` tiles that add to dK and dV in any order.
+// A visit takes 1.7 us and a walk 2 us more, so short sequences, whose blocks alone leave SMs idle, are cut into walks of six
+// visits and more, three for each SM (half of a causal grid is empty; with two, 110 us where three take 96).  2048 tokens, two groups of 16 heads: one walk a block 423 us, 128
+// visits 220, 32 visits 74.  Blocks of more than 256 visits fill the GPU with walks of 64 (128 within 2 %), and room for all
+// their sums would cost more than it gives.
+extern "C" int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int window, int kp_stride) {
+  if (Hkv <= 0 || Hq < Hkv) return 0;
+  const int most = key_visits(T, std::max(1, BM / (Hq / Hkv)), window, kp_stride);
+  if (most > 256) return 0;
+  const long blocks = static_cast<long>((S + 127) / 128) * B * Hkv;
+  const long want = (3l * nsa::sm_count() + blocks - 1) / std::max(1l, blocks);
+  return static_cast<int>(std::max(1l, std::min<long>(want, most / 6)));
+}
+
 // Backward in two kernels without per-tile global reductions: dQ from the query-tile-outer
 // kernel (its dK / dV part switched off) and dK / dV from the key-block-stationary kernel.
 // Selected mode additionally takes the inverse selection map: tok_list (tokens grouped by
@@ -2953,13 +3291,14 @@ extern "C" int nsa_attn_bwd(const void* q, const void* k, const void* v, const v
 // lengths and of CTAs per list, a CTA covering visits_per_cta * (128 / G) tokens) and
 // item_bound >= item_start[last].  head_dim 128 only; selected mode needs G >= 8.
 // delta_given: delta holds rowsum(dO * O) already (the gated combine's backward has both tensors in registers).
+// walks, part: of nsa_attn_bwd_walks (contiguous ranges).
 // add_dq: dQ is added to what dq holds; dK / dV always add to what the caller put there.
 extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                                   const float* L, float* delta, void* dq, float* dk, float* dv, int B, int T, int S,
                                   int Hq, int Hkv, int D, float scale, int causal, int window, int kp_stride, int kp_off,
                                   const int* tile_blocks, const unsigned long long* tile_masks, const int* tile_counts,
                                   int max_u, const int* tok_list, const int* list_start, const int* item_start, int nS,
-                                  int item_bound, int visits_per_cta, int delta_given, int add_dq,
+                                  int item_bound, int visits_per_cta, float* part, int walks, int delta_given, int add_dq,
                                   cudaStream_t st) {
   int rc = check_shape(Hq, Hkv, D, tile_blocks);
   if (rc) return rc;
@@ -2968,11 +3307,9 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
   if (tile_blocks && (G < 8 || tok_list == nullptr))
     return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: selected mode needs a GQA group of at least 8 and the inverse map");
   if (visits_per_cta <= 0) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: visits_per_cta must be positive");
-  CUtensorMap tq, tdo, tq1, tdo1, tk, tv;
+  CUtensorMap tq, tdo, tk, tv;
   if ((rc = make_q_map(&tq, q, B, T, Hq, Hkv, D))) return rc;
   if ((rc = make_q_map(&tdo, d_o, B, T, Hq, Hkv, D))) return rc;
-  if ((rc = make_q_map(&tq1, q, B, T, Hq, Hkv, D, 1))) return rc;
-  if ((rc = make_q_map(&tdo1, d_o, B, T, Hq, Hkv, D, 1))) return rc;
   if ((rc = make_kv_map(&tk, k, B, S, Hkv, D))) return rc;
   if ((rc = make_kv_map(&tv, v, B, S, Hkv, D))) return rc;
   const long rows = static_cast<long>(B) * T * Hq;
@@ -2996,24 +3333,33 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
     }
   }
   p.dK = dk; p.dV = dv;
-  KvWalk w{};
-  w.visits_per_cta = visits_per_cta;
-  dim3 grid;
   if (tile_blocks) {
+    KvWalk w{};
+    w.visits_per_cta = visits_per_cta;
     w.tok_list = tok_list; w.list_start = list_start; w.item_start = item_start; w.n_lists = B * Hkv * nS; w.nS = nS;
     if (item_bound <= 0) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: item_bound must be positive");
-    grid = dim3(item_bound, 1, 1);
-  } else {
-    const int n_qt = (T + p.R - 1) / p.R;
-    int max_vis = n_qt;
-    if (window > 0) max_vis = std::min(n_qt, (63 * kp_stride + window - 1) / p.R + 2);
-    grid = dim3((S + 63) / 64, (max_vis + visits_per_cta - 1) / visits_per_cta, B * Hkv);
-  }
-  {
     const int smem = 24 * HALF + 1024 + 256;
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(attn_bwd_kv_kernel, smem))) return rc; cfg = true; }
-    attn_bwd_kv_kernel<<<grid, KV_THREADS, smem, st>>>(tq, tdo, tq1, tdo1, tk, tv, p, w, scale);
+    CUtensorMap tq1, tdo1;
+    if ((rc = make_q_map(&tq1, q, B, T, Hq, Hkv, D, 1))) return rc;
+    if ((rc = make_q_map(&tdo1, d_o, B, T, Hq, Hkv, D, 1))) return rc;
+    attn_bwd_kv_kernel<<<item_bound, KV_THREADS, smem, st>>>(tq1, tdo1, tk, tv, p, w, scale);
+  } else {
+    const int most = key_visits(T, p.R, window, kp_stride);
+    KeyWalks w{};
+    w.part = walks > 1 ? part : nullptr;
+    if (walks > 1 && part == nullptr) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: several walks need room for their sums");
+    w.walks = walks > 0 ? walks : (most + visits_per_cta - 1) / visits_per_cta;
+    w.visits = (most + w.walks - 1) / w.walks;
+    static bool cfg = false;
+    if (!cfg) { if ((rc = set_smem(attn_bwd_kv_range_kernel, KVC_SMEM))) return rc; cfg = true; }
+    attn_bwd_kv_range_kernel<<<dim3((S + 127) / 128, w.walks, B * Hkv), KVC_THREADS, KVC_SMEM, st>>>(tq, tdo, tk, tv, p, w, scale);
+    if (w.part) {
+      const long rows = static_cast<long>(B) * S * Hkv;
+      attn_sum_walks_kernel<<<dim3((unsigned)((rows + 7) / 8), 2), 256, 0, st>>>(p, w, rows);
+      nsa::count_launch();
+    }
   }
   nsa::count_launch(delta_given ? 2 : 3);
   cudaError_t e = cudaGetLastError();

@@ -1043,8 +1043,12 @@ def _attn_backward_split(q, k, v, o, do, L, dq, dk, dv, causal, window, scale, k
         delta = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
     tb, tm, tc, mu = tiles[:4] if tiles is not None else (None, None, None, 0)
     inv = (None, None, None, 0, 0)
-    visits = _kv_visits()
-    if tiles is not None:
+    visits, walks, part = _kv_visits(), 0, None
+    if tiles is None:
+        walks = load().nsa_attn_bwd_walks(B, T, S, Hq, Hkv, window, kp_stride)
+        if walks > 1:
+            part = _empty(walks, 2, k.numel(), dtype=torch.float32, device=q.device)
+    else:
         idx, nS = tiles[4], tiles[5]
         visits = int(os.environ.get('NSA_B200_KV_VISITS_SEL', '64'))
         inv = inverse_blocks(idx, nS, 128 // (Hq // Hkv), visits)
@@ -1052,13 +1056,13 @@ def _attn_backward_split(q, k, v, o, do, L, dq, dk, dv, causal, window, scale, k
                                      B, T, S, Hq, Hkv, D, scale,
                                      int(causal), window, kp_stride, kp_off,
                                      _p(tb), _p(tm), _p(tc), mu, _p(inv[0]), _p(inv[1]), _p(inv[2]),
-                                     inv[3], inv[4], visits, int(given), int(add_dq),
+                                     inv[3], inv[4], visits, _p(part), walks, int(given), int(add_dq),
                                      _stream()))
 
 
 def _kv_visits() -> int:
-    """Query tiles per CTA of the dK / dV kernel over a contiguous key range."""
-    return int(os.environ.get('NSA_B200_KV_VISITS', '128'))
+    """Query tiles per CTA of the dK / dV kernel over a contiguous key range, where a key block has more than 256."""
+    return int(os.environ.get('NSA_B200_KV_VISITS', '64'))
 
 
 def _bwd_is_split(D: int, G: int, selected: bool) -> bool:
@@ -1347,6 +1351,7 @@ class _NSA(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do):
         q, k, v, kc, vc, gl, o1, o2, o3, L1, L2, L3 = ctx.saved_tensors
+        lib = load()
         stride, block, window, scale = ctx.cfg
         f32 = torch.float32
         sums = [_empty_like(L1) for _ in range(3)]
@@ -1355,10 +1360,9 @@ class _NSA(torch.autograd.Function):
         dkc, dvc, dk, dv = (_zeros(t.shape, dtype=f32, device=q.device) for t in (kc, vc, k, v))
         _attn_backward_split(q, kc, vc, o1, d1, L1, dq, dkc, dvc, True, 0, scale, stride, block - 1, None, sums[0])
         _attn_backward_split(q, k, v, o2, d2, L2, dq, dk, dv, True, 0, scale, 1, 0, ctx.tiles, sums[1], True)
-        # The window branch shares dk / dv while one CTA covers a key block: one more addition to what is there gives
+        # The window branch shares dk / dv while a key block's gradients get one addition from it: one more to what is there gives
         # the same bits on every run, two in either order would not.
-        R = 128 // (q.shape[2] // k.shape[2])
-        shared = (63 + window - 1) // R + 2 <= _kv_visits()
+        shared = lib.nsa_attn_bwd_walks(*q.shape[:2], k.shape[1], q.shape[2], k.shape[2], window, 1) > 0
         dk3, dv3 = (dk, dv) if shared else (_zeros(t.shape, dtype=f32, device=q.device) for t in (k, v))
         _attn_backward_split(q, k, v, o3, d3, L3, dq, dk3, dv3, True, window, scale, 1, 0, None, sums[2], True)
         if not shared:
