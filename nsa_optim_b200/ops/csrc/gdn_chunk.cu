@@ -135,8 +135,9 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
         const int j = n * 8 + 2 * (lane & 3);
-        // the exponent is zero where the entry is masked, so nothing overflows
-        const float e0 = __expf(j <= i ? gi - gs[j] : 0.f), e1 = __expf(j + 1 <= i ? gi - gs[j + 1] : 0.f);
+        // the exponent is zero where the entry is masked, so nothing overflows (loads first: a load under a condition is a branch)
+        const float2 gj = *reinterpret_cast<const float2*>(gs + j);
+        const float e0 = __expf(j <= i ? gi - gj.x : 0.f), e1 = __expf(j + 1 <= i ? gi - gj.y : 0.f);
         const float x0 = acc[n][2 * hh] * e0, x1 = acc[n][2 * hh + 1] * e1;
         if (warp < 4) {
           *reinterpret_cast<float2*>(As + i * PX + j) = make_float2(j < i ? bi * x0 : 0.f, j + 1 < i ? bi * x1 : 0.f);
@@ -395,6 +396,10 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
   const uint32_t trow = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
   constexpr uint32_t cWQ = 0, cKS = 128, cPT = 256;        // accumulator columns of the three products
   constexpr uint32_t idesc = tc5::make_idesc_bf16(128, 128, 0, 0);
+  uint32_t tut[CH / 16][4];                                // Tu^T, the same for every slice
+#pragma unroll
+  for (int q = 0; q < CH / 16; ++q) load_a_t(tut[q], sTu, PC, m0, q * 16);
+  bf16* dv_row = p.dv + (tok0 + static_cast<long>(t0 + r0) * p.H) * V + n16 + cl;
   bool ok = true;
   for (int s = 0; s < nvt; ++s) {
     const uint8_t* st = stages + (s & 1) * POST_STAGE;
@@ -421,21 +426,18 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
     // dv of this slice behind the MMAs: Tu^T du (row j needs i >= j only)
     float dv[2][4] = {};
 #pragma unroll
-    for (int kk = 0; kk < CH; kk += 16) {
-      if (kk < m0) continue;
-      uint32_t a[4], bb[4];
-      load_a_t(a, sTu, PC, m0, kk);
-      load_b_t_swz(bb, st, n16, kk);
-      mma2(dv[0], dv[1], a, bb);
+    for (int q = 0; q < CH / 16; ++q) {
+      if (q * 16 < m0) continue;
+      uint32_t bb[4];
+      load_b_t_swz(bb, st, n16, q * 16);
+      mma2(dv[0], dv[1], tut[q], bb);
     }
 #pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
-      const int t = t0 + r0 + 8 * hh;
-      if (t >= p.T) continue;
-      bf16* dst = p.dv + (tok0 + static_cast<long>(t) * p.H) * V + s * CH + n16 + cl;
+    for (int hh = 0; hh < 2; ++hh)
+      if (t0 + r0 + 8 * hh < p.T)
 #pragma unroll
-      for (int n = 0; n < 2; ++n) *reinterpret_cast<uint32_t*>(dst + n * 8) = pack2(dv[n][2 * hh], dv[n][2 * hh + 1]);
-    }
+        for (int n = 0; n < 2; ++n)
+          *reinterpret_cast<uint32_t*>(dv_row + static_cast<long>(8 * hh) * p.H * V + s * CH + n * 8) = pack2(dv[n][2 * hh], dv[n][2 * hh + 1]);
     if (s + 2 < nvt) {
       __syncthreads();                                     // du of this stage has been read by every warp
       if (tid == 0) {
@@ -449,16 +451,17 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
     if (next_chunk(p.resident, p.H, p.NC, nbh, nc)) {
       const int nb = nbh / p.H, nh = nbh % p.H, nt = nc * CH;
       const long nchunk = static_cast<long>(nbh) * p.NC + nc;
-      if (tid < nvt) {                                     // a slice each
-        const int x = tid * CH, row = static_cast<int>(nchunk) * CH;
+      if (lane == 0 && warp < nvt) {                       // a slice per warp
+        const int x = warp * CH, row = static_cast<int>(nchunk) * CH;
         tc5::tma_prefetch_2d(&tm_du, x, row);
         tc5::tma_prefetch_4d(&tm_do, x, nh, nt, nb);
         tc5::tma_prefetch_2d(&tm_vn, x, row);
         tc5::tma_prefetch_4d(&tm_v, x, nh, nt, nb);
         tc5::tma_prefetch_2d(&tm_S, x, static_cast<int>(nchunk) * KD);
         tc5::tma_prefetch_2d(&tm_dS, x, static_cast<int>(nchunk) * KD);
-      } else if (tid >= 128 && tid < 256) {                // 64 rows of 256 bytes
-        prefetch_l2(p.X + nchunk * CH * CH + (tid - 128) * 32);
+      }
+      if (tid < 128) {                                     // 64 rows of 256 bytes
+        prefetch_l2(p.X + nchunk * CH * CH + tid * 32);
       } else if (tid >= 256 && nt + (tid & 63) < p.T) {    // q and k, 128 bytes at a time
         const bf16* src = tid < 384 ? p.q : p.k;
         prefetch_l2(src + ((static_cast<long>(nb) * p.T + nt + (tid & 63)) * p.H + nh) * KD + (tid & 64));
@@ -633,11 +636,12 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int j = n16 + n * 8 + cl + e;
-          const float ex = __expf(j <= i ? gi - gs[j] : 0.f);
-          const float d = j < i ? sDX[i * PX + j] : 0.f;
+          const float gj = gs[j], da = sDX[i * PX + j], dq = sP[i * PX + j];     // loads first: a load under a condition is a branch
+          const float ex = __expf(j <= i ? gi - gj : 0.f);
+          const float d = j < i ? da : 0.f;
           const float araw = kk_[n][2 * hh + e] * ex;
           ok[e] = d * bi * ex;
-          oq[e] = j <= i ? sP[i * PX + j] * p.scale * ex : 0.f;
+          oq[e] = j <= i ? dq * p.scale * ex : 0.f;
           const float t = d * bi * araw + oq[e] * qk_[n][2 * hh + e];
           rb += d * araw;
           rg += t;
@@ -769,9 +773,7 @@ extern "C" int nsa_gdn_prep(const void* q, const void* k, const void* v, const f
   const int smem = 2 * CH * PK * 2 + CH * (V + 8) * 2 + 2 * CH * PX * 4 + 2 * CH * 4;
   cudaError_t e = cudaFuncSetAttribute(gdn_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn prep smem attribute");
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gdn_prep_kernel, 256, smem);
-  p.resident = per_sm * nsa::sm_count();
+  p.resident = (2 * (smem + 1024) <= 228 * 1024 ? 2 : 1) * nsa::sm_count();
   gdn_prep_kernel<<<chunk_grid(B * H, NC), 256, smem, st>>>(p);
   nsa::count_launch();
   e = cudaGetLastError();
