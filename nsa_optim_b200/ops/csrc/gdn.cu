@@ -205,13 +205,13 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       }
       if (c + 1 < NC) {
         const float g = __expf(g_last_next);       // decay of the state through chunk c + 1
-        if (!wait(m2, c, STATUS_TIMEOUT_TMEM_FULL)) break;
+        // a wait costs 200 cycles and more when there is nothing to wait for: the one for the stores goes first
+        if (!wait(freed, c, STATUS_TIMEOUT_SMEM_EMPTY) || !wait(m2, c, STATUS_TIMEOUT_TMEM_FULL)) break;
         tc5::fence_after_sync();
         float sv[HC];
         tmem_ld_half(tmem + lane_off + cS, sv);    // S entering chunk c + 1, row r
         uint32_t pk[HC / 2];
         pack_half(sv, pk);
-        if (!wait(freed, c, STATUS_TIMEOUT_SMEM_EMPTY)) break;
         write_half(Sb + ((c + 1) & 1) * 2 * BOX, r, half, pk);
         tc5::fence_proxy_async();
         tc5::fence_before_sync();
@@ -520,13 +520,12 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       }
       if (c == 0) break;
       const float g = __expf(g_last_next);
-      if (!wait(m2, it, STATUS_TIMEOUT_TMEM_FULL)) break;
+      if (!wait(freed, it, STATUS_TIMEOUT_SMEM_EMPTY) || !wait(m2, it, STATUS_TIMEOUT_TMEM_FULL)) break;
       tc5::fence_after_sync();
       float ds[HC];
       tmem_ld_half(tmem + lane_off + cDs, ds);     // gradient of the state leaving chunk c - 1
       uint32_t pk[HC / 2];
       pack_half(ds, pk);
-      if (!wait(freed, it, STATUS_TIMEOUT_SMEM_EMPTY)) break;
       write_half(dSb, r, half, pk);
       tc5::fence_proxy_async();
       tc5::fence_before_sync();
