@@ -337,12 +337,12 @@ __device__ __forceinline__ void arrive_warp(uint64_t* bar) {
 // ---------------------------------------------------------------------------------------
 // chunk_out: y = P x + exp(cum) (C H) + D x.
 // Sixteen warps compute the weights of one item, then finish the rows of the item before, whose products ran meanwhile;
-// the seventeenth loads, scans, issues and stores.  C B^T stays in registers for all heads of a segment, P goes to tensor
+// three more issue, copy and scan the step sizes.  C B^T stays in registers for all heads of a segment, P goes to tensor
 // memory as the A operand, y leaves from the place of x.
 // ---------------------------------------------------------------------------------------
 constexpr int OUT_ST = 4;                             // stages of (x, H)
 constexpr int OUT_SMEM = 1024 + (4 + 2 * OUT_ST) * BOXB + 2 * (2 * L + 192) * 4 + 256;
-__global__ void __launch_bounds__(544, 1)
+__global__ void __launch_bounds__(608, 1)
 ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_b,
                      const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_h,
                      const __grid_constant__ CUtensorMap tm_y, const SsdParams p) {
@@ -354,14 +354,15 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   float* scan = reinterpret_cast<float*>(stages + 2 * OUT_ST * BOXB);   // even and odd items: cum, dts, colf
   uint64_t* bars = reinterpret_cast<uint64_t*>(scan + 2 * (2 * L + 192));
   uint64_t *full = bars, *cb = bars + OUT_ST, *ms = cb + 1, *sread = cb + 2;
-  uint64_t *scanned = cb + 3, *ready = cb + 5, *done = cb + 7, *left = cb + 9;    // even and odd items
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(cb + 11);
+  uint64_t *scanned = cb + 3, *ready = cb + 5, *done = cb + 7;        // even and odd items
+  uint64_t* left = cb + 9;                             // per stage
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(left + OUT_ST);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    for (int i = 0; i < OUT_ST; ++i) tc5::mbar_init(full + i, 1);
+    for (int i = 0; i < OUT_ST; ++i) { tc5::mbar_init(full + i, 1); tc5::mbar_init(left + i, 16); }
     tc5::mbar_init(cb, 1);
     tc5::mbar_init(ms, 1);
     tc5::mbar_init(sread, 16);
@@ -369,7 +370,6 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
       tc5::mbar_init(scanned + i, 1);
       tc5::mbar_init(ready + i, 16);
       tc5::mbar_init(done + i, 1);
-      tc5::mbar_init(left + i, 16);
     }
     tc5::fence_barrier_init();
   }
@@ -379,58 +379,22 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const uint32_t cS = 0, cP = 128, cYi = 256, cYo = 384;     // the last three: 64 columns for even and odd items each
-  if (warp == 16) {
+  auto wait = [&](uint64_t* bar, int phase, int code) {
+    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+  };
+  if (warp == 16) {                                    // products
     constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);
     constexpr uint32_t id_y = tc5::make_idesc_bf16(128, PD, 0, 1);
     const bool lead = tc5::elect_one();                // converged warp, elected lane issues (see ssd_chunk_state_kernel)
-    auto wait = [&](uint64_t* bar, int phase, int code) {
-      return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
-    };
-    Items cur(p), ahead(p), behind(p);                 // the item of a step, the next to be loaded and scanned, the next to be stored
-    const int n = cur.n, item0 = blockIdx.x * p.quota;
-    auto load = [&](int k) {                           // item k, which is `ahead`
-      const int s = k % OUT_ST;
-      uint8_t* st = stages + s * 2 * BOXB;
-      tc5::mbar_expect_tx(full + s, 2 * BOXB);
-      tc5::tma_load_4d(st, &tm_x, full + s, 0, ahead.h, ahead.t0, ahead.b);
-      tc5::tma_load_2d(st + BOXB, &tm_h, full + s, 0, (item0 + k) * NS);
-    };
-    auto load_bc = [&]() {                             // of the chunk of `cur`
-      tc5::mbar_expect_tx(cb, 4 * BOXB);
-      tc5::tma_load_3d(sC, &tm_c, cb, 0, cur.t0, cur.b);
-      tc5::tma_load_3d(sC + BOXB, &tm_c, cb, 64, cur.t0, cur.b);
-      tc5::tma_load_3d(sB, &tm_b, cb, 0, cur.t0, cur.b);
-      tc5::tma_load_3d(sB + BOXB, &tm_b, cb, 64, cur.t0, cur.b);
-    };
-    auto store = [&](int k) {                          // item k, which is `behind`; rows past T are clipped by the copy engine
-      tc5::tma_store_4d(&tm_y, stages + (k % OUT_ST) * 2 * BOXB, 0, behind.h, behind.t0, behind.b);
-      tc5::tma_store_commit();
-    };
-    auto scan_item = [&](int k, float4 dt, float a) {
-      float* at = scan + (k & 1) * (2 * L + 192);
-      chunk_scan_warp<true>(dt, a, at, at + L, at + 2 * L);
-      arrive_warp(scanned + (k & 1));
-    };
-    if (lead) load_bc();
-    for (int k = 0; k < 2 && k < n; ++k, ahead.next()) {
-      if (lead) load(k);
-      scan_item(k, load_dt4(p, ahead), p.A[ahead.h]);
-    }
+    Items cur(p);
+    const int n = cur.n;
     const uint64_t cc = tc5::desc_kmajor(tc5::smem_u32(sC)), bb = tc5::desc_kmajor(tc5::smem_u32(sB));
-    bool ok = true;
     int seg = 0;
     for (int k = 0; k < n; ++k, cur.next()) {
       const int buf = k & 1, s = k % OUT_ST;
-      float4 dt_next = make_float4(0.f, 0.f, 0.f, 0.f);
-      float a_next = 0.f;
-      if (k + 2 < n) { dt_next = load_dt4(p, ahead); a_next = p.A[ahead.h]; }
       if (cur.opens(k)) {
-        if (k > 0) {                                   // C is read by the products of item k - 1
-          if (!(ok = wait(done + (buf ^ 1), (k - 1) >> 1, STATUS_TIMEOUT_TMEM_FULL))) break;
-          if (lead) load_bc();
-          if (!(ok = wait(sread, seg - 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
-        }
-        if (!(ok = wait(cb, seg, STATUS_TIMEOUT_SMEM_FULL))) break;
+        if (k > 0 && !wait(sread, seg - 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+        if (!wait(cb, seg, STATUS_TIMEOUT_SMEM_FULL)) break;
         tc5::fence_after_sync();
         if (lead) {
 #pragma unroll
@@ -443,17 +407,19 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
         __syncwarp();
         ++seg;
       }
-      if (!(ok = wait(full + s, k / OUT_ST, STATUS_TIMEOUT_SMEM_FULL))) break;
+      if (k > 1 && !wait(left + (k - 2) % OUT_ST, (k - 2) / OUT_ST, STATUS_TIMEOUT_TMEM_EMPTY)) break;      // its columns are free
+      if (!wait(full + s, k / OUT_ST, STATUS_TIMEOUT_SMEM_FULL)) break;
+      tc5::fence_after_sync();
       const uint64_t xx = tc5::desc_mnmajor(tc5::smem_u32(stages + s * 2 * BOXB), BOXB);
       const uint64_t hh = tc5::desc_mnmajor(tc5::smem_u32(stages + s * 2 * BOXB + BOXB), BOXB);
-      if (lead) {                                      // rows of item k - 2 have left these columns (see below)
+      if (lead) {
 #pragma unroll
         for (int kk = 0; kk < NS / 16; ++kk)
           tc5::mma_ss(tmem + cYi + buf * 64, cc + static_cast<uint64_t>(((kk >> 2) * BOXB + (kk & 3) * 32) >> 4),
                       hh + static_cast<uint64_t>((kk * 2048) >> 4), id_y, kk > 0 ? 1u : 0u);
       }
       __syncwarp();
-      if (!(ok = wait(ready + buf, k >> 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+      if (!wait(ready + buf, k >> 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;
       tc5::fence_after_sync();
       if (lead) {
 #pragma unroll
@@ -462,10 +428,40 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
         tc5::mma_commit(done + buf);
       }
       __syncwarp();
-      if (k + 2 < n) scan_item(k + 2, dt_next, a_next);        // this item's sums have been read
-      if (k > 0) {
-        if (!(ok = wait(left + (buf ^ 1), (k - 1) >> 1, STATUS_TIMEOUT_TMEM_EMPTY))) break;
-        tc5::fence_after_sync();
+    }
+  } else if (warp == 17) {                             // loads and stores
+    const bool lead = tc5::elect_one();
+    Items cur(p), ahead(p), behind(p);                 // the item of a step, the next to be loaded, the next to be stored
+    const int n = cur.n, item0 = blockIdx.x * p.quota;
+    auto load = [&](int k) {                           // item k, which is `ahead`
+      const int s = k % OUT_ST;
+      uint8_t* st = stages + s * 2 * BOXB;
+      tc5::mbar_expect_tx(full + s, 2 * BOXB);
+      tc5::tma_load_4d(st, &tm_x, full + s, 0, ahead.h, ahead.t0, ahead.b);
+      tc5::tma_load_2d(st + BOXB, &tm_h, full + s, 0, (item0 + k) * NS);
+    };
+    auto store = [&](int k) {                          // item k, which is `behind`; rows past T are clipped by the copy engine
+      tc5::tma_store_4d(&tm_y, stages + (k % OUT_ST) * 2 * BOXB, 0, behind.h, behind.t0, behind.b);
+      tc5::tma_store_commit();
+    };
+    bool ok = true;
+    for (int k = 0; k < n; ++k, cur.next()) {
+      if (cur.opens(k)) {                              // C and B of its chunk, over those that the products of item k - 1 read
+        if (k > 0 && !(ok = wait(done + ((k - 1) & 1), (k - 1) >> 1, STATUS_TIMEOUT_TMEM_FULL))) break;
+        if (lead) {
+          tc5::mbar_expect_tx(cb, 4 * BOXB);
+          tc5::tma_load_3d(sC, &tm_c, cb, 0, cur.t0, cur.b);
+          tc5::tma_load_3d(sC + BOXB, &tm_c, cb, 64, cur.t0, cur.b);
+          tc5::tma_load_3d(sB, &tm_b, cb, 0, cur.t0, cur.b);
+          tc5::tma_load_3d(sB + BOXB, &tm_b, cb, 64, cur.t0, cur.b);
+        }
+        __syncwarp();
+      }
+      if (k == 0) {
+        for (int i = 0; i < 2 && i < n; ++i, ahead.next())
+          if (lead) load(i);
+      } else {
+        if (!(ok = wait(left + (k - 1) % OUT_ST, (k - 1) / OUT_ST, STATUS_TIMEOUT_TMEM_EMPTY))) break;
         if (lead) store(k - 1);
         behind.next();
       }
@@ -476,7 +472,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
       ahead.next();
       __syncwarp();
     }
-    if (ok && wait(left + ((n - 1) & 1), (n - 1) >> 1, STATUS_TIMEOUT_TMEM_EMPTY)) {
+    if (ok && wait(left + (n - 1) % OUT_ST, (n - 1) / OUT_ST, STATUS_TIMEOUT_TMEM_EMPTY)) {
       if (lead) store(n - 1);
     } else if (lead) {                                 // loads may still be in flight
       for (int i = 0; i < OUT_ST; ++i) tc5::mbar_drain(full + i);
@@ -484,12 +480,26 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
     }
     if (lead) tc5::tma_store_wait_read<0>();
     __syncwarp();
+  } else if (warp == 18) {                             // sums of step sizes, two items ahead
+    Items cur(p);
+    const int n = cur.n;
+    float4 dt = load_dt4(p, cur);
+    float a = p.A[cur.h];
+    for (int k = 0; k < n; ++k) {
+      float4 dt_next = make_float4(0.f, 0.f, 0.f, 0.f);
+      float a_next = 0.f;
+      cur.next();
+      if (k + 1 < n) { dt_next = load_dt4(p, cur); a_next = p.A[cur.h]; }
+      if (k > 1 && !wait(ready + (k & 1), (k >> 1) - 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;       // those of item k - 2 have been read
+      float* at = scan + (k & 1) * (2 * L + 192);
+      chunk_scan_warp<true>(dt, a, at, at + L, at + 2 * L);
+      arrive_warp(scanned + (k & 1));
+      dt = dt_next;
+      a = a_next;
+    }
   } else {
     const int r = threadIdx.x & 127, lane = r & 31, quad = warp & 3, grp = warp >> 2;    // row, its block of 32, column block
     const uint32_t lanes = tmem + (static_cast<uint32_t>(quad * 32) << 16);
-    auto wait = [&](uint64_t* bar, int phase, int code) {
-      return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
-    };
     float s[32];                                       // C_i . B_j of the segment: row i = r, columns j = 32 grp ..
     float e_open = 0.f, dsk_open = 0.f;                // exp(cum) and skip weight of the item whose rows are still open
     Items cur(p);
@@ -560,7 +570,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
           *reinterpret_cast<uint4*>(base + (((grp * 2 + j) ^ (r & 7)) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
         tc5::fence_proxy_async();
         tc5::fence_before_sync();
-        arrive_warp(left + buf);
+        arrive_warp(left + q % OUT_ST);
       }
       e_open = e;
       dsk_open = dsk;
@@ -1533,7 +1543,7 @@ extern "C" int nsa_ssd_chunk_out(const void* Cm, long ld_c, const void* Bm, long
   static bool cfg = false;
   if (!cfg) { if ((rc = smem_attr(ssd_chunk_out_kernel, OUT_SMEM))) return rc; cfg = true; }
   if ((rc = map_v(&ty, y, B, T, H, static_cast<long>(H) * PD))) return rc;
-  ssd_chunk_out_kernel<<<deal_items(p), 544, OUT_SMEM, st>>>(tc, tb, tx, th, ty, p);
+  ssd_chunk_out_kernel<<<deal_items(p), 608, OUT_SMEM, st>>>(tc, tb, tx, th, ty, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_chunk_out launch");
