@@ -826,57 +826,39 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // 16-token cells, a selection block four cells).  Same pipeline as the forward kernel above
 // without the P V product: Q in tensor memory, K stream through the shared-memory ring, the two
 // softmax groups on alternate 64-key visits.
+// A tile has T / 2048 visits in the mean, so half of a CTA's time is its start and its end, and two CTAs share an SM: four
+// stages of K, 256 columns of tensor memory, scores taken 32 at a time.  The sum over heads halves the bins that a lane keeps in
+// each step (16 heads: 15 shuffles, and 64 where every lane sums every bin; the same tree of additions, the same bits), so a token's bins
+// leave as one 64-byte write.  32 query and 2 KV heads, one CTA per SM and all bins everywhere -> now: 2 x 2048 tokens 35 -> 26 us,
+// 16384 295 -> 186, 65536 3615 -> 2220.
 // --------------------------------------------------------------------------------------
-constexpr int IMP_STAGES = 6;
+constexpr int IMP_STAGES = 4;
+constexpr int IMP_SMEM = (4 + 2 * IMP_STAGES) * HALF + 1024 + 256;
 
-__global__ void __launch_bounds__(320, 1)
-attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                   const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
+__global__ void __launch_bounds__(320, 2)
+attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const AttnParams p) {
   constexpr int D = 128;
   constexpr int QT = 4 * HALF;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sKV = sQ + QT;                        // [stages][K: 2 k-blocks of [64][64] | V: same]
-  float* merge = reinterpret_cast<float*>(sKV + IMP_STAGES * 2 * HALF);   // [2][128]: group 1's m and l
-  uint64_t* bars = reinterpret_cast<uint64_t*>(merge + 256);
+  uint8_t* sK = sQ + QT;                         // [stages][2 k-blocks of [64][64]]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sK + IMP_STAGES * 2 * HALF);
   uint64_t* q_full = bars;
-  uint64_t* kv_full = bars + 1;                  // [stages]
-  uint64_t* kv_empty = kv_full + IMP_STAGES;      // [stages]
-  uint64_t* s_full = kv_empty + IMP_STAGES;       // [2]
+  uint64_t* k_full = bars + 1;                   // [stages]
+  uint64_t* k_empty = k_full + IMP_STAGES;       // [stages]
+  uint64_t* s_full = k_empty + IMP_STAGES;       // [2]
   uint64_t* s_empty = s_full + 2;                // [2]
-  uint64_t* p_full = s_empty + 2;                // [2]
-  uint64_t* qt_full = p_full + 2;                // softmax -> MMA: Q is in tensor memory
-  uint64_t* acc_done = qt_full + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+  uint64_t* qt_full = s_empty + 2;               // softmax -> MMA: Q is in tensor memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(qt_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // always causal: longest tiles first
   const int q0 = qt * p.R;
-  const int t_hi = min(q0 + p.R, p.T) - 1;
-  const bool selected = p.tile_blocks != nullptr;
-  const long tile_slot = (static_cast<long>(b) * p.Hkv + h) * gridDim.x + qt;
-  const int* blocks = selected ? p.tile_blocks + tile_slot * p.max_u : nullptr;
-  const unsigned long long* masks = selected ? p.tile_masks + tile_slot * p.max_u : nullptr;
-  int kb0 = 0, n_vis;
-  if (selected) {
-    n_vis = min(p.tile_counts[tile_slot], p.max_u);
-  } else {
-    long last = p.S - 1;
-    if (p.causal) {
-      long lim = static_cast<long>(t_hi) - p.kp_off;
-      lim = lim < 0 ? -1 : lim / p.kp_stride;
-      last = lim < last ? lim : last;
-    }
-    long first = 0;
-    if (p.window > 0) {
-      const long lo = static_cast<long>(q0) - p.window + 1 - p.kp_off;
-      first = lo <= 0 ? 0 : (lo + p.kp_stride - 1) / p.kp_stride;
-    }
-    kb0 = static_cast<int>(first / 64);
-    n_vis = last < first ? 0 : static_cast<int>(last / 64) + 1 - kb0;
-  }
+  const int lim = min(q0 + p.R, p.T) - 1 - p.kp_off;
+  const int last = min(lim < 0 ? -1 : lim / p.kp_stride, p.S - 1);
+  const int n_vis = last < 0 ? 0 : last / 64 + 1;
 
   if (warp == 8 && lane == 0) {        // descriptor fetch off the first copy's critical path
     tc5::prefetch_tensormap(&tm_q);
@@ -885,23 +867,17 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   if (tid == 0) {
     *abort_flag = 0;
     tc5::mbar_init(q_full, 1);
-    for (int i = 0; i < IMP_STAGES; ++i) { tc5::mbar_init(kv_full + i, 1); tc5::mbar_init(kv_empty + i, 1); }
-    for (int i = 0; i < 2; ++i) {
-      tc5::mbar_init(s_full + i, 1);
-      tc5::mbar_init(s_empty + i, 128);
-      tc5::mbar_init(p_full + i, 128);
-    }
+    for (int i = 0; i < IMP_STAGES; ++i) { tc5::mbar_init(k_full + i, 1); tc5::mbar_init(k_empty + i, 1); }
+    for (int i = 0; i < 2; ++i) { tc5::mbar_init(s_full + i, 1); tc5::mbar_init(s_empty + i, 128); }
     tc5::mbar_init(qt_full, 256);
-    tc5::mbar_init(acc_done, 1);
     tc5::fence_barrier_init();
   }
-  if (warp == 9) { tc5::tmem_alloc(tmem_slot, 512); tc5::tmem_relinquish(); }
+  if (warp == 9) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  // columns: S of group g at g*64; O of group g at 128 + g*128
-  constexpr uint32_t cO = 128, cQ = 384;
+  constexpr uint32_t cQ = 128;                   // S of group g at g*64
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
@@ -910,47 +886,29 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 #pragma unroll
       for (int kb = 0; kb < 2; ++kb) tc5::tma_load_5d(sQ + kb * 2 * HALF, &tm_q, q_full, kb * 64, 0, h, q0, b);
       bool ok = true;
-      int issued = 0;
-      int blk_n = selected ? blocks[0] : 0;
-      for (int v = 0; v < n_vis; ++v) {
+      for (int v = 0; v < n_vis && ok; ++v) {
         const int st = v % IMP_STAGES;
-        const int blk = blk_n;
-        if (selected && v + 1 < n_vis) blk_n = blocks[v + 1];
-        if (!tc5::mbar_wait(kv_empty + st, ((v / IMP_STAGES) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY)) { ok = false; break; }
-        const int s0 = selected ? (blk < 0 ? 0 : blk * 64) : (kb0 + v) * 64;
-        uint8_t* kd = sKV + st * 2 * HALF;
-        tc5::mbar_expect_tx(kv_full + st, 2 * HALF);
+        ok = tc5::mbar_wait(k_empty + st, ((v / IMP_STAGES) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY);
+        if (!ok) break;
+        uint8_t* kd = sK + st * 2 * HALF;
+        tc5::mbar_expect_tx(k_full + st, 2 * HALF);
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) tc5::tma_load_4d(kd + kb * HALF, &tm_k, kv_full + st, kb * 64, h, s0, b);
-        issued = v + 1;
+        for (int kb = 0; kb < 2; ++kb) tc5::tma_load_4d(kd + kb * HALF, &tm_k, k_full + st, kb * 64, h, v * 64, b);
       }
-      if (!ok) {
-        // let the copies already issued land before the CTA's shared memory is released
-        for (int j = max(0, issued - IMP_STAGES); j < issued; ++j) {
-          const long long t0 = clock64();
-          for (uint32_t i = 0; i < tc5::kMaxPolls; ++i) {
-            if (tc5::mbar_try_wait(kv_full + (j % IMP_STAGES), (j / IMP_STAGES) & 1)) break;
-            if ((i & 255u) == 255u && clock64() - t0 > tc5::kMaxWaitCycles) break;
-          }
-        }
-        const long long t0 = clock64();
-        for (uint32_t i = 0; i < tc5::kMaxPolls; ++i) {
-          if (tc5::mbar_try_wait(q_full, 0)) break;
-          if ((i & 255u) == 255u && clock64() - t0 > tc5::kMaxWaitCycles) break;
-        }
-      }
+      if (!ok)         // let the copies already issued land before the CTA's shared memory is released
+        for (int i = 0; i < 1 + IMP_STAGES; ++i) tc5::mbar_drain(bars + i);
     }
   } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer (converged warp, elected lane issues)
     if (n_vis > 0) {
       const bool lead = tc5::elect_one();
       constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 64, 0, 0);
-      const uint64_t bK0 = tc5::desc_kmajor(tc5::smem_u32(sKV));
+      const uint64_t bK0 = tc5::desc_kmajor(tc5::smem_u32(sK));
       bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(qt_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
       if (ok) tc5::fence_after_sync();
       for (int v = 0; v < n_vis && ok; ++v) {
         const int st = v % IMP_STAGES, g = v & 1;
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(kv_full + st, (v / IMP_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+        ok = __all_sync(0xffffffffu, tc5::mbar_wait(k_full + st, (v / IMP_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
                                      tc5::mbar_wait(s_empty + g, ((v >> 1) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
         if (!ok) break;
         tc5::fence_after_sync();
@@ -961,7 +919,7 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             tc5::mma_ts(tmem + g * 64, tmem + cQ + kk * 8, bK + static_cast<uint64_t>(((kk >> 2) * HALF + (kk & 3) * 32) >> 4), id_s,
                         kk > 0 ? 1u : 0u);
           tc5::mma_commit(s_full + g);
-          tc5::mma_commit(kv_empty + st);          // the K stage is free once S is complete
+          tc5::mma_commit(k_empty + st);           // the K stage is free once S is complete
         }
         __syncwarp();
       }
@@ -977,6 +935,9 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     const float sc = p.scale_log2;
     const float Lrow = row_ok ? p.L_in[rowi] : 0.f;
     const float negL = Lrow == -INFINITY ? -INFINITY : -Lrow;     // a row that sees no key: -inf - inf, not -inf + inf
+    float* const row = p.imp + ((static_cast<long>(b) * p.Hkv + h) * p.T + t) * p.nS;
+    const int first = p.G <= 16 ? gh * 16 / p.G : gh >> 1;        // the bins whose sum over heads this lane ends with
+    const int mine = !row_ok || (p.G == 32 && (gh & 1)) ? 0 : max(1, 16 / p.G);
     bool ok = true;
     if (n_vis > 0) {
       // Q: shared memory (swizzled [128 rows][64] k-blocks) -> TMEM; thread (r, grp) copies k-block grp of its row
@@ -997,49 +958,67 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     }
     int n_mine = 0;
     for (int v = grp; v < n_vis && ok; v += 2, ++n_mine) {
-      const int sb = (kb0 + v) * 64;
       if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + grp, n_mine & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
         ok = false;
         break;
       }
       tc5::fence_after_sync();
-      uint32_t sv[64];
-      tmem_ld64(tmem + lane_off + grp * 64, sv);
-      tc5::fence_before_sync();
-      tc5::mbar_arrive(s_empty + grp);
       // compressed key i covers 16-token cells i and i+1; a selection block is 4 cells
       float bins[17];
 #pragma unroll
       for (int i = 0; i < 17; ++i) bins[i] = 0.f;
-      if (row_ok) {
-        const bool check = (sb + 63 >= p.S) || ((sb + 63) * p.kp_stride + p.kp_off > t);
-        if (check) mask_scores<64>(p, sv, sb, t);
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {                    // masked scores are -inf: their probability is 0
+      for (int c = 0; c < 64; c += 32) {
+        uint32_t sv[32];
+        tc5::tmem_ld_x32(tmem + lane_off + grp * 64 + c, sv);
+        tc5::tmem_ld_wait();
+        if (c == 32) {
+          tc5::fence_before_sync();
+          tc5::mbar_arrive(s_empty + grp);
+        }
+        if (!row_ok) continue;
+        const int sb = v * 64 + c;
+        if ((sb + 31 >= p.S) || ((sb + 31) * p.kp_stride + p.kp_off > t)) mask_scores<32>(p, sv, sb, t);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {                    // masked scores are -inf: their probability is 0
           const float pr = exp2f(fmaf(__uint_as_float(sv[i]), sc, negL));
-          bins[i / 4] += pr;
-          bins[(i + 1) / 4] += pr;
+          bins[(c + i) / 4] += pr;
+          bins[(c + i + 1) / 4] += pr;
         }
       }
-      for (int o = p.G >> 1; o > 0; o >>= 1)
 #pragma unroll
-        for (int i = 0; i < 17; ++i) bins[i] += __shfl_xor_sync(0xffffffffu, bins[i], o);
-      if (gh == 0 && row_ok) {
-        // bins 1..15 receive keys of this visit only: plain stores.  Bin 0 also receives the last key
-        // of the previous visit (its bin 16), so only those two go through a reduction.
-        const int jb = sb / 4;
-        float* dst = p.imp + ((static_cast<long>(b) * p.Hkv + h) * p.T + t) * p.nS;
+      for (int step = 0; step < 5; ++step) {              // the lane with bit o of its head keeps the upper n bins, the other the lower
+        const int n = 8 >> step, o = p.G >> (step + 1);
+        if (o == 0) break;
+        if (n > 0) {
 #pragma unroll
-        for (int i = 1; i < 16; ++i)
-          if (jb + i < p.nS) dst[jb + i] = bins[i];
-        if (jb < p.nS && bins[0] != 0.f) atomicAdd(dst + jb, bins[0]);
-        if (jb + 16 < p.nS && bins[16] != 0.f) atomicAdd(dst + jb + 16, bins[16]);
+          for (int i = 0; i < n; ++i) {
+            const float lo = bins[i], hi = bins[n + i];
+            const float got = __shfl_xor_sync(0xffffffffu, gh & o ? lo : hi, o);
+            bins[i] = (gh & o ? hi : lo) + got;
+          }
+        } else {
+          bins[0] += __shfl_xor_sync(0xffffffffu, bins[0], o);
+        }
+        bins[16] += __shfl_xor_sync(0xffffffffu, bins[16], o);
       }
+      // bins 1..15 receive keys of this visit only: plain stores.  Bin 0 also receives the last key
+      // of the previous visit (its bin 16), so only those two go through a reduction.
+      const int jb = v * 16;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int j = first + i;
+        if (i < mine && jb + j < p.nS) {
+          if (j > 0) row[jb + j] = bins[i];
+          else if (bins[i] != 0.f) atomicAdd(row + jb, bins[i]);
+        }
+      }
+      if (gh == 0 && row_ok && jb + 16 < p.nS && bins[16] != 0.f) atomicAdd(row + jb + 16, bins[16]);
     }
   }
   tc5::fence_before_sync();
   __syncthreads();
-  if (warp == 9) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 512); }
+  if (warp == 9) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 256); }
 }
 
 // --------------------------------------------------------------------------------------
@@ -3213,10 +3192,9 @@ extern "C" int nsa_attn_importance(const void* q, const void* k_cmp, const float
   const int smem = (D / 64) * 2 * HALF * 5 + 4 * HALF + 1024 + 2048;
   static const bool legacy = [] { const char* e = getenv("NSA_B200_ATTN_IMP"); return e && !strcmp(e, "legacy"); }();
   if (D == 128 && !legacy && 128 % (Hq / Hkv) == 0) {
-    const int smem_ts = (4 + 2 * IMP_STAGES) * HALF + 1024 + 1024 + 256;
     static bool cfg = false;
-    if (!cfg) { if ((rc = set_smem(attn_importance_ts_kernel, smem_ts))) return rc; cfg = true; }
-    attn_importance_ts_kernel<<<grid, 320, smem_ts, st>>>(tq, tk, tk, p);
+    if (!cfg) { if ((rc = set_smem(attn_importance_ts_kernel, IMP_SMEM))) return rc; cfg = true; }
+    attn_importance_ts_kernel<<<grid, 320, IMP_SMEM, st>>>(tq, tk, p);
   } else if (D == 128) {
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(attn_fwd_kernel<128, 1>, smem))) return rc; cfg = true; }
