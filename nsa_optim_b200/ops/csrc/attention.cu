@@ -820,6 +820,301 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 }
 
 // --------------------------------------------------------------------------------------
+// Forward, two CTAs per SM: the pipeline of the kernel above with one softmax group per CTA instead of two, which takes
+// all visits of its tile.  An SM works on two tiles then, and the start and the end of one (4 K cycles to the first
+// scores, 4 K from the last to the exit) run beside the visits of the other; nothing is merged.  Half of the shared memory and of the tensor memory
+// is left to a CTA: two stages of K and of V, S and P and O in 256 columns, Q in shared memory.
+// 8192 tokens x 32 query and 2 KV heads: 591 -> 510 us, without causality 1089 -> 1068, window 512 158 -> 113; 16384 2235 -> 2091.
+// (Visits of 128 keys in one CTA, P over S: 16384 2386 us, window 512 174; S then waits for P V of the visit before.)
+// --------------------------------------------------------------------------------------
+constexpr int FW1_STAGES = 2;
+constexpr int FW1_SMEM = (4 + 4 * FW1_STAGES) * HALF + 1024 + 256;
+
+template <bool LONGEST_FIRST>
+__global__ void __launch_bounds__(224, 2)
+attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                     const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
+  constexpr int D = 128;
+  constexpr int QT = 4 * HALF;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sQ = smem;                            // [2 k-blocks][128 rows][64]
+  uint8_t* sK = sQ + QT;                         // [stages][2 k-blocks of [64][64]]
+  uint8_t* sV = sK + FW1_STAGES * 2 * HALF;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + FW1_STAGES * 2 * HALF);
+  uint64_t* q_full = bars;
+  uint64_t* k_full = bars + 1;                   // [stages]
+  uint64_t* v_full = k_full + FW1_STAGES;        // [stages]
+  uint64_t* k_empty = v_full + FW1_STAGES;       // [stages]
+  uint64_t* v_empty = k_empty + FW1_STAGES;      // [stages]
+  uint64_t* s_full = v_empty + FW1_STAGES;
+  uint64_t* s_empty = s_full + 1;
+  uint64_t* p_full = s_empty + 1;
+  uint64_t* p_empty = p_full + 1;                // P V of the previous visit is done
+  uint64_t* acc_done = p_empty + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int qt = LONGEST_FIRST ? gridDim.x - 1 - blockIdx.x : blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int q0 = qt * p.R;
+  const int t_hi = min(q0 + p.R, p.T) - 1;
+  const bool selected = p.tile_blocks != nullptr;
+  const long tile_slot = (static_cast<long>(b) * p.Hkv + h) * gridDim.x + qt;
+  const int* blocks = selected ? p.tile_blocks + tile_slot * p.max_u : nullptr;
+  const unsigned long long* masks = selected ? p.tile_masks + tile_slot * p.max_u : nullptr;
+  int kb0 = 0, n_vis;
+  if (selected) {
+    n_vis = min(p.tile_counts[tile_slot], p.max_u);
+  } else {
+    long last = p.S - 1;
+    if (p.causal) {
+      long lim = static_cast<long>(t_hi) - p.kp_off;
+      lim = lim < 0 ? -1 : lim / p.kp_stride;
+      last = lim < last ? lim : last;
+    }
+    long first = 0;
+    if (p.window > 0) {
+      const long lo = static_cast<long>(q0) - p.window + 1 - p.kp_off;
+      first = lo <= 0 ? 0 : (lo + p.kp_stride - 1) / p.kp_stride;
+    }
+    kb0 = static_cast<int>(first / 64);
+    n_vis = last < first ? 0 : static_cast<int>(last / 64) + 1 - kb0;
+  }
+
+  if (warp == 4 && lane == 0) {        // descriptor fetch off the first copy's critical path
+    tc5::prefetch_tensormap(&tm_q);
+    tc5::prefetch_tensormap(&tm_k);
+    tc5::prefetch_tensormap(&tm_v);
+  }
+  if (tid == 0) {
+    *abort_flag = 0;
+    tc5::mbar_init(q_full, 1);
+    for (int i = 0; i < 4 * FW1_STAGES; ++i) tc5::mbar_init(k_full + i, 1);
+    tc5::mbar_init(s_full, 1);
+    tc5::mbar_init(s_empty, 128);
+    tc5::mbar_init(p_full, 128);
+    tc5::mbar_init(p_empty, 1);
+    tc5::mbar_init(acc_done, 1);
+    tc5::fence_barrier_init();
+  }
+  if (warp == 5) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
+  tc5::fence_before_sync();
+  __syncthreads();
+  tc5::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  constexpr uint32_t cP = 64, cO = 128;          // S at 0
+
+  if (warp == 4) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0 && n_vis > 0) {
+      tc5::mbar_expect_tx(q_full, QT);
+#pragma unroll
+      for (int kb = 0; kb < 2; ++kb) tc5::tma_load_5d(sQ + kb * 2 * HALF, &tm_q, q_full, kb * 64, 0, h, q0, b);
+      bool ok = true;
+      int blk_n = selected ? blocks[0] : 0;
+      for (int v = 0; v < n_vis && ok; ++v) {
+        const int st = v % FW1_STAGES;
+        const uint32_t par = ((v / FW1_STAGES) & 1) ^ 1;
+        const int s0 = selected ? max(blk_n, 0) * 64 : (kb0 + v) * 64;
+        if (selected && v + 1 < n_vis) blk_n = blocks[v + 1];
+        ok = tc5::mbar_wait(k_empty + st, par, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY);
+        if (!ok) break;
+        tc5::mbar_expect_tx(k_full + st, 2 * HALF);
+#pragma unroll
+        for (int kb = 0; kb < 2; ++kb) tc5::tma_load_4d(sK + (2 * st + kb) * HALF, &tm_k, k_full + st, kb * 64, h, s0, b);
+        ok = tc5::mbar_wait(v_empty + st, par, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY);
+        if (!ok) break;
+        tc5::mbar_expect_tx(v_full + st, 2 * HALF);
+#pragma unroll
+        for (int kb = 0; kb < 2; ++kb) tc5::tma_load_4d(sV + (2 * st + kb) * HALF, &tm_v, v_full + st, kb * 64, h, s0, b);
+      }
+      if (!ok)         // let the copies already issued land before the CTA's shared memory is released
+        for (int i = 0; i < 1 + 2 * FW1_STAGES; ++i) tc5::mbar_drain(bars + i);
+    }
+  } else if (warp == 5) {
+    // ------------------------------------------------------------------ MMA issuer 1: S = Q K^T
+    if (n_vis > 0) {
+      const bool lead = tc5::elect_one();
+      constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 64, 0, 0);
+      const uint64_t aQ = tc5::desc_kmajor(tc5::smem_u32(sQ)), bK0 = tc5::desc_kmajor(tc5::smem_u32(sK));
+      bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL));
+      for (int v = 0; v < n_vis && ok; ++v) {
+        const int st = v % FW1_STAGES;
+        ok = __all_sync(0xffffffffu, tc5::mbar_wait(k_full + st, (v / FW1_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+                                     tc5::mbar_wait(s_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
+        if (!ok) break;
+        tc5::fence_after_sync();
+        const uint64_t bK = bK0 + static_cast<uint64_t>((st * 2 * HALF) >> 4);
+        if (lead) {
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            tc5::mma_ss(tmem, aQ + static_cast<uint64_t>(((kk >> 2) * 2 * HALF + (kk & 3) * 32) >> 4),
+                        bK + static_cast<uint64_t>(((kk >> 2) * HALF + (kk & 3) * 32) >> 4), id_s, kk > 0 ? 1u : 0u);
+          tc5::mma_commit(s_full);
+          tc5::mma_commit(k_empty + st);
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp == 6) {
+    // ------------------------------------------------------------------ MMA issuer 2: O += P V
+    if (n_vis > 0) {
+      const bool lead = tc5::elect_one();
+      constexpr uint32_t id_o = tc5::make_idesc_bf16(128, D, 0, 1);
+      const uint64_t bV0 = tc5::desc_mnmajor(tc5::smem_u32(sV), HALF);
+      bool ok = true;
+      for (int u = 0; u < n_vis; ++u) {
+        const int st = u % FW1_STAGES;
+        ok = __all_sync(0xffffffffu, tc5::mbar_wait(v_full + st, (u / FW1_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+                                     tc5::mbar_wait(p_full, u & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+        if (!ok) break;
+        tc5::fence_after_sync();
+        const uint64_t bV = bV0 + static_cast<uint64_t>((st * 2 * HALF) >> 4);
+        if (lead) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            tc5::mma_ts(tmem + cO, tmem + cP + kk * 8, bV + static_cast<uint64_t>((kk * 2048) >> 4), id_o, (u > 0 || kk > 0) ? 1u : 0u);
+          tc5::mma_commit(p_empty);                // the P columns are free, the O accumulator is at rest
+          tc5::mma_commit(v_empty + st);
+        }
+        __syncwarp();
+      }
+      if (ok && lead) tc5::mma_commit(acc_done);
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax
+    const int r = tid;
+    const int tok_local = r / p.G, gh = r % p.G;
+    const int t = q0 + tok_local;
+    const bool row_ok = t < p.T;
+    const uint32_t lane_off = static_cast<uint32_t>(warp * 32) << 16;
+    const long rowi = (static_cast<long>(b) * p.T + (row_ok ? t : 0)) * p.Hq + h * p.G + gh;
+    const float sc = p.scale_log2;
+    float m_ref = -INFINITY, l_sum = 0.f;
+    bool ok = true;
+    int blk_n = 0;
+    unsigned long long msk_n = 0ull;
+    if (selected && n_vis > 0) { blk_n = blocks[0]; msk_n = masks[0]; }
+    for (int v = 0; v < n_vis && ok; ++v) {
+      int sb;
+      bool row_sel = row_ok;
+      if (!selected) sb = (kb0 + v) * 64;
+      else {
+        const int blk = blk_n;
+        const unsigned long long msk = msk_n;
+        if (v + 1 < n_vis) { blk_n = blocks[v + 1]; msk_n = masks[v + 1]; }
+        sb = blk < 0 ? -1 : blk * 64;
+        row_sel = row_ok && blk >= 0 && ((msk >> (tok_local & 63)) & 1ull);
+      }
+      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full, v & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+        ok = false;
+        break;
+      }
+      tc5::fence_after_sync();
+      uint32_t sv[64];
+      tmem_ld64(tmem + lane_off, sv);
+      tc5::fence_before_sync();
+      tc5::mbar_arrive(s_empty);                 // S of the next visit may be computed while this one is exponentiated
+      bool check = false;
+      float mx = -INFINITY;
+      if (row_sel) {
+        check = sb + 63 >= p.S;
+        if (p.causal) check = check || ((sb + 63) * p.kp_stride + p.kp_off > t);
+        if (p.window > 0) check = check || (sb * p.kp_stride + p.kp_off <= t - p.window);
+        if (check) mask_scores<64>(p, sv, sb, t);
+        // four independent chains: one serial chain of 64 dependent maxima is about 250 cycles of
+        // pure latency on the critical path of every visit
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int i = 0; i < 64; i += 4) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) m4[q] = fmaxf(m4[q], __uint_as_float(sv[i + q]));
+        }
+        mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      }
+      mx *= sc;
+      float alpha = 1.f;
+      if (mx != -INFINITY && (m_ref == -INFINITY || mx > m_ref + 8.f)) {
+        alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - mx);
+        m_ref = mx;
+      }
+      uint32_t pk[32];
+      float psum = 0.f;
+      if (!row_sel || m_ref == -INFINITY) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pk[i] = 0u;
+      } else {
+        float s4[4] = {0.f, 0.f, 0.f, 0.f};               // independent partial sums (see the maxima above)
+#pragma unroll
+        for (int i = 0; i < 64; i += 2) {                 // masked scores are -inf: their probability is 0
+          const float a = exp2f(fmaf(__uint_as_float(sv[i]), sc, -m_ref));
+          const float c = exp2f(fmaf(__uint_as_float(sv[i + 1]), sc, -m_ref));
+          s4[(i >> 1) & 3] += a + c;
+          pk[i / 2] = tc5::pack_bf16(a, c);
+        }
+        psum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      }
+      l_sum = l_sum * alpha + psum;
+      // P V of the previous visit must be done before P is overwritten or O rescaled
+      if (!__all_sync(0xffffffffu, tc5::mbar_wait(p_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY))) {
+        ok = false;
+        break;
+      }
+      tc5::fence_after_sync();
+      if (v > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+#pragma unroll 1
+        for (int q = 0; q < D; q += 16) {
+          uint32_t o[16];
+          tc5::tmem_ld_x16(tmem + lane_off + cO + q, o);
+          tc5::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tc5::tmem_st_x16(tmem + lane_off + cO + q, o);
+          tc5::tmem_st_wait();
+        }
+      }
+      tc5::tmem_st_x32(tmem + lane_off + cP, pk);
+      tc5::tmem_st_wait();
+      tc5::fence_before_sync();
+      tc5::mbar_arrive(p_full);
+    }
+    const bool done = __all_sync(0xffffffffu, ok && n_vis > 0 &&
+                                 tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+    if (done) tc5::fence_after_sync();
+    const bool have = done && l_sum > 0.f;
+    const float f = have ? 1.f / l_sum : 0.f;
+    if (row_ok) p.L[rowi] = have ? m_ref + log2f(l_sum) : -INFINITY;
+    bf16* dst = p.O + rowi * D;
+#pragma unroll
+    for (int q4 = 0; q4 < 4; ++q4) {
+      uint32_t a[32];
+      if (done) {
+        tc5::tmem_ld_x32(tmem + lane_off + cO + q4 * 32, a);
+        tc5::tmem_ld_wait();
+      }
+      if (row_ok) {
+        float o[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = have ? __uint_as_float(a[i]) * f : 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint4 o4;
+          o4.x = tc5::pack_bf16(o[8 * i], o[8 * i + 1]);
+          o4.y = tc5::pack_bf16(o[8 * i + 2], o[8 * i + 3]);
+          o4.z = tc5::pack_bf16(o[8 * i + 4], o[8 * i + 5]);
+          o4.w = tc5::pack_bf16(o[8 * i + 6], o[8 * i + 7]);
+          reinterpret_cast<uint4*>(dst + q4 * 32)[i] = o4;
+        }
+      }
+    }
+  }
+  tc5::fence_before_sync();
+  __syncthreads();
+  if (warp == 5) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 256); }
+}
+
+// --------------------------------------------------------------------------------------
 // Block importance for top-n selection, warp-specialised (head_dim 128).  A second pass over the
 // compressed keys with the row statistics L of the compressed branch: p = 2^(S c - L), summed over
 // the G heads of the group and binned into selection blocks (a compressed key covers two
@@ -3129,6 +3424,19 @@ void fill_params(AttnParams& p, int B, int T, int S, int Hq, int Hkv, int D, flo
 }
 }  // namespace
 
+// Two CTAs per SM with one softmax group each, or one with two?  A lone CTA takes its visits in one chain where the other form has two,
+// so there must be two CTAs and more for each SM, and of long tiles so many that the last ones weigh little.  Up to 20 visits
+// (two groups, one group): 152 CTAs x 19 visits 17 us, 22; 200 x 13 16.0, 17.5; 300 x 9 23.7, 18.7; 300 x 19 27, 27; 4096 x 9 311, 222.
+// More: 300 x 75 60, 72; 400 x 50 69.8, 69.7; 600 x 38 70, 55; 1200 x 75 220, 184; groups of one or two heads, whose neighbouring tiles
+// share no keys, are slower up to 1024 CTAs (600 x 75 129, 132; 1024 x 128 304, 309; 1536 x 192 695, 686).
+// Compressed keys always take two groups: their L goes into the choice of blocks, where a last bit decides between near ties (with one
+// group, compressed and selected branch together 1159 us at 16384 tokens, 1298 with two, a few rows took another block than before).
+static bool fwd_two_per_sm(const AttnParams& p, long ctas) {
+  if (p.kp_stride > 1) return false;
+  const int visits = (std::min(p.S, p.window > 0 ? p.window + p.R : p.S) + 63) / 64;
+  return ctas >= nsa::sm_count() * (visits <= 20 ? 2l : p.G >= 4 ? 4l : 8l);
+}
+
 extern "C" int nsa_attn_fwd(const void* q, const void* k, const void* v, void* o, float* L, int B, int T, int S,
                             int Hq, int Hkv, int D, float scale, int causal, int window, int kp_stride, int kp_off,
                             const int* tile_blocks, const unsigned long long* tile_masks, const int* tile_counts,
@@ -3146,7 +3454,13 @@ extern "C" int nsa_attn_fwd(const void* q, const void* k, const void* v, void* o
   const int smem = (D / 64) * 2 * HALF * 5 + 4 * HALF + 1024 + 2048;
   static const bool legacy = [] { const char* e = getenv("NSA_B200_ATTN_FWD"); return e && !strcmp(e, "legacy"); }();
   static const bool smem_operands = [] { const char* e = getenv("NSA_B200_ATTN_FWD"); return e && !strcmp(e, "smem"); }();
-  if (D == 128 && !legacy && !smem_operands) {
+  if (D == 128 && !legacy && !smem_operands && fwd_two_per_sm(p, static_cast<long>(grid.x) * Hkv * B)) {
+    auto* kernel = longest_first(p) ? attn_fwd_half_kernel<true> : attn_fwd_half_kernel<false>;
+    static bool cfg[2] = {};
+    bool& ready = cfg[longest_first(p)];
+    if (!ready) { if ((rc = set_smem(kernel, FW1_SMEM))) return rc; ready = true; }
+    kernel<<<grid, 224, FW1_SMEM, st>>>(tq, tk, tv, p);
+  } else if (D == 128 && !legacy && !smem_operands) {
     const int smem_ts = (4 + 4 * FWT_STAGES) * HALF + 1024 + 1024 + 256;
     auto* kernel = longest_first(p) ? attn_fwd_ts_kernel<true> : attn_fwd_ts_kernel<false>;
     static bool cfg[2] = {};
