@@ -83,7 +83,8 @@ constexpr int WARP_MMA = 8, WARP_LOAD = 9;
 // A chunk's tiles are asked for into L2 this many chunks ahead: two stages alone leave a load from memory one chunk's time,
 // and the chain then waits for it.  256 chunks x 64 CTAs, forward and backward: 472 and 526 us with one thread for copies,
 // stores and products, 455 and 597 with warps for each, 395 and 492 with the prefetch and operands released where their last
-// product is issued, 356 and 365 with u and do as tiles too (rows of their own per thread are 32 lines an instruction).
+// product is issued, 356 and 365 with u and do as tiles too (rows of their own per thread are 32 lines an instruction),
+// 336 and 361 with the wait for a tile's last stores in front of the one for the state.
 constexpr int AHEAD = 6;
 __device__ __forceinline__ void arrive_warp(uint64_t* bar) {
   __syncwarp();

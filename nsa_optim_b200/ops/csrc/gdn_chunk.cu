@@ -306,7 +306,7 @@ __device__ __forceinline__ void tmem_cols(uint32_t taddr, float (&out)[N]) {
 // columns stream through two TMA stages (as warp products with register accumulators they were two thirds of the
 // kernel: 700 us at 16384 tokens x 16 heads).  What is left are 64-row products, done by warps; they are two thirds of a CTA's 42000 cycles,
 // and one CTA fills an SM, so the next chunk's tiles are asked for into L2 meanwhile (670 us without that and with
-// 2 x 4 tiles for dA, 641 now).  Per token and head
+// 2 x 4 tiles for dA, 641 with both, 632 with the operands of dv read once per chunk and no loads under conditions).  Per token and head
 // 3.5 KB come in and 1 KB goes out, against 6 KB alone for the per-V-tile partials of dw, dq and dk that the sequential
 // pass would otherwise write and re-read.
 __global__ void __launch_bounds__(512, 1)
