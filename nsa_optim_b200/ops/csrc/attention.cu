@@ -3556,10 +3556,11 @@ extern "C" int nsa_attn_bwd(const void* q, const void* k, const void* v, const v
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_attn_bwd launch");
 }
 
-// Query tiles that one 128-key block can be visited by, at most
-static int key_visits(int T, int R, int window, int kp_stride) {
+// Query tiles that one 128-key block can be visited by, at most.  A window limits them only where causality does too: without
+// it a key is seen by every token up to a window after it.
+static int key_visits(int T, int R, int causal, int window, int kp_stride) {
   const int n_qt = (T + R - 1) / R;
-  return window > 0 ? std::min(n_qt, (127 * kp_stride + window - 1) / R + 2) : n_qt;
+  return causal && window > 0 ? std::min(n_qt, (127 * kp_stride + window - 1) / R + 2) : n_qt;
 }
 // Walks per 128-key block for nsa_attn_bwd_split over contiguous ranges, whose sums it wants room for (`part`, floats: walks x 2 x
 // B S Hkv D) if they are more than one; 0: walks of `visits_per_cta` tiles that add to dK and dV in any order.
@@ -3567,9 +3568,9 @@ static int key_visits(int T, int R, int window, int kp_stride) {
 // visits and more, three for each SM (half of a causal grid is empty; with two, 110 us where three take 96).  2048 tokens, two groups of 16 heads: one walk a block 423 us, 128
 // visits 220, 32 visits 74.  Blocks of more than 256 visits fill the GPU with walks of 64 (128 within 2 %), and room for all
 // their sums would cost more than it gives.
-extern "C" int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int window, int kp_stride) {
+extern "C" int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride) {
   if (Hkv <= 0 || Hq < Hkv) return 0;
-  const int most = key_visits(T, std::max(1, BM / (Hq / Hkv)), window, kp_stride);
+  const int most = key_visits(T, std::max(1, BM / (Hq / Hkv)), causal, window, kp_stride);
   if (most > 256) return 0;
   const long blocks = static_cast<long>((S + 127) / 128) * B * Hkv;
   const long want = (3l * nsa::sm_count() + blocks - 1) / std::max(1l, blocks);
@@ -3638,7 +3639,7 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
     if ((rc = make_q_map(&tdo1, d_o, B, T, Hq, Hkv, D, 1))) return rc;
     attn_bwd_kv_kernel<<<item_bound, KV_THREADS, smem, st>>>(tq1, tdo1, tk, tv, p, w, scale);
   } else {
-    const int most = key_visits(T, p.R, window, kp_stride);
+    const int most = key_visits(T, p.R, causal, window, kp_stride);
     KeyWalks w{};
     w.part = walks > 1 ? part : nullptr;
     if (walks > 1 && part == nullptr) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: several walks need room for their sums");

@@ -20,7 +20,7 @@ SIGNATURES = {
     "nsa_affine_quant": "ippppliiip",
     "nsa_attn_bwd": "ippppppppppiiiiiifiiiipppip",
     "nsa_attn_bwd_split": "ippppppppppiiiiiifiiiipppipppiiipiiip",
-    "nsa_attn_bwd_walks": "iiiiiiii",
+    "nsa_attn_bwd_walks": "iiiiiiiii",
     "nsa_attn_fwd": "ipppppiiiiiifiiiipppip",
     "nsa_attn_importance": "ippppiiiiiifiiip",
     "nsa_comm_allgather": "ippliipuqip",
