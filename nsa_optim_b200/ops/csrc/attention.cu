@@ -3418,7 +3418,8 @@ void fill_params(AttnParams& p, int B, int T, int S, int Hq, int Hkv, int D, flo
   p = AttnParams{};
   p.B = B; p.T = T; p.S = S; p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.R = BM / p.G; p.D = D;
   p.scale_log2 = scale * 1.4426950408889634f;
-  p.causal = causal; p.window = window; p.kp_stride = kp_stride; p.kp_off = kp_off;
+  p.causal = causal; p.kp_stride = kp_stride; p.kp_off = kp_off;
+  p.window = std::min(window, T);      // T tokens reach over the whole sequence: positions plus a window stay in 32 bits
   p.tile_blocks = tb; p.tile_masks = tmk; p.tile_counts = tc; p.max_u = max_u;
   p.status = nsa::status_ptr();
 }
@@ -3560,7 +3561,7 @@ extern "C" int nsa_attn_bwd(const void* q, const void* k, const void* v, const v
 // it a key is seen by every token up to a window after it.
 static int key_visits(int T, int R, int causal, int window, int kp_stride) {
   const int n_qt = (T + R - 1) / R;
-  return causal && window > 0 ? std::min(n_qt, (127 * kp_stride + window - 1) / R + 2) : n_qt;
+  return causal && window > 0 ? std::min(n_qt, (127 * kp_stride + std::min(window, T) - 1) / R + 2) : n_qt;
 }
 // Walks per 128-key block for nsa_attn_bwd_split over contiguous ranges, whose sums it wants room for (`part`, floats: walks x 2 x
 // B S Hkv D) if they are more than one; 0: walks of `visits_per_cta` tiles that add to dK and dV in any order.

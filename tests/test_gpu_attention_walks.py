@@ -48,3 +48,10 @@ def test_key_gradients(native, B, T, Hq, Hkv, window):
                                       (1100, 32, 1)])
 def test_key_gradients_without_causality(native, T, Hq, Hkv, window):
     _check(native, 1, T, Hq, Hkv, window, False)
+
+
+# "No limit" written as a number: positions plus the window pass 2^31.  Several walks a block, and more than 256 tiles
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("T,Hq,Hkv,window", [(300, 16, 1, 2 ** 31 - 1), (300, 2, 2, 2 ** 31 - 129), (1100, 32, 1, 2 ** 31 - 1), (300, 16, 1, 300)])
+def test_key_gradients_of_the_widest_windows(native, T, Hq, Hkv, window, causal):
+    _check(native, 1, T, Hq, Hkv, window, causal)
