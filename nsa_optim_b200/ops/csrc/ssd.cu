@@ -293,6 +293,12 @@ __device__ __forceinline__ float4 load_dt4(const SsdParams& p, const Items& at) 
   return make_float4(t < p.T ? src[0] : 0.f, t + 1 < p.T ? src[p.H] : 0.f, t + 2 < p.T ? src[2 * p.H] : 0.f,
                      t + 3 < p.T ? src[3 * p.H] : 0.f);
 }
+// The sum that the lane before ends with.  (Taking this lane's own part off its sum instead would give rows in front of a long or
+// non-finite step that step's rounding error, or a NaN.)
+__device__ __forceinline__ float sum_before(float run) {
+  const float v = __shfl_up_sync(0xffffffffu, run, 1);
+  return (threadIdx.x & 31) == 0 ? 0.f : v;
+}
 // One warp: cum[] = inclusive sums of dt A in units of log 2, dts[] = dt, for 128 rows.  Pairs of rows in different blocks of
 // 32 need no exponential of their own: with m the sum at the end of an earlier block, exp(c_i - c_j) = exp(c_i - m)
 // exp(m - c_j), and both exponents are <= 0.  colf[] receives the factors that belong to columns:
@@ -312,7 +318,7 @@ __device__ __forceinline__ void chunk_scan_warp(float4 dt, float a, float* cum, 
     const float n = __shfl_up_sync(0xffffffffu, run, o);
     if (lane >= o) run += n;
   }
-  const float off = run - v.w;
+  const float off = sum_before(run);
   v = make_float4((off + v.x) * LOG2E, (off + v.y) * LOG2E, (off + v.z) * LOG2E, run * LOG2E);
   *reinterpret_cast<float4*>(cum + 4 * lane) = v;
   *reinterpret_cast<float4*>(dts + 4 * lane) = dt;
@@ -1154,7 +1160,7 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
         const float n = __shfl_up_sync(0xffffffffu, run, o);
         if (lane >= o) run += n;
       }
-      const float off = run - c.w, tot = __shfl_sync(0xffffffffu, run, 31);
+      const float off = sum_before(run), tot = __shfl_sync(0xffffffffu, run, 31);
       auto weight = [&](float cum, float d) { return BACK ? exp2f(cum * LOG2E) : exp2f((tot - cum) * LOG2E) * d; };
       float* sc = scale + s * (L + 4);
       *reinterpret_cast<float4*>(sc + 4 * lane) =

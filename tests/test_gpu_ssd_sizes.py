@@ -45,6 +45,27 @@ def test_ssd_walk_and_runs(native, B, T, H, skip):
     test_ssd_sizes(native, B, T, H, skip)
 
 
+# A step that forgets everything, or is not finite, at each place of the four that a lane scans, in the second chunk: what comes
+# before it does not see it.  One head (a kernel per chunk) and many (one walk over the chunks).
+@pytest.mark.parametrize("at", [168, 169, 171])
+@pytest.mark.parametrize("T,H", [(300, 40), (1500, 1)])
+def test_steps_before_a_long_one(native, T, H, at):
+    torch.manual_seed(at)
+    x, Bm, Cm, dy = (torch.randn(1, T, h, n, device="cuda").bfloat16() for h, n in ((H, 64), (1, 128), (1, 128), (H, 64)))
+    dt, A = torch.rand(1, T, H, device="cuda") * 0.1 + 0.01, -torch.ones(H, device="cuda")
+    plain = native.ssd_scan(x, dt, A, Bm, Cm)
+    for bad in (float("inf"), float("nan"), 1e6):
+        dt[:, at] = bad
+        assert torch.equal(native.ssd_scan(x, dt, A, Bm, Cm)[:, :at], plain[:, :at]), bad
+    leaves = [t.detach().requires_grad_() for t in (x, dt, A, Bm, Cm)]
+    got = torch.autograd.grad(native.ssd_scan(*leaves), leaves, dy)
+    ref = [t.detach().double().requires_grad_() for t in leaves]
+    want = torch.autograd.grad(_reference(*ref, None), ref, dy.double())
+    for name, i in (("dx", 0), ("dB", 3), ("dC", 4)):
+        a, b = got[i][:, :at].double(), want[i][:, :at]
+        assert (a - b).norm() < 1e-2 * b.norm(), name                                # as above
+
+
 @pytest.mark.parametrize("nc,E", [(1, 7), (7, 12), (8, 64), (9, 1000), (30, 8192)])
 @pytest.mark.parametrize("back", [False, True])
 def test_state_pass(native, nc, E, back):
