@@ -95,29 +95,6 @@ __device__ __forceinline__ void tld64(uint32_t taddr, float (&out)[64]) {
   for (int j = 0; j < 32; ++j) { out[j] = __uint_as_float(a[j]); out[32 + j] = __uint_as_float(b[j]); }
 }
 
-// Inclusive scan of `a` over the 128 rows of the chunk, by every group of 128 threads of the CTA (with the same
-// result); cum[] and dts[] (shared, 128 floats each) receive every row's value.  Returns this row's inclusive sum.
-__device__ __forceinline__ float chunk_scan(float a, float dt, float* cum, float* dts, float* warp_tot) {
-  const int r = threadIdx.x & 127, lane = r & 31, w = r >> 5;
-  float v = a;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float n = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += n;
-  }
-  if (lane == 31 && threadIdx.x < 128) warp_tot[w] = v;
-  __syncthreads();
-  float off = 0.f;
-  for (int k = 0; k < w; ++k) off += warp_tot[k];
-  v += off;
-  if (threadIdx.x < 128) {
-    cum[r] = v;
-    dts[r] = dt;
-  }
-  __syncthreads();
-  return v;
-}
-
 // Two fp32 lanes per instruction; each lane rounds as the scalar instruction does.
 __device__ __forceinline__ float2 mul2(const float2& a, const float2& b) {
   float2 d;
@@ -163,6 +140,35 @@ struct SsdParams {
   KernelStatus* status;
 };
 
+// dt of four neighbouring rows per lane of a chunk that starts at t0 (one warp)
+__device__ __forceinline__ float4 load_dt4(const SsdParams& p, int b, int t0, int h) {
+  const int t = t0 + 4 * (threadIdx.x & 31);
+  const float* src = p.dt + (static_cast<long>(b) * p.T + t) * p.H + h;
+  return make_float4(t < p.T ? src[0] : 0.f, t + 1 < p.T ? src[p.H] : 0.f, t + 2 < p.T ? src[2 * p.H] : 0.f,
+                     t + 3 < p.T ? src[3 * p.H] : 0.f);
+}
+// One warp: inclusive sums of dt A over the chunk, in units of log 2.  Every kernel forms its decays from these, as differences of
+// sums: the gradients of dt and A are differences of terms that different kernels compute, and cancel as far as the decays agree.
+// (The sum before a lane comes from the lane before.  Taking this lane's own part off its sum instead would give rows in front of
+// a long or non-finite step that step's rounding error, or a NaN.)
+__device__ __forceinline__ float4 chunk_sums(float4 dt, float a) {
+  const int lane = threadIdx.x & 31;
+  float4 v = make_float4(dt.x * a, dt.y * a, dt.z * a, dt.w * a);
+  v.y += v.x;
+  v.z += v.y;
+  v.w += v.z;
+  float run = v.w;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float n = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run += n;
+  }
+  float off = __shfl_up_sync(0xffffffffu, run, 1);
+  if (lane == 0) off = 0.f;
+  // products of their own: fused with the subtractions that follow they would round differently from one kernel to the next
+  return make_float4(__fmul_rn(off + v.x, LOG2E), __fmul_rn(off + v.y, LOG2E), __fmul_rn(off + v.z, LOG2E), __fmul_rn(run, LOG2E));
+}
+
 // ---------------------------------------------------------------------------------------
 // chunk_state.  MODE 0: rows of Bm scaled by exp(tot - cum_j) dt_j, values = x.
 //               MODE 1: rows of Cm scaled by exp(cum_i),            values = dy.
@@ -183,7 +189,6 @@ ssd_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_c
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* cum = reinterpret_cast<float*>(bars + 4);
   float* dts = cum + L;
-  float* warp_tot = dts + L;
 
   const int r = threadIdx.x, warp = r >> 5;
   const int h = blockIdx.x, c = p.c0 + blockIdx.y, b = blockIdx.z;    // see each_slab
@@ -198,19 +203,20 @@ ssd_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_c
     tc5::tma_load_3d(sBC + BOXB, &tm_bc, full, 64, t0, b);
     tc5::tma_load_4d(sV, &tm_v, full, 0, h, t0, b);
   }
-  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 64); tc5::tmem_relinquish(); }
-  const int t = t0 + r;
-  const float dt = t < p.T ? p.dt[(static_cast<long>(b) * p.T + t) * p.H + h] : 0.f;
-  const float a = dt * p.A[h];
-  const float cm = chunk_scan(a, dt, cum, dts, warp_tot);
-  const float tot = cum[L - 1];
+  if (warp == 1) { tc5::tmem_alloc(tmem_slot, 64); tc5::tmem_relinquish(); }
+  if (warp == 0) {
+    const float4 dt = load_dt4(p, b, t0, h);
+    reinterpret_cast<float4*>(cum)[r] = chunk_sums(dt, p.A[h]);
+    reinterpret_cast<float4*>(dts)[r] = dt;
+  }
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  const float tot = cum[L - 1];
   bool ok = tc5::mbar_wait(full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL);
   if (ok) {
-    const float sc = MODE == 0 ? exp2f((tot - cm) * LOG2E) * dt : exp2f(cm * LOG2E);
+    const float sc = MODE == 0 ? exp2f(tot - cum[r]) * dts[r] : exp2f(cum[r]);
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       float v[64];
@@ -256,11 +262,11 @@ ssd_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_c
       const int i = j * 128 + r;
       dst[i] = stage[(i & ~15) + ((i ^ (i >> 4)) & 15)];
     }
-    if (MODE == 0 && r == 0 && p.gamma_out) p.gamma_out[(static_cast<long>(b) * p.nc + c) * p.H + h] = exp2f(tot * LOG2E);
+    if (MODE == 0 && r == 0 && p.gamma_out) p.gamma_out[(static_cast<long>(b) * p.nc + c) * p.H + h] = exp2f(tot);
   }
   tc5::fence_before_sync();
   __syncthreads();
-  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 64); }
+  if (warp == 1) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 64); }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -286,19 +292,6 @@ struct Items {
   __device__ bool closes(int k) const { return k + 1 == n || h + 1 == H; }     // last one
 };
 
-// dt of four neighbouring rows of the item's chunk, for chunk_scan_warp
-__device__ __forceinline__ float4 load_dt4(const SsdParams& p, const Items& at) {
-  const int t = at.t0 + 4 * (threadIdx.x & 31);
-  const float* src = p.dt + (static_cast<long>(at.b) * p.T + t) * p.H + at.h;
-  return make_float4(t < p.T ? src[0] : 0.f, t + 1 < p.T ? src[p.H] : 0.f, t + 2 < p.T ? src[2 * p.H] : 0.f,
-                     t + 3 < p.T ? src[3 * p.H] : 0.f);
-}
-// The sum that the lane before ends with.  (Taking this lane's own part off its sum instead would give rows in front of a long or
-// non-finite step that step's rounding error, or a NaN.)
-__device__ __forceinline__ float sum_before(float run) {
-  const float v = __shfl_up_sync(0xffffffffu, run, 1);
-  return (threadIdx.x & 31) == 0 ? 0.f : v;
-}
 // One warp: cum[] = inclusive sums of dt A in units of log 2, dts[] = dt, for 128 rows.  Pairs of rows in different blocks of
 // 32 need no exponential of their own: with m the sum at the end of an earlier block, exp(c_i - c_j) = exp(c_i - m)
 // exp(m - c_j), and both exponents are <= 0.  colf[] receives the factors that belong to columns:
@@ -308,18 +301,7 @@ __device__ __forceinline__ int later_block(int q) { return 16 * q * (7 - q) - 32
 template <bool FWD>
 __device__ __forceinline__ void chunk_scan_warp(float4 dt, float a, float* cum, float* dts, float* colf) {
   const int lane = threadIdx.x & 31, blk = lane >> 3;
-  float4 v = make_float4(dt.x * a, dt.y * a, dt.z * a, dt.w * a);
-  v.y += v.x;
-  v.z += v.y;
-  v.w += v.z;
-  float run = v.w;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float n = __shfl_up_sync(0xffffffffu, run, o);
-    if (lane >= o) run += n;
-  }
-  const float off = sum_before(run);
-  v = make_float4((off + v.x) * LOG2E, (off + v.y) * LOG2E, (off + v.z) * LOG2E, run * LOG2E);
+  const float4 v = chunk_sums(dt, a);
   *reinterpret_cast<float4*>(cum + 4 * lane) = v;
   *reinterpret_cast<float4*>(dts + 4 * lane) = dt;
   auto ex = [](float x) { return exp2f(fminf(x, 0.f)); };
@@ -490,13 +472,13 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   } else if (warp == 18) {                             // sums of step sizes, two items ahead
     Items cur(p);
     const int n = cur.n;
-    float4 dt = load_dt4(p, cur);
+    float4 dt = load_dt4(p, cur.b, cur.t0, cur.h);
     float a = p.A[cur.h];
     for (int k = 0; k < n; ++k) {
       float4 dt_next = make_float4(0.f, 0.f, 0.f, 0.f);
       float a_next = 0.f;
       cur.next();
-      if (k + 1 < n) { dt_next = load_dt4(p, cur); a_next = p.A[cur.h]; }
+      if (k + 1 < n) { dt_next = load_dt4(p, cur.b, cur.t0, cur.h); a_next = p.A[cur.h]; }
       if (k > 1 && !wait(ready + (k & 1), (k >> 1) - 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;       // those of item k - 2 have been read
       float* at = scan + (k & 1) * (2 * L + 192);
       chunk_scan_warp<true>(dt, a, at, at + L, at + 2 * L);
@@ -724,7 +706,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
       __syncwarp();
     };
     if (lead) load(0);
-    chunk_scan_warp<false>(load_dt4(p, ahead), p.A[ahead.h], cum, dts, colf);
+    chunk_scan_warp<false>(load_dt4(p, ahead.b, ahead.t0, ahead.h), p.A[ahead.h], cum, dts, colf);
     arrive_warp(scanned);
     ahead.next();
     // A step issues the rest of item k and the first products of item k + 1 between them, so that the scores of k + 1 are
@@ -758,7 +740,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
       }
       float4 dt_next = make_float4(0.f, 0.f, 0.f, 0.f);
       float a_next = 0.f;
-      if (more) { dt_next = load_dt4(p, ahead); a_next = p.A[ahead.h]; }
+      if (more) { dt_next = load_dt4(p, ahead.b, ahead.t0, ahead.h); a_next = p.A[ahead.h]; }
       ahead.next();
       if (!(ok = wait(ready, k, STATUS_TIMEOUT_TMEM_EMPTY))) break;
       tc5::fence_after_sync();
@@ -1118,12 +1100,7 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
   } else if (warp == 17) {
     const bool lead = tc5::elect_one();
     const float a = p.A[h];
-    auto load_dt = [&](int i) {
-      const int t = chunk_of(i) * L + 4 * lane;
-      const float* src = p.dt + (static_cast<long>(b) * p.T + t) * p.H + h;
-      return make_float4(t < p.T ? src[0] : 0.f, t + 1 < p.T ? src[p.H] : 0.f, t + 2 < p.T ? src[2 * p.H] : 0.f,
-                         t + 3 < p.T ? src[3 * p.H] : 0.f);
-    };
+    auto load_dt = [&](int i) { return load_dt4(p, b, chunk_of(i) * L, h); };
     // into L2 a few chunks ahead: the stages alone leave a load from memory less time than it takes
     constexpr int AHEAD = 8;
     auto prefetch = [&](int i) {
@@ -1150,22 +1127,12 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
       }
       prefetch(i + AHEAD);
       __syncwarp();
-      float4 c = make_float4(dt.x * a, dt.y * a, dt.z * a, dt.w * a);
-      c.y += c.x;
-      c.z += c.y;
-      c.w += c.z;
-      float run = c.w;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float n = __shfl_up_sync(0xffffffffu, run, o);
-        if (lane >= o) run += n;
-      }
-      const float off = sum_before(run), tot = __shfl_sync(0xffffffffu, run, 31);
-      auto weight = [&](float cum, float d) { return BACK ? exp2f(cum * LOG2E) : exp2f((tot - cum) * LOG2E) * d; };
+      const float4 c = chunk_sums(dt, a);
+      const float tot = __shfl_sync(0xffffffffu, c.w, 31);
+      auto weight = [&](float cum, float d) { return BACK ? exp2f(cum) : exp2f(tot - cum) * d; };
       float* sc = scale + s * (L + 4);
-      *reinterpret_cast<float4*>(sc + 4 * lane) =
-          make_float4(weight(off + c.x, dt.x), weight(off + c.y, dt.y), weight(off + c.z, dt.z), weight(run, dt.w));
-      if (lane == 0) sc[L] = exp2f(tot * LOG2E);
+      *reinterpret_cast<float4*>(sc + 4 * lane) = make_float4(weight(c.x, dt.x), weight(c.y, dt.y), weight(c.z, dt.z), weight(c.w, dt.w));
+      if (lane == 0) sc[L] = exp2f(tot);
       arrive_warp(full + s);
       dt = dt_next;
     }

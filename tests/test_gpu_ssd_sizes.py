@@ -66,6 +66,24 @@ def test_steps_before_a_long_one(native, T, H, at):
         assert (a - b).norm() < 1e-2 * b.norm(), name                                # as above
 
 
+# dA holds the sums over the tokens from each one on of dy.y - x.dx, times its step.  Terms of different kernels cancel in them: up to the
+# rounding of the bf16 operands, averaged over a row's products, where the kernels agree on the decays.  With a step of 1e6 the sums
+# of steps are multiples of 1/16 and decays rounded in different ways are up to 6 % apart.  One walk over the chunks, and two kernels.
+@pytest.mark.parametrize("T,H,at", [(700, 64, 168), (700, 64, 171), (2000, 64, 300), (1500, 2, 171)])
+def test_decays_agree_behind_a_long_step(native, T, H, at):
+    torch.manual_seed(at)
+    x, Bm, Cm, dy = (torch.randn(1, T, h, n, device="cuda").bfloat16() for h, n in ((H, 64), (1, 128), (1, 128), (H, 64)))
+    dt, A = torch.rand(1, T, H, device="cuda") * 0.1 + 0.01, -torch.ones(H, device="cuda")
+    dt[:, at] = 1e6
+    leaves = [t.detach().requires_grad_() for t in (x, dt, A, Bm, Cm)]
+    dA = torch.autograd.grad(native.ssd_scan(*leaves), leaves, dy)[2]
+    ref = [t.detach().double().requires_grad_() for t in leaves]
+    y = _reference(*ref, None)
+    want = torch.autograd.grad(y, ref, dy.double())[2]
+    terms = (y.detach() * dy.double()).sum(-1)[0, at:]                              # (tokens, H): what cancels
+    assert ((dA - want).abs() <= 1e6 * 2 ** -9 * 128 ** -0.5 * terms.norm(dim=0)).all()
+
+
 @pytest.mark.parametrize("nc,E", [(1, 7), (7, 12), (8, 64), (9, 1000), (30, 8192)])
 @pytest.mark.parametrize("back", [False, True])
 def test_state_pass(native, nc, E, back):
