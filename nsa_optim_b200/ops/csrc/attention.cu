@@ -824,7 +824,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // all visits of its tile.  An SM works on two tiles then, and the start and the end of one (4 K cycles to the first
 // scores, 4 K from the last to the exit) run beside the visits of the other; nothing is merged.  Half of the shared memory and of the tensor memory
 // is left to a CTA: two stages of K and of V, S and P and O in 256 columns, Q in shared memory.
-// 8192 tokens x 32 query and 2 KV heads: 591 -> 510 us, without causality 1089 -> 1068, window 512 158 -> 113; 16384 2235 -> 2091.
+// 8192 tokens x 32 query and 2 KV heads: 599 -> 517 us, without causality 1110 -> 1072, window 512 163 -> 121; 16384 2200 -> 1960.
 // (Visits of 128 keys in one CTA, P over S: 16384 2386 us, window 512 174; S then waits for P V of the visit before.)
 // --------------------------------------------------------------------------------------
 constexpr int FW1_STAGES = 2;
@@ -992,6 +992,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const long rowi = (static_cast<long>(b) * p.T + (row_ok ? t : 0)) * p.Hq + h * p.G + gh;
     const float sc = p.scale_log2;
     float m_ref = -INFINITY, l_sum = 0.f;
+    int refs = 0;                                // references taken so far
     bool ok = true;
     int blk_n = 0;
     unsigned long long msk_n = 0ull;
@@ -1034,10 +1035,13 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
       }
       mx *= sc;
+      // The largest probability of the visit that sets the reference is 1, which bf16 holds exactly.  A row's first two visits
+      // both set it, as those of the two groups of the other form do: with one, the output is 1 to 1.5 % further from 64 bits.
       float alpha = 1.f;
-      if (mx != -INFINITY && (m_ref == -INFINITY || mx > m_ref + 8.f)) {
+      if (mx != -INFINITY && (m_ref == -INFINITY || mx > m_ref + 8.f || (refs == 1 && mx > m_ref - 8.f))) {
         alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - mx);
         m_ref = mx;
+        ++refs;
       }
       uint32_t pk[32];
       float psum = 0.f;
@@ -3426,16 +3430,17 @@ void fill_params(AttnParams& p, int B, int T, int S, int Hq, int Hkv, int D, flo
 }  // namespace
 
 // Two CTAs per SM with one softmax group each, or one with two?  A lone CTA takes its visits in one chain where the other form has two,
-// so there must be two CTAs and more for each SM, and of long tiles so many that the last ones weigh little.  Up to 20 visits
-// (two groups, one group): 152 CTAs x 19 visits 17 us, 22; 200 x 13 16.0, 17.5; 300 x 9 23.7, 18.7; 300 x 19 27, 27; 4096 x 9 311, 222.
-// More: 300 x 75 60, 72; 400 x 50 69.8, 69.7; 600 x 38 70, 55; 1200 x 75 220, 184; groups of one or two heads, whose neighbouring tiles
-// share no keys, are slower up to 1024 CTAs (600 x 75 129, 132; 1024 x 128 304, 309; 1536 x 192 695, 686).
+// so there must be two CTAs and more for each SM, and of long tiles so many that the last ones weigh little.  Up to 16 visits
+// (two groups, one group): 200 CTAs x 13 visits 16.0 us, 17.5; 300 x 9 23.7, 19.2; 400 x 9 31.2, 29.7; 1200 x 9 97, 73.
+// More: 300 x 19 26.8, 27.9; 300 x 75 60, 72; 400 x 50 70, 70; 600 x 38 70, 56; 1200 x 75 221, 187; groups of one or two heads, whose
+// neighbouring tiles share no keys, are slower up to 1024 CTAs (600 x 75 129, 132; 1024 x 128 304, 309; 1536 x 192 686, 681).
+// A selected block counts as the keys of a sequence do: how many blocks the tokens of a tile share is not known here.
 // Compressed keys always take two groups: their L goes into the choice of blocks, where a last bit decides between near ties (with one
 // group, compressed and selected branch together 1159 us at 16384 tokens, 1298 with two, a few rows took another block than before).
 static bool fwd_two_per_sm(const AttnParams& p, long ctas) {
   if (p.kp_stride > 1) return false;
   const int visits = (std::min(p.S, p.window > 0 ? p.window + p.R : p.S) + 63) / 64;
-  return ctas >= nsa::sm_count() * (visits <= 20 ? 2l : p.G >= 4 ? 4l : 8l);
+  return ctas >= nsa::sm_count() * (visits <= 16 ? 2l : p.G >= 4 ? 4l : 8l);
 }
 
 extern "C" int nsa_attn_fwd(const void* q, const void* k, const void* v, void* o, float* L, int B, int T, int S,

@@ -22,10 +22,12 @@ def _check(native, q, k, v, seen, got):
 
 
 @pytest.mark.parametrize("B,T,Hq,Hkv,causal,window", [
-    (1, 1184, 32, 2, True, 0), (1, 1176, 32, 2, True, 0),      # 296 and 294 tiles of up to 19 visits
+    (2, 592, 32, 2, True, 0), (2, 584, 32, 2, True, 0),        # 296 and 292 tiles of up to 10 visits
+    (1, 1184, 32, 2, True, 0), (1, 1176, 32, 2, True, 0),      # 296 and 294 tiles of up to 19 visits: one CTA per SM
     (4, 1191, 16, 2, False, 0), (2, 1500, 32, 2, True, 100), (40, 33, 16, 8, True, 0), (300, 1, 2, 1, True, 0), (19, 130, 16, 16, False, 64),
-    (1, 1200, 32, 1, True, 0),                                 # groups of 32: 300 tiles of 4 tokens
-    (2, 1340, 32, 2, True, 700), (1, 2400, 32, 2, False, 0),   # more than 20 visits
+    (1, 1200, 32, 1, True, 0), (2, 600, 32, 1, True, 0),       # groups of 32: 300 tiles of 4 tokens
+    (2, 1340, 32, 2, True, 700), (1, 2400, 32, 2, False, 0),   # 12 visits of a window; more than 16 without and with one
+    (1, 2400, 32, 2, True, 1300), (2, 1340, 32, 2, True, 1000),
     (8, 1400, 16, 8, True, 0)])
 def test_forward(native, B, T, Hq, Hkv, causal, window):
     g = torch.Generator("cuda").manual_seed(T)
@@ -37,14 +39,36 @@ def test_forward(native, B, T, Hq, Hkv, causal, window):
     _check(native, q, k, v, seen.expand(B, Hkv, T, T), native.attention(q, k, v, causal, window))
 
 
-@pytest.mark.parametrize("T,Hq,Hkv", [(1184, 32, 2), (2380, 32, 2)])
-def test_selected(native, T, Hq, Hkv):
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 1184, 32, 2), (2, 600, 32, 2), (1, 2380, 32, 2)])
+def test_selected(native, B, T, Hq, Hkv):
     g = torch.Generator("cuda").manual_seed(T)
-    q, k, v = (torch.randn(1, T, h, 128, device="cuda", generator=g).bfloat16() for h in (Hq, Hkv, Hkv))
+    q, k, v = (torch.randn(B, T, h, 128, device="cuda", generator=g).bfloat16() for h in (Hq, Hkv, Hkv))
     nS, t = -(-T // 64), torch.arange(T, device="cuda")
     own = (t // 64)[None, None, :, None]
-    pick = torch.randint(0, nS, (1, Hkv, T, 4), device="cuda", generator=g)
-    idx = torch.cat([own.expand(1, Hkv, T, 1), torch.where(pick <= own, pick, -1)], -1).to(torch.int32)
-    took = torch.zeros(1, Hkv, T, nS + 1, dtype=torch.bool, device="cuda").scatter_(-1, torch.where(idx < 0, nS, idx).long(), True)
+    pick = torch.randint(0, nS, (B, Hkv, T, 4), device="cuda", generator=g)
+    idx = torch.cat([own.expand(B, Hkv, T, 1), torch.where(pick <= own, pick, -1)], -1).to(torch.int32)
+    took = torch.zeros(B, Hkv, T, nS + 1, dtype=torch.bool, device="cuda").scatter_(-1, torch.where(idx < 0, nS, idx).long(), True)
     seen = took[..., :nS].repeat_interleave(64, -1)[..., :T] & (t[None, :] <= t[:, None])
     _check(native, q, k, v, seen, native.selected_attention(q, k, v, idx))
+
+
+@pytest.mark.parametrize("T,Hq,Hkv,window", [(3000, 16, 8, 64), (3000, 16, 2, 300), (2400, 16, 8, 0)])
+def test_as_close_to_64_bits_as_one_cta_per_sm(native, T, Hq, Hkv, window):
+    # The same rows with few tiles, a KV head at a time, take the other form.  Both round probabilities to bf16 and hold a largest one of
+    # two visits exactly; holding that of one alone is 6 % further off here with the short window and 1 % without.  Of 2^17 rows the
+    # errors differ by chance by less than 2^-8.5 of themselves.
+    g = torch.Generator("cuda").manual_seed(T + Hq)
+    q, k, v = (torch.randn(1, T, h, 128, device="cuda", generator=g).bfloat16() for h in (Hq, Hkv, Hkv))
+    t, G = torch.arange(T, device="cuda"), Hq // Hkv
+    seen = t[None, :] <= t[:, None]
+    if window:
+        seen = seen & (t[None, :] > t[:, None] - window)
+    many, few = native.attention(q, k, v, True, window), []
+    off = torch.zeros(2, dtype=torch.float64, device="cuda")
+    for h in range(Hkv):
+        qh, kh, vh = q[:, :, h * G:(h + 1) * G], k[:, :, h:h + 1], v[:, :, h:h + 1]
+        s = (qh.double().transpose(1, 2) @ kh.double().permute(0, 2, 3, 1) * 128 ** -0.5).masked_fill(~seen, -float("inf"))
+        want = (s.softmax(-1) @ vh.double().transpose(1, 2)).transpose(1, 2)
+        for i, got in enumerate((many[:, :, h * G:(h + 1) * G], native.attention(qh, kh, vh, True, window))):
+            off[i] += (got.double() - want).square().sum()
+    assert off[0].sqrt() <= (1 + 2 ** -8.5) * off[1].sqrt(), off.sqrt()
