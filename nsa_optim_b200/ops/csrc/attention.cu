@@ -2469,9 +2469,10 @@ struct KeyWalks {
   int walks;                 // walks per key block
   float* part;               // [walks][2][B, S, Hkv, D] sums of a walk, added up in order afterwards; null: added to dV and dK
 };
-// Query tiles of walk y of the 128 keys from s0 on: v0 and how many (none: <= 0)
+// Query tiles of walk y of the KEYS keys from s0 on: v0 and how many (none: <= 0)
+template <int KEYS>
 __device__ __forceinline__ int key_walk(const AttnParams& p, int visits, int s0, int y, int& v0) {
-  const int s_hi = min(s0 + 127, p.S - 1), n_qt = (p.T + p.R - 1) / p.R;
+  const int s_hi = min(s0 + KEYS - 1, p.S - 1), n_qt = (p.T + p.R - 1) / p.R;
   const int qt_lo = p.causal ? max(0, (s0 * p.kp_stride + p.kp_off) / p.R) : 0;
   if (p.window > 0) {                          // short ranges: chunks counted from the block's first tile
     v0 = qt_lo + y * visits;
@@ -2491,7 +2492,7 @@ __global__ void __launch_bounds__(256) attn_sum_walks_kernel(const AttnParams p,
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int y = 0; y < w.walks; ++y) {
     int v0;
-    if (key_walk(p, w.visits, s0, y, v0) <= 0) continue;
+    if (key_walk<128>(p, w.visits, s0, y, v0) <= 0) continue;
     const float4 v = part[2 * n * y];
     acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
   }
@@ -2534,7 +2535,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   const int b = blockIdx.z / p.Hkv, h = blockIdx.z - b * p.Hkv;
   const int s0 = blockIdx.x * KEYS;              // key block fastest: concurrent CTAs share a Q/dO range in L2
   int v0;
-  const int n_vis = key_walk(p, w.visits, s0, blockIdx.y, v0);
+  const int n_vis = key_walk<KEYS>(p, w.visits, s0, blockIdx.y, v0);
   if (n_vis <= 0) return;
   if (tc5::smem_u32(smem_kvc) & 1023u) {         // the swizzle needs it; never seen otherwise
     if (tid == 0) status_report(p.status, STATUS_BAD_ARGUMENT, blockIdx.x, static_cast<int>(tc5::smem_u32(smem_kvc)));
@@ -2811,10 +2812,11 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 }
 
 // --------------------------------------------------------------------------------------
-// Backward for dK / dV of selected blocks, key-block stationary.  A CTA owns one 64-key block of one KV head and
-// walks over "visits" of 128 rows (R tokens x G heads) that come from the inverse selection map: for every (batch, KV head,
-// block) the ascending list of tokens that selected it, R tokens per visit, each token's G query rows fetched
-// by its own TMA box.
+// Backward for dK / dV, key-block stationary, 64 keys a CTA.  It walks over "visits" of 128 rows (R tokens x G heads):
+//   SELECTED: from the inverse selection map, for every (batch, KV head, block) the ascending list of tokens that selected it,
+//     R tokens per visit, each token's G query rows fetched by its own TMA box;
+//   else: the query tiles of an analytic range, all of them in one CTA, for ranges too short for the kernel above
+//     (see nsa_attn_bwd_walks).
 // dV^T (D x 64) += dO^T P and dK^T (D x 64) += Q^T dS stay in TMEM for the whole walk, so global
 // memory sees one fp32 reduction per CTA instead of one per (query tile, key tile) pair.
 // Roles: warps 0-7 softmax (thread (r, ch) = row r, 32 key columns), warp 8 TMA producer,
@@ -2831,9 +2833,11 @@ struct KvWalk {
 };
 
 constexpr int KV_THREADS = 384;
+constexpr int KV_SMEM = 24 * HALF + 1024 + 256;
 
+template <bool SELECTED>
 __global__ void __launch_bounds__(KV_THREADS, 1)
-attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_constant__ CUtensorMap tm_do1,
+attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const AttnParams p, const KvWalk w, const float scale) {
   constexpr int D = 128;
@@ -2860,17 +2864,25 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_const
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // ---- which block, which visits (uniform over the CTA; CTAs without work leave before any setup)
-  const int item = blockIdx.x;
-  if (item >= w.item_start[w.n_lists]) return;
-  int lst = 0;                                   // largest list with item_start[list] <= item
-  for (int hi = w.n_lists; hi - lst > 1;) {
-    const int mid = (lst + hi) >> 1;
-    if (w.item_start[mid] <= item) lst = mid; else hi = mid;
+  int b, h, s0, v0, n_vis, lst0 = 0, cnt = 0;
+  if (SELECTED) {
+    const int item = blockIdx.x;
+    if (item >= w.item_start[w.n_lists]) return;
+    int lst = 0;                                 // largest list with item_start[list] <= item
+    for (int hi = w.n_lists; hi - lst > 1;) {
+      const int mid = (lst + hi) >> 1;
+      if (w.item_start[mid] <= item) lst = mid; else hi = mid;
+    }
+    const int bh = lst / w.nS;
+    b = bh / p.Hkv; h = bh - b * p.Hkv; s0 = (lst - bh * w.nS) * 64;
+    lst0 = w.list_start[lst];
+    cnt = w.list_start[lst + 1] - lst0;
+    v0 = (item - w.item_start[lst]) * w.visits_per_cta;
+    n_vis = min(w.visits_per_cta, (cnt + p.R - 1) / p.R - v0);
+  } else {
+    b = blockIdx.y / p.Hkv; h = blockIdx.y - b * p.Hkv; s0 = blockIdx.x * 64;
+    n_vis = key_walk<64>(p, p.T, s0, 0, v0);
   }
-  const int bh = lst / w.nS, b = bh / p.Hkv, h = bh - b * p.Hkv, s0 = (lst - bh * w.nS) * 64;
-  const int lst0 = w.list_start[lst], cnt = w.list_start[lst + 1] - lst0;
-  const int v0 = (item - w.item_start[lst]) * w.visits_per_cta;
-  const int n_vis = min(w.visits_per_cta, (cnt + p.R - 1) / p.R - v0);
   if (n_vis <= 0) return;
 
   if (tid == 0) {
@@ -2916,14 +2928,22 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_const
       if (!ok) break;
       uint8_t* dq_ = sQ + buf * QT;
       uint8_t* dd_ = sDO + buf * QT;
-      for (int j = lane; j < p.R; j += 32) {
-        const int li = (v0 + v) * p.R + j;
-        const int tok = li < cnt ? __ldg(w.tok_list + lst0 + li) : 0;   // rows past the list read token 0 and are masked
-        const int off = j * p.G * 128;
+      if (SELECTED) {
+        for (int j = lane; j < p.R; j += 32) {
+          const int li = (v0 + v) * p.R + j;
+          const int tok = li < cnt ? __ldg(w.tok_list + lst0 + li) : 0;   // rows past the list read token 0 and are masked
+          const int off = j * p.G * 128;
+#pragma unroll
+          for (int kb = 0; kb < 2; ++kb) {
+            tc5::tma_load_5d(dq_ + kb * 2 * HALF + off, &tm_q, q_full + buf, kb * 64, 0, h, tok, b);
+            tc5::tma_load_5d(dd_ + kb * 2 * HALF + off, &tm_do, q_full + buf, kb * 64, 0, h, tok, b);
+          }
+        }
+      } else if (lane == 0) {
 #pragma unroll
         for (int kb = 0; kb < 2; ++kb) {
-          tc5::tma_load_5d(dq_ + kb * 2 * HALF + off, &tm_q1, q_full + buf, kb * 64, 0, h, tok, b);
-          tc5::tma_load_5d(dd_ + kb * 2 * HALF + off, &tm_do1, q_full + buf, kb * 64, 0, h, tok, b);
+          tc5::tma_load_5d(dq_ + kb * 2 * HALF, &tm_q, q_full + buf, kb * 64, 0, h, (v0 + v) * p.R, b);
+          tc5::tma_load_5d(dd_ + kb * 2 * HALF, &tm_do, q_full + buf, kb * 64, 0, h, (v0 + v) * p.R, b);
         }
       }
       __syncwarp();
@@ -3016,11 +3036,12 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_const
     const float sc = p.scale_log2;
     const int sb = s0 + ch * 32;                   // this thread's first key
     bool ok = true;
-    // The row's token (from the inverse list) and its L / delta are fetched one and
+    // The row's token (selected blocks: from the inverse list) and its L / delta are fetched one and
     // two visits ahead, so the two dependent global loads are off the per-visit critical path.
     auto token_of = [&](int v) -> int {
       if (v >= n_vis) return -1;
       const int li = (v0 + v) * p.R + tok_local;
+      if (!SELECTED) return li < p.T ? li : -1;
       return li < cnt ? w.tok_list[lst0 + li] : -1;
     };
     int t_cur = token_of(0), t_nxt = token_of(1);
@@ -3562,25 +3583,74 @@ extern "C" int nsa_attn_bwd(const void* q, const void* k, const void* v, const v
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_attn_bwd launch");
 }
 
-// Query tiles that one 128-key block can be visited by, at most.  A window limits them only where causality does too: without
-// it a key is seen by every token up to a window after it.
-static int key_visits(int T, int R, int causal, int window, int kp_stride) {
-  const int n_qt = (T + R - 1) / R;
-  return causal && window > 0 ? std::min(n_qt, (127 * kp_stride + std::min(window, T) - 1) / R + 2) : n_qt;
-}
-// Walks per 128-key block for nsa_attn_bwd_split over contiguous ranges, whose sums it wants room for (`part`, floats: walks x 2 x
-// B S Hkv D) if they are more than one; 0: walks of `visits_per_cta` tiles that add to dK and dV in any order.
-// A visit takes 1.7 us and a walk 2 us more, so short sequences, whose blocks alone leave SMs idle, are cut into walks of six
-// visits and more, three for each SM (half of a causal grid is empty; with two, 110 us where three take 96).  2048 tokens, two groups of 16 heads: one walk a block 423 us, 128
-// visits 220, 32 visits 74.  Blocks of more than 256 visits fill the GPU with walks of 64 (128 within 2 %), and room for all
-// their sums would cost more than it gives.
+// Query tiles [lo, hi) that see the `keys` keys of block i of a contiguous range, and the most that any block has.  A window limits
+// them only where causality does too: without it a key is seen by every token up to a window after it.
+struct KeyRange {
+  int S, R, causal, window, kp_stride, keys, n_qt, blocks, most;
+  KeyRange(int T, int S, int R, int causal, int window, int kp_stride, int keys)
+      : S(S), R(R), causal(causal), window(std::min(window, T)), kp_stride(kp_stride), keys(keys), n_qt((T + R - 1) / R),
+        blocks((S + keys - 1) / keys), most(n_qt) {
+    if (causal && window > 0) most = std::min(n_qt, ((keys - 1) * kp_stride + this->window - 1) / R + 2);
+  }
+  int lo(int i) const { return causal ? std::min<long>(n_qt, static_cast<long>(i) * keys * kp_stride / R) : 0; }
+  int hi(int i) const {
+    if (window <= 0) return n_qt;
+    return static_cast<int>(std::min<long>(n_qt, ((std::min(i * static_cast<long>(keys) + keys, static_cast<long>(S)) - 1) * kp_stride + window - 1) / R + 1));
+  }
+};
+// Time of one form of the dK / dV kernel, as measured: a CTA's start and end and its longest walk; whole waves of mean walks; the chip's
+// throughput, with the longest walk behind it where there is more than a wave.
+struct KeyCost {
+  double start, visit, busy_start, busy_visit, tail, wave;
+  double us(long ctas, long visits, int longest) const {
+    const long sms = nsa::sm_count(), waves = (ctas + sms - 1) / sms;
+    return std::max({start + visit * longest, waves * (wave + 1.81 * visits / ctas),
+                     (busy_start * ctas + busy_visit * visits) / sms + (waves > 1 ? tail * longest : 0.)});
+  }
+};
+// How nsa_attn_bwd_split takes a contiguous range.  -1: 64 keys a CTA and one walk.  1 and more: 128 keys and as many walks, whose sums
+// go to `part` (walks x 2 x B S Hkv D floats) if they are several.  0: blocks of more than 256 visits, in walks of `visits_per_cta`
+// tiles that add to dK and dV in any order (they fill the GPU, and room for all their sums would cost more than it gives).
+// 64 keys have less to set up and a visit of 1.4 us instead of 1.8, and are the better form where there are few visits and SMs enough;
+// walks keep all SMs busy where blocks are few.  The constants are fitted to 209 shapes of 64 to 8192 tokens, 1 to 16 KV heads,
+// groups of 1 to 32 and windows, each in both forms and with up to 64 walks; the choice is 0.3 % behind the best in the mean and 16 % at
+// worst.  us with 64 keys, and with 128 and 1 / 2 / 4 / 8 / 16 walks (queries / KV heads, windows w): 300 16/8 12.9, 17.1 16.7 15.1;
+// 1000 32/8 w64 13.2, 20.4 22.9 29.7; 1000 32/2 181, 210 116 69 45 33; 2000 32/8 w512 66, 47 66 72 96; 3000 16/16 141, 114 145 165 215 282.
 extern "C" int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride) {
-  if (Hkv <= 0 || Hq < Hkv) return 0;
-  const int most = key_visits(T, std::max(1, BM / (Hq / Hkv)), causal, window, kp_stride);
-  if (most > 256) return 0;
-  const long blocks = static_cast<long>((S + 127) / 128) * B * Hkv;
-  const long want = (3l * nsa::sm_count() + blocks - 1) / std::max(1l, blocks);
-  return static_cast<int>(std::max(1l, std::min<long>(want, most / 6)));
+  if (B <= 0 || T <= 0 || S <= 0 || Hkv <= 0 || Hq < Hkv) return 0;
+  const int R = std::max(1, BM / (Hq / Hkv));
+  const long heads = static_cast<long>(B) * Hkv, sms = nsa::sm_count();
+  const KeyRange wide(T, S, R, causal, window, kp_stride, 128), narrow(T, S, R, causal, window, kp_stride, 64);
+  if (wide.most > 256) return 0;
+  constexpr KeyCost by_128{8.3, 1.79, 10.1, 1.6, 1.26, 8.2}, by_64{6.2, 1.43, 7.2, 1.06, 1.16, 5.1};
+  long total = 0;
+  int longest = 0;
+  for (int i = 0; i < narrow.blocks; ++i) {
+    const int n = std::max(0, narrow.hi(i) - narrow.lo(i));
+    total += n;
+    longest = std::max(longest, n);
+  }
+  int best = -1;
+  double least = by_64.us(heads * narrow.blocks, heads * total, longest);
+  for (int visits = wide.most; visits > 0; --visits) {
+    const int walks = (wide.most + visits - 1) / visits;
+    if (walks > 1 && (walks - 1) * wide.blocks * heads > 3 * sms) break;     // bounds the room for sums: 128 KB for each walk of a block
+    if (walks > 1 && (wide.most + walks - 1) / walks != visits) continue;    // as many walks as a longer visit count has
+    long ctas = 0;                                                           // with something to do
+    total = 0;
+    longest = 0;
+    for (int i = 0; i < wide.blocks; ++i) {
+      const int lo = wide.lo(i), n = std::max(0, wide.hi(i) - lo);
+      if (n == 0) continue;
+      ctas += window > 0 ? (n + visits - 1) / visits : (wide.n_qt + visits - 1) / visits - lo / visits;      // see key_walk
+      total += n;
+      longest = std::max(longest, std::min(visits, n));
+    }
+    double us = by_128.us(heads * ctas, heads * total, longest);
+    if (walks > 1) us += 2.2 + walks * heads * S * 1.9e-4;
+    if (us < least) { least = us; best = walks; }
+  }
+  return best;
 }
 
 // Backward in two kernels without per-tile global reductions: dQ from the query-tile-outer
@@ -3637,15 +3707,18 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
     w.visits_per_cta = visits_per_cta;
     w.tok_list = tok_list; w.list_start = list_start; w.item_start = item_start; w.n_lists = B * Hkv * nS; w.nS = nS;
     if (item_bound <= 0) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: item_bound must be positive");
-    const int smem = 24 * HALF + 1024 + 256;
     static bool cfg = false;
-    if (!cfg) { if ((rc = set_smem(attn_bwd_kv_kernel, smem))) return rc; cfg = true; }
+    if (!cfg) { if ((rc = set_smem(attn_bwd_kv_kernel<true>, KV_SMEM))) return rc; cfg = true; }
     CUtensorMap tq1, tdo1;
     if ((rc = make_q_map(&tq1, q, B, T, Hq, Hkv, D, 1))) return rc;
     if ((rc = make_q_map(&tdo1, d_o, B, T, Hq, Hkv, D, 1))) return rc;
-    attn_bwd_kv_kernel<<<item_bound, KV_THREADS, smem, st>>>(tq1, tdo1, tk, tv, p, w, scale);
+    attn_bwd_kv_kernel<true><<<item_bound, KV_THREADS, KV_SMEM, st>>>(tq1, tdo1, tk, tv, p, w, scale);
+  } else if (walks < 0) {
+    static bool cfg = false;
+    if (!cfg) { if ((rc = set_smem(attn_bwd_kv_kernel<false>, KV_SMEM))) return rc; cfg = true; }
+    attn_bwd_kv_kernel<false><<<dim3((S + 63) / 64, B * Hkv), KV_THREADS, KV_SMEM, st>>>(tq, tdo, tk, tv, p, KvWalk{}, scale);
   } else {
-    const int most = key_visits(T, p.R, causal, window, kp_stride);
+    const int most = KeyRange(T, S, p.R, causal, window, kp_stride, 128).most;
     KeyWalks w{};
     w.part = walks > 1 ? part : nullptr;
     if (walks > 1 && part == nullptr) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: several walks need room for their sums");

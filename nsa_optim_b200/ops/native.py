@@ -1362,7 +1362,7 @@ class _NSA(torch.autograd.Function):
         _attn_backward_split(q, k, v, o2, d2, L2, dq, dk, dv, True, 0, scale, 1, 0, ctx.tiles, sums[1], True)
         # The window branch shares dk / dv while a key block's gradients get one addition from it: one more to what is there gives
         # the same bits on every run, two in either order would not.
-        shared = lib.nsa_attn_bwd_walks(*q.shape[:2], k.shape[1], q.shape[2], k.shape[2], 1, window, 1) > 0
+        shared = lib.nsa_attn_bwd_walks(*q.shape[:2], k.shape[1], q.shape[2], k.shape[2], 1, window, 1) != 0
         dk3, dv3 = (dk, dv) if shared else (_zeros(t.shape, dtype=f32, device=q.device) for t in (k, v))
         _attn_backward_split(q, k, v, o3, d3, L3, dq, dk3, dv3, True, window, scale, 1, 0, None, sums[2], True)
         if not shared:

@@ -1,4 +1,4 @@
-"""dK / dV over contiguous key ranges: blocks of 128 keys that the sequence ends inside, groups from one head to 32, windows around a
+"""dK / dV over contiguous key ranges: blocks of 64 and of 128 keys that the sequence ends inside, groups from one head to 32, windows around a
 block's length, one walk a block and several, and several sequences; twice the same bits where the sums are ordered."""
 import pytest
 import torch
@@ -55,3 +55,20 @@ def test_key_gradients_without_causality(native, T, Hq, Hkv, window):
 @pytest.mark.parametrize("T,Hq,Hkv,window", [(300, 16, 1, 2 ** 31 - 1), (300, 2, 2, 2 ** 31 - 129), (1100, 32, 1, 2 ** 31 - 1), (300, 16, 1, 300)])
 def test_key_gradients_of_the_widest_windows(native, T, Hq, Hkv, window, causal):
     _check(native, 1, T, Hq, Hkv, window, causal)
+
+
+# Every form on ranges that the rule may give to another: 64 keys a CTA, one walk of 128 keys, several, one visit each
+@pytest.mark.parametrize("form", [-1, 1, 2, 5, 64])
+@pytest.mark.parametrize("B,T,Hq,Hkv,window,causal", [(1, 1, 4, 4, 0, True), (2, 65, 8, 1, 0, True), (1, 127, 16, 16, 0, True), (1, 300, 16, 8, 64, True),
+                                                      (1, 300, 16, 8, 64, False), (1, 520, 32, 2, 129, True), (2, 333, 16, 2, 0, False)])
+def test_forms(native, monkeypatch, B, T, Hq, Hkv, window, causal, form):
+    monkeypatch.setattr(native.load(), "nsa_attn_bwd_walks", lambda *args: form)
+    _check(native, B, T, Hq, Hkv, window, causal)
+
+
+# Where few tiles visit a block the smaller blocks are faster, also with a window, and where blocks are few several walks are.  us
+# (64 keys; 128 keys and one walk; and several): 7.4, 10; 12.9, 17; 9.5, 14.4; 20, 32, 24; 181, 210, 33; 51, 46, 56
+@pytest.mark.parametrize("T,Hq,Hkv,window,low,high", [(128, 16, 16, 0, -1, -1), (300, 16, 8, 0, -1, -1), (1000, 16, 8, 64, -1, -1),
+                                                      (3000, 16, 2, 64, -1, -1), (1000, 32, 2, 0, 12, 20), (1500, 16, 16, 0, 1, 1)])
+def test_choice_of_form(native, T, Hq, Hkv, window, low, high):
+    assert low <= native.load().nsa_attn_bwd_walks(1, T, T, Hq, Hkv, 1, window, 1) <= high
