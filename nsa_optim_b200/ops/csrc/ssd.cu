@@ -1444,12 +1444,15 @@ extern "C" int nsa_ssd_finish(const float* dB_part, const float* dC_part, const 
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_finish launch");
 }
 
-// One pass over the chunks (nsa_ssd_states) or chunk_state and the state pass.  The walk takes 1.15 us a chunk for up to one head per
-// SM; the two kernels 0.0205 us per (chunk, head), 17 us for two launches at least.  16384 tokens, 64 heads: 141 us
-// against 169; 48: 141 and 121; 24: 140 and 69; two sequences of 8192 x 64: 82 and 162; 1000 tokens x 32: 14 and 19.
+// One pass over the chunks (nsa_ssd_states) or chunk_state and the state pass.  The walk takes 3.2 us and 1.13 a chunk for up to one head
+// per SM.  The two kernels take 6.6 us and 0.095 a chunk (the pass is a chain), 5.1 and 0.0165 per (chunk, head), or 0.019 per
+// (chunk, head), whichever is the most, and have a gap between them.  Walk and two kernels, us: 300 tokens x 1 head 6.3, 6.7;
+// 1000 x 1 11.1, 6.6; 1000 x 32 12.0, 9.1; 1000 x 48 12.3, 11.4; 777 x 64 11.0, 12.9; 1500 x 64 17, 19.2; 1000 x 128 13.4, 22.1;
+// 16384 x 48 141, 121; 16384 x 64 141, 169; 2 x 8192 x 32 72, 83.
 extern "C" int nsa_ssd_states_in_one(int B, int T, int H) {
-  const long heads = static_cast<long>(B) * H, chunks = (T + L - 1) / L, sms = nsa::sm_count();
-  return 1.15 * chunks * ((heads + sms - 1) / sms) + 4. <= std::max(17., 0.0205 * heads * chunks);
+  const long heads = static_cast<long>(B) * H, chunks = (T + L - 1) / L, items = heads * chunks, sms = nsa::sm_count();
+  const double walk = (3.2 + 1.13 * chunks) * ((heads + sms - 1) / sms);
+  return walk <= std::max({6.6 + 0.095 * chunks, 5.1 + 0.0165 * items, 0.019 * items}) + 0.5;
 }
 
 // back = 0: bc = B rows, v = x -> states entering the chunks; back = 1: bc = C rows, v = dy -> gradients of the states leaving them.

@@ -40,9 +40,15 @@ def test_ssd_sizes(native, B, T, H, skip):
 # 32 sequences x heads and more: the states come from one walk over the chunks (one chunk, as many as it has stages, more); runs of
 # (chunk, head) items that end inside a chunk, at its end, and go over several
 @pytest.mark.parametrize("B,T,H,skip", [(32, 5, 1, True), (1, 256, 32, True), (2, 384, 16, False), (1, 513, 48, True), (2, 700, 70, True),
-                                        (1, 1100, 33, False)])
+                                        (1, 1100, 33, False), (1, 1100, 70, False)])
 def test_ssd_walk_and_runs(native, B, T, H, skip):
     test_ssd_sizes(native, B, T, H, skip)
+
+
+@pytest.mark.parametrize("B,T,H,one", [(1, 300, 1, True), (1, 1000, 1, False), (1, 1000, 48, False), (1, 777, 64, True), (1, 16384, 48, False),
+                                       (1, 16384, 64, True)])
+def test_choice_of_state_kernels(native, B, T, H, one):
+    assert bool(native.load().nsa_ssd_states_in_one(B, T, H)) == one              # times of both: see there
 
 
 # A step that forgets everything, or is not finite, at each place of the four that a lane scans, in the second chunk: what comes
