@@ -666,7 +666,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
     auto krow = [](int kk) { return static_cast<uint64_t>((kk * 2048) >> 4); };
     auto box = [&](int k, int i) { return tc5::smem_u32(stages + ((k & 1) * 4 + i) * BOXB); };      // x, dy, H, dHn of item k
     int seg = 0;
-    auto open_segment = [&]() {                        // C and B of the chunk of `cur`, S^T = B C^T
+    auto load_chunk = [&]() {                          // C and B of the chunk of `cur`
       if (lead) {
         tc5::mbar_expect_tx(cb, 4 * BOXB);
         tc5::tma_load_3d(sC, &tm_c, cb, 0, cur.t0, cur.b);
@@ -675,6 +675,8 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
         tc5::tma_load_3d(sB + BOXB, &tm_b, cb, 64, cur.t0, cur.b);
       }
       __syncwarp();
+    };
+    auto open_segment = [&]() {                        // S^T = B C^T
       if (!wait(cb, seg, STATUS_TIMEOUT_SMEM_FULL)) return false;
       tc5::fence_after_sync();
       if (lead) {
@@ -705,6 +707,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
       }
       __syncwarp();
     };
+    load_chunk();
     if (lead) load(0);
     chunk_scan_warp<false>(load_dt4(p, ahead.b, ahead.t0, ahead.h), p.A[ahead.h], cum, dts, colf);
     arrive_warp(scanned);
@@ -785,9 +788,9 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
       if (same) {
         state_rows(k + 1);
       } else if (more) {                               // every product and every reader of the segment is through: C and B may go
-        ok = wait(left, k, STATUS_TIMEOUT_TMEM_EMPTY) && open_segment() &&
-             wait(full + ((k + 1) & 1), (k + 1) >> 1, STATUS_TIMEOUT_SMEM_FULL);
-        if (!ok) break;
+        if (!(ok = wait(left, k, STATUS_TIMEOUT_TMEM_EMPTY))) break;
+        load_chunk();
+        if (!(ok = open_segment() && wait(full + ((k + 1) & 1), (k + 1) >> 1, STATUS_TIMEOUT_SMEM_FULL))) break;
         tc5::fence_after_sync();
         scores(k + 1);
         state_rows(k + 1);
@@ -965,15 +968,31 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
           tc5::fence_after_sync();
           const long chunk = static_cast<long>(cur.b) * p.nc + cur.t0 / L;
           const int slot = blockIdx.x - static_cast<int>(chunk * p.H / p.quota);
-          const long o = (tok * p.slots + slot) * NS + grp * 32;
+          // Sixteen columns at a time through the warp's own piece of dS (its products are complete), so that four lanes write 64 bytes
+          // of a row: a lane that writes its own row leaves 16 bytes in each of 32 rows, which took 5 of 16 us of a CTA with one item.
+          uint8_t* piece = sDS + (grp >> 1) * BOXB + quad * 32 * 128;
+          const int j0 = (grp & 1) * 4, col = lane & 3;
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             float v[32];
             tld32(lanes + (q ? cDC : cDB) + grp * 32, v);
-            float* dst = (q ? p.dC_part : p.dB_part) + o;
-            if (t < p.T)
+            float* part = q ? p.dC_part : p.dB_part;
 #pragma unroll
-              for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<float4*>(piece + lane * 128 + (((j0 + j) ^ (lane & 7)) << 4)) =
+                    make_float4(v[hf * 16 + 4 * j], v[hf * 16 + 4 * j + 1], v[hf * 16 + 4 * j + 2], v[hf * 16 + 4 * j + 3]);
+              __syncwarp();
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int row = i * 8 + (lane >> 2), tr = cur.t0 + quad * 32 + row;
+                const float4 w = *reinterpret_cast<const float4*>(piece + row * 128 + (((j0 + col) ^ (row & 7)) << 4));
+                if (tr < p.T)
+                  *reinterpret_cast<float4*>(part + ((static_cast<long>(cur.b) * p.T + tr) * p.slots + slot) * NS + grp * 32 + hf * 16 + col * 4) = w;
+              }
+              __syncwarp();
+            }
           }
         }
       }
