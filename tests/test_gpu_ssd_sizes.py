@@ -158,3 +158,9 @@ def test_state_pass_of_few_elements_is_a_short_chain(native):
         b.synchronize()
         times.append(a.elapsed_time(b) / 20 * 1e3)
     assert min(times[2:]) <= 60, times
+
+
+# Partial sums per token on both sides of the rule for how many are in flight: 1, 2 to 4, 5, and one per head, more than sixteen
+@pytest.mark.parametrize("B,T,H", [(1, 130, 1), (1, 2048, 32), (1, 1500, 24), (1, 140, 5), (2, 129, 17), (1, 128, 40)])
+def test_ssd_partial_sums(native, B, T, H):
+    test_ssd_sizes(native, B, T, H, True)
