@@ -1452,7 +1452,7 @@ extern "C" int nsa_ssd_state_bwd(const float* dHprev, const float* gamma, float*
 // chunk can fall into.
 extern "C" int nsa_ssd_grad_slots(int B, int T, int H) {
   const int quota = items_per_cta(B, T, H);
-  return H < 2 ? 1 : (H - 2) / quota + 2;
+  return H < 2 || quota == 0 ? 1 : (H - 2) / quota + 2;
 }
 
 // dB_part, dC_part [B, T, slots, 128] fp32 of nsa_ssd_chunk_grad -> dB, dC [B, T, 128] bf16; q, k, r (or null), dt [B, T, H], A [H]

@@ -160,7 +160,14 @@ def test_state_pass_of_few_elements_is_a_short_chain(native):
     assert min(times[2:]) <= 60, times
 
 
-# Partial sums per token on both sides of the rule for how many are in flight: 1, 2 to 4, 5, and one per head, more than sixteen
-@pytest.mark.parametrize("B,T,H", [(1, 130, 1), (1, 2048, 32), (1, 1500, 24), (1, 140, 5), (2, 129, 17), (1, 128, 40)])
+# Partial sums per token on both sides of the rule for how many are in flight: room for 1, 2, 4, 5, 13, 17 and 40
+@pytest.mark.parametrize("B,T,H", [(1, 130, 1), (16, 900, 8), (7, 1000, 24), (1, 140, 5), (1, 1500, 24), (2, 129, 17), (1, 128, 40)])
 def test_ssd_partial_sums(native, B, T, H):
     test_ssd_sizes(native, B, T, H, True)
+
+
+def test_no_items(native):
+    # sizes that nothing can be launched for are refused by the kernels' entry points; asking what they need is no crash
+    for sizes in ((0, 100, 8), (1, 0, 8), (1, 100, 0)):
+        assert native.load().nsa_ssd_grad_slots(*sizes) >= 0
+        assert native.load().nsa_ssd_states_in_one(*sizes) in (0, 1)
