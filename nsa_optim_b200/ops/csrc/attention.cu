@@ -2502,10 +2502,6 @@ __global__ void __launch_bounds__(256) attn_sum_walks_kernel(const AttnParams p,
 
 constexpr int KVC_THREADS = 352;
 constexpr int KVC_SMEM = 28 * HALF + 2 * 2 * 128 * 4 + 256;
-__device__ __forceinline__ void arrive_warp(uint64_t* bar) {
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) tc5::mbar_arrive(bar);
-}
 
 __global__ void __launch_bounds__(KVC_THREADS, 1)
 attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
@@ -2689,7 +2685,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       if (v >= 2 && !wait(st_empty + (v & 1), (v >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY)) break;
       *reinterpret_cast<float4*>(st + 4 * lane) = make_float4(negL[0], negL[1], negL[2], negL[3]);
       *reinterpret_cast<float4*>(st + 128 + 4 * lane) = make_float4(nds[0], nds[1], nds[2], nds[3]);
-      arrive_warp(st_full + (v & 1));
+      tc5::arrive_warp(st_full + (v & 1));
     }
   } else {
     // ------------------------------------------------------------------ softmax warps: key lane, query rows 64 ch ..
@@ -2749,7 +2745,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         tc5::tmem_st_x16(lanes + cS + q * 16, pk);
         tc5::tmem_st_wait();
         tc5::fence_before_sync();
-        arrive_warp(p_full + q);
+        tc5::arrive_warp(p_full + q);
       }
       if (!(ok = wait(dp_full, v, STATUS_TIMEOUT_TMEM_FULL))) break;
       tc5::fence_after_sync();

@@ -7,6 +7,7 @@
 // Weight gradients of the norms and the convolution are reduced deterministically:
 // a persistent grid accumulates per-CTA partial sums into a scratch buffer
 // [grid, width] (fp32) that a second kernel adds up in a fixed order.
+#include "f32x2.cuh"
 #include "host.cuh"
 #include <cuda_bf16.h>
 
@@ -655,15 +656,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Two fp32 lanes per instruction; each lane rounds as the scalar instruction does.
-__device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(reinterpret_cast<unsigned long long&>(d))
-      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
-        "l"(reinterpret_cast<const unsigned long long&>(c)));
-  return d;
-}
 struct Quad {        // four channels
   float2 a, b;
 };

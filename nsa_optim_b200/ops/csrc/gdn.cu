@@ -71,7 +71,7 @@ __device__ __forceinline__ void pack_half(const float (&in)[HC], uint32_t (&pack
 struct FwdParams {
   const float* gc;      // [BH, NC, 64]
   int store_states;     // also write v_new and S_all (the backward needs them)
-  int NC, V, H;
+  int NC, H;
   float scale;
   KernelStatus* status;
 };
@@ -86,10 +86,6 @@ constexpr int WARP_MMA = 8, WARP_LOAD = 9;
 // product is issued, 356 and 365 with u and do as tiles too (rows of their own per thread are 32 lines an instruction),
 // 336 and 361 with the wait for a tile's last stores in front of the one for the state.
 constexpr int AHEAD = 6;
-__device__ __forceinline__ void arrive_warp(uint64_t* bar) {
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) tc5::mbar_arrive(bar);
-}
 
 // stage: k-block kb of [w ; q] (2 x 16 KB), k (16 KB), [0 ; qk] (16 KB, first half zero)
 constexpr int FWD_STAGE = 8 * BOX;
@@ -166,8 +162,8 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       tmem_st_half(tmem + lane_off + cS, z);
     }
     tc5::fence_before_sync();
-    arrive_warp(sready);
-    arrive_warp(scaled);
+    tc5::arrive_warp(sready);
+    tc5::arrive_warp(scaled);
     const bool upper = r < CH;                     // rows of w S and v_new; the others hold q S and the output
     // The gates are in flight for a whole chunk.
     float g_row = gc[r & 63], g_last = gc[CH - 1];
@@ -182,7 +178,7 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       if (upper) {
         if (!wait(full_u + (c & 1), c >> 1, STATUS_TIMEOUT_SMEM_FULL)) break;
         read_half(Us + (c & 1) * BOX, r, half, uf);
-        arrive_warp(empty_u + (c & 1));
+        tc5::arrive_warp(empty_u + (c & 1));
       }
       if (!wait(m1, c, STATUS_TIMEOUT_TMEM_FULL)) break;
       tc5::fence_after_sync();
@@ -199,7 +195,7 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         write_half(Vs, r, half, ps);               // read by the products of chunk c - 1, complete since m2
         write_half(Vb + (c & 1) * BOX, r, half, pk);
         tc5::fence_proxy_async();
-        arrive_warp(vready);
+        tc5::arrive_warp(vready);
       } else {
 #pragma unroll
         for (int j = 0; j < HC; ++j) d1[j] *= sq;
@@ -216,12 +212,12 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         write_half(Sb + ((c + 1) & 1) * 2 * BOX, r, half, pk);
         tc5::fence_proxy_async();
         tc5::fence_before_sync();
-        arrive_warp(sready);
+        tc5::arrive_warp(sready);
 #pragma unroll
         for (int j = 0; j < HC; ++j) sv[j] *= g;
         tmem_st_half(tmem + lane_off + cS, sv);
         tc5::fence_before_sync();
-        arrive_warp(scaled);
+        tc5::arrive_warp(scaled);
       } else if (!wait(freed, c, STATUS_TIMEOUT_SMEM_EMPTY)) {
         break;
       }
@@ -237,7 +233,7 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         write_half(Ob + (c & 1) * BOX, r - CH, half, pk);
         tc5::fence_proxy_async();
         tc5::fence_before_sync();
-        arrive_warp(oready);
+        tc5::arrive_warp(oready);
       }
       g_row = g_row_next;
       g_last = g_last_next;
@@ -360,7 +356,7 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         tc5::tma_store_commit();
         tc5::tma_store_wait_read<1>();
       }
-      arrive_warp(freed);
+      tc5::arrive_warp(freed);
     }
     if (ok && wait(oready, NC - 1, STATUS_TIMEOUT_TMEM_EMPTY)) store_o(NC - 1);
     if (lead) {
@@ -377,7 +373,7 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 struct BwdParams {
   const float* gc;       // [BH, NC, 64]
   float* dgamma_part;    // [VTILES, BH, NC]
-  int NC, V, BH, H, T;
+  int NC, BH, H;
   float scale;
   KernelStatus* status;
 };
@@ -457,8 +453,8 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       tmem_st_half(tmem + lane_off + cDs, z);
     }
     tc5::fence_before_sync();
-    arrive_warp(sready);
-    arrive_warp(scaled);
+    tc5::arrive_warp(sready);
+    tc5::arrive_warp(scaled);
     auto stage_row = [&](int it, float g_row) {    // sq do of step `it`
       if (!wait(full + (it & 1), it >> 1, STATUS_TIMEOUT_SMEM_FULL)) return false;
       float f[HC];
@@ -470,7 +466,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       pack_half(f, pk);
       write_half(sDOs, r - CH, half, pk);
       tc5::fence_proxy_async();
-      arrive_warp(oready);
+      tc5::arrive_warp(oready);
       return true;
     };
     // dgamma of step `it`, whose leaving gradient is ds: partial per warp; the last use of the entering state in the stage
@@ -484,8 +480,8 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
       if ((threadIdx.x & 31) == 0) red[s * 8 + warp] = part;
-      arrive_warp(gready);
-      arrive_warp(empty_s + s);
+      tc5::arrive_warp(gready);
+      tc5::arrive_warp(empty_s + s);
       return true;
     };
     float g_row = gc[(NC - 1) * CH + (r & 63)], g_last = gc[(NC - 1) * CH + CH - 1];
@@ -517,7 +513,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         write_half(sDU + (it & 1) * BOX, r, half, pk);
         tc5::fence_proxy_async();
         tc5::fence_before_sync();
-        arrive_warp(uready);
+        tc5::arrive_warp(uready);
       }
       if (c == 0) break;
       const float g = __expf(g_last_next);
@@ -530,7 +526,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       write_half(dSb, r, half, pk);
       tc5::fence_proxy_async();
       tc5::fence_before_sync();
-      arrive_warp(sready);
+      tc5::arrive_warp(sready);
       if (!upper && !stage_row(it + 1, g_row_next)) break;
       {
         float sv[HC];
@@ -539,7 +535,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         tmem_st_half(tmem + lane_off + cDs, sv);
       }
       tc5::fence_before_sync();
-      arrive_warp(scaled);
+      tc5::arrive_warp(scaled);
       ok = gamma_part(it + 1, ds);
       g_row = g_row_next;
       g_last = g_last_next;
@@ -666,7 +662,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         tc5::tma_store_commit();
         tc5::tma_store_wait_read<1>();             // dS of this chunk and du of the one before have been read
       }
-      arrive_warp(freed);
+      tc5::arrive_warp(freed);
     }
     if (lead) tc5::tma_store_wait_read<0>();
     __syncwarp();
@@ -714,7 +710,7 @@ extern "C" int nsa_gdn_seq_fwd(const void* q, const void* k, const void* w, cons
   tvn = tw; tsa = tw;                              // never used without the states
   if (states && (rc = make_rows_map(&tvn, v_new, rows, V, CH))) return rc;
   if (states && (rc = make_rows_map(&tsa, S_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
-  FwdParams p{gc, states, NC, V, H, scale, nsa::status_ptr()};
+  FwdParams p{gc, states, NC, H, scale, nsa::status_ptr()};
   if ((rc = set_smem(gdn_seq_fwd_kernel, FWD_SMEM, "gdn fwd smem attribute"))) return rc;
   gdn_seq_fwd_kernel<<<dim3(V / VT, BH), 352, FWD_SMEM, st>>>(tw, tu, tq, tk, tqk, tvn, to, tsa, p);
   nsa::count_launch();
@@ -740,7 +736,7 @@ extern "C" int nsa_gdn_seq_bwd(const void* q, const void* k, const void* w, cons
   if ((rc = make_token_map(&tdo, d_o, B, T, H, V))) return rc;
   if ((rc = make_rows_map(&tdu, du, rows, V, CH))) return rc;
   if ((rc = make_rows_map(&tds, dS_all, static_cast<long>(BH) * NC * KD, V, KD))) return rc;
-  BwdParams p{gc, dgamma_part, NC, V, BH, H, T, scale, nsa::status_ptr()};
+  BwdParams p{gc, dgamma_part, NC, BH, H, scale, nsa::status_ptr()};
   if ((rc = set_smem(gdn_seq_bwd_kernel, BWD_SMEM, "gdn bwd smem attribute"))) return rc;
   gdn_seq_bwd_kernel<<<dim3(V / VT, BH), 352, BWD_SMEM, st>>>(tw, tq, tk, ts, tqk, tdo, tdu, tds, p);
   nsa::count_launch();

@@ -6,6 +6,7 @@
 //     Tu = X diag(beta), Tw = X diag(beta e^gc)                       u = Tu v, w = Tw k
 //     qk[i][j] = scale (q_i . k_j) e^(gc_i - gc_j)    (j <= i)
 // q, k, v and the gates are read token-major as the caller has them, gradients leave the same way.
+#include "f32x2.cuh"
 #include "host.cuh"
 #include "mma16.cuh"
 #include "tc5.cuh"
@@ -15,16 +16,6 @@ using namespace mma16;
 constexpr int CH = 64, KD = 128;
 constexpr int PK = KD + 8, PC = CH + 8;          // tile pitches (elements)
 constexpr int PX = 68;                           // pitch of the fp32 64 x 64 tiles: rows 16-byte aligned, spread over the banks
-
-// Two fp32 lanes per instruction; each lane rounds as the scalar instruction does.
-__device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(reinterpret_cast<unsigned long long&>(d))
-      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
-        "l"(reinterpret_cast<const unsigned long long&>(c)));
-  return d;
-}
 
 // Per-chunk gate quantities: the CTA's first warp does the work, two tokens a lane; the caller synchronises.
 // gs: cumulative log-decay, bs: beta.

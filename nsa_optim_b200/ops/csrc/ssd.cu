@@ -17,6 +17,7 @@
 // Decay factors are formed per element in registers (exp2 of a difference that is <= 0), never
 // stored; the [128 x 128] P and dS tiles live only on chip, as bf16 MMA operands.
 #include <algorithm>
+#include "f32x2.cuh"
 #include "host.cuh"
 #include "tc5.cuh"
 
@@ -95,22 +96,6 @@ __device__ __forceinline__ void tld64(uint32_t taddr, float (&out)[64]) {
   for (int j = 0; j < 32; ++j) { out[j] = __uint_as_float(a[j]); out[32 + j] = __uint_as_float(b[j]); }
 }
 
-// Two fp32 lanes per instruction; each lane rounds as the scalar instruction does.
-__device__ __forceinline__ float2 mul2(const float2& a, const float2& b) {
-  float2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(reinterpret_cast<unsigned long long&>(d))
-      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
-  return d;
-}
-__device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(reinterpret_cast<unsigned long long&>(d))
-      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
-        "l"(reinterpret_cast<const unsigned long long&>(c)));
-  return d;
-}
 __device__ __forceinline__ float2 unpack2(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); }
 
 // OR over the sixteen computing warps of a kernel that has one more
@@ -317,10 +302,6 @@ __device__ __forceinline__ void chunk_scan_warp(float4 dt, float a, float* cum, 
     }
   }
 }
-__device__ __forceinline__ void arrive_warp(uint64_t* bar) {
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) tc5::mbar_arrive(bar);
-}
 
 // ---------------------------------------------------------------------------------------
 // chunk_out: y = P x + exp(cum) (C H) + D x.
@@ -482,7 +463,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
       if (k > 1 && !wait(ready + (k & 1), (k >> 1) - 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;       // those of item k - 2 have been read
       float* at = scan + (k & 1) * (2 * L + 192);
       chunk_scan_warp<true>(dt, a, at, at + L, at + 2 * L);
-      arrive_warp(scanned + (k & 1));
+      tc5::arrive_warp(scanned + (k & 1));
       dt = dt_next;
       a = a_next;
     }
@@ -504,7 +485,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
           tc5::fence_after_sync();
           tld32(lanes + cS + grp * 32, s);
           tc5::fence_before_sync();
-          arrive_warp(sread);
+          tc5::arrive_warp(sread);
           ++seg;
         }
         if (!wait(scanned + buf, k >> 1, STATUS_TIMEOUT_SMEM_FULL)) break;
@@ -538,7 +519,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
         tc5::tmem_st_x16(lanes + cP + buf * 64 + grp * 16, pk);
         tc5::tmem_st_wait();
         tc5::fence_before_sync();
-        arrive_warp(ready + buf);
+        tc5::arrive_warp(ready + buf);
       }
       if (k > 0) {                                     // rows of the item before, whose products ran meanwhile
         const int q = k - 1, buf = q & 1;
@@ -559,7 +540,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
           *reinterpret_cast<uint4*>(base + (((grp * 2 + j) ^ (r & 7)) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
         tc5::fence_proxy_async();
         tc5::fence_before_sync();
-        arrive_warp(left + q % OUT_ST);
+        tc5::arrive_warp(left + q % OUT_ST);
       }
       e_open = e;
       dsk_open = dsk;
@@ -710,7 +691,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
     load_chunk();
     if (lead) load(0);
     chunk_scan_warp<false>(load_dt4(p, ahead.b, ahead.t0, ahead.h), p.A[ahead.h], cum, dts, colf);
-    arrive_warp(scanned);
+    tc5::arrive_warp(scanned);
     ahead.next();
     // A step issues the rest of item k and the first products of item k + 1 between them, so that the scores of k + 1 are
     // there when the warps have finished the rows of k, and the sums over heads run behind their work.
@@ -782,7 +763,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
       __syncwarp();
       if (more) {                                      // this item's sums of step sizes have been read
         chunk_scan_warp<false>(dt_next, a_next, cum, dts, colf);
-        arrive_warp(scanned);
+        tc5::arrive_warp(scanned);
       }
       cur.next();
       if (same) {
@@ -824,7 +805,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
           tc5::fence_after_sync();
           tld32(lanes + cR + grp * 32, s);
           tc5::fence_before_sync();
-          arrive_warp(sread);
+          tc5::arrive_warp(sread);
         }
         ++seg;
       }
@@ -926,7 +907,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
           tc5::tmem_st_wait();
           tc5::fence_proxy_async();
           tc5::fence_before_sync();
-          arrive_warp(ready);
+          tc5::arrive_warp(ready);
         }
       }
       ok = ok && wait(m2, k, STATUS_TIMEOUT_TMEM_FULL);
@@ -999,7 +980,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
       if (!ok) continue;                               // the next item's vote ends the walk
       tc5::fence_proxy_async();
       tc5::fence_before_sync();
-      arrive_warp(left);
+      tc5::arrive_warp(left);
     }
   }
   tc5::fence_before_sync();
@@ -1063,7 +1044,7 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
         const float g = decay[(i - 1) & 1];            // of the chunk before
         tld32(acc + ((i - 1) & 1) * 64, a);
         tc5::fence_before_sync();
-        arrive_warp(taken + ((i - 1) & 1));
+        tc5::arrive_warp(taken + ((i - 1) & 1));
         const float2 g2 = make_float2(g, g);
 #pragma unroll
         for (int j = 0; j < 16; ++j) st[j] = fma2(g2, st[j], make_float2(a[2 * j], a[2 * j + 1]));
@@ -1074,7 +1055,7 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
       if (i > 0 && !wait(freed, i - 1, STATUS_TIMEOUT_SMEM_EMPTY)) break;
       st_row32(sOut, r, half * 32, pk);
       tc5::fence_proxy_async();
-      arrive_warp(oready);
+      tc5::arrive_warp(oready);
     }
   } else if (warp < 16) {                              // row t of B (C), 64 columns
     for (int i = 0; i + 1 < nc; ++i) {
@@ -1096,7 +1077,7 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
       // the decay goes along to the product's readers, who have taken the one two chunks back
       if (i > 1 && !wait(taken + (i & 1), (i >> 1) - 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;
       if (threadIdx.x == 256) decay[i & 1] = scale[s * (L + 4) + L];
-      arrive_warp(ready + (i & 1));
+      tc5::arrive_warp(ready + (i & 1));
     }
   } else if (warp == 16) {
     constexpr uint32_t idesc = tc5::make_idesc_bf16(128, PD, 1, 1);
@@ -1152,7 +1133,7 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
       float* sc = scale + s * (L + 4);
       *reinterpret_cast<float4*>(sc + 4 * lane) = make_float4(weight(c.x, dt.x), weight(c.y, dt.y), weight(c.z, dt.z), weight(c.w, dt.w));
       if (lane == 0) sc[L] = exp2f(tot);
-      arrive_warp(full + s);
+      tc5::arrive_warp(full + s);
       dt = dt_next;
     }
     // stages whose last use was not waited for above
@@ -1169,7 +1150,7 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
         tc5::tma_store_commit();
         tc5::tma_store_wait_read<0>();
       }
-      arrive_warp(freed);
+      tc5::arrive_warp(freed);
     }
     if (lead) tc5::tma_store_wait_read<0>();
     __syncwarp();
