@@ -26,7 +26,7 @@ def _check(native, q, k, v, seen, got):
     (1, 1184, 32, 2, True, 0), (1, 1176, 32, 2, True, 0),      # 296 and 294 tiles of up to 19 visits: one CTA per SM
     (4, 1191, 16, 2, False, 0), (2, 1500, 32, 2, True, 100), (40, 33, 16, 8, True, 0), (300, 1, 2, 1, True, 0), (19, 130, 16, 16, False, 64),
     (1, 1200, 32, 1, True, 0), (2, 600, 32, 1, True, 0),       # groups of 32: 300 tiles of 4 tokens
-    (2, 1340, 32, 2, True, 700), (1, 2400, 32, 2, False, 0),   # 12 visits of a window; more than 16 without and with one
+    (2, 1340, 32, 2, True, 700), (1, 2400, 32, 2, False, 0),   # 12 visits of a window; 38; with windows 21 and 16
     (1, 2400, 32, 2, True, 1300), (2, 1340, 32, 2, True, 1000),
     (8, 1400, 16, 8, True, 0)])
 def test_forward(native, B, T, Hq, Hkv, causal, window):
