@@ -455,6 +455,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 512); }
 }
 
+// Q (or dO) from shared memory (k-blocks of [128 rows][64], 128B swizzle) into tensor memory: half `half` of row r, columns of two bf16.
+template <int D>
+__device__ __forceinline__ void q_half_to_tmem(uint32_t taddr, const uint8_t* tile, int r, int half) {
+  constexpr int N = D / 4, PIECES = D / 16;      // words and 16-byte pieces of half a row
+  uint32_t w[N];
+#pragma unroll
+  for (int j = 0; j < PIECES; ++j) {
+    const int piece = half * PIECES + j;
+    const uint4 x = *reinterpret_cast<const uint4*>(tile + (piece >> 3) * 2 * HALF + r * 128 + (((piece & 7) ^ (r & 7)) << 4));
+    w[4 * j] = x.x; w[4 * j + 1] = x.y; w[4 * j + 2] = x.z; w[4 * j + 3] = x.w;
+  }
+  if constexpr (D == 128) tc5::tmem_st_x32(taddr + half * N, w);
+  else tc5::tmem_st_x16(taddr + half * N, w);
+  tc5::tmem_st_wait();                           // the registers are not to be rewritten before
+}
+
 // --------------------------------------------------------------------------------------
 // Forward, warp-specialised, Q and P in tensor memory (head_dim 128, output mode).  Visits are
 // 64-key blocks as in the dQ kernel.  Warp 8 streams K/V through a 5-stage ring, warp 9 issues
@@ -472,19 +488,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // place or overwrites P.
 // --------------------------------------------------------------------------------------
 constexpr int FWT_STAGES = 5;
+constexpr int fwt_smem(int D) { return D / 64 * (2 + 2 * FWT_STAGES) * HALF + 1024 + 1024 + 256; }
 
 // The order of the tiles is a template argument here: chosen at run time it costs registers and 2 % without causality.
-template <bool LONGEST_FIRST>
+template <int D, bool LONGEST_FIRST>
 __global__ void __launch_bounds__(352, 1)
 attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
-  constexpr int D = 128;
-  constexpr int QT = 4 * HALF;
+  constexpr int KB = D / 64;                     // 64-column k-blocks of an operand
+  constexpr int QT = KB * 2 * HALF, KVT = KB * HALF;   // [128 rows][D] of Q, [64 keys][D] of K or V
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sKV = sQ + QT;                        // [stages][K: 2 k-blocks of [64][64] | V: same]
-  float* merge = reinterpret_cast<float*>(sKV + FWT_STAGES * 4 * HALF);   // [2][128]: group 1's m and l
+  uint8_t* sKV = sQ + QT;                        // [stages][K: KB k-blocks of [64][64] | V: same]
+  float* merge = reinterpret_cast<float*>(sKV + FWT_STAGES * 2 * KVT);   // [2][128]: group 1's m and l
   uint64_t* bars = reinterpret_cast<uint64_t*>(merge + 256);
   uint64_t* q_full = bars;
   uint64_t* kv_full = bars + 1;                  // [stages]
@@ -549,15 +566,15 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  // columns: S of group g at g*64; O of group g at 128 + g*128; Q at 384; P of group g at 448 + g*32
-  constexpr uint32_t cO = 128, cQ = 384, cP = 448;
+  // columns: S of group g at g*64, O of group g at 128 + g*D, then Q, and P of group g at cP + g*32
+  constexpr uint32_t cO = 128, cQ = cO + 2 * D, cP = cQ + D / 2;
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0 && n_vis > 0) {
       tc5::mbar_expect_tx(q_full, QT);
 #pragma unroll
-      for (int kb = 0; kb < 2; ++kb) tc5::tma_load_5d(sQ + kb * 2 * HALF, &tm_q, q_full, kb * 64, 0, h, q0, b);
+      for (int kb = 0; kb < KB; ++kb) tc5::tma_load_5d(sQ + kb * 2 * HALF, &tm_q, q_full, kb * 64, 0, h, q0, b);
       bool ok = true;
       int issued = 0;
       int blk_n = selected ? blocks[0] : 0;
@@ -567,12 +584,12 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         if (selected && v + 1 < n_vis) blk_n = blocks[v + 1];
         if (!tc5::mbar_wait(kv_empty + st, ((v / FWT_STAGES) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY)) { ok = false; break; }
         const int s0 = selected ? (blk < 0 ? 0 : blk * 64) : (kb0 + v) * 64;
-        uint8_t* kd = sKV + st * 4 * HALF;
-        tc5::mbar_expect_tx(kv_full + st, 4 * HALF);
+        uint8_t* kd = sKV + st * 2 * KVT;
+        tc5::mbar_expect_tx(kv_full + st, 2 * KVT);
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
+        for (int kb = 0; kb < KB; ++kb) {
           tc5::tma_load_4d(kd + kb * HALF, &tm_k, kv_full + st, kb * 64, h, s0, b);
-          tc5::tma_load_4d(kd + 2 * HALF + kb * HALF, &tm_v, kv_full + st, kb * 64, h, s0, b);
+          tc5::tma_load_4d(kd + KVT + kb * HALF, &tm_v, kv_full + st, kb * 64, h, s0, b);
         }
         issued = v + 1;
       }
@@ -611,7 +628,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                      tc5::mbar_wait(s_empty + g, ((v >> 1) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
         if (!ok) break;
         tc5::fence_after_sync();
-        const uint64_t bK = bK0 + static_cast<uint64_t>((st * 4 * HALF) >> 4);
+        const uint64_t bK = bK0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
         if (lead) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk)
@@ -627,7 +644,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (n_vis > 0) {
       const bool lead = tc5::elect_one();
       constexpr uint32_t id_o = tc5::make_idesc_bf16(128, D, 0, 1);
-      const uint64_t bVmn0 = tc5::desc_mnmajor(tc5::smem_u32(sKV) + 2 * HALF, HALF);
+      const uint64_t bVmn0 = tc5::desc_mnmajor(tc5::smem_u32(sKV) + KVT, HALF);
       bool ok = true;
       for (int u = 0; u < n_vis; ++u) {
         const int st = u % FWT_STAGES, g = u & 1;
@@ -636,11 +653,11 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                      tc5::mbar_wait(p_full + g, (u >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
         if (!ok) break;
         tc5::fence_after_sync();
-        const uint64_t bV = bVmn0 + static_cast<uint64_t>((st * 4 * HALF) >> 4);
+        const uint64_t bV = bVmn0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
         if (lead) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)          // O_g += P V
-            tc5::mma_ts(tmem + cO + g * 128, tmem + cP + g * 32 + kk * 8, bV + static_cast<uint64_t>((kk * 2048) >> 4), id_o,
+            tc5::mma_ts(tmem + cO + g * D, tmem + cP + g * 32 + kk * 8, bV + static_cast<uint64_t>((kk * 2048) >> 4), id_o,
                         (u > 1 || kk > 0) ? 1u : 0u);
           // a commit covers the MMAs of this thread; S of this visit completed before P could be written
           tc5::mma_commit(kv_empty + st);
@@ -662,18 +679,10 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     float m_ref = -INFINITY, l_sum = 0.f;
     bool ok = true;
     if (n_vis > 0) {
-      // Q: shared memory (swizzled [128 rows][64] k-blocks) -> TMEM; thread (r, grp) copies k-block grp of its row
+      // Q: shared memory (swizzled [128 rows][64] k-blocks) -> TMEM; thread (r, grp) copies half grp of its row
       ok = __all_sync(0xffffffffu, tc5::mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL));
       if (ok) {
-        uint32_t w[32];
-        const uint8_t* rowp = sQ + grp * 2 * HALF + r * 128;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const uint4 x = *reinterpret_cast<const uint4*>(rowp + ((j ^ (r & 7)) << 4));
-          w[4 * j] = x.x; w[4 * j + 1] = x.y; w[4 * j + 2] = x.z; w[4 * j + 3] = x.w;
-        }
-        tc5::tmem_st_x32(tmem + lane_off + cQ + grp * 32, w);
-        tc5::tmem_st_wait();
+        q_half_to_tmem<D>(tmem + lane_off + cQ, sQ, r, grp);
         tc5::fence_before_sync();
         tc5::mbar_arrive(qt_full);
       }
@@ -752,11 +761,11 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
         for (int q4 = 0; q4 < D / 32; ++q4) {
           uint32_t o[32];
-          tc5::tmem_ld_x32(tmem + lane_off + cO + grp * 128 + q4 * 32, o);
+          tc5::tmem_ld_x32(tmem + lane_off + cO + grp * D + q4 * 32, o);
           tc5::tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tc5::tmem_st_x32(tmem + lane_off + cO + grp * 128 + q4 * 32, o);
+          tc5::tmem_st_x32(tmem + lane_off + cO + grp * D + q4 * 32, o);
         }
         tc5::tmem_st_wait();
       }
@@ -765,7 +774,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tc5::fence_before_sync();
       tc5::mbar_arrive(p_full + grp);
     }
-    // ---- merge the two groups' partial results and write O (thread (r, grp): columns grp*64..)
+    // ---- merge the two groups' partial results and write O (thread (r, grp): half grp of the columns)
     const bool done = __all_sync(0xffffffffu, ok && n_vis > 0 &&
                                  tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
     if (done) tc5::fence_after_sync();
@@ -784,14 +793,14 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const bool have = done && l_tot > 0.f;
     const float f0 = have ? w0 / l_tot : 0.f, f1 = have ? w1 / l_tot : 0.f;
     if (row_ok && grp == 0) p.L[rowi] = have ? m + log2f(l_tot) : -INFINITY;
-    bf16* dst = p.O + rowi * D + grp * 64;
+    bf16* dst = p.O + rowi * D + grp * (D / 2);
     // every thread of a warp takes the same branches below (done, and the visit counts, are uniform)
     const bool use0 = done && n_vis > 0, use1 = done && n_vis > 1;
 #pragma unroll
-    for (int q4 = 0; q4 < 2; ++q4) {
+    for (int q4 = 0; q4 < D / 64; ++q4) {
       uint32_t a[32], c[32];
-      if (use0) tc5::tmem_ld_x32(tmem + lane_off + cO + grp * 64 + q4 * 32, a);
-      if (use1) tc5::tmem_ld_x32(tmem + lane_off + cO + 128 + grp * 64 + q4 * 32, c);
+      if (use0) tc5::tmem_ld_x32(tmem + lane_off + cO + grp * (D / 2) + q4 * 32, a);
+      if (use1) tc5::tmem_ld_x32(tmem + lane_off + cO + D + grp * (D / 2) + q4 * 32, c);
       if (use0 || use1) tc5::tmem_ld_wait();
       if (row_ok) {
         float o[32];
@@ -825,23 +834,24 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // scores, 4 K from the last to the exit) run beside the visits of the other; nothing is merged.  Half of the shared memory and of the tensor memory
 // is left to a CTA: two stages of K and of V, S and P and O in 256 columns, Q in shared memory.
 // 8192 tokens x 32 query and 2 KV heads: 599 -> 517 us, without causality 1110 -> 1072, window 512 163 -> 121; 16384 2200 -> 1960.
+// head_dim 64, 128 columns less: 4096 tokens x 16 and 8 heads, with one group per CTA there too, 192 -> 101 us; 8192 x 16 / 8, window 512, 170 -> 60.
 // (Visits of 128 keys in one CTA, P over S: 16384 2386 us, window 512 174; S then waits for P V of the visit before.)
 // --------------------------------------------------------------------------------------
 constexpr int FW1_STAGES = 2;
-constexpr int FW1_SMEM = (4 + 4 * FW1_STAGES) * HALF + 1024 + 256;
+constexpr int fw1_smem(int D) { return D / 64 * (2 + 2 * FW1_STAGES) * HALF + 1024 + 256; }
 
-template <bool LONGEST_FIRST>
+template <int D, bool LONGEST_FIRST>
 __global__ void __launch_bounds__(224, 2)
 attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
-  constexpr int D = 128;
-  constexpr int QT = 4 * HALF;
+  constexpr int KB = D / 64;                     // 64-column k-blocks of an operand
+  constexpr int QT = KB * 2 * HALF, KVT = KB * HALF;   // [128 rows][D] of Q, [64 keys][D] of K or V
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;                            // [2 k-blocks][128 rows][64]
-  uint8_t* sK = sQ + QT;                         // [stages][2 k-blocks of [64][64]]
-  uint8_t* sV = sK + FW1_STAGES * 2 * HALF;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + FW1_STAGES * 2 * HALF);
+  uint8_t* sQ = smem;                            // [KB k-blocks][128 rows][64]
+  uint8_t* sK = sQ + QT;                         // [stages][KB k-blocks of [64][64]]
+  uint8_t* sV = sK + FW1_STAGES * KVT;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + FW1_STAGES * KVT);
   uint64_t* q_full = bars;
   uint64_t* k_full = bars + 1;                   // [stages]
   uint64_t* v_full = k_full + FW1_STAGES;        // [stages]
@@ -910,7 +920,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if (lane == 0 && n_vis > 0) {
       tc5::mbar_expect_tx(q_full, QT);
 #pragma unroll
-      for (int kb = 0; kb < 2; ++kb) tc5::tma_load_5d(sQ + kb * 2 * HALF, &tm_q, q_full, kb * 64, 0, h, q0, b);
+      for (int kb = 0; kb < KB; ++kb) tc5::tma_load_5d(sQ + kb * 2 * HALF, &tm_q, q_full, kb * 64, 0, h, q0, b);
       bool ok = true;
       int blk_n = selected ? blocks[0] : 0;
       for (int v = 0; v < n_vis && ok; ++v) {
@@ -920,14 +930,14 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         if (selected && v + 1 < n_vis) blk_n = blocks[v + 1];
         ok = tc5::mbar_wait(k_empty + st, par, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY);
         if (!ok) break;
-        tc5::mbar_expect_tx(k_full + st, 2 * HALF);
+        tc5::mbar_expect_tx(k_full + st, KVT);
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) tc5::tma_load_4d(sK + (2 * st + kb) * HALF, &tm_k, k_full + st, kb * 64, h, s0, b);
+        for (int kb = 0; kb < KB; ++kb) tc5::tma_load_4d(sK + (KB * st + kb) * HALF, &tm_k, k_full + st, kb * 64, h, s0, b);
         ok = tc5::mbar_wait(v_empty + st, par, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY);
         if (!ok) break;
-        tc5::mbar_expect_tx(v_full + st, 2 * HALF);
+        tc5::mbar_expect_tx(v_full + st, KVT);
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) tc5::tma_load_4d(sV + (2 * st + kb) * HALF, &tm_v, v_full + st, kb * 64, h, s0, b);
+        for (int kb = 0; kb < KB; ++kb) tc5::tma_load_4d(sV + (KB * st + kb) * HALF, &tm_v, v_full + st, kb * 64, h, s0, b);
       }
       if (!ok)         // let the copies already issued land before the CTA's shared memory is released
         for (int i = 0; i < 1 + 2 * FW1_STAGES; ++i) tc5::mbar_drain(bars + i);
@@ -945,7 +955,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                                      tc5::mbar_wait(s_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
         if (!ok) break;
         tc5::fence_after_sync();
-        const uint64_t bK = bK0 + static_cast<uint64_t>((st * 2 * HALF) >> 4);
+        const uint64_t bK = bK0 + static_cast<uint64_t>((st * KVT) >> 4);
         if (lead) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk)
@@ -970,7 +980,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                                      tc5::mbar_wait(p_full, u & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
         if (!ok) break;
         tc5::fence_after_sync();
-        const uint64_t bV = bV0 + static_cast<uint64_t>((st * 2 * HALF) >> 4);
+        const uint64_t bV = bV0 + static_cast<uint64_t>((st * KVT) >> 4);
         if (lead) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
@@ -1091,7 +1101,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if (row_ok) p.L[rowi] = have ? m_ref + log2f(l_sum) : -INFINITY;
     bf16* dst = p.O + rowi * D;
 #pragma unroll
-    for (int q4 = 0; q4 < 4; ++q4) {
+    for (int q4 = 0; q4 < D / 32; ++q4) {
       uint32_t a[32];
       if (done) {
         tc5::tmem_ld_x32(tmem + lane_off + cO + q4 * 32, a);
@@ -1877,33 +1887,36 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // warps 9, 10 and 11 issue S = Q K^T, dP = dO V^T (double-buffered in TMEM) and dQ += dS K
 // (resident in TMEM).  Visits are 64-key blocks: the contiguous range allowed by causality / window, or the
 // entries of the tile's union list (selected mode, with the per-token bit masks).
-// Needs D = 128.  All softmax threads share a visit: dS takes the place of S, so a buffer is held until dS is consumed, and groups
+// head_dim 64 leaves room for a third S / dP buffer.  All softmax threads share a visit: dS takes the place of S, so a buffer is held until dS is consumed, and groups
 // on alternate visits (as in the forward) hold it longer than they overlap (8192 tokens x 32 heads: 819 us against 693).
 // --------------------------------------------------------------------------------------
 constexpr int DQT_STAGES = 5;
+constexpr int dqt_smem(int D) { return D / 64 * (4 + 2 * DQT_STAGES) * HALF + 1024 + 256; }
 
+template <int D>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const AttnParams p, const float scale) {
-  constexpr int D = 128;
-  constexpr int QT = 4 * HALF;
+  constexpr int KB = D / 64;                     // 64-column k-blocks of an operand
+  constexpr int QT = KB * 2 * HALF, KVT = KB * HALF;   // [128 rows][D] of Q or dO, [64 keys][D] of K or V
+  constexpr int BUFS = D == 128 ? 2 : 3;         // of S and dP: what tensor memory holds beside Q, dO and dQ
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
   uint8_t* sDO = sQ + QT;
-  uint8_t* sKV = sDO + QT;                       // [stages][K: 2 k-blocks of [64][64] | V: same]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + DQT_STAGES * 4 * HALF);
+  uint8_t* sKV = sDO + QT;                       // [stages][K: KB k-blocks of [64][64] | V: same]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + DQT_STAGES * 2 * KVT);
   uint64_t* q_full = bars;
   uint64_t* kv_full = bars + 1;                  // [stages] TMA -> MMA
   uint64_t* kv_empty = kv_full + DQT_STAGES;      // [stages] MMA -> TMA
-  uint64_t* s_full = kv_empty + DQT_STAGES;       // [2] MMA -> softmax
-  uint64_t* s_empty = s_full + 2;                // [2] softmax -> MMA
+  uint64_t* s_full = kv_empty + DQT_STAGES;       // [BUFS] MMA -> softmax
+  uint64_t* s_empty = s_full + BUFS;             // [BUFS] softmax -> MMA
   // One dS barrier per S buffer: warps whose rows are all masked finish a visit early and may
   // already be in the next visit (other buffer); with a single barrier their second arrival
   // would complete the phase of the visit the slower warps are still writing.
-  uint64_t* ds_full = s_empty + 2;               // [2] softmax -> MMA
-  uint64_t* qt_full = ds_full + 2;               // softmax -> MMA: Q and dO are in tensor memory
+  uint64_t* ds_full = s_empty + BUFS;            // [BUFS] softmax -> MMA
+  uint64_t* qt_full = ds_full + BUFS;            // softmax -> MMA: Q and dO are in tensor memory
   uint64_t* acc_done = qt_full + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -1945,9 +1958,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     *abort_flag = 0;
     tc5::mbar_init(q_full, 1);
     for (int i = 0; i < DQT_STAGES; ++i) { tc5::mbar_init(kv_full + i, 1); tc5::mbar_init(kv_empty + i, 1); }
-    for (int i = 0; i < 2; ++i) { tc5::mbar_init(s_full + i, 2); tc5::mbar_init(s_empty + i, 1); }
-    tc5::mbar_init(ds_full, 256);
-    tc5::mbar_init(ds_full + 1, 256);
+    for (int i = 0; i < BUFS; ++i) { tc5::mbar_init(s_full + i, 2); tc5::mbar_init(s_empty + i, 1); tc5::mbar_init(ds_full + i, 256); }
     tc5::mbar_init(qt_full, 256);
     tc5::mbar_init(acc_done, 1);
     tc5::fence_barrier_init();
@@ -1957,14 +1968,14 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  constexpr uint32_t cDQ = 256, cQ = 384, cDO = 448;   // S/dP of buffer i at i*128 + {0, 64}
+  constexpr uint32_t cDQ = BUFS * 128, cQ = cDQ + D, cDO = cQ + D / 2;   // S/dP of buffer i at i*128 + {0, 64}
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0 && n_vis > 0) {
       tc5::mbar_expect_tx(q_full, 2 * QT);
 #pragma unroll
-      for (int kb = 0; kb < 2; ++kb) {
+      for (int kb = 0; kb < KB; ++kb) {
         tc5::tma_load_5d(sQ + kb * 2 * HALF, &tm_q, q_full, kb * 64, 0, h, q0, b);
         tc5::tma_load_5d(sDO + kb * 2 * HALF, &tm_do, q_full, kb * 64, 0, h, q0, b);
       }
@@ -1979,12 +1990,12 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         int s0;
         if (!selected) s0 = (kb0 + v) * 64;
         else s0 = blk < 0 ? 0 : blk * 64;
-        uint8_t* kd = sKV + st * 4 * HALF;
-        tc5::mbar_expect_tx(kv_full + st, 4 * HALF);
+        uint8_t* kd = sKV + st * 2 * KVT;
+        tc5::mbar_expect_tx(kv_full + st, 2 * KVT);
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
+        for (int kb = 0; kb < KB; ++kb) {
           tc5::tma_load_4d(kd + kb * HALF, &tm_k, kv_full + st, kb * 64, h, s0, b);
-          tc5::tma_load_4d(kd + 2 * HALF + kb * HALF, &tm_v, kv_full + st, kb * 64, h, s0, b);
+          tc5::tma_load_4d(kd + KVT + kb * HALF, &tm_v, kv_full + st, kb * 64, h, s0, b);
         }
         issued = v + 1;
       }
@@ -2014,17 +2025,17 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const bool lead = tc5::elect_one();
       const bool is_dp = warp == 10;
       constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 64, 0, 0);
-      const uint64_t b0 = tc5::desc_kmajor(tc5::smem_u32(sKV) + (is_dp ? 2 * HALF : 0));   // stage 0, K or V, k-step 0
+      const uint64_t b0 = tc5::desc_kmajor(tc5::smem_u32(sKV) + (is_dp ? KVT : 0));   // stage 0, K or V, k-step 0
       const uint32_t acol = is_dp ? cDO : cQ, dcol = is_dp ? 64u : 0u;
       bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(qt_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
       if (ok) tc5::fence_after_sync();
       for (int v = 0; v < n_vis && ok; ++v) {
-        const int st = v % DQT_STAGES, buf = v & 1;
+        const int st = v % DQT_STAGES, buf = v % BUFS;
         ok = __all_sync(0xffffffffu, tc5::mbar_wait(kv_full + st, (v / DQT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(s_empty + buf, ((v >> 1) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
+                                     tc5::mbar_wait(s_empty + buf, ((v / BUFS) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
         if (!ok) break;
         tc5::fence_after_sync();
-        const uint64_t bB = b0 + static_cast<uint64_t>((st * 4 * HALF) >> 4);
+        const uint64_t bB = b0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
         if (lead) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk)      // a k-step of 16 bf16 is 8 TMEM columns of the A operand
@@ -2043,12 +2054,12 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const uint64_t bKmn0 = tc5::desc_mnmajor(tc5::smem_u32(sKV), HALF);    // the K tile as an MN-major operand
       bool ok = true;
       for (int u = 0; u < n_vis; ++u) {
-        const int st = u % DQT_STAGES, buf = u & 1;
+        const int st = u % DQT_STAGES, buf = u % BUFS;
         ok = __all_sync(0xffffffffu, tc5::mbar_wait(kv_full + st, (u / DQT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(ds_full + buf, (u >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+                                     tc5::mbar_wait(ds_full + buf, (u / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
         if (!ok) break;
         tc5::fence_after_sync();
-        const uint64_t bKmn = bKmn0 + static_cast<uint64_t>((st * 4 * HALF) >> 4);
+        const uint64_t bKmn = bKmn0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
         if (lead) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)          // dQ += dS K: keys 0-31 sit in columns 0-15, keys 32-63 in columns 32-47
@@ -2078,22 +2089,11 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const float sc = p.scale_log2;
     bool ok = true;
     if (n_vis > 0) {
-      // Q and dO: shared memory (swizzled [128 rows][64] k-blocks) -> TMEM, thread (r, ch) copies the
-      // 64 elements of k-block ch of its row as 32 packed words
+      // Q and dO: shared memory (swizzled [128 rows][64] k-blocks) -> TMEM, thread (r, ch) copies half ch of its row
       ok = __all_sync(0xffffffffu, tc5::mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL));
       if (ok) {
-        uint32_t w[32];
-#pragma unroll
-        for (int which = 0; which < 2; ++which) {
-          const uint8_t* rowp = (which ? sDO : sQ) + ch * 2 * HALF + r * 128;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint4 x = *reinterpret_cast<const uint4*>(rowp + ((j ^ (r & 7)) << 4));
-            w[4 * j] = x.x; w[4 * j + 1] = x.y; w[4 * j + 2] = x.z; w[4 * j + 3] = x.w;
-          }
-          tc5::tmem_st_x32(tmem + lane_off + (which ? cDO : cQ) + ch * 32, w);
-          tc5::tmem_st_wait();                     // before the registers are reused for the second operand
-        }
+        q_half_to_tmem<D>(tmem + lane_off + cQ, sQ, r, ch);
+        q_half_to_tmem<D>(tmem + lane_off + cDO, sDO, r, ch);
         tc5::fence_before_sync();
         tc5::mbar_arrive(qt_full);
       }
@@ -2103,7 +2103,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     int blk_n = (selected && n_vis > 0) ? blocks[0] : 0;
     unsigned long long msk_n = (selected && n_vis > 0) ? masks[0] : 0ull;
     for (int v = 0; v < n_vis && ok; ++v) {
-      const int buf = v & 1;
+      const int buf = v % BUFS;
       int sb;
       bool row_sel = row_ok;
       if (!selected) sb = (kb0 + v) * 64 + ch * 32;
@@ -2114,7 +2114,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         sb = blk < 0 ? -1 : blk * 64 + ch * 32;
         row_sel = row_ok && blk >= 0 && ((msk >> (tok_local & 63)) & 1ull);
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + buf, (v >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + buf, (v / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
         ok = false;
         break;
       }
@@ -2146,20 +2146,20 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tc5::mbar_arrive(ds_full + buf);
     }
     // what dQ is added to, fetched behind the last products (16384 tokens x 32 heads, three branches: 2129 -> 2065 us)
-    uint4 old[8];
+    uint4 old[D / 16];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      old[i] = p.add_dq && row_ok ? reinterpret_cast<const uint4*>(p.dQb + rowi * D + ch * 64)[i] : make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 0; i < D / 16; ++i)
+      old[i] = p.add_dq && row_ok ? reinterpret_cast<const uint4*>(p.dQb + rowi * D + ch * (D / 2))[i] : make_uint4(0u, 0u, 0u, 0u);
     // ---- dQ: thread (r, ch) stores D-half ch of row r
     const bool have = __all_sync(0xffffffffu, ok && n_vis > 0 &&
                                  tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
     if (have) tc5::fence_after_sync();
-    bf16* dst = p.dQb + rowi * D + ch * 64;
+    bf16* dst = p.dQb + rowi * D + ch * (D / 2);
 #pragma unroll
-    for (int q4 = 0; q4 < 2; ++q4) {
+    for (int q4 = 0; q4 < D / 64; ++q4) {
       uint32_t a[32];
       if (have) {
-        tc5::tmem_ld_x32(tmem + lane_off + cDQ + ch * 64 + q4 * 32, a);
+        tc5::tmem_ld_x32(tmem + lane_off + cDQ + ch * (D / 2) + q4 * 32, a);
         tc5::tmem_ld_wait();
       } else {
 #pragma unroll
@@ -2462,6 +2462,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // (64 keys a CTA and P, dS through shared memory: every product had 64 columns, which costs the tensor pipe as much as 128 when
 // both operands come from shared memory.  8192 tokens x 32 query and 2 KV heads: 1390 us; now 884.  A visit is 3100 cycles here:
 // exponentials 1200, dV and S 1100, the rest signals between them.  S for half tiles costs its products twice, 3250.)
+// head_dim 64 leaves room for two S^T, so S(v+1) is issued in front of dV(v) and the exponentials of v+1 wait for dS(v) alone.  With the dQ
+// kernel, 4096 tokens x 16 and 8 heads: 722 us where one kernel did both with reductions to memory for each tile, now 272.
 // Roles: warps 0-7 softmax (key lane, 64 query rows each), warp 8 TMA producer, warp 9 MMA issuer, warp 10 row statistics.
 // --------------------------------------------------------------------------------------
 struct KeyWalks {
@@ -2481,11 +2483,13 @@ __device__ __forceinline__ int key_walk(const AttnParams& p, int visits, int s0,
   v0 = max(qt_lo, y * visits);                 // long ranges: absolute chunks, the same Q/dO range for every key block
   return min(n_qt, (y + 1) * visits) - v0;
 }
-// dV, dK += the walks' sums, in order.  A warp owns a (key, head) row of D = 128.
+// dV, dK += the walks' sums, in order.  D / 4 lanes own a (key, head) row.
+template <int D>
 __global__ void __launch_bounds__(256) attn_sum_walks_kernel(const AttnParams p, const KeyWalks w, const long rows) {
-  const long row = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  constexpr int LANES = D / 4;
+  const long row = static_cast<long>(blockIdx.x) * (256 / LANES) + threadIdx.x / LANES;
   if (row >= rows) return;
-  const long i = row * 32 + (threadIdx.x & 31), n = rows * 32;               // in float4
+  const long i = row * LANES + threadIdx.x % LANES, n = rows * LANES;        // in float4
   const int s0 = static_cast<int>(row / p.Hkv % p.S) & ~127;
   float4* out = reinterpret_cast<float4*>(blockIdx.y ? p.dK : p.dV) + i;
   const float4* part = reinterpret_cast<const float4*>(w.part) + blockIdx.y * n + i;
@@ -2501,14 +2505,16 @@ __global__ void __launch_bounds__(256) attn_sum_walks_kernel(const AttnParams p,
 }
 
 constexpr int KVC_THREADS = 352;
-constexpr int KVC_SMEM = 28 * HALF + 2 * 2 * 128 * 4 + 256;
+constexpr int kvc_smem(int D) { return D / 64 * 14 * HALF + 2 * 2 * 128 * 4 + 256; }
 
+template <int D>
 __global__ void __launch_bounds__(KVC_THREADS, 1)
 attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                          const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                          const AttnParams p, const KeyWalks w, const float scale) {
-  constexpr int D = 128, KEYS = 128;
-  constexpr int TILE = 4 * HALF;                 // [128 rows][128] bf16: two 64-column k-blocks
+  constexpr int KEYS = 128, KB = D / 64;         // KB: 64-column k-blocks of an operand
+  constexpr int TILE = KB * 2 * HALF;            // [128 rows][D] bf16
+  constexpr int BUFS = D == 128 ? 1 : 2;         // of S^T: what tensor memory holds beside dP^T, dV and dK
   constexpr int ROW = D * 4 + 16;                // bytes from one key's sums to the next on their way out
   static_assert(2 * KEYS * ROW <= 5 * TILE, "attention: dK and dV on their way out");
   extern __shared__ __align__(1024) uint8_t smem_kvc[];
@@ -2522,9 +2528,10 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   uint64_t *q_full = bars + 2, *q_empty = bars + 5;              // [3]
   uint64_t *do_full = bars + 8, *do_empty = bars + 10;           // [2]
   uint64_t *st_full = bars + 12, *st_empty = bars + 14;          // [2]
-  uint64_t *s_full = bars + 16, *dp_full = bars + 17, *ds_full = bars + 18;
-  uint64_t* p_full = bars + 19;                                  // [2]: the first and last 32 of each thread's 64 rows
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
+  uint64_t *dp_full = bars + 16, *ds_full = bars + 17;
+  uint64_t* s_full = bars + 18;                                  // [BUFS]
+  uint64_t* p_full = s_full + BUFS;                              // [BUFS][2]: the first and last 32 of each thread's 64 rows
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_full + 2 * BUFS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -2541,11 +2548,9 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   if (tid == 0) {
     *abort_flag = 0;
     for (int i = 0; i < 14; ++i) tc5::mbar_init(bars + i, 1);
-    for (int i = 0; i < 2; ++i) {
-      tc5::mbar_init(st_empty + i, 8);
-      tc5::mbar_init(p_full + i, 8);
-    }
-    tc5::mbar_init(s_full, 1);
+    for (int i = 0; i < 2; ++i) tc5::mbar_init(st_empty + i, 8);
+    for (int i = 0; i < BUFS; ++i) tc5::mbar_init(s_full + i, 1);
+    for (int i = 0; i < 2 * BUFS; ++i) tc5::mbar_init(p_full + i, 8);
     tc5::mbar_init(dp_full, 1);
     tc5::mbar_init(ds_full, 8);
     tc5::fence_barrier_init();
@@ -2555,7 +2560,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  constexpr uint32_t cS = 0, cDP = 128, cDV = 256, cDK = 384;
+  constexpr uint32_t cS = 0, cDP = BUFS * 128, cDV = cDP + 128, cDK = cDV + D;   // S^T of buffer i at i * 128
   auto wait = [&](uint64_t* bar, int phase, int code) {
     return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
   };
@@ -2566,7 +2571,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     if (lead) {
       tc5::mbar_expect_tx(kv_full, 2 * TILE);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {              // k-block i / 2, 64 keys; keys past the end read zero
+      for (int i = 0; i < 2 * KB; ++i) {         // k-block i / 2, 64 keys; keys past the end read zero
         tc5::tma_load_4d(sK + i * HALF, &tm_k, kv_full, (i >> 1) * 64, h, s0 + (i & 1) * 64, b);
         tc5::tma_load_4d(sV + i * HALF, &tm_v, kv_full, (i >> 1) * 64, h, s0 + (i & 1) * 64, b);
       }
@@ -2577,15 +2582,15 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       if (v >= 3 && !(ok = wait(q_empty + qb, v / 3 - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
       if (lead) {
         tc5::mbar_expect_tx(q_full + qb, TILE);
-        tc5::tma_load_5d(sQ + qb * TILE, &tm_q, q_full + qb, 0, 0, h, q0, b);
-        tc5::tma_load_5d(sQ + qb * TILE + 2 * HALF, &tm_q, q_full + qb, 64, 0, h, q0, b);
+#pragma unroll
+        for (int i = 0; i < KB; ++i) tc5::tma_load_5d(sQ + qb * TILE + i * 2 * HALF, &tm_q, q_full + qb, i * 64, 0, h, q0, b);
       }
       __syncwarp();
       if (v >= 2 && !(ok = wait(do_empty + ob, (v >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
       if (lead) {
         tc5::mbar_expect_tx(do_full + ob, TILE);
-        tc5::tma_load_5d(sDO + ob * TILE, &tm_do, do_full + ob, 0, 0, h, q0, b);
-        tc5::tma_load_5d(sDO + ob * TILE + 2 * HALF, &tm_do, do_full + ob, 64, 0, h, q0, b);
+#pragma unroll
+        for (int i = 0; i < KB; ++i) tc5::tma_load_5d(sDO + ob * TILE + i * 2 * HALF, &tm_do, do_full + ob, i * 64, 0, h, q0, b);
       }
       __syncwarp();
     }
@@ -2599,7 +2604,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer (converged warp, elected lane issues)
     const bool lead = tc5::elect_one();
-    constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0), id_t = tc5::make_idesc_bf16(128, 128, 0, 1);
+    constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0), id_t = tc5::make_idesc_bf16(128, D, 0, 1);
     const uint64_t aK = tc5::desc_kmajor(tc5::smem_u32(sK)), aV = tc5::desc_kmajor(tc5::smem_u32(sV));
     const uint64_t bQ0 = tc5::desc_kmajor(tc5::smem_u32(sQ)), bDO0 = tc5::desc_kmajor(tc5::smem_u32(sDO));
     const uint64_t tQ0 = tc5::desc_mnmajor(tc5::smem_u32(sQ), 2 * HALF), tDO0 = tc5::desc_mnmajor(tc5::smem_u32(sDO), 2 * HALF);
@@ -2611,8 +2616,8 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       if (lead) {
         const uint64_t bQ = bQ0 + at(v % 3);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) tc5::mma_ss(tmem + cS, aK + kblock(kk), bQ + kblock(kk), id_s, kk > 0 ? 1u : 0u);
-        tc5::mma_commit(s_full);
+        for (int kk = 0; kk < D / 16; ++kk) tc5::mma_ss(tmem + cS + (v % BUFS) * 128, aK + kblock(kk), bQ + kblock(kk), id_s, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(s_full + v % BUFS);
       }
       __syncwarp();
       return true;
@@ -2633,9 +2638,10 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     auto rows16 = [](int kk) { return static_cast<uint32_t>((kk >> 2) * 64 + (kk & 3) * 8); };
     bool ok = wait(kv_full, 0, STATUS_TIMEOUT_SMEM_FULL) && scores(0) && grads(0);
     for (int v = 0; v < n_vis && ok; ++v) {
+      if (BUFS > 1 && v + 1 < n_vis && !(ok = scores(v + 1))) break;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        if (ok) ok = wait(p_full + half, v, STATUS_TIMEOUT_TMEM_EMPTY);
+        if (ok) ok = wait(p_full + v % BUFS * 2 + half, v / BUFS, STATUS_TIMEOUT_TMEM_EMPTY);
         if (!ok) break;
         tc5::fence_after_sync();
         if (lead) {
@@ -2643,14 +2649,14 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 #pragma unroll
           for (int i = 0; i < 4; ++i) {          // dV += P^T dO; rows 32 half .. of both threads' 64
             const int kk = (i >> 1) * 4 + half * 2 + (i & 1);
-            tc5::mma_ts(tmem + cDV, tmem + cS + rows16(kk), tDO + static_cast<uint64_t>((kk * 2048) >> 4), id_t,
+            tc5::mma_ts(tmem + cDV, tmem + cS + (v % BUFS) * 128 + rows16(kk), tDO + static_cast<uint64_t>((kk * 2048) >> 4), id_t,
                         (v > 0 || half > 0 || i > 0) ? 1u : 0u);
           }
           if (half) tc5::mma_commit(do_empty + (v & 1));
         }
         __syncwarp();
       }
-      if (!ok || (v + 1 < n_vis && !(ok = scores(v + 1)))) break;
+      if (!ok || (BUFS == 1 && v + 1 < n_vis && !(ok = scores(v + 1)))) break;
       if (!(ok = wait(ds_full, v, STATUS_TIMEOUT_TMEM_EMPTY))) break;
       tc5::fence_after_sync();
       if (lead) {
@@ -2690,7 +2696,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   } else {
     // ------------------------------------------------------------------ softmax warps: key lane, query rows 64 ch ..
     const int ch = warp >> 2, key = s0 + (warp & 3) * 32 + lane;
-    const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + ch * 64;
+    const uint32_t lane_row = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16), lanes = lane_row + ch * 64;
     const float sc = p.scale_log2;
     const int kpos = key * p.kp_stride + p.kp_off;
     const int w_lo = s0 + (warp & 3) * 32, w_hi = w_lo + 31;     // keys of this warp
@@ -2709,13 +2715,13 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         hi = min(hi, max(0, min(64, (p.T - t0) * p.G - ch * 64)));
         if (key >= p.S) hi = 0;
       }
-      if (!(ok = wait(st_full + (v & 1), v >> 1, STATUS_TIMEOUT_SMEM_FULL) && wait(s_full, v, STATUS_TIMEOUT_TMEM_FULL))) break;
+      if (!(ok = wait(st_full + (v & 1), v >> 1, STATUS_TIMEOUT_SMEM_FULL) && wait(s_full + v % BUFS, v / BUFS, STATUS_TIMEOUT_TMEM_FULL))) break;
       tc5::fence_after_sync();
       float pr[64];
       {
         uint32_t a[32], c[32];
-        tc5::tmem_ld_x32(lanes + cS, a);
-        tc5::tmem_ld_x32(lanes + cS + 32, c);
+        tc5::tmem_ld_x32(lanes + cS + (v % BUFS) * 128, a);
+        tc5::tmem_ld_x32(lanes + cS + (v % BUFS) * 128 + 32, c);
         tc5::tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
@@ -2742,10 +2748,10 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
           pk[j / 2] = tc5::pack_bf16(pr[i], pr[i + 1]);
           pk[j / 2 + 1] = tc5::pack_bf16(pr[i + 2], pr[i + 3]);
         }
-        tc5::tmem_st_x16(lanes + cS + q * 16, pk);
+        tc5::tmem_st_x16(lanes + cS + (v % BUFS) * 128 + q * 16, pk);
         tc5::tmem_st_wait();
         tc5::fence_before_sync();
-        tc5::arrive_warp(p_full + q);
+        tc5::arrive_warp(p_full + v % BUFS * 2 + q);
       }
       if (!(ok = wait(dp_full, v, STATUS_TIMEOUT_TMEM_FULL))) break;
       tc5::fence_after_sync();
@@ -2772,18 +2778,19 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         tc5::mbar_arrive(st_empty + (v & 1));
       }
     }
-    // ---- accumulators -> global.  A thread holds half a key's row; rows go through shared memory (free now, pitch spread over
+    // ---- accumulators -> global.  A thread holds half a key's row (D / 64 loads of 32 columns each for dV and dK); rows go through shared memory (free now, pitch spread over
     //      the banks) and are added to global memory by one bulk reduction each: scattered 16-byte reductions were most of a CTA's
     //      fixed cost of 14 us.
     const bool have = ok && wait(acc_done, 0, STATUS_TIMEOUT_TMEM_FULL);
     if (have) {
       tc5::fence_after_sync();
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < 2 * KB; ++q) {
         uint32_t a[32];
-        tc5::tmem_ld_x32(lanes + (q < 2 ? cDV : cDK) + (q & 1) * 32, a);
+        const int c = ch * (D / 2) + (q % KB) * 32;
+        tc5::tmem_ld_x32(lane_row + (q < KB ? cDV : cDK) + c, a);
         tc5::tmem_ld_wait();
-        float4* dst = reinterpret_cast<float4*>(sQ + (q < 2 ? 0 : KEYS * ROW) + (tid & 127) * ROW + (ch * 64 + (q & 1) * 32) * 4);
+        float4* dst = reinterpret_cast<float4*>(sQ + (q < KB ? 0 : KEYS * ROW) + (tid & 127) * ROW + c * 4);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           dst[i] = make_float4(__uint_as_float(a[4 * i]), __uint_as_float(a[4 * i + 1]), __uint_as_float(a[4 * i + 2]),
@@ -3454,9 +3461,12 @@ void fill_params(AttnParams& p, int B, int T, int S, int Hq, int Hkv, int D, flo
 // A selected block counts as the keys of a sequence do: how many blocks the tokens of a tile share is not known here.
 // Compressed keys always take two groups: their L goes into the choice of blocks, where a last bit decides between near ties (with one
 // group, compressed and selected branch together 1159 us at 16384 tokens, 1298 with two, a few rows took another block than before).
+// head_dim 64 has shorter visits, and their start and end weigh more (two groups, one group): 152 CTAs x 5 visits 10.0 us, 8.8; 250 x 9
+// 17.8, 16.9; 250 x 16 18.1, 20.3; 500 x 16 34, 32; 500 x 32 50, 53 and 50, 41; 512 x 64 86, 97 and 85, 77; 1000 x 32 95, 87; 1024 x 128 299, 302 and 291, 253.
 static bool fwd_two_per_sm(const AttnParams& p, long ctas) {
   if (p.kp_stride > 1) return false;
   const int visits = (std::min(p.S, p.window > 0 ? p.window + p.R : p.S) + 63) / 64;
+  if (p.D == 64) return ctas > nsa::sm_count() * (visits <= 10 ? 1l : visits <= 16 ? 2l : 6l);
   return ctas >= nsa::sm_count() * (visits <= 16 ? 2l : p.G >= 4 ? 4l : 8l);
 }
 
@@ -3477,19 +3487,21 @@ extern "C" int nsa_attn_fwd(const void* q, const void* k, const void* v, void* o
   const int smem = (D / 64) * 2 * HALF * 5 + 4 * HALF + 1024 + 2048;
   static const bool legacy = [] { const char* e = getenv("NSA_B200_ATTN_FWD"); return e && !strcmp(e, "legacy"); }();
   static const bool smem_operands = [] { const char* e = getenv("NSA_B200_ATTN_FWD"); return e && !strcmp(e, "smem"); }();
-  if (D == 128 && !legacy && !smem_operands && fwd_two_per_sm(p, static_cast<long>(grid.x) * Hkv * B)) {
-    auto* kernel = longest_first(p) ? attn_fwd_half_kernel<true> : attn_fwd_half_kernel<false>;
-    static bool cfg[2] = {};
-    bool& ready = cfg[longest_first(p)];
-    if (!ready) { if ((rc = set_smem(kernel, FW1_SMEM))) return rc; ready = true; }
-    kernel<<<grid, 224, FW1_SMEM, st>>>(tq, tk, tv, p);
-  } else if (D == 128 && !legacy && !smem_operands) {
-    const int smem_ts = (4 + 4 * FWT_STAGES) * HALF + 1024 + 1024 + 256;
-    auto* kernel = longest_first(p) ? attn_fwd_ts_kernel<true> : attn_fwd_ts_kernel<false>;
-    static bool cfg[2] = {};
-    bool& ready = cfg[longest_first(p)];
-    if (!ready) { if ((rc = set_smem(kernel, smem_ts))) return rc; ready = true; }
-    kernel<<<grid, 352, smem_ts, st>>>(tq, tk, tv, p);
+  const bool wide = D == 128;
+  if ((wide || kp_stride == 1) && !legacy && !smem_operands && fwd_two_per_sm(p, static_cast<long>(grid.x) * Hkv * B)) {
+    const int bytes = fw1_smem(D), form = wide * 2 + longest_first(p);
+    void (*const kernels[4])(CUtensorMap, CUtensorMap, CUtensorMap, AttnParams) = {
+        attn_fwd_half_kernel<64, false>, attn_fwd_half_kernel<64, true>, attn_fwd_half_kernel<128, false>, attn_fwd_half_kernel<128, true>};
+    static bool cfg[4] = {};
+    if (!cfg[form]) { if ((rc = set_smem(kernels[form], bytes))) return rc; cfg[form] = true; }
+    kernels[form]<<<grid, 224, bytes, st>>>(tq, tk, tv, p);
+  } else if ((wide || kp_stride == 1) && !legacy && !smem_operands) {
+    const int bytes = fwt_smem(D), form = wide * 2 + longest_first(p);
+    void (*const kernels[4])(CUtensorMap, CUtensorMap, CUtensorMap, AttnParams) = {
+        attn_fwd_ts_kernel<64, false>, attn_fwd_ts_kernel<64, true>, attn_fwd_ts_kernel<128, false>, attn_fwd_ts_kernel<128, true>};
+    static bool cfg[4] = {};
+    if (!cfg[form]) { if ((rc = set_smem(kernels[form], bytes))) return rc; cfg[form] = true; }
+    kernels[form]<<<grid, 352, bytes, st>>>(tq, tk, tv, p);
   } else if (D == 128 && !legacy) {
     const int smem_ws = (4 + 4 * FW_STAGES + 4) * HALF + 1024 + 1024 + 256;
     static bool cfg = false;
@@ -3612,13 +3624,14 @@ struct KeyCost {
 // groups of 1 to 32 and windows, each in both forms and with up to 64 walks; the choice is 0.3 % behind the best in the mean and 16 % at
 // worst.  us with 64 keys, and with 128 and 1 / 2 / 4 / 8 / 16 walks (queries / KV heads, windows w): 300 16/8 12.9, 17.1 16.7 15.1;
 // 1000 32/8 w64 13.2, 20.4 22.9 29.7; 1000 32/2 181, 210 116 69 45 33; 2000 32/8 w512 66, 47 66 72 96; 3000 16/16 141, 114 145 165 215 282.
-extern "C" int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride) {
+static int choose_walks(int D, int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride) {
   if (B <= 0 || T <= 0 || S <= 0 || Hkv <= 0 || Hq < Hkv) return 0;
   const int R = std::max(1, BM / (Hq / Hkv));
   const long heads = static_cast<long>(B) * Hkv, sms = nsa::sm_count();
   const KeyRange wide(T, S, R, causal, window, kp_stride, 128), narrow(T, S, R, causal, window, kp_stride, 64);
   if (wide.most > 256) return 0;
-  constexpr KeyCost by_128{8.3, 1.79, 10.1, 1.6, 1.26, 8.2}, by_64{6.2, 1.43, 7.2, 1.06, 1.16, 5.1};
+  const KeyCost by_128 = D == 128 ? KeyCost{8.3, 1.79, 10.1, 1.6, 1.26, 8.2} : KeyCost{7., 1.3, 8., 1.2, 1., 7.};
+  constexpr KeyCost by_64{6.2, 1.43, 7.2, 1.06, 1.16, 5.1};
   long total = 0;
   int longest = 0;
   for (int i = 0; i < narrow.blocks; ++i) {
@@ -3626,8 +3639,8 @@ extern "C" int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int caus
     total += n;
     longest = std::max(longest, n);
   }
-  int best = -1;
-  double least = by_64.us(heads * narrow.blocks, heads * total, longest);
+  int best = D == 128 ? -1 : 1;
+  double least = D == 128 ? by_64.us(heads * narrow.blocks, heads * total, longest) : 1e30;
   for (int visits = wide.most; visits > 0; --visits) {
     const int walks = (wide.most + visits - 1) / visits;
     if (walks > 1 && (walks - 1) * wide.blocks * heads > 3 * sms) break;     // bounds the room for sums: 128 KB for each walk of a block
@@ -3647,6 +3660,12 @@ extern "C" int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int caus
     if (us < least) { least = us; best = walks; }
   }
   return best;
+}
+extern "C" int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride) {
+  return choose_walks(128, B, T, S, Hq, Hkv, causal, window, kp_stride);
+}
+extern "C" int nsa_attn_bwd_walks_d64(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride) {
+  return choose_walks(64, B, T, S, Hq, Hkv, causal, window, kp_stride);
 }
 
 // Backward in two kernels without per-tile global reductions: dQ from the query-tile-outer
@@ -3668,7 +3687,7 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
   int rc = check_shape(Hq, Hkv, D, tile_blocks);
   if (rc) return rc;
   const int G = Hq / Hkv;
-  if (D != 128) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: head_dim must be 128");
+  if (D != 128 && (tile_blocks || walks < 0)) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: selected blocks and 64 keys a CTA need head_dim 128");
   if (tile_blocks && (G < 8 || tok_list == nullptr))
     return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: selected mode needs a GQA group of at least 8 and the inverse map");
   if (visits_per_cta <= 0) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: visits_per_cta must be positive");
@@ -3685,11 +3704,12 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
   {
     const dim3 grid((T + p.R - 1) / p.R, Hkv, B);
     static const bool smem_operands = [] { const char* e = getenv("NSA_B200_ATTN_DQ"); return e && !strcmp(e, "smem"); }();
-    if (!smem_operands) {
-      const int smem = (8 + 4 * DQT_STAGES) * HALF + 1024 + 256;
-      static bool cfg = false;
-      if (!cfg) { if ((rc = set_smem(attn_bwd_dq_ts_kernel, smem))) return rc; cfg = true; }
-      attn_bwd_dq_ts_kernel<<<grid, 384, smem, st>>>(tq, tdo, tk, tv, p, scale);
+    if (!smem_operands || D == 64) {
+      auto* kernel = D == 128 ? attn_bwd_dq_ts_kernel<128> : attn_bwd_dq_ts_kernel<64>;
+      static bool cfg[2] = {};
+      bool& ready = cfg[D == 128];
+      if (!ready) { if ((rc = set_smem(kernel, dqt_smem(D)))) return rc; ready = true; }
+      kernel<<<grid, 384, dqt_smem(D), st>>>(tq, tdo, tk, tv, p, scale);
     } else {
       const int smem = (8 + 4 * DQ_STAGES + 2) * HALF + 1024 + 256;
       static bool cfg = false;
@@ -3720,12 +3740,16 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
     if (walks > 1 && part == nullptr) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: several walks need room for their sums");
     w.walks = walks > 0 ? walks : (most + visits_per_cta - 1) / visits_per_cta;
     w.visits = (most + w.walks - 1) / w.walks;
-    static bool cfg = false;
-    if (!cfg) { if ((rc = set_smem(attn_bwd_kv_range_kernel, KVC_SMEM))) return rc; cfg = true; }
-    attn_bwd_kv_range_kernel<<<dim3((S + 127) / 128, w.walks, B * Hkv), KVC_THREADS, KVC_SMEM, st>>>(tq, tdo, tk, tv, p, w, scale);
+    auto* kernel = D == 128 ? attn_bwd_kv_range_kernel<128> : attn_bwd_kv_range_kernel<64>;
+    static bool cfg[2] = {};
+    bool& ready = cfg[D == 128];
+    if (!ready) { if ((rc = set_smem(kernel, kvc_smem(D)))) return rc; ready = true; }
+    kernel<<<dim3((S + 127) / 128, w.walks, B * Hkv), KVC_THREADS, kvc_smem(D), st>>>(tq, tdo, tk, tv, p, w, scale);
     if (w.part) {
-      const long rows = static_cast<long>(B) * S * Hkv;
-      attn_sum_walks_kernel<<<dim3((unsigned)((rows + 7) / 8), 2), 256, 0, st>>>(p, w, rows);
+      const long rows = static_cast<long>(B) * S * Hkv, per_cta = 256 / (D / 4);
+      const dim3 grid((unsigned)((rows + per_cta - 1) / per_cta), 2);
+      if (D == 128) attn_sum_walks_kernel<128><<<grid, 256, 0, st>>>(p, w, rows);
+      else attn_sum_walks_kernel<64><<<grid, 256, 0, st>>>(p, w, rows);
       nsa::count_launch();
     }
   }

@@ -85,7 +85,8 @@ int nsa_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
     delta, void* dq, float* dk, float* dv, int B, int T, int S, int Hq, int Hkv, int D, float scale, int causal, int
     window, int kp_stride, int kp_off, const int* tile_blocks, const unsigned long long* tile_masks, const int*
     tile_counts, int max_u, cudaStream_t st);
-int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride);
+int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride);      // head_dim 128
+int nsa_attn_bwd_walks_d64(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride);  // head_dim 64
 int nsa_attn_bwd_split(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* L,
     float* delta, void* dq, float* dk, float* dv, int B, int T, int S, int Hq, int Hkv, int D, float scale, int causal,
     int window, int kp_stride, int kp_off, const int* tile_blocks, const unsigned long long* tile_masks, const int*

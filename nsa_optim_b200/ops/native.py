@@ -1045,7 +1045,8 @@ def _attn_backward_split(q, k, v, o, do, L, dq, dk, dv, causal, window, scale, k
     inv = (None, None, None, 0, 0)
     visits, walks, part = _kv_visits(), 0, None
     if tiles is None:
-        walks = load().nsa_attn_bwd_walks(B, T, S, Hq, Hkv, int(causal), window, kp_stride)
+        walks_of = load().nsa_attn_bwd_walks if D == 128 else load().nsa_attn_bwd_walks_d64
+        walks = walks_of(B, T, S, Hq, Hkv, int(causal), window, kp_stride)
         if walks > 1:
             part = _empty(walks, 2, k.numel(), dtype=torch.float32, device=q.device)
     else:
@@ -1066,7 +1067,7 @@ def _kv_visits() -> int:
 
 
 def _bwd_is_split(D: int, G: int, selected: bool) -> bool:
-    return D == 128 and os.environ.get("NSA_B200_ATTN_BWD", "split") == "split" and (not selected or G >= 8)
+    return os.environ.get("NSA_B200_ATTN_BWD", "split") == "split" and (not selected or (D == 128 and G >= 8))
 
 
 class _Attn(torch.autograd.Function):

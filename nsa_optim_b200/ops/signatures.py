@@ -21,6 +21,7 @@ SIGNATURES = {
     "nsa_attn_bwd": "ippppppppppiiiiiifiiiipppip",
     "nsa_attn_bwd_split": "ippppppppppiiiiiifiiiipppipppiiipiiip",
     "nsa_attn_bwd_walks": "iiiiiiiii",
+    "nsa_attn_bwd_walks_d64": "iiiiiiiii",
     "nsa_attn_fwd": "ipppppiiiiiifiiiipppip",
     "nsa_attn_importance": "ippppiiiiiifiiip",
     "nsa_comm_allgather": "ippliipuqip",
