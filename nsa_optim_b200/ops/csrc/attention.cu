@@ -71,6 +71,19 @@ __host__ __device__ __forceinline__ bool longest_first(const AttnParams& p) {
 }
 __device__ __forceinline__ int query_tile(const AttnParams& p) { return longest_first(p) ? gridDim.x - 1 - blockIdx.x : blockIdx.x; }
 
+// The same for kernels with one grid dimension: tile qt of n, KV head h, sequence b.  Longest first goes over all heads and sequences: a
+// head after the other, the longest tiles of the last one start late (4096 tokens x 16 and 8 heads of 64, SMs busy 77 % of the time).
+// The order is a template argument in the forward: chosen at run time it costs registers there, and 2 % without causality.
+struct QueryTile { int qt, n, h, b; };
+__device__ __forceinline__ QueryTile query_tile(const AttnParams& p, bool longest) {
+  const int heads = p.B * p.Hkv, n = gridDim.x / heads;
+  int i, bh;
+  if (longest) { i = blockIdx.x / heads; bh = blockIdx.x - i * heads; i = n - 1 - i; }
+  else { bh = blockIdx.x / n; i = blockIdx.x - bh * n; }
+  const int b = bh / p.Hkv;
+  return {i, n, bh - b * p.Hkv, b};
+}
+
 // Which key tiles a query tile visits, for contiguous-range modes.
 __device__ __forceinline__ void key_tile_range(const AttnParams& p, int t_lo, int t_hi, int& j0, int& j1) {
   // keys with pos <= t_hi (causal) and pos > t_lo - window (window)
@@ -490,7 +503,6 @@ __device__ __forceinline__ void q_half_to_tmem(uint32_t taddr, const uint8_t* ti
 constexpr int FWT_STAGES = 5;
 constexpr int fwt_smem(int D) { return D / 64 * (2 + 2 * FWT_STAGES) * HALF + 1024 + 1024 + 256; }
 
-// The order of the tiles is a template argument here: chosen at run time it costs registers and 2 % without causality.
 template <int D, bool LONGEST_FIRST>
 __global__ void __launch_bounds__(352, 1)
 attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -516,11 +528,11 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = LONGEST_FIRST ? gridDim.x - 1 - blockIdx.x : blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const auto [qt, n_qt, h, b] = query_tile(p, LONGEST_FIRST);
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
-  const long tile_slot = (static_cast<long>(b) * p.Hkv + h) * gridDim.x + qt;
+  const long tile_slot = (static_cast<long>(b) * p.Hkv + h) * n_qt + qt;
   const int* blocks = selected ? p.tile_blocks + tile_slot * p.max_u : nullptr;
   const unsigned long long* masks = selected ? p.tile_masks + tile_slot * p.max_u : nullptr;
   int kb0 = 0, n_vis;
@@ -834,7 +846,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // scores, 4 K from the last to the exit) run beside the visits of the other; nothing is merged.  Half of the shared memory and of the tensor memory
 // is left to a CTA: two stages of K and of V, S and P and O in 256 columns, Q in shared memory.
 // 8192 tokens x 32 query and 2 KV heads: 599 -> 517 us, without causality 1110 -> 1072, window 512 163 -> 121; 16384 2200 -> 1960.
-// head_dim 64, 128 columns less: 4096 tokens x 16 and 8 heads, with one group per CTA there too, 192 -> 101 us; 8192 x 16 / 8, window 512, 170 -> 60.
+// head_dim 64, 128 columns less: 4096 tokens x 16 and 8 heads 192 -> 68 us; 8192 x 16 / 8, window 512, 170 -> 58.
 // (Visits of 128 keys in one CTA, P over S: 16384 2386 us, window 512 174; S then waits for P V of the visit before.)
 // --------------------------------------------------------------------------------------
 constexpr int FW1_STAGES = 2;
@@ -866,11 +878,11 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = LONGEST_FIRST ? gridDim.x - 1 - blockIdx.x : blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const auto [qt, n_qt, h, b] = query_tile(p, LONGEST_FIRST);
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
-  const long tile_slot = (static_cast<long>(b) * p.Hkv + h) * gridDim.x + qt;
+  const long tile_slot = (static_cast<long>(b) * p.Hkv + h) * n_qt + qt;
   const int* blocks = selected ? p.tile_blocks + tile_slot * p.max_u : nullptr;
   const unsigned long long* masks = selected ? p.tile_masks + tile_slot * p.max_u : nullptr;
   int kb0 = 0, n_vis;
@@ -1163,7 +1175,7 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // always causal: longest tiles first
+  const auto [qt, n_qt, h, b] = query_tile(p, true);   // always causal
   const int q0 = qt * p.R;
   const int lim = min(q0 + p.R, p.T) - 1 - p.kp_off;
   const int last = min(lim < 0 ? -1 : lim / p.kp_stride, p.S - 1);
@@ -1922,11 +1934,11 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = query_tile(p), h = blockIdx.y, b = blockIdx.z;
+  const auto [qt, n_qt, h, b] = query_tile(p, longest_first(p));
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
   const bool selected = p.tile_blocks != nullptr;
-  const long tile_slot = (static_cast<long>(b) * p.Hkv + h) * gridDim.x + qt;
+  const long tile_slot = (static_cast<long>(b) * p.Hkv + h) * n_qt + qt;
   const int* blocks = selected ? p.tile_blocks + tile_slot * p.max_u : nullptr;
   const unsigned long long* masks = selected ? p.tile_masks + tile_slot * p.max_u : nullptr;
   int kb0 = 0, n_vis;
@@ -2463,7 +2475,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // both operands come from shared memory.  8192 tokens x 32 query and 2 KV heads: 1390 us; now 884.  A visit is 3100 cycles here:
 // exponentials 1200, dV and S 1100, the rest signals between them.  S for half tiles costs its products twice, 3250.)
 // head_dim 64 leaves room for two S^T, so S(v+1) is issued in front of dV(v) and the exponentials of v+1 wait for dS(v) alone.  With the dQ
-// kernel, 4096 tokens x 16 and 8 heads: 722 us where one kernel did both with reductions to memory for each tile, now 272.
+// kernel, 4096 tokens x 16 and 8 heads: 722 us where one kernel did both with reductions to memory for each tile, now 195.
 // Roles: warps 0-7 softmax (key lane, 64 query rows each), warp 8 TMA producer, warp 9 MMA issuer, warp 10 row statistics.
 // --------------------------------------------------------------------------------------
 struct KeyWalks {
@@ -2535,8 +2547,9 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int b = blockIdx.z / p.Hkv, h = blockIdx.z - b * p.Hkv;
-  const int s0 = blockIdx.x * KEYS;              // key block fastest: concurrent CTAs share a Q/dO range in L2
+  // Heads fastest: under causality the first key blocks have the longest walks, and the last CTAs to start are short
+  const int heads = p.B * p.Hkv, block = blockIdx.x / heads, b = (blockIdx.x - block * heads) / p.Hkv, h = blockIdx.x - block * heads - b * p.Hkv;
+  const int s0 = block * KEYS;
   int v0;
   const int n_vis = key_walk<KEYS>(p, w.visits, s0, blockIdx.y, v0);
   if (n_vis <= 0) return;
@@ -3454,20 +3467,17 @@ void fill_params(AttnParams& p, int B, int T, int S, int Hq, int Hkv, int D, flo
 }  // namespace
 
 // Two CTAs per SM with one softmax group each, or one with two?  A lone CTA takes its visits in one chain where the other form has two,
-// so there must be two CTAs and more for each SM, and of long tiles so many that the last ones weigh little.  Up to 16 visits
-// (two groups, one group): 200 CTAs x 13 visits 16.0 us, 17.5; 300 x 9 23.7, 19.2; 400 x 9 31.2, 29.7; 1200 x 9 97, 73.
-// More: 300 x 19 26.8, 27.9; 300 x 75 60, 72; 400 x 50 70, 70; 600 x 38 70, 56; 1200 x 75 221, 187; groups of one or two heads, whose
-// neighbouring tiles share no keys, are slower up to 1024 CTAs (600 x 75 129, 132; 1024 x 128 304, 309; 1536 x 192 686, 681).
+// so all SMs must have two CTAs for most of the time: three tiles for each SM, or more than one where tiles are short.  us of two groups and
+// of one, head_dim 64: 160 CTAs x 5 visits 10.8, 8.9; 250 x 9 17.6, 14.6; 256 x 16 17.9, 18.9; 500 x 16 34, 26; 256 x 32 26, 32; 504 x 32 49, 39;
+// 256 x 64 42, 61; 512 x 64 82, 68; 1024 x 128 290, 246.  head_dim 128: 160 x 5 12.8, 10.5; 250 x 9 19.9, 17.3; 256 x 16 20.0, 20.7; 500 x 16
+// 38, 30; 256 x 32 29.5, 34.7; 504 x 32 53, 44; 512 x 128 152, 132; 2048 x 128 594, 511.  Groups of 1 to 16 heads differ by less than 5 %.
 // A selected block counts as the keys of a sequence do: how many blocks the tokens of a tile share is not known here.
 // Compressed keys always take two groups: their L goes into the choice of blocks, where a last bit decides between near ties (with one
 // group, compressed and selected branch together 1159 us at 16384 tokens, 1298 with two, a few rows took another block than before).
-// head_dim 64 has shorter visits, and their start and end weigh more (two groups, one group): 152 CTAs x 5 visits 10.0 us, 8.8; 250 x 9
-// 17.8, 16.9; 250 x 16 18.1, 20.3; 500 x 16 34, 32; 500 x 32 50, 53 and 50, 41; 512 x 64 86, 97 and 85, 77; 1000 x 32 95, 87; 1024 x 128 299, 302 and 291, 253.
 static bool fwd_two_per_sm(const AttnParams& p, long ctas) {
   if (p.kp_stride > 1) return false;
   const int visits = (std::min(p.S, p.window > 0 ? p.window + p.R : p.S) + 63) / 64;
-  if (p.D == 64) return ctas > nsa::sm_count() * (visits <= 10 ? 1l : visits <= 16 ? 2l : 6l);
-  return ctas >= nsa::sm_count() * (visits <= 16 ? 2l : p.G >= 4 ? 4l : 8l);
+  return visits <= 12 ? ctas > nsa::sm_count() : ctas >= 3l * nsa::sm_count();
 }
 
 extern "C" int nsa_attn_fwd(const void* q, const void* k, const void* v, void* o, float* L, int B, int T, int S,
@@ -3488,20 +3498,21 @@ extern "C" int nsa_attn_fwd(const void* q, const void* k, const void* v, void* o
   static const bool legacy = [] { const char* e = getenv("NSA_B200_ATTN_FWD"); return e && !strcmp(e, "legacy"); }();
   static const bool smem_operands = [] { const char* e = getenv("NSA_B200_ATTN_FWD"); return e && !strcmp(e, "smem"); }();
   const bool wide = D == 128;
-  if ((wide || kp_stride == 1) && !legacy && !smem_operands && fwd_two_per_sm(p, static_cast<long>(grid.x) * Hkv * B)) {
+  const unsigned tiles = grid.x * Hkv * B;
+  if ((wide || kp_stride == 1) && !legacy && !smem_operands && fwd_two_per_sm(p, tiles)) {
     const int bytes = fw1_smem(D), form = wide * 2 + longest_first(p);
     void (*const kernels[4])(CUtensorMap, CUtensorMap, CUtensorMap, AttnParams) = {
         attn_fwd_half_kernel<64, false>, attn_fwd_half_kernel<64, true>, attn_fwd_half_kernel<128, false>, attn_fwd_half_kernel<128, true>};
     static bool cfg[4] = {};
     if (!cfg[form]) { if ((rc = set_smem(kernels[form], bytes))) return rc; cfg[form] = true; }
-    kernels[form]<<<grid, 224, bytes, st>>>(tq, tk, tv, p);
+    kernels[form]<<<tiles, 224, bytes, st>>>(tq, tk, tv, p);
   } else if ((wide || kp_stride == 1) && !legacy && !smem_operands) {
     const int bytes = fwt_smem(D), form = wide * 2 + longest_first(p);
     void (*const kernels[4])(CUtensorMap, CUtensorMap, CUtensorMap, AttnParams) = {
         attn_fwd_ts_kernel<64, false>, attn_fwd_ts_kernel<64, true>, attn_fwd_ts_kernel<128, false>, attn_fwd_ts_kernel<128, true>};
     static bool cfg[4] = {};
     if (!cfg[form]) { if ((rc = set_smem(kernels[form], bytes))) return rc; cfg[form] = true; }
-    kernels[form]<<<grid, 352, bytes, st>>>(tq, tk, tv, p);
+    kernels[form]<<<tiles, 352, bytes, st>>>(tq, tk, tv, p);
   } else if (D == 128 && !legacy) {
     const int smem_ws = (4 + 4 * FW_STAGES + 4) * HALF + 1024 + 1024 + 256;
     static bool cfg = false;
@@ -3543,7 +3554,7 @@ extern "C" int nsa_attn_importance(const void* q, const void* k_cmp, const float
   if (D == 128 && !legacy && 128 % (Hq / Hkv) == 0) {
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(attn_importance_ts_kernel, IMP_SMEM))) return rc; cfg = true; }
-    attn_importance_ts_kernel<<<grid, 320, IMP_SMEM, st>>>(tq, tk, p);
+    attn_importance_ts_kernel<<<grid.x * Hkv * B, 320, IMP_SMEM, st>>>(tq, tk, p);
   } else if (D == 128) {
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(attn_fwd_kernel<128, 1>, smem))) return rc; cfg = true; }
@@ -3609,10 +3620,10 @@ struct KeyRange {
 // Time of one form of the dK / dV kernel, as measured: a CTA's start and end and its longest walk; whole waves of mean walks; the chip's
 // throughput, with the longest walk behind it where there is more than a wave.
 struct KeyCost {
-  double start, visit, busy_start, busy_visit, tail, wave;
+  double start, visit, busy_start, busy_visit, tail, wave, wave_visit;
   double us(long ctas, long visits, int longest) const {
     const long sms = nsa::sm_count(), waves = (ctas + sms - 1) / sms;
-    return std::max({start + visit * longest, waves * (wave + 1.81 * visits / ctas),
+    return std::max({start + visit * longest, waves * (wave + wave_visit * visits / ctas),
                      (busy_start * ctas + busy_visit * visits) / sms + (waves > 1 ? tail * longest : 0.)});
   }
 };
@@ -3620,18 +3631,18 @@ struct KeyCost {
 // go to `part` (walks x 2 x B S Hkv D floats) if they are several.  0: blocks of more than 256 visits, in walks of `visits_per_cta`
 // tiles that add to dK and dV in any order (they fill the GPU, and room for all their sums would cost more than it gives).
 // 64 keys have less to set up and a visit of 1.4 us instead of 1.8, and are the better form where there are few visits and SMs enough;
-// walks keep all SMs busy where blocks are few.  The constants are fitted to 209 shapes of 64 to 8192 tokens, 1 to 16 KV heads,
-// groups of 1 to 32 and windows, each in both forms and with up to 64 walks; the choice is 0.3 % behind the best in the mean and 16 % at
-// worst.  us with 64 keys, and with 128 and 1 / 2 / 4 / 8 / 16 walks (queries / KV heads, windows w): 300 16/8 12.9, 17.1 16.7 15.1;
-// 1000 32/8 w64 13.2, 20.4 22.9 29.7; 1000 32/2 181, 210 116 69 45 33; 2000 32/8 w512 66, 47 66 72 96; 3000 16/16 141, 114 145 165 215 282.
+// walks keep all SMs busy where blocks are few.  The constants are fitted to 127 shapes (head_dim 64: 253, which has no form of 64 keys) of
+// 64 to 8192 tokens, 1 to 16 KV heads, groups of 1 to 32 and windows, each in both forms and with up to 64 walks; the choice is 0.3 % behind the
+// best in the mean and 10 % (14 %) at worst.  us with 64 keys, and with 128 and 1 / 2 / 4 / 8 / 16 walks (queries / KV heads, windows w): 300 16/8 12.9, 17.1 16.7 15.1;
+// 1000 32/8 w64 13.2, 20.4 22.9 29.7; 1000 32/2 181, 210 116 69 45 33; 2000 32/8 w512 66, 47 66 72 96; 3000 16/16 139, 95 139; head_dim 64: 300 16/8 14.6 13.8 12.7, 1000 32/2 190 105 61 40 28, 3000 16/16 84 105.
 static int choose_walks(int D, int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride) {
   if (B <= 0 || T <= 0 || S <= 0 || Hkv <= 0 || Hq < Hkv) return 0;
   const int R = std::max(1, BM / (Hq / Hkv));
   const long heads = static_cast<long>(B) * Hkv, sms = nsa::sm_count();
   const KeyRange wide(T, S, R, causal, window, kp_stride, 128), narrow(T, S, R, causal, window, kp_stride, 64);
   if (wide.most > 256) return 0;
-  const KeyCost by_128 = D == 128 ? KeyCost{8.3, 1.79, 10.1, 1.6, 1.26, 8.2} : KeyCost{7., 1.3, 8., 1.2, 1., 7.};
-  constexpr KeyCost by_64{6.2, 1.43, 7.2, 1.06, 1.16, 5.1};
+  const KeyCost by_128 = D == 128 ? KeyCost{7.9, 1.9, 8.05, 1.95, .28, 8.1, 1.82} : KeyCost{6.6, 1.65, 6.8, 2.16, .1, 7.1, .65};
+  constexpr KeyCost by_64{6.2, 1.43, 7.2, 1.06, 1.16, 5.1, 1.81};
   long total = 0;
   int longest = 0;
   for (int i = 0; i < narrow.blocks; ++i) {
@@ -3643,7 +3654,7 @@ static int choose_walks(int D, int B, int T, int S, int Hq, int Hkv, int causal,
   double least = D == 128 ? by_64.us(heads * narrow.blocks, heads * total, longest) : 1e30;
   for (int visits = wide.most; visits > 0; --visits) {
     const int walks = (wide.most + visits - 1) / visits;
-    if (walks > 1 && (walks - 1) * wide.blocks * heads > 3 * sms) break;     // bounds the room for sums: 128 KB for each walk of a block
+    if (walks > 1 && (walks - 1) * wide.blocks * heads > 3 * sms) break;     // bounds the room for sums: at most 128 KB for each walk of a block
     if (walks > 1 && (wide.most + walks - 1) / walks != visits) continue;    // as many walks as a longer visit count has
     long ctas = 0;                                                           // with something to do
     total = 0;
@@ -3656,7 +3667,7 @@ static int choose_walks(int D, int B, int T, int S, int Hq, int Hkv, int causal,
       longest = std::max(longest, std::min(visits, n));
     }
     double us = by_128.us(heads * ctas, heads * total, longest);
-    if (walks > 1) us += 2.2 + walks * heads * S * 1.9e-4;
+    if (walks > 1) us += 2.2 + walks * heads * S * (D == 128 ? 1.9e-4 : 1e-4);
     if (us < least) { least = us; best = walks; }
   }
   return best;
@@ -3709,7 +3720,7 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
       static bool cfg[2] = {};
       bool& ready = cfg[D == 128];
       if (!ready) { if ((rc = set_smem(kernel, dqt_smem(D)))) return rc; ready = true; }
-      kernel<<<grid, 384, dqt_smem(D), st>>>(tq, tdo, tk, tv, p, scale);
+      kernel<<<grid.x * Hkv * B, 384, dqt_smem(D), st>>>(tq, tdo, tk, tv, p, scale);
     } else {
       const int smem = (8 + 4 * DQ_STAGES + 2) * HALF + 1024 + 256;
       static bool cfg = false;
@@ -3744,7 +3755,7 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
     static bool cfg[2] = {};
     bool& ready = cfg[D == 128];
     if (!ready) { if ((rc = set_smem(kernel, kvc_smem(D)))) return rc; ready = true; }
-    kernel<<<dim3((S + 127) / 128, w.walks, B * Hkv), KVC_THREADS, kvc_smem(D), st>>>(tq, tdo, tk, tv, p, w, scale);
+    kernel<<<dim3((S + 127) / 128 * B * Hkv, w.walks), KVC_THREADS, kvc_smem(D), st>>>(tq, tdo, tk, tv, p, w, scale);
     if (w.part) {
       const long rows = static_cast<long>(B) * S * Hkv, per_cta = 256 / (D / 4);
       const dim3 grid((unsigned)((rows + per_cta - 1) / per_cta), 2);

@@ -45,7 +45,8 @@ def _check(native, B, T, Hq, Hkv, window, causal):
 
 @pytest.mark.parametrize("B,T,Hq,Hkv,window", [
     (1, 1, 4, 4, 0), (2, 17, 2, 2, 5), (1, 128, 64, 1, 0), (1, 129, 16, 2, 0), (2, 300, 16, 8, 0), (1, 640, 32, 2, 127), (1, 900, 32, 1, 129),
-    (1, 700, 8, 8, 300), (4, 777, 16, 8, 512), (1, 2100, 32, 1, 0), (40, 33, 16, 8, 0), (19, 130, 16, 16, 64), (2, 1500, 16, 16, 0), (2, 592, 32, 2, 0)])
+    (1, 700, 8, 8, 300), (4, 777, 16, 8, 512), (1, 2100, 32, 1, 0), (40, 33, 16, 8, 0), (19, 130, 16, 16, 64), (2, 1500, 16, 16, 0),
+    (1, 592, 32, 2, 0), (1, 600, 32, 2, 0), (1, 1768, 32, 2, 0), (1, 1776, 32, 2, 0)])    # 148, 150, 442 and 444 tiles: one CTA per SM and two
 def test_causal(native, B, T, Hq, Hkv, window):
     _check(native, B, T, Hq, Hkv, window, True)
 
