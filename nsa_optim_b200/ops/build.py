@@ -1,4 +1,4 @@
-"""Builds the native library ``libnsa_b200.so`` from ``ops/csrc/*.cu`` for sm_100a, in-tree.
+"""Builds the native library ``libnsa_b200.so`` from ``ops/csrc/*.cu`` for sm_100a and the extension module ``_nsa_host.so``, in-tree.
 
     python -m nsa_optim_b200.ops.build [--force] [--verbose] [--debug]
 
@@ -25,6 +25,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libnsa_b200.so")
+HOST = os.path.join(HERE, "_nsa_host.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "--use_fast_math", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3"]
@@ -61,6 +62,29 @@ def _compile(nvcc: str, name: str, extra: List[str], verbose: bool, obj_dir: str
     return obj
 
 
+def build_host(force: bool = False) -> str:
+    """Builds ``_nsa_host.so`` (``csrc/host_ops.cpp``), the host side of the ops against PyTorch's C++ interface.  It finds the kernel
+    library's entry points when ``ops/native.py`` binds it, so one build serves release and debug libraries."""
+    src = os.path.join(SRC, "host_ops.cpp")
+    deps = [src, os.path.join(SRC, "nsa_b200.h")]
+    if not force and os.path.exists(HOST) and os.path.getmtime(HOST) >= max(map(os.path.getmtime, deps)):
+        return HOST
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(nvcc_path()))
+    dirs = [SRC, os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+            os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared"] + [x for d in dirs for x in ("-I", d)]
+           + [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", src, "-o", HOST, "-L", os.path.join(base, "lib"),
+              "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ldl"])
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for host_ops.cpp:\n{r.stdout}\n{r.stderr}")
+    return HOST
+
+
 def build(force: bool = False, verbose: bool = False, debug: bool = False, out: str = None,
           only: List[str] = None) -> str:
     """Builds the library.  ``debug`` adds -DNSA_DEBUG_BOUNDS; a debug build goes to its own object
@@ -83,13 +107,16 @@ def build(force: bool = False, verbose: bool = False, debug: bool = False, out: 
         if stale:
             todo.append(name)
     if todo:
-        with cf.ThreadPoolExecutor(max_workers=min(8, len(todo))) as ex:
+        with cf.ThreadPoolExecutor(max_workers=min(8, len(todo) + 1)) as ex:
+            host = ex.submit(build_host, force)
             list(ex.map(lambda n: _compile(nvcc, n, extra, verbose, obj_dir), todo))
+            host.result()
     if todo or not os.path.exists(lib):
         cmd = [nvcc, "-shared", "-o", lib] + objs + ["-lcudart"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_host()
     return lib
 
 

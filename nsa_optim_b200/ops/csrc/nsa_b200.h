@@ -40,6 +40,16 @@ int nsa_rmsnorm_bwd(const void* x, const void* gate, const void* w, const void* 
 int nsa_rmsnorm_bwd_noalloc(const void* x, const void* gate, const void* w, const void* dy, const float* rstd,
                             void* dx, void* dgate, void* dw_bf16, float* dw_f32, long rows, int d, int mode,
                             cudaStream_t st);
+/* A gate of row pitch ldg (gated modes), a gradient dres added to dx, and h = x + r with y = rmsnorm(h) w. */
+int nsa_rmsnorm_fwd_ldg(const void* x, const void* gate, long ldg, const void* w, void* y, float* rstd, long rows, int d,
+                        float eps, int mode, cudaStream_t st);
+int nsa_rmsnorm_bwd_ldg(const void* x, const void* gate, long ldg, const void* w, const void* dy, const float* rstd,
+                        void* dx, void* dgate, void* dw_bf16, float* dw_f32, float* partial, long rows, int d, int mode,
+                        cudaStream_t st);
+int nsa_rmsnorm_bwd_res(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx,
+                        void* dw_bf16, float* dw_f32, float* partial, long rows, int d, cudaStream_t st);
+int nsa_rmsnorm_add_fwd(const void* x, const void* r, const void* w, void* h, void* y, float* rstd, long rows, int d,
+                        float eps, cudaStream_t st);
 int nsa_l2norm_fwd(const void* x, void* y, float* rinv, long rows, int d, float eps, cudaStream_t st);
 int nsa_l2norm_bwd(const void* y, const void* dy, const float* rinv, void* dx, long rows, int d, cudaStream_t st);
 int nsa_swiglu_fwd(const void* g, const void* u, void* y, long rows, int cols, long ldg, long ldu, cudaStream_t st);
@@ -120,6 +130,15 @@ int nsa_gate_combine_bwd(const void* o1, const void* o2, const void* o3, const v
     g3, const void* d_o, void* do1, void* do2, void* do3, void* dg1, void* dg2, void* dg3, long rows, int D, cudaStream_t
     st);
 
+/* Gates (or, with sig, their logits) of row pitch ldg; e1..e3 null or rowsum(do_i * o_i).  Mean pooling of windows. */
+int nsa_gate_combine_fwd_ex(const void* o1, const void* o2, const void* o3, const void* g1, const void* g2, const void*
+    g3, long ldg, int Hq, int sig, void* o, long rows, int D, cudaStream_t st);
+int nsa_gate_combine_bwd_ex(const void* o1, const void* o2, const void* o3, const void* g1, const void* g2, const void*
+    g3, long ldg, int Hq, int sig, const void* d_o, void* do1, void* do2, void* do3, void* dg1, void* dg2, void* dg3,
+    float* e1, float* e2, float* e3, long rows, int D, cudaStream_t st);
+int nsa_pool_fwd(const void* x, void* y, int B, int T, int width, long ldx, int block, int stride, cudaStream_t st);
+int nsa_pool_bwd(const void* dy, void* dx, int B, int T, int width, int block, int stride, cudaStream_t st);
+
 /* ---- Gated DeltaNet: per-chunk kernels (csrc/gdn_chunk.cu), state recurrence (csrc/gdn.cu) ---- */
 int nsa_gdn_prep(const void* q, const void* k, const void* v, const float* g, const float* beta, void* w, void* u,
     void* qk, float* X, float* gc, int B, int T, int H, int K, int V, float scale, cudaStream_t st);
@@ -133,6 +152,9 @@ int nsa_gdn_post(const void* q, const void* k, const void* v, const void* d_o, c
     void* dk, void* dv, float* dg, float* dbeta, int B, int T, int H, int K, int V, float scale, cudaStream_t st);
 
 /* ---- GEMM (csrc/gemm.cu) ---- */
+/* C32 (zeroed or to be added to) += op(A) op(B), the reduction cut into split_k parts. */
+int nsa_gemm_bf16_splitk(const void* A, const void* B, float* C32, int M, int N, int K, int lda, int ldb, int ldc,
+    int a_mn, int b_mn, int split_k, cudaStream_t stream);
 int nsa_gemm_bf16_ag(const void* A, void* C, int M, int N, int K, int lda, int ldc, const void* const* shards, void*
     full, long shard_elems, long b_elem_offset, int W, int rank, unsigned* chunk_flags, int chunks_per_shard, const
     unsigned* peer_flags, unsigned epoch, long long max_cycles, int copy_ctas, cudaStream_t stream);
@@ -163,6 +185,9 @@ int nsa_ssd_chunk_grad(const void* Cm, long ld_c, const void* Bm, long ld_b, con
     dB_part, float* dC_part, float* q_out, float* k_out, float* r_out, int B, int T, int H, int N, int P, cudaStream_t st);
 
 /* ---- further entry points of attention.cu ---- */
+int nsa_inverse_chunks(int BH, int T, int nS);
+int nsa_inverse_blocks(const int* idx, int* tok_list, int* list_start, int* item_start, int* hist, int* count, int BH,
+    int T, int n, int nS, int R, int visits_per_cta, cudaStream_t st);
 int nsa_select_blocks(const float* imp, int* idx, long rows, int T, int nS, int sel_block, int top_n, cudaStream_t
     st);
 

@@ -24,6 +24,8 @@ from .signatures import declare
 
 _LIB_PATH = os.environ.get("NSA_B200_LIB") or os.path.join(os.path.dirname(os.path.abspath(__file__)), "libnsa_b200.so")
 _lib: Optional[ctypes.CDLL] = None
+_host = None
+_SPLITK_MAX = int(os.environ.get("NSA_B200_SPLITK_MAX", "2"))
 
 SUPPORTED = {
     "linear", "rms_norm", "gated_rms_norm", "swiglu", "l2_norm", "rope", "embedding",
@@ -68,24 +70,29 @@ def lib_path() -> str:
 
 
 def load() -> ctypes.CDLL:
-    global _lib
+    global _lib, _host
     if _lib is None:
         if not os.path.exists(_LIB_PATH):
             raise FileNotFoundError(f"{_LIB_PATH} is missing; run `python -m nsa_optim_b200.ops.build`")
         lib = ctypes.CDLL(_LIB_PATH)
         declare(lib)
-        _lib = lib
+        from . import _nsa_host
+        _nsa_host.bind(_LIB_PATH, globals(), _SPLITK_MAX)
+        _host, _lib = _nsa_host, lib
     return _lib
+
+
+def _h():
+    """The extension module that prepares, allocates and launches (``csrc/host_ops.cpp``)."""
+    if _host is None:
+        load()
+    return _host
 
 
 def supports(op: str, t: Tensor) -> bool:
     if op not in SUPPORTED or not t.is_cuda:
         return False
-    if op in ("adamw", "adamw_lowbit"):
-        return t.dtype in (torch.bfloat16, torch.float32)
-    if op == "embedding":
-        return t.dtype == torch.bfloat16
-    return t.dtype == torch.bfloat16
+    return t.dtype == torch.bfloat16 or (t.dtype == torch.float32 and op in ("adamw", "adamw_lowbit"))
 
 
 def _check(rc: int) -> None:
@@ -190,12 +197,6 @@ def _empty_like(t: Tensor, dtype=None) -> Tensor:
     return torch.empty_like(t, dtype=dtype, memory_format=torch.contiguous_format)
 
 
-def _zeros_like(t: Tensor, dtype=None) -> Tensor:
-    if _CANARY and t.is_cuda:
-        return _guarded(tuple(t.shape), dtype or t.dtype, t.device, True)
-    return torch.zeros_like(t, dtype=dtype, memory_format=torch.contiguous_format)
-
-
 def check_canaries() -> int:
     """Verify and release the guard zones recorded so far; returns how many buffers were checked."""
     torch.cuda.synchronize()
@@ -234,28 +235,13 @@ def _as_2d(x: Tensor) -> Tensor:
     return x2
 
 
-_SPLITK_MAX = int(os.environ.get("NSA_B200_SPLITK_MAX", "2"))
-_gemm_which = "default"
-
-
 def split_k_choice(M: int, N: int, K: int, clusters: int = 74) -> int:
     """Parts to cut the reduction of an M x N x K GEMM into.  The pair kernel gives each CTA pair
     256 x 256 tiles; with few tiles and a long reduction (weight gradients: K = tokens) the last wave
     is mostly empty, and splitting the reduction fills it.  Two parts added into a zeroed fp32 C
     give the same bits in either order, so the default limit of 2 keeps results reproducible;
     ``NSA_B200_SPLITK_MAX`` raises it."""
-    if K < 8192 or M <= 128:
-        return 1
-    tiles = -(-M // 256) * -(-N // 256)
-    if tiles >= 6 * clusters:
-        return 1
-
-    def eff(S):
-        w = tiles * S / clusters
-        return w / -(-w // 1)
-
-    best = max(range(1, _SPLITK_MAX + 1), key=lambda S: eff(S) - 0.01 * S)
-    return best if eff(best) > eff(1) + 0.04 else 1
+    return _h().split_k_choice(M, N, K, clusters)
 
 
 def gemm(a: Tensor, b: Tensor, a_mn: bool, b_mn: bool, out: Optional[Tensor] = None,
@@ -265,69 +251,27 @@ def gemm(a: Tensor, b: Tensor, a_mn: bool, b_mn: bool, out: Optional[Tensor] = N
     True -> B is (K, N).  Row pitches may exceed the logical width (sliced views).  ``split_k``
     (default: chosen by :func:`split_k_choice`) cuts the reduction into parts that run on different
     CTA pairs and meet in fp32 through TMA reduce-add stores."""
-    a, b = _as_2d(a), _as_2d(b)
-    M, K = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
-    N, Kb = (b.shape[1], b.shape[0]) if b_mn else (b.shape[0], b.shape[1])
-    if K != Kb:
-        raise ValueError(f"gemm: reduction sizes differ ({K} vs {Kb})")
-    if out is None:
-        out = _empty(M, N, dtype=out_dtype, device=a.device)
-    if split_k is None:
-        split_k = split_k_choice(M, N, K) if (max_ctas == 0 and _gemm_which != "single") else 1
-    if split_k > 1 and M > 128:
-        direct = out.dtype == torch.float32 and out.stride(1) == 1 and out.stride(0) % 4 == 0 and out.data_ptr() % 16 == 0
-        if direct:
-            ws = out
-            if not accumulate:
-                ws.zero_()
-        else:
-            ws = out.float() if accumulate else _zeros(M, N, dtype=torch.float32, device=a.device)
-        _check(load().nsa_gemm_bf16_splitk(_p(a), _p(b), _p(ws), M, N, K, a.stride(0),
-                                           b.stride(0), ws.stride(0), int(a_mn), int(b_mn),
-                                           split_k, _stream()))
-        if not direct:
-            out.copy_(ws)
-        return out
-    _check(load().nsa_gemm_bf16(_p(a), _p(b), _p(out), M, N, K, a.stride(0),
-                                b.stride(0), out.stride(0), int(a_mn), int(b_mn),
-                                int(out.dtype == torch.float32), int(accumulate), max_ctas,
-                                _stream()))
-    return out
+    return _h().matmul(a, b, a_mn, b_mn, out, out_dtype, accumulate, max_ctas, split_k or 0)
 
 
 def gemm_select(which: str = "default") -> None:
     """Kernel used by plain GEMMs from now on: "pair" (two CTAs per 256 x 256 tile), "single"
     (one CTA per 128 x 256 tile) or "default" (pair unless NSA_B200_GEMM=single)."""
-    global _gemm_which
-    _gemm_which = which
     load().nsa_gemm_select({"default": 0, "single": 1, "pair": 2}[which])
-
-
-def _project(x2: Tensor, w: Tensor, lead) -> Tensor:
-    """x2 w^T in the shape (*lead, out features): the output is allocated as the caller wants it."""
-    y = _empty(*lead, w.shape[0], dtype=torch.bfloat16, device=x2.device)
-    gemm(x2, w, False, False, out=y if y.dim() == 2 else y.view(-1, w.shape[0]))
-    return y
+    _host.gemm_single(which == "single")
 
 
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x: Tensor, w: Tensor):
-        x2 = _as_2d(x)
+        y, x2 = _h().linear_fwd(x, w)
         ctx.save_for_backward(x2, w)
-        ctx.xshape = x.shape
-        return _project(x2, w, x.shape[:-1])
+        return y
 
     @staticmethod
     def backward(ctx, dy: Tensor):
         x2, w = ctx.saved_tensors
-        dy2 = _as_2d(dy)
-        dx = dw = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dy2, w, False, True).view(ctx.xshape)          # dy (M,N) @ w (N,K)
-        if ctx.needs_input_grad[1]:
-            dw = gemm(dy2, x2, True, True)                            # dy^T (N,M) @ x (M,K)
-        return dx, dw
+        return _host.multi_linear_bwd(x2, (w,), (dy,), ctx.needs_input_grad[0], ctx.needs_input_grad[1])
 
 
 class _MultiLinear(torch.autograd.Function):
@@ -337,36 +281,21 @@ class _MultiLinear(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x: Tensor, run_first, *ws: Tensor):
-        x2 = _as_2d(x)
+        if run_first is None:
+            *ys, x2 = _h().multi_linear_fwd(x, ws)
+        else:
+            x2 = _as_2d(x)
+            ys = [run_first(x2, ws[0]).view(*x.shape[:-1], ws[0].shape[0])]
+            ys += _h().multi_linear_fwd(x, ws[1:])[:-1]
         ctx.save_for_backward(x2, *ws)
-        ctx.xshape = x.shape
-        ys = []
-        for i, w in enumerate(ws):
-            if i == 0 and run_first is not None:
-                ys.append(run_first(x2, w).view(*x.shape[:-1], w.shape[0]))
-            else:
-                ys.append(_project(x2, w, x.shape[:-1]))
         return tuple(ys)
 
     @staticmethod
     def backward(ctx, *dys):
         x2, *ws = ctx.saved_tensors
-        dx = None
-        dws = []
-        for i, (dy, w) in enumerate(zip(dys, ws)):
-            if dy is None:
-                dws.append(None)
-                continue
-            dy2 = _as_2d(dy)
-            if ctx.needs_input_grad[0]:
-                if dx is None:
-                    dx = gemm(dy2, w, False, True)
-                else:
-                    gemm(dy2, w, False, True, out=dx, accumulate=True, split_k=1)
-            dws.append(gemm(dy2, x2, True, True) if ctx.needs_input_grad[2 + i] else None)
-        if dx is not None:
-            dx = dx.view(ctx.xshape)
-        return (dx, None) + tuple(dws)
+        wanted = sum(1 << i for i, need in enumerate(ctx.needs_input_grad[2:]) if need)
+        dx, *dws = _host.multi_linear_bwd(x2, tuple(ws), dys, ctx.needs_input_grad[0], wanted)
+        return (dx, None, *dws)
 
 
 def multi_linear(x: Tensor, ws) -> tuple:
@@ -421,16 +350,12 @@ class _LinearGather(torch.autograd.Function):
         x2 = _as_2d(x)
         y = run(x2, w)
         ctx.save_for_backward(x2, w)
-        ctx.xshape = x.shape
         return y.view(*x.shape[:-1], w.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
         x2, w = ctx.saved_tensors
-        dy2 = _as_2d(dy)
-        dx = gemm(dy2, w, False, True).view(ctx.xshape) if ctx.needs_input_grad[0] else None
-        dw = gemm(dy2, x2, True, True) if ctx.needs_input_grad[1] else None
-        return dx, dw, None
+        return (*_host.multi_linear_bwd(x2, (w,), (dy,), ctx.needs_input_grad[0], ctx.needs_input_grad[1]), None)
 
 
 def linear(x: Tensor, w: Tensor) -> Tensor:
@@ -449,65 +374,26 @@ def linear(x: Tensor, w: Tensor) -> Tensor:
 # --------------------------------------------------------------------------------------
 # norms
 # --------------------------------------------------------------------------------------
-def _rms_fwd(x2, gate2, w, eps, mode):
-    rows, d = x2.shape
-    y = _empty_like(x2)
-    rstd = _empty(rows, dtype=torch.float32, device=x2.device)
-    _check(load().nsa_rmsnorm_fwd(_p(x2), _p(gate2), _p(w), _p(y), _p(rstd), rows, d,
-                                  eps, mode, _stream()))
-    return y, rstd
-
-
-def _rms_bwd(x2, gate2, w, dy2, rstd, mode):
-    rows, d = x2.shape
-    dx = _empty_like(x2)
-    dg = _empty_like(x2) if mode != 0 else None
-    dw = _empty(d, dtype=torch.bfloat16, device=x2.device)
-    parts = load().nsa_rmsnorm_bwd_parts(rows, d)
-    partial = _empty(parts * d, dtype=torch.float32, device=x2.device)
-    _check(load().nsa_rmsnorm_bwd(_p(x2), _p(gate2), _p(w), _p(dy2), _p(rstd), _p(dx), _p(dg), _p(dw), None,
-                                  _p(partial), rows, d, mode, _stream()))
-    return dx, dg, dw
-
-
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps):
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        wb = w.to(torch.bfloat16)
-        y, rstd = _rms_fwd(x2, None, wb, eps, 0)
-        ctx.save_for_backward(x2, wb, rstd)
+        y, xc, wb, rstd = _h().rms_fwd(x, w, eps)
+        ctx.save_for_backward(xc, wb, rstd)
         ctx.wdtype = w.dtype
-        return y.view(x.shape)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
-        x2, wb, rstd = ctx.saved_tensors
-        dx, _, dw = _rms_bwd(x2, None, wb, dy.reshape(x2.shape).contiguous(), rstd, 0)
-        return dx.view(dy.shape), dw.to(ctx.wdtype), None
+        xc, wb, rstd = ctx.saved_tensors
+        return (*_host.rms_bwd(xc, wb, rstd, dy, None, ctx.wdtype), None)
 
 
-def _rms_bwd_res(x2, w, dy2, rstd, dres2):
-    rows, d = x2.shape
-    dx = _empty_like(x2)
-    dw = _empty(d, dtype=torch.bfloat16, device=x2.device)
-    parts = load().nsa_rmsnorm_bwd_parts(rows, d)
-    partial = _empty(parts * d, dtype=torch.float32, device=x2.device)
-    _check(load().nsa_rmsnorm_bwd_res(_p(x2), _p(w), _p(dy2), _p(rstd), _p(dres2), _p(dx), _p(dw), None,
-                                      _p(partial), rows, d, _stream()))
-    return dx, dw
-
-
-def _norm_grads(ctx, h2, wb, rstd, dres, dy):
-    """Gradient at the input of a plain norm that also receives `dres` by the residual route."""
+def _norm_grads(ctx, dres, dy):
+    """Gradients of a plain norm's input, which also receives `dres` by the residual route, and weight."""
     if dy is None:
-        return (dres, None)
-    dy2 = dy.reshape(h2.shape).contiguous()
-    if dres is None:
-        dx, _, dw = _rms_bwd(h2, None, wb, dy2, rstd, 0)
-    else:
-        dx, dw = _rms_bwd_res(h2, wb, dy2, rstd, dres.reshape(h2.shape).contiguous())
-    return dx.view(dy.shape), dw.to(ctx.wdtype)
+        return dres, None
+    h, wb, rstd = ctx.saved_tensors
+    return _host.rms_bwd(h, wb, rstd, dy, dres, ctx.wdtype)
 
 
 class _RMSNormSkip(torch.autograd.Function):
@@ -517,18 +403,14 @@ class _RMSNormSkip(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w, eps):
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        wb = w.to(torch.bfloat16)
-        y, rstd = _rms_fwd(x2, None, wb, eps, 0)
-        ctx.save_for_backward(x2, wb, rstd)
+        y, xc, wb, rstd = _h().rms_fwd(x, w, eps)
+        ctx.save_for_backward(xc, wb, rstd)
         ctx.wdtype = w.dtype
-        return y.view(x.shape), x.view_as(x)
+        return y, x.view_as(x)
 
     @staticmethod
     def backward(ctx, dy, dskip):
-        x2, wb, rstd = ctx.saved_tensors
-        dx, dw = _norm_grads(ctx, x2, wb, rstd, dskip, dy)
-        return dx, dw, None
+        return (*_norm_grads(ctx, dskip, dy), None)
 
 
 class _AddRMSNorm(torch.autograd.Function):
@@ -537,23 +419,14 @@ class _AddRMSNorm(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, r, w, eps):
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        r2 = r.reshape(-1, r.shape[-1]).contiguous()
-        wb = w.to(torch.bfloat16)
-        rows, d = x2.shape
-        h = _empty_like(x2)
-        y = _empty_like(x2)
-        rstd = _empty(rows, dtype=torch.float32, device=x2.device)
-        _check(load().nsa_rmsnorm_add_fwd(_p(x2), _p(r2), _p(wb), _p(h), _p(y), _p(rstd), rows, d,
-                                          eps, _stream()))
+        h, y, wb, rstd = _h().add_rms_fwd(x, r, w, eps)
         ctx.save_for_backward(h, wb, rstd)
         ctx.wdtype = w.dtype
-        return h.view(x.shape), y.view(x.shape)
+        return h, y
 
     @staticmethod
     def backward(ctx, dh, dy):
-        h2, wb, rstd = ctx.saved_tensors
-        dx, dw = _norm_grads(ctx, h2, wb, rstd, dh, dy)
+        dx, dw = _norm_grads(ctx, dh, dy)
         return dx, dx, dw, None
 
 
@@ -571,58 +444,19 @@ def add_rms_norm(x, r, w, eps=1e-6):
     return _run(_AddRMSNorm, x, r, w, eps)
 
 
-def _gate_rows(gate: Tensor):
-    """(2-D gate, row pitch): a column slice of a wider row-major matrix is used in place when its
-    rows are 16-byte aligned; anything else is made contiguous."""
-    d = gate.shape[-1]
-    if gate.dim() >= 2 and gate.stride(-1) == 1 and gate.data_ptr() % 16 == 0:
-        pitch = gate.stride(-2)
-        exp, ok = pitch, pitch % 8 == 0 and pitch >= d
-        for k in range(gate.dim() - 2, -1, -1):
-            if gate.shape[k] != 1 and gate.stride(k) != exp:
-                ok = False
-            exp *= gate.shape[k]
-        if ok:
-            rows = gate.numel() // d
-            return torch.as_strided(gate, (rows, d), (pitch, 1)), pitch
-    g2 = gate.reshape(-1, d).contiguous()
-    return g2, d
-
-
-def _row_pitch(t: Tensor) -> int:
-    """Elements from one row (last dimension) to the next.  Read from a saved tensor as it comes back: saved-tensor
-    hooks (activations kept on the host) return a pitched view as a dense tensor."""
-    return t.shape[-1] if t.is_contiguous() else t.stride(-2)
-
-
 class _GatedRMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gate, w, eps, norm_before_gate):
-        mode = 1 if norm_before_gate else 2
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        g2, ldg = _gate_rows(gate)
-        wb = w.to(torch.bfloat16)
-        rows, d = x2.shape
-        y = _empty_like(x2)
-        rstd = _empty(rows, dtype=torch.float32, device=x2.device)
-        _check(load().nsa_rmsnorm_fwd_ldg(_p(x2), _p(g2), ldg, _p(wb), _p(y), _p(rstd), rows, d,
-                                          eps, mode, _stream()))
-        ctx.save_for_backward(x2, g2, wb, rstd)
-        ctx.mode, ctx.wdtype, ctx.gshape = mode, w.dtype, gate.shape
-        return y.view(x.shape)
+        ctx.mode, ctx.wdtype, ctx.gshape = 1 if norm_before_gate else 2, w.dtype, gate.shape
+        y, xc, g2, wb, rstd = _h().gated_rms_fwd(x, gate, w, eps, ctx.mode)
+        ctx.save_for_backward(xc, g2, wb, rstd)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
-        x2, g2, wb, rstd = ctx.saved_tensors
-        rows, d = x2.shape
-        dy2 = dy.reshape(x2.shape).contiguous()
-        dx, dg = _empty_like(x2), _empty_like(x2)
-        dw = _empty(d, dtype=torch.bfloat16, device=x2.device)
-        parts = load().nsa_rmsnorm_bwd_parts(rows, d)
-        partial = _empty(parts * d, dtype=torch.float32, device=x2.device)
-        _check(load().nsa_rmsnorm_bwd_ldg(_p(x2), _p(g2), _row_pitch(g2), _p(wb), _p(dy2), _p(rstd), _p(dx), _p(dg), _p(dw),
-                                          None, _p(partial), rows, d, ctx.mode, _stream()))
-        return dx.view(dy.shape), dg.view(ctx.gshape), dw.to(ctx.wdtype), None, None
+        xc, g2, wb, rstd = ctx.saved_tensors
+        dx, dg, dw = _host.gated_rms_bwd(xc, g2, wb, rstd, dy, ctx.mode, ctx.wdtype)
+        return dx, dg.view(ctx.gshape), dw, None, None
 
 
 def rms_norm(x, w, eps=1e-6):
@@ -644,21 +478,13 @@ def gated_rms_norm(x, gate, w, eps=1e-6, norm_before_gate=True):
 class _L2Norm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, eps):
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        rows, d = x2.shape
-        y = _empty_like(x2)
-        rinv = _empty(rows, dtype=torch.float32, device=x.device)
-        _check(load().nsa_l2norm_fwd(_p(x2), _p(y), _p(rinv), rows, d, eps, _stream()))
+        y, rinv = _h().l2_fwd(x, eps)
         ctx.save_for_backward(y, rinv)
-        return y.view(x.shape)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
-        y, rinv = ctx.saved_tensors
-        dy2 = dy.reshape(y.shape).contiguous()
-        dx = _empty_like(y)
-        _check(load().nsa_l2norm_bwd(_p(y), _p(dy2), _p(rinv), _p(dx), y.shape[0], y.shape[1], _stream()))
-        return dx.view(dy.shape), None
+        return _host.l2_bwd(*ctx.saved_tensors, dy), None
 
 
 def l2_norm(x, eps=1e-6):
@@ -672,34 +498,16 @@ def l2_norm(x, eps=1e-6):
 # --------------------------------------------------------------------------------------
 # SwiGLU, RoPE
 # --------------------------------------------------------------------------------------
-def _rows_view(t: Tensor) -> Tensor:
-    t2 = t.reshape(-1, t.shape[-1])
-    if t2.stride(-1) != 1 or t2.stride(0) % 8 or t2.data_ptr() % 16:
-        t2 = t2.contiguous()
-    return t2
-
-
 class _SwiGLU(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gate, up):
-        g2, u2 = _rows_view(gate), _rows_view(up)
-        rows, cols = g2.shape
-        y = _empty(rows, cols, dtype=gate.dtype, device=gate.device)
-        _check(load().nsa_swiglu_fwd(_p(g2), _p(u2), _p(y), rows, cols, g2.stride(0),
-                                     u2.stride(0), _stream()))
+        y, g2, u2 = _h().swiglu_fwd(gate, up)
         ctx.save_for_backward(g2, u2)
-        return y.view(gate.shape)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
-        g2, u2 = ctx.saved_tensors
-        rows, cols = g2.shape
-        dy2 = dy.reshape(rows, cols).contiguous()
-        dg = _empty(rows, cols, dtype=dy.dtype, device=dy.device)
-        du = _empty(rows, cols, dtype=dy.dtype, device=dy.device)
-        _check(load().nsa_swiglu_bwd(_p(g2), _p(u2), _p(dy2), _p(dg), _p(du), rows, cols,
-                                     g2.stride(0), u2.stride(0), cols, _stream()))
-        return dg.view(dy.shape), du.view(dy.shape)
+        return _host.swiglu_bwd(*ctx.saved_tensors, dy)
 
 
 def swiglu(gate, up):
@@ -709,27 +517,18 @@ def swiglu(gate, up):
     return _run(_SwiGLU, gate, up)
 
 
-def _rope_call(x: Tensor, cos: Tensor, sin: Tensor, backward: bool) -> Tensor:
-    B, T, H, D = x.shape
-    xc = x.contiguous()
-    y = _empty_like(xc)
-    _check(load().nsa_rope(_p(xc), _p(cos), _p(sin), _p(y), B, T, H, D,
-                           int(backward), _stream()))
-    return y
-
-
 class _RoPE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, cos, sin):
         cos = cos.float().contiguous()
         sin = sin.float().contiguous()
         ctx.save_for_backward(cos, sin)
-        return _rope_call(x, cos, sin, False)
+        return _h().rope(x, cos, sin, False)
 
     @staticmethod
     def backward(ctx, dy):
         cos, sin = ctx.saved_tensors
-        return _rope_call(dy, cos, sin, True), None, None
+        return _host.rope(dy, cos, sin, True), None, None
 
 
 def rope(x, cos, sin):
@@ -745,37 +544,15 @@ def rope(x, cos, sin):
 class _Conv1d(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, activation):
-        B, T, C = x.shape
-        xv = x if (x.stride(2) == 1 and x.stride(1) % 8 == 0 and x.stride(0) == T * x.stride(1)
-                   and x.data_ptr() % 16 == 0) else x.contiguous()
-        wb = weight.to(torch.bfloat16).contiguous()
-        bb = None if bias is None else bias.to(torch.bfloat16).contiguous()
-        y = _empty(B, T, C, dtype=x.dtype, device=x.device)
-        _check(load().nsa_conv1d_fwd(_p(xv), _p(wb), _p(bb), _p(y), B, T, C,
-                                     xv.stride(1), weight.shape[-1], int(activation), _stream()))
+        y, xv, wb, bb = _h().conv_fwd(x, weight, bias, activation)
         ctx.save_for_backward(xv, wb, bb)
         ctx.activation, ctx.wdtype = activation, weight.dtype
-        ctx.has_bias = bias is not None
         return y
 
     @staticmethod
     def backward(ctx, dy):
         xv, wb, bb = ctx.saved_tensors
-        B, T, C = xv.shape
-        W = wb.shape[-1]
-        dyc = dy.contiguous()
-        dx = _empty(B, T, C, dtype=dy.dtype, device=dy.device)
-        parts = load().nsa_conv1d_bwd_parts(B, T, C)
-        partial = _empty(parts * (W + 1) * C, dtype=torch.float32, device=dy.device)
-        out = ctx.wdtype if ctx.wdtype == torch.bfloat16 else torch.float32
-        dw = _empty(C, W, dtype=out, device=dy.device)
-        db = _empty(C, dtype=out, device=dy.device) if ctx.has_bias else None
-        _check(load().nsa_conv1d_bwd(_p(xv), _p(wb), _p(bb), _p(dyc), _p(dx), _p(partial), _p(dw), _p(db),
-                                     int(out == torch.float32), B, T, C, xv.stride(1),
-                                     W, int(ctx.activation), _stream()))
-        dw = dw.to(ctx.wdtype)
-        db = db.to(ctx.wdtype) if ctx.has_bias else None
-        return dx, dw, db, None
+        return (*_host.conv_bwd(xv, wb, bb, dy, ctx.activation, ctx.wdtype), None)
 
 
 def causal_conv1d(x, weight, bias, activation=True):
@@ -791,13 +568,10 @@ def causal_conv1d(x, weight, bias, activation=True):
 class _Embedding(torch.autograd.Function):
     @staticmethod
     def forward(ctx, ids, weight):
-        flat = ids.reshape(-1).contiguous()
-        n, d = flat.numel(), weight.shape[1]
-        y = _empty(n, d, dtype=weight.dtype, device=weight.device)
-        _check(load().nsa_embedding_fwd(_p(flat), _p(weight), _p(y), n, d, weight.shape[0], _stream()))
+        y, flat = _h().embedding_fwd(ids, weight)
         ctx.save_for_backward(flat)
         ctx.wshape, ctx.wdtype = weight.shape, weight.dtype
-        return y.view(*ids.shape, d)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
@@ -826,33 +600,10 @@ class _LinearCE(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, hidden, weight, labels, ignore_index, chunk):
-        N, d = hidden.shape
-        V = weight.shape[0]
-        h = _as_2d(hidden)
-        labels = labels.contiguous()
-        need_h, need_w = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-        n_valid = (labels != ignore_index).sum().clamp_min(1).float()
-        inv = (1.0 / n_valid).reshape(1)
-        loss_rows = _empty(N, dtype=torch.float32, device=hidden.device)
-        dh = _empty_like(h) if need_h else None
-        dw = None
-        if need_w:                                   # the first chunk's GEMM writes it whole
-            dw = (_empty if N > 0 else _zeros)(V, d, dtype=torch.float32, device=hidden.device)
-        logits = _empty(min(chunk, N), V, dtype=torch.bfloat16, device=hidden.device)
-        for s0 in range(0, N, chunk):
-            s1 = min(N, s0 + chunk)
-            lg = logits[: s1 - s0]
-            gemm(h[s0:s1], weight, False, False, out=lg)
-            _check(load().nsa_cross_entropy(_p(lg), _p(labels[s0:s1]), _p(loss_rows[s0:s1]), _p(inv), s1 - s0,
-                                            V, lg.stride(0), ignore_index,
-                                            int(need_h or need_w), _stream()))
-            if need_h:
-                gemm(lg, weight, False, True, out=dh[s0:s1])                   # dlogits (n,V) @ W (V,d)
-            if need_w:
-                gemm(lg, h[s0:s1], True, True, out=dw, accumulate=(s0 > 0))    # dlogits^T (V,n) @ h (n,d)
+        loss, dh, dw = _h().cross_entropy_fwd(hidden, weight, labels, ignore_index, chunk, *ctx.needs_input_grad[:2])
         ctx.save_for_backward(dh, dw)
         ctx.wdtype = weight.dtype
-        return loss_rows.sum() * inv[0]
+        return loss
 
     @staticmethod
     def backward(ctx, gout):
@@ -868,10 +619,7 @@ def _scaled_by(t: Tensor, s: Tensor, dtype: torch.dtype) -> Tensor:
         return (t * s).to(dtype)
     if dtype != torch.bfloat16 or t.dtype not in (torch.float32, torch.bfloat16) or not t.is_contiguous() or t.data_ptr() % 16:
         return (t * s).to(dtype)
-    out = _empty(t.shape, dtype=dtype, device=t.device)
-    sf = s.reshape(1).float()
-    _check(load().nsa_scale_bf16(_p(t), _p(out), _p(sf), t.numel(), int(t.dtype == torch.float32), _stream()))
-    return out
+    return _h().scale(t, s)
 
 
 def linear_cross_entropy(hidden, weight, labels, ignore_index=-100, chunk=4096):
@@ -884,56 +632,18 @@ def linear_cross_entropy(hidden, weight, labels, ignore_index=-100, chunk=4096):
 # --------------------------------------------------------------------------------------
 # optimizer steps
 # --------------------------------------------------------------------------------------
-def _require_numel(what: str, t: Optional[Tensor], n: int) -> None:
-    """The update kernels index every state tensor with the parameter's element count; a state
-    restored from a checkpoint of another sharding would make them run past its end."""
-    if t is not None and t.numel() != n:
-        raise ValueError(f"optimizer state '{what}' has {t.numel()} elements, the kernel needs {n}")
-
-
-def _adamw_words(items, block: int) -> ctypes.Array:
-    """Seven 64-bit words per tensor, (p, g, m, v, a, b, n).  Every state tensor is checked against n; with ``block``
-    the last two are the scales of the quantised moments, else an fp32 master copy (or None) and nothing."""
-    words = []
-    for p, g, m, v, a, b in items:
-        n = p.numel()
-        na = n // block if block else n
-        if (g.numel() != n or m.numel() != n or v.numel() != n or (a is not None and a.numel() != na)
-                or (b is not None and b.numel() != na)):
-            for what, t in (("grad", g), ("exp_avg", m), ("exp_avg_sq", v)):
-                _require_numel(what, t, n)
-            _require_numel("exp_avg_absmax" if block else "master", a, na)
-            _require_numel("exp_avg_sq_absmax", b, na)
-        words += (p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), 0 if a is None else a.data_ptr(),
-                  0 if b is None else b.data_ptr(), n)
-    return (ctypes.c_longlong * len(words))(*words)
-
-
 def adamw_multi(items, step, lr, b1, b2, eps, wd, grad_scale) -> None:
-    """AdamW over (p, g, exp_avg, exp_avg_sq, master or None, None) tuples that share a device, dtypes and step."""
-    p, g = items[0][:2]
-    words = _adamw_words(items, 0)
-    gs = None if grad_scale is None else grad_scale.reshape(1).float()
-    _check(load().nsa_adamw_multi(words, len(items), _p(gs), int(p.dtype == torch.float32),
-                                  int(g.dtype == torch.float32), step, lr, b1, b2,
-                                  eps, wd, _stream()))
+    """AdamW over (p, g, exp_avg, exp_avg_sq, master or None, None) tuples that share a device, dtypes and step.  The kernels index
+    every state tensor with the parameter's element count: a state restored from a checkpoint of another sharding is refused."""
+    _h().adamw(items, grad_scale, step, lr, b1, b2, eps, wd)
 
 
 def adamw8bit_multi(items, step, lr, b1, b2, eps, wd, grad_scale, block) -> None:
     """8-bit AdamW over (p, g, codes m, codes v, scales m, scales v) tuples that share a device, dtypes and step."""
     if block != 256:
         raise ValueError("the native 8-bit AdamW kernel uses 256-element blocks")
-    for it in items:
-        if it[0].numel() % block:
-            raise ValueError(f"8-bit AdamW needs a multiple of {block} elements, got {it[0].numel()}")
-    p, g = items[0][:2]
-    words = _adamw_words(items, block)
-    gs = None if grad_scale is None else grad_scale.reshape(1).float()
-    cs = quant.codebook(8, True, p.device)
-    cu = quant.codebook(8, False, p.device)
-    _check(load().nsa_adamw8bit_multi(words, len(items), _p(cs), _p(cu), _p(gs), int(p.dtype == torch.float32),
-                                      int(g.dtype == torch.float32), step, lr, b1,
-                                      b2, eps, wd, _stream()))
+    dev = items[0][0].device
+    _h().adamw8bit(items, quant.codebook(8, True, dev), quant.codebook(8, False, dev), grad_scale, step, lr, b1, b2, eps, wd, block)
 
 
 def adamw_step(p, g, m, v, master, step, lr, b1, b2, eps, wd, grad_scale):
@@ -954,44 +664,16 @@ class _GatedDelta(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, scale):
-        B, T, H, K = q.shape
-        V = v.shape[-1]
-        BH, nc = B * H, -(-T // 64)
-        dev, bf, f32 = q.device, torch.bfloat16, torch.float32
         train = any(ctx.needs_input_grad)
-        w, u = _empty(BH, nc, 64, K, dtype=bf, device=dev), _empty(BH, nc, 64, V, dtype=bf, device=dev)
-        qk, gc = _empty(BH, nc, 64, 64, dtype=bf, device=dev), _empty(BH, nc, 64, dtype=f32, device=dev)
-        X = _empty(BH, nc, 64, 64, dtype=f32, device=dev) if train else None
-        o = _empty(B, T, H, V, dtype=bf, device=dev)
-        v_new = _empty(BH, nc, 64, V, dtype=bf, device=dev) if train else None
-        S = _empty(BH, nc, K, V, dtype=bf, device=dev) if train else None
-        lib, st = load(), _stream()
-        dims = (B, T, H, K, V, scale, st)
-        _check(lib.nsa_gdn_prep(_p(q), _p(k), _p(v), _p(g), _p(beta), _p(w), _p(u), _p(qk), _p(X), _p(gc), *dims))
-        _check(lib.nsa_gdn_seq_fwd(_p(q), _p(k), _p(w), _p(u), _p(qk), _p(gc), _p(o), _p(v_new), _p(S), *dims))
+        o, *kept = _h().gdn_fwd(q, k, v, g, beta, scale, train)
         if train:
-            ctx.save_for_backward(q, k, v, beta, w, qk, gc, X, v_new, S)
+            ctx.save_for_backward(q, k, v, beta, *kept)
             ctx.scale = scale
         return o
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v, beta, w, qk, gc, X, v_new, S = ctx.saved_tensors
-        B, T, H, K = q.shape
-        V = v.shape[-1]
-        BH, nc = B * H, gc.shape[1]
-        dev = q.device
-        do = do.to(torch.bfloat16).contiguous()
-        du, dS = _empty_like(v_new), _empty_like(S)
-        dgamma = _empty(V // 64, BH, nc, dtype=torch.float32, device=dev)
-        dq, dk, dv = _empty_like(q), _empty_like(k), _empty_like(v)
-        dg, dbeta = _empty_like(beta), _empty_like(beta)
-        lib, st = load(), _stream()
-        dims = (B, T, H, K, V, ctx.scale, st)
-        _check(lib.nsa_gdn_seq_bwd(_p(q), _p(k), _p(w), _p(qk), _p(S), _p(do), _p(gc), _p(du), _p(dS), _p(dgamma), *dims))
-        _check(lib.nsa_gdn_post(_p(q), _p(k), _p(v), _p(do), _p(beta), _p(gc), _p(X), _p(v_new), _p(du), _p(S), _p(dS), _p(dgamma),
-                                _p(dq), _p(dk), _p(dv), _p(dg), _p(dbeta), *dims))
-        return dq, dk, dv, dg, dbeta, None
+        return (*_host.gdn_bwd(*ctx.saved_tensors, do, ctx.scale), None)
 
 
 def _dense16(t: Tensor) -> Tensor:
@@ -1020,52 +702,6 @@ def gated_delta_rule(q, k, v, g, beta, scale=None, chunk=64):
 # --------------------------------------------------------------------------------------
 # attention family (csrc/attention.cu)
 # --------------------------------------------------------------------------------------
-def _attn_forward(q, k, v, causal, window, scale, kp_stride, kp_off, tiles):
-    """(output, L) of contiguous q, k, v; see :class:`_Attn`."""
-    B, T, Hq, D = q.shape
-    S, Hkv = k.shape[1], k.shape[2]
-    o = _empty_like(q)
-    L = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
-    tb, tm, tc, mu = tiles[:4] if tiles is not None else (None, None, None, 0)
-    _check(load().nsa_attn_fwd(_p(q), _p(k), _p(v), _p(o), _p(L), B, T, S, Hq,
-                               Hkv, D, scale, int(causal), window,
-                               kp_stride, kp_off, _p(tb), _p(tm), _p(tc), mu, _stream()))
-    return o, L
-
-
-def _attn_backward_split(q, k, v, o, do, L, dq, dk, dv, causal, window, scale, kp_stride, kp_off, tiles, delta=None, add_dq=False):
-    """dQ from the query-tile-outer kernel, dK / dV from the key-block-stationary kernel.  dk and dv (fp32) are added
-    to, dq (bf16) is written or, with ``add_dq``, added to; ``delta`` is rowsum(do * o) where the caller has it."""
-    B, T, Hq, D = q.shape
-    S, Hkv = k.shape[1], k.shape[2]
-    given = delta is not None
-    if not given:
-        delta = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
-    tb, tm, tc, mu = tiles[:4] if tiles is not None else (None, None, None, 0)
-    inv = (None, None, None, 0, 0)
-    visits, walks, part = _kv_visits(), 0, None
-    if tiles is None:
-        walks_of = load().nsa_attn_bwd_walks if D == 128 else load().nsa_attn_bwd_walks_d64
-        walks = walks_of(B, T, S, Hq, Hkv, int(causal), window, kp_stride)
-        if walks > 1:
-            part = _empty(walks, 2, k.numel(), dtype=torch.float32, device=q.device)
-    else:
-        idx, nS = tiles[4], tiles[5]
-        visits = int(os.environ.get('NSA_B200_KV_VISITS_SEL', '64'))
-        inv = inverse_blocks(idx, nS, 128 // (Hq // Hkv), visits)
-    _check(load().nsa_attn_bwd_split(_p(q), _p(k), _p(v), _p(o), _p(do), _p(L), _p(delta), _p(dq), _p(dk), _p(dv),
-                                     B, T, S, Hq, Hkv, D, scale,
-                                     int(causal), window, kp_stride, kp_off,
-                                     _p(tb), _p(tm), _p(tc), mu, _p(inv[0]), _p(inv[1]), _p(inv[2]),
-                                     inv[3], inv[4], visits, _p(part), walks, int(given), int(add_dq),
-                                     _stream()))
-
-
-def _kv_visits() -> int:
-    """Query tiles per CTA of the dK / dV kernel over a contiguous key range, where a key block has more than 256."""
-    return int(os.environ.get('NSA_B200_KV_VISITS', '64'))
-
-
 def _bwd_is_split(D: int, G: int, selected: bool) -> bool:
     return os.environ.get("NSA_B200_ATTN_BWD", "split") == "split" and (not selected or (D == 128 and G >= 8))
 
@@ -1078,8 +714,7 @@ class _Attn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, causal, window, scale, kp_stride, kp_off, tiles):
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        o, L = _attn_forward(q, k, v, causal, window, scale, kp_stride, kp_off, tiles)
+        o, L, q, k, v = _h().attn_fwd(q, k, v, causal, window, scale, kp_stride, kp_off, tiles)
         ctx.save_for_backward(q, k, v, o, L)
         ctx.cfg = (causal, window, scale, kp_stride, kp_off)
         ctx.tiles = tiles
@@ -1089,23 +724,16 @@ class _Attn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do, _dL):
         q, k, v, o, L = ctx.saved_tensors
-        causal, window, scale, kp_stride, kp_off = ctx.cfg
+        (causal, window, _, kp_stride, _), tiles, lists, walks = ctx.cfg, ctx.tiles, None, 0
         B, T, Hq, D = q.shape
         S, Hkv = k.shape[1], k.shape[2]
-        do = do.contiguous()
-        dq = _empty_like(q)
-        dk = _zeros(k.shape, dtype=torch.float32, device=q.device)
-        dv = _zeros(v.shape, dtype=torch.float32, device=q.device)
-        if _bwd_is_split(D, Hq // Hkv, ctx.tiles is not None):
-            _attn_backward_split(q, k, v, o, do, L, dq, dk, dv, *ctx.cfg, ctx.tiles)
-        else:
-            tb, tm, tc, mu = ctx.tiles[:4] if ctx.tiles is not None else (None, None, None, 0)
-            delta = _empty(B, T, Hq, dtype=torch.float32, device=q.device)
-            _check(load().nsa_attn_bwd(_p(q), _p(k), _p(v), _p(o), _p(do), _p(L), _p(delta), _p(dq), _p(dk), _p(dv),
-                                       B, T, S, Hq, Hkv, D, scale,
-                                       int(causal), window, kp_stride, kp_off,
-                                       _p(tb), _p(tm), _p(tc), mu, _stream()))
-        return dq, dk.to(k.dtype), dv.to(v.dtype), None, None, None, None, None, None
+        split = _bwd_is_split(D, Hq // Hkv, tiles is not None)
+        if split and tiles is None:
+            walks_of = load().nsa_attn_bwd_walks if D == 128 else load().nsa_attn_bwd_walks_d64
+            walks = walks_of(B, T, S, Hq, Hkv, int(causal), window, kp_stride)
+        elif split:
+            lists = inverse_blocks(tiles[4], tiles[5], 128 // (Hq // Hkv), int(os.environ.get("NSA_B200_KV_VISITS_SEL", "64")))
+        return (*_host.attn_bwd(q, k, v, o, do, L, *ctx.cfg, tiles, lists, walks, split), None, None, None, None, None, None)
 
 
 def _attn_ok(q, k) -> bool:
@@ -1125,17 +753,8 @@ def attention(q, k, v, causal=True, window=0, scale=None):
 def union_blocks(idx: Tensor, G: int, nS: int):
     """idx (B, Hkv, T, top_n) int32 selection-block ids (-1 = none) -> per query tile
     (128 // G tokens) ascending union list, token bit masks and counts."""
-    B, Hkv, T, top_n = idx.shape
-    R = 128 // G
-    nqt = -(-T // R)
-    max_u = min(R * top_n, nS)
-    max_u += max_u & 1
-    tb = _empty(B, Hkv, nqt, max_u, dtype=torch.int32, device=idx.device)
-    tm = _empty(B, Hkv, nqt, max_u, dtype=torch.int64, device=idx.device)
-    tc = _empty(B, Hkv, nqt, dtype=torch.int32, device=idx.device)
-    _check(load().nsa_union_blocks(_p(idx), _p(tb), _p(tm), _p(tc), B, T, Hkv, G,
-                                   top_n, nS, max_u, _stream()))
-    return tb, tm, tc, max_u
+    tb, tm, tc = _h().union_blocks(idx, G, nS)
+    return tb, tm, tc, tb.shape[-1]
 
 
 def inverse_blocks(idx: Tensor, nS: int, R: int, visits_per_cta: int):
@@ -1144,18 +763,8 @@ def inverse_blocks(idx: Tensor, nS: int, R: int, visits_per_cta: int):
     B, Hkv, T, n = idx.shape
     if not idx.is_cuda or nS > 12288 or n > 32:
         return _inverse_blocks_torch(idx, nS, R, visits_per_cta)
-    dev = idx.device
-    idx = idx.to(torch.int32).contiguous()
-    lists = B * Hkv * nS
-    chunks = load().nsa_inverse_chunks(B * Hkv, T, nS)
-    tok = _empty(B * Hkv * T * n, dtype=torch.int32, device=dev)
-    list_start = _empty(lists + 1, dtype=torch.int32, device=dev)
-    item_start = _empty(lists + 1, dtype=torch.int32, device=dev)
-    hist = _empty(B * Hkv * chunks * nS, dtype=torch.int32, device=dev)
-    count = _empty(lists, dtype=torch.int32, device=dev)
-    _check(load().nsa_inverse_blocks(_p(idx), _p(tok), _p(list_start), _p(item_start), _p(hist), _p(count), B * Hkv,
-                                     T, n, nS, R, visits_per_cta, _stream()))
-    bound = (B * Hkv * T * n) // (R * visits_per_cta) + lists
+    tok, list_start, item_start = _h().inverse_blocks(idx, nS, R, visits_per_cta)
+    bound = (B * Hkv * T * n) // (R * visits_per_cta) + B * Hkv * nS
     return tok, list_start, item_start, nS, bound
 
 
@@ -1211,13 +820,7 @@ def nsa_attention_indexed(q, k, v, idx, g_slc, g_swa, sel_block=64, window=512, 
 
 
 def nsa_importance(q, k_cmp, L_cmp, nS, stride, block, scale):
-    B, T, Hq, D = q.shape
-    Hkv = k_cmp.shape[2]
-    imp = _zeros(B, Hkv, T, nS, dtype=torch.float32, device=q.device)
-    _check(load().nsa_attn_importance(_p(q.contiguous()), _p(k_cmp.contiguous()), _p(L_cmp), _p(imp), B, T,
-                                      k_cmp.shape[1], Hq, Hkv, D, scale,
-                                      stride, block - 1, nS, _stream()))
-    return imp
+    return _h().importance(q, k_cmp, L_cmp, nS, stride, block, scale)
 
 
 def nsa_select(imp: Tensor, sel_block: int, top_n: int) -> Tensor:
@@ -1226,11 +829,7 @@ def nsa_select(imp: Tensor, sel_block: int, top_n: int) -> Tensor:
     are visible.  One warp per row (``nsa_select_kernel``); more than 2048 blocks use torch.topk."""
     B, H, T, nS = imp.shape
     if imp.is_cuda and nS <= 2048 and imp.dtype == torch.float32:
-        imp = imp.contiguous()
-        idx = _empty(B, H, T, top_n, dtype=torch.int32, device=imp.device)
-        _check(load().nsa_select_blocks(_p(imp), _p(idx), B * H * T, T, nS, sel_block,
-                                        top_n, _stream()))
-        return idx
+        return _h().select(imp, sel_block, top_n)
     return _nsa_select_torch(imp, sel_block, top_n)
 
 
@@ -1280,31 +879,12 @@ class _GateCombine(torch.autograd.Function):
 def _gate_logits_forward(o1, o2, o3, gates):
     """(combined output, bf16 logits) with the three gates as logits straight from the gate projection: ``gates`` is
     (B, T, 3*Hq) (or wider; columns [0, Hq) compressed, [Hq, 2Hq) selected, [2Hq, 3Hq) window)."""
-    Hq, D = o1.shape[-2], o1.shape[-1]
-    gl = gates.to(torch.bfloat16)
-    if gl.stride(-1) != 1 or not gl.is_contiguous():
-        gl = gl.contiguous()
-    g0, step = gl.data_ptr(), Hq * gl.element_size()
-    o = _empty_like(o1)
-    _check(load().nsa_gate_combine_fwd_ex(_p(o1), _p(o2), _p(o3), g0, g0 + step, g0 + 2 * step,
-                                          gl.shape[-1], Hq, 1, _p(o), o1.numel() // D, D,
-                                          _stream()))
-    return o, gl
+    return _h().gates_fwd(o1, o2, o3, gates)
 
 
 def _gate_logits_backward(o1, o2, o3, gl, do, sums=(None, None, None)):
     """(do1, do2, do3, d logits); ``sums``, three fp32 tensors of one value per row, receive rowsum(do_i * o_i)."""
-    do = do.contiguous()
-    Hq, D, ldg = o1.shape[-2], o1.shape[-1], gl.shape[-1]
-    step = Hq * gl.element_size()
-    d1, d2, d3 = _empty_like(o1), _empty_like(o1), _empty_like(o1)
-    dgl = _zeros_like(gl) if ldg > 3 * Hq else _empty_like(gl)
-    g0, dg0 = gl.data_ptr(), dgl.data_ptr()
-    _check(load().nsa_gate_combine_bwd_ex(_p(o1), _p(o2), _p(o3), g0, g0 + step, g0 + 2 * step,
-                                          ldg, Hq, 1, _p(do), _p(d1), _p(d2), _p(d3), dg0,
-                                          dg0 + step, dg0 + 2 * step, _p(sums[0]), _p(sums[1]), _p(sums[2]),
-                                          o1.numel() // D, D, _stream()))
-    return d1, d2, d3, dgl
+    return _h().gates_bwd(o1, o2, o3, gl, do, *sums)
 
 
 class _GateCombineLogits(torch.autograd.Function):
@@ -1339,11 +919,11 @@ class _NSA(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, kc, vc, gates, stride, block, sel_block, top_n, window, scale):
-        q, k, v, kc, vc = (t.contiguous() for t in (q, k, v, kc, vc))
-        o1, L1 = _attn_forward(q, kc, vc, True, 0, scale, stride, block - 1, None)
+        h = _h()
+        o1, L1, q, kc, vc = h.attn_fwd(q, kc, vc, True, 0, scale, stride, block - 1, None)
         tiles = _nsa_select_tiles(q, kc, L1, -(-q.shape[1] // sel_block), stride, block, sel_block, top_n, scale)
-        o2, L2 = _attn_forward(q, k, v, True, 0, scale, 1, 0, tiles)
-        o3, L3 = _attn_forward(q, k, v, True, window, scale, 1, 0, None)
+        o2, L2, _, k, v = h.attn_fwd(q, k, v, True, 0, scale, 1, 0, tiles)
+        o3, L3, *_ = h.attn_fwd(q, k, v, True, window, scale, 1, 0, None)
         o, gl = _gate_logits_forward(o1, o2, o3, gates)
         ctx.save_for_backward(q, k, v, kc, vc, gl, o1, o2, o3, L1, L2, L3)
         ctx.cfg, ctx.tiles, ctx.gdtype = (stride, block, window, scale), tiles, gates.dtype
@@ -1352,24 +932,10 @@ class _NSA(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do):
         q, k, v, kc, vc, gl, o1, o2, o3, L1, L2, L3 = ctx.saved_tensors
-        lib = load()
-        stride, block, window, scale = ctx.cfg
-        f32 = torch.float32
-        sums = [_empty_like(L1) for _ in range(3)]
-        d1, d2, d3, dgl = _gate_logits_backward(o1, o2, o3, gl, do, sums)
-        dq = _empty_like(q)
-        dkc, dvc, dk, dv = (_zeros(t.shape, dtype=f32, device=q.device) for t in (kc, vc, k, v))
-        _attn_backward_split(q, kc, vc, o1, d1, L1, dq, dkc, dvc, True, 0, scale, stride, block - 1, None, sums[0])
-        _attn_backward_split(q, k, v, o2, d2, L2, dq, dk, dv, True, 0, scale, 1, 0, ctx.tiles, sums[1], True)
-        # The window branch shares dk / dv while a key block's gradients get one addition from it: one more to what is there gives
-        # the same bits on every run, two in either order would not.
-        shared = lib.nsa_attn_bwd_walks(*q.shape[:2], k.shape[1], q.shape[2], k.shape[2], 1, window, 1) != 0
-        dk3, dv3 = (dk, dv) if shared else (_zeros(t.shape, dtype=f32, device=q.device) for t in (k, v))
-        _attn_backward_split(q, k, v, o3, d3, L3, dq, dk3, dv3, True, window, scale, 1, 0, None, sums[2], True)
-        if not shared:
-            dk, dv = dk + dk3, dv + dv3
-        return (dq, dk.to(k.dtype), dv.to(v.dtype), dkc.to(kc.dtype), dvc.to(vc.dtype), dgl.to(ctx.gdtype),
-                None, None, None, None, None, None)
+        e1, e2, e3 = (_empty_like(L1) for _ in range(3))
+        d1, d2, d3, dgl = _gate_logits_backward(o1, o2, o3, gl, do, (e1, e2, e3))
+        grads = _host.nsa_bwd(q, k, v, kc, vc, o1, d1, L1, e1, o2, d2, L2, e2, o3, d3, L3, e3, ctx.tiles, *ctx.cfg)
+        return (*grads, dgl.to(ctx.gdtype), None, None, None, None, None, None)
 
 
 class _Pool(torch.autograd.Function):
@@ -1379,26 +945,12 @@ class _Pool(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, block, stride):
-        B, T, H, D = x.shape
-        width = H * D
-        ok = (x.stride(3) == 1 and x.stride(2) == D and x.stride(1) % 8 == 0 and x.stride(0) == T * x.stride(1)
-              and x.data_ptr() % 16 == 0)
-        xv = x if ok else x.contiguous()
-        nC = (T - block) // stride + 1
-        y = _empty(B, nC, H, D, dtype=x.dtype, device=x.device)
-        _check(load().nsa_pool_fwd(_p(xv), _p(y), B, T, width, xv.stride(1), block,
-                                   stride, _stream()))
-        ctx.shape, ctx.block, ctx.stride = (B, T, H, D), block, stride
-        return y
+        ctx.cfg = x.shape[1], block, stride
+        return _h().pool_fwd(x, block, stride)
 
     @staticmethod
     def backward(ctx, dy):
-        B, T, H, D = ctx.shape
-        dy = dy.contiguous()
-        dx = _empty(B, T, H, D, dtype=dy.dtype, device=dy.device)
-        _check(load().nsa_pool_bwd(_p(dy), _p(dx), B, T, H * D, ctx.block, ctx.stride,
-                                   _stream()))
-        return dx, None, None
+        return _host.pool_bwd(dy, *ctx.cfg), None, None
 
 
 def nsa_compress(x, block, stride):
@@ -1472,98 +1024,20 @@ class _SSDStatePass(torch.autograd.Function):
         return dS, dgamma
 
 
-def _token_view(t: Tensor, inner: int):
-    """(B, T, ..., inner-contiguous) view -> (tensor, token stride in elements) usable by a TMA
-    map with rows = tokens; copies when the view is not row-strided."""
-    B, T = t.shape[0], t.shape[1]
-    width = t[0, 0].numel()
-    ok = (t.stride(-1) == 1 and t.stride(0) == T * t.stride(1) and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0
-          and t[0, 0].is_contiguous())
-    if not ok:
-        t = t.contiguous()
-    return t, t.stride(1) if ok else width
-
-
 class _SSD(torch.autograd.Function):
     """Mamba-2 SSD through the tcgen05 chunk kernels of ``csrc/ssd.cu`` (chunk 128, d_state 128,
     headdim 64, one B/C group)."""
 
     @staticmethod
     def forward(ctx, x, dt, A, Bm, Cm, D):
-        Bsz, T, H, P = x.shape
-        N = Bm.shape[-1]
-        nc = -(-T // 128)
-        x, ldx = _token_view(x, P)
-        Bm, ldb = _token_view(Bm, N)
-        Cm, ldc = _token_view(Cm, N)
-        dt = dt.float().contiguous()
-        A = A.float().contiguous()
-        Df = None if D is None else D.float().contiguous()
-        dev = x.device
-        lib = load()
-        Hb, gamma = _SSD.states(lib, False, Bm, ldb, x, ldx, dt, A, None)
-        y = _empty(Bsz, T, H, P, dtype=torch.bfloat16, device=dev)
-        _check(lib.nsa_ssd_chunk_out(_p(Cm), ldc, _p(Bm), ldb, _p(x), ldx, _p(Hb), _p(dt), _p(A),
-                                     _p(Df), _p(y), Bsz, T, H, N, P, _stream()))
-        ctx.save_for_backward(x, dt, A, Bm, Cm, Df if Df is not None else _empty(0, device=dev), gamma, Hb)
+        y, *kept = _h().ssd_fwd(x, dt, A, Bm, Cm, D)
+        ctx.save_for_backward(*kept)
         ctx.has_D = D is not None
         return y
 
     @staticmethod
-    def states(lib, back, rows, ld_rows, v, ld_v, dt, A, gamma):
-        """bf16 states entering the chunks (back: gradients of those leaving them), and the chunks' decays where the two-kernel
-        form needs them."""
-        Bsz, T, H, P = v.shape
-        N, nc, dev = rows.shape[-1], -(-T // 128), v.device
-        dims = (Bsz, T, H, N, P, _stream())
-        out = _empty(Bsz, nc, H, N, P, dtype=torch.bfloat16, device=dev)
-        if lib.nsa_ssd_states_in_one(Bsz, T, H):
-            _check(lib.nsa_ssd_states(back, _p(rows), ld_rows, _p(v), ld_v, _p(dt), _p(A), _p(out), *dims))
-            return out, _empty(0, device=dev)
-        if not back:
-            gamma = _empty(Bsz, nc, H, dtype=torch.float32, device=dev)
-        local = _empty(Bsz, nc, H, N, P, dtype=torch.float32, device=dev)
-        _check(lib.nsa_ssd_chunk_state(back, _p(rows), ld_rows, _p(v), ld_v, _p(dt), _p(A), _p(local),
-                                       None if back else _p(gamma), *dims))
-        if back:
-            _check(lib.nsa_ssd_state_bwd(_p(local), _p(gamma), None, _p(out), Bsz, nc, H, N * P,
-                                         _stream()))
-        else:
-            _check(lib.nsa_ssd_state_fwd(_p(local), _p(gamma), None, _p(out), None, Bsz, nc, H,
-                                         N * P, _stream()))
-        return out, gamma
-
-    @staticmethod
     def backward(ctx, dy):
-        x, dt, A, Bm, Cm, Df, gamma, Hb = ctx.saved_tensors
-        ldx, ldb, ldc = (_row_pitch(t.flatten(2)) for t in (x, Bm, Cm))
-        Df = Df if ctx.has_D else None
-        Bsz, T, H, P = x.shape
-        N = Bm.shape[-1]
-        nc = Hb.shape[1]
-        dev = x.device
-        dy = dy.contiguous()
-        lib = load()
-        dHn, _ = _SSD.states(lib, True, Cm, ldc, dy, H * P, dt, A, gamma)
-        dx = _empty(Bsz, T, H, P, dtype=torch.bfloat16, device=dev)
-        # dB / dC: fp32 sums over the heads that one CTA has of a chunk, added up afterwards
-        slots = lib.nsa_ssd_grad_slots(Bsz, T, H)
-        dB_part, dC_part = (_empty(Bsz, T, slots, N, dtype=torch.float32, device=dev) for _ in range(2))
-        q = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
-        k = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
-        rdx = _empty(Bsz, T, H, dtype=torch.float32, device=dev) if ctx.has_D else None
-        _check(lib.nsa_ssd_chunk_grad(_p(Cm), ldc, _p(Bm), ldb, _p(x), ldx, _p(dy), _p(Hb), _p(dHn), _p(dt),
-                                      _p(A), _p(Df), _p(dx), _p(dB_part), _p(dC_part), _p(q), _p(k), _p(rdx), Bsz, T,
-                                      H, N, P, _stream()))
-        # d(cum_t) = dy_t.(y_t - D x_t) - x_t.dx_t ;  a_k = dt_k A enters every cum_t with t >= k
-        dB, dC = (_empty(Bsz, T, 1, N, dtype=torch.bfloat16, device=dev) for _ in range(2))
-        ddt = _empty(Bsz, T, H, dtype=torch.float32, device=dev)
-        dA = _empty(H, dtype=torch.float32, device=dev)
-        dD = _empty(H, dtype=torch.float32, device=dev) if ctx.has_D else None
-        scratch = _empty(3 * Bsz * nc * H, dtype=torch.float32, device=dev)
-        _check(lib.nsa_ssd_finish(_p(dB_part), _p(dC_part), _p(q), _p(k), _p(rdx), _p(dt), _p(A), _p(scratch), _p(dB), _p(dC), _p(ddt),
-                                  _p(dA), _p(dD), Bsz, T, H, _stream()))
-        return dx, ddt, dA, dB, dC, dD
+        return _host.ssd_bwd(*ctx.saved_tensors, dy, ctx.has_D)
 
 
 def copy_columns(dst: Tensor, src: Tensor) -> bool:

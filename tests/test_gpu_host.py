@@ -1,0 +1,66 @@
+"""The ops' host side: guard zones around every output, forward and backward, several threads on streams of their own, and shapes that are
+refused before anything is launched."""
+import threading
+
+import pytest
+import torch
+from test_gpu_unrecorded import _cases
+
+pytestmark = pytest.mark.gpu
+
+
+def _results(op, inputs):
+    leaves = [t.detach().clone().requires_grad_() for t in inputs]
+    y = op(*leaves)
+    ys = y if isinstance(y, tuple) else (y,)
+    return [t.detach() for t in ys] + list(torch.autograd.grad(ys, leaves, [torch.ones_like(t) for t in ys]))
+
+
+def test_guard_zones_give_the_same_bits(native, monkeypatch):
+    cases = _cases(native)
+    want = {name: _results(op, inputs) for name, (op, *inputs) in cases.items()}
+    monkeypatch.setattr(native, "_CANARY", True)
+    for name, (op, *inputs) in cases.items():
+        native._guards.clear()
+        got = _results(op, inputs)
+        assert len(native._guards) >= len(got) and native.check_canaries() > 0, name
+        assert all(torch.equal(a, b) for a, b in zip(got, want[name])), name
+
+
+def test_threads(native):
+    cases = _cases(native)
+    want = {name: _results(op, inputs) for name, (op, *inputs) in cases.items()}
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work():
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            for _ in range(3):
+                for name, (op, *inputs) in cases.items():
+                    got = _results(op, inputs)
+                    stream.synchronize()
+                    if not all(torch.equal(a, b) for a, b in zip(got, want[name])):
+                        wrong.append(name)
+
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
+def test_refused_shapes(native):
+    r = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)                # noqa: E731
+    f = torch.zeros(8, 32, device="cuda")
+    for call in (lambda: native.causal_conv1d(r(1, 1, 8, 64), r(64, 4), None), lambda: native.rope(r(1, 8, 2, 1, 64), f, f),
+                 lambda: native.linear_cross_entropy(r(1, 8, 64), r(64, 64), torch.zeros(8, device="cuda", dtype=torch.long)),
+                 lambda: native.attention(r(1, 8, 2, 64, 1), r(1, 8, 2, 64), r(1, 8, 2, 64)), lambda: native.nsa_compress(r(1, 64, 2, 8, 8), 32, 16),
+                 lambda: native.ssd_scan(r(1, 1, 8, 2, 64), f, f, r(1, 8, 1, 128), r(1, 8, 1, 128)),
+                 lambda: native.gemm(r(8, 64), r(8, 32), False, False),
+                 lambda: native.adamw_multi([(r(8), r(8), f[0, :8], f[0, :4], None, None)], 1, 1e-3, .9, .95, 1e-8, 0.0, None)):
+        before = native.launch_count()
+        with pytest.raises((ValueError, IndexError, RuntimeError)):
+            call()
+        assert native.launch_count() == before
