@@ -3251,50 +3251,66 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const bf16* __restrict_
 // Inverse of the selection map: for every (batch, kv head, block) the ascending list of tokens that
 // selected the block (what the key-stationary dK/dV pass walks).  Counting, scanning and filling,
 // with no sort and no atomics on global memory, so the lists are the same on every run:
-//   1. one warp per (b*h, chunk of tokens) builds the chunk's histogram over blocks;
+//   1. one CTA per (b*h, chunk of tokens) builds the chunk's histogram over blocks;
 //   2. per list, an exclusive scan of the histograms along the chunks gives each chunk's offset
 //      inside the list, and the total gives the list's length;
 //   3. one thread block scans the lengths into list starts (and the CTA counts per list);
-//   4. the warps of step 1 walk their tokens again in the same order and write them.
+//   4. the CTAs of step 1 go through their tokens again and write them.
 // An entry is dropped if it is negative, out of range or repeats an earlier entry of the same token.
 // --------------------------------------------------------------------------------------
-// A walk is one warp stepping through its tokens, so short chunks are what spreads it over the GPU (chunks of 256 left 128 warps
-// for 16384 tokens x 2 heads and took 106 us per walk).  The histograms, one row of counts per chunk, pass through memory four
-// times; beyond 25 MB long chunks are the faster ones (100000 tokens, 1563 blocks: x 2 heads, 20 MB with chunks of 64, 235 us and
-// 265 with 256; x 4 heads 404 and 312; 131072 tokens x 8 heads 2045 and 886).
+// The histograms, one row of counts per chunk, pass through memory four times; beyond 25 MB long chunks are the faster ones (step 2
+// alone: 100000 tokens, 1563 blocks, 2 heads, 20 MB with chunks of 64, 100 us; 4 heads with chunks of 256 19 us).
 inline int inverse_chunk(int BH, int T, int nS) { return static_cast<long>(BH) * ((T + 63) / 64) * nS <= 6l << 20 ? 64 : 256; }
 
-// mode 0: hist[(bh * chunks + chunk) * nS + blk] = entries of the chunk; mode 1: fill tok_list.
-// The warp takes the chunk's tokens one after the other, lane j looking at entry j of the token's
-// list (n <= 32): a token's valid entries name distinct blocks, so the lanes touch distinct counters,
-// and tokens reach every list in ascending order.
-__global__ void __launch_bounds__(32) nsa_inverse_walk_kernel(const int* __restrict__ idx, int* __restrict__ hist,
-                                                              const int* __restrict__ chunk_off,
-                                                              const int* __restrict__ list_start, int* __restrict__ tok_list,
-                                                              int T, int n, int nS, int chunks, int len, int mode) {
-  extern __shared__ int bins[];                   // nS running counts of this chunk
-  const int chunk = blockIdx.x, lane = threadIdx.x;
-  const long bh = blockIdx.y;
-  for (int i = lane; i < nS; i += 32) bins[i] = 0;
-  __syncwarp();
-  const long slot = (bh * chunks + chunk) * nS;
+// mode 0: hist[(bh * chunks + chunk) * nS + blk] = tokens of the chunk that selected the block; mode 1: fill tok_list.
+// 64 tokens at a time are one word of bits per block, set by all threads at once: a repeat of an entry sets the same bit, and a
+// token's place in a list is the number of bits below its own.  (One warp stepping through its tokens was bound by the latency of a
+// step, 0.4 us: both walks of 16384 tokens x 2 heads 52 us, now 8.8; 1111 tokens 46, 5.4; 131072 x 8 heads 832, 197.)
+constexpr int WALK_THREADS = 256;
+__global__ void __launch_bounds__(WALK_THREADS) nsa_inverse_walk_kernel(const int* __restrict__ idx, int* __restrict__ hist,
+                                                                        const int* __restrict__ chunk_off,
+                                                                        const int* __restrict__ list_start, int* __restrict__ tok_list,
+                                                                        int T, int n, int nS, int chunks, int len, int mode) {
+  extern __shared__ unsigned long long chosen[];  // [nS] tokens of these 64 that chose the block
+  int* before = reinterpret_cast<int*>(chosen + nS);   // [nS] tokens of the chunk's 64s before that did
+  constexpr int PER = 64 / (WALK_THREADS / 32);   // a warp takes every eighth token, lane j its entry j (n <= 32)
+  const int chunk = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+  const long bh = blockIdx.y, slot = (bh * chunks + chunk) * nS;
   const int t_end = min(T, (chunk + 1) * len);
-  int v_next = (lane < n && chunk * len < t_end) ? idx[(bh * T + chunk * len) * n + lane] : -1;
-  for (int t = chunk * len; t < t_end; ++t) {
-    const int v = v_next;
-    if (t + 1 < t_end && lane < n) v_next = idx[(bh * T + t + 1) * n + lane];      // next token's entry, ahead of use
-    const bool in_range = lane < n && v >= 0 && v < nS;
-    const unsigned same = __match_any_sync(0xffffffffu, in_range ? v : -1 - lane);
-    const bool first = (same & ((1u << lane) - 1u)) == 0u;                          // not a repeat of an earlier entry
-    if (in_range && first) {
-      const int before = bins[v];
-      if (mode == 1) tok_list[list_start[bh * nS + v] + chunk_off[slot + v] + before] = t;
-      bins[v] = before + 1;
+  for (int i = tid; i < nS; i += WALK_THREADS) { chosen[i] = 0ull; before[i] = 0; }
+  __syncthreads();
+  for (int t0 = chunk * len; t0 < t_end; t0 += 64) {
+    const int tokens = min(64, t_end - t0);
+    const int* mine = idx + (bh * T + t0) * n;
+    int v[PER], at[PER];                          // this thread's entries, all loads in flight at once
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const int t = tid / 32 + k * (WALK_THREADS / 32);
+      v[k] = lane < n && t < tokens ? mine[t * n + lane] : -1;
+      if (v[k] >= nS) v[k] = -1;
     }
-    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+      if (v[k] >= 0) {
+        const int t = tid / 32 + k * (WALK_THREADS / 32);
+        atomicOr(reinterpret_cast<unsigned*>(chosen + v[k]) + t / 32, 1u << (t & 31));   // (64 bits at once are a loop of exchanges: 7 us more)
+        if (mode == 1) at[k] = list_start[bh * nS + v[k]] + chunk_off[slot + v[k]];
+      }
+    __syncthreads();
+    if (mode == 1) {
+#pragma unroll
+      for (int k = 0; k < PER; ++k)
+        if (v[k] >= 0) {
+          const int t = tid / 32 + k * (WALK_THREADS / 32);
+          tok_list[at[k] + before[v[k]] + __popcll(chosen[v[k]] & ((1ull << t) - 1ull))] = t0 + t;
+        }
+      __syncthreads();
+    }
+    for (int i = tid; i < nS; i += WALK_THREADS) { before[i] += __popcll(chosen[i]); chosen[i] = 0ull; }
+    __syncthreads();
   }
   if (mode == 0)
-    for (int i = lane; i < nS; i += 32) hist[slot + i] = bins[i];
+    for (int i = tid; i < nS; i += WALK_THREADS) hist[slot + i] = before[i];
 }
 
 // offsets of the chunks inside each list (in place over hist) and the list's length
@@ -3817,10 +3833,13 @@ extern "C" int nsa_inverse_blocks(const int* idx, int* tok_list, int* list_start
   const int len = inverse_chunk(BH, T, nS), chunks = nsa_inverse_chunks(BH, T, nS);
   const long lists = static_cast<long>(BH) * nS;
   const dim3 grid(chunks, BH);
-  nsa_inverse_walk_kernel<<<grid, 32, nS * 4, st>>>(idx, hist, nullptr, nullptr, nullptr, T, n, nS, chunks, len, 0);
+  const int bytes = nS * 12;
+  if (bytes > 48 * 1024)
+    if (int rc = set_smem(nsa_inverse_walk_kernel, bytes)) return rc;
+  nsa_inverse_walk_kernel<<<grid, WALK_THREADS, bytes, st>>>(idx, hist, nullptr, nullptr, nullptr, T, n, nS, chunks, len, 0);
   nsa_inverse_offsets_kernel<<<(unsigned)((lists + 31) / 32), 256, 0, st>>>(hist, count, lists, nS, chunks);
   nsa_inverse_scan_kernel<<<1, 1024, 0, st>>>(count, list_start, item_start, lists, R, visits_per_cta);
-  nsa_inverse_walk_kernel<<<grid, 32, nS * 4, st>>>(idx, nullptr, hist, list_start, tok_list, T, n, nS, chunks, len, 1);
+  nsa_inverse_walk_kernel<<<grid, WALK_THREADS, bytes, st>>>(idx, nullptr, hist, list_start, tok_list, T, n, nS, chunks, len, 1);
   nsa::count_launch(4);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_inverse_blocks launch");
