@@ -641,17 +641,15 @@ __global__ void __launch_bounds__(256) rope_kernel(const bf16* __restrict__ x, c
 // accesses, a warp covers 256 contiguous bytes of a row) and walks `rows` consecutive time steps
 // with the last three rows in registers, so every element is read and widened once.  The rows ahead
 // travel through a ring of shared memory that a lane fills (cp.async) and reads for itself alone: no barriers,
-// and 12 rows of a warp stay in flight without holding registers.  The taps are packed fp32 FMAs (two channels per
-// instruction).  A CTA is CW channel tiles by 8 / CW time segments: four tiles (1 KB of a row) where there are as many, one or
-// two for tensors of up to 128 or 256 channels, whose warps would otherwise have nothing to do (524288 x 128,
-// forward and backward: 565 us with six idle warps in eight, 181 now).
+// and 8 rows of a warp stay in flight without holding registers.  Taps, sigmoid and derivative are packed fp32 operations (two
+// channels per instruction); groups of rows wholly inside a segment go without a test per row, and addresses are stepped, not formed
+// (16384 x 4352, bias and SiLU: forward 64 -> 58 us, 4.9 TB/s, backward 126 -> 105, 4.1 TB/s; 150 instructions a row and warp there,
+// now 106, and half of the issue slots: 128 registers leave four warps to a scheduler.  Group-wise order of the steps: 111.  Longer or
+// shorter segments and three CTAs per SM with spills: 111, 121, 252).  A CTA is CW channel tiles by 8 / CW time segments: two tiles, or one
+// for tensors of up to 128 channels, whose warps would otherwise have nothing to do (four tiles: 108; 4352 channels are 34).
 // ------------------------------------------------------------------------------------
-constexpr int CT_WARPS = 8, CT_C = 128, CT_U = 4, CT_RING = 4;
+constexpr int CT_WARPS = 8, CT_C = 128, CT_U = 4, CT_RING = 3;
 
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pred) {   // zero fill when !pred
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gmem), "r"(pred ? 8 : 0) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -689,8 +687,49 @@ __device__ __forceinline__ void conv_taps(const bf16* __restrict__ w, const bf16
   bv = Quad{make_float2(s[0], s[1]), make_float2(s[2], s[3])};
 }
 
+// Two lanes of silu and of its derivative; the exponential and the reciprocal are the scalar functions'.
+__device__ __forceinline__ float2 sigmoid2(const float2& x) {
+  const float2 e = mul2(x, make_float2(-1.4426950408889634f, -1.4426950408889634f));
+  const float2 d = fma2(make_float2(exp2f(e.x), exp2f(e.y)), make_float2(1.f, 1.f), make_float2(1.f, 1.f));
+  return make_float2(__fdividef(1.f, d.x), __fdividef(1.f, d.y));
+}
+__device__ __forceinline__ float2 silu2(const float2& x) { return mul2(x, sigmoid2(x)); }
+__device__ __forceinline__ float2 dsilu2(const float2& x) {
+  const float2 s = sigmoid2(x), one = make_float2(1.f, 1.f);
+  return mul2(s, fma2(x, fma2(s, make_float2(-1.f, -1.f), one), one));
+}
+
+// Copies groups of CT_U rows of a lane's four channels into its ring, one after the other; rows past `rows` read as zero.
+struct ConvFeed {
+  const bf16 *src, *base;
+  long pitch;
+  int left, slot = 0;
+  uint32_t ring;
+  __device__ __forceinline__ ConvFeed(const bf16* p, long pitch, int rows, uint2* ring)
+      : src(p), base(p), pitch(pitch), left(rows), ring(static_cast<uint32_t>(__cvta_generic_to_shared(ring))) {}
+  __device__ __forceinline__ void next(bool commit = true) {
+    const uint32_t d = ring + slot * (CT_U * 32 * 8);
+    if (left >= CT_U) {
+#pragma unroll
+      for (int u = 0; u < CT_U; ++u) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + u * 256), "l"(src) : "memory");
+        src += pitch;
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < CT_U; ++u) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + u * 256), "l"(u < left ? src : base), "r"(u < left ? 8 : 0) : "memory");
+        src += pitch;
+      }
+    }
+    left -= CT_U;
+    slot = (slot + 1) % CT_RING;
+    if (commit) cp_async_commit();
+  }
+};
+
 template <int CW>
-__global__ void __launch_bounds__(CT_WARPS * 32, 4) conv1d_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
+__global__ void __launch_bounds__(CT_WARPS * 32, 3) conv1d_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                                       const bf16* __restrict__ bias, bf16* __restrict__ y,
                                                                       int T, int C, long ldx, int act, int rows) {
   __shared__ uint2 ring_all[CT_WARPS][CT_RING * CT_U][32];
@@ -698,40 +737,37 @@ __global__ void __launch_bounds__(CT_WARPS * 32, 4) conv1d_fwd_kernel(const bf16
   const int c = (blockIdx.x * CW + warp % CW) * CT_C + lane * 4;
   const int t0 = (blockIdx.y * (CT_WARPS / CW) + warp / CW) * rows;
   if (c >= C || t0 >= T) return;
-  uint2(*ring)[32] = ring_all[warp];
+  uint2* ring = &ring_all[warp][0][lane];
   const bf16* xp = x + static_cast<long>(blockIdx.z) * T * ldx + c;
   bf16* yp = y + (static_cast<long>(blockIdx.z) * T + t0) * C + c;
   const int n = min(rows, T - t0);                  // rows of this segment
   const bf16* xs = xp + static_cast<long>(t0) * ldx;
-  auto issue = [&](int g) {                         // rows g * CT_U .. of the segment
+  ConvFeed feed(xs, ldx, n, ring);
 #pragma unroll
-    for (int u = 0; u < CT_U; ++u) {
-      const int r = g * CT_U + u;
-      cp_async8(&ring[(g % CT_RING) * CT_U + u][lane], r < n ? xs + r * ldx : xs, r < n);
-    }
-    cp_async_commit();
-  };
-#pragma unroll
-  for (int g = 0; g < CT_RING - 1; ++g) issue(g);
+  for (int g = 0; g < CT_RING - 1; ++g) feed.next();
   auto before = [&](int k) {
     return quad_unpack(t0 >= k ? *reinterpret_cast<const uint2*>(xs - k * ldx) : make_uint2(0u, 0u));
   };
   Quad x0 = before(3), x1 = before(2), x2 = before(1);
   Quad wv[4], bv;
   conv_taps(w, bias, c, true, wv, bv);
-  for (int g = 0; g * CT_U < n; ++g) {
-    issue(g + CT_RING - 1);
+  auto row = [&](int u, int g) {
+    const Quad x3 = quad_unpack(ring[((g % CT_RING) * CT_U + u) * 32]);
+    Quad o = quad_fma(wv[3], x3, quad_fma(wv[2], x2, quad_fma(wv[1], x1, quad_fma(wv[0], x0, bv))));
+    x0 = x1; x1 = x2; x2 = x3;
+    if (act) o = Quad{silu2(o.a), silu2(o.b)};
+    *reinterpret_cast<uint2*>(yp) = quad_pack(o);
+    yp += C;
+  };
+  int g = 0;
+  for (; (g + 1) * CT_U <= n; ++g) {
+    feed.next();
     cp_async_wait<CT_RING - 1>();
 #pragma unroll
-    for (int u = 0; u < CT_U; ++u) {
-      const Quad x3 = quad_unpack(ring[(g % CT_RING) * CT_U + u][lane]);
-      Quad o = quad_fma(wv[3], x3, quad_fma(wv[2], x2, quad_fma(wv[1], x1, quad_fma(wv[0], x0, bv))));
-      x0 = x1; x1 = x2; x2 = x3;
-      if (act) o = Quad{make_float2(silu_f(o.a.x), silu_f(o.a.y)), make_float2(silu_f(o.b.x), silu_f(o.b.y))};
-      if (g * CT_U + u < n) *reinterpret_cast<uint2*>(yp) = quad_pack(o);
-      yp += C;
-    }
+    for (int u = 0; u < CT_U; ++u) row(u, g);
   }
+  cp_async_wait<0>();
+  for (int u = 0; g * CT_U + u < n; ++u) row(u, g);
 }
 
 // Backward: dpre[t] = dy[t] (times SiLU'(pre[t]), pre recomputed from x), dx[s] = sum_j w[j] dpre[s + 3 - j],
@@ -757,23 +793,15 @@ __global__ void __launch_bounds__(CT_WARPS * 32, 2) conv1d_bwd_kernel(const bf16
 #pragma unroll
   for (int j = 0; j < 4; ++j) dw[j] = quad_zero();
   if (c < C && t0 < T) {
-    uint2 (*rx)[32] = sm.x[warp], (*rg)[32] = sm.g[warp];
+    uint2 *rx = &sm.x[warp][0][lane], *rg = &sm.g[warp][0][lane];
     const bf16* xs = x + (static_cast<long>(blockIdx.z) * T + t0) * ldx + c;
     const bf16* gs = dy + (static_cast<long>(blockIdx.z) * T + t0) * C + c;
     bf16* dp = dx + (static_cast<long>(blockIdx.z) * T + t0) * C + c;
     const int n = min(rows, T - t0);             // rows of this segment
     const int ne = min(n + 3, T - t0);           // dpre is needed on [0, ne); rows past T count as zero
-    auto issue = [&](int g) {
+    ConvFeed fx(xs, ldx, ne, rx), fg(gs, C, ne, rg);
 #pragma unroll
-      for (int u = 0; u < CT_U; ++u) {
-        const int r = g * CT_U + u, slot = (g % CT_RING) * CT_U + u;
-        cp_async8(&rx[slot][lane], r < ne ? xs + r * ldx : xs, r < ne);
-        cp_async8(&rg[slot][lane], r < ne ? gs + static_cast<long>(r) * C : gs, r < ne);
-      }
-      cp_async_commit();
-    };
-#pragma unroll
-    for (int g = 0; g < CT_RING - 1; ++g) issue(g);
+    for (int g = 0; g < CT_RING - 1; ++g) { fx.next(false); fg.next(); }
     auto before = [&](int k) {
       return quad_unpack(t0 >= k ? *reinterpret_cast<const uint2*>(xs - k * ldx) : make_uint2(0u, 0u));
     };
@@ -782,35 +810,48 @@ __global__ void __launch_bounds__(CT_WARPS * 32, 2) conv1d_bwd_kernel(const bf16
     conv_taps(w, bias, c, true, wv, bv);
     Quad d0 = quad_zero(), d1 = quad_zero(), d2 = quad_zero();
     dp -= 3L * C;
-    for (int g = 0; g * CT_U < n + 3; ++g) {
-      issue(g + CT_RING - 1);
+    // row u of group g: the gradients of its taps if it is counted here, dx three rows behind if that is in the segment
+    auto row = [&](int u, int g, bool counted, bool behind) {
+      const Quad x3 = quad_unpack(rx[((g % CT_RING) * CT_U + u) * 32]);
+      Quad d3 = quad_unpack(rg[((g % CT_RING) * CT_U + u) * 32]);   // zero past T, and so is dpre
+      if (act) {
+        const Quad p = quad_fma(wv[3], x3, quad_fma(wv[2], x2, quad_fma(wv[1], x1, quad_fma(wv[0], x0, bv))));
+        d3.a = mul2(d3.a, dsilu2(p.a));
+        d3.b = mul2(d3.b, dsilu2(p.b));
+      }
+      if (counted) {
+        dw[0] = quad_fma(d3, x0, dw[0]);
+        dw[1] = quad_fma(d3, x1, dw[1]);
+        dw[2] = quad_fma(d3, x2, dw[2]);
+        dw[3] = quad_fma(d3, x3, dw[3]);
+        db = quad_fma(d3, Quad{make_float2(1.f, 1.f), make_float2(1.f, 1.f)}, db);
+      }
+      if (behind)
+        *reinterpret_cast<uint2*>(dp) =
+            quad_pack(quad_fma(wv[3], d0, quad_fma(wv[2], d1, quad_fma(wv[1], d2, quad_fma(wv[0], d3, quad_zero())))));
+      dp += C;
+      x0 = x1; x1 = x2; x2 = x3;
+      d0 = d1; d1 = d2; d2 = d3;
+    };
+    int g = 0;
+    if (n >= CT_U) {                             // the first group has nothing three rows behind but in its last row
+      fx.next(false); fg.next();
       cp_async_wait<CT_RING - 1>();
 #pragma unroll
-      for (int u = 0; u < CT_U; ++u) {
-        const int r = g * CT_U + u, slot = (g % CT_RING) * CT_U + u;
-        const Quad x3 = quad_unpack(rx[slot][lane]);
-        Quad d3 = quad_unpack(rg[slot][lane]);   // zero past T, and so is dpre
-        if (act) {
-          const Quad p = quad_fma(wv[3], x3, quad_fma(wv[2], x2, quad_fma(wv[1], x1, quad_fma(wv[0], x0, bv))));
-          d3.a.x *= dsilu_f(p.a.x); d3.a.y *= dsilu_f(p.a.y);
-          d3.b.x *= dsilu_f(p.b.x); d3.b.y *= dsilu_f(p.b.y);
-        }
-        if (r < n) {
-          dw[0] = quad_fma(d3, x0, dw[0]);
-          dw[1] = quad_fma(d3, x1, dw[1]);
-          dw[2] = quad_fma(d3, x2, dw[2]);
-          dw[3] = quad_fma(d3, x3, dw[3]);
-          db.a.x += d3.a.x; db.a.y += d3.a.y; db.b.x += d3.b.x; db.b.y += d3.b.y;
-        }
-        if (r >= 3 && r < n + 3)
-          *reinterpret_cast<uint2*>(dp) =
-              quad_pack(quad_fma(wv[3], d0, quad_fma(wv[2], d1, quad_fma(wv[1], d2, quad_fma(wv[0], d3, quad_zero())))));
-        dp += C;
-        x0 = x1; x1 = x2; x2 = x3;
-        d0 = d1; d1 = d2; d2 = d3;
-      }
+      for (int u = 0; u < CT_U; ++u) row(u, 0, true, u >= 3);
+      g = 1;
+    }
+    for (; (g + 1) * CT_U <= n; ++g) {
+      fx.next(false); fg.next();
+      cp_async_wait<CT_RING - 1>();
+#pragma unroll
+      for (int u = 0; u < CT_U; ++u) row(u, g, true, true);
     }
     cp_async_wait<0>();
+    for (int r = g * CT_U; r < n + 3; ++r) {     // at most six rows, all in flight already: three groups are
+      const int at = r / CT_U;
+      row(r - at * CT_U, at, r < n, r >= 3);
+    }
   }
   __syncthreads();                               // the rings become the reduction buffer
   float(*sred)[5][CT_C] = reinterpret_cast<float(*)[5][CT_C]>(conv_smem);
@@ -831,7 +872,7 @@ __global__ void __launch_bounds__(CT_WARPS * 32, 2) conv1d_bwd_kernel(const bf16
 }
 
 // partial [parts][5][C] -> dw (C, 4) and db (C), fp32 or bf16, in a fixed order.  CTA: 32 channels, G groups of parts: 8 warps for
-// the few hundred parts of wide tensors, 32 where few channels leave thousands of parts to few CTAs.
+// a few parts, 32 for more (64 parts of 4352 channels 10.3 -> 4.1 us: the loads of a thread follow one another).
 template <typename OT, int G>
 __global__ void __launch_bounds__(G * 32) conv1d_dw_kernel(const float* __restrict__ partial, int parts, int C,
                                                            OT* __restrict__ dw, OT* __restrict__ db) {
@@ -1246,7 +1287,7 @@ extern "C" int nsa_rope(const void* x, const float* cos_t, const float* sin_t, v
 }
 
 // Channel tiles of a CTA.
-static int conv_tiles(int C) { return C <= CT_C ? 1 : C <= 2 * CT_C ? 2 : 4; }
+static int conv_tiles(int C) { return C <= CT_C ? 1 : 2; }
 // Time steps per warp: 64 keeps the rows read twice (3 of x ahead of a segment, 3 of dpre behind it) under
 // a tenth; short sequences take 32, 16 or 8 so that every SM still finds 32 warps; beyond 8.4 M steps (of two segments
 // a CTA) 128 or 256, so that the grid's second dimension (at most 65535) reaches as far as 33.5 M.
@@ -1269,7 +1310,7 @@ extern "C" int nsa_conv1d_fwd(const void* x, const void* w, const void* bias, vo
 #define NSA_CONV_FWD(CW) \
   conv1d_fwd_kernel<CW><<<grid, CT_WARPS * 32, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)y, T, C, ldx, act, rows)
   const int cw = conv_tiles(C);
-  if (cw == 1) NSA_CONV_FWD(1); else if (cw == 2) NSA_CONV_FWD(2); else NSA_CONV_FWD(4);
+  if (cw == 1) NSA_CONV_FWD(1); else NSA_CONV_FWD(2);
 #undef NSA_CONV_FWD
   nsa::count_launch();
   return 0;
@@ -1286,18 +1327,18 @@ extern "C" int nsa_conv1d_bwd(const void* x, const void* w, const void* bias, co
   const dim3 grid = conv_grid(B, T, C, rows);
   static_assert(sizeof(ConvBwdSmem) >= CT_WARPS * 5 * CT_C * 4, "conv1d: reduction buffer");
   const int cw = conv_tiles(C);
-  auto* kernel = cw == 1 ? conv1d_bwd_kernel<1> : cw == 2 ? conv1d_bwd_kernel<2> : conv1d_bwd_kernel<4>;
-  static bool cfg[3] = {};
-  if (!cfg[cw / 2]) {
+  auto* kernel = cw == 1 ? conv1d_bwd_kernel<1> : conv1d_bwd_kernel<2>;
+  static bool cfg[2] = {};
+  if (!cfg[cw - 1]) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ConvBwdSmem));
     if (e != cudaSuccess) return nsa::fail_cuda(e, "conv1d_bwd: shared memory attribute");
-    cfg[cw / 2] = true;
+    cfg[cw - 1] = true;
   }
   kernel<<<grid, CT_WARPS * 32, sizeof(ConvBwdSmem), st>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (const bf16*)dy, (bf16*)dx,
                                                     partial, T, C, ldx, act, rows);
   const int parts = static_cast<int>(nsa_conv1d_bwd_parts(B, T, C));
 #define NSA_CONV_DW(OT, G) conv1d_dw_kernel<OT, G><<<(C + 31) / 32, G * 32, 0, st>>>(partial, parts, C, (OT*)dw, (OT*)db)
-  if (parts <= 256) { if (dw_fp32) NSA_CONV_DW(float, 8); else NSA_CONV_DW(bf16, 8); }
+  if (parts <= 32) { if (dw_fp32) NSA_CONV_DW(float, 8); else NSA_CONV_DW(bf16, 8); }
   else { if (dw_fp32) NSA_CONV_DW(float, 32); else NSA_CONV_DW(bf16, 32); }
 #undef NSA_CONV_DW
   nsa::count_launch(2);
