@@ -37,7 +37,7 @@ using at::Tensor;
   X(nsa_cross_entropy) X(nsa_scale_bf16) X(nsa_attn_fwd) X(nsa_attn_bwd) X(nsa_attn_bwd_split) X(nsa_attn_bwd_walks)                 \
   X(nsa_attn_importance) X(nsa_union_blocks) X(nsa_inverse_chunks) X(nsa_inverse_blocks) X(nsa_select_blocks)                        \
   X(nsa_gate_combine_fwd_ex) X(nsa_gate_combine_bwd_ex) X(nsa_pool_fwd) X(nsa_pool_bwd) X(nsa_gdn_prep) X(nsa_gdn_seq_fwd)           \
-  X(nsa_gdn_seq_bwd) X(nsa_gdn_post) X(nsa_ssd_states_in_one) X(nsa_ssd_states) X(nsa_ssd_chunk_state) X(nsa_ssd_state_fwd)         \
+  X(nsa_gdn_seq_bwd) X(nsa_gdn_post) X(nsa_ssd_states_form) X(nsa_ssd_states) X(nsa_ssd_chunk_state) X(nsa_ssd_state_fwd)         \
   X(nsa_ssd_state_bwd) X(nsa_ssd_chunk_out) X(nsa_ssd_chunk_grad) X(nsa_ssd_grad_slots) X(nsa_ssd_finish) X(nsa_adamw_multi)         \
   X(nsa_adamw8bit_multi)
 
@@ -913,7 +913,7 @@ std::pair<Tensor, Tensor> ssd_states(bool back, const Tensor& rows, long ld_rows
   const auto dev = v.device();
   const Tensor out = alloc({B, nc, H, N, P}, BF, dev);
   const int b = dim(B), t = dim(T), h = dim(H), n = dim(N), p = dim(P);
-  if (have(lib.nsa_ssd_states_in_one)(b, t, h)) {
+  if (have(lib.nsa_ssd_states_form)(b, t, h)) {
     launch(lib.nsa_ssd_states, static_cast<int>(back), ptr(rows), ld_rows, ptr(v), ld_v, fp(dt), fp(A), ptr(out), b, t, h, n, p);
     return {out, alloc({0}, F32, dev)};
   }

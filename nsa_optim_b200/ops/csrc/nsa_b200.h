@@ -173,6 +173,7 @@ int nsa_ssd_finish(const float* dB_part, const float* dC_part, const float* q, c
     float* dt, const float* A, float* scratch, void* dB, void* dC, float* ddt, float* dA, float* dD, int B, int T, int H,
     cudaStream_t st);
 int nsa_ssd_states_in_one(int B, int T, int H);
+int nsa_ssd_states_form(int B, int T, int H);
 int nsa_ssd_states(int back, const void* bc, long ld_bc, const void* v, long ld_v, const float* dt, const float* A, void*
     out, int B, int T, int H, int N, int P, cudaStream_t st);
 int nsa_ssd_chunk_state(int mode, const void* bc, long ld_bc, const void* v, long ld_v, const float* dt, const float*

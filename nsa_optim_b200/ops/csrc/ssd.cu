@@ -989,39 +989,50 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
 }
 
 // ---------------------------------------------------------------------------------------
-// States entering the chunks (BACK: gradients of the states leaving them) in one pass: one CTA per (head, sequence) walks the
-// chunks, the state in registers; only its bf16 copies reach memory, where chunk_state and the state pass move 20 bytes per element
-// of it.  Eight warps scale a chunk's rows of B (C) in place, eight add the product of the chunk before to the state; the others
-// issue, load with the scan of the step sizes, and store.  (Rows of x are half as many elements, but scaled x rounds
-// differently from what the gradients pair it with: dA was a quarter further from its 64-bit value.)  16384 tokens x 64 heads: 168 us as
-// two kernels, 141 now; 1800 of the 2000 cycles of a chunk are shared-memory traffic (copies in, scaling, operands, states out).
+// States entering the chunks (BACK: gradients of the states leaving them) in one pass: a CTA walks the chunks of one (head,
+// sequence), the state in registers; only its bf16 copies reach memory, where chunk_state and the state pass move 20 bytes per element
+// of it.  Two groups of four warps scale the rows of B (C) of every other chunk in place, eight warps add the product of the chunk before to
+// the state; the others issue, load, and scan the step sizes, two warps with every other chunk.  (Rows of x are half as many elements, but
+// scaled x rounds differently from what the gradients pair it with: dA was a quarter further from its 64-bit value.)
+// Bound by the latency of a chunk's steps in each role (waits, proxy fences, loads): 16384 tokens x 64 heads 141 us with one group
+// of scaling warps, one scan (its loads alone 1.1 K cycles a chunk), two products in flight and one output buffer; 121 now, and 90 with the
+// state's rows in halves on two CTAs.
 // ---------------------------------------------------------------------------------------
-constexpr int WALK_ST = 4;                             // stages of B (C) and x (dy)
-constexpr int WALK_SMEM = 1024 + (3 * WALK_ST + 1) * BOXB + WALK_ST * (L + 4) * 4 + 256;
-template <bool BACK>
-__global__ void __launch_bounds__(608, 1)
+__host__ __device__ constexpr int walk_stages(int parts) { return parts == 1 ? 4 : 6; }       // of B (C) and x (dy)
+constexpr int WALK_ACC = 4;                            // products in tensor memory
+constexpr int walk_smem(int parts) { return (2 / parts + 1) * walk_stages(parts) * BOXB + 2 * BOXB / parts + walk_stages(parts) * (L + 4) * 4 + 256; }
+// PARTS 2: a CTA has half of the state's rows (blockIdx.x = 2 head + part), so that few heads use twice the SMs and a chunk's steps are
+// shorter.
+template <bool BACK, int PARTS>
+__global__ void __launch_bounds__(PARTS == 1 ? 672 : 640, 1)
 ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant__ CUtensorMap tm_v,
                 const __grid_constant__ CUtensorMap tm_out, const SsdParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sOut = smem + 3 * WALK_ST * BOXB;           // [128 n][64 p]
-  float* scale = reinterpret_cast<float*>(sOut + BOXB);      // per stage: row scales, decay of the chunk
+  extern __shared__ __align__(1024) uint8_t smem_walk[];     // the stages leave no room to align by hand
+  uint8_t* smem = smem_walk;
+  if (tc5::smem_u32(smem) & 1023u) {                   // the swizzle needs it; never seen otherwise
+    if (threadIdx.x == 0) status_report(p.status, STATUS_BAD_ARGUMENT, blockIdx.x, static_cast<int>(tc5::smem_u32(smem)));
+    return;
+  }
+  constexpr int WALK_ST = walk_stages(PARTS), OUT = BOXB / PARTS;
+  constexpr int ROWS = NS / PARTS, BOXES = 2 / PARTS, STAGE = (BOXES + 1) * BOXB;      // of the state, of B (C), of both operands
+  uint8_t* sOut = smem + WALK_ST * STAGE;              // [2][ROWS n][64 p]
+  float* scale = reinterpret_cast<float*>(sOut + 2 * OUT);      // per stage: row scales, decay of the chunk
   uint64_t* bars = reinterpret_cast<uint64_t*>(scale + WALK_ST * (L + 4));
-  uint64_t *full = bars, *empty = bars + WALK_ST, *ready = bars + 2 * WALK_ST, *done = ready + 2, *taken = ready + 4;   // [2] each: even and odd chunks
-  uint64_t *oready = ready + 6, *freed = ready + 7;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ready + 8);
+  uint64_t *full = bars, *empty = bars + WALK_ST, *ready = bars + 2 * WALK_ST, *done = ready + WALK_ACC, *taken = done + WALK_ACC;   // a product's
+  uint64_t *written = taken + WALK_ACC, *left = written + 2;       // an output buffer's
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(left + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* decay = reinterpret_cast<float*>(tmem_slot + 2);        // [2]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.x, b = blockIdx.y, nc = p.nc;
+  float* decay = reinterpret_cast<float*>(tmem_slot + 2);        // [WALK_ACC]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.x / PARTS, n0 = blockIdx.x % PARTS * ROWS,
+            b = blockIdx.y, nc = p.nc;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int i = 0; i < WALK_ST; ++i) { tc5::mbar_init(full + i, 2); tc5::mbar_init(empty + i, 1); }
-    for (int i = 0; i < 2; ++i) { tc5::mbar_init(ready + i, 8); tc5::mbar_init(done + i, 1); tc5::mbar_init(taken + i, 8); }
-    tc5::mbar_init(oready, 8);
-    tc5::mbar_init(freed, 1);
+    for (int i = 0; i < WALK_ACC; ++i) { tc5::mbar_init(ready + i, 4); tc5::mbar_init(done + i, 1); tc5::mbar_init(taken + i, 8); }
+    for (int i = 0; i < 2; ++i) { tc5::mbar_init(written + i, 8 / PARTS); tc5::mbar_init(left + i, 1); }
     tc5::fence_barrier_init();
   }
-  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 128); tc5::tmem_relinquish(); }
+  if (warp == 0) { tc5::tmem_alloc(tmem_slot, WALK_ACC * 64); tc5::tmem_relinquish(); }
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
@@ -1030,8 +1041,58 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
     return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
   };
   auto chunk_of = [&](int i) { return BACK ? nc - 1 - i : i; };
+  auto leave = [&](int i) {                            // chunk i's buffer to memory, one thread
+    tc5::tma_store_2d(&tm_out, sOut + (i & 1) * OUT, 0, ((b * nc + chunk_of(i)) * p.H + h) * NS + n0);
+    tc5::tma_store_commit();
+  };
   const int r = threadIdx.x & 127, half = (warp >> 2) & 1;      // row and half of its columns, for the first sixteen warps
-  if (warp < 8) {                                      // state: row n, columns p = 32 half ..
+  if (PARTS == 2 && warp < 8) {
+    // State, twice: the four warps of either half keep all of it and store that of every other chunk, which takes as long as the rest
+    // (the proxy fence alone a quarter).  64 rows are sixteen lanes of each quarter of tensor memory; see the load for the layout.
+    const uint32_t acc = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const int n = (warp & 3) * 16 + (lane >> 2);
+    uint8_t* out = sOut + half * OUT;
+    float2 st[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) st[j] = make_float2(0.f, 0.f);
+    for (int i = 0; i < nc; ++i) {
+      if (i > 0) {
+        uint32_t a[32];
+        if (!wait(done + (i - 1) % WALK_ACC, (i - 1) / WALK_ACC, STATUS_TIMEOUT_TMEM_FULL)) break;
+        tc5::fence_after_sync();
+        const float g = decay[(i - 1) % WALK_ACC];            // of the chunk before
+        tc5::tmem_ld_16x256b_x8(acc + (i - 1) % WALK_ACC * 64, a);
+        tc5::tmem_ld_wait();
+        tc5::fence_before_sync();
+        tc5::arrive_warp(taken + (i - 1) % WALK_ACC);
+        const float2 g2 = make_float2(g, g);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) st[j] = fma2(g2, st[j], make_float2(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1])));
+      }
+      if ((i & 1) != half) continue;
+      const bool first = (warp & 3) == 0;              // of the four: sees to their stores
+      if (i > 1) {
+        if (first) {
+          if (lane == 0) tc5::tma_store_wait_read<0>();
+          tc5::arrive_warp(left + half);
+        }
+        if (!wait(left + half, (i >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY)) break;
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {                   // columns 8 (j / 2) + 2 (lane % 4), rows n and n + 8
+        const int row = n + (j & 1) * 8;
+        *reinterpret_cast<uint32_t*>(out + row * 128 + (((j >> 1) ^ (row & 7)) << 4) + (lane & 3) * 4) = tc5::pack_bf16(st[j].x, st[j].y);
+      }
+      tc5::fence_proxy_async();
+      tc5::arrive_warp(written + half);
+      if (!first) continue;
+      if (!wait(written + half, i >> 1, STATUS_TIMEOUT_SMEM_FULL)) break;
+      if (lane == 0) leave(i);
+      __syncwarp();
+    }
+    if ((warp & 3) == 0 && lane == 0) tc5::tma_store_wait_read<0>();
+    __syncwarp();
+  } else if (warp < 8) {                               // state: row r, columns p = 32 half ..
     const uint32_t acc = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * 32;
     float2 st[16];
 #pragma unroll
@@ -1039,12 +1100,12 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
     for (int i = 0; i < nc; ++i) {
       if (i > 0) {
         float a[32];
-        if (!wait(done + ((i - 1) & 1), (i - 1) >> 1, STATUS_TIMEOUT_TMEM_FULL)) break;
+        if (!wait(done + (i - 1) % WALK_ACC, (i - 1) / WALK_ACC, STATUS_TIMEOUT_TMEM_FULL)) break;
         tc5::fence_after_sync();
-        const float g = decay[(i - 1) & 1];            // of the chunk before
-        tld32(acc + ((i - 1) & 1) * 64, a);
+        const float g = decay[(i - 1) % WALK_ACC];            // of the chunk before
+        tld32(acc + (i - 1) % WALK_ACC * 64, a);
         tc5::fence_before_sync();
-        tc5::arrive_warp(taken + ((i - 1) & 1));
+        tc5::arrive_warp(taken + (i - 1) % WALK_ACC);
         const float2 g2 = make_float2(g, g);
 #pragma unroll
         for (int j = 0; j < 16; ++j) st[j] = fma2(g2, st[j], make_float2(a[2 * j], a[2 * j + 1]));
@@ -1052,55 +1113,56 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
       uint32_t pk[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) pk[j] = tc5::pack_bf16(st[j].x, st[j].y);
-      if (i > 0 && !wait(freed, i - 1, STATUS_TIMEOUT_SMEM_EMPTY)) break;
-      st_row32(sOut, r, half * 32, pk);
+      if (i > 1 && !wait(left + (i & 1), (i >> 1) - 1, STATUS_TIMEOUT_SMEM_EMPTY)) break;
+      st_row32(sOut + (i & 1) * OUT, r, half * 32, pk);
       tc5::fence_proxy_async();
-      tc5::arrive_warp(oready);
+      tc5::arrive_warp(written + (i & 1));
     }
-  } else if (warp < 16) {                              // row t of B (C), 64 columns
-    for (int i = 0; i + 1 < nc; ++i) {
+  } else if (warp < 16) {                              // row t of B (C), of every other chunk
+    for (int i = half; i + 1 < nc; i += 2) {
       const int s = i % WALK_ST;
       if (!wait(full + s, i / WALK_ST, STATUS_TIMEOUT_SMEM_FULL)) break;
       const float sc = scale[s * (L + 4) + r];
       const float2 f = make_float2(sc, sc);
-      uint8_t* row = smem + (s * 3 + half) * BOXB + r * 128;
-      uint4 v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const uint4*>(row + ((j ^ (r & 7)) << 4));
+      for (int k = 0; k < BOXES; ++k) {
+        uint8_t* row = smem + s * STAGE + k * BOXB + r * 128;
+        uint4 v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float2 a = mul2(unpack2(v[j].x), f), c = mul2(unpack2(v[j].y), f), d = mul2(unpack2(v[j].z), f), e = mul2(unpack2(v[j].w), f);
-        *reinterpret_cast<uint4*>(row + ((j ^ (r & 7)) << 4)) =
-            make_uint4(tc5::pack_bf16(a.x, a.y), tc5::pack_bf16(c.x, c.y), tc5::pack_bf16(d.x, d.y), tc5::pack_bf16(e.x, e.y));
+        for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const uint4*>(row + ((j ^ (r & 7)) << 4));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float2 a = mul2(unpack2(v[j].x), f), c = mul2(unpack2(v[j].y), f), d = mul2(unpack2(v[j].z), f), e = mul2(unpack2(v[j].w), f);
+          *reinterpret_cast<uint4*>(row + ((j ^ (r & 7)) << 4)) =
+              make_uint4(tc5::pack_bf16(a.x, a.y), tc5::pack_bf16(c.x, c.y), tc5::pack_bf16(d.x, d.y), tc5::pack_bf16(e.x, e.y));
+        }
       }
       tc5::fence_proxy_async();
-      // the decay goes along to the product's readers, who have taken the one two chunks back
-      if (i > 1 && !wait(taken + (i & 1), (i >> 1) - 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;
-      if (threadIdx.x == 256) decay[i & 1] = scale[s * (L + 4) + L];
-      tc5::arrive_warp(ready + (i & 1));
+      // the decay goes along to the product's readers, who have taken the one that was in its place
+      if (i >= WALK_ACC && !wait(taken + i % WALK_ACC, i / WALK_ACC - 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      if (r == 0) decay[i % WALK_ACC] = scale[s * (L + 4) + L];
+      tc5::arrive_warp(ready + i % WALK_ACC);
     }
   } else if (warp == 16) {
-    constexpr uint32_t idesc = tc5::make_idesc_bf16(128, PD, 1, 1);
+    constexpr uint32_t idesc = tc5::make_idesc_bf16(ROWS, PD, 1, 1);
     const bool lead = tc5::elect_one();                // converged warp, elected lane issues (see ssd_chunk_state_kernel)
     for (int i = 0; i + 1 < nc; ++i) {                 // nothing follows the last chunk
       const int s = i % WALK_ST;
-      const uint64_t a0 = tc5::desc_mnmajor(tc5::smem_u32(smem + s * 3 * BOXB), BOXB);
-      const uint64_t v0 = tc5::desc_mnmajor(tc5::smem_u32(smem + (s * 3 + 2) * BOXB), BOXB);
-      if (!wait(ready + (i & 1), i >> 1, STATUS_TIMEOUT_TMEM_EMPTY)) break;       // also: the product two chunks back has been taken
+      const uint64_t a0 = tc5::desc_mnmajor(tc5::smem_u32(smem + s * STAGE), BOXB);
+      const uint64_t v0 = tc5::desc_mnmajor(tc5::smem_u32(smem + s * STAGE + BOXES * BOXB), BOXB);
+      if (!wait(ready + i % WALK_ACC, i / WALK_ACC, STATUS_TIMEOUT_TMEM_EMPTY)) break;       // also: its place in tensor memory is free
       tc5::fence_after_sync();
       if (lead) {
 #pragma unroll
         for (int kk = 0; kk < L / 16; ++kk)
-          tc5::mma_ss(tmem + (i & 1) * 64, a0 + static_cast<uint64_t>((kk * 2048) >> 4), v0 + static_cast<uint64_t>((kk * 2048) >> 4), idesc, kk > 0 ? 1u : 0u);
-        tc5::mma_commit(done + (i & 1));
+          tc5::mma_ss(tmem + i % WALK_ACC * 64, a0 + static_cast<uint64_t>((kk * 2048) >> 4), v0 + static_cast<uint64_t>((kk * 2048) >> 4), idesc, kk > 0 ? 1u : 0u);
+        tc5::mma_commit(done + i % WALK_ACC);
         tc5::mma_commit(empty + s);
       }
       __syncwarp();
     }
   } else if (warp == 17) {
     const bool lead = tc5::elect_one();
-    const float a = p.A[h];
-    auto load_dt = [&](int i) { return load_dt4(p, b, chunk_of(i) * L, h); };
     // into L2 a few chunks ahead: the stages alone leave a load from memory less time than it takes
     constexpr int AHEAD = 8;
     auto prefetch = [&](int i) {
@@ -1108,56 +1170,62 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
       const int t0 = chunk_of(i) * L;
       tc5::tma_prefetch_4d(&tm_v, 0, h, t0, b);
       if (i % p.H != h) return;                        // shared by all heads
-      tc5::tma_prefetch_3d(&tm_bc, 0, t0, b);
-      tc5::tma_prefetch_3d(&tm_bc, 64, t0, b);
+#pragma unroll
+      for (int k = 0; k < BOXES; ++k) tc5::tma_prefetch_3d(&tm_bc, n0 + k * 64, t0, b);
     };
     for (int i = WALK_ST; i < AHEAD; ++i) prefetch(i);
     bool ok = true;
-    float4 dt = load_dt(0);
     for (int i = 0; i + 1 < nc; ++i) {
       const int s = i % WALK_ST, t0 = chunk_of(i) * L;
-      uint8_t* st = smem + s * 3 * BOXB;
-      const float4 dt_next = load_dt(i + 1);
+      uint8_t* st = smem + s * STAGE;
       if (i >= WALK_ST && !(ok = wait(empty + s, i / WALK_ST - 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
       if (lead) {
-        tc5::mbar_expect_tx(full + s, 3 * BOXB);
-        tc5::tma_load_3d(st, &tm_bc, full + s, 0, t0, b);
-        tc5::tma_load_3d(st + BOXB, &tm_bc, full + s, 64, t0, b);
-        tc5::tma_load_4d(st + 2 * BOXB, &tm_v, full + s, 0, h, t0, b);
+        tc5::mbar_expect_tx(full + s, STAGE);
+#pragma unroll
+        for (int k = 0; k < BOXES; ++k) tc5::tma_load_3d(st + k * BOXB, &tm_bc, full + s, n0 + k * 64, t0, b);
+        tc5::tma_load_4d(st + BOXES * BOXB, &tm_v, full + s, 0, h, t0, b);
       }
       prefetch(i + AHEAD);
       __syncwarp();
-      const float4 c = chunk_sums(dt, a);
-      const float tot = __shfl_sync(0xffffffffu, c.w, 31);
-      auto weight = [&](float cum, float d) { return BACK ? exp2f(cum) : exp2f(tot - cum) * d; };
-      float* sc = scale + s * (L + 4);
-      *reinterpret_cast<float4*>(sc + 4 * lane) = make_float4(weight(c.x, dt.x), weight(c.y, dt.y), weight(c.z, dt.z), weight(c.w, dt.w));
-      if (lane == 0) sc[L] = exp2f(tot);
-      tc5::arrive_warp(full + s);
-      dt = dt_next;
     }
     // stages whose last use was not waited for above
     for (int i = nc > WALK_ST + 1 ? nc - WALK_ST : 0; i + 1 < nc && ok; ++i) ok = wait(empty + i % WALK_ST, i / WALK_ST, STATUS_TIMEOUT_SMEM_EMPTY);
     if (!ok && lead)                                   // loads may still be in flight
       for (int i = 0; i < WALK_ST; ++i) tc5::mbar_drain(full + i);
     __syncwarp();
-  } else {
-    const bool lead = tc5::elect_one();
-    for (int i = 0; i < nc; ++i) {
-      if (!wait(oready, i, STATUS_TIMEOUT_TMEM_EMPTY)) break;
-      if (lead) {
-        tc5::tma_store_2d(&tm_out, sOut, 0, ((b * nc + chunk_of(i)) * p.H + h) * NS);
-        tc5::tma_store_commit();
-        tc5::tma_store_wait_read<0>();
-      }
-      tc5::arrive_warp(freed);
+  } else if (warp < 20) {                              // row scales and decay of every other chunk, the next one's step sizes in flight
+    const float a = p.A[h];
+    auto load_dt = [&](int i) { return load_dt4(p, b, chunk_of(min(i, nc - 1)) * L, h); };
+    float4 dt = load_dt(warp - 18), next = load_dt(warp - 16);
+    for (int i = warp - 18; i + 1 < nc; i += 2) {
+      const int s = i % WALK_ST;
+      const float4 c = chunk_sums(dt, a);
+      const float tot = __shfl_sync(0xffffffffu, c.w, 31);
+      auto weight = [&](float cum, float d) { return BACK ? exp2f(cum) : exp2f(tot - cum) * d; };
+      const float4 w = make_float4(weight(c.x, dt.x), weight(c.y, dt.y), weight(c.z, dt.z), weight(c.w, dt.w));
+      dt = next;
+      next = load_dt(i + 4);
+      if (i >= WALK_ST && !wait(empty + s, i / WALK_ST - 1, STATUS_TIMEOUT_SMEM_EMPTY)) break;
+      float* sc = scale + s * (L + 4);
+      *reinterpret_cast<float4*>(sc + 4 * lane) = w;
+      if (lane == 0) sc[L] = exp2f(tot);
+      tc5::arrive_warp(full + s);
     }
-    if (lead) tc5::tma_store_wait_read<0>();
+  } else {                                             // PARTS 1: the stores of all eight state warps
+    for (int i = 0; i < nc; ++i) {
+      if (!wait(written + (i & 1), i >> 1, STATUS_TIMEOUT_SMEM_FULL)) break;
+      if (lane == 0) {
+        leave(i);
+        tc5::tma_store_wait_read<1>();                 // the one before has left its buffer
+      }
+      if (i > 0) tc5::arrive_warp(left + ((i - 1) & 1));
+    }
+    if (lane == 0) tc5::tma_store_wait_read<0>();
     __syncwarp();
   }
   tc5::fence_before_sync();
   __syncthreads();
-  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 128); }
+  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, WALK_ACC * 64); }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1405,8 +1473,8 @@ int map_v(CUtensorMap* m, const void* base, int B, int T, int H, long ld) {
   uint32_t box[4] = {64, 1, (uint32_t)L, 1};
   return nsa::make_tmap_bf16(m, base, 4, dims, strides, box, 1);
 }
-int map_state(CUtensorMap* m, const void* base, long rows) {
-  return nsa::make_tmap_2d_bf16(m, base, PD, rows, PD, 64, NS);
+int map_state(CUtensorMap* m, const void* base, long rows, int box_rows = NS) {
+  return nsa::make_tmap_2d_bf16(m, base, PD, rows, PD, 64, box_rows);
 }
 template <typename K>
 int smem_attr(K kern, int bytes) {
@@ -1459,8 +1527,8 @@ extern "C" int nsa_ssd_finish(const float* dB_part, const float* dC_part, const 
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_finish launch");
 }
 
-// One pass over the chunks (nsa_ssd_states) or chunk_state and the state pass.  The walk takes 3.2 us and 1.13 a chunk for up to one head
-// per SM.  The two kernels take 6.6 us and 0.095 a chunk (the pass is a chain), 5.1 and 0.0165 per (chunk, head), or 0.019 per
+// One pass over the chunks (nsa_ssd_states) or chunk_state and the state pass.  The walk is counted with 3.2 us and 1.13 a chunk for up to one
+// head per SM, which it has since become 0.2 a chunk faster than; the line matters beyond half as many heads as SMs (see below).  The two kernels take 6.6 us and 0.095 a chunk (the pass is a chain), 5.1 and 0.0165 per (chunk, head), or 0.019 per
 // (chunk, head), whichever is the most, and have a gap between them.  Walk and two kernels, us: 300 tokens x 1 head 6.3, 6.7;
 // 1000 x 1 11.1, 6.6; 1000 x 32 12.0, 9.1; 1000 x 48 12.3, 11.4; 777 x 64 11.0, 12.9; 1500 x 64 17, 19.2; 1000 x 128 13.4, 22.1;
 // 16384 x 48 141, 121; 16384 x 64 141, 169; 2 x 8192 x 32 72, 83.
@@ -1468,6 +1536,19 @@ extern "C" int nsa_ssd_states_in_one(int B, int T, int H) {
   const long heads = static_cast<long>(B) * H, chunks = (T + L - 1) / L, items = heads * chunks, sms = nsa::sm_count();
   const double walk = (3.2 + 1.13 * chunks) * ((heads + sms - 1) / sms);
   return walk <= std::max({6.6 + 0.095 * chunks, 5.1 + 0.0165 * items, 0.019 * items}) + 0.5;
+}
+
+// How the states are best formed: 0 chunk_state and the state pass, 1 one walk over the chunks per head, 2 two walks with half of the
+// state's rows each.  The halves take 3.0 us and 0.56 a chunk, and 0.0019 more a chunk for each head (memory); they are the better form as long
+// as all of them run at once, except where heads are few and chunks many.  us of halves, one walk and two kernels: 300 tokens x 1 head
+// 4.7, 5.9, 6.7; 1000 x 32 8.7, 10.5, 9.1; 1000 x 64 9.2, 10.9, 13.5; 4000 x 32 24.5, 32, 21; 4000 x 64 26, 34, 40; 16384 x 48 87, 120, 122; 16384 x 64
+// 90, 121, 169; 16384 x 128 181, 127.
+extern "C" int nsa_ssd_states_form(int B, int T, int H) {
+  if (B <= 0 || T <= 0 || H <= 0) return 0;
+  const long heads = static_cast<long>(B) * H, chunks = (T + L - 1) / L, items = heads * chunks, sms = nsa::sm_count();
+  const double two = std::max({6.6 + 0.095 * chunks, 5.1 + 0.0165 * items, 0.019 * items}) + 0.5;
+  if (chunks > 1 && 2 * heads <= sms && 3.0 + (0.56 + 0.0019 * heads) * chunks <= two) return 2;
+  return nsa_ssd_states_in_one(B, T, H) ? 1 : 0;
 }
 
 // back = 0: bc = B rows, v = x -> states entering the chunks; back = 1: bc = C rows, v = dy -> gradients of the states leaving them.
@@ -1481,14 +1562,13 @@ extern "C" int nsa_ssd_states(int back, const void* bc, long ld_bc, const void* 
   CUtensorMap tb, tv, to;
   if ((rc = map_bc(&tb, bc, B, T, ld_bc))) return rc;
   if ((rc = map_v(&tv, v, B, T, H, ld_v))) return rc;
-  if ((rc = map_state(&to, out, static_cast<long>(B) * p.nc * H * NS))) return rc;
-  static bool cfg = false;
-  if (!cfg) {
-    if ((rc = smem_attr(ssd_walk_kernel<true>, WALK_SMEM)) || (rc = smem_attr(ssd_walk_kernel<false>, WALK_SMEM))) return rc;
-    cfg = true;
-  }
-  if (back) ssd_walk_kernel<true><<<dim3(H, B), 608, WALK_SMEM, st>>>(tb, tv, to, p);
-  else ssd_walk_kernel<false><<<dim3(H, B), 608, WALK_SMEM, st>>>(tb, tv, to, p);
+  const int parts = nsa_ssd_states_form(B, T, H) == 2 ? 2 : 1, bytes = walk_smem(parts);
+  if ((rc = map_state(&to, out, static_cast<long>(B) * p.nc * H * NS, NS / parts))) return rc;
+  auto* kernel = parts == 2 ? (back ? ssd_walk_kernel<true, 2> : ssd_walk_kernel<false, 2>) : back ? ssd_walk_kernel<true, 1> : ssd_walk_kernel<false, 1>;
+  static bool cfg[4] = {};
+  bool& ready = cfg[parts * 2 - 2 + (back != 0)];
+  if (!ready) { if ((rc = smem_attr(kernel, bytes))) return rc; ready = true; }
+  kernel<<<dim3(H * parts, B), parts == 1 ? 672 : 640, bytes, st>>>(tb, tv, to, p);
   nsa::count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_states launch");

@@ -85,6 +85,7 @@ SIGNATURES = {
     "nsa_ssd_state_bwd": "ippppiiilp",
     "nsa_ssd_state_fwd": "ipppppiiilp",
     "nsa_ssd_states": "iiplplpppiiiiip",
+    "nsa_ssd_states_form": "iiii",
     "nsa_ssd_states_in_one": "iiii",
     "nsa_status_read": "ipi",
     "nsa_sumsq": "iplippip",
