@@ -59,6 +59,7 @@ struct AttnParams {
   int add_dq;                       // dQ is added to what dQb holds (fp32 sum, one rounding)
   float* dK;                        // [B, S, Hkv, D] fp32, pre-zeroed
   float* dV;
+  bf16 *dKb, *dVb;                  // not null: the whole gradients, written as bf16 (dK, dV unused)
   KernelStatus* status;
 };
 
@@ -2495,7 +2496,18 @@ __device__ __forceinline__ int key_walk(const AttnParams& p, int visits, int s0,
   v0 = max(qt_lo, y * visits);                 // long ranges: absolute chunks, the same Q/dO range for every key block
   return min(n_qt, (y + 1) * visits) - v0;
 }
-// dV, dK += the walks' sums, in order.  D / 4 lanes own a (key, head) row.
+// Zero gradients of the keys s0 .. s0 + keys - 1 of a head (all threads of a CTA).
+template <int D>
+__device__ void zero_rows(const AttnParams& p, int b, int h, int s0, int keys) {
+  for (int i = threadIdx.x; i < keys * (D / 8); i += blockDim.x) {
+    const int s = s0 + i / (D / 8);
+    if (s >= p.S) break;
+    const long o = ((static_cast<long>(b) * p.S + s) * p.Hkv + h) * (D / 8) + i % (D / 8);
+    reinterpret_cast<uint4*>(p.dKb)[o] = make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4*>(p.dVb)[o] = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+// dV, dK += (or = in bf16) the walks' sums, in order.  D / 4 lanes own a (key, head) row.
 template <int D>
 __global__ void __launch_bounds__(256) attn_sum_walks_kernel(const AttnParams p, const KeyWalks w, const long rows) {
   constexpr int LANES = D / 4;
@@ -2503,7 +2515,6 @@ __global__ void __launch_bounds__(256) attn_sum_walks_kernel(const AttnParams p,
   if (row >= rows) return;
   const long i = row * LANES + threadIdx.x % LANES, n = rows * LANES;        // in float4
   const int s0 = static_cast<int>(row / p.Hkv % p.S) & ~127;
-  float4* out = reinterpret_cast<float4*>(blockIdx.y ? p.dK : p.dV) + i;
   const float4* part = reinterpret_cast<const float4*>(w.part) + blockIdx.y * n + i;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int y = 0; y < w.walks; ++y) {
@@ -2512,6 +2523,11 @@ __global__ void __launch_bounds__(256) attn_sum_walks_kernel(const AttnParams p,
     const float4 v = part[2 * n * y];
     acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
   }
+  if (p.dKb) {
+    reinterpret_cast<uint2*>(blockIdx.y ? p.dKb : p.dVb)[i] = make_uint2(tc5::pack_bf16(acc.x, acc.y), tc5::pack_bf16(acc.z, acc.w));
+    return;
+  }
+  float4* out = reinterpret_cast<float4*>(blockIdx.y ? p.dK : p.dV) + i;
   const float4 old = *out;
   *out = make_float4(old.x + acc.x, old.y + acc.y, old.z + acc.z, old.w + acc.w);
 }
@@ -2552,7 +2568,10 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   const int s0 = block * KEYS;
   int v0;
   const int n_vis = key_walk<KEYS>(p, w.visits, s0, blockIdx.y, v0);
-  if (n_vis <= 0) return;
+  if (n_vis <= 0) {                              // nothing sees these keys
+    if (p.dKb && w.part == nullptr) zero_rows<D>(p, b, h, s0, KEYS);
+    return;
+  }
   if (tc5::smem_u32(smem_kvc) & 1023u) {         // the swizzle needs it; never seen otherwise
     if (tid == 0) status_report(p.status, STATUS_BAD_ARGUMENT, blockIdx.x, static_cast<int>(tc5::smem_u32(smem_kvc)));
     return;
@@ -2792,9 +2811,9 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       }
     }
     // ---- accumulators -> global.  A thread holds half a key's row (D / 64 loads of 32 columns each for dV and dK); rows go through shared memory (free now, pitch spread over
-    //      the banks) and are added to global memory by one bulk reduction each: scattered 16-byte reductions were most of a CTA's
+    //      the banks) and are added to global memory by one bulk reduction each (or stored by a bulk copy, as bf16 where they are whole): scattered 16-byte reductions were most of a CTA's
     //      fixed cost of 14 us.
-    const bool have = ok && wait(acc_done, 0, STATUS_TIMEOUT_TMEM_FULL);
+    const bool have = ok && wait(acc_done, 0, STATUS_TIMEOUT_TMEM_FULL), bf16_out = p.dKb != nullptr && w.part == nullptr;
     if (have) {
       tc5::fence_after_sync();
 #pragma unroll
@@ -2803,7 +2822,18 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         const int c = ch * (D / 2) + (q % KB) * 32;
         tc5::tmem_ld_x32(lane_row + (q < KB ? cDV : cDK) + c, a);
         tc5::tmem_ld_wait();
-        float4* dst = reinterpret_cast<float4*>(sQ + (q < KB ? 0 : KEYS * ROW) + (tid & 127) * ROW + c * 4);
+        uint8_t* mine = sQ + (q < KB ? 0 : KEYS * ROW) + (tid & 127) * ROW;
+        if (bf16_out) {
+          uint4* dst = reinterpret_cast<uint4*>(mine + c * 2);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            dst[i] = make_uint4(tc5::pack_bf16(__uint_as_float(a[8 * i]), __uint_as_float(a[8 * i + 1])),
+                                tc5::pack_bf16(__uint_as_float(a[8 * i + 2]), __uint_as_float(a[8 * i + 3])),
+                                tc5::pack_bf16(__uint_as_float(a[8 * i + 4]), __uint_as_float(a[8 * i + 5])),
+                                tc5::pack_bf16(__uint_as_float(a[8 * i + 6]), __uint_as_float(a[8 * i + 7])));
+          continue;
+        }
+        float4* dst = reinterpret_cast<float4*>(mine + c * 4);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           dst[i] = make_float4(__uint_as_float(a[4 * i]), __uint_as_float(a[4 * i + 1]), __uint_as_float(a[4 * i + 2]),
@@ -2817,6 +2847,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       const long o = ((static_cast<long>(b) * p.S + s0 + row) * p.Hkv + h) * D;
       const uint8_t* src = sQ + ch * KEYS * ROW + row * ROW;
       if (w.part) tc5::bulk_store(w.part + (blockIdx.y * 2 + ch) * (static_cast<long>(p.B) * p.S * p.Hkv * D) + o, src, D * 4);
+      else if (bf16_out) tc5::bulk_store((ch ? p.dKb : p.dVb) + o, src, D * 2);
       else tc5::bulk_reduce_add_f32((ch ? p.dK : p.dV) + o, src, D * 4);
       tc5::tma_store_commit();
       tc5::tma_store_wait_read<0>();
@@ -2899,7 +2930,10 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     b = blockIdx.y / p.Hkv; h = blockIdx.y - b * p.Hkv; s0 = blockIdx.x * 64;
     n_vis = key_walk<64>(p, p.T, s0, 0, v0);
   }
-  if (n_vis <= 0) return;
+  if (n_vis <= 0) {                              // nothing sees these keys
+    if (!SELECTED && p.dKb) zero_rows<D>(p, b, h, s0, 64);
+    return;
+  }
 
   if (tid == 0) {
     *abort_flag = 0;
@@ -3127,11 +3161,13 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tc5::fence_proxy_async();
       tc5::mbar_arrive(p_full);
     }
-    // ---- accumulators -> global: lane = d, columns = keys; one fp32 reduction per element
+    // ---- accumulators -> global: lane = d, columns = keys; one fp32 reduction per element, or one bf16 where the sums are whole
     if (__all_sync(0xffffffffu, ok && tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
       tc5::fence_after_sync();
       const int d = (warp & 3) * 32 + lane;
-      float* dst = (warp < 4 ? p.dV : p.dK) + ((static_cast<long>(b) * p.S + s0) * p.Hkv + h) * D + d;
+      const long o = ((static_cast<long>(b) * p.S + s0) * p.Hkv + h) * D + d;
+      float* dst = (warp < 4 ? p.dV : p.dK) + o;
+      bf16* dst_b = (warp < 4 ? p.dVb : p.dKb) + o;
       const uint32_t col = warp < 4 ? cDV : cDK;
 #pragma unroll
       for (int c0 = 0; c0 < 64; c0 += 32) {
@@ -3140,7 +3176,10 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tc5::tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i)
-          if (s0 + c0 + i < p.S) atomicAdd(dst + static_cast<long>(c0 + i) * p.Hkv * D, __uint_as_float(a[i]));
+          if (s0 + c0 + i < p.S) {
+            if (!SELECTED && p.dKb) dst_b[static_cast<long>(c0 + i) * p.Hkv * D] = __float2bfloat16_rn(__uint_as_float(a[i]));
+            else atomicAdd(dst + static_cast<long>(c0 + i) * p.Hkv * D, __uint_as_float(a[i]));
+          }
       }
     }
   }
@@ -3703,14 +3742,15 @@ extern "C" int nsa_attn_bwd_walks_d64(int B, int T, int S, int Hq, int Hkv, int 
 // item_bound >= item_start[last].  head_dim 128 only; selected mode needs G >= 8.
 // delta_given: delta holds rowsum(dO * O) already (the gated combine's backward has both tensors in registers).
 // walks, part: of nsa_attn_bwd_walks (contiguous ranges).
-// add_dq: dQ is added to what dq holds; dK / dV always add to what the caller put there.
+// add_dq: dQ is added to what dq holds.  dK / dV add to what the caller put there (fp32), or with write_kv are bf16 tensors that
+// receive the whole gradients (contiguous ranges with walks != 0): four launches less, 17 of 130 us where the host is the bound.
 extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                                  const float* L, float* delta, void* dq, float* dk, float* dv, int B, int T, int S,
+                                  const float* L, float* delta, void* dq, void* dk, void* dv, int B, int T, int S,
                                   int Hq, int Hkv, int D, float scale, int causal, int window, int kp_stride, int kp_off,
                                   const int* tile_blocks, const unsigned long long* tile_masks, const int* tile_counts,
                                   int max_u, const int* tok_list, const int* list_start, const int* item_start, int nS,
                                   int item_bound, int visits_per_cta, float* part, int walks, int delta_given, int add_dq,
-                                  cudaStream_t st) {
+                                  int write_kv, cudaStream_t st) {
   int rc = check_shape(Hq, Hkv, D, tile_blocks);
   if (rc) return rc;
   const int G = Hq / Hkv;
@@ -3744,7 +3784,9 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
       attn_bwd_dq_kernel<<<grid, 320, smem, st>>>(tq, tdo, tk, tv, p, scale);
     }
   }
-  p.dK = dk; p.dV = dv;
+  if (write_kv && (tile_blocks || walks == 0)) return nsa::fail(NSA_ERR_SHAPE, "attn_bwd_split: these dK and dV are sums in memory");
+  if (write_kv) { p.dKb = (bf16*)dk; p.dVb = (bf16*)dv; }
+  else { p.dK = (float*)dk; p.dV = (float*)dv; }
   if (tile_blocks) {
     KvWalk w{};
     w.visits_per_cta = visits_per_cta;

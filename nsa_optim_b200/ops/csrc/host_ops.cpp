@@ -631,17 +631,20 @@ Inverse inverse_lists(const Tensor& idx_, long nS, long R, long visits) {
   return v;
 }
 
-// dQ from the query-tile kernel, dK and dV (fp32, added to) from the key-block kernel.  given: rowsum(dO * O) where the caller has it.
+// dQ from the query-tile kernel, dK and dV (fp32, added to; bf16, written) from the key-block kernel.  given: rowsum(dO * O) where the caller has it.
 void attn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& dO, const Tensor& L, const Tensor& dq,
                    const Tensor& dk, const Tensor& dv, const Range& r, const Tiles& t, const Inverse& inv, long visits, long walks,
                    const Tensor& given, bool add_dq) {
   const Tensor delta = given.defined() ? given : alloc(q.sizes().slice(0, 3), F32, q.device());
   const Tensor part = walks > 1 ? alloc({walks, 2, k.numel()}, F32, q.device()) : Tensor();
-  launch(lib.nsa_attn_bwd_split, ptr(q), ptr(k), ptr(v), ptr(o), ptr(dO), fp(L), fp(delta), ptr(dq), fp(dk), fp(dv), dim(q.size(0)),
+  launch(lib.nsa_attn_bwd_split, ptr(q), ptr(k), ptr(v), ptr(o), ptr(dO), fp(L), fp(delta), ptr(dq), ptr(dk), ptr(dv), dim(q.size(0)),
          dim(q.size(1)), dim(k.size(1)), dim(q.size(2)), dim(k.size(2)), dim(q.size(3)), r.scale, r.causal, r.window, r.kp_stride, r.kp_off,
          ip(t.blocks), t.mask(), ip(t.counts), t.max_u, ip(inv.tok), ip(inv.list_start), ip(inv.item_start), t.any() ? t.nS : 0,
-         dim(inv.bound), dim(visits), fp(part), dim(walks), static_cast<int>(given.defined()), static_cast<int>(add_dq));
+         dim(inv.bound), dim(visits), fp(part), dim(walks), static_cast<int>(given.defined()), static_cast<int>(add_dq),
+         static_cast<int>(dk.scalar_type() == BF));
 }
+// dK or dV: written whole by contiguous ranges of several walks, one, or 64 keys a CTA; else to be added to
+Tensor key_grad(const Tensor& k, bool whole) { return alloc(k.sizes(), whole ? BF : F32, k.device(), !whole); }
 // Query tiles per CTA of the dK / dV kernel over a contiguous range, where a key block has more than 256, and over a list of tokens
 long range_visits() { return env_long("NSA_B200_KV_VISITS", 64); }
 long list_visits() { return env_long("NSA_B200_KV_VISITS_SEL", 64); }
@@ -678,7 +681,8 @@ OP(attn_bwd) {                                   // q, k, v, o, dO, L, range, ti
     const bool split = a.b();
     return [=]() -> List {
       const Tensor dO = dense(dO_), dq = alloc(q.sizes(), q.scalar_type(), q.device());
-      const Tensor dk = alloc(k.sizes(), F32, q.device(), true), dv = alloc(v.sizes(), F32, q.device(), true);
+      const bool whole = split && !t.any() && walks != 0;
+      const Tensor dk = key_grad(k, whole), dv = key_grad(v, whole);
       if (split) {
         attn_backward(q, k, v, o, dO, L, dq, dk, dv, r, t, inv, t.any() ? list_visits() : range_visits(), walks, Tensor(), false);
       } else {
@@ -835,12 +839,12 @@ OP(nsa_bwd) {                                    // q, k, v, kc, vc, o1, d1, L1,
       const auto dev = q.device();
       const int B = dim(q.size(0)), T = dim(q.size(1)), Hq = dim(q.size(2)), Hkv = dim(k.size(2));
       const Tensor dq = alloc(q.sizes(), q.scalar_type(), dev);
-      Tensor dkc = alloc(kc.sizes(), F32, dev, true), dvc = alloc(vc.sizes(), F32, dev, true);
       Tensor dk = alloc(k.sizes(), F32, dev, true), dv = alloc(v.sizes(), F32, dev, true);
       auto walks = [&](const Tensor& keys, int win, int kp) { return have(lib.nsa_attn_bwd_walks)(B, T, dim(keys.size(1)), Hq, Hkv, 1, win, kp); };
       const long visits = range_visits(), per_list = list_visits();
-      attn_backward(q, kc, vc, o[0], d[0], L[0], dq, dkc, dvc, {1, 0, scale, stride, block - 1}, Tiles(), Inverse(), visits, walks(kc, 0, stride),
-                    e[0], false);
+      const int pooled = walks(kc, 0, stride);
+      const Tensor dkc = key_grad(kc, pooled != 0), dvc = key_grad(vc, pooled != 0);
+      attn_backward(q, kc, vc, o[0], d[0], L[0], dq, dkc, dvc, {1, 0, scale, stride, block - 1}, Tiles(), Inverse(), visits, pooled, e[0], false);
       const Inverse lists = inverse_lists(t.idx, t.nS, 128 / (Hq / Hkv), per_list);
       attn_backward(q, k, v, o[1], d[1], L[1], dq, dk, dv, {1, 0, scale, 1, 0}, t, lists, per_list, 0, e[1], true);
       // The window branch shares dk / dv while a key block's gradients get one addition from it: one more to what is there gives

@@ -98,10 +98,10 @@ int nsa_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
 int nsa_attn_bwd_walks(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride);      // head_dim 128
 int nsa_attn_bwd_walks_d64(int B, int T, int S, int Hq, int Hkv, int causal, int window, int kp_stride);  // head_dim 64
 int nsa_attn_bwd_split(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* L,
-    float* delta, void* dq, float* dk, float* dv, int B, int T, int S, int Hq, int Hkv, int D, float scale, int causal,
+    float* delta, void* dq, void* dk, void* dv, int B, int T, int S, int Hq, int Hkv, int D, float scale, int causal,
     int window, int kp_stride, int kp_off, const int* tile_blocks, const unsigned long long* tile_masks, const int*
     tile_counts, int max_u, const int* tok_list, const int* list_start, const int* item_start, int nS, int item_bound,
-    int visits_per_cta, float* part, int walks, int delta_given, int add_dq, cudaStream_t st);
+    int visits_per_cta, float* part, int walks, int delta_given, int add_dq, int write_kv, cudaStream_t st);
 int nsa_union_blocks(const int* idx, int* tile_blocks, unsigned long long* tile_masks, int* tile_counts, int B, int
     T, int Hkv, int G, int top_n, int nS, int max_u, cudaStream_t st);
 

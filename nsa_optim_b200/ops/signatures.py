@@ -19,7 +19,7 @@ SIGNATURES = {
     "nsa_affine_dequant": "ippppliip",
     "nsa_affine_quant": "ippppliiip",
     "nsa_attn_bwd": "ippppppppppiiiiiifiiiipppip",
-    "nsa_attn_bwd_split": "ippppppppppiiiiiifiiiipppipppiiipiiip",
+    "nsa_attn_bwd_split": "ippppppppppiiiiiifiiiipppipppiiipiiiip",
     "nsa_attn_bwd_walks": "iiiiiiiii",
     "nsa_attn_bwd_walks_d64": "iiiiiiiii",
     "nsa_attn_fwd": "ipppppiiiiiifiiiipppip",
