@@ -1900,13 +1900,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // warps 9, 10 and 11 issue S = Q K^T, dP = dO V^T (double-buffered in TMEM) and dQ += dS K
 // (resident in TMEM).  Visits are 64-key blocks: the contiguous range allowed by causality / window, or the
 // entries of the tile's union list (selected mode, with the per-token bit masks).
-// head_dim 64 leaves room for a third S / dP buffer.  All softmax threads share a visit: dS takes the place of S, so a buffer is held until dS is consumed, and groups
-// on alternate visits (as in the forward) hold it longer than they overlap (8192 tokens x 32 heads: 819 us against 693).
+// head_dim 64 leaves room for a third S / dP buffer.
+// Without GROUPS all softmax threads share a visit, and dS takes the place of S: a buffer is held until dS is consumed.  With GROUPS (tiles of
+// many visits, see dq_in_groups) two groups of softmax warps take alternate visits; S is free again as soon as the scores are in registers,
+// they are exponentiated before dP is waited for, and dS takes the place of dP, so that the chain from one dQ to the next is dP, dS and dQ
+// alone.  A group's visit is 2240 cycles, two of them side by side, of 768 tensor work and 512 of exponentials each (8192 tokens
+// x 32 heads: 682 us without, 638 with groups; groups with dS in the place of S 819; one group of all warps with both waits 810).
 // --------------------------------------------------------------------------------------
 constexpr int DQT_STAGES = 5;
 constexpr int dqt_smem(int D) { return D / 64 * (4 + 2 * DQT_STAGES) * HALF + 1024 + 256; }
 
-template <int D>
+template <int D, bool GROUPS>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -1924,11 +1928,13 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   uint64_t* kv_full = bars + 1;                  // [stages] TMA -> MMA
   uint64_t* kv_empty = kv_full + DQT_STAGES;      // [stages] MMA -> TMA
   uint64_t* s_full = kv_empty + DQT_STAGES;       // [BUFS] MMA -> softmax
-  uint64_t* s_empty = s_full + BUFS;             // [BUFS] softmax -> MMA
+  uint64_t* dp_full = s_full + BUFS;             // [BUFS] MMA -> softmax
+  uint64_t* s_empty = dp_full + BUFS;            // [BUFS] softmax -> MMA: the scores are in registers
+  uint64_t* dp_empty = s_empty + BUFS;           // [BUFS] MMA -> MMA: dS, in dP's place, is consumed
   // One dS barrier per S buffer: warps whose rows are all masked finish a visit early and may
   // already be in the next visit (other buffer); with a single barrier their second arrival
   // would complete the phase of the visit the slower warps are still writing.
-  uint64_t* ds_full = s_empty + BUFS;            // [BUFS] softmax -> MMA
+  uint64_t* ds_full = dp_empty + BUFS;            // [BUFS] softmax -> MMA
   uint64_t* qt_full = ds_full + BUFS;            // softmax -> MMA: Q and dO are in tensor memory
   uint64_t* acc_done = qt_full + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
@@ -1971,7 +1977,13 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     *abort_flag = 0;
     tc5::mbar_init(q_full, 1);
     for (int i = 0; i < DQT_STAGES; ++i) { tc5::mbar_init(kv_full + i, 1); tc5::mbar_init(kv_empty + i, 1); }
-    for (int i = 0; i < BUFS; ++i) { tc5::mbar_init(s_full + i, 2); tc5::mbar_init(s_empty + i, 1); tc5::mbar_init(ds_full + i, 256); }
+    for (int i = 0; i < BUFS; ++i) {
+      tc5::mbar_init(s_full + i, GROUPS ? 1 : 2);
+      tc5::mbar_init(dp_full + i, 1);
+      tc5::mbar_init(s_empty + i, GROUPS ? 128 : 1);
+      tc5::mbar_init(dp_empty + i, 1);
+      tc5::mbar_init(ds_full + i, GROUPS ? 128 : 256);
+    }
     tc5::mbar_init(qt_full, 256);
     tc5::mbar_init(acc_done, 1);
     tc5::fence_barrier_init();
@@ -2031,8 +2043,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   } else if (warp == 9 || warp == 10) {
     // ------------------------------------------------------------------ MMA issuers 1 and 2: S = Q K^T, dP = dO V^T
     // Three issuing warps, each converged with one elected lane issuing (see the forward kernel):
-    // warp 9 issues S, warp 10 dP, warp 11 dQ += dS K.  s_full counts one commit of each of the
-    // first two.  The address field (bits 0-13, address >> 4) of a shared-memory descriptor is
+    // warp 9 issues S, warp 10 dP, warp 11 dQ += dS K.  The address field (bits 0-13, address >> 4) of a shared-memory descriptor is
     // advanced by adding the byte offset >> 4.
     if (n_vis > 0) {
       const bool lead = tc5::elect_one();
@@ -2040,12 +2051,13 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 64, 0, 0);
       const uint64_t b0 = tc5::desc_kmajor(tc5::smem_u32(sKV) + (is_dp ? KVT : 0));   // stage 0, K or V, k-step 0
       const uint32_t acol = is_dp ? cDO : cQ, dcol = is_dp ? 64u : 0u;
+      uint64_t *made = GROUPS && is_dp ? dp_full : s_full, *free = GROUPS && is_dp ? dp_empty : s_empty;
       bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(qt_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
       if (ok) tc5::fence_after_sync();
       for (int v = 0; v < n_vis && ok; ++v) {
         const int st = v % DQT_STAGES, buf = v % BUFS;
         ok = __all_sync(0xffffffffu, tc5::mbar_wait(kv_full + st, (v / DQT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(s_empty + buf, ((v / BUFS) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
+                                     tc5::mbar_wait(free + buf, ((v / BUFS) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t bB = b0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
@@ -2054,7 +2066,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           for (int kk = 0; kk < D / 16; ++kk)      // a k-step of 16 bf16 is 8 TMEM columns of the A operand
             tc5::mma_ts(tmem + buf * 128 + dcol, tmem + acol + kk * 8, bB + static_cast<uint64_t>(((kk >> 2) * HALF + (kk & 3) * 32) >> 4),
                         id_s, kk > 0 ? 1u : 0u);
-          tc5::mma_commit(s_full + buf);
+          tc5::mma_commit(made + buf);
         }
         __syncwarp();
       }
@@ -2075,13 +2087,13 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         const uint64_t bKmn = bKmn0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
         if (lead) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)          // dQ += dS K: keys 0-31 sit in columns 0-15, keys 32-63 in columns 32-47
-            tc5::mma_ts(tmem + cDQ, tmem + buf * 128 + (kk >> 1) * 32 + (kk & 1) * 8, bKmn + static_cast<uint64_t>((kk * 2048) >> 4),
+          for (int kk = 0; kk < 4; ++kk)          // dQ += dS K; without groups keys 0-31 sit in columns 0-15, keys 32-63 in columns 32-47
+            tc5::mma_ts(tmem + cDQ, tmem + buf * 128 + (GROUPS ? 64 + kk * 8 : (kk >> 1) * 32 + (kk & 1) * 8), bKmn + static_cast<uint64_t>((kk * 2048) >> 4),
                         id_q, (u > 0 || kk > 0) ? 1u : 0u);
           // S and dP of this visit completed before dS could be written, so the commits of this warp
           // alone release the stage and the buffer
           tc5::mma_commit(kv_empty + st);
-          tc5::mma_commit(s_empty + buf);          // the S / dP / dS columns of this buffer are free again
+          tc5::mma_commit((GROUPS ? dp_empty : s_empty) + buf);     // the columns of dS are free again
         }
         __syncwarp();
       }
@@ -2113,18 +2125,19 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
     // selected mode: the block id and token mask of visit v+1 are fetched during visit v, so the
     // global-memory latency is off the per-visit critical path
-    int blk_n = (selected && n_vis > 0) ? blocks[0] : 0;
-    unsigned long long msk_n = (selected && n_vis > 0) ? masks[0] : 0ull;
-    for (int v = 0; v < n_vis && ok; ++v) {
+    const int first = GROUPS ? ch : 0, step = GROUPS ? 2 : 1;
+    int blk_n = (selected && first < n_vis) ? blocks[first] : 0;
+    unsigned long long msk_n = (selected && first < n_vis) ? masks[first] : 0ull;
+    for (int v = first; v < n_vis && ok; v += step) {
       const int buf = v % BUFS;
       int sb;
       bool row_sel = row_ok;
-      if (!selected) sb = (kb0 + v) * 64 + ch * 32;
+      if (!selected) sb = (kb0 + v) * 64 + (GROUPS ? 0 : ch * 32);
       else {
         const int blk = blk_n;
         const unsigned long long msk = msk_n;
-        if (v + 1 < n_vis) { blk_n = blocks[v + 1]; msk_n = masks[v + 1]; }
-        sb = blk < 0 ? -1 : blk * 64 + ch * 32;
+        if (v + step < n_vis) { blk_n = blocks[v + step]; msk_n = masks[v + step]; }
+        sb = blk < 0 ? -1 : blk * 64 + (GROUPS ? 0 : ch * 32);
         row_sel = row_ok && blk >= 0 && ((msk >> (tok_local & 63)) & 1ull);
       }
       if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + buf, (v / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
@@ -2132,30 +2145,66 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         break;
       }
       tc5::fence_after_sync();
-      uint32_t sv[32], dv[32], ds[16];
-      tc5::tmem_ld_x32(tmem + lane_off + buf * 128 + ch * 32, sv);
-      tc5::tmem_ld_x32(tmem + lane_off + buf * 128 + 64 + ch * 32, dv);
-      tc5::tmem_ld_wait();
-      if (!row_sel) {
+      if constexpr (GROUPS) {
+        uint32_t sv[64];
+        tmem_ld64(tmem + lane_off + buf * 128, sv);
+        tc5::fence_before_sync();
+        tc5::mbar_arrive(s_empty + buf);           // S of a later visit may be computed while this one is exponentiated
+        if (row_sel) {
+          bool check = sb + 63 >= p.S;
+          if (p.causal) check = check || ((sb + 63) * p.kp_stride + p.kp_off > t);
+          if (p.window > 0) check = check || (sb * p.kp_stride + p.kp_off <= t - p.window);
+          if (check) mask_scores<64>(p, sv, sb, t);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) ds[i] = 0u;
-      } else {
-        bool check = sb + 31 >= p.S;
-        if (p.causal) check = check || ((sb + 31) * p.kp_stride + p.kp_off > t);
-        if (p.window > 0) check = check || (sb * p.kp_stride + p.kp_off <= t - p.window);
-        if (check) mask_scores<32>(p, sv, sb, t);
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {                 // masked scores are -inf: their probability is 0
-          const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), sc, negL));
-          const float p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), sc, negL));
-          ds[i / 2] = tc5::pack_bf16(p0 * fmaf(__uint_as_float(dv[i]), scale, nds),
-                                     p1 * fmaf(__uint_as_float(dv[i + 1]), scale, nds));
+          for (int i = 0; i < 64; ++i)                      // masked scores are -inf: their probability is 0
+            sv[i] = __float_as_uint(exp2f(fmaf(__uint_as_float(sv[i]), sc, negL)));
         }
+        if (!__all_sync(0xffffffffu, tc5::mbar_wait(dp_full + buf, (v / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+          ok = false;
+          break;
+        }
+        tc5::fence_after_sync();
+        uint32_t ds[32];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t dv[32];
+          tc5::tmem_ld_x32(tmem + lane_off + buf * 128 + 64 + c * 32, dv);
+          tc5::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            const float p0 = __uint_as_float(sv[c * 32 + i]), p1 = __uint_as_float(sv[c * 32 + i + 1]);
+            ds[c * 16 + i / 2] = row_sel ? tc5::pack_bf16(p0 * fmaf(__uint_as_float(dv[i]), scale, nds), p1 * fmaf(__uint_as_float(dv[i + 1]), scale, nds)) : 0u;
+          }
+        }
+        tc5::tmem_st_x32(tmem + lane_off + buf * 128 + 64, ds);      // in the place of dP, which is in registers
+        tc5::tmem_st_wait();
+        tc5::fence_before_sync();
+      } else {
+        uint32_t sv[32], dv[32], ds[16];
+        tc5::tmem_ld_x32(tmem + lane_off + buf * 128 + ch * 32, sv);
+        tc5::tmem_ld_x32(tmem + lane_off + buf * 128 + 64 + ch * 32, dv);
+        tc5::tmem_ld_wait();
+        if (!row_sel) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) ds[i] = 0u;
+        } else {
+          bool check = sb + 31 >= p.S;
+          if (p.causal) check = check || ((sb + 31) * p.kp_stride + p.kp_off > t);
+          if (p.window > 0) check = check || (sb * p.kp_stride + p.kp_off <= t - p.window);
+          if (check) mask_scores<32>(p, sv, sb, t);
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {                 // masked scores are -inf: their probability is 0
+            const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), sc, negL));
+            const float p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), sc, negL));
+            ds[i / 2] = tc5::pack_bf16(p0 * fmaf(__uint_as_float(dv[i]), scale, nds),
+                                       p1 * fmaf(__uint_as_float(dv[i + 1]), scale, nds));
+          }
+        }
+        // dS replaces the first half of this thread's own S columns
+        tc5::tmem_st_x16(tmem + lane_off + buf * 128 + ch * 32, ds);
+        tc5::tmem_st_wait();
+        tc5::fence_before_sync();
       }
-      // dS replaces the first half of this thread's own S columns
-      tc5::tmem_st_x16(tmem + lane_off + buf * 128 + ch * 32, ds);
-      tc5::tmem_st_wait();
-      tc5::fence_before_sync();
       tc5::mbar_arrive(ds_full + buf);
     }
     // what dQ is added to, fetched behind the last products (16384 tokens x 32 heads, three branches: 2129 -> 2065 us)
@@ -3521,6 +3570,13 @@ void fill_params(AttnParams& p, int B, int T, int S, int Hq, int Hkv, int D, flo
 }
 }  // namespace
 
+// dQ with groups of softmax warps on alternate visits?  us without, with groups, head_dim 128: 300 tokens x 16 / 8 heads 9.2, 9.6; 1000 x 32 / 2 22.8,
+// 22.9; 2500 x 32 / 8 90.7, 86.3; 4096 x 16 / 8 103, 96; 8192 x 32 / 2 682, 638, window 512 177, 177.  A tile of few visits is set up as
+// long as before and ends a longer step later.  head_dim 64, whose third buffer does for all warps: 4096 x 16 / 8 92, 94; 8192 x 32 / 2 641, 641.
+static bool dq_in_groups(const AttnParams& p) {
+  return p.D == 128 && (std::min(p.S, p.window > 0 ? p.window + p.R : p.S) + 63) / 64 > 16;
+}
+
 // Two CTAs per SM with one softmax group each, or one with two?  A lone CTA takes its visits in one chain where the other form has two,
 // so all SMs must have two CTAs for most of the time: three tiles for each SM, or more than one where tiles are short.  us of two groups and
 // of one, head_dim 64: 160 CTAs x 5 visits 10.8, 8.9; 250 x 9 17.6, 14.6; 256 x 16 17.9, 18.9; 500 x 16 34, 26; 256 x 32 26, 32; 504 x 32 49, 39;
@@ -3772,9 +3828,10 @@ extern "C" int nsa_attn_bwd_split(const void* q, const void* k, const void* v, c
     const dim3 grid((T + p.R - 1) / p.R, Hkv, B);
     static const bool smem_operands = [] { const char* e = getenv("NSA_B200_ATTN_DQ"); return e && !strcmp(e, "smem"); }();
     if (!smem_operands || D == 64) {
-      auto* kernel = D == 128 ? attn_bwd_dq_ts_kernel<128> : attn_bwd_dq_ts_kernel<64>;
-      static bool cfg[2] = {};
-      bool& ready = cfg[D == 128];
+      const bool groups = dq_in_groups(p);
+      auto* kernel = D == 64 ? attn_bwd_dq_ts_kernel<64, false> : groups ? attn_bwd_dq_ts_kernel<128, true> : attn_bwd_dq_ts_kernel<128, false>;
+      static bool cfg[3] = {};
+      bool& ready = cfg[D == 64 ? 0 : 1 + groups];
       if (!ready) { if ((rc = set_smem(kernel, dqt_smem(D)))) return rc; ready = true; }
       kernel<<<grid.x * Hkv * B, 384, dqt_smem(D), st>>>(tq, tdo, tk, tv, p, scale);
     } else {
