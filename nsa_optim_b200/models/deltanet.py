@@ -78,8 +78,7 @@ class GatedDeltaNetMixer(nn.Module):
         q = ops.l2_norm(q.view(B, T, H, K))
         k = ops.l2_norm(k.view(B, T, H, K))
         v = v.view(B, T, H, V)
-        beta = torch.sigmoid(outs[3].float())
-        g = -torch.exp(self.A_log.float()) * F.softplus(outs[4].float() + self.dt_bias.float())
+        g, beta = ops.delta_gates(outs[4], outs[3], self.dt_bias, self.A_log)
         o = ops.gated_delta_rule(q, k, v, g, beta, scale=K ** -0.5, chunk=self.chunk_size)
         if self.use_gate:
             gate = outs[5].view(B, T, H, V)

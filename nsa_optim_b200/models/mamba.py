@@ -64,8 +64,7 @@ class Mamba2Mixer(nn.Module):
         z, xBC, dt = split_last(zxbcdt, [d_in, d_in + 2 * gn, H])
         xBC = ops.causal_conv1d(xBC, self.conv1d.weight.squeeze(1), self.conv1d.bias, activation=True)
         x, Bm, Cm = split_last(xBC, [d_in, gn, gn])
-        dt = F.softplus(dt.float() + self.dt_bias.float())
-        A = -torch.exp(self.A_log.float())
+        dt, A = ops.step_sizes(dt, self.dt_bias, self.A_log)
         y = ops.ssd_scan(x.reshape(B, T, H, self.headdim), dt, A,
                          Bm.reshape(B, T, self.ngroups, self.d_state),
                          Cm.reshape(B, T, self.ngroups, self.d_state), self.D, self.chunk_size)

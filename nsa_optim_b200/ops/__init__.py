@@ -226,6 +226,18 @@ def causal_conv1d(x: Tensor, weight: Tensor, bias: Optional[Tensor], activation:
     return torch_impl.causal_conv1d(x, weight, bias, activation)
 
 
+def step_sizes(dt: Tensor, dt_bias: Tensor, A_log: Tensor):
+    """(softplus(dt + dt_bias), -exp(A_log)) in fp32: step sizes and decay rates of the Mamba-2 scan."""
+    out = native_module().step_sizes(dt, dt_bias, A_log) if _use_native(dt, "ssd_scan") else None
+    return torch_impl.step_sizes(dt, dt_bias, A_log) if out is None else out
+
+
+def delta_gates(a: Tensor, b: Tensor, dt_bias: Tensor, A_log: Tensor):
+    """(-exp(A_log) softplus(a + dt_bias), sigmoid(b)) in fp32: log-decay and beta of the gated delta rule."""
+    out = native_module().delta_gates(a, b, dt_bias, A_log) if _use_native(a, "gated_delta_rule") else None
+    return torch_impl.delta_gates(a, b, dt_bias, A_log) if out is None else out
+
+
 def ssd_scan(x, dt, A, Bm, Cm, D=None, chunk: int = 256) -> Tensor:
     if _use_native(x, "ssd_scan"):
         return native_module().ssd_scan(x, dt, A, Bm, Cm, D, chunk)

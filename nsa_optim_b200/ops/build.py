@@ -28,6 +28,7 @@ LIB = os.path.join(HERE, "libnsa_b200.so")
 HOST = os.path.join(HERE, "_nsa_host.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+EXACT = {"gates.cu"}          # without fast math: the bits of PyTorch's kernels
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "--use_fast_math", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3"]
 
 
@@ -50,7 +51,8 @@ def _newest_header() -> float:
 def _compile(nvcc: str, name: str, extra: List[str], verbose: bool, obj_dir: str = OBJ) -> str:
     src = os.path.join(SRC, name)
     obj = os.path.join(obj_dir, name[:-3] + ".o")
-    cmd = [nvcc] + ARCH + COMMON + extra + ["-I", SRC, "-c", src, "-o", obj]
+    common = [f for f in COMMON if name not in EXACT or f != "--use_fast_math"]
+    cmd = [nvcc] + ARCH + common + extra + ["-I", SRC, "-c", src, "-o", obj]
     if verbose:
         cmd.insert(1, "-Xptxas=-v")
         print(" ".join(cmd), flush=True)

@@ -39,7 +39,7 @@ using at::Tensor;
   X(nsa_gate_combine_fwd_ex) X(nsa_gate_combine_bwd_ex) X(nsa_pool_fwd) X(nsa_pool_bwd) X(nsa_gdn_prep) X(nsa_gdn_seq_fwd)           \
   X(nsa_gdn_seq_bwd) X(nsa_gdn_post) X(nsa_ssd_states_form) X(nsa_ssd_states) X(nsa_ssd_chunk_state) X(nsa_ssd_state_fwd)         \
   X(nsa_ssd_state_bwd) X(nsa_ssd_chunk_out) X(nsa_ssd_chunk_grad) X(nsa_ssd_grad_slots) X(nsa_ssd_finish) X(nsa_adamw_multi)         \
-  X(nsa_adamw8bit_multi)
+  X(nsa_adamw8bit_multi) X(nsa_gates)
 
 struct Lib {
 #define X(f) decltype(&::f) f = nullptr;
@@ -977,6 +977,28 @@ OP(ssd_bwd) {                                    // x, dt, A, B, C, D, decays, s
   });
 }
 
+// Rows of one pitch, the last dimension dense: used in place
+Tensor pitched(const Tensor& t) {
+  bool ok = t.stride(-1) == 1;
+  for (long k = t.dim() - 2; k > 0; --k) ok = ok && t.stride(k - 1) == t.size(k) * t.stride(k);
+  return ok ? t : t.contiguous();
+}
+OP(gates) {                                      // a, b or None, bias, A_log -> g and beta, or dt and A (fp32)
+  return entry(py, np, [](Args& a) {
+    const Tensor& x = a.t();
+    const Tensor b = a.opt();
+    const Tensor &bias = a.t(), &A_log = a.t();
+    return [=]() -> List {
+      const Tensor xp = pitched(x), bp = b.defined() ? pitched(b) : b, bc = dense(bias), Ac = dense(A_log);
+      const long H = x.size(-1);
+      const Tensor out0 = alloc(x.sizes(), F32, x.device()), out1 = b.defined() ? alloc(x.sizes(), F32, x.device()) : alloc({H}, F32, x.device());
+      launch(lib.nsa_gates, ptr(xp), xp.stride(-2), ptr(bp), b.defined() ? bp.stride(-2) : 0l, ptr(bc), static_cast<int>(bc.scalar_type() == F32),
+             ptr(Ac), static_cast<int>(Ac.scalar_type() == F32), fp(out0), fp(out1), rows_of(xp), dim(H));
+      return {out0, out1};
+    };
+  });
+}
+
 // ------------------------------------------------------------------------------------- optimizer lists
 void need(const char* what, PyObject* o, long n) {
   if (o == Py_None) return;
@@ -1093,7 +1115,7 @@ PyMethodDef methods[] = {
     M(bind), M(gemm_single), M(split_k_choice), M(rms_fwd), M(add_rms_fwd), M(rms_bwd), M(gated_rms_fwd), M(gated_rms_bwd), M(l2_fwd), M(l2_bwd),
     M(swiglu_fwd), M(swiglu_bwd), M(rope), M(conv_fwd), M(conv_bwd), M(embedding_fwd), M(matmul), M(linear_fwd), M(multi_linear_fwd),
     M(multi_linear_bwd), M(cross_entropy_fwd), M(scale), M(attn_fwd), M(attn_bwd), M(union_blocks), M(inverse_blocks), M(importance), M(select),
-    M(gates_fwd), M(gates_bwd), M(pool_fwd), M(pool_bwd), M(nsa_bwd), M(gdn_fwd), M(gdn_bwd), M(ssd_fwd), M(ssd_bwd), M(adamw), M(adamw8bit),
+    M(gates_fwd), M(gates_bwd), M(pool_fwd), M(pool_bwd), M(nsa_bwd), M(gdn_fwd), M(gdn_bwd), M(ssd_fwd), M(ssd_bwd), M(gates), M(adamw), M(adamw8bit),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_nsa_host", "Host side of the native ops.", -1, methods};
 }  // namespace

@@ -151,6 +151,10 @@ int nsa_gdn_post(const void* q, const void* k, const void* v, const void* d_o, c
     const float* X, const void* v_new, const void* du, const void* S, const void* dS, const float* dgamma, void* dq,
     void* dk, void* dv, float* dg, float* dbeta, int B, int T, int H, int K, int V, float scale, cudaStream_t st);
 
+/* ---- step sizes and gates of the recurrent mixers (csrc/gates.cu), rows of pitch lda / ldb; b null: dt and A ---- */
+int nsa_gates(const void* a, long lda, const void* b, long ldb, const void* bias, int bias_fp32, const void* A_log, int A_fp32,
+    float* out0, float* out1, long rows, int H, cudaStream_t st);
+
 /* ---- GEMM (csrc/gemm.cu) ---- */
 /* C32 (zeroed or to be added to) += op(A) op(B), the reduction cut into split_k parts. */
 int nsa_gemm_bf16_splitk(const void* A, const void* B, float* C32, int M, int N, int K, int lda, int ldb, int ldc,

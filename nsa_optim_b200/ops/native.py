@@ -119,17 +119,19 @@ class _NoRecord:
     mark_non_differentiable = save_for_backward
 
 
-def _run(fn, *args):
-    """fn.apply(*args); where autograd has nothing to record, the forward alone (a third of the host time of a small op).
-    Transforms, forward-mode derivatives and tracers see the function as before."""
+def _recorded(args) -> bool:
+    """Whether autograd, a transform, a forward-mode derivative or a tracer has something to see in a call."""
     if torch.is_grad_enabled():
         for a in args:
             if isinstance(a, Tensor) and a.requires_grad:
-                return fn.apply(*args)
-    if (torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0 or torch._C._is_tracing()
-            or torch.compiler.is_compiling()):
-        return fn.apply(*args)
-    return fn.forward(_NoRecord(), *args)
+                return True
+    return (torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0 or torch._C._is_tracing()
+            or torch.compiler.is_compiling())
+
+
+def _run(fn, *args):
+    """fn.apply(*args); where nothing is recorded, the forward alone (a third of the host time of a small op)."""
+    return fn.apply(*args) if _recorded(args) else fn.forward(_NoRecord(), *args)
 
 
 def launch_count() -> int:
@@ -1038,6 +1040,24 @@ class _SSD(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         return _host.ssd_bwd(*ctx.saved_tensors, dy, ctx.has_D)
+
+
+def _gates(a, b, dt_bias, A_log):
+    """The two results of one launch (``csrc/gates.cu``), or None where autograd records or the layout is another."""
+    f32, bf = torch.float32, torch.bfloat16
+    if (a.dtype != bf or a.dim() < 2 or a.numel() == 0 or dt_bias.dtype not in (f32, bf) or A_log.dtype not in (f32, bf)
+            or dt_bias.shape != a.shape[-1:] or A_log.shape != a.shape[-1:] or (b is not None and (b.dtype != bf or b.shape != a.shape))
+            or _recorded((a, b, dt_bias, A_log))):
+        return None
+    return _h().gates(a, b, dt_bias, A_log)
+
+
+def step_sizes(dt, dt_bias, A_log):
+    return _gates(dt, None, dt_bias, A_log)
+
+
+def delta_gates(a, b, dt_bias, A_log):
+    return _gates(a, b, dt_bias, A_log)
 
 
 def copy_columns(dst: Tensor, src: Tensor) -> bool:

@@ -42,6 +42,7 @@ SIGNATURES = {
     "nsa_gate_combine_bwd_ex": "ippppppliipppppppppplip",
     "nsa_gate_combine_fwd": "ippppppplip",
     "nsa_gate_combine_fwd_ex": "ippppppliiplip",
+    "nsa_gates": "iplplpipipplip",
     "nsa_gdn_post": "ipppppppppppppppppiiiiifp",
     "nsa_gdn_prep": "ippppppppppiiiiifp",
     "nsa_gdn_seq_bwd": "ippppppppppiiiiifp",

@@ -250,6 +250,14 @@ def nsa_attention(q: Tensor, k: Tensor, v: Tensor, g_cmp: Tensor, g_slc: Tensor,
 
 
 # ------------------------------------------------------------------ Mamba-2 SSD (chunked)
+def step_sizes(dt: Tensor, dt_bias: Tensor, A_log: Tensor) -> Tuple[Tensor, Tensor]:
+    return F.softplus(dt.float() + dt_bias.float()), -torch.exp(A_log.float())
+
+
+def delta_gates(a: Tensor, b: Tensor, dt_bias: Tensor, A_log: Tensor) -> Tuple[Tensor, Tensor]:
+    return -torch.exp(A_log.float()) * F.softplus(a.float() + dt_bias.float()), torch.sigmoid(b.float())
+
+
 def ssd_scan(x: Tensor, dt: Tensor, A: Tensor, Bm: Tensor, Cm: Tensor, D: Optional[Tensor] = None,
              chunk: int = 256, initial_state: Optional[Tensor] = None, return_state: bool = False):
     """Chunked evaluation of ``oracle.ssd_scan``.  fp32 decays and states, matmuls in the
