@@ -430,7 +430,10 @@ long split_k(long M, long N, long K, long clusters) {
   long best = 1;
   for (long S = 2; S <= g_splitk_max; ++S)
     if (fill(S) - 0.01 * S > fill(best) - 0.01 * best) best = S;
-  return fill(best) > fill(1) + 0.04 ? best : 1;
+  // Parts cost a pass that clears the fp32 sums and one that converts them, 1.6 ps an element; of the time that fuller waves save,
+  // 1.25 fs a product, two fifths remain (sums pass through L2, and under the power cap idle SMs let the others clock higher).  5632 x
+  // 2048: K = 8192 143 us in one part, 133 + 18 in two; K = 65536 saves 80.
+  return fill(best) > fill(1) + 0.04 && K * (1 / fill(1) - 1 / fill(best)) > 3200 ? best : 1;
 }
 
 // C = op(A) op(B); a_mn: A is (K, M), b_mn: B is (K, N).  out undefined: allocated as (M, N).  parts 0: chosen.
