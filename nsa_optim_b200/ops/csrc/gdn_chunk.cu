@@ -246,23 +246,43 @@ struct PostParams {
   float *dg, *dbeta;                    // [B, T, H]
   int B, T, H, NC, V;
   float scale;
-  int resident;
   KernelStatus* status;
 };
 
-// Stage: 64 columns of [du ; do], [v_new ; v] (128 rows each), S, dS, as 128-byte-swizzled TMA tiles.
+// Tiles of 64 value columns, 128-byte-swizzled as TMA writes them: [du ; do] and [v_new ; v] (128 rows each) in one of two
+// places, S and dS in a third.
 constexpr int TILE = 128 * 128;
-constexpr int POST_STAGE = 4 * TILE;
-constexpr int PF = KD + 4;                                                 // pitch of the fp32 [64][128] tiles
-constexpr int POST_SMEM = 2 * POST_STAGE + 2 * CH * PK * 2 + CH * PX * 4 + CH * PC * 2 + (2 + 16) * CH * 4 + 64 + 1024;
+constexpr int POST_A1 = 2 * TILE, POST_B = POST_A1 + 2 * CH * PK * 2;      // the tail's tiles of k and q fill the second place
+constexpr int POST_TILES = POST_B + 2 * TILE;
+constexpr int POST_RED = 16;                                               // rows of partial sums
+constexpr int POST_SMEM = POST_TILES + CH * PC * 2 + (2 + POST_RED) * CH * 4 + 128 + 1024;
+constexpr int FX = CH * CH * 4, FF = CH * KD * 4;                          // fp32 tiles of the tail, rows without padding
 static_assert(PC <= PK && CH * PC * 2 <= CH * PX * 4, "gdn prep: operand tiles");
-static_assert(4 * CH * PX * 4 + CH * PK * 2 + 3 * CH * PC * 2 <= 2 * POST_STAGE, "gdn post: tail tiles");
-static_assert(2 * CH * PF * 4 <= 4 * CH * PX * 4, "gdn post: result tiles");
+static_assert(POST_B % 1024 == 0 && 2 * TILE <= 2 * CH * PK * 2, "gdn post: swizzled tiles");
+static_assert(2 * FX <= POST_A1 && CH * PC * 2 <= FX, "gdn post: X, dX and what takes their places");
+static_assert(TILE + FX <= 2 * TILE && FF <= POST_A1 && FF <= 2 * TILE, "gdn post: dw, X^T dX, results");
+static_assert(2 * (POST_SMEM + 1024) <= 228 * 1024, "gdn post: two CTAs per SM");
 
-// B fragments of 16 columns n0.. from a swizzled tile stored [k][64 n]
+// Fragments of a swizzled tile.  A: rows m0.., reduction k0..; B: 16 columns n0.. from [n][k] or (_t) from [k][n].
+__device__ __forceinline__ void ldsm4_swz(uint32_t (&r)[4], const uint8_t* tile, int row, int chunk) {
+  ldsm4(r, reinterpret_cast<const bf16*>(tile + row * 128 + ((chunk ^ (row & 7)) << 4)));
+}
+__device__ __forceinline__ void load_a_swz(uint32_t (&r)[4], const uint8_t* tile, int m0, int k0) {
+  const int l = threadIdx.x & 31;
+  ldsm4_swz(r, tile, m0 + (l & 15), (k0 >> 3) + (l >> 4));
+}
+__device__ __forceinline__ void load_b_swz(uint32_t (&r)[4], const uint8_t* tile, int n0, int k0) {
+  const int l = threadIdx.x & 31, i = l >> 3;
+  ldsm4_swz(r, tile, n0 + (i >> 1) * 8 + (l & 7), (k0 >> 3) + (i & 1));
+}
 __device__ __forceinline__ void load_b_t_swz(uint32_t (&r)[4], const uint8_t* tile, int n0, int k0) {
   const int l = threadIdx.x & 31, i = l >> 3, row = k0 + (i & 1) * 8 + (l & 7), chunk = (n0 >> 3) + (i >> 1);
   ldsm4_t(r, reinterpret_cast<const bf16*>(tile + row * 128 + ((chunk ^ (row & 7)) << 4)));
+}
+// Element (r, c) of an fp32 tile of W columns: groups of four are spread over the banks by row.
+template <int W>
+__device__ __forceinline__ int spread(int r, int c) {
+  return r * W + ((((c >> 2) ^ r) & 15) << 2) + (c & ~63) + (c & 3);
 }
 __device__ __forceinline__ float dot32(const float (&a)[32], const bf16* b) {
   float s = 0.f;
@@ -278,90 +298,88 @@ __device__ __forceinline__ float dot32(const float (&a)[32], const bf16* b) {
   }
   return s;
 }
-template <int N>
-__device__ __forceinline__ void tmem_cols(uint32_t taddr, float (&out)[N]) {
-  uint32_t a[N];
-  if constexpr (N == 32) tc5::tmem_ld_x32(taddr, a);
-  else tc5::tmem_ld_x16(taddr, a);
+__device__ __forceinline__ void tmem_cols(uint32_t taddr, float (&out)[32]) {
+  uint32_t a[32];
+  tc5::tmem_ld_x32(taddr, a);
   tc5::tmem_ld_wait();
 #pragma unroll
-  for (int j = 0; j < N; ++j) out[j] = __uint_as_float(a[j]);
+  for (int j = 0; j < 32; ++j) out[j] = __uint_as_float(a[j]);
 }
 
-// One CTA of sixteen warps per (chunk, head): every gradient of the chunk once du (of the sequential pass) and
+// One CTA of sixteen warps per (chunk, head), two per SM: every gradient of the chunk once du (of the sequential pass) and
 // the two states are known.
 //     dw = -du S^T, dqs = do S^T, dks = v_new dS^T, dqk = do v_new^T, dTu = du v^T, dTw = dw k^T
 //     dX = (dTu + dTw e^gc) beta (columns), dA = -(X^T dX X^T), then through the definitions above.
-// The five products that sum over the value dimension are three full tcgen05 tiles of the stacked operands,
-// [du ; do] S^T, [v_new ; v] dS^T and [du ; do] [v_new ; v]^T, accumulated in tensor memory while slices of 64 value
-// columns stream through two TMA stages (as warp products with register accumulators they were two thirds of the
-// kernel: 700 us at 16384 tokens x 16 heads).  What is left are 64-row products, done by warps; they are two thirds of a CTA's 42000 cycles,
-// and one CTA fills an SM, so the next chunk's tiles are asked for into L2 meanwhile (670 us without that and with
-// 2 x 4 tiles for dA, 641 with both, 632 with the operands of dv read once per chunk and no loads under conditions).  Per token and head
-// 3.5 KB come in and 1 KB goes out, against 6 KB alone for the per-V-tile partials of dw, dq and dk that the sequential
-// pass would otherwise write and re-read.
-__global__ void __launch_bounds__(512, 1)
+// Of the products that sum over the value dimension, those with a state are two full tcgen05 tiles of the stacked operands,
+// [du ; do] S^T and [v_new ; v] dS^T, accumulated in tensor memory (half of it per CTA) while slices of 64 value columns stream
+// through; dqk and dTu, of which only the lower triangle counts, are warp products whose accumulators stay in the registers that
+// the tail wants them in.  The rest are 64-row products in a chain of phases.  One CTA per SM left the SM idle in that chain (a
+// chunk took 42000 cycles, a quarter of them issued an instruction), so two share it and each fills the other's waits: 112 KB
+// hold three 32 KB places for the slices and every tile of the tail lies over them (fp32 tiles without padding, Tw^T as a row
+// scaling of Tu^T), and 64-row products leave out the blocks above the diagonal.  What bounds it now is the shared-memory pipe, 70 %
+// busy; asking for the next chunk's tiles in L2 ahead only delays this one's (462 us without, 485 with).  16384 tokens x 16 heads,
+// values 256 wide: 637 us with one CTA per SM, 449 with two of sixteen warps at 64 registers, 455 with two of eight and one that copies and
+// issues.  Per token and head 3.5 KB come in and 1 KB goes out, against 6 KB alone for the per-V-tile partials of dw, dq
+// and dk that the sequential pass would otherwise write and re-read.
+__global__ void __launch_bounds__(512, 2)
 gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_vn, const __grid_constant__ CUtensorMap tm_v,
                 const __grid_constant__ CUtensorMap tm_S, const __grid_constant__ CUtensorMap tm_dS, const PostParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  bf16* sK = reinterpret_cast<bf16*>(stages + 2 * POST_STAGE);
-  bf16* sQ = sK + CH * PK;
-  float* Xs = reinterpret_cast<float*>(sQ + CH * PK);
-  bf16* sTu = reinterpret_cast<bf16*>(Xs + CH * PX);
+  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  bf16* sTu = reinterpret_cast<bf16*>(tiles + POST_TILES);
   float* gs = reinterpret_cast<float*>(sTu + CH * PC);
   float* bs = gs + CH;
-  float* red = bs + CH;                                    // [16][64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(red + 16 * CH);
-  uint64_t *full = bars, *done = bars + 2;                 // [2] each
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
+  float* red = bs + CH;                                    // [POST_RED][64]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(red + POST_RED * CH);
+  uint64_t *full_a = bars, *used_a = bars + 2, *done = bars + 4, *full_b = bars + 6;   // [2] each, full_b one
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  // over the stages once they are done
-  float* sDX = reinterpret_cast<float*>(stages);           // [64][PX], later dA
-  float* sY = sDX + CH * PX;
-  float* sT = sY + CH * PX;                                // dTu
-  float* sP = sT + CH * PX;                                // dqk
-  float* sFQ = sDX;                                        // [64][PF] over the four above, at the very end
-  float* sFK = sFQ + CH * PF;
-  bf16* sW = reinterpret_cast<bf16*>(sP + CH * PX);        // dw [64][PK]
-  bf16* sTw = sW + CH * PK;
-  bf16* sDK = sTw + CH * PC;                               // d(k k^T)
-  bf16* sDQ = sDK + CH * PC;                               // d(q k^T)
+  // the tail, over the slices: k and q over the second place while the last slice is in the first
+  float* Xs = reinterpret_cast<float*>(tiles);
+  float* sDX = reinterpret_cast<float*>(tiles + FX);
+  bf16* sDQ = reinterpret_cast<bf16*>(tiles);              // d(q k^T), over X
+  bf16* sDK = reinterpret_cast<bf16*>(tiles + FX);         // d(k k^T), over dX
+  bf16* sK = reinterpret_cast<bf16*>(tiles + POST_A1);
+  bf16* sQ = sK + CH * PK;
+  uint8_t* sW = tiles + POST_B;                            // dw, two swizzled tiles of 64 columns
+  float* sY = reinterpret_cast<float*>(tiles + POST_B + TILE);   // X^T dX, then dA
+  float* sFQ = reinterpret_cast<float*>(tiles);            // [64][128] at the very end
+  float* sFK = reinterpret_cast<float*>(tiles + POST_B);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bh = blockIdx.x, h = bh % p.H, b = bh / p.H, c = blockIdx.z * gridDim.y + blockIdx.y;   // see chunk_grid
   if (c >= p.NC) return;
   const int t0 = c * CH, V = p.V, nvt = V / CH;
   const long tok0 = static_cast<long>(b) * p.T * p.H + h;
   const long chunk = static_cast<long>(bh) * p.NC + c;
-  auto load_slice = [&](int s) {                           // one thread
-    uint8_t* d = stages + (s & 1) * POST_STAGE;
-    uint64_t* bar = full + (s & 1);
+  auto place = [&](int s) { return (nvt - 1 - s) & 1; };   // the last slice is in the first place
+  auto load_a_part = [&](int s) {                          // one thread
+    uint8_t* d = tiles + place(s) * POST_A1;
+    uint64_t* bar = full_a + place(s);
     const int row = static_cast<int>(chunk) * CH, x = s * CH;
-    tc5::mbar_expect_tx(bar, POST_STAGE);
+    tc5::mbar_expect_tx(bar, 2 * TILE);
     tc5::tma_load_2d(d, &tm_du, bar, x, row);
     tc5::tma_load_4d(d + TILE / 2, &tm_do, bar, x, h, t0, b);
     tc5::tma_load_2d(d + TILE, &tm_vn, bar, x, row);
     tc5::tma_load_4d(d + TILE + TILE / 2, &tm_v, bar, x, h, t0, b);
-    tc5::tma_load_2d(d + 2 * TILE, &tm_S, bar, x, static_cast<int>(chunk) * KD);
-    tc5::tma_load_2d(d + 3 * TILE, &tm_dS, bar, x, static_cast<int>(chunk) * KD);
+  };
+  auto load_b_part = [&](int s) {
+    tc5::mbar_expect_tx(full_b, 2 * TILE);
+    tc5::tma_load_2d(tiles + POST_B, &tm_S, full_b, s * CH, static_cast<int>(chunk) * KD);
+    tc5::tma_load_2d(tiles + POST_B + TILE, &tm_dS, full_b, s * CH, static_cast<int>(chunk) * KD);
   };
   if (tid == 0) {
     *abort_flag = 0;
-    for (int i = 0; i < 2; ++i) { tc5::mbar_init(full + i, 1); tc5::mbar_init(done + i, 1); }
+    for (int i = 0; i < 2; ++i) { tc5::mbar_init(full_a + i, 1); tc5::mbar_init(used_a + i, 16); tc5::mbar_init(done + i, 1); }
+    tc5::mbar_init(full_b, 1);
     tc5::fence_barrier_init();
-    load_slice(0);
-    if (nvt > 1) load_slice(1);
+    load_a_part(0);
+    load_b_part(0);
+    if (nvt > 1) load_a_part(1);
   }
-  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 512); tc5::tmem_relinquish(); }
-  for (int i = tid; i < CH * (KD / 8); i += 512) {
-    const int r = i / (KD / 8), cc = (i % (KD / 8)) * 8, t = t0 + r;
-    const bool ok = t < p.T;
-    const long off = (tok0 + static_cast<long>(ok ? t : 0) * p.H) * KD + cc;
-    cp_async16(sK + r * PK + cc, p.k + off, ok);
-    cp_async16(sQ + r * PK + cc, p.q + off, ok);
-  }
-  cp_async_commit();
+  if (warp == 0) { tc5::tmem_alloc(tmem_slot, 256); tc5::tmem_relinquish(); }
+  const float4* xg = reinterpret_cast<const float4*>(p.X + chunk * CH * CH) + tid;
+  const float4 x4[2] = {xg[0], xg[512]};                   // X, for Tu
   if (tid < CH) {
     gs[tid] = p.gc[chunk * CH + tid];
     bs[tid] = t0 + tid < p.T ? p.beta[tok0 + static_cast<long>(t0 + tid) * p.H] : 0.f;
@@ -370,141 +388,147 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
   __syncthreads();
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  for (int i = tid; i < CH * CH / 4; i += 512) {
-    const int r = i / (CH / 4), j = (i % (CH / 4)) * 4;
-    const float4 x = *reinterpret_cast<const float4*>(p.X + (chunk * CH + r) * CH + j);
-    *reinterpret_cast<float4*>(Xs + r * PX + j) = x;
-    *reinterpret_cast<uint2*>(sTu + r * PC + j) = make_uint2(pack2(x.x * bs[j], x.y * bs[j + 1]), pack2(x.z * bs[j + 2], x.w * bs[j + 3]));
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = (tid + i * 512) / (CH / 4), j = (tid & 15) * 4;
+    *reinterpret_cast<uint2*>(sTu + r * PC + j) =
+        make_uint2(pack2(x4[i].x * bs[j], x4[i].y * bs[j + 1]), pack2(x4[i].z * bs[j + 2], x4[i].w * bs[j + 3]));
   }
-  cp_async_wait<0>();
   __syncthreads();
   // fragment view of warp products: rows m0.., 32 (of 128) or 16 (of 64) columns
   const int m0 = (warp & 3) * 16, n32 = (warp >> 2) * 32, n16 = (warp >> 2) * 16;
   const int r0 = m0 + (lane >> 2), cl = 2 * (lane & 3);    // first row and column offset of this lane's accumulator elements
+  const bool lower = n16 <= m0;                            // of a 64 x 64 product: not all above the diagonal
   // tensor-memory view: lane row (0..63 the upper operand of a stack, 64..127 the lower), 32 columns from n32
   const int row = (warp & 3) * 32 + lane, ri = row & 63;
   const bool upper = row < CH;                             // uniform in a warp
-  const uint32_t trow = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-  constexpr uint32_t cWQ = 0, cKS = 128, cPT = 256;        // accumulator columns of the three products
+  const uint32_t trow = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + n32;
+  constexpr uint32_t cWQ = 0, cKS = 128;                   // accumulator columns of the two products
   constexpr uint32_t idesc = tc5::make_idesc_bf16(128, 128, 0, 0);
-  uint32_t tut[CH / 16][4];                                // Tu^T, the same for every slice
-#pragma unroll
-  for (int q = 0; q < CH / 16; ++q) load_a_t(tut[q], sTu, PC, m0, q * 16);
-  bf16* dv_row = p.dv + (tok0 + static_cast<long>(t0 + r0) * p.H) * V + n16 + cl;
-  bool ok = true;
-  for (int s = 0; s < nvt; ++s) {
-    const uint8_t* st = stages + (s & 1) * POST_STAGE;
-    if (!tc5::mbar_wait(full + (s & 1), (s >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL)) ok = false;
-    if (__syncthreads_or(!ok)) { ok = false; break; }
-    if (warp == 0) {
-      const bool lead = tc5::elect_one();                  // converged warp, elected lane issues
-      tc5::fence_after_sync();
-      const uint64_t uo = tc5::desc_kmajor(tc5::smem_u32(st)), nv = tc5::desc_kmajor(tc5::smem_u32(st + TILE));
-      const uint64_t S = tc5::desc_kmajor(tc5::smem_u32(st + 2 * TILE)), dS = tc5::desc_kmajor(tc5::smem_u32(st + 3 * TILE));
-      if (lead) {
-#pragma unroll
-        for (int kk = 0; kk < CH / 16; ++kk) {
-          const uint64_t off = static_cast<uint64_t>((kk * 32) >> 4);
-          const uint32_t acc = s > 0 || kk > 0 ? 1u : 0u;
-          tc5::mma_ss(tmem + cWQ, uo + off, S + off, idesc, acc);
-          tc5::mma_ss(tmem + cKS, nv + off, dS + off, idesc, acc);
-          tc5::mma_ss(tmem + cPT, uo + off, nv + off, idesc, acc);
-        }
-        tc5::mma_commit(done + (s & 1));
-      }
-      __syncwarp();
-    }
-    // dv of this slice behind the MMAs: Tu^T du (row j needs i >= j only)
-    float dv[2][4] = {};
-#pragma unroll
-    for (int q = 0; q < CH / 16; ++q) {
-      if (q * 16 < m0) continue;
-      uint32_t bb[4];
-      load_b_t_swz(bb, st, n16, q * 16);
-      mma2(dv[0], dv[1], tut[q], bb);
-    }
-#pragma unroll
-    for (int hh = 0; hh < 2; ++hh)
-      if (t0 + r0 + 8 * hh < p.T)
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-          *reinterpret_cast<uint32_t*>(dv_row + static_cast<long>(8 * hh) * p.H * V + s * CH + n * 8) = pack2(dv[n][2 * hh], dv[n][2 * hh + 1]);
-    if (s + 2 < nvt) {
-      __syncthreads();                                     // du of this stage has been read by every warp
-      if (tid == 0) {
-        if (tc5::mbar_wait(done + (s & 1), (s >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) load_slice(s + 2);
-        else ok = false;
-      }
-    }
-  }
+  constexpr int ISSUER = 14;                               // copies and issues too: it has nothing of dTu and dqk
+  auto wait = [&](uint64_t* bar, int use, int code) {
+    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, use & 1, abort_flag, p.status, code)) != 0;
+  };
+  float dtu[2][4] = {}, dqk[2][4] = {};                    // rows m0.., columns n16..
   {
-    int nbh, nc;
-    if (next_chunk(p.resident, p.H, p.NC, nbh, nc)) {
-      const int nb = nbh / p.H, nh = nbh % p.H, nt = nc * CH;
-      const long nchunk = static_cast<long>(nbh) * p.NC + nc;
-      if (lane == 0 && warp < nvt) {                       // a slice per warp
-        const int x = warp * CH, row = static_cast<int>(nchunk) * CH;
-        tc5::tma_prefetch_2d(&tm_du, x, row);
-        tc5::tma_prefetch_4d(&tm_do, x, nh, nt, nb);
-        tc5::tma_prefetch_2d(&tm_vn, x, row);
-        tc5::tma_prefetch_4d(&tm_v, x, nh, nt, nb);
-        tc5::tma_prefetch_2d(&tm_S, x, static_cast<int>(nchunk) * KD);
-        tc5::tma_prefetch_2d(&tm_dS, x, static_cast<int>(nchunk) * KD);
+    bf16* dv_row = p.dv + (tok0 + static_cast<long>(t0 + r0) * p.H) * V + n16 + cl;
+    bool ok = true;
+    for (int s = 0; s < nvt; ++s) {
+      const uint8_t* st = tiles + place(s) * POST_A1;
+      if (!(ok = wait(full_a + place(s), s >> 1, STATUS_TIMEOUT_SMEM_FULL))) break;
+      if (warp == ISSUER) {
+        if (!(ok = wait(full_b, s, STATUS_TIMEOUT_SMEM_FULL))) break;
+        const bool lead = tc5::elect_one();                // converged warp, elected lane issues
+        tc5::fence_after_sync();
+        const uint32_t sa = tc5::smem_u32(st), sb = tc5::smem_u32(tiles + POST_B);
+        const uint64_t uo = tc5::desc_kmajor(sa), nv = tc5::desc_kmajor(sa + TILE), S = tc5::desc_kmajor(sb), dS = tc5::desc_kmajor(sb + TILE);
+        if (lead) {
+#pragma unroll
+          for (int kk = 0; kk < CH / 16; ++kk) {
+            const uint64_t off = static_cast<uint64_t>((kk * 32) >> 4);
+            const uint32_t acc = s > 0 || kk > 0 ? 1u : 0u;
+            tc5::mma_ss(tmem + cWQ, uo + off, S + off, idesc, acc);
+            tc5::mma_ss(tmem + cKS, nv + off, dS + off, idesc, acc);
+          }
+          tc5::mma_commit(done + (s & 1));
+        }
+        __syncwarp();
+        if (s + 1 < nvt) {                                 // the states' place is free once the MMAs are through
+          if (!(ok = wait(done + (s & 1), s >> 1, STATUS_TIMEOUT_TMEM_FULL))) break;
+          if (lead) load_b_part(s + 1);
+          __syncwarp();
+        }
       }
-      if (tid < 128) {                                     // 64 rows of 256 bytes
-        prefetch_l2(p.X + nchunk * CH * CH + tid * 32);
-      } else if (tid >= 256 && nt + (tid & 63) < p.T) {    // q and k, 128 bytes at a time
-        const bf16* src = tid < 384 ? p.q : p.k;
-        prefetch_l2(src + ((static_cast<long>(nb) * p.T + nt + (tid & 63)) * p.H + nh) * KD + (tid & 64));
+      // behind the MMAs: dTu += du v^T, dqk += do v_new^T
+      if (lower) {
+#pragma unroll
+        for (int kk = 0; kk < CH; kk += 16) {
+          uint32_t a[4], bb[4];
+          load_a_swz(a, st, m0, kk);
+          load_b_swz(bb, st + TILE + TILE / 2, n16, kk);
+          mma2(dtu[0], dtu[1], a, bb);
+          load_a_swz(a, st + TILE / 2, m0, kk);
+          load_b_swz(bb, st + TILE, n16, kk);
+          mma2(dqk[0], dqk[1], a, bb);
+        }
+      }
+      if (s + 1 == nvt) {                                  // k and q into the place of the slice before
+        if (s > 0 && !(ok = wait(used_a + 1, (s - 1) >> 1, STATUS_TIMEOUT_SMEM_EMPTY) &&
+                            wait(done + ((s - 1) & 1), (s - 1) >> 1, STATUS_TIMEOUT_TMEM_FULL))) break;
+#pragma unroll
+        for (int i = tid; i < CH * (KD / 8); i += 512) {
+          const int r = i / (KD / 8), cc = (i % (KD / 8)) * 8, t = t0 + r;
+          const bool in = t < p.T;
+          const long off = (tok0 + static_cast<long>(in ? t : 0) * p.H) * KD + cc;
+          cp_async16(sK + r * PK + cc, p.k + off, in);
+          cp_async16(sQ + r * PK + cc, p.q + off, in);
+        }
+        cp_async_commit();
+      }
+      // dv of this slice: Tu^T du (row j needs i >= j only)
+      float dv[2][4] = {};
+#pragma unroll
+      for (int q = 0; q < CH / 16; ++q) {
+        if (q * 16 < m0) continue;
+        uint32_t a[4], bb[4];
+        load_a_t(a, sTu, PC, m0, q * 16);
+        load_b_t_swz(bb, st, n16, q * 16);
+        mma2(dv[0], dv[1], a, bb);
+      }
+      if (s + 1 < nvt) tc5::arrive_warp(used_a + place(s));
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh)
+        if (t0 + r0 + 8 * hh < p.T)
+#pragma unroll
+          for (int n = 0; n < 2; ++n)
+            *reinterpret_cast<uint32_t*>(dv_row + static_cast<long>(8 * hh) * p.H * V + s * CH + n * 8) = pack2(dv[n][2 * hh], dv[n][2 * hh + 1]);
+      if (warp == ISSUER && s + 2 < nvt) {                 // its MMAs are through, see above
+        if (!(ok = wait(used_a + place(s), s >> 1, STATUS_TIMEOUT_SMEM_EMPTY))) break;
+        if (tc5::elect_one()) load_a_part(s + 2);
+        __syncwarp();
       }
     }
-  }
-  // the last two commits cover every product
-  if (ok) {
-    const int s = nvt - 1;
-    if (!tc5::mbar_wait(done + (s & 1), (s >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) ok = false;
-  }
-  if (__syncthreads_or(!ok)) {
-    if (tid == 0) {                                        // slices may still be in flight
-      tc5::mbar_drain(full);
-      tc5::mbar_drain(full + 1);
+    // the last commit covers every product
+    if (ok) ok = wait(done + ((nvt - 1) & 1), (nvt - 1) >> 1, STATUS_TIMEOUT_TMEM_FULL);
+    cp_async_wait<0>();
+    if (__syncthreads_or(!ok)) {
+      if (tid == 0) {                                      // slices may still be in flight
+        tc5::mbar_drain(full_a);
+        tc5::mbar_drain(full_a + 1);
+        tc5::mbar_drain(full_b);
+      }
+      __syncthreads();
+      if (warp == 0) tc5::tmem_dealloc(tmem, 256);
+      return;
     }
-    __syncthreads();
-    if (warp == 0) tc5::tmem_dealloc(tmem, 512);
-    return;
   }
   tc5::fence_after_sync();
+#pragma unroll
+  for (int i = tid; i < CH * CH / 4; i += 512) {
+    const int r = i / (CH / 4), j = (i % (CH / 4)) * 4;
+    cp_async16(Xs + spread<CH>(r, j), p.X + (chunk * CH + r) * CH + j, true);
+  }
+  cp_async_commit();
   const float g_last = gs[CH - 1];
-  // ---- out of tensor memory: dw as an operand, dTu and dqk as fp32 tiles, and the row sums q . dqs and k . dks (gates
-  //      that scale rows of q and k); dqs and dks stay where they are until the end
+  // ---- out of tensor memory: dw as an operand and the row sums q . dqs and k . dks (gates that scale rows of q and k);
+  //      dqs and dks stay where they are until the end
   {
-    float a[32], t16[16];
-    tmem_cols(trow + cWQ + n32, a);
-    float dot;
+    float a[32], dot;
+    tmem_cols(trow + cWQ, a);
     if (upper) {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<uint4*>(sW + ri * PK + n32 + 8 * j) =
+        *reinterpret_cast<uint4*>(sW + (n32 >> 6) * (TILE / 2) + ri * 128 + ((((n32 & 63) / 8 + j) ^ (ri & 7)) << 4)) =
             make_uint4(pack2(-a[8 * j], -a[8 * j + 1]), pack2(-a[8 * j + 2], -a[8 * j + 3]), pack2(-a[8 * j + 4], -a[8 * j + 5]),
                        pack2(-a[8 * j + 6], -a[8 * j + 7]));
-      tmem_cols(trow + cKS + n32, a);
+      tmem_cols(trow + cKS, a);
       dot = dot32(a, sK + ri * PK + n32);
     } else {
       dot = dot32(a, sQ + ri * PK + n32);
     }
     red[((upper ? 4 : 0) + (warp >> 2)) * CH + ri] = dot;
-    tmem_cols(trow + cPT + (upper ? CH : 0) + n16, t16);
-    float* dst = (upper ? sT : sP) + ri * PX + n16;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(dst + 4 * j) = make_float4(t16[4 * j], t16[4 * j + 1], t16[4 * j + 2], t16[4 * j + 3]);
   }
-  for (int i = tid; i < CH * CH / 4; i += 512) {
-    const int r = i / (CH / 4), j = (i % (CH / 4)) * 4;
-    const float4 x = *reinterpret_cast<const float4*>(Xs + r * PX + j);
-    *reinterpret_cast<uint2*>(sTw + r * PC + j) =
-        make_uint2(pack2(x.x * bs[j] * __expf(gs[j]), x.y * bs[j + 1] * __expf(gs[j + 1])),
-                   pack2(x.z * bs[j + 2] * __expf(gs[j + 2]), x.w * bs[j + 3] * __expf(gs[j + 3])));
-  }
+  cp_async_wait<0>();
   __syncthreads();
   // gradient of gc_i and beta_i, collected by thread i < 64
   float dgc = 0.f, dbeta = 0.f, dlast = 0.f;
@@ -518,14 +542,16 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
   // ---- dTw = dw k^T, dX
   {
     float aw[2][4] = {};
+    if (lower) {
 #pragma unroll
-    for (int kk = 0; kk < KD; kk += 16) {
-      uint32_t a[4], bb[4];
-      load_a(a, sW, PK, m0, kk);
-      load_b(bb, sK, PK, n16, kk);
-      mma2(aw[0], aw[1], a, bb);
+      for (int kk = 0; kk < KD; kk += 16) {
+        uint32_t a[4], bb[4];
+        load_a_swz(a, sW + (kk >> 6) * (TILE / 2), m0, kk & 63);
+        load_b(bb, sK, PK, n16, kk);
+        mma2(aw[0], aw[1], a, bb);
+      }
     }
-    __syncthreads();                                       // red is read
+    float* part = red + 8 * CH;                            // sums of beta and gc, per 16 rows
 #pragma unroll
     for (int n = 0; n < 2; ++n)
 #pragma unroll
@@ -536,8 +562,8 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           const int i = r0 + 8 * hh;
-          const float x = Xs[i * PX + j], tw = aw[n][2 * hh + e] * eg, d = sT[i * PX + j] + tw;
-          sDX[i * PX + j] = j <= i ? d * bj : 0.f;
+          const float x = Xs[spread<CH>(i, j)], tw = aw[n][2 * hh + e] * eg, d = dtu[n][2 * hh + e] + tw;
+          sDX[spread<CH>(i, j)] = j <= i ? d * bj : 0.f;
           cb += d * x;                                     // x is zero above the diagonal
           cg += tw * x;
         }
@@ -548,72 +574,89 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
           cg += __shfl_xor_sync(0xffffffffu, cg, o);
         }
         if (lane < 4) {
-          red[(warp & 3) * CH + j] = cb;
-          red[(4 + (warp & 3)) * CH + j] = cg;
+          part[(warp & 3) * CH + j] = cb;
+          part[(4 + (warp & 3)) * CH + j] = cg;
         }
       }
   }
   __syncthreads();
   if (tid < CH)
 #pragma unroll
-    for (int n = 0; n < 4; ++n) { dbeta += red[n * CH + tid]; dgc += red[(4 + n) * CH + tid]; }
-  // ---- dA = -(X^T dX X^T) below the diagonal, fp32; 4 x 4 tiles of eight warps (2 x 4 of sixteen read shared memory twice as
-  //      often as they multiply).  Warp w owns rows 8 w .. 8 w + 7.
+    for (int n = 0; n < 4; ++n) { dbeta += red[(8 + n) * CH + tid]; dgc += red[(12 + n) * CH + tid]; }
+  // ---- dA = -(X^T dX X^T) below the diagonal, fp32.  Warp w owns rows a = 4 w .. 4 w + 3 of y = X^T dX and of dA, so there is
+  //      no barrier in between.  y[a][c] is wanted for c < a only and its sum starts at i = a: the warps of the upper half, whose
+  //      sums are long and rows short, give half of the sum to the lanes that would have the other columns.
   {
-    const int ra = (tid >> 4) * 4, cc = tid & 15;
-    if (tid < 256) {
-      float2 y[4][2] = {};
+    const int a0 = warp * 4;
+    {
+      const bool split = warp < 8;
+      const int cc = (split ? lane & 15 : lane) * 2;
+      const int len = split ? (CH - a0) / 2 : CH - a0, from = a0 + (split ? (lane >> 4) * len : 0);
+      float2 y[2][2] = {};                                 // rows a0, a0 + 1 and a0 + 2, a0 + 3; two columns
 #pragma unroll 4
-      for (int i = warp * 8; i < CH; ++i) {                // X[i][a] is zero for i < a
-        const float4 x = *reinterpret_cast<const float4*>(Xs + i * PX + ra), d = *reinterpret_cast<const float4*>(sDX + i * PX + cc * 4);
-        const float2 d0 = make_float2(d.x, d.y), d1 = make_float2(d.z, d.w);
-        const float xa[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          y[e][0] = fma2(make_float2(xa[e], xa[e]), d0, y[e][0]);
-          y[e][1] = fma2(make_float2(xa[e], xa[e]), d1, y[e][1]);
-        }
+      for (int i = from; i < from + len; ++i) {            // X[i][a] is zero for i < a
+        const float4 x = *reinterpret_cast<const float4*>(Xs + spread<CH>(i, a0));
+        const float2 d = *reinterpret_cast<const float2*>(sDX + spread<CH>(i, cc));
+        const float2 d0 = make_float2(d.x, d.x), d1 = make_float2(d.y, d.y);
+        y[0][0] = fma2(make_float2(x.x, x.y), d0, y[0][0]);
+        y[0][1] = fma2(make_float2(x.x, x.y), d1, y[0][1]);
+        y[1][0] = fma2(make_float2(x.z, x.w), d0, y[1][0]);
+        y[1][1] = fma2(make_float2(x.z, x.w), d1, y[1][1]);
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        *reinterpret_cast<float4*>(sY + (ra + e) * PX + cc * 4) = make_float4(y[e][0].x, y[e][0].y, y[e][1].x, y[e][1].y);
-    }
-    __syncthreads();
-    if (tid < 256) {
-      float2 s[4][4] = {};                                 // even and odd j
-#pragma unroll 2
-      for (int j = 0; j < warp * 8 + 8; j += 4) {          // X[b][j] is zero for j > b, and b < a
-        float4 ya[4];
+      for (int e = 0; e < 2; ++e) {
+        if (split) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) ya[e] = *reinterpret_cast<const float4*>(sY + (ra + e) * PX + j);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float4 x = *reinterpret_cast<const float4*>(Xs + (cc + 16 * k) * PX + j);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            s[e][k] = fma2(make_float2(ya[e].x, ya[e].y), make_float2(x.x, x.y), s[e][k]);
-            s[e][k] = fma2(make_float2(ya[e].z, ya[e].w), make_float2(x.z, x.w), s[e][k]);
+          for (int k = 0; k < 2; ++k) {
+            y[e][k].x += __shfl_xor_sync(0xffffffffu, y[e][k].x, 16);
+            y[e][k].y += __shfl_xor_sync(0xffffffffu, y[e][k].y, 16);
           }
         }
+        if (!split || lane < 16) {
+          *reinterpret_cast<float2*>(sY + spread<CH>(a0 + 2 * e, cc)) = make_float2(y[e][0].x, y[e][1].x);
+          *reinterpret_cast<float2*>(sY + spread<CH>(a0 + 2 * e + 1, cc)) = make_float2(y[e][0].y, y[e][1].y);
+        }
       }
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) sDX[(ra + e) * PX + cc + 16 * k] = -(s[e][k].x + s[e][k].y);
     }
+    __syncwarp();
+    float2 s[4][2] = {};                                   // even and odd j; columns b = lane and lane + 32
+#pragma unroll 2
+    for (int j = 0; j < a0 + 4; j += 4) {                  // X[b][j] is zero for j > b, and b < a
+      float4 ya[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ya[e] = *reinterpret_cast<const float4*>(sY + spread<CH>(a0 + e, j));
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (32 * k > a0) continue;
+        const float4 x = *reinterpret_cast<const float4*>(Xs + spread<CH>(lane + 32 * k, j));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s[e][k] = fma2(make_float2(ya[e].x, ya[e].y), make_float2(x.x, x.y), s[e][k]);
+          s[e][k] = fma2(make_float2(ya[e].z, ya[e].w), make_float2(x.z, x.w), s[e][k]);
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (32 * k <= a0) sY[spread<CH>(a0 + e, lane + 32 * k)] = -(s[e][k].x + s[e][k].y);
   }
-  __syncthreads();
+  __syncthreads();                                         // X and dX are read
   // ---- through the definitions of A and qk
   {
     float kk_[2][4] = {}, qk_[2][4] = {};
+    if (lower) {
 #pragma unroll
-    for (int kk = 0; kk < KD; kk += 16) {
-      uint32_t a[4], bb[4];
-      load_b(bb, sK, PK, n16, kk);
-      load_a(a, sK, PK, m0, kk);
-      mma2(kk_[0], kk_[1], a, bb);
-      load_a(a, sQ, PK, m0, kk);
-      mma2(qk_[0], qk_[1], a, bb);
+      for (int kk = 0; kk < KD; kk += 16) {
+        uint32_t a[4], bb[4];
+        load_b(bb, sK, PK, n16, kk);
+        load_a(a, sK, PK, m0, kk);
+        mma2(kk_[0], kk_[1], a, bb);
+        load_a(a, sQ, PK, m0, kk);
+        mma2(qk_[0], qk_[1], a, bb);
+      }
     }
     float col[2][2] = {};
 #pragma unroll
@@ -627,12 +670,12 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int j = n16 + n * 8 + cl + e;
-          const float gj = gs[j], da = sDX[i * PX + j], dq = sP[i * PX + j];     // loads first: a load under a condition is a branch
+          const float gj = gs[j], da = sY[spread<CH>(i, j)];                   // loads first: a load under a condition is a branch
           const float ex = __expf(j <= i ? gi - gj : 0.f);
           const float d = j < i ? da : 0.f;
           const float araw = kk_[n][2 * hh + e] * ex;
           ok[e] = d * bi * ex;
-          oq[e] = j <= i ? dq * p.scale * ex : 0.f;
+          oq[e] = j <= i ? dqk[n][2 * hh + e] * p.scale * ex : 0.f;
           const float t = d * bi * araw + oq[e] * qk_[n][2 * hh + e];
           rb += d * araw;
           rg += t;
@@ -672,49 +715,68 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
     red[13 * CH + tid] = dlast;
     if (t0 + tid < p.T) p.dbeta[tok0 + static_cast<long>(t0 + tid) * p.H] = dbeta;
   }
-  // ---- dq = sq dqs + dqkr k;  dk = sk dks + dkk k + dkk^T k + dqkr^T q + Tw^T dw
+  // ---- dq = sq dqs + dqkr k;  dk = sk dks + dkk k + dkk^T k + dqkr^T q + Tw^T dw,  Tw^T = diag(e^gc) Tu^T
   {
     float aQ[4][4] = {}, aK[4][4] = {};
 #pragma unroll
     for (int kk = 0; kk < CH; kk += 16) {
-      uint32_t a1[4], a2[4], a3[4], a4[4], a5[4];
-      load_a(a1, sDQ, PC, m0, kk);
-      load_a(a2, sDK, PC, m0, kk);
-      load_a_t(a3, sDK, PC, m0, kk);
-      load_a_t(a4, sDQ, PC, m0, kk);
-      load_a_t(a5, sTw, PC, m0, kk);
+      if (kk < m0) continue;                               // Tu is lower triangular
+      uint32_t a[4], bb[4];
+      load_a_t(a, sTu, PC, m0, kk);
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
-        uint32_t bb[4];
-        load_b_t(bb, sK, PK, n32 + n * 16, kk);
-        mma2(aQ[2 * n], aQ[2 * n + 1], a1, bb);
-        mma2(aK[2 * n], aK[2 * n + 1], a2, bb);
-        mma2(aK[2 * n], aK[2 * n + 1], a3, bb);
-        load_b_t(bb, sQ, PK, n32 + n * 16, kk);
-        mma2(aK[2 * n], aK[2 * n + 1], a4, bb);
-        load_b_t(bb, sW, PK, n32 + n * 16, kk);
-        mma2(aK[2 * n], aK[2 * n + 1], a5, bb);
+        load_b_t_swz(bb, sW + (n32 >> 6) * (TILE / 2), (n32 & 63) + n * 16, kk);
+        mma2(aK[2 * n], aK[2 * n + 1], a, bb);
       }
     }
+    const float e0 = __expf(gs[r0]), e1 = __expf(gs[r0 + 8]);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) { aK[n][0] *= e0; aK[n][1] *= e0; aK[n][2] *= e1; aK[n][3] *= e1; }
+#pragma unroll
+    for (int kk = 0; kk < CH; kk += 16) {                  // so are dkk and dqkr
+      uint32_t a1[4], a2[4], bb[4];
+      if (kk <= m0) {
+        load_a(a1, sDQ, PC, m0, kk);
+        load_a(a2, sDK, PC, m0, kk);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          load_b_t(bb, sK, PK, n32 + n * 16, kk);
+          mma2(aQ[2 * n], aQ[2 * n + 1], a1, bb);
+          mma2(aK[2 * n], aK[2 * n + 1], a2, bb);
+        }
+      }
+      if (kk >= m0) {
+        load_a_t(a1, sDK, PC, m0, kk);
+        load_a_t(a2, sDQ, PC, m0, kk);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          load_b_t(bb, sK, PK, n32 + n * 16, kk);
+          mma2(aK[2 * n], aK[2 * n + 1], a1, bb);
+          load_b_t(bb, sQ, PK, n32 + n * 16, kk);
+          mma2(aK[2 * n], aK[2 * n + 1], a2, bb);
+        }
+      }
+    }
+    __syncthreads();                                       // the operands are read
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
-        const int o = (r0 + 8 * hh) * PF + n32 + n * 8 + cl;
+        const int o = spread<KD>(r0 + 8 * hh, n32 + n * 8 + cl);
         *reinterpret_cast<float2*>(sFQ + o) = make_float2(aQ[n][2 * hh], aQ[n][2 * hh + 1]);
         *reinterpret_cast<float2*>(sFK + o) = make_float2(aK[n][2 * hh], aK[n][2 * hh + 1]);
       }
   }
   __syncthreads();                                         // the tiles of q and k become those of dq and dk
   {
-    float a[32];
-    tmem_cols(trow + (upper ? cKS : cWQ) + n32, a);
     const float sc = upper ? __expf(g_last - gs[ri]) : p.scale * __expf(gs[ri]);
-    const float* add = (upper ? sFK : sFQ) + ri * PF + n32;
+    const float* add = upper ? sFK : sFQ;
     bf16* dst = (upper ? sK : sQ) + ri * PK + n32;
+    float a[32];
+    tmem_cols(trow + (upper ? cKS : cWQ), a);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float4 f = *reinterpret_cast<const float4*>(add + 4 * j);
+      const float4 f = *reinterpret_cast<const float4*>(add + spread<KD>(ri, n32 + 4 * j));
       *reinterpret_cast<uint2*>(dst + 4 * j) = make_uint2(pack2(sc * a[4 * j] + f.x, sc * a[4 * j + 1] + f.y),
                                                           pack2(sc * a[4 * j + 2] + f.z, sc * a[4 * j + 3] + f.w));
     }
@@ -747,7 +809,7 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
     *reinterpret_cast<uint4*>(p.dq + off) = *reinterpret_cast<const uint4*>(sQ + r * PK + cc);
     *reinterpret_cast<uint4*>(p.dk + off) = *reinterpret_cast<const uint4*>(sK + r * PK + cc);
   }
-  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 512); }
+  if (warp == 0) { tc5::fence_after_sync(); tc5::tmem_dealloc(tmem, 256); }
 }
 // One CTA per (chunk, head), heads fastest so that CTAs that run together touch neighbouring pieces of the same token rows.
 // y ends at 65535 chunks (4.2 M tokens); longer sequences go on in z, whose last layer may reach past the end.
@@ -794,7 +856,7 @@ extern "C" int nsa_gdn_post(const void* q, const void* k, const void* v, const v
   if ((rc = nsa::make_tmap_2d_bf16(&tS, S, V, chunks * KD, V, 64, KD))) return rc;
   if ((rc = nsa::make_tmap_2d_bf16(&tdS, dS, V, chunks * KD, V, 64, KD))) return rc;
   PostParams p{(const bf16*)q, (const bf16*)k, beta, gc, X, dgamma, (bf16*)dq, (bf16*)dk, (bf16*)dv, dg, dbeta, B, T, H, NC, V, scale,
-               nsa::sm_count(), nsa::status_ptr()};
+               nsa::status_ptr()};
   cudaError_t e = cudaFuncSetAttribute(gdn_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, POST_SMEM);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn post smem attribute");
   gdn_post_kernel<<<chunk_grid(B * H, NC), 512, POST_SMEM, st>>>(tdu, tdo, tvn, tv, tS, tdS, p);

@@ -39,6 +39,12 @@ def test_gdn_sizes(native, B, T, H, V):
     _check(native, _inputs(B, T, H, V, 0.3))
 
 
+@pytest.mark.parametrize("T,H,V", [(1300, 16, 64), (1283, 15, 320), (1000, 20, 512)])
+def test_gdn_more_chunks_than_sms(native, T, H, V):
+    # two chunks' gradients share an SM; one, five and eight slices of the values
+    _check(native, _inputs(1, T, H, V, 0.3))
+
+
 @pytest.mark.parametrize("decay", [0.0, 8.0, -0.01])       # no decay, e^-500 across a chunk, slow growth
 def test_gdn_gates(native, decay):
     _check(native, _inputs(1, 200, 2, 256, decay))
