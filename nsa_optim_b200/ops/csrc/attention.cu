@@ -633,12 +633,12 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const bool lead = tc5::elect_one();
       constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 64, 0, 0);
       const uint64_t bK0 = tc5::desc_kmajor(tc5::smem_u32(sKV));
-      bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(qt_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+      bool ok = tc5::mbar_wait_warp(qt_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
       if (ok) tc5::fence_after_sync();
       for (int v = 0; v < n_vis && ok; ++v) {
         const int st = v % FWT_STAGES, g = v & 1;
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(kv_full + st, (v / FWT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(s_empty + g, ((v >> 1) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
+        ok = tc5::mbar_wait_warp(kv_full + st, (v / FWT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+             tc5::mbar_wait_warp(s_empty + g, ((v >> 1) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY);
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t bK = bK0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
@@ -662,8 +662,8 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       for (int u = 0; u < n_vis; ++u) {
         const int st = u % FWT_STAGES, g = u & 1;
         // V of this stage: the copy that completes kv_full brings K and V together
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(kv_full + st, (u / FWT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(p_full + g, (u >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+        ok = tc5::mbar_wait_warp(kv_full + st, (u / FWT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+             tc5::mbar_wait_warp(p_full + g, (u >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t bV = bVmn0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
@@ -693,7 +693,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     bool ok = true;
     if (n_vis > 0) {
       // Q: shared memory (swizzled [128 rows][64] k-blocks) -> TMEM; thread (r, grp) copies half grp of its row
-      ok = __all_sync(0xffffffffu, tc5::mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL));
+      ok = tc5::mbar_wait_warp(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL);
       if (ok) {
         q_half_to_tmem<D>(tmem + lane_off + cQ, sQ, r, grp);
         tc5::fence_before_sync();
@@ -715,7 +715,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         sb = blk < 0 ? -1 : blk * 64;
         row_sel = row_ok && blk >= 0 && ((msk >> (tok_local & 63)) & 1ull);
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + grp, n_mine & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+      if (!tc5::mbar_wait_warp(s_full + grp, n_mine & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
@@ -765,7 +765,7 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       }
       l_sum = l_sum * alpha + psum;
       // P V of the group's previous visit must be done before P is overwritten or O rescaled
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(p_empty + grp, (n_mine & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY))) {
+      if (!tc5::mbar_wait_warp(p_empty + grp, (n_mine & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) {
         ok = false;
         break;
       }
@@ -788,8 +788,8 @@ attn_fwd_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tc5::mbar_arrive(p_full + grp);
     }
     // ---- merge the two groups' partial results and write O (thread (r, grp): half grp of the columns)
-    const bool done = __all_sync(0xffffffffu, ok && n_vis > 0 &&
-                                 tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+    const bool done = ok && n_vis > 0 &&
+                      tc5::mbar_wait_warp(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
     if (done) tc5::fence_after_sync();
     if (grp == 1) { merge[r] = m_ref; merge[128 + r] = l_sum; }
     asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -961,11 +961,11 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const bool lead = tc5::elect_one();
       constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 64, 0, 0);
       const uint64_t aQ = tc5::desc_kmajor(tc5::smem_u32(sQ)), bK0 = tc5::desc_kmajor(tc5::smem_u32(sK));
-      bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL));
+      bool ok = tc5::mbar_wait_warp(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL);
       for (int v = 0; v < n_vis && ok; ++v) {
         const int st = v % FW1_STAGES;
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(k_full + st, (v / FW1_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(s_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
+        ok = tc5::mbar_wait_warp(k_full + st, (v / FW1_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+             tc5::mbar_wait_warp(s_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY);
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t bK = bK0 + static_cast<uint64_t>((st * KVT) >> 4);
@@ -989,8 +989,8 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       bool ok = true;
       for (int u = 0; u < n_vis; ++u) {
         const int st = u % FW1_STAGES;
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(v_full + st, (u / FW1_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(p_full, u & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+        ok = tc5::mbar_wait_warp(v_full + st, (u / FW1_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+             tc5::mbar_wait_warp(p_full, u & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t bV = bV0 + static_cast<uint64_t>((st * KVT) >> 4);
@@ -1031,7 +1031,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         sb = blk < 0 ? -1 : blk * 64;
         row_sel = row_ok && blk >= 0 && ((msk >> (tok_local & 63)) & 1ull);
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full, v & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+      if (!tc5::mbar_wait_warp(s_full, v & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
@@ -1084,7 +1084,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       l_sum = l_sum * alpha + psum;
       // P V of the previous visit must be done before P is overwritten or O rescaled
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(p_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY))) {
+      if (!tc5::mbar_wait_warp(p_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) {
         ok = false;
         break;
       }
@@ -1106,8 +1106,8 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tc5::fence_before_sync();
       tc5::mbar_arrive(p_full);
     }
-    const bool done = __all_sync(0xffffffffu, ok && n_vis > 0 &&
-                                 tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+    const bool done = ok && n_vis > 0 &&
+                      tc5::mbar_wait_warp(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
     if (done) tc5::fence_after_sync();
     const bool have = done && l_sum > 0.f;
     const float f = have ? 1.f / l_sum : 0.f;
@@ -1226,12 +1226,12 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       const bool lead = tc5::elect_one();
       constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 64, 0, 0);
       const uint64_t bK0 = tc5::desc_kmajor(tc5::smem_u32(sK));
-      bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(qt_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+      bool ok = tc5::mbar_wait_warp(qt_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
       if (ok) tc5::fence_after_sync();
       for (int v = 0; v < n_vis && ok; ++v) {
         const int st = v % IMP_STAGES, g = v & 1;
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(k_full + st, (v / IMP_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(s_empty + g, ((v >> 1) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
+        ok = tc5::mbar_wait_warp(k_full + st, (v / IMP_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+             tc5::mbar_wait_warp(s_empty + g, ((v >> 1) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY);
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t bK = bK0 + static_cast<uint64_t>((st * 2 * HALF) >> 4);
@@ -1263,7 +1263,7 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     bool ok = true;
     if (n_vis > 0) {
       // Q: shared memory (swizzled [128 rows][64] k-blocks) -> TMEM; thread (r, grp) copies k-block grp of its row
-      ok = __all_sync(0xffffffffu, tc5::mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL));
+      ok = tc5::mbar_wait_warp(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL);
       if (ok) {
         uint32_t w[32];
         const uint8_t* rowp = sQ + grp * 2 * HALF + r * 128;
@@ -1280,7 +1280,7 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     }
     int n_mine = 0;
     for (int v = grp; v < n_vis && ok; v += 2, ++n_mine) {
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + grp, n_mine & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+      if (!tc5::mbar_wait_warp(s_full + grp, n_mine & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
@@ -1534,7 +1534,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         sb = blk < 0 ? -1 : blk * 64;
         row_sel = row_ok && blk >= 0 && ((msk >> (tok_local & 63)) & 1ull);
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + grp, n_mine & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+      if (!tc5::mbar_wait_warp(s_full + grp, n_mine & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
@@ -1596,7 +1596,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
         tc5::tmem_st_wait();
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(p_empty + grp, (n_mine & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY))) {
+      if (!tc5::mbar_wait_warp(p_empty + grp, (n_mine & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY)) {
         ok = false;
         break;
       }
@@ -1606,8 +1606,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tc5::mbar_arrive(p_full + grp);
     }
     // ---- merge the two groups' partial results and write O (thread (r, grp): columns grp*64..)
-    const bool done = __all_sync(0xffffffffu, ok && n_vis > 0 &&
-                                 tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+    const bool done = ok && n_vis > 0 &&
+                      tc5::mbar_wait_warp(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
     if (done) tc5::fence_after_sync();
     if (grp == 1) { merge[r] = m_ref; merge[128 + r] = l_sum; }
     asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -2052,12 +2052,12 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const uint64_t b0 = tc5::desc_kmajor(tc5::smem_u32(sKV) + (is_dp ? KVT : 0));   // stage 0, K or V, k-step 0
       const uint32_t acol = is_dp ? cDO : cQ, dcol = is_dp ? 64u : 0u;
       uint64_t *made = GROUPS && is_dp ? dp_full : s_full, *free = GROUPS && is_dp ? dp_empty : s_empty;
-      bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(qt_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+      bool ok = tc5::mbar_wait_warp(qt_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
       if (ok) tc5::fence_after_sync();
       for (int v = 0; v < n_vis && ok; ++v) {
         const int st = v % DQT_STAGES, buf = v % BUFS;
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(kv_full + st, (v / DQT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(free + buf, ((v / BUFS) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
+        ok = tc5::mbar_wait_warp(kv_full + st, (v / DQT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+             tc5::mbar_wait_warp(free + buf, ((v / BUFS) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY);
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t bB = b0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
@@ -2080,8 +2080,8 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       bool ok = true;
       for (int u = 0; u < n_vis; ++u) {
         const int st = u % DQT_STAGES, buf = u % BUFS;
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(kv_full + st, (u / DQT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(ds_full + buf, (u / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+        ok = tc5::mbar_wait_warp(kv_full + st, (u / DQT_STAGES) & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+             tc5::mbar_wait_warp(ds_full + buf, (u / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t bKmn = bKmn0 + static_cast<uint64_t>((st * 2 * KVT) >> 4);
@@ -2115,7 +2115,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     bool ok = true;
     if (n_vis > 0) {
       // Q and dO: shared memory (swizzled [128 rows][64] k-blocks) -> TMEM, thread (r, ch) copies half ch of its row
-      ok = __all_sync(0xffffffffu, tc5::mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL));
+      ok = tc5::mbar_wait_warp(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL);
       if (ok) {
         q_half_to_tmem<D>(tmem + lane_off + cQ, sQ, r, ch);
         q_half_to_tmem<D>(tmem + lane_off + cDO, sDO, r, ch);
@@ -2140,7 +2140,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         sb = blk < 0 ? -1 : blk * 64 + (GROUPS ? 0 : ch * 32);
         row_sel = row_ok && blk >= 0 && ((msk >> (tok_local & 63)) & 1ull);
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + buf, (v / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+      if (!tc5::mbar_wait_warp(s_full + buf, (v / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
@@ -2159,7 +2159,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           for (int i = 0; i < 64; ++i)                      // masked scores are -inf: their probability is 0
             sv[i] = __float_as_uint(exp2f(fmaf(__uint_as_float(sv[i]), sc, negL)));
         }
-        if (!__all_sync(0xffffffffu, tc5::mbar_wait(dp_full + buf, (v / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+        if (!tc5::mbar_wait_warp(dp_full + buf, (v / BUFS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
           ok = false;
           break;
         }
@@ -2213,8 +2213,8 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     for (int i = 0; i < D / 16; ++i)
       old[i] = p.add_dq && row_ok ? reinterpret_cast<const uint4*>(p.dQb + rowi * D + ch * (D / 2))[i] : make_uint4(0u, 0u, 0u, 0u);
     // ---- dQ: thread (r, ch) stores D-half ch of row r
-    const bool have = __all_sync(0xffffffffu, ok && n_vis > 0 &&
-                                 tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+    const bool have = ok && n_vis > 0 &&
+                      tc5::mbar_wait_warp(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
     if (have) tc5::fence_after_sync();
     bf16* dst = p.dQb + rowi * D + ch * (D / 2);
 #pragma unroll
@@ -2441,7 +2441,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         sb = blk < 0 ? -1 : blk * 64 + ch * 32;
         row_sel = row_ok && blk >= 0 && ((msk >> (tok_local & 63)) & 1ull);
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + buf, (v >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+      if (!tc5::mbar_wait_warp(s_full + buf, (v >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
@@ -2468,7 +2468,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                      p1 * fmaf(__uint_as_float(dv[i + 1]), scale, nds));
         }
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(ds_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY))) {
+      if (!tc5::mbar_wait_warp(ds_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY)) {
         ok = false;
         break;
       }
@@ -2482,8 +2482,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tc5::mbar_arrive(ds_full);
     }
     // ---- dQ: thread (r, ch) stores D-half ch of row r
-    const bool have = __all_sync(0xffffffffu, ok && n_vis > 0 &&
-                                 tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL));
+    const bool have = ok && n_vis > 0 &&
+                      tc5::mbar_wait_warp(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
     if (have) tc5::fence_after_sync();
     bf16* dst = p.dQb + rowi * D + ch * 64;
 #pragma unroll
@@ -2643,7 +2643,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   const uint32_t tmem = *tmem_slot;
   constexpr uint32_t cS = 0, cDP = BUFS * 128, cDV = cDP + 128, cDK = cDV + D;   // S^T of buffer i at i * 128
   auto wait = [&](uint64_t* bar, int phase, int code) {
-    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+    return tc5::mbar_wait_warp(bar, phase & 1, abort_flag, p.status, code);
   };
 
   if (warp == 8) {
@@ -3074,12 +3074,12 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 64, 0, 0);
       const uint64_t aQ0 = tc5::desc_kmajor(tc5::smem_u32(sQ)), aDO0 = tc5::desc_kmajor(tc5::smem_u32(sDO));
       const uint64_t bK0 = tc5::desc_kmajor(tc5::smem_u32(sK)), bV0 = tc5::desc_kmajor(tc5::smem_u32(sV));
-      bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL));
+      bool ok = tc5::mbar_wait_warp(kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL);
       for (int v = 0; v < n_vis && ok; ++v) {
         const int buf = v & 1;
         const uint32_t ph = (v >> 1) & 1;
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(q_full + buf, ph, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
-                                     tc5::mbar_wait(s_empty + buf, ph ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY));
+        ok = tc5::mbar_wait_warp(q_full + buf, ph, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL) &&
+             tc5::mbar_wait_warp(s_empty + buf, ph ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY);
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t aQ = aQ0 + static_cast<uint64_t>((buf * QT) >> 4), aDO = aDO0 + static_cast<uint64_t>((buf * QT) >> 4);
@@ -3109,7 +3109,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       bool ok = true;
       for (int u = 0; u < n_vis; ++u) {
         const int buf = u & 1;
-        ok = __all_sync(0xffffffffu, tc5::mbar_wait(p_full, u & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL));
+        ok = tc5::mbar_wait_warp(p_full, u & 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_FULL);
         if (!ok) break;
         tc5::fence_after_sync();
         const uint64_t aA = a0 + static_cast<uint64_t>((buf * QT) >> 4);
@@ -3165,7 +3165,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         t_cur = t_nxt; L_cur = Ln; d_cur = dn;
         t_nxt = token_of(v + 2);
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(s_full + buf, (v >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+      if (!tc5::mbar_wait_warp(s_full + buf, (v >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
@@ -3193,7 +3193,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                      p1 * fmaf(__uint_as_float(dv[i + 1]), scale, nds));
         }
       }
-      if (!__all_sync(0xffffffffu, tc5::mbar_wait(p_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY))) {
+      if (!tc5::mbar_wait_warp(p_empty, (v & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_SMEM_EMPTY)) {
         ok = false;
         break;
       }
@@ -3211,7 +3211,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tc5::mbar_arrive(p_full);
     }
     // ---- accumulators -> global: lane = d, columns = keys; one fp32 reduction per element, or one bf16 where the sums are whole
-    if (__all_sync(0xffffffffu, ok && tc5::mbar_wait(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL))) {
+    if (ok && tc5::mbar_wait_warp(acc_done, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) {
       tc5::fence_after_sync();
       const int d = (warp & 3) * 32 + lane;
       const long o = ((static_cast<long>(b) * p.S + s0) * p.Hkv + h) * D + d;

@@ -150,7 +150,7 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   // TMEM columns: D1 = [w ; q] S [0, 64)   S [64, 128)   D2 = [0 ; qk] v_new [128, 192)
   const uint32_t cD1 = 0, cS = 64, cD2 = 128;
   auto wait = [&](uint64_t* bar, int phase, int code) {
-    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+    return tc5::mbar_wait_warp(bar, phase & 1, abort_flag, p.status, code);
   };
   const float* gc = p.gc + static_cast<long>(bh) * NC * CH;
   if (warp < 8) {
@@ -440,7 +440,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   // TMEM columns: Da = [k ; w] dS [0,64)   Dd = [qk^T ; 0] do [64,128)   dS [128,192)
   const uint32_t cDa = 0, cDd = 64, cDs = 128;
   auto wait = [&](uint64_t* bar, int phase, int code) {
-    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+    return tc5::mbar_wait_warp(bar, phase & 1, abort_flag, p.status, code);
   };
   const float* gc = p.gc + static_cast<long>(bh) * NC * CH;
   if (warp < 8) {

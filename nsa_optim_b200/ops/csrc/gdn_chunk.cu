@@ -407,7 +407,7 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
   constexpr uint32_t idesc = tc5::make_idesc_bf16(128, 128, 0, 0);
   constexpr int ISSUER = 14;                               // copies and issues too: it has nothing of dTu and dqk
   auto wait = [&](uint64_t* bar, int use, int code) {
-    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, use & 1, abort_flag, p.status, code)) != 0;
+    return tc5::mbar_wait_warp(bar, use & 1, abort_flag, p.status, code);
   };
   float dtu[2][4] = {}, dqk[2][4] = {};                    // rows m0.., columns n16..
   {

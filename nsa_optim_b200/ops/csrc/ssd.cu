@@ -350,7 +350,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   const uint32_t tmem = *tmem_slot;
   const uint32_t cS = 0, cP = 128, cYi = 256, cYo = 384;     // the last three: 64 columns for even and odd items each
   auto wait = [&](uint64_t* bar, int phase, int code) {
-    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+    return tc5::mbar_wait_warp(bar, phase & 1, abort_flag, p.status, code);
   };
   if (warp == 16) {                                    // products
     constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);
@@ -615,7 +615,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
   // B dHn, then dx [128, 192).  C H [192, 256): of each 16, 8 become exp(cum) dy and 8 s x (16 p).  dB, dC [256, 512).
   const uint32_t cR = 0, cX = 128, cY = 192, cDB = 256, cDC = 384;
   auto wait = [&](uint64_t* bar, int phase, int code) {
-    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+    return tc5::mbar_wait_warp(bar, phase & 1, abort_flag, p.status, code);
   };
   if (warp == 16) {
     constexpr uint32_t id_s = tc5::make_idesc_bf16(128, 128, 0, 0);     // K-major x K-major -> [128 x 128]
@@ -1038,7 +1038,7 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
   tc5::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   auto wait = [&](uint64_t* bar, int phase, int code) {
-    return __all_sync(0xffffffffu, tc5::mbar_wait(bar, phase & 1, abort_flag, p.status, code)) != 0;
+    return tc5::mbar_wait_warp(bar, phase & 1, abort_flag, p.status, code);
   };
   auto chunk_of = [&](int i) { return BACK ? nc - 1 - i : i; };
   auto leave = [&](int i) {                            // chunk i's buffer to memory, one thread

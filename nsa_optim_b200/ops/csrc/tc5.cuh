@@ -92,6 +92,25 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// The same for a whole converged warp.  Every poll is voted on, so the branches are uniform: with a branch per lane in the loop a wait costs the
+// warp 130 cycles and more for the reconvergence alone, also where the phase has long completed (one lane polling for the
+// others is worse: a chain of eight such waits per step took twice as long).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                               KernelStatus* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  for (uint32_t i = 0; i < kMaxPolls; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 255u) == 255u) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+      if (__any_sync(0xffffffffu, clock64() - t0 > kMaxWaitCycles)) break;
+    }
+  }
+  *abort_flag = 1;
+  status_report(status, code, blockIdx.x, parity);
+  return false;
+}
+
 // After a wait that gave up: gives a copy that may still be in flight towards `bar` a bounded chance (10 ms) to land before the
 // CTA's shared memory goes to another CTA.  The open phase is read from the barrier (waiting for either parity would not
 // wait at all: one of the two is always complete); where no copy is on its way, the limit passes.
