@@ -84,7 +84,8 @@ constexpr int WARP_MMA = 8, WARP_LOAD = 9;
 // and the chain then waits for it.  256 chunks x 64 CTAs, forward and backward: 472 and 526 us with one thread for copies,
 // stores and products, 455 and 597 with warps for each, 395 and 492 with the prefetch and operands released where their last
 // product is issued, 356 and 365 with u and do as tiles too (rows of their own per thread are 32 lines an instruction),
-// 336 and 361 with the wait for a tile's last stores in front of the one for the state.
+// 336 and 361 with the wait for a tile's last stores in front of the one for the state, 316 and 321 with waits that vote and, backward,
+// qk^T do issued in front of the wait for the state (that alone: 354 to 346).
 constexpr int AHEAD = 6;
 
 // stage: k-block kb of [w ; q] (2 x 16 KB), k (16 KB), [0 ; qk] (16 KB, first half zero)
@@ -202,7 +203,7 @@ gdn_seq_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       }
       if (c + 1 < NC) {
         const float g = __expf(g_last_next);       // decay of the state through chunk c + 1
-        // a wait costs 200 cycles and more when there is nothing to wait for: the one for the stores goes first
+        // the wait for the stores, which are through by now, goes first and is off the chain
         if (!wait(freed, c, STATUS_TIMEOUT_SMEM_EMPTY) || !wait(m2, c, STATUS_TIMEOUT_TMEM_FULL)) break;
         tc5::fence_after_sync();
         float sv[HC];
@@ -552,24 +553,26 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       const uint64_t a = tc5::desc_kmajor(st), dom = tc5::desc_mnmajor(tc5::smem_u32(sDO + s * BOX), BOX);
       const uint64_t qk = tc5::desc_mnmajor(st + 8 * BOX, BOX), qdm = tc5::desc_mnmajor(st + 4 * BOX, BOX);
       const uint64_t wm = tc5::desc_mnmajor(st + BOX, 2 * BOX), dum = tc5::desc_mnmajor(tc5::smem_u32(sDU + s * BOX), BOX);
-      if (!wait(full + s, it >> 1, STATUS_TIMEOUT_SMEM_FULL) || !wait(sready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
+      // Dd waits for nothing but its tiles (its last rows were read before the du that the products of step it - 1 waited for)
+      if (!wait(full + s, it >> 1, STATUS_TIMEOUT_SMEM_FULL)) break;
+      tc5::fence_after_sync();
+      if (lead) {
+#pragma unroll
+        for (int kk = 0; kk < CH / 16; ++kk)      // Dd = [qk^T ; 0] do
+          tc5::mma_ss(tmem + cDd, qk + static_cast<uint64_t>((kk * 2048) >> 4), dom + static_cast<uint64_t>((kk * 2048) >> 4), id_d, kk > 0 ? 1u : 0u);
+      }
+      __syncwarp();
+      if (!wait(sready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
       tc5::fence_after_sync();
       if (lead) {
 #pragma unroll
         for (int kk = 0; kk < KD / 16; ++kk)      // Da = [k ; w] dS
           tc5::mma_ss(tmem + cDa, a + static_cast<uint64_t>(((kk >> 2) * 2 * BOX + (kk & 3) * 32) >> 4),
                       dsbm + static_cast<uint64_t>((kk * 2048) >> 4), id_a, kk > 0 ? 1u : 0u);
-      }
-      __syncwarp();
-      if (!wait(oready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
-      tc5::fence_after_sync();
-      if (lead) {
-#pragma unroll
-        for (int kk = 0; kk < CH / 16; ++kk)      // Dd = [qk^T ; 0] do
-          tc5::mma_ss(tmem + cDd, qk + static_cast<uint64_t>((kk * 2048) >> 4), dom + static_cast<uint64_t>((kk * 2048) >> 4), id_d, kk > 0 ? 1u : 0u);
         tc5::mma_commit(m1);
       }
       __syncwarp();
+      if (!wait(oready, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
       if (!wait(scaled, it, STATUS_TIMEOUT_TMEM_EMPTY)) break;
       tc5::fence_after_sync();
       if (lead) {
