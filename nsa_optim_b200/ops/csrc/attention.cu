@@ -1,7 +1,7 @@
-// Attention family on tcgen05: one forward kernel and one backward kernel cover dense causal
-// GQA attention, sliding-window attention, and the three branches of native sparse attention
-// (compressed-block attention, selected-block attention, plus the block-importance pass that
-// feeds top-n selection).
+// Attention family on tcgen05: dense causal GQA attention, sliding-window attention, and the three branches of native sparse
+// attention (compressed-block attention, selected-block attention, plus the block-importance pass that feeds top-n
+// selection).  The first kernels (attn_fwd_kernel, attn_bwd_kernel), described here, do all of it; they run where no
+// warp-specialised kernel further down does: selected blocks and importances at head_dim 64, selected blocks in GQA groups below 8.
 //
 // Tiling.  A query tile is 128 rows = R consecutive tokens x G query heads of one KV head
 // (G = Hq / Hkv, R = 128 / G), so one K/V tile serves the whole GQA group.  A key tile is 128

@@ -37,16 +37,6 @@ __device__ __forceinline__ void load_gates(const float* g, const float* beta, lo
   }
 }
 
-// The inputs of the CTA that will run on this SM next are asked for into L2 (resident: CTAs that run together): a chunk's loads
-// then wait for L2 and not for memory.
-__device__ __forceinline__ bool next_chunk(int resident, int H, int NC, int& bh, int& c) {
-  const long next = (static_cast<long>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x + resident;
-  bh = static_cast<int>(next % gridDim.x);
-  c = static_cast<int>(next / gridDim.x);
-  return c < NC;
-}
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
 struct PrepParams {
   const bf16 *q, *k, *v;       // [B, T, H, .]
   const float *g, *beta;       // [B, T, H]
@@ -54,25 +44,26 @@ struct PrepParams {
   float *X, *gc;               // [BH, NC, 64, 64] or null, [BH, NC, 64]
   int T, H, NC, V;
   float scale;
-  int resident;
 };
 
 // One CTA of eight warps per (chunk, head).  What bounds it is its chain of phases, not the memory traffic of q, k, v, u, w (2 KB
-// per token and head, 87 us at the copy rate for 16384 tokens x 16 heads), so two CTAs have to share an SM: the operands
-// of the last products take the places of q and A, which are through by then (values 256 wide: 101 KB; with tiles of their
-// own, 122 KB and one CTA per SM, 283 us; now 198).  The triangular inverse is the longest dependent phase and runs as
+// per token and head, 87 us at the copy rate for 16384 tokens x 16 heads), so three CTAs share an SM (70 KB each, for every width of
+// the values): v passes through in pieces of 128 columns, over q and X, which are through by then, and Tu and Tw
+// take the place of A.  16384 tokens x 16 heads, values 256 wide: 283 us with one CTA per SM, 198 with two (101 KB, all of v at once), 170
+// with three, 165 without asking for the next chunk's inputs in L2.  The triangular inverse is the longest dependent phase and runs as
 // two 32-column substitutions side by side, joined by two 32 x 32 products over all threads.
-__global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
+__global__ void __launch_bounds__(256, 3) gdn_prep_kernel(const PrepParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  const int V = p.V, PV = V + 8;
+  const int V = p.V;
   bf16* sK = reinterpret_cast<bf16*>(smem_raw);            // rows 0..63 k, 64..127 q
-  bf16* sV = sK + 2 * CH * PK;
-  float* As = reinterpret_cast<float*>(sV + CH * PV);      // [64][PX]
-  float* Xs = As + CH * PX;
+  float* As = reinterpret_cast<float*>(sK + 2 * CH * PK);  // [64][PX]
+  bf16* sTu = reinterpret_cast<bf16*>(As);                 // Tu and Tw over A once its inverse is known
+  bf16* sTw = sTu + CH * PC;
+  float* Xs = reinterpret_cast<float*>(sTw + CH * PC);     // [64][PX]
   float* gs = Xs + CH * PX;
-  bf16* sTu = sK + CH * PK;                                // over q once q k^T is done
-  bf16* sTw = reinterpret_cast<bf16*>(As);                 // over A once its inverse is known
   float* bs = gs + CH;
+  // 128 columns of v: over q once q k^T is done, over X once Tu and Tw are
+  auto piece = [&](int i) { return i & 1 ? reinterpret_cast<bf16*>(Xs) : sK + CH * PK; };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bh = blockIdx.x, h = bh % p.H, b = bh / p.H, c = blockIdx.z * gridDim.y + blockIdx.y;   // see chunk_grid
   if (c >= p.NC) return;
@@ -86,22 +77,17 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
     cp_async16(sK + (CH + r) * PK + cc, p.q + off, ok);
   }
   cp_async_commit();
-  const int v8 = V / 8;
-  for (int i = tid; i < CH * v8; i += 256) {
-    const int r = i / v8, cc = (i - r * v8) * 8, t = t0 + r;
-    const bool ok = t < p.T;
-    cp_async16(sV + r * PV + cc, p.v + (tok0 + static_cast<long>(ok ? t : 0) * p.H) * V + cc, ok);
-  }
-  cp_async_commit();
+  auto load_v = [&](int i) {                               // piece i
+    const int c8 = min(16, (V - 128 * i) / 8), shift = c8 == 16 ? 4 : 3;   // 16-byte columns: 16 or 8
+    for (int e = tid; e < CH * c8; e += 256) {
+      const int r = e >> shift, cc = (e & (c8 - 1)) * 8, t = t0 + r;
+      const bool ok = t < p.T;
+      cp_async16(piece(i) + r * PK + cc, p.v + (tok0 + static_cast<long>(ok ? t : 0) * p.H) * V + 128 * i + cc, ok);
+    }
+    cp_async_commit();
+  };
   load_gates(p.g, p.beta, tok0, p.T, t0, p.H, gs, bs);
-  int nbh, nc;
-  if (next_chunk(p.resident, p.H, p.NC, nbh, nc) && nc * CH + (tid & 63) < p.T) {        // a row each, 128 bytes at a time
-    const long row = (static_cast<long>(nbh / p.H) * p.T + nc * CH + (tid & 63)) * p.H + nbh % p.H;
-    const bf16* src = tid < 64 ? p.k + row * KD : tid < 128 ? p.q + row * KD : p.v + row * V + (tid < 192 ? 0 : 64);
-    const int step = tid < 128 ? 64 : 128, end = tid < 128 ? KD : V - (tid < 192 ? 0 : 64);
-    for (int x = 0; x < end; x += step) prefetch_l2(src + x);
-  }
-  cp_async_wait<1>();
+  cp_async_wait<0>();
   __syncthreads();
   const long chunk = static_cast<long>(bh) * p.NC + c;
   if (tid < CH) p.gc[chunk * CH + tid] = gs[tid];
@@ -140,6 +126,7 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
     }
   }
   __syncthreads();
+  load_v(0);
   // ---- X = (I + A)^-1.  Diagonal 32 x 32 blocks: thread (block, column) substitutes forward
   if (warp < 2) {
     const float* Ad = As + warp * 32 * PX + warp * 32;
@@ -196,18 +183,15 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
                                                              pack2(u2 * __expf(gs[j + 2]), u3 * __expf(gs[j + 3])));
   }
   __syncthreads();
-  // ---- u = Tu v and w = Tw k, 16 columns at a time; a warp is the only reader of its columns and
-  //      puts the result in their place
-  for (int unit = warp; unit < (V + KD) / 16; unit += 8) {
-    const bool is_u = unit < V / 16;
-    bf16* src = is_u ? sV : sK;
-    const bf16* tm = is_u ? sTu : sTw;
-    const int pitch = is_u ? PV : PK, n0 = (is_u ? unit : unit - V / 16) * 16;
+  // ---- w = Tw k and u = Tu v, 128 columns at a time, 16 a warp, which is the only reader of its columns and puts the
+  //      result in their place
+  auto multiply = [&](const bf16* tm, bf16* src) {
+    const int n0 = warp * 16;
     float acc[4][2][4] = {};
 #pragma unroll
     for (int kk = 0; kk < CH; kk += 16) {
       uint32_t bb[4];
-      load_b_t(bb, src, pitch, n0, kk);
+      load_b_t(bb, src, PK, n0, kk);
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
         if (kk > m * 16) continue;                 // the matrices are lower triangular
@@ -223,17 +207,31 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(const PrepParams p) {
       for (int n = 0; n < 2; ++n)
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh)
-          *reinterpret_cast<uint32_t*>(src + (m * 16 + (lane >> 2) + 8 * hh) * pitch + n0 + n * 8 + 2 * (lane & 3)) =
+          *reinterpret_cast<uint32_t*>(src + (m * 16 + (lane >> 2) + 8 * hh) * PK + n0 + n * 8 + 2 * (lane & 3)) =
               pack2(acc[m][n][2 * hh], acc[m][n][2 * hh + 1]);
-  }
-  __syncthreads();
-  for (int i = tid; i < CH * v8; i += 256) {
-    const int r = i / v8, cc = (i - r * v8) * 8;
-    *reinterpret_cast<uint4*>(p.u + (chunk * CH + r) * V + cc) = *reinterpret_cast<const uint4*>(sV + r * PV + cc);
-  }
-  for (int i = tid; i < CH * (KD / 8); i += 256) {
-    const int r = i / (KD / 8), cc = (i % (KD / 8)) * 8;
-    *reinterpret_cast<uint4*>(p.w + (chunk * CH + r) * KD + cc) = *reinterpret_cast<const uint4*>(sK + r * PK + cc);
+  };
+  const int pieces = (V + 127) / 128;
+  if (pieces > 1) load_v(1);
+  multiply(sTw, sK);
+  for (int i = 0; i < pieces; ++i) {
+    if (i > 0) {
+      cp_async_wait<0>();
+      __syncthreads();                             // the piece is there, and the one before has left
+      if (i + 1 < pieces) load_v(i + 1);
+    }
+    const int c8 = min(16, (V - 128 * i) / 8), shift = c8 == 16 ? 4 : 3;
+    bf16* src = piece(i);
+    if (warp * 2 < c8) multiply(sTu, src);
+    __syncthreads();
+    for (int e = tid; e < CH * c8; e += 256) {
+      const int r = e >> shift, cc = (e & (c8 - 1)) * 8;
+      *reinterpret_cast<uint4*>(p.u + (chunk * CH + r) * V + 128 * i + cc) = *reinterpret_cast<const uint4*>(src + r * PK + cc);
+    }
+    if (i == 0)
+      for (int e = tid; e < CH * (KD / 8); e += 256) {
+        const int r = e / (KD / 8), cc = (e % (KD / 8)) * 8;
+        *reinterpret_cast<uint4*>(p.w + (chunk * CH + r) * KD + cc) = *reinterpret_cast<const uint4*>(sK + r * PK + cc);
+      }
   }
 }
 
@@ -257,7 +255,6 @@ constexpr int POST_TILES = POST_B + 2 * TILE;
 constexpr int POST_RED = 16;                                               // rows of partial sums
 constexpr int POST_SMEM = POST_TILES + CH * PC * 2 + (2 + POST_RED) * CH * 4 + 128 + 1024;
 constexpr int FX = CH * CH * 4, FF = CH * KD * 4;                          // fp32 tiles of the tail, rows without padding
-static_assert(PC <= PK && CH * PC * 2 <= CH * PX * 4, "gdn prep: operand tiles");
 static_assert(POST_B % 1024 == 0 && 2 * TILE <= 2 * CH * PK * 2, "gdn post: swizzled tiles");
 static_assert(2 * FX <= POST_A1 && CH * PC * 2 <= FX, "gdn post: X, dX and what takes their places");
 static_assert(TILE + FX <= 2 * TILE && FF <= POST_A1 && FF <= 2 * TILE, "gdn post: dw, X^T dX, results");
@@ -822,11 +819,11 @@ extern "C" int nsa_gdn_prep(const void* q, const void* k, const void* v, const f
                             void* qk, float* X, float* gc, int B, int T, int H, int K, int V, float scale, cudaStream_t st) {
   if (K != KD || V % 64 || V > 512) return nsa::fail(NSA_ERR_SHAPE, "gdn: key width must be 128, value width a multiple of 64 up to 512");
   const int NC = (T + CH - 1) / CH;
-  PrepParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, g, beta, (bf16*)w, (bf16*)u, (bf16*)qk, X, gc, T, H, NC, V, scale, 0};
-  const int smem = 2 * CH * PK * 2 + CH * (V + 8) * 2 + 2 * CH * PX * 4 + 2 * CH * 4;
+  PrepParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, g, beta, (bf16*)w, (bf16*)u, (bf16*)qk, X, gc, T, H, NC, V, scale};
+  constexpr int smem = 2 * CH * PK * 2 + 2 * CH * PC * 2 + CH * PX * 4 + 2 * CH * 4;
+  static_assert(3 * (smem + 1024) <= 228 * 1024 && CH * PX * 4 <= 2 * CH * PC * 2 && CH * PK * 2 <= CH * PX * 4, "gdn prep: three CTAs per SM, tiles");
   cudaError_t e = cudaFuncSetAttribute(gdn_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return nsa::fail_cuda(e, "gdn prep smem attribute");
-  p.resident = (2 * (smem + 1024) <= 228 * 1024 ? 2 : 1) * nsa::sm_count();
   gdn_prep_kernel<<<chunk_grid(B * H, NC), 256, smem, st>>>(p);
   nsa::count_launch();
   e = cudaGetLastError();
