@@ -878,7 +878,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc5::warp_index(), lane = tid & 31;
   const auto [qt, n_qt, h, b] = query_tile(p, LONGEST_FIRST);
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
@@ -1175,7 +1175,7 @@ attn_importance_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(qt_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc5::warp_index(), lane = tid & 31;
   const auto [qt, n_qt, h, b] = query_tile(p, true);   // always causal
   const int q0 = qt * p.R;
   const int lim = min(q0 + p.R, p.T) - 1 - p.kp_off;
@@ -1940,7 +1940,7 @@ attn_bwd_dq_ts_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = GROUPS ? tid >> 5 : tc5::warp_index(), lane = tid & 31;
   const auto [qt, n_qt, h, b] = query_tile(p, longest_first(p));
   const int q0 = qt * p.R;
   const int t_hi = min(q0 + p.R, p.T) - 1;
@@ -2611,7 +2611,7 @@ attn_bwd_kv_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_full + 2 * BUFS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc5::warp_index(), lane = tid & 31;
   // Heads fastest: under causality the first key blocks have the longest walks, and the last CTAs to start are short
   const int heads = p.B * p.Hkv, block = blockIdx.x / heads, b = (blockIdx.x - block * heads) / p.Hkv, h = blockIdx.x - block * heads - b * p.Hkv;
   const int s0 = block * KEYS;
@@ -2958,7 +2958,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc5::warp_index(), lane = tid & 31;
   // ---- which block, which visits (uniform over the CTA; CTAs without work leave before any setup)
   int b, h, s0, v0, n_vis, lst0 = 0, cnt = 0;
   if (SELECTED) {

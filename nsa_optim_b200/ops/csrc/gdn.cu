@@ -406,7 +406,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   float* red = reinterpret_cast<float*>(tmem_slot + 2);     // [2][8]
 
   const int r = threadIdx.x & 127, half = (threadIdx.x >> 7) & 1;
-  const int warp = threadIdx.x >> 5;
+  const int warp = tc5::warp_index();
   const int vt = blockIdx.x, bh = blockIdx.y, h = bh % p.H, b = bh / p.H;
   const int NC = p.NC;
 
@@ -446,7 +446,7 @@ gdn_seq_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const float* gc = p.gc + static_cast<long>(bh) * NC * CH;
   if (warp < 8) {
     const uint32_t lane_off = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * HC;   // lanes and columns of this thread
-    const bool upper = r < CH;                     // rows of k dS and du; the others bring do
+    const bool upper = (warp & 3) < 2;                     // rows of k dS and du; the others bring do
     {
       float z[HC];
 #pragma unroll

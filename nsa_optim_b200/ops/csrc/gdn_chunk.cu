@@ -343,7 +343,7 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
   float* sY = reinterpret_cast<float*>(tiles + POST_B + TILE);   // X^T dX, then dA
   float* sFQ = reinterpret_cast<float*>(tiles);            // [64][128] at the very end
   float* sFK = reinterpret_cast<float*>(tiles + POST_B);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc5::warp_index(), lane = tid & 31;
   const int bh = blockIdx.x, h = bh % p.H, b = bh / p.H, c = blockIdx.z * gridDim.y + blockIdx.y;   // see chunk_grid
   if (c >= p.NC) return;
   const int t0 = c * CH, V = p.V, nvt = V / CH;
@@ -398,7 +398,7 @@ gdn_post_kernel(const __grid_constant__ CUtensorMap tm_du, const __grid_constant
   const bool lower = n16 <= m0;                            // of a 64 x 64 product: not all above the diagonal
   // tensor-memory view: lane row (0..63 the upper operand of a stack, 64..127 the lower), 32 columns from n32
   const int row = (warp & 3) * 32 + lane, ri = row & 63;
-  const bool upper = row < CH;                             // uniform in a warp
+  const bool upper = (warp & 3) < 2;
   const uint32_t trow = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + n32;
   constexpr uint32_t cWQ = 0, cKS = 128;                   // accumulator columns of the two products
   constexpr uint32_t idesc = tc5::make_idesc_bf16(128, 128, 0, 0);

@@ -329,7 +329,7 @@ ssd_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(left + OUT_ST);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = tc5::warp_index();
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int i = 0; i < OUT_ST; ++i) { tc5::mbar_init(full + i, 1); tc5::mbar_init(left + i, 16); }
@@ -588,7 +588,7 @@ ssd_chunk_grad_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = tc5::warp_index();
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     tc5::mbar_init(full, 1);
@@ -1023,7 +1023,7 @@ ssd_walk_kernel(const __grid_constant__ CUtensorMap tm_bc, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(left + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* decay = reinterpret_cast<float*>(tmem_slot + 2);        // [WALK_ACC]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.x / PARTS, n0 = blockIdx.x % PARTS * ROWS,
+  const int warp = tc5::warp_index(), lane = threadIdx.x & 31, h = blockIdx.x / PARTS, n0 = blockIdx.x % PARTS * ROWS,
             b = blockIdx.y, nc = p.nc;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
