@@ -618,7 +618,21 @@ long env_long(const char* name, long otherwise) {
 }
 
 // (token lists, list starts, first CTA of a list, bound of the CTAs): see native.inverse_blocks
-struct Inverse { Tensor tok, list_start, item_start; long bound = 0; };
+struct Inverse {
+  Tensor tok, list_start, item_start;
+  long bound = 0;
+  static Inverse of(Args& a) {                   // None or (tok, list_start, item_start, nS, bound)
+    Inverse v;
+    PyObject* o = a.next();
+    if (o == Py_None) return v;
+    TORCH_CHECK_TYPE(PyTuple_Check(o) && PyTuple_GET_SIZE(o) == 5, "_nsa_host: inverse lists have to be a tuple of five");
+    PyObject* p[5];
+    for (int i = 0; i < 5; ++i) p[i] = PyTuple_GET_ITEM(o, i);
+    Args g{p, 5};
+    v.tok = g.t(); v.list_start = g.t(); v.item_start = g.t(); g.l(); v.bound = g.l();
+    return v;
+  }
+};
 Inverse inverse_lists(const Tensor& idx_, long nS, long R, long visits) {
   const Tensor idx = to(idx_, I32).contiguous();
   const long BH = idx.size(0) * idx.size(1), T = idx.size(2), n = idx.size(3), lists = BH * nS;
@@ -671,15 +685,7 @@ OP(attn_bwd) {                                   // q, k, v, o, dO, L, range, ti
     const Tensor &q = a.t(), &k = a.t(), &v = a.t(), &o = a.t(), &dO_ = a.t(), &L = a.t();
     const Range r = Range::of(a);
     const Tiles t = Tiles::of(a);
-    Inverse inv;
-    PyObject* lists = a.next();
-    if (lists != Py_None) {                      // (tok, list_start, item_start, nS, bound)
-      TORCH_CHECK_TYPE(PyTuple_Check(lists) && PyTuple_GET_SIZE(lists) == 5, "_nsa_host: inverse lists have to be a tuple of five");
-      PyObject* p[5];
-      for (int i = 0; i < 5; ++i) p[i] = PyTuple_GET_ITEM(lists, i);
-      Args g{p, 5};
-      inv.tok = g.t(); inv.list_start = g.t(); inv.item_start = g.t(); g.l(); inv.bound = g.l();
-    }
+    const Inverse inv = Inverse::of(a);
     const long walks = a.l();
     const bool split = a.b();
     return [=]() -> List {
@@ -830,12 +836,13 @@ OP(pool_bwd) {                                   // dy, T, block, stride -> dx
   });
 }
 
-OP(nsa_bwd) {                                    // q, k, v, kc, vc, o1, d1, L1, e1, ... of three branches, tiles, stride, block, window, scale
+OP(nsa_bwd) {                                    // q, k, v, kc, vc, o1, d1, L1, e1, ... of three branches, tiles, inverse lists, stride, block, window, scale
   return entry(py, np, [](Args& a) {             // -> dq, dk, dv, dkc, dvc
     const Tensor &q = a.t(), &k = a.t(), &v = a.t(), &kc = a.t(), &vc = a.t();
     Tensor o[3], d[3], L[3], e[3];
     for (int i = 0; i < 3; ++i) { o[i] = a.t(); d[i] = a.t(); L[i] = a.t(); e[i] = a.t(); }
     const Tiles t = Tiles::of(a);
+    const Inverse lists = Inverse::of(a);
     const int stride = a.w(), block = a.w(), window = a.w();
     const float scale = a.f();
     return [=]() -> List {
@@ -848,7 +855,6 @@ OP(nsa_bwd) {                                    // q, k, v, kc, vc, o1, d1, L1,
       const int pooled = walks(kc, 0, stride);
       const Tensor dkc = key_grad(kc, pooled != 0), dvc = key_grad(vc, pooled != 0);
       attn_backward(q, kc, vc, o[0], d[0], L[0], dq, dkc, dvc, {1, 0, scale, stride, block - 1}, Tiles(), Inverse(), visits, pooled, e[0], false);
-      const Inverse lists = inverse_lists(t.idx, t.nS, 128 / (Hq / Hkv), per_list);
       attn_backward(q, k, v, o[1], d[1], L[1], dq, dk, dv, {1, 0, scale, 1, 0}, t, lists, per_list, 0, e[1], true);
       // The window branch shares dk / dv while a key block's gradients get one addition from it: one more to what is there gives
       // the same bits on every run, two in either order would not.

@@ -734,7 +734,7 @@ class _Attn(torch.autograd.Function):
             walks_of = load().nsa_attn_bwd_walks if D == 128 else load().nsa_attn_bwd_walks_d64
             walks = walks_of(B, T, S, Hq, Hkv, int(causal), window, kp_stride)
         elif split:
-            lists = inverse_blocks(tiles[4], tiles[5], 128 // (Hq // Hkv), int(os.environ.get("NSA_B200_KV_VISITS_SEL", "64")))
+            lists = _inverse_of(tiles, Hq // Hkv)
         return (*_host.attn_bwd(q, k, v, o, do, L, *ctx.cfg, tiles, lists, walks, split), None, None, None, None, None, None)
 
 
@@ -768,6 +768,11 @@ def inverse_blocks(idx: Tensor, nS: int, R: int, visits_per_cta: int):
     tok, list_start, item_start = _h().inverse_blocks(idx, nS, R, visits_per_cta)
     bound = (B * Hkv * T * n) // (R * visits_per_cta) + B * Hkv * nS
     return tok, list_start, item_start, nS, bound
+
+
+def _inverse_of(tiles, G: int):
+    """Inverse lists of a selection's tiles, in the groups of tokens of one CTA of the dK / dV kernel."""
+    return inverse_blocks(tiles[4], tiles[5], 128 // G, int(os.environ.get("NSA_B200_KV_VISITS_SEL", "64")))
 
 
 def _inverse_blocks_torch(idx: Tensor, nS: int, R: int, visits_per_cta: int):
@@ -936,7 +941,8 @@ class _NSA(torch.autograd.Function):
         q, k, v, kc, vc, gl, o1, o2, o3, L1, L2, L3 = ctx.saved_tensors
         e1, e2, e3 = (_empty_like(L1) for _ in range(3))
         d1, d2, d3, dgl = _gate_logits_backward(o1, o2, o3, gl, do, (e1, e2, e3))
-        grads = _host.nsa_bwd(q, k, v, kc, vc, o1, d1, L1, e1, o2, d2, L2, e2, o3, d3, L3, e3, ctx.tiles, *ctx.cfg)
+        lists = _inverse_of(ctx.tiles, q.shape[2] // k.shape[2])
+        grads = _host.nsa_bwd(q, k, v, kc, vc, o1, d1, L1, e1, o2, d2, L2, e2, o3, d3, L3, e3, ctx.tiles, lists, *ctx.cfg)
         return (*grads, dgl.to(ctx.gdtype), None, None, None, None, None, None)
 
 
