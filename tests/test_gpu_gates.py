@@ -42,3 +42,15 @@ def test_recorded_calls_stay_differentiable(native):
     with torch.no_grad():
         ops.step_sizes(a, bias, A_log)
     assert native.launch_count() == before + 1
+
+
+def test_parameters_on_the_host_are_treated_as_by_pytorch(native):
+    a, b, bias, A_log = _inputs(1, 40, 6, torch.float32)
+    before = native.launch_count()
+    for call in (lambda: ops.step_sizes(a, bias.cpu(), A_log), lambda: ops.delta_gates(a, b, bias.cpu(), A_log),
+                 lambda: ops.delta_gates(a, b, bias, A_log.cpu())):
+        with pytest.raises(RuntimeError):
+            call()
+    assert all(x.device == y.device and torch.equal(x.nan_to_num(123.0), y.nan_to_num(123.0))
+               for x, y in zip(ops.step_sizes(a, bias, A_log.cpu()), torch_impl.step_sizes(a, bias, A_log.cpu())))
+    assert native.launch_count() == before

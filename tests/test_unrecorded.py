@@ -61,3 +61,15 @@ def test_transforms_see_the_function(applied, monkeypatch, grad):
         monkeypatch.setattr(torch.compiler, "is_compiling", lambda: True)
         native._run(_Double, x, 6.0)
     assert applied == [1.0, 2.0, 3.0, 4.0, 5.0, 6.0]
+
+
+@pytest.mark.parametrize("elsewhere", [None, "b", "dt_bias", "A_log"])
+def test_gates_of_tensors_on_several_devices_are_left_to_pytorch(monkeypatch, elsewhere):
+    calls = []
+    monkeypatch.setattr(native, "_h", lambda: type("Host", (), {"gates": lambda self, *a: calls.append(a) or "launched"})())
+    t = {n: torch.zeros(*s, dtype=torch.bfloat16, device="cpu" if n == elsewhere else "meta")
+         for n, s in (("a", (1, 4, 8)), ("b", (1, 4, 8)), ("dt_bias", (8,)), ("A_log", (8,)))}
+    assert native.delta_gates(**t) == (None if elsewhere else "launched")
+    del t["b"]
+    assert native.step_sizes(t["a"], t["dt_bias"], t["A_log"]) == (None if elsewhere in ("dt_bias", "A_log") else "launched")
+    assert len(calls) == (2 if elsewhere is None else elsewhere == "b")
