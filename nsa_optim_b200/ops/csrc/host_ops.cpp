@@ -22,6 +22,7 @@
 
 #include <cmath>
 #include <cstdlib>
+#include <limits>
 #include <vector>
 
 #include "nsa_b200.h"
@@ -147,6 +148,13 @@ struct Args {
     const unsigned long v = PyLong_AsUnsignedLongMask(o);
     if (v == static_cast<unsigned long>(-1) && PyErr_Occurred()) throw python_error();
     return static_cast<long>(v);
+  }
+  long count() {                                 // as above, but wider numbers become the largest or the smallest
+    PyObject* o = next();
+    int over = 0;
+    const long v = PyLong_AsLongAndOverflow(o, &over);
+    if (v == -1 && PyErr_Occurred()) throw python_error();
+    return over > 0 ? std::numeric_limits<long>::max() : over < 0 ? std::numeric_limits<long>::min() : v;
   }
   int w() { return static_cast<int>(l()); }
   bool b() { return l() != 0; }
@@ -539,10 +547,11 @@ OP(multi_linear_bwd) {                           // x rows, weights, gradients, 
 OP(cross_entropy_fwd) {                          // hidden, w, labels, ignore, chunk, want dh, want dw -> loss, dh, dw (fp32)
   return entry(py, np, [](Args& a) {
     const Tensor &hidden = a.t(), &w = a.t(), &labels_ = a.t();
-    const long ignore = a.l(), chunk = a.l();
+    const long ignore = a.l(), chunk = a.count();
     const bool need_h = a.b(), need_w = a.b();
     return [=]() -> List {
       want_dims(hidden, 2);
+      TORCH_CHECK_VALUE(chunk > 0, "cross entropy: chunks of ", chunk, " tokens");
       const long N = hidden.size(0), d = hidden.size(1), V = w.size(0);
       const Tensor h = matrix(hidden), labels = labels_.contiguous();
       const Tensor inv = labels.ne(ignore).sum().clamp_min(1).to(F32).reciprocal().reshape(1);
@@ -550,8 +559,8 @@ OP(cross_entropy_fwd) {                          // hidden, w, labels, ignore, c
       const Tensor dh = need_h ? alloc({N, d}, h.scalar_type(), h.device()) : Tensor();
       const Tensor dw = need_w ? alloc({V, d}, F32, h.device(), N == 0) : Tensor();   // the first chunk's product writes it whole
       const Tensor logits = alloc({std::min(chunk, N), V}, BF, h.device());
-      for (long s0 = 0; s0 < N; s0 += chunk) {
-        const long n = std::min(chunk, N - s0);
+      for (long s0 = 0, n; s0 < N; s0 += n) {
+        n = std::min(chunk, N - s0);
         const Tensor lg = logits.narrow(0, 0, n), hs = h.narrow(0, s0, n);
         gemm(hs, w, false, false, lg);
         launch(lib.nsa_cross_entropy, ptr(lg), static_cast<const long*>(ptr(labels.narrow(0, s0, n))), fp(loss.narrow(0, s0, n)), fp(inv), n,

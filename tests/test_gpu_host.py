@@ -64,3 +64,19 @@ def test_refused_shapes(native):
         with pytest.raises((ValueError, IndexError, RuntimeError)):
             call()
         assert native.launch_count() == before
+
+
+def test_chunks_of_the_cross_entropy(native):
+    g = torch.Generator("cuda").manual_seed(0)
+    h, w = (torch.randn(n, 64, device="cuda", generator=g).bfloat16().requires_grad_() for n in (300, 128))
+    ids = torch.randint(0, 128, (300,), device="cuda", generator=g)
+    before = native.launch_count()
+    for chunk in (0, -1, -2 ** 70):
+        with pytest.raises(ValueError):
+            native.linear_cross_entropy(h, w, ids, chunk=chunk)
+        with pytest.raises(ValueError):
+            native.linear_cross_entropy(h[:0], w, ids[:0], chunk=chunk)
+    assert native.launch_count() == before
+    grads = lambda **kw: torch.autograd.grad(native.linear_cross_entropy(h, w, ids, **kw), (h, w))       # noqa: E731
+    for chunk in (300, 2 ** 63 - 1, 2 ** 70):
+        assert all(torch.equal(a, b) for a, b in zip(grads(chunk=chunk), grads()))
