@@ -256,7 +256,7 @@ OP(rms_bwd) {                                    // x, w, rstd, dy, gradient of 
 // made contiguous.
 Tensor gate_rows(const Tensor& g) {
   const long d = g.size(-1);
-  if (g.dim() >= 2 && g.stride(-1) == 1 && aligned(g)) {
+  if (g.dim() >= 2 && d > 0 && g.stride(-1) == 1 && aligned(g)) {
     const long pitch = g.stride(-2);
     long expect = pitch;
     bool ok = pitch % 8 == 0 && pitch >= d;
@@ -716,6 +716,7 @@ OP(attn_bwd) {                                   // q, k, v, o, dO, L, range, ti
 
 // ------------------------------------------------------------------------------------- native sparse attention
 Tiles union_lists(const Tensor& idx, long G, long nS) {
+  TORCH_CHECK_VALUE(G > 0 && G <= 128, "union_blocks: groups of ", G, " query heads");
   const long B = idx.size(0), H = idx.size(1), T = idx.size(2), n = idx.size(3), R = 128 / G, tiles = (T + R - 1) / R;
   long most = std::min(R * n, nS);
   most += most & 1;
@@ -821,6 +822,7 @@ OP(pool_fwd) {                                   // x, block, stride -> y
     const int block = a.w(), stride = a.w();
     return [=]() -> Tensor {
       want_dims(x, 4);
+      TORCH_CHECK_VALUE(block > 0 && stride > 0, "nsa_compress: blocks of ", block, " tokens every ", stride);
       const long B = x.size(0), T = x.size(1), H = x.size(2), D = x.size(3);
       const bool ok = x.stride(3) == 1 && x.stride(2) == D && x.stride(1) % 8 == 0 && x.stride(0) == T * x.stride(1) && aligned(x);
       const Tensor xv = ok ? x : x.contiguous(), y = alloc({B, (T - block) / stride + 1, H, D}, x.scalar_type(), x.device());

@@ -80,3 +80,16 @@ def test_chunks_of_the_cross_entropy(native):
     grads = lambda **kw: torch.autograd.grad(native.linear_cross_entropy(h, w, ids, **kw), (h, w))       # noqa: E731
     for chunk in (300, 2 ** 63 - 1, 2 ** 70):
         assert all(torch.equal(a, b) for a, b in zip(grads(chunk=chunk), grads()))
+
+
+def test_sizes_of_zero_are_refused(native):
+    # each is a divisor on the host: an exception, not the end of the process
+    r = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)                # noqa: E731
+    idx = torch.zeros(1, 1, 8, 1, device="cuda", dtype=torch.int32)
+    before = native.launch_count()
+    for call in (lambda: native.nsa_compress(r(1, 64, 2, 8), 32, 0), lambda: native.nsa_compress(r(1, 64, 2, 8), 0, 16),
+                 lambda: native.nsa_compress(r(1, 64, 2, 8), 32, -16), lambda: native.union_blocks(idx, 0, 1), lambda: native.union_blocks(idx, 256, 1),
+                 lambda: native.gated_rms_norm(r(4, 8), r(4, 16)[:, 8:8], r(8))):
+        with pytest.raises((ValueError, RuntimeError)):
+            call()
+    assert native.launch_count() == before
