@@ -21,7 +21,6 @@
 #include <torch/csrc/utils/object_ptr.h>
 
 #include <cmath>
-#include <cstdlib>
 #include <limits>
 #include <vector>
 
@@ -621,11 +620,6 @@ std::pair<Tensor, Tensor> attn_forward(const Tensor& q, const Tensor& k, const T
   return {o, L};
 }
 
-long env_long(const char* name, long otherwise) {
-  const char* e = getenv(name);
-  return e ? atol(e) : otherwise;
-}
-
 // (token lists, list starts, first CTA of a list, bound of the CTAs): see native.inverse_blocks
 struct Inverse {
   Tensor tok, list_start, item_start;
@@ -671,9 +665,6 @@ void attn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
 }
 // dK or dV: written whole by contiguous ranges of several walks, one, or 64 keys a CTA; else to be added to
 Tensor key_grad(const Tensor& k, bool whole) { return alloc(k.sizes(), whole ? BF : F32, k.device(), !whole); }
-// Query tiles per CTA of the dK / dV kernel over a contiguous range, where a key block has more than 256, and over a list of tokens
-long range_visits() { return env_long("NSA_B200_KV_VISITS", 64); }
-long list_visits() { return env_long("NSA_B200_KV_VISITS_SEL", 64); }
 
 OP(attn_fwd) {                                   // q, k, v, range, tiles -> o, L, q, k, v dense
   return entry(py, np, [](Args& a) {
@@ -689,20 +680,20 @@ OP(attn_fwd) {                                   // q, k, v, range, tiles -> o, 
   });
 }
 
-OP(attn_bwd) {                                   // q, k, v, o, dO, L, range, tiles, inverse lists or None, walks -> dq, dk, dv
+OP(attn_bwd) {                                   // q, k, v, o, dO, L, range, tiles, inverse lists or None, visits, walks, split -> dq, dk, dv
   return entry(py, np, [](Args& a) {
     const Tensor &q = a.t(), &k = a.t(), &v = a.t(), &o = a.t(), &dO_ = a.t(), &L = a.t();
     const Range r = Range::of(a);
     const Tiles t = Tiles::of(a);
     const Inverse inv = Inverse::of(a);
-    const long walks = a.l();
+    const long visits = a.l(), walks = a.l();      // visits: query tiles per CTA of the dK / dV kernel, see native._range_visits
     const bool split = a.b();
     return [=]() -> List {
       const Tensor dO = dense(dO_), dq = alloc(q.sizes(), q.scalar_type(), q.device());
       const bool whole = split && !t.any() && walks != 0;
       const Tensor dk = key_grad(k, whole), dv = key_grad(v, whole);
       if (split) {
-        attn_backward(q, k, v, o, dO, L, dq, dk, dv, r, t, inv, t.any() ? list_visits() : range_visits(), walks, Tensor(), false);
+        attn_backward(q, k, v, o, dO, L, dq, dk, dv, r, t, inv, visits, walks, Tensor(), false);
       } else {
         const Tensor delta = alloc(q.sizes().slice(0, 3), F32, q.device());
         launch(lib.nsa_attn_bwd, ptr(q), ptr(k), ptr(v), ptr(o), ptr(dO), fp(L), fp(delta), ptr(dq), fp(dk), fp(dv), dim(q.size(0)), dim(q.size(1)),
@@ -847,13 +838,14 @@ OP(pool_bwd) {                                   // dy, T, block, stride -> dx
   });
 }
 
-OP(nsa_bwd) {                                    // q, k, v, kc, vc, o1, d1, L1, e1, ... of three branches, tiles, inverse lists, stride, block, window, scale
-  return entry(py, np, [](Args& a) {             // -> dq, dk, dv, dkc, dvc
+OP(nsa_bwd) {                                    // q, k, v, kc, vc, o1, d1, L1, e1, ... of three branches, tiles, inverse lists, visits of ranges
+  return entry(py, np, [](Args& a) {             // and lists, stride, block, window, scale -> dq, dk, dv, dkc, dvc
     const Tensor &q = a.t(), &k = a.t(), &v = a.t(), &kc = a.t(), &vc = a.t();
     Tensor o[3], d[3], L[3], e[3];
     for (int i = 0; i < 3; ++i) { o[i] = a.t(); d[i] = a.t(); L[i] = a.t(); e[i] = a.t(); }
     const Tiles t = Tiles::of(a);
     const Inverse lists = Inverse::of(a);
+    const long visits = a.l(), per_list = a.l();
     const int stride = a.w(), block = a.w(), window = a.w();
     const float scale = a.f();
     return [=]() -> List {
@@ -862,7 +854,6 @@ OP(nsa_bwd) {                                    // q, k, v, kc, vc, o1, d1, L1,
       const Tensor dq = alloc(q.sizes(), q.scalar_type(), dev);
       Tensor dk = alloc(k.sizes(), F32, dev, true), dv = alloc(v.sizes(), F32, dev, true);
       auto walks = [&](const Tensor& keys, int win, int kp) { return have(lib.nsa_attn_bwd_walks)(B, T, dim(keys.size(1)), Hq, Hkv, 1, win, kp); };
-      const long visits = range_visits(), per_list = list_visits();
       const int pooled = walks(kc, 0, stride);
       const Tensor dkc = key_grad(kc, pooled != 0), dvc = key_grad(vc, pooled != 0);
       attn_backward(q, kc, vc, o[0], d[0], L[0], dq, dkc, dvc, {1, 0, scale, stride, block - 1}, Tiles(), Inverse(), visits, pooled, e[0], false);

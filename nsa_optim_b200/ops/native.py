@@ -704,6 +704,17 @@ def gated_delta_rule(q, k, v, g, beta, scale=None, chunk=64):
 # --------------------------------------------------------------------------------------
 # attention family (csrc/attention.cu)
 # --------------------------------------------------------------------------------------
+def _range_visits() -> int:
+    """Query tiles per CTA of the dK / dV kernel over a contiguous key range, where a key block has more than 256.  The environment is
+    read here, under the GIL: another thread's assignment to os.environ may move what a native getenv walks."""
+    return int(os.environ.get("NSA_B200_KV_VISITS", "64"))
+
+
+def _list_visits() -> int:
+    """The same over a list of tokens."""
+    return int(os.environ.get("NSA_B200_KV_VISITS_SEL", "64"))
+
+
 def _bwd_is_split(D: int, G: int, selected: bool) -> bool:
     return os.environ.get("NSA_B200_ATTN_BWD", "split") == "split" and (not selected or (D == 128 and G >= 8))
 
@@ -727,6 +738,7 @@ class _Attn(torch.autograd.Function):
     def backward(ctx, do, _dL):
         q, k, v, o, L = ctx.saved_tensors
         (causal, window, _, kp_stride, _), tiles, lists, walks = ctx.cfg, ctx.tiles, None, 0
+        visits = _range_visits() if tiles is None else _list_visits()
         B, T, Hq, D = q.shape
         S, Hkv = k.shape[1], k.shape[2]
         split = _bwd_is_split(D, Hq // Hkv, tiles is not None)
@@ -734,8 +746,8 @@ class _Attn(torch.autograd.Function):
             walks_of = load().nsa_attn_bwd_walks if D == 128 else load().nsa_attn_bwd_walks_d64
             walks = walks_of(B, T, S, Hq, Hkv, int(causal), window, kp_stride)
         elif split:
-            lists = _inverse_of(tiles, Hq // Hkv)
-        return (*_host.attn_bwd(q, k, v, o, do, L, *ctx.cfg, tiles, lists, walks, split), None, None, None, None, None, None)
+            lists = _inverse_of(tiles, Hq // Hkv, visits)
+        return (*_host.attn_bwd(q, k, v, o, do, L, *ctx.cfg, tiles, lists, visits, walks, split), None, None, None, None, None, None)
 
 
 def _attn_ok(q, k) -> bool:
@@ -770,9 +782,9 @@ def inverse_blocks(idx: Tensor, nS: int, R: int, visits_per_cta: int):
     return tok, list_start, item_start, nS, bound
 
 
-def _inverse_of(tiles, G: int):
-    """Inverse lists of a selection's tiles, in the groups of tokens of one CTA of the dK / dV kernel."""
-    return inverse_blocks(tiles[4], tiles[5], 128 // G, int(os.environ.get("NSA_B200_KV_VISITS_SEL", "64")))
+def _inverse_of(tiles, G: int, visits: int):
+    """Inverse lists of a selection's tiles for a dK / dV kernel of ``visits`` query tiles per CTA."""
+    return inverse_blocks(tiles[4], tiles[5], 128 // G, visits)
 
 
 def _inverse_blocks_torch(idx: Tensor, nS: int, R: int, visits_per_cta: int):
@@ -941,8 +953,10 @@ class _NSA(torch.autograd.Function):
         q, k, v, kc, vc, gl, o1, o2, o3, L1, L2, L3 = ctx.saved_tensors
         e1, e2, e3 = (_empty_like(L1) for _ in range(3))
         d1, d2, d3, dgl = _gate_logits_backward(o1, o2, o3, gl, do, (e1, e2, e3))
-        lists = _inverse_of(ctx.tiles, q.shape[2] // k.shape[2])
-        grads = _host.nsa_bwd(q, k, v, kc, vc, o1, d1, L1, e1, o2, d2, L2, e2, o3, d3, L3, e3, ctx.tiles, lists, *ctx.cfg)
+        visits = _list_visits()
+        lists = _inverse_of(ctx.tiles, q.shape[2] // k.shape[2], visits)
+        grads = _host.nsa_bwd(q, k, v, kc, vc, o1, d1, L1, e1, o2, d2, L2, e2, o3, d3, L3, e3, ctx.tiles, lists,
+                              _range_visits(), visits, *ctx.cfg)
         return (*grads, dgl.to(ctx.gdtype), None, None, None, None, None, None)
 
 
