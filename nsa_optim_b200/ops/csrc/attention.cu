@@ -3922,13 +3922,14 @@ extern "C" int nsa_inverse_blocks(const int* idx, int* tok_list, int* list_start
                                   int BH, int T, int n, int nS, int R, int visits_per_cta, cudaStream_t st) {
   if (BH <= 0 || T <= 0 || n <= 0 || nS <= 0 || R <= 0 || visits_per_cta <= 0)
     return nsa::fail(NSA_ERR_SHAPE, "nsa_inverse_blocks: empty problem");
-  if (nS * 4 > 48 * 1024 || n > 32) return nsa::fail(NSA_ERR_SHAPE, "nsa_inverse_blocks: at most 12288 selection blocks and 32 entries per token");
+  constexpr int MOST = 12288;
+  if (nS > MOST || n > 32) return nsa::fail(NSA_ERR_SHAPE, "nsa_inverse_blocks: at most 12288 selection blocks and 32 entries per token");
   const int len = inverse_chunk(BH, T, nS), chunks = nsa_inverse_chunks(BH, T, nS);
   const long lists = static_cast<long>(BH) * nS;
   const dim3 grid(chunks, BH);
   const int bytes = nS * 12;
-  if (bytes > 48 * 1024)
-    if (int rc = set_smem(nsa_inverse_walk_kernel, bytes)) return rc;
+  if (bytes > 48 * 1024)                         // the same limit in every call: another thread's must not lower it in front of a launch
+    if (int rc = set_smem(nsa_inverse_walk_kernel, MOST * 12)) return rc;
   nsa_inverse_walk_kernel<<<grid, WALK_THREADS, bytes, st>>>(idx, hist, nullptr, nullptr, nullptr, T, n, nS, chunks, len, 0);
   nsa_inverse_offsets_kernel<<<(unsigned)((lists + 31) / 32), 256, 0, st>>>(hist, count, lists, nS, chunks);
   nsa_inverse_scan_kernel<<<1, 1024, 0, st>>>(count, list_start, item_start, lists, R, visits_per_cta);
