@@ -136,6 +136,7 @@ struct Args {
     std::vector<Tensor> v(PyTuple_GET_SIZE(o));
     for (size_t k = 0; k < v.size(); ++k) {
       PyObject* x = PyTuple_GET_ITEM(o, k);
+      TORCH_CHECK_TYPE(x == Py_None || THPVariable_Check(x), "_nsa_host: argument ", i - 1, " has to be a tuple of tensors and None");
       if (x != Py_None) v[k] = THPVariable_Unpack(x);
     }
     return v;
@@ -1017,46 +1018,64 @@ void need(const char* what, PyObject* o, long n) {
   TORCH_CHECK_VALUE(have == n, "optimizer state '", what, "' has ", have, " elements, the kernel needs ", n);
 }
 
+// A list or tuple (another sequence becomes a list), held while its items are read
+struct Sequence {
+  THPObjectPtr held;
+  explicit Sequence(PyObject* o) {
+    TORCH_CHECK_TYPE(PySequence_Check(o), "_nsa_host: the tensors to update have to be a sequence of sequences");
+    held = PySequence_Fast(o, "_nsa_host: the tensors to update have to be a sequence of sequences");
+    if (!held) throw python_error();
+  }
+  long size() const { return PySequence_Fast_GET_SIZE(held.get()); }
+  PyObject* operator[](long i) const { return PySequence_Fast_GET_ITEM(held.get(), i); }
+};
+
 // Seven 64-bit words per tensor, (p, g, m, v, a, b, n).  Every state tensor is checked against n; with a block the last two are the
 // scales of the quantised moments, else an fp32 master copy (or None) and nothing.
-std::vector<long long> adamw_words(PyObject* items, long block) {
-  TORCH_CHECK_TYPE(PyList_Check(items), "_nsa_host: the tensors to update have to be a list");
+struct Updates {
   std::vector<long long> words;
-  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(items); ++i) {
-    PyObject* it = PyList_GET_ITEM(items, i);
-    TORCH_CHECK_TYPE(PyTuple_Check(it) && PyTuple_GET_SIZE(it) == 6, "_nsa_host: six tensors or None for each parameter");
-    PyObject* o[6];
-    for (int k = 0; k < 6; ++k) {
-      o[k] = PyTuple_GET_ITEM(it, k);
-      TORCH_CHECK_TYPE(THPVariable_Check(o[k]) || (k > 3 && o[k] == Py_None), "_nsa_host: six tensors or None for each parameter");
+  int count = 0, p_fp32 = 0, g_fp32 = 0;         // the types are those of the first
+  Updates(PyObject* list, long block) {
+    const Sequence items(list);
+    count = dim(items.size());
+    TORCH_CHECK_INDEX(count > 0, "_nsa_host: no tensors to update");
+    words.reserve(7 * count);
+    for (long i = 0; i < count; ++i) {
+      const Sequence it(items[i]);
+      TORCH_CHECK_VALUE(it.size() == 6, "_nsa_host: six tensors or None for each parameter");
+      PyObject* o[6];
+      for (int k = 0; k < 6; ++k) {
+        o[k] = it[k];
+        TORCH_CHECK_TYPE(THPVariable_Check(o[k]) || (k > 3 && o[k] == Py_None), "_nsa_host: six tensors or None for each parameter");
+      }
+      const long n = THPVariable_Unpack(o[0]).numel(), na = block ? n / block : n;
+      TORCH_CHECK_VALUE(!block || n % block == 0, "8-bit AdamW needs a multiple of ", block, " elements, got ", n);
+      need("grad", o[1], n);
+      need("exp_avg", o[2], n);
+      need("exp_avg_sq", o[3], n);
+      need(block ? "exp_avg_absmax" : "master", o[4], na);
+      need("exp_avg_sq_absmax", o[5], na);
+      for (PyObject* x : o) words.push_back(x == Py_None ? 0 : reinterpret_cast<long long>(THPVariable_Unpack(x).data_ptr()));
+      words.push_back(n);
+      if (i == 0) {
+        p_fp32 = THPVariable_Unpack(o[0]).scalar_type() == F32;
+        g_fp32 = THPVariable_Unpack(o[1]).scalar_type() == F32;
+      }
     }
-    const long n = THPVariable_Unpack(o[0]).numel(), na = block ? n / block : n;
-    TORCH_CHECK_VALUE(!block || n % block == 0, "8-bit AdamW needs a multiple of ", block, " elements, got ", n);
-    need("grad", o[1], n);
-    need("exp_avg", o[2], n);
-    need("exp_avg_sq", o[3], n);
-    need(block ? "exp_avg_absmax" : "master", o[4], na);
-    need("exp_avg_sq_absmax", o[5], na);
-    for (PyObject* x : o) words.push_back(x == Py_None ? 0 : reinterpret_cast<long long>(THPVariable_Unpack(x).data_ptr()));
-    words.push_back(n);
   }
-  return words;
-}
+};
 
 OP(adamw) {                                      // items, gradient scale or None, step, lr, b1, b2, eps, wd
   HANDLE_TH_ERRORS
   Args a{py, np};
-  const auto words = adamw_words(a.next(), 0);
-  const Tensor& p = THPVariable_Unpack(PyTuple_GET_ITEM(PyList_GET_ITEM(py[0], 0), 0));
-  const Tensor& g = THPVariable_Unpack(PyTuple_GET_ITEM(PyList_GET_ITEM(py[0], 0), 1));
+  const Updates u(a.next(), 0);
   const Tensor s = a.opt();
   const int step = a.w();
   const float lr = a.f(), b1 = a.f(), b2 = a.f(), eps = a.f(), wd = a.f();
   {
     Call call;
     const Tensor sf = s.defined() ? s.reshape(1).to(F32) : s;
-    launch(lib.nsa_adamw_multi, words.data(), static_cast<int>(words.size() / 7), fp(sf), static_cast<int>(p.scalar_type() == F32),
-           static_cast<int>(g.scalar_type() == F32), step, lr, b1, b2, eps, wd);
+    launch(lib.nsa_adamw_multi, u.words.data(), u.count, fp(sf), u.p_fp32, u.g_fp32, step, lr, b1, b2, eps, wd);
   }
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
@@ -1070,14 +1089,11 @@ OP(adamw8bit) {                                  // items, code books, gradient 
   const Tensor s = a.opt();
   const int step = a.w();
   const float lr = a.f(), b1 = a.f(), b2 = a.f(), eps = a.f(), wd = a.f();
-  const auto words = adamw_words(items, a.l());
-  const Tensor& p = THPVariable_Unpack(PyTuple_GET_ITEM(PyList_GET_ITEM(items, 0), 0));
-  const Tensor& g = THPVariable_Unpack(PyTuple_GET_ITEM(PyList_GET_ITEM(items, 0), 1));
+  const Updates u(items, a.l());
   {
     Call call;
     const Tensor sf = s.defined() ? s.reshape(1).to(F32) : s;
-    launch(lib.nsa_adamw8bit_multi, words.data(), static_cast<int>(words.size() / 7), fp(cs), fp(cu), fp(sf),
-           static_cast<int>(p.scalar_type() == F32), static_cast<int>(g.scalar_type() == F32), step, lr, b1, b2, eps, wd);
+    launch(lib.nsa_adamw8bit_multi, u.words.data(), u.count, fp(cs), fp(cu), fp(sf), u.p_fp32, u.g_fp32, step, lr, b1, b2, eps, wd);
   }
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS

@@ -93,3 +93,23 @@ def test_sizes_of_zero_are_refused(native):
         with pytest.raises((ValueError, RuntimeError)):
             call()
     assert native.launch_count() == before
+
+
+def test_arguments_of_the_wrong_kind_are_refused(native):
+    r = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)                # noqa: E731
+    f = lambda *s: torch.zeros(*s, device="cuda")                                      # noqa: E731
+    hyper = (1, 1e-3, .9, .95, 1e-8, 0.0, None)
+    item = (r(256), r(256), f(256), f(256), None, None)
+    before = native.launch_count()
+    for call, error in ((lambda: native.adamw_multi([], *hyper), IndexError), (lambda: native.adamw8bit_multi([], *hyper, 256), IndexError),
+                        (lambda: native.adamw_multi([item[:5]], *hyper), ValueError), (lambda: native.adamw_multi([3], *hyper), TypeError),
+                        (lambda: native.adamw_multi([(3,) + item[1:]], *hyper), TypeError), (lambda: native.adamw_multi(3, *hyper), TypeError),
+                        (lambda: native._h().multi_linear_fwd(r(256, 64), (r(64, 64), 3)), TypeError)):
+        with pytest.raises(error):
+            call()
+    assert native.launch_count() == before
+    ref = torch.ones(256, device="cuda")
+    for kind in (list, tuple):                       # any sequence of sequences
+        p, g = ref.clone(), ref.clone()
+        native.adamw_multi(kind([kind([p, g, f(256), f(256), None, None])]), *hyper)
+        assert native.launch_count() > before and (p < 1).all()
