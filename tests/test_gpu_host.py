@@ -2,6 +2,7 @@
 refused before anything is launched."""
 import threading
 
+import numpy as np
 import pytest
 import torch
 from test_gpu_unrecorded import _cases
@@ -113,3 +114,18 @@ def test_arguments_of_the_wrong_kind_are_refused(native):
         p, g = ref.clone(), ref.clone()
         native.adamw_multi(kind([kind([p, g, f(256), f(256), None, None])]), *hyper)
         assert native.launch_count() > before and (p < 1).all()
+
+
+def test_flags_of_any_kind(native):
+    g = torch.Generator("cuda").manual_seed(0)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16().requires_grad_()   # noqa: E731
+    x, w, q, k, a, b = r(1, 20, 64), r(64, 4), r(1, 20, 4, 64), r(1, 20, 2, 64), r(64, 40).detach(), r(64, 24).detach()
+    for on in (True, False):
+        for op, inputs in ((lambda f: native.causal_conv1d(x, w, None, f), (x, w)), (lambda f: native.attention(q, k, k, f), (q, k))):
+            want = [y := op(on), *torch.autograd.grad(y, inputs, torch.ones_like(y))]
+            for flag in (np.bool_(on), float(on), int(on), torch.tensor(on)):
+                got = [y := op(flag), *torch.autograd.grad(y, inputs, torch.ones_like(y))]
+                assert all(torch.equal(s, t) for s, t in zip(got, want))
+        out = torch.ones(40, 24, device="cuda")
+        want = native.gemm(a, b, True, True, out=out.clone(), accumulate=on)
+        assert torch.equal(native.gemm(a, b, np.True_, np.True_, out=out.clone(), accumulate=np.bool_(on)), want)
