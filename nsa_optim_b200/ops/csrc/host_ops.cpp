@@ -268,7 +268,7 @@ Tensor gate_rows(const Tensor& g) {
   }
   return g.reshape({-1, d}).contiguous();
 }
-// Elements from one row (last dimension) to the next.  Read from a saved tensor as it comes back: saved-tensor hooks (activations
+// Elements from one row (last dimension) to the next; a single row of a dense tensor may have any stride.  Read from a saved tensor as it comes back: saved-tensor hooks (activations
 // kept on the host) return a pitched view as a dense tensor.
 long row_pitch(const Tensor& t) { return t.is_contiguous() ? t.size(-1) : t.stride(-2); }
 
@@ -281,7 +281,7 @@ OP(gated_rms_fwd) {                              // x, gate, w, eps, mode -> y, 
       const Tensor xc = dense(x), g = gate_rows(gate), wb = to(w, BF);
       const long d = xc.size(-1), rows = rows_of(xc);
       const Tensor y = alloc(x.sizes(), x.scalar_type(), x.device()), rstd = alloc({rows}, F32, x.device());
-      launch(lib.nsa_rmsnorm_fwd_ldg, ptr(xc), ptr(g), g.stride(0), ptr(wb), ptr(y), fp(rstd), rows, dim(d), eps, mode);
+      launch(lib.nsa_rmsnorm_fwd_ldg, ptr(xc), ptr(g), row_pitch(g), ptr(wb), ptr(y), fp(rstd), rows, dim(d), eps, mode);
       return {y, xc, g, wb, rstd};
     };
   });
@@ -920,7 +920,8 @@ Tensor token_rows(const Tensor& t) {
                   t.select(0, 0).select(0, 0).is_contiguous();
   return ok ? t : t.contiguous();
 }
-long token_pitch(const Tensor& t) { return row_pitch(t.flatten(2)); }      // as it came back from the saved tensors
+// Elements from a token to the next, also of a saved tensor as it comes back.  Not the stride of a dense tensor: a single token may have any.
+long token_pitch(const Tensor& t) { return t.is_contiguous() ? c10::multiply_integers(t.sizes().slice(2)) : t.stride(1); }
 
 // bf16 states entering the chunks (back: gradients of those leaving them), and the chunks' decays where the two-kernel form needs them
 std::pair<Tensor, Tensor> ssd_states(bool back, const Tensor& rows, long ld_rows, const Tensor& v, long ld_v, const Tensor& dt, const Tensor& A,
@@ -952,9 +953,10 @@ OP(ssd_fwd) {                                    // x, dt, A, B, C, D or None ->
       const Tensor x = token_rows(x_), Bm = token_rows(B_), Cm = token_rows(C_);
       const Tensor dt = to(dt_, F32).contiguous(), A = to(A_, F32).contiguous(), D = D_.defined() ? to(D_, F32).contiguous() : D_;
       const long B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), N = Bm.size(-1);
-      auto [states, gamma] = ssd_states(false, Bm, Bm.stride(1), x, x.stride(1), dt, A, Tensor());
+      const long ldx = token_pitch(x), ldb = token_pitch(Bm), ldc = token_pitch(Cm);
+      auto [states, gamma] = ssd_states(false, Bm, ldb, x, ldx, dt, A, Tensor());
       const Tensor y = alloc({B, T, H, P}, BF, x.device());
-      launch(lib.nsa_ssd_chunk_out, ptr(Cm), Cm.stride(1), ptr(Bm), Bm.stride(1), ptr(x), x.stride(1), ptr(states), fp(dt), fp(A), fp(D), ptr(y),
+      launch(lib.nsa_ssd_chunk_out, ptr(Cm), ldc, ptr(Bm), ldb, ptr(x), ldx, ptr(states), fp(dt), fp(A), fp(D), ptr(y),
              dim(B), dim(T), dim(H), dim(N), dim(P));
       return {y, x, dt, A, Bm, Cm, D.defined() ? D : alloc({0}, F32, x.device()), gamma, states};
     };

@@ -138,3 +138,20 @@ def test_norm_backward_of_many_rows_is_memory_bound(native, rows, d, limit):
 
     copy = fastest(lambda: dst.copy_(src))
     assert fastest(lambda: torch.autograd.grad(y, [x, w], dy, retain_graph=True)) <= limit * copy
+
+
+def test_a_single_row_of_any_pitch(native):
+    # one token of a wider row, which counts as dense: its stride is no pitch that the kernels could take
+    g = torch.Generator("cuda").manual_seed(0)
+    cut = lambda h, n: torch.randn(1, 5, h * n + 1, device="cuda", generator=g).bfloat16()[..., :h * n].view(1, 5, h, n)[:, :1]      # noqa: E731
+    x, Bm, Cm, gate = cut(3, 64), cut(1, 128), cut(1, 128), cut(1, 256)[:, :, 0][0]
+    w = torch.rand(256, device="cuda", generator=g).bfloat16()
+    dt, A, D = torch.rand(1, 1, 3, device="cuda"), -torch.rand(3, device="cuda"), torch.rand(3, device="cuda")
+    assert all(t.is_contiguous() and t.stride(t.dim() // 4) % 8 for t in (x, Bm, Cm, gate))
+    for op, inputs in ((native.ssd_scan, (x, dt, A, Bm, Cm, D)), (native.gated_rms_norm, (gate, gate, w)), (native.gated_rms_norm, (gate, gate, w, 1e-6, False))):
+        results = []
+        for dense in (False, True):
+            leaves = [(t.clone(memory_format=torch.contiguous_format) if dense else t).detach().requires_grad_() if isinstance(t, torch.Tensor) else t for t in inputs]
+            y = op(*leaves)
+            results.append([y.detach(), *torch.autograd.grad(y, [t for t in leaves if isinstance(t, torch.Tensor)], torch.ones_like(y))])
+        assert all(torch.equal(a, b) for a, b in zip(*results))
