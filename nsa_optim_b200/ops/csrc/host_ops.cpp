@@ -156,6 +156,13 @@ struct Args {
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return over > 0 ? std::numeric_limits<long>::max() : over < 0 ? std::numeric_limits<long>::min() : v;
   }
+  std::vector<bool> bools() {                    // a tuple of truth values
+    PyObject* o = next();
+    TORCH_CHECK_TYPE(PyTuple_Check(o), "_nsa_host: argument ", i - 1, " has to be a tuple");
+    std::vector<bool> v(PyTuple_GET_SIZE(o));
+    for (size_t k = 0; k < v.size(); ++k) v[k] = PyTuple_GET_ITEM(o, k) == Py_True;
+    return v;
+  }
   int w() { return static_cast<int>(l()); }
   bool b() { return l() != 0; }
   float f() {
@@ -520,12 +527,13 @@ OP(multi_linear_fwd) {                           // x, weights -> outputs..., x 
   });
 }
 
-OP(multi_linear_bwd) {                           // x rows, weights, gradients, want dx, want each dw (bits) -> dx, dw...
+OP(multi_linear_bwd) {                           // x rows, weights, gradients, want dx, want each dw -> dx, dw...
   return entry(py, np, [](Args& a) {
     const Tensor& x2 = a.t();
     const List ws = a.ts(), dys = a.ts();
     const bool want_x = a.b();
-    const long want_w = a.l();
+    const std::vector<bool> want_w = a.bools();
+    TORCH_CHECK_VALUE(dys.size() == ws.size() && want_w.size() == ws.size(), "_nsa_host: as many gradients as weights");
     return [=]() -> List {
       List r(1 + ws.size());
       std::vector<int64_t> shape;
@@ -536,7 +544,7 @@ OP(multi_linear_bwd) {                           // x rows, weights, gradients, 
           if (!r[0].defined()) { r[0] = gemm(dy, ws[i], false, true); shape = dys[i].sizes().vec(); }
           else gemm(dy, ws[i], false, true, r[0], BF, true, 0, 1);
         }
-        if (want_w >> i & 1) r[1 + i] = gemm(dy, x2, true, true);
+        if (want_w[i]) r[1 + i] = gemm(dy, x2, true, true);
       }
       if (r[0].defined()) r[0] = in_shape(r[0], shape, x2.size(1));
       return r;

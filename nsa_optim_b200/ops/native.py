@@ -273,7 +273,7 @@ class _Linear(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy: Tensor):
         x2, w = ctx.saved_tensors
-        return _host.multi_linear_bwd(x2, (w,), (dy,), ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        return _host.multi_linear_bwd(x2, (w,), (dy,), ctx.needs_input_grad[0], ctx.needs_input_grad[1:])
 
 
 class _MultiLinear(torch.autograd.Function):
@@ -295,8 +295,7 @@ class _MultiLinear(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *dys):
         x2, *ws = ctx.saved_tensors
-        wanted = sum(1 << i for i, need in enumerate(ctx.needs_input_grad[2:]) if need)
-        dx, *dws = _host.multi_linear_bwd(x2, tuple(ws), dys, ctx.needs_input_grad[0], wanted)
+        dx, *dws = _host.multi_linear_bwd(x2, tuple(ws), dys, ctx.needs_input_grad[0], ctx.needs_input_grad[2:])
         return (dx, None, *dws)
 
 
@@ -357,7 +356,7 @@ class _LinearGather(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x2, w = ctx.saved_tensors
-        return (*_host.multi_linear_bwd(x2, (w,), (dy,), ctx.needs_input_grad[0], ctx.needs_input_grad[1]), None)
+        return (*_host.multi_linear_bwd(x2, (w,), (dy,), ctx.needs_input_grad[0], ctx.needs_input_grad[1:2]), None)
 
 
 def linear(x: Tensor, w: Tensor) -> Tensor:

@@ -129,3 +129,14 @@ def test_flags_of_any_kind(native):
         out = torch.ones(40, 24, device="cuda")
         want = native.gemm(a, b, True, True, out=out.clone(), accumulate=on)
         assert torch.equal(native.gemm(a, b, np.True_, np.True_, out=out.clone(), accumulate=np.bool_(on)), want)
+
+
+def test_more_than_64_projections_of_one_input(native):
+    g = torch.Generator("cuda").manual_seed(0)
+    x = torch.randn(200, 64, device="cuda", generator=g).bfloat16().requires_grad_()
+    ws = [torch.randn(8, 64, device="cuda", generator=g).bfloat16().requires_grad_(i > 3) for i in range(67)]
+    ys = native.multi_linear(x, ws)
+    wanted = [w for w in ws if w.requires_grad]
+    got = torch.autograd.grad(ys, wanted, [torch.ones_like(y) for y in ys])
+    one = torch.autograd.grad(native.linear(x, wanted[0]), wanted[0], torch.ones_like(ys[0]))[0]
+    assert all(torch.equal(w, one) for w in got)         # all of them x summed over its rows
