@@ -77,3 +77,31 @@ def test_selected(native, B, T, Hq, Hkv):
     seen = took[..., :nS].repeat_interleave(64, -1)[..., :T] & (t[None, :] <= t[:, None])
     got, want = native.selected_attention(q, k, v, idx).double(), _reference(q.double(), k.double(), v.double(), seen)
     assert (got - want).norm() <= 3 * 2 ** -9 * want.norm()
+
+
+# Keys of 32 tokens every 16: the first 31 tokens see none (L = -inf).  32 tokens have one key; a group of 32 heads over 2100 tokens has more than 256
+# query tiles, whose sums meet in memory
+@pytest.mark.parametrize("walks", [None, 1, 3])
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 32, 4, 2), (2, 300, 16, 8), (1, 1000, 16, 1), (1, 2080, 8, 4), (1, 2100, 32, 1)])
+def test_compressed_keys(native, monkeypatch, B, T, Hq, Hkv, walks):
+    if walks:
+        monkeypatch.setattr(native.load(), "nsa_attn_bwd_walks_d64", lambda *args: walks)
+    g = torch.Generator("cuda").manual_seed(T)
+    S = (T - 32) // 16 + 1
+    mk = lambda t, h: torch.randn(B, t, h, 64, device="cuda", generator=g).bfloat16().requires_grad_()      # noqa: E731
+    x, dy = [mk(T, Hq), mk(S, Hkv), mk(S, Hkv)], mk(T, Hq).detach()
+    seen = torch.arange(S, device="cuda")[None, :] * 16 + 31 <= torch.arange(T, device="cuda")[:, None]
+    y, L = native._Attn.apply(*x, True, 0, 0.125, 16, 31, None)
+    got = [y.detach()] + list(torch.autograd.grad(y, x, dy))
+    ref = [t.detach().double().requires_grad_() for t in x]
+    # unseen keys at -1e30 and not -inf, whose softmax over nothing has no gradient; its result is taken out afterwards
+    G = Hq // Hkv
+    q, k, v = ref[0].transpose(1, 2), *(t.transpose(1, 2).repeat_interleave(G, 1) for t in ref[1:])
+    s = (q @ k.transpose(-1, -2) * 0.125).masked_fill(~seen, -1e30)
+    w = ((s.softmax(-1) * seen) @ v).transpose(1, 2)
+    want = [w.detach()] + list(torch.autograd.grad(w, ref, dy.double()))
+    native.check_status()
+    assert torch.isneginf(L[:, :31]).all() and torch.isfinite(L[:, 31:]).all()
+    assert not y[:, :31].any() and not got[1][:, :31].any()
+    for a, b in zip(got, want):                    # as in _check; S = 1: score gradients are differences of equal sums
+        assert (a.double() - b).norm() <= 3 * 2 ** -9 * b.norm() + 2 ** -18 * a.numel() ** 0.5
