@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "nsa_b200.h"
 #include "status.cuh"
 
 enum : int {

@@ -22,6 +22,11 @@ int nsa_sm_count(void);
 int nsa_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                   int a_mn, int b_mn, int out_fp32, int accumulate, int max_ctas, cudaStream_t stream);
 
+/* Kernel of plain GEMMs from now on: 0 default, 1 one CTA per tile, 2 CTA pairs. */
+void nsa_gemm_select(int which);
+/* CTA pairs that run at once. */
+int nsa_gemm_pair_clusters(void);
+
 /* mode 0: y = rmsnorm(x) w; 1: rmsnorm(x) w silu(gate); 2: rmsnorm(x silu(gate)) w. */
 int nsa_rmsnorm_fwd(const void* x, const void* gate, const void* w, void* y, float* rstd, long rows, int d,
                     float eps, int mode, cudaStream_t st);
