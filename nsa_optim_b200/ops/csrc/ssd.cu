@@ -1543,14 +1543,15 @@ extern "C" int nsa_ssd_finish(const float* dB_part, const float* dC_part, const 
   return e == cudaSuccess ? 0 : nsa::fail_cuda(e, "nsa_ssd_finish launch");
 }
 
-// One pass over the chunks (nsa_ssd_states) or chunk_state and the state pass.  The walk is counted with 3.2 us and 1.13 a chunk for up to one
-// head per SM, which it has since become 0.2 a chunk faster than; the line matters beyond half as many heads as SMs (see below).  The two kernels take 6.6 us and 0.095 a chunk (the pass is a chain), 5.1 and 0.0165 per (chunk, head), or 0.019 per
-// (chunk, head), whichever is the most, and have a gap between them.  Walk and two kernels, us: 300 tokens x 1 head 6.3, 6.7;
-// 1000 x 1 11.1, 6.6; 1000 x 32 12.0, 9.1; 1000 x 48 12.3, 11.4; 777 x 64 11.0, 12.9; 1500 x 64 17, 19.2; 1000 x 128 13.4, 22.1;
-// 16384 x 48 141, 121; 16384 x 64 141, 169; 2 x 8192 x 32 72, 83.
+// One pass over the chunks (nsa_ssd_states) or chunk_state and the state pass.  The walk is counted with 3.2 us, and 1.13 a chunk for each head
+// per SM: 0.2 more than a chunk has come to take, which decides nothing, as up to half as many heads as SMs have the halves below for
+// where it would, and beyond that the walk is the faster form at every length.  The two kernels take 6.6 us and 0.095 a chunk (the pass is a
+// chain), 5.1 and 0.0165 per (chunk, head), or 0.019 per (chunk, head), whichever is the most, and have a gap between them.  Walk and two
+// kernels, us: 1300 tokens x 1 head 12.5, 7.3; 2000 x 24 17.2, 11.4; 4000 x 32 31, 20.5; 300 x 75 5.8, 9.3; 4000 x 75 31, 50; 1000 x 128 10.6,
+// 20.8; 200 x 149 8.1, 11.2 (a head more than SMs: the start is not paid again); 3000 x 149 51, 72; 129 x 320 11.7, 18.2; 4000 x 320 105, 195.
 extern "C" int nsa_ssd_states_in_one(int B, int T, int H) {
   const long heads = static_cast<long>(B) * H, chunks = (T + L - 1) / L, items = heads * chunks, sms = nsa::sm_count();
-  const double walk = (3.2 + 1.13 * chunks) * ((heads + sms - 1) / sms);
+  const double walk = 3.2 + 1.13 * chunks * ((heads + sms - 1) / sms);
   return walk <= std::max({6.6 + 0.095 * chunks, 5.1 + 0.0165 * items, 0.019 * items}) + 0.5;
 }
 

@@ -19,3 +19,16 @@ def test_halves(native, B, T, H, skip):
 def test_form(native, B, T, H, form):
     if torch.cuda.get_device_properties(0).multi_processor_count == 148:
         assert native.load().nsa_ssd_states_form(B, T, H) == form
+
+
+# the kernels that run: by the time of both forms where heads are few, one walk beyond half as many heads as SMs, a head more than SMs among them
+@pytest.mark.parametrize("B,T,H,form", [(1, 300, 1, 2), (1, 1000, 1, 2), (1, 1300, 1, 0), (1, 1000, 48, 2), (1, 777, 64, 2), (1, 4000, 32, 0), (1, 16384, 48, 2),
+                                        (1, 300, 75, 1), (1, 16384, 148, 1), (1, 129, 149, 1), (1, 300, 149, 1), (2, 200, 80, 1), (3, 129, 99, 1),
+                                        (4, 8000, 80, 1)])
+def test_form_by_heads(native, B, T, H, form):
+    test_form(native, B, T, H, form)
+
+
+@pytest.mark.parametrize("B,T,H,skip", [(1, 300, 149, True), (3, 129, 99, False)])
+def test_more_heads_than_sms(native, B, T, H, skip):
+    _check(native, B, T, H, skip)
