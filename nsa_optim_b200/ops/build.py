@@ -19,6 +19,7 @@ import os
 import shutil
 import subprocess
 import sys
+import threading
 from typing import List
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -66,24 +67,38 @@ def _compile(nvcc: str, name: str, extra: List[str], verbose: bool, obj_dir: str
 
 def build_host(force: bool = False) -> str:
     """Builds ``_nsa_host.so`` (``csrc/host_ops.cpp``), the host side of the ops against PyTorch's C++ interface.  It finds the kernel
-    library's entry points when ``ops/native.py`` binds it, so one build serves release and debug libraries."""
-    src = os.path.join(SRC, "host_ops.cpp")
-    deps = [src, os.path.join(SRC, "nsa_b200.h")]
-    if not force and os.path.exists(HOST) and os.path.getmtime(HOST) >= max(map(os.path.getmtime, deps)):
-        return HOST
+    library's entry points when ``ops/native.py`` binds it, so one build serves release and debug libraries.  Built again when a source is
+    newer, and when PyTorch, Python or the flags are others than it was built with (``_build/_nsa_host.stamp``)."""
     import sysconfig
 
     import torch
+    src = os.path.join(SRC, "host_ops.cpp")
+    deps = [src, os.path.join(SRC, "nsa_b200.h")]
     base = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(nvcc_path()))
     dirs = [SRC, os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
             os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
-    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared"] + [x for d in dirs for x in ("-I", d)]
-           + [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", src, "-o", HOST, "-L", os.path.join(base, "lib"),
-              "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ldl"])
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"g++ failed for host_ops.cpp:\n{r.stdout}\n{r.stderr}")
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    libs = ["-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ldl"]
+    made_with = "\n".join([torch.__version__, str(torch.version.git_version), sys.version, str(sysconfig.get_config_var("SOABI"))] + flags + libs)
+    stamp = os.path.join(OBJ, "_nsa_host.stamp")
+    if not force and os.path.exists(HOST) and os.path.getmtime(HOST) >= max(map(os.path.getmtime, deps)) and os.path.exists(stamp):
+        with open(stamp) as f:
+            if f.read() == made_with:
+                return HOST
+    os.makedirs(OBJ, exist_ok=True)
+    part = os.path.join(OBJ, f"_nsa_host.{os.getpid()}.{threading.get_ident()}.so")      # another process may be loading the one that is there
+    cmd = ["g++"] + flags + [x for d in dirs for x in ("-I", d)] + [src, "-o", part, "-L", os.path.join(base, "lib")] + libs
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed for host_ops.cpp:\n{r.stdout}\n{r.stderr}")
+        os.replace(part, HOST)
+    finally:
+        if os.path.exists(part):
+            os.remove(part)
+    with open(stamp, "w") as f:
+        f.write(made_with)
     return HOST
 
 
