@@ -1065,10 +1065,11 @@ class _SSD(torch.autograd.Function):
 def _gates(a, b, dt_bias, A_log):
     """The two results of one launch (``csrc/gates.cu``), or None where autograd records, the layout is another or a tensor
     is elsewhere, which PyTorch's expressions refuse or take as they do."""
-    f32, bf, dev = torch.float32, torch.bfloat16, a.device
-    if (a.dtype != bf or a.dim() < 2 or a.numel() == 0 or dt_bias.dtype not in (f32, bf) or A_log.dtype not in (f32, bf)
-            or dt_bias.shape != a.shape[-1:] or A_log.shape != a.shape[-1:] or (b is not None and (b.dtype != bf or b.shape != a.shape or b.device != dev))
-            or dt_bias.device != dev or A_log.device != dev or _recorded((a, b, dt_bias, A_log))):
+    f32, bf, shape, at = torch.float32, torch.bfloat16, a.shape, a.get_device()
+    row = shape[-1:]
+    if (a.dtype != bf or len(shape) < 2 or a.numel() == 0 or dt_bias.dtype not in (f32, bf) or A_log.dtype not in (f32, bf)
+            or dt_bias.shape != row or A_log.shape != row or dt_bias.get_device() != at or A_log.get_device() != at
+            or (b is not None and (b.dtype != bf or b.shape != shape or b.get_device() != at)) or _recorded((a, b, dt_bias, A_log))):
         return None
     return _h().gates(a, b, dt_bias, A_log)
 

@@ -2,6 +2,7 @@
 forward-mode derivative's, tracer's or compiler's."""
 import pytest
 import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
 from torch.autograd import forward_ad
 
 from nsa_optim_b200.ops import native
@@ -67,8 +68,9 @@ def test_transforms_see_the_function(applied, monkeypatch, grad):
 def test_gates_of_tensors_on_several_devices_are_left_to_pytorch(monkeypatch, elsewhere):
     calls = []
     monkeypatch.setattr(native, "_h", lambda: type("Host", (), {"gates": lambda self, *a: calls.append(a) or "launched"})())
-    t = {n: torch.zeros(*s, dtype=torch.bfloat16, device="cpu" if n == elsewhere else "meta")
-         for n, s in (("a", (1, 4, 8)), ("b", (1, 4, 8)), ("dt_bias", (8,)), ("A_log", (8,)))}
+    with FakeTensorMode():                               # stand-ins for tensors of a GPU
+        t = {n: torch.empty(*s, dtype=torch.bfloat16, device="cpu" if n == elsewhere else "cuda:0")
+             for n, s in (("a", (1, 4, 8)), ("b", (1, 4, 8)), ("dt_bias", (8,)), ("A_log", (8,)))}
     assert native.delta_gates(**t) == (None if elsewhere else "launched")
     del t["b"]
     assert native.step_sizes(t["a"], t["dt_bias"], t["A_log"]) == (None if elsewhere in ("dt_bias", "A_log") else "launched")
