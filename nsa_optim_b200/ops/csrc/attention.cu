@@ -486,7 +486,7 @@ __device__ __forceinline__ void q_half_to_tmem(uint32_t taddr, const uint8_t* ti
 }
 
 // --------------------------------------------------------------------------------------
-// Forward, warp-specialised, Q and P in tensor memory (head_dim 128, output mode).  Visits are
+// Forward, warp-specialised, Q and P in tensor memory (output mode).  Visits are
 // 64-key blocks as in the dQ kernel.  Warp 8 streams K/V through a 5-stage ring, warp 9 issues
 // S = Q K^T and warp 10 issues O += P V.  Q is copied once into TMEM and each softmax group writes
 // its probabilities into TMEM columns of its own, so both MMAs take their A operand from TMEM and
@@ -3789,7 +3789,7 @@ extern "C" int nsa_attn_bwd_walks_d64(int B, int T, int S, int Hq, int Hkv, int 
 // Selected mode additionally takes the inverse selection map: tok_list (tokens grouped by
 // (b, h, block), ascending), list_start / item_start ([B*Hkv*nS + 1] exclusive prefixes of list
 // lengths and of CTAs per list, a CTA covering visits_per_cta * (128 / G) tokens) and
-// item_bound >= item_start[last].  head_dim 128 only; selected mode needs G >= 8.
+// item_bound >= item_start[last].  Selected mode and 64 keys a CTA (walks -1) need head_dim 128, selected mode G >= 8 as well.
 // delta_given: delta holds rowsum(dO * O) already (the gated combine's backward has both tensors in registers).
 // walks, part: of nsa_attn_bwd_walks (contiguous ranges).
 // add_dq: dQ is added to what dq holds.  dK / dV add to what the caller put there (fp32), or with write_kv are bf16 tensors that

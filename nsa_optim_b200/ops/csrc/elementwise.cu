@@ -1289,8 +1289,8 @@ extern "C" int nsa_rope(const void* x, const float* cos_t, const float* sin_t, v
 // Channel tiles of a CTA.
 static int conv_tiles(int C) { return C <= CT_C ? 1 : 2; }
 // Time steps per warp: 64 keeps the rows read twice (3 of x ahead of a segment, 3 of dpre behind it) under
-// a tenth; short sequences take 32, 16 or 8 so that every SM still finds 32 warps; beyond 8.4 M steps (of two segments
-// a CTA) 128 or 256, so that the grid's second dimension (at most 65535) reaches as far as 33.5 M.
+// a tenth; short sequences take 32, 16 or 8 so that every SM still finds 32 warps; beyond 16.8 M steps (of four segments
+// a CTA, eight up to 128 channels) 128 or 256, so that the grid's second dimension (at most 65535) reaches as far as 67 M.
 static int conv_rows(int B, int T, int C) {
   int rows = 64;
   while (rows < 256 && static_cast<long>(rows) * (CT_WARPS / conv_tiles(C)) * 65535 < T) rows <<= 1;

@@ -1,8 +1,9 @@
-"""ctypes bindings and autograd wrappers for the sm_100a kernels in ``ops/csrc``.
+"""Autograd wrappers for the sm_100a kernels in ``ops/csrc``.
 
 The shared library ``libnsa_b200.so`` lives beside this file (built by ``ops/build.py``) and
 exports plain C entry points that take device pointers, sizes and a stream; output tensors
-are allocated here with PyTorch.  Each differentiable op is one ``autograd.Function`` whose
+are allocated with PyTorch, by the extension module ``_nsa_host`` (``csrc/host_ops.cpp``) for most ops and here
+for the others, whose entry points are called through ctypes.  Each differentiable op is one ``autograd.Function`` whose
 forward and backward both call native kernels.  ``SUPPORTED`` lists the ops that have a
 native implementation; ``ops/__init__.py`` consults :func:`supports`.
 
