@@ -254,7 +254,8 @@ def gemm(a: Tensor, b: Tensor, a_mn: bool, b_mn: bool, out: Optional[Tensor] = N
     True -> B is (K, N).  Row pitches may exceed the logical width (sliced views).  ``split_k``
     (default: chosen by :func:`split_k_choice`) cuts the reduction into parts that run on different
     CTA pairs and meet in fp32 through TMA reduce-add stores."""
-    return _h().matmul(a, b, int(a_mn), int(b_mn), out, out_dtype, int(accumulate), max_ctas, split_k or 0)
+    parts = 0 if split_k is None else max(split_k, 1)        # 0: to be chosen
+    return _h().matmul(a, b, int(a_mn), int(b_mn), out, out_dtype, int(accumulate), max_ctas, parts)
 
 
 def gemm_select(which: str = "default") -> None:

@@ -180,3 +180,16 @@ def test_multi_linear_matches_separate_linears(native):
     ref = sum(g.float().view(T, -1) @ w.float() for g, w in zip(gs, ws)).view(1, T, d)
     assert (dx.float() - ref).abs().max().item() <= 2e-2 * ref.abs().max().item() + 1e-2
     assert (x.grad.float() - ref).abs().max().item() <= 2e-2 * ref.abs().max().item() + 1e-2
+
+
+@pytest.mark.parametrize("parts", [0, -3, 1])
+def test_a_reduction_that_is_not_to_be_cut(native, parts):
+    # 1024 x 512 tiles are few and the reduction is long: left to choose, it is cut in two
+    M, N, K = 1024, 512, 65536
+    assert native.split_k_choice(M, N, K) == 2
+    g = torch.Generator("cuda").manual_seed(0)
+    a, b = (torch.randn(K, n, device="cuda", generator=g).bfloat16() for n in (M, N))
+    one, two = (native.gemm(a, b, True, True, out_dtype=torch.float32, split_k=s) for s in (1, 2))
+    assert not torch.equal(one, two)
+    assert torch.equal(native.gemm(a, b, True, True, out_dtype=torch.float32, split_k=parts), one)
+    assert torch.equal(native.gemm(a, b, True, True, out_dtype=torch.float32), two)
