@@ -165,6 +165,14 @@ struct Args {
   }
   int w() { return static_cast<int>(l()); }
   bool b() { return l() != 0; }
+  int flag() {                                   // as int() takes it: NumPy's truth values are not integers
+    PyObject* o = next();
+    if (o == Py_True) return 1;
+    if (o == Py_False) return 0;
+    THPObjectPtr n(PyNumber_Long(o));
+    if (!n) throw python_error();
+    return static_cast<int>(PyLong_AsUnsignedLongMask(n.get()));
+  }
   float f() {
     const double v = PyFloat_AsDouble(next());
     if (v == -1.0 && PyErr_Occurred()) throw python_error();
@@ -384,7 +392,7 @@ OP(conv_fwd) {                                   // x, w, bias or None, activati
   return entry(py, np, [](Args& a) {
     const Tensor &x = a.t(), &w = a.t();
     const Tensor bias = a.opt();
-    const int act = a.w();
+    const int act = a.flag();
     return [=]() -> List {
       want_dims(x, 3);
       const long B = x.size(0), T = x.size(1), C = x.size(2);
@@ -402,7 +410,7 @@ OP(conv_bwd) {                                   // x rows, w, bias or None, dy,
     const Tensor &x = a.t(), &w = a.t();
     const Tensor bias = a.opt();
     const Tensor& dy = a.t();
-    const int act = a.w();
+    const int act = a.flag();
     const auto wtype = a.dtype();
     return [=]() -> List {
       const long B = x.size(0), T = x.size(1), C = x.size(2), W = w.size(-1);
@@ -493,10 +501,10 @@ Tensor in_shape(const Tensor& g, std::vector<int64_t> shape, int64_t last) {
 OP(matmul) {                                     // a, b, a_mn, b_mn, out or None, dtype, accumulate, max_ctas, parts -> C
   return entry(py, np, [](Args& g) {
     const Tensor &a = g.t(), &b = g.t();
-    const bool a_mn = g.b(), b_mn = g.b();
+    const bool a_mn = g.flag(), b_mn = g.flag();
     const Tensor out = g.opt();
     const auto type = g.dtype();
-    const bool accumulate = g.b();
+    const bool accumulate = g.flag();
     const int max_ctas = g.w();
     const long parts = g.l();
     return [=]() -> Tensor { return gemm(a, b, a_mn, b_mn, out, type, accumulate, max_ctas, parts); };
@@ -598,7 +606,7 @@ struct Range {                                   // causal, window, scale, kp_st
   float scale;
   int kp_stride, kp_off;
   static Range of(Args& a) {
-    const int causal = a.w(), window = a.w();
+    const int causal = a.flag(), window = a.w();
     const float scale = a.f();
     const int kp_stride = a.w(), kp_off = a.w();
     return {causal, window, scale, kp_stride, kp_off};

@@ -255,7 +255,7 @@ def gemm(a: Tensor, b: Tensor, a_mn: bool, b_mn: bool, out: Optional[Tensor] = N
     (default: chosen by :func:`split_k_choice`) cuts the reduction into parts that run on different
     CTA pairs and meet in fp32 through TMA reduce-add stores."""
     parts = 0 if split_k is None else max(split_k, 1)        # 0: to be chosen
-    return _h().matmul(a, b, int(a_mn), int(b_mn), out, out_dtype, int(accumulate), max_ctas, parts)
+    return _h().matmul(a, b, a_mn, b_mn, out, out_dtype, accumulate, max_ctas, parts)
 
 
 def gemm_select(which: str = "default") -> None:
@@ -547,7 +547,6 @@ def rope(x, cos, sin):
 class _Conv1d(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, activation):
-        activation = int(activation)                     # any truth value: NumPy's are not integers
         y, xv, wb, bb = _h().conv_fwd(x, weight, bias, activation)
         ctx.save_for_backward(xv, wb, bb)
         ctx.activation, ctx.wdtype = activation, weight.dtype
@@ -746,7 +745,7 @@ class _Attn(torch.autograd.Function):
         split = _bwd_is_split(D, Hq // Hkv, tiles is not None)
         if split and tiles is None:
             walks_of = load().nsa_attn_bwd_walks if D == 128 else load().nsa_attn_bwd_walks_d64
-            walks = walks_of(B, T, S, Hq, Hkv, causal, window, kp_stride)
+            walks = walks_of(B, T, S, Hq, Hkv, int(causal), window, kp_stride)
         elif split:
             lists = _inverse_of(tiles, Hq // Hkv, visits)
         return (*_host.attn_bwd(q, k, v, o, do, L, *ctx.cfg, tiles, lists, visits, walks, split), None, None, None, None, None, None)
@@ -763,7 +762,7 @@ def attention(q, k, v, causal=True, window=0, scale=None):
         _fallback("attention")
         return torch_impl.attention(q, k, v, causal, window, scale)
     scale = q.shape[-1] ** -0.5 if scale is None else scale
-    return _run(_Attn, q, k, v, int(causal), int(window), float(scale), 1, 0, None)[0]
+    return _run(_Attn, q, k, v, causal, int(window), float(scale), 1, 0, None)[0]
 
 
 def union_blocks(idx: Tensor, G: int, nS: int):
